@@ -109,6 +109,22 @@ SYMBOLS = {
 }
 
 _LIB = None
+_HOST = None
+
+
+def host():
+    """The native half of the Python entry points (_host.so), loaded once; ``RuntimeError`` when it is not there."""
+    global _HOST
+    if _HOST is None:
+        load()
+        try:
+            import torch  # noqa: F401  (the module links torch's libraries)
+            from . import _host
+        except ImportError as e:
+            raise RuntimeError(f"{PKG}/_host.so cannot be loaded ({e}): build it with `python -m "
+                               "open_ommx_serve_b200.build`. There is no slower path.") from e
+        _HOST = _host
+    return _HOST
 
 
 def load():

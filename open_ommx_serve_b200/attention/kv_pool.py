@@ -47,7 +47,7 @@ import torch
 
 from .. import _lib
 from .kv_window import WindowSpec
-from .pack import alloc_planes, ommx_pack_kv_into, planes_struct
+from .pack import alloc_planes, ommx_pack_kv_into
 
 _CAPTURED_WRITE_CHECK = os.environ.get("OMMX_KV_CAPTURED_WRITE_CHECK", "1").strip().lower() not in {"0", "false", "off", "no"}
 
@@ -172,49 +172,24 @@ class MultiSeqKVPool:
 
     _ring_row = _ring_slot_dev
 
-    def _pool_struct(self, a_pool) -> None:
-        a_pool.planes = planes_struct(self.planes, k=self.k, outlier_map=self.kv_outlier_map)
-        a_pool.k_hist, a_pool.v_hist = self.k_hist.data_ptr(), self.v_hist.data_ptr()
-        a_pool.num_seqs, a_pool.ring_cap = self.num_seqs, self.ring_cap
-        a_pool.sink_tokens, a_pool.recent_window = self.sink, self.recent
-        a_pool.seq_len = self.seq_dev.data_ptr()
-        a_pool.req_to_token, a_pool.req_to_group = self._req_to_token.data_ptr(), self._req_to_group.data_ptr()
-        a_pool.pages_per_seq, a_pool.groups_per_seq = self.P_per_seq, self.G_per_seq
-
-    def _append_args(self, B: int, advance, K=None, V=None, *, slots=None, write_pos=None, outputs=True) -> "_lib.KVAppendArgs":
-        a = _lib.KVAppendArgs()
-        self._pool_struct(a.pool)
-        if K is not None:
-            a.k_new, a.v_new = K.data_ptr(), V.data_ptr()
-            a.new_stride_b, a.new_stride_h = int(K.stride(0)), int(K.stride(1))
+    def _append_args(self, B: int, advance, K=None, V=None, *, slots=None, write_pos=None, outputs=True) -> tuple:
+        """The arguments of one store call, checked; ``_call`` runs it."""
         if slots is None and write_pos is None:
-            a.slots = None if self._sel is None else self._sel.data_ptr()
             if self._sel is not None and int(B) != int(self._sel.numel()):
                 raise ValueError(f"batch {B} does not match the {int(self._sel.numel())} selected slots")
         else:
-            is64 = {torch.int64: 1, torch.int32: 0}
             dt = (slots if slots is not None else write_pos).dtype
-            if dt not in is64 or (slots is not None and write_pos is not None and slots.dtype != write_pos.dtype):
+            if dt not in (torch.int64, torch.int32) or (slots is not None and write_pos is not None and slots.dtype != write_pos.dtype):
                 raise ValueError("slot / position index tensors must both be int32 or both int64")
             for t in (slots, write_pos):
                 if t is not None and (not t.is_cuda or not t.is_contiguous() or int(t.numel()) != int(B)):
                     raise ValueError(f"slot / position index tensors must be contiguous CUDA tensors of {B} entries")
-            a.slots = None if slots is None else slots.data_ptr()
-            a.write_pos = None if write_pos is None else write_pos.data_ptr()
-            a.index_is_int64 = is64[dt]
-        a.batch, a.advance = int(B), int(advance)
-        a.outlier_select, a.use_pow2 = 1, 1
-        if outputs:
-            a.k_tail, a.v_tail, a.max_tail = self.k_tail.data_ptr(), self.v_tail.data_ptr(), self.max_tail_len
-            a.b_seq_len, a.b_tail_len = self.b_seq.data_ptr(), self.b_tail.data_ptr()
-        a.status = self.status.data_ptr()
-        return a
+        return B, advance, K, V, slots, write_pos, outputs
 
-    def _call(self, a) -> None:
-        lib = _lib.load()
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            _lib.check(lib.ommx_b200_kv_append_decode(a, stream), "ommx_b200_kv_append_decode")
+    def _call(self, a: tuple) -> None:
+        rc = _lib.host().kv_append(self, *a)
+        if rc:
+            _lib.check(rc, "ommx_b200_kv_append_decode")
 
     def _rows(self, K: torch.Tensor, V: torch.Tensor, B: int):
         K, V = K.reshape(B, self.H, self.D), V.reshape(B, self.H, self.D)
@@ -385,20 +360,14 @@ class MultiSeqKVPool:
                 "kv_outlier_map": bool(self.kv_outlier_map), "kv_int8_scale": True}
 
     def _gather_tail(self, sel, tidx, kt, vt) -> None:
-        lib = _lib.load()
-        pool = _lib.KVPool()
-        self._pool_struct(pool)
         B, T = int(tidx.shape[0]), int(tidx.shape[1])
         if tidx.dtype not in (torch.int32, torch.int64) or (sel is not None and sel.dtype != tidx.dtype):
             raise ValueError("sel / tail index tensors must both be int32 or both int64")
         if tuple(kt.shape) != (B, T, self.H, self.D) or not kt.is_contiguous() or not vt.is_contiguous() or tuple(vt.shape) != tuple(kt.shape):
             raise ValueError(f"k_tail / v_tail must be contiguous [{B}, {T}, {self.H}, {self.D}]")
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            _lib.check(lib.ommx_b200_kv_gather_tail(pool, None if sel is None else sel.contiguous().data_ptr(),
-                                                    tidx.contiguous().data_ptr(), 1 if tidx.dtype == torch.int64 else 0,
-                                                    B, T, kt.data_ptr(), vt.data_ptr(), self.status.data_ptr(), stream),
-                       "ommx_b200_kv_gather_tail")
+        rc = _lib.host().kv_gather_tail(self, sel, tidx, kt, vt)
+        if rc:
+            _lib.check(rc, "ommx_b200_kv_gather_tail")
 
     def tail_bf16_batched(self, slots: Sequence[int]):
         """``(k_tail [B,T,H,D], v_tail, b_tail_len [B])`` of the listed requests: sink and recent rows, zero

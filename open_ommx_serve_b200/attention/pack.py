@@ -130,36 +130,32 @@ def ommx_pack_kv_into(K, V, planes: dict, *, dst_pages=None, dst_groups=None,
     (``None`` = 0,1,2,...).  No host synchronisation; errors the device sees (page or slot out of
     range, non-finite input) are OR-ed into ``status`` (int32 ``[1]``) when it is given.
     """
-    lib = _lib.load()
+    rc = _lib.host().pack_into(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, use_pow2,
+                               kv_outlier_map, status)
+    if rc is None:
+        _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, kv_outlier_map)
+    if rc:
+        _lib.check(rc, "ommx_b200_pack_kv")
+
+
+def _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, kv_outlier_map):
+    """The exception for arguments the host module declined: the same conditions, one by one.  Always raises."""
     if not K.is_cuda:
         raise RuntimeError("ommx_pack_kv_into needs CUDA tensors (no CPU path)")
     if tuple(K.shape) != tuple(V.shape) or K.dim() != 3:
         raise ValueError(f"K/V shape mismatch: {tuple(K.shape)} vs {tuple(V.shape)}")
     if K.dtype != V.dtype:
         raise ValueError("K and V must share a dtype")
-    if K.stride(-1) != 1 or V.stride(-1) != 1 or K.stride() != V.stride():
-        K, V = K.contiguous(), V.contiguous()
-    sel = str(outlier_select).lower()
-    if sel not in ("signed", "abs"):
+    if str(outlier_select).lower() not in ("signed", "abs"):
         raise ValueError(f"outlier_select must be signed|abs; got {outlier_select!r}")
-    a = _lib.PackArgs()
-    a.k, a.v = K.data_ptr(), V.data_ptr()
-    a.in_dtype = _dtype_code(K)
-    a.num_tokens = int(K.shape[0])
-    a.stride_token, a.stride_head = int(K.stride(0)), int(K.stride(1))
+    _dtype_code(K)
     for name, t in (("dst_pages", dst_pages), ("dst_groups", dst_groups)):
         if t is not None and (t.dtype != torch.int32 or not t.is_cuda or not t.is_contiguous()):
             raise ValueError(f"{name} must be a contiguous int32 CUDA tensor")
-    a.dst_pages, a.dst_groups = _ptr(dst_pages), _ptr(dst_groups)
-    a.outlier_select = 1 if sel == "signed" else 0
-    a.use_pow2 = 1 if use_pow2 else 0
-    a.planes = planes_struct(planes, k=int(outliers_per_vector), outlier_map=bool(kv_outlier_map))
-    if a.planes.n_kv_heads != int(K.shape[1]) or a.planes.head_dim != int(K.shape[2]):
+    p = planes_struct(planes, k=int(outliers_per_vector), outlier_map=bool(kv_outlier_map))
+    if p.n_kv_heads != int(K.shape[1]) or p.head_dim != int(K.shape[2]):
         raise ValueError("K/V geometry does not match the destination planes")
-    a.status = _ptr(status)
-    with torch.cuda.device(K.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        _lib.check(lib.ommx_b200_pack_kv(a, stream), "ommx_b200_pack_kv")
+    raise ValueError("ommx_pack_kv_into: an argument has the wrong kind, rank or range")
 
 
 def ommx_pack_kv_canonical_block(
@@ -218,6 +214,8 @@ def ommx_pack_kv_canonical_block(
         raise ValueError(f"num_tokens={T} must be a multiple of {gt} and page_size")
     if D % gc != 0 or D % 4 != 0:
         raise ValueError(f"head_dim={D} must be a multiple of {gc}")
+    if str(outlier_select).lower() not in ("signed", "abs"):
+        raise ValueError(f"outlier_select must be signed|abs; got {outlier_select!r}")
     if k < 0 or k > gt:
         raise ValueError(f"outliers_per_vector={k} out of range [0, {gt}]")
     if k > 0 and repr_l == "combinadic":
@@ -237,33 +235,23 @@ def ommx_pack_kv_canonical_block(
     device = torch.device(device)
     Kd, Vd = K.to(device), V.to(device)
     use_map = bool(kv_outlier_map) and k > 0
-    planes = alloc_planes(T // int(page_size), T // gt, H, D, page_size=int(page_size),
-                          outliers_per_vector=k, kv_outlier_map=use_map,
-                          scale_kind=_scale_kind(scale_dtype, use_int8), device=device)
-    status = torch.zeros(1, dtype=torch.int32, device=device) if check_finite else None
-    ommx_pack_kv_into(Kd, Vd, planes, outliers_per_vector=k, outlier_select=outlier_select,
-                      use_pow2=bool(use_pow2), kv_outlier_map=use_map, status=status)
-    if check_finite:
-        bits = int(status.item())
-        if bits & _lib.ST_NONFINITE:
-            raise ValueError("KV pack: non-finite input (NaN/inf) - it would poison a whole group's scale")
-        if bits:
-            raise RuntimeError(f"KV pack: device reported {_lib.status_text(bits)}")
-    G, pages = T // gt, T // int(page_size)
-    if k > 0 and repr_l == "relidx7":
-        # same outlier set, other index encoding: k ascending 7-bit positions per frame (the value plane is shared)
-        lib = _lib.load()
-        oidx = torch.zeros(G, H, D, (7 * k + 7) // 8, dtype=torch.uint8, device=device)
-        with torch.cuda.device(device):
-            _lib.check(lib.ommx_b200_outlier_index_convert(planes["k_obmp"].data_ptr(), oidx.data_ptr(), G * H * D, k, 1, None,
-                                                           torch.cuda.current_stream().cuda_stream),
-                       "ommx_b200_outlier_index_convert")
-        planes["k_oidx"], planes["k_obmp"] = oidx, None
+    ran = _lib.host().pack_block(Kd, Vd, page_size, k, repr_l == "relidx7", str(outlier_select).lower() == "signed",
+                                 use_pow2, use_map, _scale_kind(scale_dtype, use_int8), check_finite)
+    if ran is None:
+        if Kd.dtype != Vd.dtype:
+            raise ValueError("K and V must share a dtype")
+        _dtype_code(Kd)
+        raise ValueError("ommx_pack_kv_canonical_block: an argument has the wrong kind, rank or range")
+    if isinstance(ran, int):
+        _lib.check(ran, "ommx_b200_pack_kv")
+    planes, bits = ran
+    if bits & _lib.ST_NONFINITE:
+        raise ValueError("KV pack: non-finite input (NaN/inf) - it would poison a whole group's scale")
+    if bits:
+        raise RuntimeError(f"KV pack: device reported {_lib.status_text(bits)}")
     planes.update({
         "k_field_bytes": (4 if repr_l == "bitmap" else (7 * k + 7) // 8) if k > 0 else 0,
-        "req_to_token": torch.arange(pages, dtype=torch.int32, device=device).reshape(1, pages),
-        "req_to_group": torch.arange(G, dtype=torch.int32, device=device).reshape(1, G),
-        "head_dim": D, "n_kv_heads": H, "num_tokens": T, "n_groups": G, "page_size": int(page_size),
+        "head_dim": D, "n_kv_heads": H, "num_tokens": T, "n_groups": T // gt, "page_size": int(page_size),
         "outliers_per_vector": k, "outlier_repr": repr_l, "outlier_select": str(outlier_select).lower(),
         "group_tokens": gt, "group_channels": gc, "k_format": kfmt, "v_format": vfmt,
         "k_base_bits": 2, "oval_bits": 4, "use_pow2": bool(use_pow2),

@@ -24,6 +24,7 @@ from .. import _lib
 from .pack import planes_struct
 
 _LAUNCHES = {"stage1": 0, "bitmap": 0, "abl": 0}
+_HOST = None                                   # the native half of the launcher, loaded at the first call
 
 ABL_FLAG_NAMES = ("OMMX_ABL_NO_OUTLIER", "OMMX_ABL_V_NODEQUANT", "OMMX_ABL_K_NODEQUANT",
                   "OMMX_ABL_NO_UNPACK",          # here bit 3 streams the planes and computes nothing
@@ -96,18 +97,6 @@ def _auto_num_kv_splits(seq_len: int, batch_size: int, device: Any = None, kv_he
     return int(lib.ommx_b200_auto_num_kv_splits(int(seq_len), int(batch_size), int(kv_heads)))
 
 
-def _make_attn_logits(batch, head_num, num_kv_splits, head_dim, device):
-    return torch.empty((batch, head_num, num_kv_splits, head_dim + 1), dtype=torch.float32, device=device)
-
-
-def _o_dtype(t: torch.Tensor) -> int:
-    if t.dtype == torch.float32:
-        return _lib.OMMX_DT_F32
-    if t.dtype == torch.bfloat16:
-        return _lib.OMMX_DT_BF16
-    raise NotImplementedError(f"o dtype {t.dtype}: float32 or bfloat16")
-
-
 def ommx_paged_decode_attention_canonical(
     q,
     k_base, k_scale, k_zp, k_oidx, k_oval,
@@ -166,7 +155,41 @@ def ommx_paged_decode_attention_canonical(
     (``sharding.PeerHeadGather.plan``); stage 2 then also stores this rank's rows into every rank's
     gathered buffer and returns when all ranks' rows of the layer have arrived in this rank's.
     """
-    lib = _lib.load()
+    host = _HOST or _load_host()
+    ran = host.decode(
+        q, k_base, k_scale, k_zp, k_oidx, k_oval, v_main, v_scale, v_zp, k_tail, v_tail, b_tail_len, o, lse, req_to_token,
+        req_to_group, b_seq_len, sm_scale, page_size, logit_cap, k_outliers_per_vector, k_format, combinadic_read, bitmap_read,
+        k_obmp, k_fp4_mapscale, k_fp4_mapcenter, kv_outlier_map, num_kv_splits, max_seq_len, max_tail_len, attn_logits,
+        packed_start_offset, seg_group_base, status, _stage, static_workspace, head_gather)
+    if ran is None:
+        _explain_refusal(
+            q, k_base, k_scale, k_zp, k_oidx, k_oval, v_main, v_scale, v_zp, k_tail, v_tail, b_tail_len, o, lse,
+            req_to_token, req_to_group, b_seq_len, page_size=page_size, k_outliers_per_vector=k_outliers_per_vector,
+            k_format=k_format, combinadic_read=combinadic_read, bitmap_read=bitmap_read, k_obmp=k_obmp,
+            k_fp4_mapscale=k_fp4_mapscale, k_fp4_mapcenter=k_fp4_mapcenter, kv_outlier_map=kv_outlier_map,
+            num_kv_splits=num_kv_splits, max_seq_len=max_seq_len, max_tail_len=max_tail_len, attn_logits=attn_logits,
+            packed_start_offset=packed_start_offset, seg_group_base=seg_group_base, _stage=_stage,
+            static_workspace=static_workspace, head_gather=head_gather)
+    if ran < 0:
+        _lib.check(ran, "ommx_b200_decode_static_ws" if static_workspace else "ommx_b200_decode")
+    if ran:
+        _LAUNCHES["abl"] |= ran          # ablation knobs in effect (differential timing only; a leaked export shows here)
+    _LAUNCHES["stage1"] += 1
+    if bitmap_read or env_truthy(os.environ.get("OMMX_VLLM_KV_BITMAP_READ")):
+        _LAUNCHES["bitmap"] += 1
+
+
+def _load_host():
+    global _HOST
+    _HOST = _lib.host()
+    return _HOST
+
+
+def _explain_refusal(q, k_base, k_scale, k_zp, k_oidx, k_oval, v_main, v_scale, v_zp, k_tail, v_tail, b_tail_len, o, lse,
+                     req_to_token, req_to_group, b_seq_len, *, page_size, k_outliers_per_vector, k_format, combinadic_read,
+                     bitmap_read, k_obmp, k_fp4_mapscale, k_fp4_mapcenter, kv_outlier_map, num_kv_splits, max_seq_len,
+                     max_tail_len, attn_logits, packed_start_offset, seg_group_base, _stage, static_workspace, head_gather):
+    """The exception for arguments the host module declined: the same conditions, one by one.  Always raises."""
     if not q.is_cuda:
         raise RuntimeError("ommx_paged_decode_attention_canonical needs CUDA tensors (no CPU path)")
     kfmt = str(k_format).lower()
@@ -243,10 +266,7 @@ def ommx_paged_decode_attention_canonical(
     if static_workspace:
         if int(_stage) != 0:
             raise ValueError("static_workspace=True runs both stages on the library's own workspace; _stage must be 0")
-        attn_logits = None
-    else:
-        if attn_logits is None:
-            attn_logits = _make_attn_logits(batch, head_num, num_kv_splits + 1, D, q.device)
+    elif attn_logits is not None:
         if attn_logits.dtype != torch.float32 or attn_logits.device != q.device or attn_logits.dim() != 4:
             raise ValueError("attn_logits must be a float32 [batch, heads, splits, head_dim+1] tensor on q's device")
         if int(attn_logits.shape[0]) < batch or int(attn_logits.shape[1]) < head_num:
@@ -267,22 +287,17 @@ def ommx_paged_decode_attention_canonical(
         raise NotImplementedError(f"q dtype {q.dtype}: this build serves bfloat16 queries")
     if q.stride(-1) != 1 or o.stride(-1) != 1:
         raise ValueError("q and o must have a unit last stride")
-    tables64 = req_to_token.dtype == torch.int64
     if req_to_token.dtype not in (torch.int32, torch.int64) or req_to_group.dtype != req_to_token.dtype:
         raise ValueError("req_to_token / req_to_group must both be int32 or both int64")
     if b_seq_len.dtype != torch.int32 or (b_tail_len is not None and b_tail_len.dtype != torch.int32):
         raise ValueError("b_seq_len / b_tail_len must be int32")
 
-    a = _lib.DecodeArgs()
-    a.q, a.q_dtype, a.batch, a.n_q_heads = q.data_ptr(), _lib.OMMX_DT_BF16, batch, head_num
-    a.q_stride_b, a.q_stride_h = int(q.stride(0)), int(q.stride(1))
-    planes = {"k_base": k_base, "k_scale": k_scale, "k_zp": k_zp, "k_obmp": k_obmp if (k > 0 and bitmap_read) else None,
-              "k_oidx": k_oidx if relidx7_read else None,
-              "k_oval": k_oval if k > 0 else None,
-              "k_fp4_mapscale": k_fp4_mapscale if use_map else None,
-              "k_fp4_mapcenter": k_fp4_mapcenter if use_map else None,
-              "v_main": v_main, "v_scale": v_scale, "v_zp": v_zp}
-    a.planes = planes_struct(planes, k=k, outlier_map=use_map, relidx7=relidx7_read)
+    planes_struct({"k_base": k_base, "k_scale": k_scale, "k_zp": k_zp, "k_obmp": k_obmp if (k > 0 and bitmap_read) else None,
+                   "k_oidx": k_oidx if relidx7_read else None,
+                   "k_oval": k_oval if k > 0 else None,
+                   "k_fp4_mapscale": k_fp4_mapscale if use_map else None,
+                   "k_fp4_mapcenter": k_fp4_mapcenter if use_map else None,
+                   "v_main": v_main, "v_scale": v_scale, "v_zp": v_zp}, k=k, outlier_map=use_map, relidx7=relidx7_read)
     if max_tail > 0:
         if k_tail is None or v_tail is None or b_tail_len is None:
             raise ValueError("max_tail_len > 0 needs k_tail, v_tail and b_tail_len")
@@ -290,44 +305,15 @@ def ommx_paged_decode_attention_canonical(
             raise NotImplementedError("k_tail / v_tail must be bfloat16")
         if k_tail.stride() != v_tail.stride() or k_tail.stride(-1) != 1:
             raise ValueError("k_tail and v_tail must share strides, with a unit last stride")
-        a.k_tail, a.v_tail = k_tail.data_ptr(), v_tail.data_ptr()
-        a.tail_stride_b, a.tail_stride_t, a.tail_stride_h = (int(s) for s in k_tail.stride()[:3])
-        a.b_tail_len = b_tail_len.data_ptr()
-    a.b_seq_len = b_seq_len.data_ptr()
-    a.req_to_token, a.req_to_group = req_to_token.data_ptr(), req_to_group.data_ptr()
-    a.table_is_int64 = 1 if tables64 else 0
-    a.r2t_stride_b, a.r2g_stride_b = int(req_to_token.stride(0)), int(req_to_group.stride(0))
-    a.o, a.o_dtype = o.data_ptr(), _o_dtype(o)
-    a.o_stride_b, a.o_stride_h = int(o.stride(0)), int(o.stride(1))
-    a.lse, a.lse_stride_b = lse.data_ptr(), int(lse.stride(0))
+    if o.dtype not in (torch.float32, torch.bfloat16):
+        raise NotImplementedError(f"o dtype {o.dtype}: float32 or bfloat16")
     if lse.dtype != torch.float32:
         raise ValueError("lse must be float32")
-    if attn_logits is not None:
-        a.attn_logits = attn_logits.data_ptr()
-        a.al_stride_b, a.al_stride_h, a.al_stride_s = (int(s) for s in attn_logits.stride()[:3])
-    a.num_kv_splits, a.max_seq_len, a.max_tail_len = num_kv_splits, max_seq, max_tail
-    a.seg_group_base, a.packed_start_offset = seg_group_base, start_offset
-    a.sm_scale, a.logit_cap = float(sm_scale), float(logit_cap)
-    a.status = None if status is None else status.data_ptr()
-    # ablation knobs (differential timing only; recorded so a leaked export cannot pass as served)
-    abl = sum(1 << i for i, n in enumerate(ABL_FLAG_NAMES) if env_truthy(os.environ.get(n)))
-    a.abl_flags = abl
-    if head_gather is not None:
-        if int(_stage) == 1:
-            raise ValueError("head_gather belongs to stage 2; _stage=1 runs stage 1 alone")
-        a.gather = head_gather.check(batch, head_num, D, q.device)
-    _LAUNCHES["abl"] |= abl
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        if static_workspace:
-            entry, what = lib.ommx_b200_decode_static_ws, "ommx_b200_decode_static_ws"
-        else:
-            entry = (lib.ommx_b200_decode, lib.ommx_b200_decode_stage1, lib.ommx_b200_decode_stage2)[int(_stage)]
-            what = "ommx_b200_decode"
-        _lib.check(entry(a, stream), what)
-    _LAUNCHES["stage1"] += 1
-    if bitmap_read:
-        _LAUNCHES["bitmap"] += 1
+    if int(_stage) not in (0, 1, 2):
+        raise ValueError(f"_stage={_stage} must be 0, 1 or 2")
+    if head_gather is not None and int(_stage) == 1:
+        raise ValueError("head_gather belongs to stage 2; _stage=1 runs stage 1 alone")
+    raise ValueError("ommx_paged_decode_attention_canonical: an argument has the wrong kind, rank or range")
 
 
 def merge_attention_states(o_parts, lse_parts, *, valid_lens=None, out=None, lse_out=None):

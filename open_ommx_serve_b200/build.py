@@ -1,8 +1,9 @@
-"""Build libommx_b200.so in-tree with nvcc for sm_100a.
+"""Build libommx_b200.so (nvcc, sm_100a) and the Python host module _host.so (g++) in-tree.
 
-    python -m open_ommx_serve_b200.build          # rebuild if a source is newer than the library
+    python -m open_ommx_serve_b200.build          # rebuild what is older than its sources
 
-The library is plain CUDA C++ behind a C ABI (include/ommx_b200.h); it links nothing from torch.
+The library is plain CUDA C++ behind a C ABI (include/ommx_b200.h); it links nothing from torch.  _host.so is the
+Python entry points' native half: it reads torch tensors and calls that ABI.
 """
 from __future__ import annotations
 
@@ -10,12 +11,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libommx_b200.so")
 SOURCES = ("ommx_capi.cu", "ommx_pack.cu", "ommx_decode.cu")
 HEADERS = ("ommx_common.cuh", "ommx_decode_tc.cuh", "ommx_tables.inc", os.path.join("..", "..", "include", "ommx_b200.h"))
+HOST_LIB = os.path.join(PKG, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "ommx_host.cpp")
 NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC")
 
@@ -27,26 +31,47 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found (set NVCC=/path/to/nvcc)")
 
 
+def _older(target: str, sources) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(f) > os.path.getmtime(target) for f in sources)
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in SOURCES + HEADERS)
+    return _older(LIB, [os.path.join(CSRC, f) for f in SOURCES + HEADERS])
+
+
+def _run(cmd) -> str:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("the build failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    return res.stderr
+
+
+def build_host(force: bool = False) -> str:
+    """Compile ``_host.so`` against the torch that this interpreter imports; returns its path."""
+    if not force and not _older(HOST_LIB, (HOST_SOURCE, os.path.join(PKG, "..", "include", "ommx_b200.h"))):
+        return HOST_LIB
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    _run([os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
+          f"-I{cuda}/include", "-o", HOST_LIB, HOST_SOURCE, f"-L{PKG}", "-l:" + os.path.basename(LIB),
+          f"-L{root}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
+    return HOST_LIB
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the CUDA sources into ``libommx_b200.so`` next to this file; returns its path."""
-    if not force and not needs_build():
-        return LIB
-    cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB, *[os.path.join(CSRC, s) for s in SOURCES]]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
-    if verbose:
-        sys.stderr.write(res.stderr)
+    """Compile the CUDA sources into ``libommx_b200.so`` next to this file and ``_host.so`` beside it; returns the
+    library's path."""
+    if force or needs_build():
+        cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB, *[os.path.join(CSRC, s) for s in SOURCES]]
+        if verbose:
+            cmd[1:1] = ["-Xptxas", "-v"]
+        log = _run(cmd)
+        if verbose:
+            sys.stderr.write(log)
+    build_host(force)
     return LIB
 
 
