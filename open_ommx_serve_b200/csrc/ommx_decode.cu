@@ -35,11 +35,12 @@ namespace ommx {
 
 constexpr int HD = 128;                 // head_dim this build serves
 constexpr int NCW = 8;                  // (group, head) units in flight per CTA, one MMA warp each
-// Two warp layouts.  Narrow (4 or 8 local kv heads: 14 copies per ring stage): 15 decode warps + 1 producer warp, which
-// also builds the last tile half once its copies are out.  Wide (1 or 2 local kv heads: a stage is 8 or 4 groups, 112 or
-// 56 small copies): 16 decode warps + 4 producer warps, because one warp issues a bulk copy only every ~60 cycles and
-// the issues of different warps overlap (112 copies: 6400 cycles from one warp, 2000 from four).
-template <bool WIDE> struct WarpLayout {
+// Two warp layouts.  Narrow (4 or 8 local kv heads: 14 or 28 copies per ring stage): 15 decode warps + 1 producer warp,
+// which also builds the last tile half once its copies are out.  Wide (1 or 2 local kv heads: a stage is 8 or 4 groups,
+// 112 or 56 small copies): 16 decode warps + 4 producer warps, because one warp issues a bulk copy only every ~60 cycles
+// and the issues of different warps overlap (112 copies: 6400 cycles from one warp, 2000 from four).
+template <int H> struct WarpLayout {
+    static constexpr bool WIDE = H <= 2;
     static constexpr int NDW = WIDE ? 16 : 15;            // decode warps (stateless sidecar builders, items dealt round-robin)
     static constexpr int NPW = WIDE ? 4 : 1;              // producer warps
     static constexpr int PRODUCER_WARP = NCW + NDW;       // the first of them
@@ -55,14 +56,15 @@ template <bool WIDE> struct WarpLayout {
 constexpr int REGS_MMA = 128, REGS_DECODE = 56, REGS_PRODUCER = 24;
 constexpr int MAX_STAGES = 4;           // ring depth (3 when the planes of a stage are large)
 constexpr int DT_STRIDE = 272;          // bytes per sidecar-tile row (256 data + 16 pad)
-constexpr int ROW_ZP = 32;              // q.zp partial sums, fp32: [channel half][8 query heads of the kv head]
-constexpr int ROW_KF = 33;              // K scale factors 2^(e+4), fp16, in code-fragment order
-constexpr int ROW_VF = 34;              // V scale factors, fp16, fragment order (rows 34, 35: two copies)
-constexpr int ROW_ZT = 36;              // V zero-points [scale group][token], fp16 (rows 36, 37: two copies)
-constexpr int DT_ROWS = 38;             // rows 0..31: outlier deltas [token][channel], fp16
+constexpr int ROW_KF = 32;              // K scale factors 2^(e+4) * 4^-slot, fp16, in code-fragment order
+constexpr int ROW_VF = 33;              // V scale factors, fp16, fragment order (rows 33, 34: two copies)
+constexpr int ROW_ZT = 35;              // V zero-points [scale group][token], fp16 (rows 35, 36: two copies)
+constexpr int ZT_STRIDE = 68;           // bytes from one scale group's zero-points to the next (64 + a bank)
+constexpr int DT_ROWS = 37;             // rows 0..31: outlier deltas [token][channel in fragment order], fp16
 constexpr int DT_BYTES = DT_ROWS * DT_STRIDE;
-constexpr int MAX_SPLIT_GROUPS = 512;   // groups one CTA can index (16K tokens per split)
+constexpr int MAX_SPLIT_GROUPS = 512;   // groups of the longest split that the entry points accept (16K tokens)
 constexpr int MAX_SPLIT_PAGES = 1024;
+constexpr int MAX_PIECES = 256;         // pieces of sequences one CTA can work on (32 bytes of shared memory each)
 constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;   // about a second of SM clock: the wait has failed
 
 struct S1Params {
@@ -80,6 +82,7 @@ struct S1Params {
     float *al;
     int64_t al_sb, al_sh, al_ss;
     int32_t S, seg_group_base;
+    int32_t ncta, waves;                 // CTAs of the launch (one per SM at most), rounds of them that B * S splits would take
     float sm_scale, logit_cap;
     int32_t *status;
     int32_t abl;
@@ -125,15 +128,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // clock (cheap to read); nanosleep or the global timer in this loop would put their own latency
 // on every producer/consumer hand-off.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long limit = WAIT_LIMIT_CYCLES) {
+    long long t_end = 0;
 #pragma unroll 1
-    for (int i = 0; i < 64; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    const long long t_end = clock64() + limit;
-#pragma unroll 1
-    for (uint32_t i = 1;; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 63u) == 0 && clock64() > t_end) return false;
+    for (uint32_t i = 1; !mbar_try_wait(bar, parity); ++i) {
+        if ((i & 63u) == 0) {
+            const long long now = clock64();
+            if (t_end == 0) t_end = now + limit;
+            else if (now > t_end) return false;
+        }
     }
+    return true;
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -149,6 +153,18 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                         uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// two 16x16 byte matrices (rows from lanes 0-15 and 16-31), transposed: r[2m], r[2m+1] = rows 4j..4j+3 of columns g and
+// g + 8 of matrix m (lane = 4g + j)
+__device__ __forceinline__ void ldsm_b8_trans_x2(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
 __device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t &r0, uint32_t &r1) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
@@ -161,6 +177,11 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {       // clamped to the finite range
+    uint32_t r;
+    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
 __device__ __forceinline__ uint32_t hmul2_f16(uint32_t a, uint32_t b) {
@@ -212,11 +233,19 @@ __device__ __forceinline__ uint32_t pow2_f16_bits(int e, bool &clamped) {
 }
 // the reference rounds an outlier's delta to bf16; keep that rounding point, then store it as fp16
 // (exact: 8 significant bits fit in 11)
-__device__ __forceinline__ uint32_t f16_bits_of_bf16_rounded(float x) {
-    uint16_t r;
-    const float xb = bf16_round_f32(x);
-    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(r) : "f"(xb));
-    return (uint32_t)r;
+__device__ __forceinline__ uint32_t f16x2_of_bf16_rounded(float lo, float hi) {
+    uint32_t b;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b) : "f"(hi), "f"(lo));
+    return pack_f16x2_sat(__uint_as_float(b << 16), __uint_as_float(b & 0xFFFF0000u));
+}
+// the FP4 levels of four outliers (16 bits of the nibble stream) as the upper bytes of their fp16 values; the lower
+// bytes are zero.  A nibble is the byte selector of the magnitude table; its sign bit, which as a selector bit replicates
+// a byte's sign, turns 0x80 into 0xFF in a second lookup.
+__device__ __forceinline__ uint32_t fp4_levels_hi(uint32_t nibbles) {
+    const uint32_t mag = __byte_perm(0x3E3C3800u, 0x46444240u, nibbles & 0x7777u);
+    uint32_t sgn;
+    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(sgn) : "r"(0x80808080u), "r"(nibbles));
+    return mag | ((sgn << 7) & 0x80808080u);
 }
 __device__ __forceinline__ uint32_t f16_bits_sat(float x) {
     uint16_t r;
@@ -234,6 +263,136 @@ __device__ __forceinline__ int code_slot(int i) { return i < 5 ? i : i - 5; }
 __device__ __forceinline__ int ring_slot(int it, int ns) { return ns == 4 ? (it & 3) : it % ns; }
 __device__ __forceinline__ uint32_t ring_phase(int it, int ns) { return (uint32_t)(ns == 4 ? (it >> 2) : it / ns) & 1u; }
 
+// ---- how the groups of a launch are shared out over its CTAs ------------------------------------------
+// The packed groups of all sequences form one running list, and CTA i takes groups [i * per, (i + 1) * per) of it, whatever
+// sequences they belong to: every CTA has the same work up to one group, also when the lengths are ragged (32 sequences of
+// 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us around its steady state).  A piece of
+// a sequence writes its partial result to workspace slot (its CTA - the first CTA of the sequence), and the caller's
+// workspace has S slots per sequence, which bounds `per` from below.  Where that bound makes the shares longer than S equal
+// splits per sequence dealt out one by one would be, those are taken instead (per = 0): item x is split x % S of sequence x / S.
+struct SharePlan {
+    int per, total;                      // groups per CTA (0: equal splits per sequence), groups of all sequences
+};
+__device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
+__device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, int ncta, int waves) {
+    SharePlan s;
+    s.total = total;
+    s.per = max(1, (total + ncta - 1) / ncta);
+    const int equal = (longest + S - 1) / S;
+    if (B == 1) {
+        s.per = max(s.per, equal);                             // a lone sequence starts at a CTA's beginning: exactly ceil(n / per) slots
+    } else {
+        if (S >= 2) s.per = max(s.per, (longest - 2) / (S - 1) + 1);   // anywhere else it touches up to (n - 2) / per + 2 CTAs
+        if (S < 2 || (waves <= MAX_PIECES && waves * equal <= s.per)) s.per = 0;
+    }
+    return s;
+}
+// called by whole warps; every lane gets the same answer
+__device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, int ncta, int waves, int lane) {
+    int n = 0, mx = 0;
+    if (B == 1) {
+        n = mx = groups_of(b_seq_len[0]);
+    } else {
+        for (int i = lane; i < B; i += 32) {
+            const int g = groups_of(b_seq_len[i]);
+            n += g;
+            mx = max(mx, g);
+        }
+        n = __reduce_add_sync(0xFFFFFFFFu, n);
+        mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    }
+    return share_plan_of(n, mx, B, S, ncta, waves);
+}
+
+// One piece of work of a CTA: consecutive groups of one sequence.  `it` counts the CTA's ring stages across its pieces, so that
+// the ring never drains between two of them.  One warp lists the pieces in shared memory; the roles walk that list, because
+// the walk's own state costs a decode warp (56 registers) 9 % of its speed in spills.
+struct alignas(16) Piece {
+    int b, slot, g0, ng;                 // sequence, workspace slot, first group in the sequence, groups
+    int ntok, it0, it1, more;            // tokens, ring iterations [it0, it1), whether another piece follows
+};
+struct PieceWalk {
+    int pos, end;                        // running list: first group of the piece, end of this CTA's share; splits: item, items
+};
+template <int GS>
+__device__ __forceinline__ void piece_range(Piece &c, int seq, int g0, int ng) {
+    c.g0 = g0;
+    c.ng = ng;
+    c.ntok = min(seq - 32 * g0, 32 * ng);
+    c.it1 = c.it0 + (ng + GS - 1) / GS;
+}
+// equal splits: the first item at or after w.pos that has groups
+template <int GS> __device__ __forceinline__ bool piece_of_splits(Piece &c, PieceWalk &w, const S1Params &p) {
+    for (; w.pos < w.end; w.pos += p.ncta) {
+        c.b = w.pos / p.S;
+        c.slot = w.pos - c.b * p.S;
+        const int seq = p.b_seq_len[c.b], n = groups_of(seq), per = (n + p.S - 1) / p.S, g0 = c.slot * per;
+        if (g0 < n) {
+            piece_range<GS>(c, seq, g0, min(per, n - g0));
+            return true;
+        }
+    }
+    return false;
+}
+template <int GS> __device__ __forceinline__ bool first_piece(Piece &c, PieceWalk &w, const S1Params &p, const SharePlan &plan, int cta, int lane) {
+    c.it0 = 0;
+    if (plan.per == 0) {
+        w.pos = cta;
+        w.end = p.B * p.S;
+        return piece_of_splits<GS>(c, w, p);
+    }
+    w.pos = cta * plan.per;
+    w.end = min(w.pos + plan.per, plan.total);
+    if (w.pos >= w.end) return false;
+    int off = 0, seq, n;                                       // groups before the sequence that holds w.pos
+    if (p.B == 1) {
+        c.b = 0;
+        seq = p.b_seq_len[0];
+        n = groups_of(seq);
+    } else {
+        for (int base = 0;; base += 32) {
+            const int len = base + lane < p.B ? p.b_seq_len[base + lane] : 0;
+            const int g = groups_of(len);
+            int x = g;                                         // inclusive sums over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= o) x += y;
+            }
+            const uint32_t past = __ballot_sync(0xFFFFFFFFu, off + x > w.pos);
+            if (past) {
+                const int l = __ffs(past) - 1;
+                c.b = base + l;
+                seq = __shfl_sync(0xFFFFFFFFu, len, l);
+                n = __shfl_sync(0xFFFFFFFFu, g, l);
+                off += __shfl_sync(0xFFFFFFFFu, x, l) - n;
+                break;
+            }
+            off += __shfl_sync(0xFFFFFFFFu, x, 31);
+        }
+    }
+    c.slot = cta - off / plan.per;
+    const int g0 = w.pos - off, ng = min(n - g0, w.end - w.pos);
+    piece_range<GS>(c, seq, g0, ng);
+    return true;
+}
+template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk &w, const S1Params &p, const SharePlan &plan) {
+    c.it0 = c.it1;
+    if (plan.per == 0) {
+        w.pos += p.ncta;
+        return piece_of_splits<GS>(c, w, p);
+    }
+    w.pos += c.ng;
+    if (w.pos >= w.end) return false;
+    int seq;
+    do seq = p.b_seq_len[++c.b];                               // the share has groups left, so a later sequence has some
+    while (seq <= 0);
+    const int n = groups_of(seq), ng = min(n, w.end - w.pos);
+    c.slot = 0;                                                // it begins inside this CTA's share
+    piece_range<GS>(c, seq, 0, ng);
+    return true;
+}
+
 // KOUT: outliers per K vector known at compile time (static, unrolled splice) or -1 (runtime).
 //
 // Every MMA is m16n8k16 fp16 with the 2-bit codes as the A operand: a code field masked in place is an
@@ -247,83 +406,40 @@ __device__ __forceinline__ uint32_t ring_phase(int it, int ns) { return (uint32_
 //                              + vz^T[group][token] . P[token][head]
 // The power-of-two factors, zero-points and deltas of a unit are laid out for these fragments by the
 // decode warps (the sidecar tile), so the MMA warps multiply and accumulate and do little else.
-template <int KOUT, bool WIDE>
-__global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_kernel(const __grid_constant__ S1Params p) {
-    constexpr int NDW = WarpLayout<WIDE>::NDW, NPW = WarpLayout<WIDE>::NPW, PRODUCER_WARP = WarpLayout<WIDE>::PRODUCER_WARP;
-    constexpr int S1_THREADS = WarpLayout<WIDE>::THREADS;
+template <int KOUT, int H>
+__global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kernel(const __grid_constant__ S1Params p) {
+    constexpr bool WIDE = WarpLayout<H>::WIDE;
+    constexpr int NDW = WarpLayout<H>::NDW, NPW = WarpLayout<H>::NPW, PRODUCER_WARP = WarpLayout<H>::PRODUCER_WARP;
+    constexpr int S1_THREADS = WarpLayout<H>::THREADS;
+    constexpr int GS = NCW / H;                                     // groups per ring stage
+    constexpr int TS = H * 32;                                      // bytes per token row (all heads)
+    constexpr uint32_t SWZ = H >= 4 ? 0x70u : 0u;                   // the code planes are staged through swizzled tensor maps
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // swizzle atoms are 1 KB: align the ring by hand (the launch adds 1 KB of slack)
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int split = blockIdx.x, b = blockIdx.y;
+    const int cta = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // the first tensor-map copy otherwise pays for fetching its descriptor
-    if (threadIdx.x == S1_THREADS - 32 && p.swz != 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_k)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_v)) : "memory");
-    }
-
-    // The launch lets this grid start while the kernel before it in the stream is still running (its blocks are
-    // placed, shared memory is carved): nothing that kernel may have written - lengths, tables, the query, the
-    // planes, the split workspace a previous layer's combine still reads - is touched before this returns.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // ---- split range (same rounding as the reference, paged_decode.py:1428-1432) ----
-    const int seq = p.b_seq_len[b];
-    if (seq <= 0) return;
-    const int per = (((seq + p.S - 1) / p.S) + 31) / 32 * 32;
-    const int t0 = split * per;
-    const int t1 = min(t0 + per, seq);
-    if (t1 <= t0) return;
-    const int ntok = t1 - t0;
-    int ngroups = (ntok + 31) / 32;
-    if (ngroups > MAX_SPLIT_GROUPS || ngroups * p.ppg > MAX_SPLIT_PAGES) {   // host sizing should prevent this
-        if (threadIdx.x == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
-        return;
-    }
-    const int H = p.H, GS = p.GS, NS = p.nstages;
-    const int n_iters = (ngroups + GS - 1) / GS;
+    const int NS = p.nstages;
     const int k_out = KOUT >= 0 ? KOUT : p.k_out;
     const long long wait_limit = (p.abl & ABL_TEST_STALL) ? TEST_WAIT_LIMIT_CYCLES : WAIT_LIMIT_CYCLES;
-    // The MMA warps' query words (bf16 pairs) are requested now and turned into operand fragments after the prologue,
-    // which hides their round trip behind the table loads: q_s = this lane's 32 consecutive channels (code MMAs),
-    // q_d = the channel pairs of the delta MMAs' fragments.  Column n = lane / 4 of every MMA is query head n.
-    uint32_t q_s[16], q_d[16];
-    if (warp < NCW) {
-        const int hq_ = (warp & (H - 1)) * p.gqa + ((lane >> 2) < p.gqa ? (lane >> 2) : 0), j_ = lane & 3;
-        const __nv_bfloat16 *qrow = p.q + (int64_t)b * p.q_sb + (int64_t)hq_ * p.q_sh;
-        if (p.q_vec_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const uint4 t = __ldg(reinterpret_cast<const uint4 *>(qrow + 32 * j_) + v);
-                q_s[4 * v] = t.x; q_s[4 * v + 1] = t.y; q_s[4 * v + 2] = t.z; q_s[4 * v + 3] = t.w;
-            }
-#pragma unroll
-            for (int r = 0; r < 16; ++r) q_d[r] = __ldg(reinterpret_cast<const uint32_t *>(qrow + 16 * (r >> 1) + 8 * (r & 1) + 2 * j_));
-        } else {
-            const uint16_t *q16 = reinterpret_cast<const uint16_t *>(qrow);
-#pragma unroll
-            for (int v = 0; v < 16; ++v) q_s[v] = (uint32_t)__ldg(q16 + 32 * j_ + 2 * v) | ((uint32_t)__ldg(q16 + 32 * j_ + 2 * v + 1) << 16);
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int c = 16 * (r >> 1) + 8 * (r & 1) + 2 * j_;
-                q_d[r] = (uint32_t)__ldg(q16 + c) | ((uint32_t)__ldg(q16 + c + 1) << 16);
-            }
-        }
-    }
 
     // ---- shared memory carve-up ----
     uint8_t *s_stage = smem;                                            // nstages * stage_bytes
     uint8_t *s_tiles = s_stage + NS * p.stage_bytes;                    // NCW * DT_BYTES
-    int32_t *s_tab = reinterpret_cast<int32_t *>(s_tiles + NCW * DT_BYTES);   // page ids, then group slots
-    float *s_lut = reinterpret_cast<float *>(s_tab + MAX_SPLIT_PAGES + MAX_SPLIT_GROUPS);
+    float *s_lut = reinterpret_cast<float *>(s_tiles + NCW * DT_BYTES);
     uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_lut + 16);         // full[], empty[], tile_full[NCW], tile_empty[NCW][], tile_rows[NCW]
-    int32_t *s_abort = reinterpret_cast<int32_t *>(s_bar + 2 * MAX_STAGES + (2 + MAX_STAGES) * NCW);
-    CopyDesc *s_desc = reinterpret_cast<CopyDesc *>(s_abort + 4);
+    CopyDesc *s_desc = reinterpret_cast<CopyDesc *>(s_bar + 2 * MAX_STAGES + (2 + MAX_STAGES) * NCW);
     const uint32_t bar_full = smem_u32(s_bar), bar_empty = smem_u32(s_bar + MAX_STAGES);
     const uint32_t bar_tfull = smem_u32(s_bar + 2 * MAX_STAGES), bar_tempty = smem_u32(s_bar + 2 * MAX_STAGES + NCW);
     const uint32_t bar_trows = smem_u32(s_bar + 2 * MAX_STAGES + (1 + MAX_STAGES) * NCW);
 
-    // ---- prologue: LUT, barriers, copy descriptors and the split's page / slot tables, spread over the
-    //      whole CTA so that the producer can issue the first stage right after the barrier ----
+    // ---- prologue: LUT, barriers and copy descriptors.  None of it depends on an earlier kernel, so it runs while the
+    //      kernel before this one in the stream drains (the grid may start then, see the wait below). ----
+    // the first tensor-map copy otherwise pays for fetching its descriptor
+    if (SWZ != 0 && threadIdx.x == S1_THREADS - 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_k)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_v)) : "memory");
+    }
     if (threadIdx.x < 16) {
         const int c = threadIdx.x;
         const int mi = ((c >> 1) & 3) * 2 + (c & 1);                    // exp*2 + mant
@@ -336,13 +452,12 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
         constexpr int NB_RING = 2 * MAX_STAGES, NB_ALL = NB_RING + (2 + MAX_STAGES) * NCW;
         if (t >= 0 && t < NB_ALL) {
             uint32_t count;
-            if (t < MAX_STAGES) count = 1;                                     // full[]
+            if (t < MAX_STAGES) count = NPW;                                   // full[]: each producer warp announces its own copies
             else if (t < NB_RING) count = 3 * NCW;                             // empty[]: 8 MMA warps + 16 tile halves
             else if (t < NB_RING + NCW) count = 2;                             // tile_full[]: the two halves' deltas scattered
             else if (t < NB_RING + NCW + MAX_STAGES * NCW) count = 1;          // tile_empty[][]
             else count = 2;                                                    // tile_rows[]: the two halves' rows written
             mbar_init(bar_full + 8 * t, count);
-            if (t == 0) *s_abort = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
@@ -350,8 +465,8 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
     const int ncopies = GS * cpg;
     {
         // Copy roles (group-in-stage, plane) are tabulated once; the producer's loop body is then one
-        // descriptor load, one table lookup, one multiply-add and one copy per role, with no divergent
-        // paths, because that single warp's issue latency bounds how fast stages refill.
+        // descriptor load, one multiply-add and one copy per role, with no divergent paths, because that
+        // single warp's issue latency bounds how fast stages refill.
         const uint32_t page_b = (uint32_t)p.ps * H;                     // (token, head) rows per page
         const int c = (int)threadIdx.x - 64;                            // threads 64.. build one descriptor each
         if (c >= 0 && c < ncopies) {
@@ -368,7 +483,7 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                 d.dst = gbo + (plane == 0 ? 0u : (plane == 1 ? (uint32_t)p.o_vm : (plane == 2 ? (uint32_t)p.o_vs : (uint32_t)p.o_vz)))
                       + (uint32_t)pg * page_b * w;
                 d.tbase = pg; d.tmul = p.ppg; d.tok0 = pg * p.ps;
-                if (p.swz != 0 && plane < 2) d.gi |= (plane + 1) << 8;
+                if (SWZ != 0 && plane < 2) d.gi |= (plane + 1) << 8;
             } else {
                 const int gp = ci - 4 * p.ppg;
                 const bool on = gp < 2 || (k_out > 0 && (gp >= 4 || p.use_map));
@@ -377,190 +492,179 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                     d.src = gp == 0 ? p.k_scale : (gp == 1 ? p.k_zp : (gp == 2 ? p.k_ms : (gp == 3 ? p.k_mc : (gp == 4 ? p.k_obmp : p.k_oval))));
                     d.unit = (uint32_t)H * w;
                     d.dst = gbo + (uint32_t)(gp == 0 ? p.o_ks : (gp == 1 ? p.o_kz : (gp == 2 ? p.o_ms : (gp == 3 ? p.o_mc : (gp == 4 ? p.o_bm : p.o_ov)))));
-                    d.tbase = MAX_SPLIT_PAGES; d.tmul = 1;
+                    d.tbase = 0; d.tmul = 0;                            // tmul 0: the index is a group slot
                 }
             }
             s_desc[c] = d;
         }
-        // page ids first (s_tab[0..)), group slots behind them
-        const int g0 = p.seg_group_base + t0 / 32;                      // first logical group
-        const int npages = (ntok + p.ps - 1) / p.ps;
-        const int64_t pg0 = ((int64_t)g0 * 32) / p.ps;
-        for (int i = threadIdx.x; i < npages; i += S1_THREADS) {
-            int64_t pg = load_index(p.r2t, p.tbl64, (int64_t)b * p.r2t_sb + pg0 + i);
-            if (pg < 0 || pg >= p.num_pages) { or_status(p.status, OMMX_ST_BAD_PAGE); pg = 0; }
-            s_tab[i] = (int)pg;
-        }
-        for (int i = S1_THREADS - 1 - (int)threadIdx.x; i < ngroups; i += S1_THREADS) {
-            int64_t sl = load_index(p.r2g, p.tbl64, (int64_t)b * p.r2g_sb + g0 + i);
-            if (sl < 0 || sl >= p.num_slots) { or_status(p.status, OMMX_ST_BAD_GROUP); sl = 0; }
-            s_tab[MAX_SPLIT_PAGES + i] = (int)sl;
-        }
     }
     __syncthreads();
+    // Nothing an earlier kernel may have written - lengths, tables, the query, the planes, the split workspace a
+    // previous layer's combine still reads - is touched before this returns.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     // Stage 2 is launched as a programmatic dependent: it may start its own prologue (residual-row
-    // logits, which do not depend on this kernel) as soon as SM resources free up, and waits for this
-    // grid to finish before it reads the split partials.
+    // logits, which do not depend on this kernel but may depend on the one before it: hence after the wait)
+    // as soon as SM resources free up, and waits for this grid to finish before it reads the split partials.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+    Piece pc;
+    PieceWalk walk;
+    const SharePlan plan = share_plan(p.b_seq_len, p.B, p.S, p.ncta, p.waves, lane);
+    if (!first_piece<GS>(pc, walk, p, plan, cta, lane)) return;
+
     const int g = lane >> 2, j = lane & 3;
-    const int TS = H * 32;                                          // bytes per token row (all heads)
     const float LOG2E = 1.4426950408889634f;
     const bool no_outlier = (p.abl & ABL_NO_OUTLIER) != 0;
-    const int n_items = n_iters * NCW * 2;                          // (iteration, unit, tile half) work items of the decode role
 
-    // ---- one stage of the ring: announce its bytes, issue its copies (producer warp) ----
-    uint32_t full_total = 0;                                        // bytes of a stage with GS whole groups
-    const int whole_groups = ntok / 32;
-    const int pw = warp - PRODUCER_WARP;                            // producer warp index (meaningful for those warps only)
-    // `nshare` warps split the copies of a stage, this one taking share `share`; the `lead` among them announces the bytes
-    auto issue_stage = [&](int it, int nshare, int share, bool lead) __attribute__((always_inline)) {
+    // ---- one stage of the ring: look up its page ids and group slots, announce its bytes, issue its copies (producer
+    //      warps).  The lookup of a stage runs while the stage before it is still on its way, so that no copy waits for its
+    //      table entry; each lane leaves what it finds in s_idx for itself. ----
+    Piece *s_piece = reinterpret_cast<Piece *>(s_desc + ncopies);
+    int32_t *s_idx = reinterpret_cast<int32_t *>(s_piece + MAX_PIECES);
+    auto whole_stage = [&](const Piece &q, int it) { return 32 * GS * (it + 1 - q.it0) <= q.ntok; };
+    auto copy_on = [&](const CopyDesc &d, const Piece &q, int it) __attribute__((always_inline)) {
+        const int lg = (it - q.it0) * GS + (d.gi & 0xFF);
+        return d.unit != 0 && lg < q.ng && 32 * lg + d.tok0 < q.ntok;
+    };
+    auto lookup_stage = [&](const Piece &q, int it, int nshare, int share) __attribute__((always_inline)) {
+        const int64_t g0 = (int64_t)p.seg_group_base + q.g0 + (it - q.it0) * GS;
+#pragma unroll 1
+        for (int ci = lane * nshare + share; ci < ncopies; ci += 32 * nshare) {
+            const CopyDesc d = s_desc[ci];
+            if (!copy_on(d, q, it)) continue;
+            const bool page = d.tmul != 0;                          // tmul 0: the index is a group slot
+            const int64_t at = page ? (int64_t)q.b * p.r2t_sb + (g0 + (d.gi & 0xFF)) * d.tmul + d.tbase : (int64_t)q.b * p.r2g_sb + g0 + (d.gi & 0xFF);
+            int64_t x = load_index(page ? p.r2t : p.r2g, p.tbl64, at);
+            if (x < 0 || x >= (page ? p.num_pages : p.num_slots)) { or_status(p.status, page ? OMMX_ST_BAD_PAGE : OMMX_ST_BAD_GROUP); x = 0; }
+            s_idx[ci] = (int)x;
+        }
+    };
+    // `nshare` warps split the copies of a stage, this one taking share `share`; with `announce_all` it announces the bytes
+    // of all of them (the others then announce nothing), else its own.
+    // (A copy of another warp may land before the announcement: the phase cannot complete without the announcing arrival,
+    // and the transaction count may run negative meanwhile.)
+    auto stage_bytes_of = [&](const Piece &q, int it, bool whole, int first, int step) __attribute__((always_inline)) {
+        uint32_t mine = 0;
+#pragma unroll 1
+        for (int ci = first; ci < ncopies; ci += step) {
+            const CopyDesc d = s_desc[ci];
+            if (whole || copy_on(d, q, it)) mine += d.unit;
+        }
+        return __reduce_add_sync(0xFFFFFFFFu, mine);
+    };
+    auto issue_stage = [&](const Piece &q, int it, int nshare, int share, uint32_t announce) __attribute__((always_inline)) {
         const int s = ring_slot(it, NS);
-        const int lg0 = it * GS;
-        if (lead) {
-            uint32_t total = full_total;
-            if (lg0 + GS > whole_groups) {                          // last stage: fewer groups or a partial group
-                uint32_t mine = 0;
-                for (int c = lane; c < ncopies; c += 32) {
-                    const CopyDesc d = s_desc[c];
-                    const int lg = lg0 + (d.gi & 0xFF);
-                    if (d.unit && lg < ngroups && 32 * lg + d.tok0 < ntok) mine += d.unit;
-                }
-                total = __reduce_add_sync(0xFFFFFFFFu, mine);
-            }
-            if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, total);
+        if (announce) {
+            if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, announce);
             __syncwarp();
         }
-        // (A copy of another producer warp may land before the announcement: the phase cannot complete without the
-        // announcing arrival, and the transaction count may run negative meanwhile.)
         const uint32_t sbase = smem_u32(s_stage + (size_t)s * p.stage_bytes);
-        for (int c = lane * nshare + share; c < ncopies; c += 32 * nshare) {
-            const CopyDesc d = s_desc[c];
-            const int lg = lg0 + (d.gi & 0xFF);
+#pragma unroll 1
+        for (int ci = lane * nshare + share; ci < ncopies; ci += 32 * nshare) {
+            const CopyDesc d = s_desc[ci];
             const int kind = d.gi >> 8;
-            if (d.unit && lg < ngroups && 32 * lg + d.tok0 < ntok && !((p.abl & ABL_TEST_STALL) && it == 1)) {
-                const int64_t idx = s_tab[d.tbase + lg * d.tmul];
-                if (kind == 0) bulk_g2s(sbase + d.dst, d.src + idx * d.unit, d.unit, bar_full + 8 * s);
-                else tma_2d_g2s(sbase + d.dst, kind == 1 ? &p.tmap_k : &p.tmap_v, 0, (int32_t)idx * p.rows_per_page, bar_full + 8 * s);
+            if (copy_on(d, q, it) && !((p.abl & ABL_TEST_STALL) && it == 1)) {
+                const int idx = s_idx[ci];
+                if (kind == 0) bulk_g2s(sbase + d.dst, d.src + (int64_t)idx * d.unit, d.unit, bar_full + 8 * s);
+                else tma_2d_g2s(sbase + d.dst, kind == 1 ? &p.tmap_k : &p.tmap_v, 0, idx * p.rows_per_page, bar_full + 8 * s);
             }
         }
     };
     // The first ring fill is on every CTA's critical path: it goes out before the register budgets are resized.
     // A warp issues a bulk copy only about every 60 cycles and different warps overlap, so in the narrow layout the three
     // decode warps of the producer's warpgroup (idle until the data lands) take a quarter of the first fill each.
-    if (warp >= PRODUCER_WARP) {
-        for (int c = lane; c < ncopies; c += 32) full_total += s_desc[c].unit;
-        full_total = __reduce_add_sync(0xFFFFFFFFu, full_total);
-    }
-    if constexpr (WIDE) {
-        if (warp >= PRODUCER_WARP) issue_stage(0, NPW, pw, pw == 0);
-    } else {
-        if (warp >= PRODUCER_WARP - 3) issue_stage(0, 4, warp - (PRODUCER_WARP - 3), warp == PRODUCER_WARP);
+    if (warp >= PRODUCER_WARP - (WIDE ? 0 : 3)) {
+        constexpr int W0 = PRODUCER_WARP - (WIDE ? 0 : 3);
+        lookup_stage(pc, 0, 4, warp - W0);
+        const uint32_t bytes = WIDE ? stage_bytes_of(pc, 0, false, lane * NPW + warp - W0, 32 * NPW)
+                                    : (warp == PRODUCER_WARP ? stage_bytes_of(pc, 0, false, lane, 32) : 0u);
+        issue_stage(pc, 0, 4, warp - W0, bytes);
     }
 
+    if (warp == PRODUCER_WARP) {
+        int n = 0;
+        for (bool more = true; more; ++n) {
+            Piece cur = pc;
+            more = next_piece<GS>(pc, walk, p, plan);
+            if (more && n + 1 == MAX_PIECES) {                       // the host sizes the grid so that this cannot be
+                if (lane == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
+                more = false;
+            }
+            cur.more = more;
+            if (lane == 0) s_piece[n] = cur;
+        }
+    }
+    __syncthreads();
+    int pi = 0;
+    pc = s_piece[0];
+    auto step_piece = [&]() __attribute__((always_inline)) {
+        if (!pc.more) return false;
+        pc = s_piece[++pi];
+        return true;
+    };
+
     // ---- one work item of the decode role: half hf of the sidecar tile of (iteration it, unit) ----
+    // Channel 64 w + 16 j + 8 x + i (i = 0..7) sits in member x of the pair in register 8 w + i of lane group j in the MMAs
+    // below, i.e. in column byte 128 w + 16 i + 4 j + 2 x of the delta rows.  This half has w = hf, this lane channels
+    // 2 lane and 2 lane + 1 of it: j = dj, x = dh, i = 2 da and 2 da + 1.
+    const int da = lane & 3, dh = (lane >> 2) & 1, dj = lane >> 3;
+    // 4^-slot of those two channels' code fields, fp16
+    const uint32_t slot_scale = da == 0 ? 0x34003C00u : (da == 1 ? 0x24002C00u : (da == 2 ? 0x3C001C00u : 0x2C003400u));
     // Build the sidecar tile of a unit between two uses by its MMA warp.  A tile is built in two
-    // halves by two warps at once, because the MMA warp of the unit waits for it: half hf takes K
-    // channels 64hf..64hf+63 (lane l: channels 64hf + 2l, +1 - delta columns, zero-points, scale
-    // factors) and V tokens 16hf..16hf+15 (lane l: token 16hf + l%16, scale groups 2(l/16), +1).
+    // halves by two warps at once, because the MMA warp of the unit waits for it: half hf takes 64 of the
+    // K channels (delta columns, scale factors) and V tokens 16hf..16hf+15 (factors, zero-points).
     // Returns false when a bounded wait ran out.
-    auto decode_item = [&](const int n) __attribute__((always_inline)) -> bool {
+    auto decode_item = [&](const Piece &pc, const int n) __attribute__((always_inline)) -> bool {
         const int it = n / (2 * NCW), unit = (n >> 1) % NCW, hf = n & 1;
-        const int h = unit & (H - 1), gsel = unit >> p.hshift;       // H is a power of two
+        const int h = unit % H, gsel = unit / H;
         uint8_t *tile = s_tiles + unit * DT_BYTES;
         const int s = ring_slot(it, NS);
         const uint32_t ph = ring_phase(it, NS);
-        // The fp32 q.zp sums of this half's 64 channels: lane = (query head of the kv head, block of 8 or 16
-        // channels).  The lane's raw query values are requested before the waits below, so that the loads are
-        // in flight meanwhile.
-        const bool gq8 = p.gqa > 4;                               // 8 heads x 4 blocks of 16, else 4 heads x 8 blocks of 8
-        const int zq_head = gq8 ? lane >> 2 : lane >> 3, zq_blk = gq8 ? lane & 3 : lane & 7;
-        const int zq_c0 = 64 * hf + zq_blk * (gq8 ? 16 : 8);
-        uint4 qv0 = make_uint4(0u, 0u, 0u, 0u), qv1 = make_uint4(0u, 0u, 0u, 0u);
-        if (zq_head < p.gqa) {
-            const __nv_bfloat16 *qp = p.q + (int64_t)b * p.q_sb + (int64_t)(h * p.gqa + zq_head) * p.q_sh + zq_c0;
-            if (p.q_vec_ok) {
-                qv0 = __ldg(reinterpret_cast<const uint4 *>(qp));
-                if (gq8) qv1 = __ldg(reinterpret_cast<const uint4 *>(qp) + 1);
-            } else {
-                const uint16_t *q16 = reinterpret_cast<const uint16_t *>(qp);
-                auto pair = [&](int i) { return (uint32_t)__ldg(q16 + i) | ((uint32_t)__ldg(q16 + i + 1) << 16); };
-                qv0 = make_uint4(pair(0), pair(2), pair(4), pair(6));
-                if (gq8) qv1 = make_uint4(pair(8), pair(10), pair(12), pair(14));
-            }
-        }
         if (!mbar_wait(bar_full + 8 * s, ph, wait_limit)) {
-            if (lane == 0) { or_status(p.status, OMMX_ST_TIMEOUT); atomicExch(s_abort, 1); }
+            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
             return false;
         }
-        const int lg = it * GS + gsel;                           // local group of this unit
-        if (lg < ngroups && !(p.abl & ABL_NO_COMPUTE)) {
-            // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
-            // run up to NS groups ahead and the tiles of one unit are built by different warps, so
-            // "tile k was read" events rotate over NS barriers per unit (barrier k % NS, phase
-            // k / NS): the newest event a waiter can be missing is then always the one it waits
-            // for, never an older phase of the same parity.
+        const int lg = (it - pc.it0) * GS + gsel;                 // local group of this unit
+        // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
+        // run up to NS groups ahead and the tiles of one unit are built by different warps, so
+        // "tile k was read" events rotate over NS barriers per unit (barrier k % NS, phase
+        // k / NS): the newest event a waiter can be missing is then always the one it waits
+        // for, never an older phase of the same parity.  A unit without a group in this stage goes
+        // through the same hand-overs with nothing in them.
+        if (it > 0 && !mbar_wait(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it - 1, NS)), ring_phase(it - 1, NS), wait_limit)) {
+            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
+            return false;
+        }
+        if (lg < pc.ng && !(p.abl & ABL_NO_COMPUTE)) {
             uint8_t *gb = s_stage + (size_t)s * p.stage_bytes + (size_t)gsel * p.gb_bytes;
             const int d0 = 64 * hf + 2 * lane;                   // first of this lane's two channels
-            if (it > 0 && !mbar_wait(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it - 1, NS)), ring_phase(it - 1, NS), wait_limit)) {
-                if (lane == 0) { or_status(p.status, OMMX_ST_TIMEOUT); atomicExch(s_abort, 1); }
-                return false;
-            }
             bool clamped_any = false;
             const bool splice = k_out > 0 && !no_outlier;
-            // ---- first the rows the code MMAs and the softmax read (K factors, q.zp sums, V factors and
-            //      zero-points): they are cheap, and the MMA warp starts on them while the deltas are scattered ----
+            // ---- first the rows the code MMAs and the softmax read (K factors, V factors and zero-points): they are
+            //      cheap, and the MMA warp starts on them while the deltas are scattered ----
             const uint32_t e2 = *reinterpret_cast<const uint16_t *>(gb + p.o_ks + h * 128 + d0);
             const uint32_t z2 = *reinterpret_cast<const uint32_t *>(gb + p.o_kz + h * 256 + 2 * d0);
-            // this lane's entry in the fragment-ordered K factor row
-            const uint32_t kf_off = ROW_KF * DT_STRIDE + 64u * (2 * hf + (lane >> 4)) + 32u * ((lane >> 3) & 1) + 8u * (lane & 3) + 2u * ((lane >> 2) & 1);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const int e = max((int)(int8_t)(e2 >> (8 * c)), -126);
-                bool cl;
-                const uint32_t fb = pow2_f16_bits(e, cl);
-                clamped_any |= cl;
-                *reinterpret_cast<uint16_t *>(tile + kf_off + 4 * c) = (uint16_t)fb;
+            {
+                bool cl0, cl1;
+                const uint32_t f0 = pow2_f16_bits(max((int)(int8_t)e2, -126), cl0), f1 = pow2_f16_bits(max((int)(int8_t)(e2 >> 8), -126), cl1);
+                clamped_any = cl0 || cl1;
+                const uint32_t kf = hmul2_f16(f0 | (f1 << 16), slot_scale);                // * 4^-slot: exact, subnormals included
+                uint8_t *row = tile + ROW_KF * DT_STRIDE + 128 * hf + 64 * (da >> 1) + 16 * dj + 8 * (da & 1) + 2 * dh;
+                *reinterpret_cast<uint16_t *>(row) = (uint16_t)kf;
+                *reinterpret_cast<uint16_t *>(row + 4) = (uint16_t)(kf >> 16);
             }
-            {   // q.zp in fp32 from the raw bf16 query, as the reference forms it: 8 (16) products per lane, then the
-                // lanes of a head are summed by 3 (2) exchanges
-                auto dot4 = [](const uint4 &q, const uint4 &z, float acc) {
-                    const uint32_t qw[4] = {q.x, q.y, q.z, q.w}, zw[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        acc = fmaf(__uint_as_float(qw[i] << 16), __uint_as_float(zw[i] << 16), acc);
-                        acc = fmaf(__uint_as_float(qw[i] & 0xFFFF0000u), __uint_as_float(zw[i] & 0xFFFF0000u), acc);
-                    }
-                    return acc;
-                };
-                const uint8_t *zrow = gb + p.o_kz + h * 256 + 2 * zq_c0;
-                float sum = dot4(qv0, *reinterpret_cast<const uint4 *>(zrow), 0.f);
-                if (gq8) sum = dot4(qv1, *reinterpret_cast<const uint4 *>(zrow + 16), sum);
-                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-                if (!gq8) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
-                if (zq_blk == 0) reinterpret_cast<float *>(tile + ROW_ZP * DT_STRIDE)[8 * hf + zq_head] = sum;   // heads past gqa: 0
-            }
-            {   // V side: one token, two scale groups: power-of-two factor and zero-point of each
+            {   // V side: lane = (pair of tokens, scale group): power-of-two factors and zero-points of the two tokens
                 const int copy = it & 1;
-                const int tk = 16 * hf + (lane & 15), cg0 = 2 * (lane >> 4);
-                uint32_t ve = 0x8080u;                               // exponent -128 -> factor 0
-                uint32_t vz2 = 0u;
-                if (32 * lg + tk < ntok) {
-                    ve = *reinterpret_cast<const uint16_t *>(gb + p.o_vs + (tk * H + h) * 4 + cg0);
-                    vz2 = *reinterpret_cast<const uint32_t *>(gb + p.o_vz + (tk * H + h) * 8 + 2 * cg0);
-                }
-                uint8_t *vfr = tile + (ROW_VF + copy) * DT_STRIDE + 64 * ((tk >> 1) & 3) + 8 * hf + 4 * ((tk >> 3) & 1) + 2 * (tk & 1) + 16 * cg0;
-                uint8_t *ztr = tile + (ROW_ZT + copy) * DT_STRIDE + 2 * tk + 64 * cg0;
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    bool cl;
-                    const uint32_t fb = pow2_f16_bits((int)(int8_t)(ve >> (8 * c)), cl);
-                    clamped_any |= cl;
-                    *reinterpret_cast<uint16_t *>(vfr + 16 * c) = (uint16_t)fb;
-                    const float vz = bf16_bits_to_f32(c ? (vz2 >> 16) : (vz2 & 0xFFFFu));
-                    *reinterpret_cast<uint16_t *>(ztr + 64 * c) = (uint16_t)f16_bits_sat(vz);
-                }
+                const int tk = 16 * hf + 2 * (lane & 7), cg = lane >> 3;
+                uint32_t v0 = 0x80u, v1 = 0x80u, y0 = 0u, y1 = 0u;   // exponent -128 -> factor 0
+                const uint8_t *vs = gb + p.o_vs + (tk * H + h) * 4 + cg, *vz = gb + p.o_vz + (tk * H + h) * 8 + 2 * cg;
+                if (32 * lg + tk < pc.ntok) { v0 = vs[0]; y0 = *reinterpret_cast<const uint16_t *>(vz); }
+                if (32 * lg + tk + 1 < pc.ntok) { v1 = vs[4 * H]; y1 = *reinterpret_cast<const uint16_t *>(vz + 8 * H); }
+                bool cl0, cl1;
+                const uint32_t f0 = pow2_f16_bits((int)(int8_t)v0, cl0), f1 = pow2_f16_bits((int)(int8_t)v1, cl1);
+                clamped_any = clamped_any || cl0 || cl1;
+                *reinterpret_cast<uint32_t *>(tile + (ROW_VF + copy) * DT_STRIDE + 64 * cg + 16 * (lane & 3) + 8 * hf + 4 * ((lane >> 2) & 1)) = f0 | (f1 << 16);
+                *reinterpret_cast<uint32_t *>(tile + (ROW_ZT + copy) * DT_STRIDE + 2 * tk + ZT_STRIDE * cg) = pack_f16x2_sat(bf16_bits_to_f32(y0), bf16_bits_to_f32(y1));
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_trows + 8 * unit);
@@ -632,16 +736,19 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                 const uint32_t bmv[2] = {bm2.x, bm2.y};
                 // The code byte holding this lane's channels, row pz: byte pz*TS + h*32 + d0/4 of the (1 KB aligned)
                 // k_base block, with the 16-byte chunk bits XOR-ed by the row's swizzle term.  h*32 + d0/4 splits
-                // into a part above bit 7 (added to the row) and a part below (the XOR operand).
-                const uint32_t k_hi_rel = (uint32_t)(h >> 2) * 128u;
-                const uint8_t *k_hi = gb + k_hi_rel;
-                const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2));
+                // into a part above bit 7 (added to the row) and a part below (the XOR operand, swizzle term of the former
+                // included).
+                const uint8_t *k_hi = gb + (h >> 2) * 128;
+                const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2)) ^ (((uint32_t)(h >> 2) * 16u) & SWZ);
+                auto code_byte = [&](uint32_t pz) -> uint32_t {
+                    return k_hi[pz * TS + (k_lo ^ (((pz * TS) >> 3) & SWZ))];
+                };
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     const int e = max((int)(int8_t)(e2 >> (8 * c)), -126);
                     const float sc = __uint_as_float((uint32_t)(e + 127) << 23);
                     const float zp = bf16_bits_to_f32(c ? (z2 >> 16) : (z2 & 0xFFFFu));
-                    // delta between the outlier value and the base value it replaces, rounded once
+                    // delta between the outlier value and the base value it replaces: lvl * A + Bc - code * sc
                     float A = sc, Bc = 0.f;                     // shared map: lvl*s + zp - (code*s + zp)
                     if (p.use_map) {
                         const float ms = bf16_bits_to_f32(c ? (ms2 >> 16) : (ms2 & 0xFFFFu));
@@ -653,29 +760,34 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                     const uint32_t stream = st[c], stream_hi = sth[c];
                     (void)stream_hi;
                     const int fsh = 2 * ((d0 & 3) + c);          // bit position of the channel's code in its byte
-                    uint8_t *col = tile + 2 * d0 + 2 * c;
-                    if (KOUT > 0) {
+                    uint8_t *col = tile + 128 * hf + 32 * da + 16 * c + 4 * dj + 2 * dh;
+                    if constexpr (KOUT > 0 && KOUT % 2 == 0) {
                         if (__popc(bits) == KOUT) {
-                            // Two passes: all gathers (base-code byte, FP4 level) first, then the arithmetic and the
+                            // The code enters as the fraction of 1 + code/4, whose bits an AND and an OR make, so that 4 * sc moves to
+                            // the constant: lvl * A + (Bc + 4 sc) - (1 + code/4) * 4 sc.
+                            const float Bq = fmaf(4.f, sc, Bc), Sq = -4.f * sc;
+                            const int sh = 21 - fsh;              // moves the code to the top of the mantissa
+                            // Two passes: all gathers (bit walk, base-code byte) first, then the arithmetic and the
                             // stores.  In one pass every load would have to follow the previous outlier's store in
                             // program order (shared memory may alias), i.e. KOUT load round trips in a row.
-                            constexpr int KO = KOUT > 0 ? KOUT : 1;
-                            uint32_t pzs[KO], cbs[KO];
-                            float lvs[KO];
+                            uint32_t pzs[KOUT], cbs[KOUT];
 #pragma unroll
-                            for (int r = KO - 1; r >= 0; --r) {
-                                const int pz = 31 - __clz(bits);
+                            for (int r = KOUT - 1; r >= 0; --r) {
+                                const uint32_t pz = 31 - __clz(bits);
                                 bits ^= 1u << pz;
-                                pzs[r] = (uint32_t)pz;
-                                lvs[r] = s_lut[((r < 8 ? stream : stream_hi) >> (4 * (r & 7))) & 0xFu];
-                                const uint32_t row = (uint32_t)pz * (uint32_t)TS;
-                                cbs[r] = k_hi[row + (k_lo ^ (((row + k_hi_rel) >> 3) & p.swz))];
+                                pzs[r] = pz;
+                                cbs[r] = code_byte(pz);
                             }
 #pragma unroll
-                            for (int r = KO - 1; r >= 0; --r) {
-                                const float cf = (float)((cbs[r] >> fsh) & 3u);
-                                const float X = fmaf(cf, -sc, fmaf(lvs[r], A, Bc));
-                                *reinterpret_cast<uint16_t *>(col + pzs[r] * DT_STRIDE) = (uint16_t)f16_bits_of_bf16_rounded(X);
+                            for (int r = 0; r < KOUT; r += 2) {
+                                const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
+                                const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
+                                const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
+                                const float v0 = __uint_as_float(((cbs[r] << sh) & 0x600000u) | 0x3F800000u);
+                                const float v1 = __uint_as_float(((cbs[r + 1] << sh) & 0x600000u) | 0x3F800000u);
+                                const uint32_t X = f16x2_of_bf16_rounded(fmaf(v0, Sq, fmaf(lvf.x, A, Bq)), fmaf(v1, Sq, fmaf(lvf.y, A, Bq)));
+                                *reinterpret_cast<uint16_t *>(col + pzs[r] * DT_STRIDE) = (uint16_t)X;
+                                *reinterpret_cast<uint16_t *>(col + pzs[r + 1] * DT_STRIDE) = (uint16_t)(X >> 16);
                             }
                         } else {
                             or_status(p.status, OMMX_ST_BAD_GROUP);   // bitmask and value stream disagree
@@ -684,25 +796,26 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                         // any other k: one pass at run time
                         int r = __popc(bits) - 1;
                         while (bits) {
-                            const int pz = 31 - __clz(bits);
+                            const uint32_t pz = 31 - __clz(bits);
                             bits ^= 1u << pz;
                             const uint32_t nib = ((r < 8 ? stream : stream_hi) >> (4 * (r & 7))) & 0xFu;
                             --r;
-                            const uint32_t row = (uint32_t)pz * (uint32_t)TS;
-                            const uint32_t cb = k_hi[row + (k_lo ^ (((row + k_hi_rel) >> 3) & p.swz))];
-                            const float cf = (float)((cb >> fsh) & 3u);
+                            const float cf = (float)((code_byte(pz) >> fsh) & 3u);
                             const float X = fmaf(cf, -sc, fmaf(s_lut[nib], A, Bc));
-                            *reinterpret_cast<uint16_t *>(col + pz * DT_STRIDE) = (uint16_t)f16_bits_of_bf16_rounded(X);
+                            *reinterpret_cast<uint16_t *>(col + pz * DT_STRIDE) = (uint16_t)f16x2_of_bf16_rounded(X, X);
                         }
                     }
                 }
             }
             if (clamped_any) or_status(p.status, OMMX_ST_SCALE_RANGE);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tfull + 8 * unit);
+        } else if (lane == 0) {
+            mbar_arrive(bar_trows + 8 * unit);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_empty + 8 * s);
+        if (lane == 0) {
+            mbar_arrive(bar_tfull + 8 * unit);
+            mbar_arrive(bar_empty + 8 * s);
+        }
         return true;
     };
 
@@ -716,20 +829,21 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
     bool producer_alive = true;
     if (warp >= PRODUCER_WARP) {
         // =========================== producer warp(s) ===========================
-        for (int it = 1; it < n_iters; ++it) {
+        const int pw = warp - PRODUCER_WARP;
+        const uint32_t full_bytes = stage_bytes_of(pc, 0, true, lane * NPW + pw, 32 * NPW);   // this warp's share of a stage of whole groups
+        for (int it = 1;; ++it) {
+            if (it >= pc.it1 && !step_piece()) break;
+            lookup_stage(pc, it, NPW, pw);
+            const uint32_t bytes = whole_stage(pc, it) ? full_bytes : stage_bytes_of(pc, it, false, lane * NPW + pw, 32 * NPW);
             // the first NS fills find their slots fresh
             if (it >= NS && !mbar_wait(bar_empty + 8 * ring_slot(it, NS), ring_phase(it, NS) ^ 1, wait_limit)) {
-                if (lane == 0) { or_status(p.status, OMMX_ST_TIMEOUT); atomicExch(s_abort, 1); }
+                if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
                 producer_alive = false;
                 break;
             }
-            issue_stage(it, NPW, pw, pw == 0);
+            issue_stage(pc, it, NPW, pw, bytes);
         }
-        if constexpr (WIDE) {
-            // with several groups per stage, the epilogue's two CTA-wide barriers
-            if (GS > 1) { __syncthreads(); __syncthreads(); }
-            return;
-        }
+        if constexpr (WIDE) return;
         // Narrow layout: with every stage on its way this warp has nothing left to do, while the 15 decode warps share
         // 16 items per iteration: it joins them below for the very last item, so that the last iteration's 16 halves are
         // built side by side.
@@ -753,51 +867,72 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
             if constexpr (!WIDE) asm volatile("bar.arrive 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
         } else {
             asm volatile("bar.sync 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
+            if (!producer_alive || pc.more) return;
         }
-        const int n_first = is_producer ? n_items - 1 : dw;
-        const int n_end = WIDE ? n_items : (is_producer ? (producer_alive ? n_items : 0) : n_items - 1);
-        for (int n = n_first; n < n_end; n += NDW)
-            if (!decode_item(n)) break;
-        if (GS > 1) { __syncthreads(); __syncthreads(); }          // the epilogue's two CTA-wide barriers (see there)
-        return;
+        // the producer takes the very last item, when this CTA's pieces end with one that is known to be the last
+        for (int n = is_producer ? pc.it1 * 2 * NCW - 1 : dw;; n += NDW) {
+            const int it = n / (2 * NCW);
+            while (it >= pc.it1)
+                if (!step_piece()) return;
+            if (!WIDE && !is_producer && !pc.more && n == pc.it1 * 2 * NCW - 1) return;
+            if (!decode_item(pc, n)) return;
+        }
     }
 
     // =========================== MMA warps ===========================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 " OMMX_REGS_MMA ";");
     const int unit = warp;
-    const int h = unit & (H - 1), gsel = unit >> p.hshift;
+    const int h = unit % H, gsel = unit / H;
     const uint8_t *tile = s_tiles + unit * DT_BYTES;
     const uint32_t tile_s = smem_u32(tile);
     // Column n = g of every MMA is query head g of this kv head.
     const bool head_ok = g < p.gqa;
-    // B fragments of q, fp16.  QS: bf16(q*sm_scale) * 4^-slot for the code MMAs, register r = 8*wi + i holds
-    // channels (32j + 16wi + i, + 8), the pair a code word yields in one AND.  QD: plain bf16(q*sm_scale) for
-    // the delta MMAs, whose tile columns are channels in natural order.
-    uint32_t QS[16], QD[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const int wi = r >> 3, i = r & 7;
-        const int e0 = 16 * wi + i, e1 = e0 + 8;                  // channel 32j + e0 / + e1
-        const float f = 1.f / (float)(1 << (2 * code_slot(i)));
-        float lo = 0.f, hi = 0.f;
-        if (head_ok) {
-            lo = bf16_round_f32(bf16_bits_to_f32((q_s[e0 >> 1] >> (16 * (e0 & 1))) & 0xFFFFu) * p.sm_scale) * f;
-            hi = bf16_round_f32(bf16_bits_to_f32((q_s[e1 >> 1] >> (16 * (e1 & 1))) & 0xFFFFu) * p.sm_scale) * f;
-        }
-        QS[r] = pack_f16x2(lo, hi);
-    }
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        float lo = 0.f, hi = 0.f;
-        if (head_ok) {
-            lo = bf16_round_f32(bf16_bits_to_f32(q_d[r] & 0xFFFFu) * p.sm_scale);
-            hi = bf16_round_f32(bf16_bits_to_f32(q_d[r] >> 16) * p.sm_scale);
-        }
-        QD[r] = pack_f16x2(lo, hi);
-    }
     // per-lane fragment addresses inside the sidecar tile
     const uint32_t a_delta = tile_s + ((lane & 7) + 8 * ((lane >> 3) & 1)) * DT_STRIDE + 16 * (lane >> 4);
-    const uint8_t *p_kf = tile + ROW_KF * DT_STRIDE + 64 * j;
+    const uint8_t *p_kf = tile + ROW_KF * DT_STRIDE + 16 * j;       // 16-byte piece q2 of lane group j at 64 q2 + 16 j: one line for all four
+    // V codes: row r of a 16x16 byte matrix is token sigma(r) = 2 (r / 4) + (r / 2) % 2 + 8 (r % 2) of its 16, so that the four
+    // bytes a lane receives are tokens 2j, 8 + 2j, 2j + 1, 9 + 2j: bytes 0 and 2 sit in the two halves of a register as they
+    // are, bytes 1 and 3 after a shift.
+    const uint32_t v_off = swz128((uint32_t)((2 * ((lane & 15) >> 2) + ((lane >> 1) & 1) + 8 * (lane & 1)) * TS + h * 32 + 16 * (lane >> 4)), SWZ);
+    static_assert(SWZ == 0 || (16 * TS) % 1024 == 0, "the second half of the tokens has the same swizzle");
+    const bool do_k = !(p.abl & ABL_NO_K), do_v = !(p.abl & ABL_NO_V);
+    const bool has_delta = !(k_out == 0 || no_outlier);
+
+    bool gave_up = false;                        // a wait ran out: no more groups, but every piece still goes through its epilogue
+    do {
+    // B fragments of q.  QR: raw bf16, registers 4v..4v+3 hold channels 32v + 8j .. + 7 (zero-point MMAs).  QP: fp16 of
+    // bf16(q * sm_scale), register r = 8w + i holds channels (64w + 16j + i, + 8), the pair a code word yields in one AND (code
+    // and delta MMAs).
+    uint32_t QR[16], QP[16];
+    {
+        const uint16_t *qrow = reinterpret_cast<const uint16_t *>(p.q + (int64_t)pc.b * p.q_sb + (int64_t)(h * p.gqa + (head_ok ? g : 0)) * p.q_sh);
+        auto eight = [&](const uint16_t *q8, uint32_t (&w)[4]) __attribute__((always_inline)) {
+            if (p.q_vec_ok) {
+                const uint4 t = __ldg(reinterpret_cast<const uint4 *>(q8));
+                w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
+            } else {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) w[v] = (uint32_t)__ldg(q8 + 2 * v) | ((uint32_t)__ldg(q8 + 2 * v + 1) << 16);
+            }
+        };
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            uint32_t w[4];
+            eight(qrow + 32 * v + 8 * j, w);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) QR[4 * v + i] = head_ok ? w[i] : 0u;
+        }
+        auto scaled = [&](uint32_t b16) { return bf16_round_f32(bf16_bits_to_f32(b16 & 0xFFFFu) * p.sm_scale); };
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            uint32_t lo[4], hi[4];
+            eight(qrow + 64 * w + 16 * j, lo);
+            eight(qrow + 64 * w + 16 * j + 8, hi);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                QP[8 * w + i] = head_ok ? pack_f16x2(scaled(lo[i >> 1] >> (16 * (i & 1))), scaled(hi[i >> 1] >> (16 * (i & 1)))) : 0u;
+        }
+    }
     // ---- online softmax state of heads 2j and 2j+1 (the two columns this lane holds) ----
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     // acc[2*cg + u]: rows = channels 32cg + 4g + u (regs 0,1) and 32cg + 4g + 2 + u (regs 2,3), columns = heads
@@ -805,69 +940,72 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
 #pragma unroll
     for (int i = 0; i < 8; ++i) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f; }
     float accz[4] = {0.f, 0.f, 0.f, 0.f};        // rows = V scale groups: sum_t vz[t][cg] * P[t][head]
-    uint32_t consumed = 0;
-    const bool do_k = !(p.abl & ABL_NO_K), do_v = !(p.abl & ABL_NO_V);
-    const bool has_delta = !(k_out == 0 || no_outlier);
 
-    for (int it = 0; it < n_iters; ++it) {
+    for (int it = pc.it0; it < pc.it1 && !gave_up; ++it) {
         const int s = ring_slot(it, NS);
         const uint32_t ph = ring_phase(it, NS);
-        const int lg = it * GS + gsel;                               // local group of this warp
-        const bool active = lg < ngroups && !(p.abl & ABL_NO_COMPUTE);
+        const int lg = (it - pc.it0) * GS + gsel;                    // local group of this warp
+        const bool active = lg < pc.ng && !(p.abl & ABL_NO_COMPUTE);
         if (!mbar_wait(bar_full + 8 * s, ph, wait_limit)) {
-            if (lane == 0) { or_status(p.status, OMMX_ST_TIMEOUT); atomicExch(s_abort, 1); }
-            m_run[0] = m_run[1] = -INFINITY; l_run[0] = l_run[1] = 0.f;
+            gave_up = true;
             break;
         }
         if (active) {
             uint8_t *gb = s_stage + (size_t)s * p.stage_bytes + (size_t)gsel * p.gb_bytes;
-            const uint8_t *vreg = gb + p.o_vm;                      // v_main region of the group (1 KB aligned)
+            const uint32_t v_addr = smem_u32(gb + p.o_vm) + v_off;  // v_main region of the group (1 KB aligned)
 
             // ======================= logits =======================
-            // code words of this lane's four token rows (tokens 8*nt + g), channels 32j..32j+31
+            // code words of this lane's four token rows (tokens 8*nt + g), channels 16j..16j+15 of either half
             uint2 kw[4];
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
                 kw[nt] = make_uint2(0u, 0u);
-                if (do_k) kw[nt] = *reinterpret_cast<const uint2 *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 8 * j), p.swz));
+                if (do_k) {
+                    kw[nt].x = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 4 * j), SWZ));
+                    kw[nt].y = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 16 + 4 * j), SWZ));
+                }
             }
+            // q.zp of heads 2j and 2j+1: exact bf16 products of the raw query with the zero-points, summed in fp32, every row
+            // of the A operand being the zero-point row.  It needs no tile, so it runs while the tile is built.
+            float Z0[4] = {0.f, 0.f, 0.f, 0.f}, Z1[4] = {0.f, 0.f, 0.f, 0.f};
+            {
+                const uint8_t *zrow = gb + p.o_kz + h * 256 + 16 * j;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const uint4 z = *reinterpret_cast<const uint4 *>(zrow + 64 * v);
+                    mma_bf16(Z0, z.x, z.x, z.y, z.y, QR[4 * v], QR[4 * v + 1]);
+                    mma_bf16(Z1, z.z, z.z, z.w, z.w, QR[4 * v + 2], QR[4 * v + 3]);
+                }
+            }
+            const float Sz[2] = {(Z0[0] + Z1[0]) * p.sm_scale, (Z0[1] + Z1[1]) * p.sm_scale};
             // The unit's sidecar tile arrives in two steps: first the factor and zero-point rows, then the outlier
             // deltas.  The code MMAs run on the first, while the decode warps still scatter the deltas.
-            if (!mbar_wait(bar_trows + 8 * unit, consumed & 1u, wait_limit)) {
-                if (lane == 0) { or_status(p.status, OMMX_ST_TIMEOUT); atomicExch(s_abort, 1); }
-                m_run[0] = m_run[1] = -INFINITY; l_run[0] = l_run[1] = 0.f;
+            if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
+                gave_up = true;
                 break;
             }
-            float Sc[2][4], Sd[2][4], Sz[2];
+            float Sc[2][4], Sd[2][4];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) { Sc[mt][0] = Sc[mt][1] = Sc[mt][2] = Sc[mt][3] = 0.f; Sd[mt][0] = Sd[mt][1] = Sd[mt][2] = Sd[mt][3] = 0.f; }
             // Two accumulators take turns, so that neighbours in the instruction stream never wait on each other
             // (the asm statements keep their order, so the order written here is the order issued).
-            {
-                // q.zp of heads 2j and 2j+1: the two channel halves' fp32 partial sums, times sm_scale
-                const float2 za = *reinterpret_cast<const float2 *>(tile + ROW_ZP * DT_STRIDE + 8 * j);
-                const float2 zb = *reinterpret_cast<const float2 *>(tile + ROW_ZP * DT_STRIDE + 32 + 8 * j);
-                Sz[0] = (za.x + zb.x) * p.sm_scale;
-                Sz[1] = (za.y + zb.y) * p.sm_scale;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
+            for (int q2 = 0; q2 < 4; ++q2) {
+                const uint4 f = *reinterpret_cast<const uint4 *>(p_kf + 64 * q2);      // two k-steps' factor pairs
+#pragma unroll
+                for (int q = 2 * q2; q < 2 * q2 + 2; ++q) {
                     const int wi = q >> 2, i0 = 2 * (q & 3);
-                    const uint2 fq = reinterpret_cast<const uint2 *>(p_kf)[q];      // this k-step's two factor pairs
-                    const uint32_t b0 = hmul2_f16(QS[2 * q], fq.x), b1 = hmul2_f16(QS[2 * q + 1], fq.y);
-                    {
-                        const uint32_t wlo = wi ? kw[0].y : kw[0].x, whi = wi ? kw[1].y : kw[1].x;
-                        mma_f16(Sc[0], code_pair(wlo, i0), code_pair(whi, i0), code_pair(wlo, i0 + 1), code_pair(whi, i0 + 1), b0, b1);
-                    }
-                    {
-                        const uint32_t wlo = wi ? kw[2].y : kw[2].x, whi = wi ? kw[3].y : kw[3].x;
-                        mma_f16(Sc[1], code_pair(wlo, i0), code_pair(whi, i0), code_pair(wlo, i0 + 1), code_pair(whi, i0 + 1), b0, b1);
+                    const uint32_t b0 = hmul2_f16(QP[2 * q], q & 1 ? f.z : f.x), b1 = hmul2_f16(QP[2 * q + 1], q & 1 ? f.w : f.y);
+#pragma unroll
+                    for (int mt = 0; mt < 2; ++mt) {
+                        const uint32_t wlo = wi ? kw[2 * mt].y : kw[2 * mt].x, whi = wi ? kw[2 * mt + 1].y : kw[2 * mt + 1].x;
+                        mma_f16(Sc[mt], code_pair(wlo, i0), code_pair(whi, i0), code_pair(wlo, i0 + 1), code_pair(whi, i0 + 1), b0, b1);
                     }
                 }
             }
             if (has_delta) {
-                if (!mbar_wait(bar_tfull + 8 * unit, consumed & 1u, wait_limit)) {
-                    if (lane == 0) { or_status(p.status, OMMX_ST_TIMEOUT); atomicExch(s_abort, 1); }
-                    m_run[0] = m_run[1] = -INFINITY; l_run[0] = l_run[1] = 0.f;
+                if (!mbar_wait(bar_tfull + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
+                    gave_up = true;
                     break;
                 }
                 uint32_t d0f[4], d1f[4];                         // delta fragments of m-tile 0 / 1
@@ -875,14 +1013,14 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     ldsm_x4(a_delta + 16 * DT_STRIDE + 32 * q, d1f[0], d1f[1], d1f[2], d1f[3]);
-                    mma_f16(Sd[0], d0f[0], d0f[1], d0f[2], d0f[3], QD[2 * q], QD[2 * q + 1]);
+                    mma_f16(Sd[0], d0f[0], d0f[1], d0f[2], d0f[3], QP[2 * q], QP[2 * q + 1]);
                     if (q < 7) ldsm_x4(a_delta + 32 * (q + 1), d0f[0], d0f[1], d0f[2], d0f[3]);
-                    mma_f16(Sd[1], d1f[0], d1f[1], d1f[2], d1f[3], QD[2 * q], QD[2 * q + 1]);
+                    mma_f16(Sd[1], d1f[0], d1f[1], d1f[2], d1f[3], QP[2 * q], QP[2 * q + 1]);
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot((int)consumed, NS)));   // the next tile may be built
-            ++consumed;
+            // the next tile may be built (where warps merge below, they do it in their tiles: not before that)
+            if (lane == 0 && (GS == 1 || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
 
             // ======================= online softmax =======================
             // x[mt][r]: token 16mt + g + 8(r>>1), head 2j + (r&1)
@@ -898,12 +1036,12 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                     for (int r = 0; r < 4; ++r) x[mt][r] = p.logit_cap * tanhf(x[mt][r] / p.logit_cap);
             }
             const int tok_base = 32 * lg;
-            if (tok_base + 32 > ntok) {
+            if (tok_base + 32 > pc.ntok) {
 #pragma unroll
                 for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
-                        if (tok_base + 16 * mt + g + 8 * (r >> 1) >= ntok) x[mt][r] = -INFINITY;
+                        if (tok_base + 16 * mt + g + 8 * (r >> 1) >= pc.ntok) x[mt][r] = -INFINITY;
             }
             float corr[2], mneg[2];
 #pragma unroll
@@ -944,35 +1082,21 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                 const int copy = it & 1;
                 uint32_t VF[16];                                     // factor pairs, index 4cg + 2ks + b
                 {
-                    const uint8_t *p_vf = tile + (ROW_VF + copy) * DT_STRIDE + 64 * j;
+                    const uint8_t *p_vf = tile + (ROW_VF + copy) * DT_STRIDE + 16 * j;
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
-                        const uint4 t = reinterpret_cast<const uint4 *>(p_vf)[v];
+                        const uint4 t = *reinterpret_cast<const uint4 *>(p_vf + 64 * v);
                         VF[4 * v] = t.x; VF[4 * v + 1] = t.y; VF[4 * v + 2] = t.z; VF[4 * v + 3] = t.w;
                     }
                 }
-                const uint8_t *p_zt = tile + (ROW_ZT + copy) * DT_STRIDE + 64 * (g & 3) + 4 * j;
-                const uint32_t v_hi_rel = (uint32_t)(h >> 2) * 128u, v_lo = (uint32_t)((h & 3) * 32 + g);
+                const uint8_t *p_zt = tile + (ROW_ZT + copy) * DT_STRIDE + ZT_STRIDE * (g & 3) + 4 * j;
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
-                    const int tA = 16 * ks + 2 * j;
-                    // Byte 8cg + g of a token row's 32-byte head slice, four scale groups per row.  The swizzle term
-                    // of a row only touches bits 4..6, so two XORs give the addresses of groups 0 and 2 and the
-                    // other two are 8 bytes on.
-                    uint32_t vb[4][4];                               // [token of (tA, tA+1, tA+8, tA+9)][scale group]
-#pragma unroll
-                    for (int tt = 0; tt < 4; ++tt) {
-                        const uint32_t rowhi = (uint32_t)(tA + (tt & 1) + 8 * (tt >> 1)) * (uint32_t)TS + v_hi_rel;
-                        const uint32_t tm = (rowhi >> 3) & p.swz;
-                        const uint8_t *r0 = vreg + (rowhi + (v_lo ^ tm)), *r1 = vreg + (rowhi + ((v_lo ^ 16u) ^ tm));
-                        vb[tt][0] = r0[0]; vb[tt][1] = r0[8];
-                        vb[tt][2] = r1[0]; vb[tt][3] = r1[8];
-                    }
+                    uint32_t vc[4];                                  // by scale group: channels 32cg + 4g .. + 3 of four tokens, a byte each
+                    ldsm_b8_trans_x2(v_addr + 16 * TS * ks, vc);
 #pragma unroll
                     for (int cg = 0; cg < 4; ++cg) {
-                        // channels 32cg + 4g .. + 3 of four tokens: one byte each
-                        const uint32_t bA = vb[0][cg], bA1 = vb[1][cg], bB = vb[2][cg], bB1 = vb[3][cg];
-                        const uint32_t w01 = bA | (bA1 << 16), w89 = bB | (bB1 << 16);
+                        const uint32_t w01 = vc[cg], w89 = vc[cg] >> 8;
                         const uint32_t pb0 = hmul2_f16(T[ks][0], VF[4 * cg + 2 * ks]), pb1 = hmul2_f16(T[ks][1], VF[4 * cg + 2 * ks + 1]);
 #pragma unroll
                         for (int u = 0; u < 2; ++u)
@@ -987,10 +1111,20 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
                     mma_f16(accz, za0, 0u, za2, 0u, T[ks][0], T[ks][1]);
                 }
             }
+        } else {
+            if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
+                gave_up = true;
+                break;
+            }
+            if (lane == 0 && (GS == 1 || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
         }
         // release the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_empty + 8 * s);
+    }
+    if (gave_up) {
+        if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
+        m_run[0] = m_run[1] = -INFINITY; l_run[0] = l_run[1] = 0.f;
     }
 
     // ---- epilogue: this lane holds 16 channels of heads 2j and 2j+1; merge warps that share a head ----
@@ -1018,22 +1152,22 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
         }
     }
 
-    // Several groups per stage (fewer than 8 local kv heads): the warps that share a head merge through the ring memory,
-    // once every warp (and the producer) is done with it.  With 8 heads every warp owns its head and writes straight away.
-    float *scratch = reinterpret_cast<float *>(s_stage);             // [NCW][32 lanes][36]
+    // Several groups per stage (fewer than 8 local kv heads): the warps that share a head merge, each through the delta rows
+    // of its own tile, which nobody builds again before it is handed back below.  With 8 heads every warp owns its head and
+    // writes straight away.
+    static_assert(32 * 36 * 4 <= 32 * DT_STRIDE, "the merge fits the delta rows of a tile");
     if (GS > 1) {
-        __syncthreads();
         if (gsel > 0) {
-            float *my = scratch + ((size_t)unit * 32 + lane) * 36;
+            float *my = reinterpret_cast<float *>(s_tiles + unit * DT_BYTES) + lane * 36;
             my[0] = m_run[0]; my[1] = m_run[1]; my[2] = l_tot[0]; my[3] = l_tot[1];
 #pragma unroll
             for (int i = 0; i < 16; ++i) { my[4 + i] = outv[0][i]; my[20 + i] = outv[1][i]; }
         }
-        __syncthreads();
+        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
     }
     if (gsel == 0) {
         for (int o = 1; o < GS; ++o) {
-            const float *ot = scratch + ((size_t)(o * H + h) * 32 + lane) * 36;
+            const float *ot = reinterpret_cast<const float *>(s_tiles + (o * H + h) * DT_BYTES) + lane * 36;
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 const float m2 = ot[hh], l2 = ot[2 + hh];
@@ -1051,7 +1185,7 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
             const int head = 2 * j + hh;
             if (head < p.gqa) {
                 const float inv = l_tot[hh] > 0.f ? 1.f / l_tot[hh] : 0.f;
-                float *dst = p.al + (int64_t)b * p.al_sb + (int64_t)(h * p.gqa + head) * p.al_sh + (int64_t)split * p.al_ss;
+                float *dst = p.al + (int64_t)pc.b * p.al_sb + (int64_t)(h * p.gqa + head) * p.al_sh + (int64_t)pc.slot * p.al_ss;
 #pragma unroll
                 for (int cg = 0; cg < 4; ++cg)
 #pragma unroll
@@ -1060,6 +1194,11 @@ __global__ void __launch_bounds__(WarpLayout<WIDE>::THREADS, 1) decode_stage1_ke
             }
         }
     }
+    if (GS > 1) {
+        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
+        if (lane == 0) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(pc.it1 - 1, NS)));
+    }
+    } while (step_piece());
 }
 
 // =================================================================================================
@@ -1075,7 +1214,7 @@ struct S2Params {
     int32_t max_tail;
     const float *al;
     int64_t al_sb, al_sh, al_ss;
-    int32_t S;
+    int32_t S, B, ncta, waves;           // ncta: CTAs stage 1 shared the groups over (0: equal splits per sequence)
     void *o;
     int32_t o_bf16;
     int64_t o_sb, o_sh;
@@ -1110,12 +1249,39 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     const int hq = blockIdx.x, b = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = hq / p.gqa;
-    const int seq = p.b_seq_len[b];
+    // Lengths: this sequence's, and what the share-out of stage 1 depends on (all, longest, those before this one), in one
+    // round of loads.
+    int seq, total = 0, longest = 0, before = 0;
+    if (p.B == 1) {
+        seq = p.b_seq_len[0];
+        total = longest = groups_of(seq);
+    } else {
+        seq = p.b_seq_len[b];
+        for (int i = lane; i < p.B; i += 32) {
+            const int n = groups_of(p.b_seq_len[i]);
+            total += n;
+            longest = max(longest, n);
+            if (i < b) before += n;
+        }
+        total = __reduce_add_sync(0xFFFFFFFFu, total);
+        before = __reduce_add_sync(0xFFFFFFFFu, before);
+        longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+    }
     int tail = p.b_tail_len ? p.b_tail_len[b] : 0;
     tail = max(0, min(tail, min(p.max_tail, S2_MAX_TAIL)));
     const int D = p.D;                                                   // == HD
-    const int per = (seq > 0 && p.S > 0) ? (((seq + p.S - 1) / p.S) + 31) / 32 * 32 : 0;
-    const int nsplit = per > 0 ? min(p.S, (seq + per - 1) / per) : 0;    // splits s with s*per < seq
+    // workspace slots stage 1 wrote for this sequence
+    const int groups = groups_of(seq);
+    int nsplit = 0;
+    if (p.S > 0 && groups > 0) {
+        const int per = p.ncta > 0 ? share_plan_of(total, longest, p.B, p.S, p.ncta, p.waves).per : 0;
+        if (per == 0) {
+            const int equal = (groups + p.S - 1) / p.S;
+            nsplit = (groups + equal - 1) / equal;
+        } else {
+            nsplit = (before + groups - 1) / per - before / per + 1;
+        }
+    }
     const float *base = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh;
 
     constexpr int PRE_T = 5, PRE_S = 10;                                 // rows / splits per warp held in registers
@@ -1415,7 +1581,7 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 // Plane viewed as [bytes/128][128] uint8, box = one page, 128-byte swizzle.  Returns false when the
-// map cannot be built (the caller then stages the plane with plain bulk copies).
+// map cannot be built.
 // Encoded maps are kept in a small table keyed by (base, bytes, box rows): a serving loop calls with the
 // same planes every step and the driver call costs about a microsecond.
 static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes, int rows_per_page) {
@@ -1455,9 +1621,8 @@ static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes,
 }
 
 static size_t stage1_smem(const S1Params &p) {
-    return 1024 + (size_t)p.nstages * p.stage_bytes + (size_t)NCW * DT_BYTES + (MAX_SPLIT_GROUPS + MAX_SPLIT_PAGES) * 4 + 64
-           + (2 * MAX_STAGES + (2 + MAX_STAGES) * NCW) * 8 + 16
-           + (size_t)p.GS * (4 * p.ppg + 6) * sizeof(CopyDesc);       // the copy roles of one stage come last
+    return 1024 + (size_t)p.nstages * p.stage_bytes + (size_t)NCW * DT_BYTES + 64 + (2 * MAX_STAGES + (2 + MAX_STAGES) * NCW) * 8
+           + (size_t)p.GS * (4 * p.ppg + 6) * (sizeof(CopyDesc) + 4) + MAX_PIECES * sizeof(Piece);   // copy roles, their table entries, pieces
 }
 
 // Launch as a programmatic dependent of whatever precedes it in the stream: the grid may be placed while that
@@ -1484,9 +1649,33 @@ static int current_device(int *dev) {
     return 0;
 }
 
-template <int KOUT, bool WIDE>
-static int launch_s1_layout(const S1Params &p, dim3 grid, size_t smem, cudaStream_t st) {
-    using L = WarpLayout<WIDE>;
+static int sm_count_of(int dev) {
+    static std::atomic<int> counts[MAX_DEVICES];
+    int n = counts[dev].load(std::memory_order_acquire);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = 148; }
+        counts[dev].store(n, std::memory_order_release);
+    }
+    return n;
+}
+
+// CTAs of a stage-1 launch: one per SM, or one per group where there are fewer groups than SMs; and the rounds of them
+// that equal splits would take (capped: past the cap they are never the choice)
+static int stage1_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
+    int dev = 0;
+    if (int rc = current_device(&dev)) return rc;
+    const long long groups = (long long)a->batch * ((a->max_seq_len + 31) / 32);
+    // (a CTA lists at most MAX_PIECES pieces: more CTAs than SMs for thousands of short sequences)
+    const long long splits = (long long)a->batch * a->num_kv_splits;
+    const long long least = (min((long long)a->batch, groups) > MAX_PIECES ? (max(groups, splits) + MAX_PIECES - 1) / MAX_PIECES : 1);
+    *ncta = (int)max(min((long long)sm_count_of(dev), max(groups, 1ll)), least);
+    *waves = (int)min((splits + *ncta - 1) / *ncta, 1024ll);
+    return 0;
+}
+
+template <int KOUT, int H>
+static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
+    using L = WarpLayout<H>;
     // function attributes belong to (kernel instantiation, device): one entry per device ordinal
     static std::atomic<size_t> attr_smem[MAX_DEVICES];
     static std::atomic<int> regs_state[MAX_DEVICES];   // 0 unknown, 1 enough, 2 too few
@@ -1495,27 +1684,31 @@ static int launch_s1_layout(const S1Params &p, dim3 grid, size_t smem, cudaStrea
     int regs_ok = regs_state[dev].load(std::memory_order_acquire);
     if (regs_ok == 0) {
         cudaFuncAttributes fa;
-        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, WIDE>));
+        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, H>));
         // setmaxnreg.inc must find the registers the other roles gave back
-        const int need = NCW * 32 * REGS_MMA + (WIDE ? L::NDW * 32 * REGS_DECODE + L::NPW * 32 * REGS_PRODUCER
-                                                     : (L::THREADS - NCW * 32) * REGS_DECODE);
+        const int need = NCW * 32 * REGS_MMA + (L::WIDE ? L::NDW * 32 * REGS_DECODE + L::NPW * 32 * REGS_PRODUCER
+                                                        : (L::THREADS - NCW * 32) * REGS_DECODE);
         regs_ok = fa.numRegs * L::THREADS >= need ? 1 : 2;
         regs_state[dev].store(regs_ok, std::memory_order_release);
     }
     if (regs_ok != 1) return fail(OMMX_E_CUDA, "stage 1 was compiled with fewer registers than its warp roles need");
     if (smem > attr_smem[dev].load(std::memory_order_acquire)) {
-        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_kernel<KOUT, WIDE>,
+        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_kernel<KOUT, H>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_smem[dev].store(smem, std::memory_order_release);
     }
-    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, WIDE>, grid, L::THREADS, smem, st, p));
+    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H>, dim3(p.ncta), L::THREADS, smem, st, p));
     count_launch();
     return 0;
 }
-// one or two local kv heads: many small copies per ring stage, the wide layout's four producer warps issue them
 template <int KOUT>
-static int launch_s1(const S1Params &p, dim3 grid, size_t smem, cudaStream_t st) {
-    return p.H <= 2 ? launch_s1_layout<KOUT, true>(p, grid, smem, st) : launch_s1_layout<KOUT, false>(p, grid, smem, st);
+static int launch_s1_heads(const S1Params &p, size_t smem, cudaStream_t st) {
+    switch (p.H) {
+        case 8: return launch_s1<KOUT, 8>(p, smem, st);
+        case 4: return launch_s1<KOUT, 4>(p, smem, st);
+        case 2: return launch_s1<KOUT, 2>(p, smem, st);
+        default: return launch_s1<KOUT, 1>(p, smem, st);
+    }
 }
 
 }  // namespace ommx
@@ -1527,15 +1720,23 @@ namespace ommx {
 // kernel (decode_stage1_tc_kernel) where its shared-memory plan fits - 4 or 8 local kv heads with GQA <= 4, fewer
 // heads at any GQA <= 8 - and no differential-timing knob is set; it produces the same results within the path's
 // tolerance and is kept for further work on its pipeline.  The variable is read per call.
-static int stage1_choice() {
+static bool tensor_core_stage1() {
     const char *e = getenv("OMMX_B200_STAGE1");
-    return (e && !strcmp(e, "tc")) ? 1 : 0;
+    return e && !strcmp(e, "tc");
+}
+// Its shared memory for this call, or 0 where the default kernel serves
+static size_t tensor_core_plan(const ommx_decode_args *a, const S1Params &p, TcParams *T) {
+    if (!tensor_core_stage1() || p.abl != 0 || p.gqa > 8 || p.idx7) return 0;
+    T->s = p;
+    T->s.GS = 1;
+    T->s.stage_bytes = p.gb_bytes;
+    const int per_max = ((a->max_seq_len + a->num_kv_splits - 1) / a->num_kv_splits + 31) / 32;   // groups of the longest split
+    const size_t smem = tc_layout(*T, p.gqa <= 4 ? 4 : 8, per_max + 1);
+    return smem <= 232448 ? smem : 0;
 }
 
-static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
-    if (a->max_seq_len <= 0) return 0;                                   // tail-only decode
+static int fill_stage1(const ommx_decode_args *a, S1Params &p) {
     const ommx_kv_planes &pl = a->planes;
-    S1Params p;
     p.q = (const __nv_bfloat16 *)a->q; p.q_sb = a->q_stride_b; p.q_sh = a->q_stride_h;
     p.B = a->batch; p.Hq = a->n_q_heads; p.H = pl.n_kv_heads; p.gqa = a->n_q_heads / pl.n_kv_heads;
     p.q_vec_ok = (((uintptr_t)a->q & 15) == 0 && a->q_stride_b % 8 == 0 && a->q_stride_h % 8 == 0) ? 1 : 0;
@@ -1568,26 +1769,41 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
     p.rows_per_page = (int32_t)(page_bytes / 128);
     memset(&p.tmap_k, 0, sizeof(CUtensorMap));
     memset(&p.tmap_v, 0, sizeof(CUtensorMap));
-    if (H >= 4 && page_bytes % 1024 == 0 &&
-        make_code_map(&p.tmap_k, pl.k_base, (int64_t)pl.num_pages * page_bytes, p.rows_per_page) &&
-        make_code_map(&p.tmap_v, pl.v_main, (int64_t)pl.num_pages * page_bytes, p.rows_per_page))
+    if (H >= 4) {                                                        // a page is whole 1 KB swizzle atoms
+        if (!make_code_map(&p.tmap_k, pl.k_base, (int64_t)pl.num_pages * page_bytes, p.rows_per_page) ||
+            !make_code_map(&p.tmap_v, pl.v_main, (int64_t)pl.num_pages * page_bytes, p.rows_per_page))
+            return fail(OMMX_E_CUDA, "stage 1: the tensor maps of the code planes could not be encoded");
         p.swz = 0x70u;
+    }
     const int round_to = p.swz ? 1024 : 128;
     p.gb_bytes = (p.gb_bytes + round_to - 1) / round_to * round_to;
     p.stage_bytes = p.GS * p.gb_bytes;
     p.abl = a->abl_flags;
-    if (stage1_choice() == 1 && p.abl == 0 && p.gqa <= 8 && !p.idx7) {
+    return 0;
+}
+
+// CTAs that stage 1 shares the groups over, 0 where it makes equal splits per sequence (the tensor-core kernel): stage 2
+// works out the same workspace slots from it
+static int shared_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
+    if (tensor_core_stage1()) {
+        S1Params p;
         TcParams T;
-        T.s = p;
-        T.s.GS = 1;
-        T.s.stage_bytes = p.gb_bytes;
-        const int gqap = p.gqa <= 4 ? 4 : 8;
-        const int per_max = ((a->max_seq_len + a->num_kv_splits - 1) / a->num_kv_splits + 31) / 32;   // groups of the longest split
-        const size_t tsmem = tc_layout(T, gqap, per_max + 1);
-        if (tsmem != 0 && tsmem <= 232448) {
+        if (int rc = fill_stage1(a, p)) return rc;
+        if (tensor_core_plan(a, p, &T)) { *ncta = 0; return 0; }
+    }
+    return stage1_ctas(a, ncta, waves);
+}
+
+static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
+    if (a->max_seq_len <= 0) return 0;                                   // tail-only decode
+    S1Params p;
+    if (int rc = fill_stage1(a, p)) return rc;
+    if (tensor_core_stage1()) {
+        TcParams T;
+        if (const size_t tsmem = tensor_core_plan(a, p, &T)) {
             dim3 tgrid(a->num_kv_splits, a->batch);
-            if (gqap == 4) return H == 8 ? launch_tc<4, true>(T, tgrid, tsmem, st) : launch_tc<4, false>(T, tgrid, tsmem, st);
-            return H == 8 ? launch_tc<8, true>(T, tgrid, tsmem, st) : launch_tc<8, false>(T, tgrid, tsmem, st);
+            if (p.gqa <= 4) return p.H == 8 ? launch_tc<4, true>(T, tgrid, tsmem, st) : launch_tc<4, false>(T, tgrid, tsmem, st);
+            return p.H == 8 ? launch_tc<8, true>(T, tgrid, tsmem, st) : launch_tc<8, false>(T, tgrid, tsmem, st);
         }
     }
     // deepest ring that fits the 227 KB a CTA may use
@@ -1595,15 +1811,15 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
     while (p.nstages > 2 && stage1_smem(p) > 232448) --p.nstages;
     const size_t smem = stage1_smem(p);
     if (smem > 232448) return fail(OMMX_E_UNSUPPORTED, "stage 1 planes of one group do not fit shared memory");
-    dim3 grid(a->num_kv_splits, a->batch);
+    if (int rc = stage1_ctas(a, &p.ncta, &p.waves)) return rc;
     switch (p.k_out) {                       // the serving recipes get the unrolled two-pass splice
-        case 0: return launch_s1<0>(p, grid, smem, st);
-        case 2: return launch_s1<2>(p, grid, smem, st);
-        case 4: return launch_s1<4>(p, grid, smem, st);
-        case 6: return launch_s1<6>(p, grid, smem, st);
-        case 8: return launch_s1<8>(p, grid, smem, st);
-        case 12: return launch_s1<12>(p, grid, smem, st);
-        default: return launch_s1<-1>(p, grid, smem, st);
+        case 0: return launch_s1_heads<0>(p, smem, st);
+        case 2: return launch_s1_heads<2>(p, smem, st);
+        case 4: return launch_s1_heads<4>(p, smem, st);
+        case 6: return launch_s1_heads<6>(p, smem, st);
+        case 8: return launch_s1_heads<8>(p, smem, st);
+        case 12: return launch_s1_heads<12>(p, smem, st);
+        default: return launch_s1_heads<-1>(p, smem, st);
     }
 }
 
@@ -1620,6 +1836,9 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool after_
     p.max_tail = a->max_tail_len;
     p.al = a->attn_logits; p.al_sb = a->al_stride_b; p.al_sh = a->al_stride_h; p.al_ss = a->al_stride_s;
     p.S = a->max_seq_len > 0 ? a->num_kv_splits : 0;
+    p.B = a->batch; p.ncta = p.waves = 0;
+    if (p.S > 0)
+        if (int rc = shared_ctas(a, &p.ncta, &p.waves)) return rc;
     p.o = a->o; p.o_bf16 = (a->o_dtype == OMMX_DT_BF16); p.o_sb = a->o_stride_b; p.o_sh = a->o_stride_h;
     p.lse = a->lse; p.lse_sb = a->lse_stride_b;
     p.sm_scale = a->sm_scale; p.logit_cap = a->logit_cap;
@@ -1670,18 +1889,9 @@ extern "C" int ommx_b200_min_num_kv_splits(int32_t max_seq_len, int32_t page_siz
 
 extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, int32_t n_kv_heads) {
     (void)n_kv_heads;                       // one CTA serves all local kv heads of its token range
-    static std::atomic<int> sm_counts[ommx::MAX_DEVICES];       // per device ordinal
     int dev = 0, sm_count = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < ommx::MAX_DEVICES) {
-        sm_count = sm_counts[dev].load(std::memory_order_acquire);
-        if (sm_count == 0) {
-            int n = 0;
-            sm_count = (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) ? n : 148;
-            sm_counts[dev].store(sm_count, std::memory_order_release);
-        }
-    } else {
-        (void)cudaGetLastError();
-    }
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < ommx::MAX_DEVICES) sm_count = ommx::sm_count_of(dev);
+    else (void)cudaGetLastError();
     // One CTA runs per SM, so a launch takes (waves of CTAs) x (groups per CTA + what a CTA costs before and after its
     // steady state, about three groups' worth).  Pick the split count that minimises it: 148 at batch 1, and e.g. 18
     // rather than 19 at batch 8, where 152 CTAs would leave a second wave of four.  Ties go to fewer splits (less for
