@@ -1229,34 +1229,35 @@ struct S2Params {
     int32_t *status;
 };
 
-constexpr int S2_THREADS = 512;
-constexpr int S2_WARPS = S2_THREADS / 32;
 constexpr int S2_MAX_TAIL = 256;
 constexpr int S2_MAX_SPLITS = 1024;
 
 // One CTA per (query head, sequence).  Warps stripe over the bf16 residual rows for the logits,
 // then over the splits for the combine; every loop keeps many independent loads in flight,
 // because this kernel is pure latency (a few hundred KB through L2).
-__global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Params p) {
+// Three sizes, by what the rows of the grid need to run side by side (chosen in launch_stage2).  16 warps: one CTA per SM, all
+// of a row's loads are one round trip.  8 warps: three per SM.  4 warps: six per SM.  1024 rows (batch 32, 32 heads) took 31 us
+// with 16 warps and take 15 with 4; 512 rows 18 -> 8.7; 256 rows 9.8 -> 6.8 (8 warps).
+template <int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : (NW == 8 ? 3 : 6)) decode_stage2_kernel(const S2Params p) {
     __shared__ float s_q[HD];
     __shared__ float s_logit[S2_MAX_TAIL];
-    __shared__ float s_w[S2_MAX_SPLITS];
-    __shared__ float s_red[S2_WARPS];
-    __shared__ float s_acc[S2_WARPS][HD];
+    __shared__ float s_w[NW];
+    __shared__ float s_red[NW];
+    __shared__ float s_acc[NW][HD];
     // the next kernel in the stream (the following layer's stage 1) may be placed as SMs free up; it waits for
     // this grid to finish before it touches memory
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int hq = blockIdx.x, b = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = hq / p.gqa;
+    int tail = p.b_tail_len ? p.b_tail_len[b] : 0;                       // requested before the lengths are waited for
     // Lengths: this sequence's, and what the share-out of stage 1 depends on (all, longest, those before this one), in one
     // round of loads.
-    int seq, total = 0, longest = 0, before = 0;
-    if (p.B == 1) {
-        seq = p.b_seq_len[0];
-        total = longest = groups_of(seq);
-    } else {
-        seq = p.b_seq_len[b];
+    const int seq = p.b_seq_len[b];
+    int total = groups_of(seq), longest = total, before = 0;
+    if (p.B > 1) {
+        total = 0;
         for (int i = lane; i < p.B; i += 32) {
             const int n = groups_of(p.b_seq_len[i]);
             total += n;
@@ -1267,7 +1268,6 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
         before = __reduce_add_sync(0xFFFFFFFFu, before);
         longest = __reduce_max_sync(0xFFFFFFFFu, longest);
     }
-    int tail = p.b_tail_len ? p.b_tail_len[b] : 0;
     tail = max(0, min(tail, min(p.max_tail, S2_MAX_TAIL)));
     const int D = p.D;                                                   // == HD
     // workspace slots stage 1 wrote for this sequence
@@ -1284,19 +1284,22 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     }
     const float *base = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh;
 
-    constexpr int PRE_T = 5, PRE_S = 10;                                 // rows / splits per warp held in registers
+    constexpr int PRE_T = NW == 16 ? 5 : 6, PRE_S = NW == 16 ? 10 : 5;   // rows / splits per warp held in registers
     // ---- bf16 residual rows: logits of this q head (independent of stage 1) ----
     // The K rows of this warp (rows warp, warp+16, ...) are requested together, before the query is in shared memory:
     // this part runs after stage 1 whenever stage 1 fills every SM, so each round trip saved is a round trip per layer.
     if (tail > 0) {
         const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh;
         uint2 kpre[PRE_T];
+        auto load_k = [&](int r0) __attribute__((always_inline)) {
 #pragma unroll
-        for (int k = 0; k < PRE_T; ++k) {
-            const int r = warp + k * S2_WARPS;
-            kpre[k] = make_uint2(0u, 0u);
-            if (r < tail) kpre[k] = *reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 4 * lane);
-        }
+            for (int k = 0; k < PRE_T; ++k) {
+                const int r = r0 + k * NW;
+                kpre[k] = make_uint2(0u, 0u);
+                if (r < tail) kpre[k] = *reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 4 * lane);
+            }
+        };
+        load_k(warp);
         if (tid < D) s_q[tid] = __bfloat162float(p.q[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid]);
         __syncthreads();
         const float q0 = s_q[4 * lane], q1 = s_q[4 * lane + 1], q2 = s_q[4 * lane + 2], q3 = s_q[4 * lane + 3];
@@ -1309,17 +1312,17 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
             if (p.logit_cap > 0.f) x = p.logit_cap * tanhf(x / p.logit_cap);
             return x;
         };
+#pragma unroll 1
+        for (int r0 = warp; r0 < tail; r0 += PRE_T * NW) {
+            if (r0 != warp) load_k(r0);
 #pragma unroll
-        for (int k = 0; k < PRE_T; ++k) {
-            const int r = warp + k * S2_WARPS;
-            if (r < tail) {                                              // warp-uniform
-                const float x = logit_of(kpre[k]);
-                if (lane == 0) s_logit[r] = x;
+            for (int k = 0; k < PRE_T; ++k) {
+                const int r = r0 + k * NW;
+                if (r < tail) {                                          // warp-uniform
+                    const float x = logit_of(kpre[k]);
+                    if (lane == 0) s_logit[r] = x;
+                }
             }
-        }
-        for (int r = warp + PRE_T * S2_WARPS; r < tail; r += S2_WARPS) {
-            const float x = logit_of(*reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 4 * lane));
-            if (lane == 0) s_logit[r] = x;
         }
     }
     // residual V rows of this warp (rows warp, warp+16, ...), requested before the wait below: they do not depend on stage 1
@@ -1327,7 +1330,7 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     uint32_t vpre[PRE_T][4];                                             // raw bf16 bits: turned into floats where they are used
 #pragma unroll
     for (int k = 0; k < PRE_T; ++k) {
-        const int r = warp + k * S2_WARPS;
+        const int r = warp + k * NW;
         vpre[k][0] = vpre[k][1] = vpre[k][2] = vpre[k][3] = 0u;
         if (r < tail) {
             const uint16_t *row = reinterpret_cast<const uint16_t *>(vt + (int64_t)r * p.t_st);
@@ -1345,7 +1348,7 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     float spre[PRE_S][4], lpre[PRE_S];
 #pragma unroll
     for (int k = 0; k < PRE_S; ++k) {
-        const int s = warp + k * S2_WARPS;
+        const int s = warp + k * NW;
         spre[k][0] = spre[k][1] = spre[k][2] = spre[k][3] = 0.f;
         lpre[k] = -INFINITY;
         if (s < nsplit) {
@@ -1358,8 +1361,8 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     float m_w = -INFINITY;
 #pragma unroll
     for (int k = 0; k < PRE_S; ++k) m_w = fmaxf(m_w, lpre[k]);
-    for (int s = warp + PRE_S * S2_WARPS; s < nsplit; s += S2_WARPS) m_w = fmaxf(m_w, base[(int64_t)s * p.al_ss + D]);
-    for (int r = warp; r < tail; r += S2_WARPS) m_w = fmaxf(m_w, s_logit[r]);
+    for (int s = warp + PRE_S * NW; s < nsplit; s += NW) m_w = fmaxf(m_w, base[(int64_t)s * p.al_ss + D]);
+    for (int r = warp; r < tail; r += NW) m_w = fmaxf(m_w, s_logit[r]);
     const float m_safe = (m_w == -INFINITY) ? 0.f : m_w;
     // weighted sum: lane owns channels lane + 32*i
     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, den_w = 0.f;
@@ -1370,7 +1373,7 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
         a0 += w * spre[k][0]; a1 += w * spre[k][1]; a2 += w * spre[k][2]; a3 += w * spre[k][3];
     }
 #pragma unroll 4
-    for (int s = warp + PRE_S * S2_WARPS; s < nsplit; s += S2_WARPS) {
+    for (int s = warp + PRE_S * NW; s < nsplit; s += NW) {
         const float *row = base + (int64_t)s * p.al_ss;
         const float w = __expf(row[D] - m_safe);
         den_w += w;
@@ -1379,7 +1382,7 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     if (tail > 0) {
 #pragma unroll
         for (int k = 0; k < PRE_T; ++k) {
-            const int r = warp + k * S2_WARPS;
+            const int r = warp + k * NW;
             if (r < tail) {
                 const float w = __expf(s_logit[r] - m_safe);
                 den_w += w;
@@ -1388,7 +1391,7 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
             }
         }
 #pragma unroll 4
-        for (int r = warp + PRE_T * S2_WARPS; r < tail; r += S2_WARPS) {
+        for (int r = warp + PRE_T * NW; r < tail; r += NW) {
             const __nv_bfloat16 *row = vt + (int64_t)r * p.t_st;
             const float w = __expf(s_logit[r] - m_safe);
             den_w += w;
@@ -1405,11 +1408,11 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
     if (tid < D) {
         float g_max = s_red[0];
 #pragma unroll
-        for (int w = 1; w < S2_WARPS; ++w) g_max = fmaxf(g_max, s_red[w]);
+        for (int w = 1; w < NW; ++w) g_max = fmaxf(g_max, s_red[w]);
         const float g_safe = (g_max == -INFINITY) ? 0.f : g_max;
         float acc = 0.f, den = 0.f;
 #pragma unroll
-        for (int w = 0; w < S2_WARPS; ++w) {
+        for (int w = 0; w < NW; ++w) {
             const float e = __expf(s_red[w] - g_safe);                   // 0 for a warp that saw nothing
             acc = fmaf(s_acc[w][tid], e, acc);
             den = fmaf(s_w[w], e, den);
@@ -1440,13 +1443,13 @@ __global__ void __launch_bounds__(S2_THREADS) decode_stage2_kernel(const S2Param
         const long long t_end = clock64() + WAIT_LIMIT_CYCLES;
         const int n_words = (p.g_world - 1) * D;
         // two words per thread and round, both requested before either is looked at
-        for (int idx = tid; idx < n_words; idx += 2 * S2_THREADS) {
+        for (int idx = tid; idx < n_words; idx += 2 * (NW * 32)) {
             const uint64_t *src[2];
             float *dst[2];
             bool pending[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const int i = idx + u * S2_THREADS;
+                const int i = idx + u * (NW * 32);
                 pending[u] = i < n_words;
                 int r = pending[u] ? i / D : 0;
                 const int e = pending[u] ? i - r * D : 0;
@@ -1849,6 +1852,7 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool after_
             return fail(OMMX_E_ARG, "head gather: world must be 2..32, rank inside it, and recv / out / state set");
         p.g_world = g->world; p.g_rank = g->rank; p.g_recv = g->recv; p.g_out = g->out; p.g_state = g->state;
     }
+    int warps;
     {
         // Stage 1 runs with the largest shared-memory carve-out; asking for the same split here spares the SMs a
         // reconfiguration between the two kernels of every layer.
@@ -1856,13 +1860,18 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool after_
         int dev = 0;
         if (int rc = current_device(&dev)) return rc;
         if (carve_set[dev].load(std::memory_order_acquire) == 0) {
-            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel<16>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel<8>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel<4>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
             carve_set[dev].store(1, std::memory_order_release);
         }
+        // the largest CTAs of which all rows still run at once; past three rows per SM the small ones win even in several rounds
+        const long long rows = (long long)a->n_q_heads * a->batch;
+        warps = rows <= sm_count_of(dev) ? 16 : (rows <= 3 * sm_count_of(dev) ? 8 : 4);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a->n_q_heads, a->batch);
-    cfg.blockDim = dim3(S2_THREADS);
+    cfg.blockDim = dim3(32 * warps);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1870,7 +1879,8 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool after_
     attr[0].val.programmaticStreamSerializationAllowed = 1;   // overlap this kernel's prologue with stage 1's tail
     cfg.attrs = attr;
     cfg.numAttrs = (after_stage1 && a->max_seq_len > 0) ? 1 : 0;
-    OMMX_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_stage2_kernel, p));
+    OMMX_CUDA_TRY(warps == 16 ? cudaLaunchKernelEx(&cfg, decode_stage2_kernel<16>, p)
+                              : (warps == 8 ? cudaLaunchKernelEx(&cfg, decode_stage2_kernel<8>, p) : cudaLaunchKernelEx(&cfg, decode_stage2_kernel<4>, p)));
     count_launch();
     return 0;
 }
