@@ -266,6 +266,13 @@ int ommx_b200_kv_append_decode(const ommx_kv_append_args *args, void *stream);
 int ommx_b200_kv_gather_tail(const ommx_kv_pool *pool, const void *sel, const void *tail_idx,
                              int32_t index_is_int64, int32_t batch, int32_t rows,
                              void *k_tail, void *v_tail, int32_t *status, void *stream);
+/*
+ * The same, and the two table rows of every selected sequence (r2t_out [batch, pages_per_seq], r2g_out [batch, groups_per_seq],
+ * optional, together): what MultiSeqKVPool.decode_inputs_captured hands to the decode call, in one launch.
+ */
+int ommx_b200_kv_gather_inputs(const ommx_kv_pool *pool, const void *sel, const void *tail_idx,
+                               int32_t index_is_int64, int32_t batch, int32_t rows, void *k_tail, void *v_tail,
+                               int32_t *r2t_out, int32_t *r2g_out, int32_t *status, void *stream);
 
 /*
  * Split count this library prefers for (max context, batch, local kv heads) on the current

@@ -92,6 +92,8 @@ SYMBOLS = {
     "ommx_b200_kv_append_decode": (C.c_int, [C.POINTER(KVAppendArgs), C.c_void_p]),
     "ommx_b200_kv_gather_tail": (C.c_int, [C.POINTER(KVPool), C.c_void_p, C.c_void_p, C.c_int32, C.c_int32,
                                            C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "ommx_b200_kv_gather_inputs": (C.c_int, [C.POINTER(KVPool), C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
+                                             C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ommx_b200_peer_alloc": (C.c_int, [C.c_size_t, C.POINTER(C.c_void_p), C.c_void_p]),
     "ommx_b200_peer_open": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "ommx_b200_peer_close": (C.c_int, [C.c_void_p]),

@@ -359,15 +359,16 @@ class MultiSeqKVPool:
                 "k_format": self.k_format, "k_base_bits": self.k_base_bits, "oval_bits": self.oval_bits,
                 "kv_outlier_map": bool(self.kv_outlier_map), "kv_int8_scale": True}
 
-    def _gather_tail(self, sel, tidx, kt, vt) -> None:
+    def _gather_tail(self, sel, tidx, kt, vt, with_tables=False):
         B, T = int(tidx.shape[0]), int(tidx.shape[1])
         if tidx.dtype not in (torch.int32, torch.int64) or (sel is not None and sel.dtype != tidx.dtype):
             raise ValueError("sel / tail index tensors must both be int32 or both int64")
         if tuple(kt.shape) != (B, T, self.H, self.D) or not kt.is_contiguous() or not vt.is_contiguous() or tuple(vt.shape) != tuple(kt.shape):
             raise ValueError(f"k_tail / v_tail must be contiguous [{B}, {T}, {self.H}, {self.D}]")
-        rc = _lib.host().kv_gather_tail(self, sel, tidx, kt, vt)
-        if rc:
-            _lib.check(rc, "ommx_b200_kv_gather_tail")
+        got = _lib.host().kv_gather_tail(self, sel, tidx, kt, vt, with_tables)
+        if isinstance(got, int):
+            _lib.check(got, "ommx_b200_kv_gather_tail")
+        return got
 
     def tail_bf16_batched(self, slots: Sequence[int]):
         """``(k_tail [B,T,H,D], v_tail, b_tail_len [B])`` of the listed requests: sink and recent rows, zero
@@ -422,10 +423,8 @@ class MultiSeqKVPool:
         """Argument bundle from caller-owned fixed-address control tensors: ``sel`` ``[B]`` batch row -> pool
         slot, packed and residual lengths, ``tidx_dev`` ``[B, T]`` absolute residual token positions, and the
         residual output buffers ``kt`` / ``vt``, which one gather launch fills (reference :886-936)."""
-        self._gather_tail(sel, tidx_dev, kt, vt)
-        sel_l = sel.to(torch.long)
-        return self._bundle(self._req_to_token.index_select(0, sel_l), self._req_to_group.index_select(0, sel_l),
-                            kt, vt, b_tail_len, b_seq_len, max_seq_len)
+        r2t, r2g = self._gather_tail(sel, tidx_dev, kt, vt, with_tables=True)
+        return self._bundle(r2t, r2g, kt, vt, b_tail_len, b_seq_len, max_seq_len)
 
     def decode_inputs_batched(self, slots: Sequence[int]) -> dict:
         """Argument bundle for the listed requests at their current lengths (reference :938-1011): lengths and

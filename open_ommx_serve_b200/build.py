@@ -12,16 +12,17 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libommx_b200.so")
 SOURCES = ("ommx_capi.cu", "ommx_pack.cu", "ommx_decode.cu")
 HEADERS = ("ommx_common.cuh", "ommx_decode_tc.cuh", "ommx_tables.inc", os.path.join("..", "..", "include", "ommx_b200.h"))
+OBJ = os.path.join(PKG, "build")
 HOST_LIB = os.path.join(PKG, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "ommx_host.cpp")
-NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-shared", "-Xcompiler", "-fPIC")
+NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC")
 
 
 def _nvcc() -> str:
@@ -61,16 +62,24 @@ def build_host(force: bool = False) -> str:
     return HOST_LIB
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the CUDA sources into ``libommx_b200.so`` next to this file and ``_host.so`` beside it; returns the
-    library's path."""
-    if force or needs_build():
-        cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB, *[os.path.join(CSRC, s) for s in SOURCES]]
-        if verbose:
-            cmd[1:1] = ["-Xptxas", "-v"]
-        log = _run(cmd)
+def _compile(source: str, force: bool, verbose: bool):
+    """Object file of one CUDA source, rebuilt when it or a header is newer."""
+    src, obj = os.path.join(CSRC, source), os.path.join(OBJ, source + ".o")
+    if force or _older(obj, [src] + [os.path.join(CSRC, f) for f in HEADERS]):
+        log = _run([_nvcc(), *NVCC_FLAGS, *(("-Xptxas", "-v") if verbose else ()), "-c", "-o", obj, src])
         if verbose:
             sys.stderr.write(log)
+    return obj
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compile the CUDA sources (side by side) into ``libommx_b200.so`` next to this file and ``_host.so`` beside it;
+    returns the library's path."""
+    if force or needs_build():
+        os.makedirs(OBJ, exist_ok=True)
+        with ThreadPoolExecutor(len(SOURCES)) as pool:
+            objs = list(pool.map(lambda f: _compile(f, force, verbose), SOURCES))
+        _run([_nvcc(), *NVCC_FLAGS, "-shared", "-o", LIB, *objs])
     build_host(force)
     return LIB
 

@@ -505,24 +505,34 @@ PyObject *py_kv_append(PyObject *, PyObject *const *a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// kv_gather_tail(pool, sel, tail_idx, k_tail, v_tail): tensors the caller has checked
+// kv_gather_tail(pool, sel, tail_idx, k_tail, v_tail, with_tables): tensors the caller has checked.  Returns the C ABI's code, or
+// with_tables the two table rows of every selected sequence ([B, pages], [B, groups])
 PyObject *py_kv_gather_tail(PyObject *, PyObject *const *a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 5) { PyErr_SetString(PyExc_TypeError, "kv_gather_tail: wrong argument count"); return nullptr; }
+    if (n != 6) { PyErr_SetString(PyExc_TypeError, "kv_gather_tail: wrong argument count"); return nullptr; }
     ommx_kv_pool p;
     memset(&p, 0, sizeof(p));
     at::Device dev(at::kCUDA);
     if (!read_pool(a[0], &p, &dev)) return nullptr;
     PoolReader r{a[0]};
     const Tensor *sel = as_tensor(a[1]), *idx = as_tensor(a[2]), *kt = as_tensor(a[3]), *vt = as_tensor(a[4]);
-    if (!idx || !kt || !vt) { PyErr_SetString(PyExc_TypeError, "kv_gather_tail: tensors expected"); return nullptr; }
+    bool tables;
+    if (!idx || !kt || !vt || !as_bool(a[5], &tables)) { PyErr_SetString(PyExc_TypeError, "kv_gather_tail: tensors expected"); return nullptr; }
     const Tensor sel_c = sel ? sel->contiguous() : Tensor(), idx_c = idx->contiguous();
     int32_t *status = (int32_t *)ptr(r.tensor(N.status));
     if (!r.ok) return nullptr;
-    return PyLong_FromLong(launch(dev, [&](void *stream) {
-        return ommx_b200_kv_gather_tail(&p, ptr(sel_c), idx_c.data_ptr(), idx_c.scalar_type() == at::kLong, (int32_t)idx_c.size(0), (int32_t)idx_c.size(1),
-                                        kt->data_ptr(), vt->data_ptr(), status, stream);
-    }));
+    Tensor r2t, r2g;
+    if (tables) {
+        const c10::cuda::CUDAGuard guard(dev);
+        r2t = at::empty({idx_c.size(0), p.pages_per_seq}, kt->options().dtype(at::kInt));
+        r2g = at::empty({idx_c.size(0), p.groups_per_seq}, kt->options().dtype(at::kInt));
+    }
+    const int rc = launch(dev, [&](void *stream) {
+        return ommx_b200_kv_gather_inputs(&p, ptr(sel_c), idx_c.data_ptr(), idx_c.scalar_type() == at::kLong, (int32_t)idx_c.size(0), (int32_t)idx_c.size(1),
+                                          kt->data_ptr(), vt->data_ptr(), (int32_t *)ptr(r2t), (int32_t *)ptr(r2g), status, stream);
+    });
+    if (!tables || rc != 0) return PyLong_FromLong(rc);
+    return Py_BuildValue("(NN)", THPVariable_Wrap(r2t), THPVariable_Wrap(r2g));
     END_HANDLE_TH_ERRORS
 }
 

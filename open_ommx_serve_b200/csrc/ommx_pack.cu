@@ -636,6 +636,392 @@ __global__ void __launch_bounds__(128) pack_v_kernel(PackVParams p) {
     else reinterpret_cast<uint16_t *>(p.v_zp)[soff] = (uint16_t)f32_to_bf16_bits(zp);
 }
 
+// ---------------------------------------------------------------------------------------------
+// 16-bit inputs, signed rule, 64 channels at a time: the form every serving recipe takes.
+//
+// K: one warp per (32-token group, kv head, 64 channels), lane = two adjacent channels in the halves of a register, so that
+// selection runs on both at once: 16-bit values need no order keys, min and max of packed halves sort them directly.  The
+// KT + 1 largest and KB + 1 smallest values come from a sorting network (blocks of four sorted, then merged: 248
+// min/max per pair of channels, where insertion of 32-bit keys took 900), the picks are what is not below (above) the
+// KT-th (KB-th) value, and where equal values leave too many, the highest tokens go - the stable-sort rule.  The values behind the
+// picks are the base range.  Codes are two FMAs and one shifted add per value: (x - zp) / 4s saturated to [0, 1] in one FMA (one
+// rounding, the same as the subtraction's, because s is a power of two), times 4 onto 1.5 * 2^23, which rounds to nearest even.
+// Bound by the ALU pipe (min / max, compare and logic run at half the FMA rate).  Measured, K + V: 8192 tokens x 8 heads (42 MB)
+// 34.8 -> 17.2 us, 2.5 TB/s; 32768 tokens 122 -> 61 us; 1024 tokens 9.3 -> 5.5 us.
+// The scale, map and FP4 steps are those of pack_k_kernel, operation for operation.
+// ---------------------------------------------------------------------------------------------
+template <typename T> struct Pair16;
+template <> struct Pair16<__nv_bfloat16> {
+    typedef __nv_bfloat162 V;
+    static constexpr uint32_t EXP = 0x7F80u;                       // all ones here: infinity or NaN
+    static __device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
+    static __device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+};
+template <> struct Pair16<__half> {
+    typedef __half2 V;
+    static constexpr uint32_t EXP = 0x7C00u;
+    static __device__ __forceinline__ float lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)w)); }
+    static __device__ __forceinline__ float hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+};
+template <typename V> __device__ __forceinline__ V as_pair(uint32_t w) { return *reinterpret_cast<const V *>(&w); }
+template <typename V> __device__ __forceinline__ uint32_t pair_bits(V v) { return *reinterpret_cast<const uint32_t *>(&v); }
+// a >= b afterwards, NaN goes everywhere
+template <typename V> __device__ __forceinline__ void order2(V &a, V &b) {
+    const V hi = __hmax2_nan(a, b);
+    b = __hmin2_nan(a, b);
+    a = hi;
+}
+// one 16-bit value of half c of a pair of words
+__device__ __forceinline__ bool half_is_special(uint32_t w, uint32_t exp) {
+    return (w & exp) == exp || ((w >> 16) & exp) == exp;
+}
+
+// The rows of a group: consecutive, or in a residual ring (row `wrap` on follow behind row 0 of the ring again)
+struct GroupRows {
+    int64_t stride;                    // elements from a row to the next
+    int wrap, back;                    // rows t >= wrap lie `back` rows earlier
+    __device__ __forceinline__ int64_t at(int t) const { return (int64_t)(t < wrap ? t : t - back) * stride; }
+};
+
+// FP4 E2M1 code by three comparisons
+__device__ __forceinline__ uint32_t fp4_code(float m) {
+    const uint32_t a = __float_as_uint(m) & 0x7FFFFFFFu;
+    const bool c2 = a >= c_fp4_thresh[3];
+    const bool c1 = a >= (c2 ? c_fp4_thresh[5] : c_fp4_thresh[1]);
+    const bool c0 = a >= (c2 ? (c1 ? c_fp4_thresh[6] : c_fp4_thresh[4]) : (c1 ? c_fp4_thresh[2] : c_fp4_thresh[0]));
+    return (m < 0.f ? 8u : 0u) | (c2 ? 4u : 0u) | (c1 ? 2u : 0u) | (c0 ? 1u : 0u);
+}
+
+// Drops the highest tokens of `eq` from `picks` until `keep` picks are left
+__device__ __forceinline__ uint32_t drop_ties(uint32_t picks, uint32_t eq, int keep) {
+    for (int over = __popc(picks) - keep; over > 0; --over) {
+        const uint32_t bit = 0x80000000u >> __clz(eq);
+        picks ^= bit;
+        eq ^= bit;
+    }
+    return picks;
+}
+
+// col: this lane's channels 2 lane, 2 lane + 1 in row 0; the unit's destination group slot, page of every token and head
+template <typename T, int KT, int KB>
+__device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, const GroupRows &rows, int slot, int h, int blk, int page, int lane) {
+    typedef Pair16<T> P;
+    typedef typename P::V V;
+    constexpr int K = KT + KB;
+    constexpr int NB = (K + 1) / 2;
+    static_assert(K <= 8, "the nibble stream is kept in 32 bits");
+    uint32_t w[32];
+#pragma unroll
+    for (int t = 0; t < 32; ++t) w[t] = *reinterpret_cast<const uint32_t *>(col + rows.at(t));
+
+    // ---- the M largest, descending, and the M smallest, ascending ----
+    constexpr int M = KT >= KB ? KT + 1 : KB + 1;
+    V top[M <= 4 ? 4 : M], bot[M <= 4 ? 4 : M];
+    if constexpr (M == 1) {
+        top[0] = bot[0] = as_pair<V>(w[0]);
+#pragma unroll
+        for (int t = 1; t < 32; ++t) { top[0] = __hmax2_nan(top[0], as_pair<V>(w[t])); bot[0] = __hmin2_nan(bot[0], as_pair<V>(w[t])); }
+    } else if constexpr (M <= 4) {
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            V s0 = as_pair<V>(w[4 * b]), s1 = as_pair<V>(w[4 * b + 1]), s2 = as_pair<V>(w[4 * b + 2]), s3 = as_pair<V>(w[4 * b + 3]);
+            order2(s0, s1); order2(s2, s3); order2(s0, s2); order2(s1, s3); order2(s1, s2);
+            if (b == 0) {
+                top[0] = s0; top[1] = s1; top[2] = s2; top[3] = s3;
+                bot[0] = s3; bot[1] = s2; bot[2] = s1; bot[3] = s0;
+            } else {
+                // the larger (smaller) halves of two sorted fours are bitonic: two rounds sort them
+                top[0] = __hmax2_nan(top[0], s3); top[1] = __hmax2_nan(top[1], s2); top[2] = __hmax2_nan(top[2], s1); top[3] = __hmax2_nan(top[3], s0);
+                order2(top[0], top[2]); order2(top[1], top[3]); order2(top[0], top[1]); order2(top[2], top[3]);
+                bot[0] = __hmin2_nan(bot[0], s0); bot[1] = __hmin2_nan(bot[1], s1); bot[2] = __hmin2_nan(bot[2], s2); bot[3] = __hmin2_nan(bot[3], s3);
+                order2(bot[2], bot[0]); order2(bot[3], bot[1]); order2(bot[1], bot[0]); order2(bot[3], bot[2]);
+            }
+        }
+    } else {
+        // five of each: insertion, from infinities that every value pushes out
+#pragma unroll
+        for (int i = 0; i < M; ++i) { top[i] = as_pair<V>(P::EXP | (P::EXP << 16) | 0x80008000u); bot[i] = as_pair<V>(P::EXP | (P::EXP << 16)); }
+#pragma unroll
+        for (int t = 0; t < 32; ++t) {
+            V c = as_pair<V>(w[t]), d = c;
+#pragma unroll
+            for (int i = 0; i < M; ++i) { order2(top[i], c); order2(d, bot[i]); }
+        }
+    }
+    bool bad = half_is_special(pair_bits(top[0]), P::EXP) || half_is_special(pair_bits(bot[0]), P::EXP);
+
+    // ---- which tokens are picked ----
+    uint32_t omask[2] = {0u, 0u};
+    if constexpr (K > 0) {
+        uint32_t t0 = 0, t1 = 0, b0 = 0, b1 = 0;                      // halves: the two channels, tokens 0..15 and 16..31
+        const V thr_t = top[KT > 0 ? KT - 1 : 0], thr_b = bot[KB > 0 ? KB - 1 : 0];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const uint32_t bit = 0x00010001u << t;
+            t0 |= __hge2_mask(as_pair<V>(w[t]), thr_t) & bit;
+            t1 |= __hge2_mask(as_pair<V>(w[t + 16]), thr_t) & bit;
+            b0 |= __hle2_mask(as_pair<V>(w[t]), thr_b) & bit;
+            b1 |= __hle2_mask(as_pair<V>(w[t + 16]), thr_b) & bit;
+        }
+        uint32_t tm[2] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632)};
+        uint32_t bm[2] = {__byte_perm(b0, b1, 0x5410), __byte_perm(b0, b1, 0x7632)};
+        const bool ties = __popc(tm[0]) != KT || __popc(tm[1]) != KT || __popc(bm[0] & ~tm[0]) != KB || __popc(bm[1] & ~tm[1]) != KB;
+        if (__any_sync(0xFFFFFFFFu, ties && !bad)) {
+            // more tokens at a threshold than picks left: the lowest of them are taken, the bottom picks among what the
+            // top picks left
+            uint32_t e0 = 0, e1 = 0, f0 = 0, f1 = 0;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const uint32_t bit = 0x00010001u << t;
+                e0 |= __heq2_mask(as_pair<V>(w[t]), thr_t) & bit;
+                e1 |= __heq2_mask(as_pair<V>(w[t + 16]), thr_t) & bit;
+                f0 |= __heq2_mask(as_pair<V>(w[t]), thr_b) & bit;
+                f1 |= __heq2_mask(as_pair<V>(w[t + 16]), thr_b) & bit;
+            }
+            if (!bad) {
+                tm[0] = drop_ties(tm[0], __byte_perm(e0, e1, 0x5410), KT);
+                tm[1] = drop_ties(tm[1], __byte_perm(e0, e1, 0x7632), KT);
+                bm[0] &= ~tm[0];
+                bm[1] &= ~tm[1];
+                bm[0] = drop_ties(bm[0], __byte_perm(f0, f1, 0x5410) & bm[0], KB);
+                bm[1] = drop_ties(bm[1], __byte_perm(f0, f1, 0x7632) & bm[1], KB);
+            }
+        }
+        omask[0] = tm[0] | bm[0];
+        omask[1] = tm[1] | bm[1];
+        if (bad) {                                                    // refused input: any K tokens
+            omask[0] = omask[1] = (1u << K) - 1u;
+        }
+    }
+
+    // ---- base range, scale, zero-point; codes ----
+    const bool store_f32 = p.scale_kind == OMMX_SCALE_F32;
+    int e[2];
+    float scale[2], zp[2];
+    uint32_t cw[4] = {0u, 0u, 0u, 0u};                                 // nibble i of word j: token 8j + i, both channels' codes
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const uint32_t kx = pair_bits(top[KT]), kn = pair_bits(bot[KB]);
+        const float mx = (c ? P::hi(kx) : P::lo(kx)) + 0.f, mn = (c ? P::hi(kn) : P::lo(kn)) + 0.f;
+        scale[c] = snap_scale(__fsub_rn(mx, mn), p.use_pow2, p.scale_kind, e[c]);
+        zp[c] = store_f32 ? mn : bf16_round_f32(mn);
+        const float inv4 = __uint_as_float((uint32_t)(125 - e[c]) << 23);        // 1 / 4s
+        const float off = -zp[c] * inv4;
+        const bool by_fma = p.use_pow2 && e[c] >= -120 && e[c] <= 120 && fabsf(off) < 1e38f;
+        uint32_t acc[4];
+        if (__all_sync(0xFFFFFFFFu, by_fma)) {
+            constexpr uint32_t MAGIC = 0x4B400000u;                    // 1.5 * 2^23: its share of the sums leaves at the end
+            constexpr uint32_t MAGIC_SUM = MAGIC * 0x11111111u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[j] = 0u - MAGIC_SUM;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t x = w[8 * j + i];
+                    const float y = __saturatef(__fmaf_rn(c ? P::hi(x) : P::lo(x), inv4, off));
+                    acc[j] += __float_as_uint(__fmaf_rn(y, 4.f, 12582912.f)) * (1u << (4 * i));
+                }
+                acc[j] -= (acc[j] >> 2) & 0x11111111u;                 // 4 (saturated) is code 3
+            }
+        } else {
+            const bool by_mul = p.use_pow2 && e[c] >= -126 && e[c] <= 126;
+            const float inv = __uint_as_float((uint32_t)(by_mul ? 127 - e[c] : 127) << 23);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[j] = 0u;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t x = w[8 * j + i];
+                    const float d = __fsub_rn(c ? P::hi(x) : P::lo(x), zp[c]);
+                    acc[j] += code_0_3(by_mul ? __fmul_rn(d, inv) : __fdiv_rn(d, scale[c])) << (4 * i);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) cw[j] |= acc[j] << (2 * c);
+    }
+
+    // ---- outlier values, read back in token order ----
+    float ms[2] = {0.f, 0.f}, mc[2] = {0.f, 0.f};
+    uint32_t val[2] = {0u, 0u};
+    if constexpr (K > 0) {
+        uint16_t raw[2][K];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            uint32_t m = omask[c];
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const int t = __ffs(m) - 1;
+                m &= m - 1u;
+                raw[c][r] = *reinterpret_cast<const uint16_t *>(col + c + rows.at(t));
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (p.outlier_map) {
+                const uint32_t hx = pair_bits(KT > 0 ? top[0] : bot[KB > 0 ? KB - 1 : 0]), hn = pair_bits(KB > 0 ? bot[0] : top[KT > 0 ? KT - 1 : 0]);
+                const float omx = (c ? P::hi(hx) : P::lo(hx)) + 0.f, omn = (c ? P::hi(hn) : P::lo(hn)) + 0.f;
+                mc[c] = __fmul_rn(__fadd_rn(omx, omn), 0.5f);
+                // the reference evaluates 12.0 / range as reciprocal(range) * 12
+                ms[c] = __fmul_rn(__frcp_rn(fmaxf(__fsub_rn(omx, omn), 1e-8f)), 12.0f);
+                if (!store_f32) { mc[c] = bf16_round_f32(mc[c]); ms[c] = bf16_round_f32(ms[c]); }
+            }
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const float x = P::lo(raw[c][r]) + 0.f;
+                const float m = p.outlier_map ? __fmul_rn(__fsub_rn(x, mc[c]), ms[c]) : __fdiv_rn(__fsub_rn(x, zp[c]), scale[c]);
+                val[c] |= fp4_code(m) << (4 * r);
+            }
+        }
+    }
+
+    // ---- per-channel planes: two adjacent entries a lane ----
+    if (slot >= 0) {
+        const int64_t off = ((int64_t)slot * p.H + h) * p.D + 64 * blk + 2 * lane;
+        auto put16 = [&](void *plane, float a, float b) {
+            if (store_f32) *reinterpret_cast<float2 *>(reinterpret_cast<float *>(plane) + off) = make_float2(a, b);
+            else *reinterpret_cast<uint32_t *>(reinterpret_cast<uint16_t *>(plane) + off) = f32_to_bf16_bits(a) | (f32_to_bf16_bits(b) << 16);
+        };
+        if (p.scale_kind == OMMX_SCALE_INT8_EXP) *reinterpret_cast<uint16_t *>(reinterpret_cast<int8_t *>(p.k_scale) + off) = (uint16_t)((e[0] & 0xFF) | (e[1] << 8));
+        else put16(p.k_scale, scale[0], scale[1]);
+        put16(p.k_zp, zp[0], zp[1]);
+        if constexpr (K > 0) {
+            if (p.outlier_map) { put16(p.k_mapscale, ms[0], ms[1]); put16(p.k_mapcenter, mc[0], mc[1]); }
+            *reinterpret_cast<uint2 *>(p.k_obmp + 4 * off) = make_uint2(omask[0], omask[1]);
+            uint8_t *ov = p.k_oval + off * NB;
+            if constexpr (NB == 4) {
+                *reinterpret_cast<uint2 *>(ov) = make_uint2(val[0], val[1]);
+            } else if constexpr (NB == 3) {
+                reinterpret_cast<uint16_t *>(ov)[0] = (uint16_t)val[0];
+                reinterpret_cast<uint16_t *>(ov)[1] = (uint16_t)((val[0] >> 16) | (val[1] << 8));
+                reinterpret_cast<uint16_t *>(ov)[2] = (uint16_t)(val[1] >> 8);
+            } else if constexpr (NB == 2) {
+                *reinterpret_cast<uint32_t *>(ov) = val[0] | (val[1] << 16);
+            } else {
+                *reinterpret_cast<uint16_t *>(ov) = (uint16_t)(val[0] | (val[1] << 8));
+            }
+        }
+    }
+    if (bad) or_status(p.status, OMMX_ST_NONFINITE);
+
+    // ---- codes: (channel pair, 32 tokens) nibbles -> (token, 32 channel pairs): a 32 x 32 transpose, one lane bit a round ----
+    {
+        const bool up = lane & 16;
+        const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, up ? cw[0] : cw[2], 16), g1 = __shfl_xor_sync(0xFFFFFFFFu, up ? cw[1] : cw[3], 16);
+        if (up) { cw[0] = g0; cw[1] = g1; } else { cw[2] = g0; cw[3] = g1; }
+    }
+    {
+        const bool up = lane & 8;
+        const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, up ? cw[0] : cw[1], 8), g1 = __shfl_xor_sync(0xFFFFFFFFu, up ? cw[2] : cw[3], 8);
+        if (up) { cw[0] = g0; cw[2] = g1; } else { cw[1] = g0; cw[3] = g1; }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; v += 2) {
+        // the half of two words that the partner needs goes over in one exchange
+        uint32_t &a = cw[v], &b = cw[v + 1];
+        const bool up4 = lane & 4, up2 = lane & 2, up1 = lane & 1;
+        uint32_t g = __shfl_xor_sync(0xFFFFFFFFu, __byte_perm(a, b, up4 ? 0x5410u : 0x7632u), 4);
+        a = __byte_perm(a, g, up4 ? 0x3254u : 0x5410u);
+        b = __byte_perm(b, g, up4 ? 0x3276u : 0x7610u);
+        g = __shfl_xor_sync(0xFFFFFFFFu, __byte_perm(a, b, up2 ? 0x6420u : 0x7531u), 2);
+        a = __byte_perm(a, g, up2 ? 0x3514u : 0x5240u);
+        b = __byte_perm(b, g, up2 ? 0x3716u : 0x7260u);
+        g = __shfl_xor_sync(0xFFFFFFFFu, up1 ? ((a & 0x0F0F0F0Fu) | ((b << 4) & 0xF0F0F0F0u)) : (((a >> 4) & 0x0F0F0F0Fu) | (b & 0xF0F0F0F0u)), 1);
+        a = up1 ? ((a & 0xF0F0F0F0u) | (g & 0x0F0F0F0Fu)) : ((a & 0x0F0F0F0Fu) | ((g << 4) & 0xF0F0F0F0u));
+        b = up1 ? ((b & 0xF0F0F0F0u) | ((g >> 4) & 0x0F0F0F0Fu)) : ((b & 0x0F0F0F0Fu) | (g & 0xF0F0F0F0u));
+    }
+    // lane = token now: its 16 code bytes of these 64 channels
+    if (page >= 0)
+        *reinterpret_cast<uint4 *>(p.k_base + (((int64_t)page * p.page_size + lane % p.page_size) * p.H + h) * (p.D / 4) + 16 * blk) =
+            make_uint4(cw[0], cw[1], cw[2], cw[3]);
+}
+
+// V: one thread per (token, kv head, 32 channels), 64 contiguous bytes at `row`; loc = destination (page row * H + head), negative:
+// not written
+template <typename T>
+__device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row, int64_t loc, int cg) {
+    typedef Pair16<T> P;
+    typedef typename P::V V;
+    uint32_t w[16];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const uint4 q = reinterpret_cast<const uint4 *>(row)[v];
+        w[4 * v] = q.x; w[4 * v + 1] = q.y; w[4 * v + 2] = q.z; w[4 * v + 3] = q.w;
+    }
+    V hi2 = as_pair<V>(w[0]), lo2 = hi2;
+#pragma unroll
+    for (int i = 1; i < 16; ++i) { hi2 = __hmax2_nan(hi2, as_pair<V>(w[i])); lo2 = __hmin2_nan(lo2, as_pair<V>(w[i])); }
+    const uint32_t hb = pair_bits(hi2), lb = pair_bits(lo2);
+    const bool bad = half_is_special(hb, P::EXP) || half_is_special(lb, P::EXP);
+    const float mx = fmaxf(P::lo(hb), P::hi(hb)), mn = fminf(P::lo(lb), P::hi(lb)) + 0.f;
+    int e;
+    const float scale = snap_scale(__fsub_rn(mx, mn), p.use_pow2, p.scale_kind, e);
+    const bool store_f32 = p.scale_kind == OMMX_SCALE_F32;
+    const float zp = store_f32 ? mn : bf16_round_f32(mn);
+    const float inv4 = __uint_as_float((uint32_t)(125 - e) << 23), off = -zp * inv4;        // see pack_k_pair
+    uint32_t code[2] = {0u, 0u};
+    if (p.use_pow2 && e >= -120 && e <= 120 && fabsf(off) < 1e38f) {
+        constexpr uint32_t MAGIC_SUM = 0x4B400000u * 0x55555555u;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const float x = i & 1 ? P::hi(w[i >> 1]) : P::lo(w[i >> 1]);
+            const float y = fminf(__saturatef(__fmaf_rn(x, inv4, off)), 0.75f);
+            code[i >> 4] += __float_as_uint(__fmaf_rn(y, 4.f, 12582912.f)) * (1u << (2 * (i & 15)));
+        }
+        code[0] -= MAGIC_SUM;
+        code[1] -= MAGIC_SUM;
+    } else {
+        const bool by_mul = p.use_pow2 && e >= -126 && e <= 126;
+        const float inv = __uint_as_float((uint32_t)(by_mul ? 127 - e : 127) << 23);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const float d = __fsub_rn(i & 1 ? P::hi(w[i >> 1]) : P::lo(w[i >> 1]), zp);
+            code[i >> 4] |= code_0_3(by_mul ? __fmul_rn(d, inv) : __fdiv_rn(d, scale)) << (2 * (i & 15));
+        }
+    }
+    if (bad) or_status(p.status, OMMX_ST_NONFINITE);
+    if (loc < 0) return;
+    *reinterpret_cast<uint2 *>(p.v_main + loc * (p.D / 4) + cg * 8) = make_uint2(code[0], code[1]);
+    const int64_t at = loc * (p.D / 32) + cg;
+    if (p.scale_kind == OMMX_SCALE_INT8_EXP) reinterpret_cast<int8_t *>(p.v_scale)[at] = (int8_t)e;
+    else if (p.scale_kind == OMMX_SCALE_BF16) reinterpret_cast<uint16_t *>(p.v_scale)[at] = (uint16_t)f32_to_bf16_bits(scale);
+    else reinterpret_cast<float *>(p.v_scale)[at] = scale;
+    if (store_f32) reinterpret_cast<float *>(p.v_zp)[at] = zp;
+    else reinterpret_cast<uint16_t *>(p.v_zp)[at] = (uint16_t)f32_to_bf16_bits(zp);
+}
+
+// K and V of a block in one launch: the first `k_blocks` CTAs take K (the longer work), the rest V and fill the last wave.
+template <typename T, int KT, int KB>
+__global__ void __launch_bounds__(PACK_WARPS * 32, 7) pack16_kernel(const PackKParams kp, const PackVParams vp, int k_blocks) {
+    const int lane = threadIdx.x & 31;
+    if ((int)blockIdx.x < k_blocks) {
+        const int nblk = kp.D / 64;
+        const int unit = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5);        // (group, head, 64-channel half)
+        if (unit >= kp.num_groups * kp.H * nblk) return;
+        const int blk = unit % nblk, gh = unit / nblk, g = gh / kp.H, h = gh - g * kp.H;
+        int slot = kp.dst_groups ? kp.dst_groups[g] : g;
+        const int tok = g * 32 + lane;
+        int page = tok / kp.page_size;
+        if (kp.dst_pages) page = kp.dst_pages[page];
+        if (slot < 0 || slot >= kp.num_group_slots) { if (lane == 0) or_status(kp.status, OMMX_ST_BAD_GROUP); slot = -1; }
+        if (page < 0 || page >= kp.num_pages) { or_status(kp.status, OMMX_ST_BAD_PAGE); page = -1; }
+        const T *col = reinterpret_cast<const T *>(kp.k) + (int64_t)(g * 32) * kp.stride_token + (int64_t)h * kp.stride_head + blk * 64 + 2 * lane;
+        pack_k_pair<T, KT, KB>(kp, col, GroupRows{kp.stride_token, 32, 0}, slot, h, blk, page, lane);
+    } else {
+        const int ngv = vp.D / 32;
+        const int64_t idx = (int64_t)(blockIdx.x - k_blocks) * blockDim.x + threadIdx.x;
+        if (idx >= (int64_t)vp.num_tokens * vp.H * ngv) return;
+        const int cg = (int)(idx % ngv);
+        const int64_t th = idx / ngv;
+        const int t = (int)(th / vp.H), h = (int)(th - (int64_t)t * vp.H);
+        int page = t / vp.page_size;
+        if (vp.dst_pages) page = vp.dst_pages[page];
+        int64_t loc = ((int64_t)page * vp.page_size + t % vp.page_size) * vp.H + h;
+        if (page < 0 || page >= vp.num_pages) { or_status(vp.status, OMMX_ST_BAD_PAGE); loc = -1; }
+        pack_v_group<T>(vp, reinterpret_cast<const T *>(vp.v) + (int64_t)t * vp.stride_token + (int64_t)h * vp.stride_head + cg * 32, loc, cg);
+    }
+}
+
 template <typename T>
 static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
     const ommx_kv_planes &pl = a->planes;
@@ -650,6 +1036,35 @@ static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
     kp.k_base = (uint8_t *)pl.k_base; kp.k_scale = pl.k_scale; kp.k_zp = pl.k_zp;
     kp.k_mapscale = pl.k_mapscale; kp.k_mapcenter = pl.k_mapcenter;
     kp.k_obmp = (uint8_t *)pl.k_obmp; kp.k_oval = (uint8_t *)pl.k_oval; kp.status = a->status;
+    PackVParams vp;
+    memset(&vp.pool, 0, sizeof(vp.pool));
+    vp.v = a->v; vp.stride_token = a->stride_token; vp.stride_head = a->stride_head;
+    vp.num_tokens = a->num_tokens; vp.H = pl.n_kv_heads; vp.D = pl.head_dim; vp.page_size = pl.page_size;
+    vp.dst_pages = a->dst_pages; vp.num_pages = pl.num_pages; vp.use_pow2 = a->use_pow2; vp.scale_kind = pl.scale_kind;
+    vp.v_main = (uint8_t *)pl.v_main; vp.v_scale = pl.v_scale; vp.v_zp = pl.v_zp; vp.status = a->status;
+    const int64_t nthreads = (int64_t)a->num_tokens * pl.n_kv_heads * (pl.head_dim / 32);
+    if constexpr (sizeof(T) == 2) {
+        // The serving form: channel pairs need whole 64-channel units and rows whose 16-byte pieces are aligned
+        const uintptr_t all = (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)pl.k_base | (uintptr_t)pl.k_scale | (uintptr_t)pl.k_zp | (uintptr_t)pl.k_obmp |
+                              (uintptr_t)pl.k_oval | (uintptr_t)pl.k_mapscale | (uintptr_t)pl.k_mapcenter;
+        const int k = kp.k_out;
+        if (kp.select_signed && kp.D % 64 == 0 && all % 16 == 0 && a->stride_token % 8 == 0 && a->stride_head % 8 == 0 &&
+            (k == 0 || k == 2 || k == 4 || k == 6 || k == 8)) {
+            if (nthreads == 0) return 0;
+            const int k_blocks = (kp.num_groups * kp.H * (kp.D / 64) + PACK_WARPS - 1) / PACK_WARPS;
+            const unsigned grid = (unsigned)(k_blocks + (nthreads + 127) / 128);
+            switch (k) {
+                case 0: pack16_kernel<T, 0, 0><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
+                case 2: pack16_kernel<T, 1, 1><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
+                case 4: pack16_kernel<T, 2, 2><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
+                case 6: pack16_kernel<T, 3, 3><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
+                default: pack16_kernel<T, 4, 4><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
+            }
+            OMMX_CUDA_TRY(cudaGetLastError());
+            count_launch();
+            return 0;
+        }
+    }
     const int units = kp.num_groups * kp.H * (kp.D / PACK_BLK);
     // the lane-per-channel kernel serves the signed rule with the usual outlier counts; everything else
     // (absolute selection, odd or large k) goes through the warp-reduction kernel
@@ -669,13 +1084,6 @@ static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
         OMMX_CUDA_TRY(cudaGetLastError());
         count_launch();
     }
-    PackVParams vp;
-    memset(&vp.pool, 0, sizeof(vp.pool));
-    vp.v = a->v; vp.stride_token = a->stride_token; vp.stride_head = a->stride_head;
-    vp.num_tokens = a->num_tokens; vp.H = pl.n_kv_heads; vp.D = pl.head_dim; vp.page_size = pl.page_size;
-    vp.dst_pages = a->dst_pages; vp.num_pages = pl.num_pages; vp.use_pow2 = a->use_pow2; vp.scale_kind = pl.scale_kind;
-    vp.v_main = (uint8_t *)pl.v_main; vp.v_scale = pl.v_scale; vp.v_zp = pl.v_zp; vp.status = a->status;
-    const int64_t nthreads = (int64_t)a->num_tokens * pl.n_kv_heads * (pl.head_dim / 32);
     if (nthreads > 0) {
         pack_v_kernel<T><<<(unsigned)((nthreads + 127) / 128), 128, 0, st>>>(vp);
         OMMX_CUDA_TRY(cudaGetLastError());
@@ -776,26 +1184,177 @@ struct GatherParams {
     const void *sel, *idx;
     int32_t idx64, T, HD, ring_cap, sink, num_seqs;
     __nv_bfloat16 *k_tail, *v_tail;
+    const int32_t *r2t, *r2g;          // table rows of the selected sequences, copied when r2t_out / r2g_out are given
+    int32_t *r2t_out, *r2g_out;
+    int32_t pages_per_seq, groups_per_seq;
     int32_t *status;
 };
-__global__ void __launch_bounds__(128) kv_gather_tail_kernel(GatherParams p) {
+constexpr int GATHER_ROWS = 4;         // rows a block has in flight
+__global__ void __launch_bounds__(256) kv_gather_tail_kernel(GatherParams p) {
     const int i = blockIdx.x;
     const int r = p.sel ? pool_index(p.sel, p.idx64, i) : i;
     const bool slot_ok = r >= 0 && r < p.num_seqs;
-    for (int row = blockIdx.y; row < p.T; row += gridDim.y) {
-        const int pos = pool_index(p.idx, p.idx64, i * p.T + row);
-        const bool ok = slot_ok && pos >= 0;
-        if (!ok && threadIdx.x == 0) or_status(p.status, slot_ok ? OMMX_ST_BAD_LENGTH : OMMX_ST_BAD_GROUP);
-        const int rr = pos < p.sink ? pos : p.sink + (pos - p.sink) % (p.ring_cap - p.sink);
-        const uint4 *ks = reinterpret_cast<const uint4 *>(p.k_hist + ((int64_t)(ok ? r : 0) * p.ring_cap + (ok ? rr : 0)) * p.HD);
-        const uint4 *vs = reinterpret_cast<const uint4 *>(p.v_hist + ((int64_t)(ok ? r : 0) * p.ring_cap + (ok ? rr : 0)) * p.HD);
-        uint4 *kd = reinterpret_cast<uint4 *>(p.k_tail + ((int64_t)i * p.T + row) * p.HD);
-        uint4 *vd = reinterpret_cast<uint4 *>(p.v_tail + ((int64_t)i * p.T + row) * p.HD);
-        for (int x = threadIdx.x; x < p.HD / 8; x += blockDim.x) {
-            kd[x] = ok ? ks[x] : make_uint4(0, 0, 0, 0);
-            vd[x] = ok ? vs[x] : make_uint4(0, 0, 0, 0);
+    if (!slot_ok && blockIdx.y == 0 && threadIdx.x == 0) or_status(p.status, OMMX_ST_BAD_GROUP);
+    const int vecs = p.HD / 8;                                         // 16-byte pieces of a row
+    for (int row0 = blockIdx.y * GATHER_ROWS; row0 < p.T; row0 += gridDim.y * GATHER_ROWS) {
+        for (int x = threadIdx.x; x < 2 * vecs; x += blockDim.x) {
+            const bool is_v = x >= vecs;
+            const int piece = is_v ? x - vecs : x;
+            const uint4 *src = reinterpret_cast<const uint4 *>(is_v ? p.v_hist : p.k_hist);
+            uint4 *dst = reinterpret_cast<uint4 *>(is_v ? p.v_tail : p.k_tail);
+            uint4 w[GATHER_ROWS];
+#pragma unroll
+            for (int u = 0; u < GATHER_ROWS; ++u) {
+                w[u] = make_uint4(0, 0, 0, 0);
+                if (row0 + u >= p.T) continue;
+                const int pos = pool_index(p.idx, p.idx64, i * p.T + row0 + u);
+                if (slot_ok && pos >= 0) {
+                    const int rr = pos < p.sink ? pos : p.sink + (pos - p.sink) % (p.ring_cap - p.sink);
+                    w[u] = src[((int64_t)r * p.ring_cap + rr) * vecs + piece];
+                } else if (slot_ok && x == 0) {
+                    or_status(p.status, OMMX_ST_BAD_LENGTH);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < GATHER_ROWS; ++u)
+                if (row0 + u < p.T) dst[((int64_t)i * p.T + row0 + u) * vecs + piece] = w[u];
         }
     }
+    if (p.r2t_out) {
+        const int n = p.pages_per_seq + p.groups_per_seq;
+        for (int x = blockIdx.y * blockDim.x + threadIdx.x; x < n; x += gridDim.y * blockDim.x) {
+            if (x < p.pages_per_seq) p.r2t_out[(int64_t)i * p.pages_per_seq + x] = slot_ok ? p.r2t[(int64_t)r * p.pages_per_seq + x] : 0;
+            else p.r2g_out[(int64_t)i * p.groups_per_seq + x - p.pages_per_seq] = slot_ok ? p.r2g[(int64_t)r * p.groups_per_seq + x - p.pages_per_seq] : 0;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The whole decode-step store in one launch: one cluster of STORE_CTAS CTAs per batch row.  Five kernels in a row were five
+// launches and five drains for a few hundred KB (17 us of the GPU a step at batch 1); nothing in the step needs them in turn:
+//   * the group that a step completes ends `recent` rows before the new row, so packing does not read it, and the row that
+//     the new one overwrites in the ring left the group's 32 rows long ago (the ring holds recent + 32 at least);
+//   * the residual rows that are handed to the decode call come from the ring, except the new one, which comes from its source;
+//   * the length is advanced once every CTA of the row's cluster has read it (a cluster barrier).
+// Bound by latency: one chain slot -> length -> rows.  Needs recent >= 1, whole 64-channel units and 16-byte pieces;
+// launch_append keeps the separate kernels for anything else.
+// ---------------------------------------------------------------------------------------------
+constexpr int STORE_CTAS = 8, STORE_THREADS = 256;
+template <int KT, int KB>
+__global__ void __cluster_dims__(STORE_CTAS, 1, 1) __launch_bounds__(STORE_THREADS, 2) kv_store_kernel(const StoreParams p, const PackKParams kp, const PackVParams vp) {
+    typedef __nv_bfloat16 T;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int i = blockIdx.y, rank = blockIdx.x;
+    const int r = pool_slot(p.pool, i);
+    if (r < 0 || r >= p.num_seqs) {                                    // the same in every CTA of the cluster
+        if (p.advance && rank == 0 && threadIdx.x == 0) or_status(p.status, OMMX_ST_BAD_GROUP);
+        return;
+    }
+    const int pos = pool_pos(p.pool, i, r);
+    const bool step = p.advance && pos >= 0 && !pool_row_refused(p.pool, r, pos + 1);
+    if (p.advance && !step && rank == 0 && threadIdx.x == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
+    if (p.advance == 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this CTA has read the length
+    const int HD = p.H * p.D, vecs = HD / 8;
+    const int64_t ring = (int64_t)r * p.pool.ring_cap;                 // first ring row of the sequence
+    // 16-byte piece x of the new row
+    auto new_piece = [&](const T *src, int x) {
+        const int h = 8 * x / p.D, c = 8 * x - h * p.D;
+        return *reinterpret_cast<const uint4 *>(src + (int64_t)i * p.new_sb + (int64_t)h * p.new_sh + c);
+    };
+    if (step && rank == 0) {
+        const int64_t dst = (ring + ring_row(p.pool, pos)) * HD;
+        for (int x = threadIdx.x; x < 2 * vecs; x += STORE_THREADS) {
+            const int piece = x < vecs ? x : x - vecs;
+            reinterpret_cast<uint4 *>((x < vecs ? p.k_hist : p.v_hist) + dst)[piece] = new_piece(x < vecs ? p.k_new : p.v_new, piece);
+        }
+    }
+    // ---- residual rows and lengths for the decode call ----
+    const int seq = pos + (step ? 1 : 0);
+    const int sink = p.pool.sink, spare = seq - sink - p.pool.recent;
+    const int boundary = spare > 0 ? sink + spare / 32 * 32 : min(sink, seq);
+    const int n_sink = min(sink, seq), n_rec = max(seq - boundary, 0);
+    const int n_tail = min(n_sink + n_rec, p.max_tail);
+    if (rank == 0 && threadIdx.x == 0) {
+        // a residual buffer too small for sink + recent + a partial group would silently drop the newest rows
+        if (n_sink + n_rec > p.max_tail && (p.k_tail || p.b_tail_len)) or_status(p.status, OMMX_ST_BAD_LENGTH);
+        if (p.b_seq_len) p.b_seq_len[i] = max(boundary - sink, 0);
+        if (p.b_tail_len) p.b_tail_len[i] = n_tail;
+    }
+    if (p.k_tail) {
+        constexpr int U = 3;                                           // rows in flight
+        for (int row0 = rank; row0 < n_tail; row0 += U * STORE_CTAS) {
+            for (int x = threadIdx.x; x < 2 * vecs; x += STORE_THREADS) {
+                const bool is_v = x >= vecs;
+                const int piece = is_v ? x - vecs : x;
+                const T *hist = is_v ? p.v_hist : p.k_hist;
+                uint4 w[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int row = row0 + u * STORE_CTAS;
+                    if (row >= n_tail) continue;
+                    const int at = row < n_sink ? row : boundary + (row - n_sink);
+                    w[u] = step && at == pos ? new_piece(is_v ? p.v_new : p.k_new, piece)
+                                             : reinterpret_cast<const uint4 *>(hist + (ring + ring_row(p.pool, at)) * HD)[piece];
+                }
+                uint4 *dst = reinterpret_cast<uint4 *>(is_v ? p.v_tail : p.k_tail) + (int64_t)i * p.max_tail * vecs + piece;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int row = row0 + u * STORE_CTAS;
+                    if (row < n_tail) dst[(int64_t)row * vecs] = w[u];
+                }
+            }
+        }
+    }
+    // ---- the group this step completed, if any: K by the first four warps of each CTA, V by the others ----
+    const int grp = pool_groups_at(p.pool, pos);
+    if (step && pool_groups_at(p.pool, pos + 1) != grp) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int rec = p.pool.ring_cap - sink, first = (grp * 32) % rec;     // ring row (behind the sink rows) of token 0
+        const GroupRows rows{HD, rec - first, rec};
+        const int64_t base = (ring + sink + first) * HD;
+        const int32_t *pages = p.pool.r2t + (int64_t)r * p.pool.pages_per_seq;
+        if (warp < STORE_THREADS / 64) {
+            const int nblk = p.D / 64;
+            int slot = p.pool.r2g[(int64_t)r * p.pool.groups_per_seq + grp];
+            int page = pages[(grp * 32 + lane) / kp.page_size];
+            if (slot < 0 || slot >= kp.num_group_slots) { if (lane == 0) or_status(p.status, OMMX_ST_BAD_GROUP); slot = -1; }
+            if (page < 0 || page >= kp.num_pages) { or_status(p.status, OMMX_ST_BAD_PAGE); page = -1; }
+            for (int unit = rank + STORE_CTAS * warp; unit < p.H * nblk; unit += STORE_CTAS * (STORE_THREADS / 64)) {
+                const int h = unit / nblk, blk = unit - h * nblk;
+                pack_k_pair<T, KT, KB>(kp, p.k_hist + base + h * p.D + 64 * blk + 2 * lane, rows, slot, h, blk, page, lane);
+            }
+        } else {
+            const int ngv = p.D / 32;
+            for (int x = rank * (STORE_THREADS / 2) + (int)threadIdx.x - STORE_THREADS / 2; x < 32 * p.H * ngv; x += STORE_CTAS * (STORE_THREADS / 2)) {
+                const int cg = x % ngv, th = x / ngv, h = th % p.H, t = th / p.H;
+                const int page = pages[(grp * 32 + t) / vp.page_size];
+                int64_t loc = ((int64_t)page * vp.page_size + t % vp.page_size) * p.H + h;
+                if (page < 0 || page >= vp.num_pages) { or_status(p.status, OMMX_ST_BAD_PAGE); loc = -1; }
+                pack_v_group<T>(vp, p.v_hist + base + rows.at(t) + h * p.D + cg * 32, loc, cg);
+            }
+        }
+    }
+    if (p.advance == 1) {
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        if (step && rank == 0 && threadIdx.x == 0) p.seq_len[r] = pos + 1;
+    }
+}
+
+template <int KT, int KB>
+static int launch_store(const StoreParams &sp, const PackKParams &kp, const PackVParams &vp, int B, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(STORE_CTAS, B);
+    cfg.blockDim = dim3(STORE_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // placed while the kernel before it drains, waits for it before any access
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    OMMX_CUDA_TRY(cudaLaunchKernelEx(&cfg, kv_store_kernel<KT, KB>, sp, kp, vp));
+    count_launch();
+    return 0;
 }
 
 static int launch_append(const ommx_kv_append_args *a, cudaStream_t st) {
@@ -810,25 +1369,44 @@ static int launch_append(const ommx_kv_append_args *a, cudaStream_t st) {
     sp.k_hist = (__nv_bfloat16 *)pool.k_hist; sp.v_hist = (__nv_bfloat16 *)pool.v_hist;
     sp.k_new = (const __nv_bfloat16 *)a->k_new; sp.v_new = (const __nv_bfloat16 *)a->v_new;
     sp.new_sb = a->new_stride_b; sp.new_sh = a->new_stride_h;
-    sp.H = pl.n_kv_heads; sp.D = pl.head_dim; sp.num_seqs = pool.num_seqs; sp.advance = a->advance ? 1 : 0;
+    sp.H = pl.n_kv_heads; sp.D = pl.head_dim; sp.num_seqs = pool.num_seqs; sp.advance = a->advance;
     sp.k_tail = (__nv_bfloat16 *)a->k_tail; sp.v_tail = (__nv_bfloat16 *)a->v_tail; sp.max_tail = a->max_tail;
     sp.b_seq_len = a->b_seq_len; sp.b_tail_len = a->b_tail_len; sp.seq_len = pool.seq_len; sp.status = a->status;
     const int B = a->batch;
+    PackKParams kp;
+    kp.pool = sp.pool;
+    kp.k = pool.k_hist; kp.stride_token = (int64_t)sp.H * sp.D; kp.stride_head = sp.D;
+    kp.num_groups = B; kp.H = sp.H; kp.D = sp.D; kp.page_size = pl.page_size;
+    kp.dst_pages = nullptr; kp.dst_groups = nullptr;
+    kp.num_pages = pl.num_pages; kp.num_group_slots = pl.num_group_slots;
+    kp.k_out = pl.outliers_per_vector; kp.select_signed = 1; kp.use_pow2 = a->use_pow2;
+    kp.outlier_map = pl.kv_outlier_map; kp.scale_kind = pl.scale_kind;
+    kp.k_base = (uint8_t *)pl.k_base; kp.k_scale = pl.k_scale; kp.k_zp = pl.k_zp;
+    kp.k_mapscale = pl.k_mapscale; kp.k_mapcenter = pl.k_mapcenter;
+    kp.k_obmp = (uint8_t *)pl.k_obmp; kp.k_oval = (uint8_t *)pl.k_oval; kp.status = a->status;
+    PackVParams vp;
+    vp.pool = sp.pool;
+    vp.v = pool.v_hist; vp.stride_token = kp.stride_token; vp.stride_head = sp.D;
+    vp.num_tokens = B * 32; vp.H = sp.H; vp.D = sp.D; vp.page_size = pl.page_size;
+    vp.dst_pages = nullptr; vp.num_pages = pl.num_pages; vp.use_pow2 = a->use_pow2; vp.scale_kind = pl.scale_kind;
+    vp.v_main = (uint8_t *)pl.v_main; vp.v_scale = pl.v_scale; vp.v_zp = pl.v_zp; vp.status = a->status;
+    const uintptr_t all = (uintptr_t)pool.k_hist | (uintptr_t)pool.v_hist | (uintptr_t)a->k_tail | (uintptr_t)a->v_tail | (uintptr_t)a->k_new | (uintptr_t)a->v_new |
+                          (uintptr_t)pl.k_base | (uintptr_t)pl.k_scale | (uintptr_t)pl.k_zp | (uintptr_t)pl.k_obmp | (uintptr_t)pl.k_oval |
+                          (uintptr_t)pl.k_mapscale | (uintptr_t)pl.k_mapcenter;
+    if (sp.D % 64 == 0 && pool.recent_window >= 1 && all % 16 == 0 && B <= 65535 &&
+        (!a->advance || (a->new_stride_b % 8 == 0 && a->new_stride_h % 8 == 0))) {
+        switch (kp.k_out) {
+            case 0: return launch_store<0, 0>(sp, kp, vp, B, st);
+            case 2: return launch_store<1, 1>(sp, kp, vp, B, st);
+            case 4: return launch_store<2, 2>(sp, kp, vp, B, st);
+            case 6: return launch_store<3, 3>(sp, kp, vp, B, st);
+            default: return launch_store<4, 4>(sp, kp, vp, B, st);
+        }
+    }
     if (a->advance) {
         kv_ring_write_kernel<<<B, 128, 0, st>>>(sp);
         OMMX_CUDA_TRY(cudaGetLastError());
         count_launch();
-        PackKParams kp;
-        kp.pool = sp.pool;
-        kp.k = pool.k_hist; kp.stride_token = (int64_t)sp.H * sp.D; kp.stride_head = sp.D;
-        kp.num_groups = B; kp.H = sp.H; kp.D = sp.D; kp.page_size = pl.page_size;
-        kp.dst_pages = nullptr; kp.dst_groups = nullptr;
-        kp.num_pages = pl.num_pages; kp.num_group_slots = pl.num_group_slots;
-        kp.k_out = pl.outliers_per_vector; kp.select_signed = 1; kp.use_pow2 = a->use_pow2;
-        kp.outlier_map = pl.kv_outlier_map; kp.scale_kind = pl.scale_kind;
-        kp.k_base = (uint8_t *)pl.k_base; kp.k_scale = pl.k_scale; kp.k_zp = pl.k_zp;
-        kp.k_mapscale = pl.k_mapscale; kp.k_mapcenter = pl.k_mapcenter;
-        kp.k_obmp = (uint8_t *)pl.k_obmp; kp.k_oval = (uint8_t *)pl.k_oval; kp.status = a->status;
         const int lane_units = B * kp.H * (kp.D / 32);
         const unsigned lane_grid = (unsigned)((lane_units + PACK_WARPS - 1) / PACK_WARPS);
         typedef __nv_bfloat16 T;
@@ -841,12 +1419,6 @@ static int launch_append(const ommx_kv_append_args *a, cudaStream_t st) {
         }
         OMMX_CUDA_TRY(cudaGetLastError());
         count_launch();
-        PackVParams vp;
-        vp.pool = sp.pool;
-        vp.v = pool.v_hist; vp.stride_token = kp.stride_token; vp.stride_head = sp.D;
-        vp.num_tokens = B * 32; vp.H = sp.H; vp.D = sp.D; vp.page_size = pl.page_size;
-        vp.dst_pages = nullptr; vp.num_pages = pl.num_pages; vp.use_pow2 = a->use_pow2; vp.scale_kind = pl.scale_kind;
-        vp.v_main = (uint8_t *)pl.v_main; vp.v_scale = pl.v_scale; vp.v_zp = pl.v_zp; vp.status = a->status;
         const int64_t nthreads = (int64_t)vp.num_tokens * vp.H * (vp.D / 32);
         pack_v_kernel<T><<<(unsigned)((nthreads + 127) / 128), 128, 0, st>>>(vp);
         OMMX_CUDA_TRY(cudaGetLastError());
@@ -1005,9 +1577,9 @@ extern "C" int ommx_b200_kv_append_decode(const ommx_kv_append_args *a, void *st
     return launch_append(a, (cudaStream_t)stream);
 }
 
-extern "C" int ommx_b200_kv_gather_tail(const ommx_kv_pool *pool, const void *sel, const void *tail_idx,
-                                        int32_t index_is_int64, int32_t batch, int32_t rows,
-                                        void *k_tail, void *v_tail, int32_t *status, void *stream) {
+extern "C" int ommx_b200_kv_gather_inputs(const ommx_kv_pool *pool, const void *sel, const void *tail_idx,
+                                          int32_t index_is_int64, int32_t batch, int32_t rows, void *k_tail, void *v_tail,
+                                          int32_t *r2t_out, int32_t *r2g_out, int32_t *status, void *stream) {
     using namespace ommx;
     if (!pool || !tail_idx || !k_tail || !v_tail) return fail(OMMX_E_ARG, "kv_gather_tail: null pointer");
     if (!pool->k_hist || !pool->v_hist) return fail(OMMX_E_ARG, "kv_gather_tail: the pool has no residual ring");
@@ -1017,13 +1589,25 @@ extern "C" int ommx_b200_kv_gather_tail(const ommx_kv_pool *pool, const void *se
         ((uintptr_t)pool->k_hist & 15) || ((uintptr_t)pool->v_hist & 15))
         return fail(OMMX_E_ARG, "kv_gather_tail: rows must be whole 16-byte pieces on 16-byte aligned buffers");
     if (pool->ring_cap - pool->sink_tokens <= 0) return fail(OMMX_E_ARG, "kv_gather_tail: ring_cap=%d sink=%d", pool->ring_cap, pool->sink_tokens);
+    if ((r2t_out != nullptr) != (r2g_out != nullptr)) return fail(OMMX_E_ARG, "kv_gather_inputs: the two table outputs go together");
+    if (r2t_out && (!pool->req_to_token || !pool->req_to_group || pool->pages_per_seq < 0 || pool->groups_per_seq < 0))
+        return fail(OMMX_E_ARG, "kv_gather_inputs: the pool has no tables");
     GatherParams g;
     g.k_hist = (const __nv_bfloat16 *)pool->k_hist; g.v_hist = (const __nv_bfloat16 *)pool->v_hist;
     g.sel = sel; g.idx = tail_idx; g.idx64 = index_is_int64 ? 1 : 0; g.T = rows; g.HD = HD;
     g.ring_cap = pool->ring_cap; g.sink = pool->sink_tokens; g.num_seqs = pool->num_seqs;
     g.k_tail = (__nv_bfloat16 *)k_tail; g.v_tail = (__nv_bfloat16 *)v_tail; g.status = status;
-    kv_gather_tail_kernel<<<dim3(batch, rows < 8 ? rows : 8), 128, 0, (cudaStream_t)stream>>>(g);
+    g.r2t = pool->req_to_token; g.r2g = pool->req_to_group; g.r2t_out = r2t_out; g.r2g_out = r2g_out;
+    g.pages_per_seq = pool->pages_per_seq; g.groups_per_seq = pool->groups_per_seq;
+    const int blocks = (rows + GATHER_ROWS - 1) / GATHER_ROWS;
+    kv_gather_tail_kernel<<<dim3(batch, blocks < 32 ? blocks : 32), 256, 0, (cudaStream_t)stream>>>(g);
     OMMX_CUDA_TRY(cudaGetLastError());
     count_launch();
     return 0;
+}
+
+extern "C" int ommx_b200_kv_gather_tail(const ommx_kv_pool *pool, const void *sel, const void *tail_idx,
+                                        int32_t index_is_int64, int32_t batch, int32_t rows,
+                                        void *k_tail, void *v_tail, int32_t *status, void *stream) {
+    return ommx_b200_kv_gather_inputs(pool, sel, tail_idx, index_is_int64, batch, rows, k_tail, v_tail, nullptr, nullptr, status, stream);
 }

@@ -147,3 +147,25 @@ def test_pack_refusals():
     with pytest.raises(NotImplementedError):
         pack(torch.cat([K, K]), torch.cat([V, V]), outliers_per_vector=6, outlier_repr="bitmap",
              group_tokens=64, device="cuda")
+
+
+@pytest.mark.parametrize("k", [0, 2, 4, 6, 8])
+@pytest.mark.parametrize("D,H", [(64, 1), (128, 3)])
+def test_pack_16_bit_inputs_with_ties(k, D, H):
+    """Channel pairs of 16-bit values: groups with few distinct values (equal values at both selection thresholds, top and
+    bottom picks competing for them), constant and zero groups, both signs of zero, half precision and bf16, every
+    scale recipe, scattered sizes."""
+    g = torch.Generator().manual_seed(900 + k)
+    K, V = gaussian_kv(90 + k, 192, H, D, mag=30.0)
+    levels = torch.tensor([-2.0, -0.5, 0.0, 0.5, 1.0, 4.0])
+    K[32:64] = levels[torch.randint(0, 6, (32, H, D), generator=g)]
+    K[64:96] = levels[torch.randint(2, 4, (32, H, D), generator=g)]
+    K[96:128] = torch.where(torch.rand(32, H, D, generator=g) < 0.5, torch.tensor(0.0), torch.tensor(3.0))
+    K[128:160] = torch.randn(1, H, D, generator=g).bfloat16().float()
+    V[32:64], V[64:96], V[96:100] = K[32:64], K[64:96], 0.0
+    for dtype in (torch.bfloat16, torch.float16):
+        Kd, Vd = K.to(dtype), V.to(dtype)
+        for pow2, omap in ((True, True), (True, False), (False, True)):
+            want = O.pack_kv(Kd.float().numpy(), Vd.float().numpy(), outliers_per_vector=k, use_pow2=pow2, kv_outlier_map=omap,
+                             kv_int8_scale=pow2)
+            assert_planes_equal(_gpu_pack(Kd, Vd, k=k, pow2=pow2, omap=omap), want, ctx=f"{dtype} pow2={pow2} map={omap}:")
