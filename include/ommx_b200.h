@@ -255,6 +255,15 @@ typedef struct ommx_kv_append_args {
 int ommx_b200_kv_append_decode(const ommx_kv_append_args *args, void *stream);
 
 /*
+ * Prefill of one sequence slot with bf16 K/V [num_tokens, n_kv_heads, head_dim] (last dim contiguous).  Replaces
+ * MultiSeqKVPool.append_block (attention/kv_pool.py:310-368): the completed groups are quantized straight into the
+ * slot's pages and group slots, the rows that stay bf16 go to the residual ring, and seq_len[slot] becomes num_tokens.
+ * Two launches, no host synchronisation.
+ */
+int ommx_b200_kv_append_block(const ommx_kv_pool *pool, int32_t slot, const void *k, const void *v, int64_t stride_token,
+                              int64_t stride_head, int32_t num_tokens, int32_t *status, void *stream);
+
+/*
  * Residual rows by absolute token position: k_tail/v_tail[i, y] = ring row of token tail_idx[i, y] of
  * sequence slot sel[i] (NULL: slot i).  Replaces _kv_gather_tail (attention/kv_store_ops.py:42-57) as
  * called by CanonicalKVStore.gather_tail_into (attention/kv_store.py:397-427) and

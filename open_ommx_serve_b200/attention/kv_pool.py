@@ -126,7 +126,9 @@ class MultiSeqKVPool:
         self._sel = None                     # batch row -> request slot (None: row i is slot i)
         self._sel_key = None
         self._r2t_sel = self._r2g_sel = None
-        self._planes_cache = None
+        self._planes_cache = self._bundle_base = None
+        self._views = {}                     # views of the step's outputs by batch size
+        self.max_packed_len = self.window.packed_len(self.max_seq_len)
         self._dbuf = None
 
     # plane tensors under the reference's attribute names
@@ -188,6 +190,9 @@ class MultiSeqKVPool:
 
     def _call(self, a: tuple) -> None:
         rc = _lib.host().kv_append(self, *a)
+        if rc is None:                        # other types, layouts or devices: convert, then again
+            B, advance, K, V, *rest = a
+            rc = _lib.host().kv_append(self, B, advance, *self._rows(K, V, B), *rest)
         if rc:
             _lib.check(rc, "ommx_b200_kv_append_decode")
 
@@ -201,12 +206,13 @@ class MultiSeqKVPool:
 
     def _host_step(self, slots) -> int:
         """Advance the host-side lengths of ``slots`` by one row each; groups that completed."""
-        total = 0
+        total, edge, seq_len, packed = 0, self.sink + self.recent, self.seq_len, self.packed_groups
         for r in slots:
-            self.seq_len[r] += 1
-            target = self.window.num_groups(self.seq_len[r])
-            total += max(0, target - self.packed_groups[r])
-            self.packed_groups[r] = max(self.packed_groups[r], target)
+            n = seq_len[r] = seq_len[r] + 1
+            target = (n - edge) // 32 if n > edge else 0          # WindowSpec.num_groups, in line
+            if target > packed[r]:
+                total += target - packed[r]
+                packed[r] = target
         return total
 
     # ── write path ───────────────────────────────────────────────────────────
@@ -217,31 +223,22 @@ class MultiSeqKVPool:
             raise IndexError(f"request slot {r} outside [0, {self.num_seqs})")
         if T > self.max_seq_len:
             raise RuntimeError(f"MultiSeqKVPool req {r} capacity {self.max_seq_len} exceeded")
-        Kb, Vb = K.to(self.device, torch.bfloat16), V.to(self.device, torch.bfloat16)
         target = self.window.num_groups(T)
-        if target > 0:
-            t0, t1 = self.sink, self.sink + target * self.gt
-            ommx_pack_kv_into(Kb[t0:t1], Vb[t0:t1], self.planes,
-                              dst_pages=self._req_to_token[r, :target * self.pages_per_group].contiguous(),
-                              dst_groups=self._req_to_group[r, :target].contiguous(),
-                              outliers_per_vector=self.k, kv_outlier_map=self.kv_outlier_map,
-                              status=self.status)
-        boundary = self.window.boundary(T)
-        lo = max(self.sink, boundary - self.gt)
-        parts = [torch.arange(0, min(self.sink, T), device=self.device)]
-        if lo < T:
-            parts.append(torch.arange(lo, T, device=self.device))
-        live = torch.cat(parts).to(torch.long)
-        rows = self._ring_slot_dev(live)
-        self.k_hist[r].index_copy_(0, rows, Kb.index_select(0, live))
-        self.v_hist[r].index_copy_(0, rows, Vb.index_select(0, live))
-        self.seq_dev[r] = T
+        host = _lib.host()
+        rc = host.kv_append_block(self, r, K, V)
+        if rc is None:
+            K, V = K.to(self.device, torch.bfloat16).reshape(T, self.H, self.D), V.to(self.device, torch.bfloat16).reshape(T, self.H, self.D)
+            if K.stride(-1) != 1 or V.stride() != K.stride():
+                K, V = K.contiguous(), V.contiguous()
+            rc = host.kv_append_block(self, r, K, V)
+        if rc is None or rc:
+            _lib.check(rc or -1, "ommx_b200_kv_append_block")
         self.seq_len[r], self.packed_groups[r] = T, target
         return target
 
     def append(self, req: int, k: torch.Tensor, v: torch.Tensor) -> int:
         """One decode step's K/V row ``[H, D]`` of request ``req``; returns groups packed (0 or 1)."""
-        return self.append_decode_batched([int(req)], k.reshape(1, self.H, self.D), v.reshape(1, self.H, self.D))
+        return self.append_decode_batched((int(req),), k, v)
 
     def append_decode_batched(self, slots: Sequence[int], K: torch.Tensor, V: torch.Tensor) -> int:
         """One new row ``[B, H, D]`` for each request of ``slots``; returns the groups packed this step."""
@@ -249,7 +246,7 @@ class MultiSeqKVPool:
         B = len(slots)
         if B == 0:
             return 0
-        if any(not 0 <= r < self.num_seqs for r in slots):
+        if min(slots) < 0 or max(slots) >= self.num_seqs:
             raise IndexError(f"request slots {slots} outside [0, {self.num_seqs})")
         identity = slots == list(range(B))
         prev = (self._sel, self._sel_key, self._r2t_sel, self._r2g_sel)
@@ -258,9 +255,8 @@ class MultiSeqKVPool:
         else:
             self.select_slots(slots)
         try:
-            Kb, Vb = self._rows(K, V, B)
+            self._call(self._append_args(B, 1, K, V))
             total = self._host_step(slots)
-            self._call(self._append_args(B, 1, Kb, Vb))
         finally:
             if identity:
                 self._sel, self._sel_key, self._r2t_sel, self._r2g_sel = prev
@@ -277,13 +273,10 @@ class MultiSeqKVPool:
             raise ValueError("K/V must be bf16 CUDA tensors [B, H, D]")
         if tuple(K.shape) != (int(B), self.H, self.D) or tuple(V.shape) != tuple(K.shape):
             raise ValueError(f"K/V must be [{B}, {self.H}, {self.D}]")
-        if K.stride(-1) != 1 or V.stride() != K.stride():
-            K, V = K.contiguous(), V.contiguous()
-        total = 0
-        if not torch.cuda.is_current_stream_capturing():
-            total = self._host_step(range(int(B)) if self._sel_key is None else self._sel_key)
         self._call(self._append_args(B, 1, K, V))
-        return total
+        if torch.cuda.is_current_stream_capturing():
+            return 0
+        return self._host_step(range(int(B)) if self._sel_key is None else self._sel_key)
 
     def append_decode_captured(self, rows: torch.Tensor, cols: torch.Tensor, K: torch.Tensor, V: torch.Tensor) -> None:
         """One new row per batch row at device-side indices: request slot ``rows[i]``, absolute
@@ -293,10 +286,9 @@ class MultiSeqKVPool:
         to the caller (``advance_seq_device``); unlike it, a 32-token group that ``cols[i]`` completes is
         quantized and packed by this call itself, so no host regroup pass has to follow."""
         B = int(rows.shape[0])
-        Kb, Vb = self._rows(K, V, B)
         if _CAPTURED_WRITE_CHECK and not torch.cuda.is_current_stream_capturing():
             self._check_captured_indices(rows, cols)
-        self._call(self._append_args(B, 2, Kb, Vb, slots=rows.contiguous(), write_pos=cols.contiguous(), outputs=False))
+        self._call(self._append_args(B, 2, K, V, slots=rows.contiguous(), write_pos=cols.contiguous(), outputs=False))
 
     def _check_captured_indices(self, rows: torch.Tensor, cols: torch.Tensor) -> None:
         """Refuse an out-of-range device-indexed write with the offending value named (reference :526-550)."""
@@ -409,14 +401,21 @@ class MultiSeqKVPool:
         """The reference's argument bundle (:925-936), with the plane entries repeated at the top level."""
         planes = dict(self.pool_planes())
         planes["req_to_token"], planes["req_to_group"] = r2t, r2g
-        out = {"planes": planes, "k_tail": kt, "v_tail": vt, "b_tail_len": b_tail, "b_seq_len": b_seq,
-               "req_to_token": r2t, "req_to_group": r2g, "packed_start_offset": 0,
-               "max_seq_len": int(max_seq_len), "max_tail_len": self.max_tail_len}
-        for name in ("k_base", "k_scale", "k_zp", "k_oidx", "k_oval", "k_obmp", "k_fp4_mapscale", "k_fp4_mapcenter",
-                     "v_main", "v_scale", "v_zp", "page_size", "kv_outlier_map"):
-            out[name] = planes[name]
-        out["k_outliers_per_vector"] = self.k
-        return out
+        if self._bundle_base is None:
+            self._bundle_base = {name: planes[name] for name in (
+                "k_base", "k_scale", "k_zp", "k_oidx", "k_oval", "k_obmp", "k_fp4_mapscale", "k_fp4_mapcenter", "v_main", "v_scale",
+                "v_zp", "page_size", "kv_outlier_map")}
+            self._bundle_base.update(k_outliers_per_vector=self.k, packed_start_offset=0, max_tail_len=self.max_tail_len)
+        return {"planes": planes, "k_tail": kt, "v_tail": vt, "b_tail_len": b_tail, "b_seq_len": b_seq, "req_to_token": r2t,
+                "req_to_group": r2g, "max_seq_len": int(max_seq_len), **self._bundle_base}
+
+    def _row_views(self, B: int) -> tuple:
+        """The first ``B`` rows of the step's outputs: residual rows, lengths, and the identity tables."""
+        v = self._views.get(B)
+        if v is None:
+            v = self._views[B] = (self.k_tail[:B], self.v_tail[:B], self.b_tail[:B], self.b_seq[:B],
+                                  self._req_to_token[:B], self._req_to_group[:B])
+        return v
 
     def decode_inputs_captured(self, sel: torch.Tensor, b_seq_len: torch.Tensor, b_tail_len: torch.Tensor,
                                tidx_dev: torch.Tensor, kt: torch.Tensor, vt: torch.Tensor, max_seq_len: int) -> dict:
@@ -439,9 +438,8 @@ class MultiSeqKVPool:
             self.select_slots(slots)
         self._call(self._append_args(B, 0))
         max_seq = max(1, max([self.packed_groups[r] for r in slots] + [0]) * self.gt)
-        return self._bundle(self._req_to_token[:B] if identity else self._r2t_sel,
-                            self._req_to_group[:B] if identity else self._r2g_sel,
-                            self.k_tail[:B], self.v_tail[:B], self.b_tail[:B], self.b_seq[:B], max_seq)
+        kt, vt, b_tail, b_seq, r2t, r2g = self._row_views(B)
+        return self._bundle(r2t if identity else self._r2t_sel, r2g if identity else self._r2g_sel, kt, vt, b_tail, b_seq, max_seq)
 
     def decode_seed_seq_device(self, slots: Sequence[int]) -> torch.Tensor:
         """Start of a device-driven decode loop over ``slots`` (reference :1015-1035): binds the batch rows to
@@ -476,10 +474,9 @@ class MultiSeqKVPool:
         decode step - ``append_decode_device`` leaves them up to date)."""
         if refresh:
             self._call(self._append_args(B, 0))
-        return self._bundle(self._req_to_token[:B] if self._sel is None else self._r2t_sel,
-                            self._req_to_group[:B] if self._sel is None else self._r2g_sel,
-                            self.k_tail[:B], self.v_tail[:B], self.b_tail[:B], self.b_seq[:B],
-                            max_seq_len if max_seq_len is not None else self.window.packed_len(self.max_seq_len))
+        kt, vt, b_tail, b_seq, r2t, r2g = self._row_views(int(B))
+        return self._bundle(r2t if self._sel is None else self._r2t_sel, r2g if self._sel is None else self._r2g_sel,
+                            kt, vt, b_tail, b_seq, max_seq_len if max_seq_len is not None else self.max_packed_len)
 
     def seq_lens(self):
         """Host copy of the device sequence lengths (synchronises; tests and logging only)."""

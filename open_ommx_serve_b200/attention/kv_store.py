@@ -50,6 +50,7 @@ class CanonicalKVStore:
         self.pages_per_group, self.G_cap, self.P_cap = p.pages_per_group, p.G_cap, p.P_cap
         self.k_hist, self.v_hist = p.k_hist[0], p.v_hist[0]          # [ring_cap, H, D] views
         self._req_to_token_full, self._req_to_group_full = p._req_to_token, p._req_to_group
+        self._planes_full = None
         self._row = torch.zeros(1, dtype=torch.int64, device=self.device)
 
     # host-side counters, shared with the pool's lists
@@ -98,7 +99,7 @@ class CanonicalKVStore:
     def append(self, k: torch.Tensor, v: torch.Tensor) -> None:
         """One decode step's K/V row ``[H, D]``: ring write, pack of a completed group, lengths."""
         counted = self.packed_groups
-        self.pool.append_decode_batched([0], k.reshape(1, self.H, self.D), v.reshape(1, self.H, self.D))
+        self.pool.append_decode_batched((0,), k, v)
         self.packed_groups = counted            # the reference counts completed groups in maybe_regroup(), not here
 
     def write_token(self, pos: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> None:
@@ -152,8 +153,10 @@ class CanonicalKVStore:
 
     def decode_planes_full(self) -> dict:
         """Full-capacity, fixed-address planes and identity tables (what a captured graph binds)."""
-        pl, p = self.pool.planes, self.pool
-        return {"k_base": pl["k_base"], "k_scale": pl["k_scale"], "k_zp": pl["k_zp"], "k_oidx": None,
+        if self._planes_full is None:
+            pl, p = self.pool.planes, self.pool
+            self._planes_full = {
+                "k_base": pl["k_base"], "k_scale": pl["k_scale"], "k_zp": pl["k_zp"], "k_oidx": None,
                 "k_oval": pl.get("k_oval"), "k_crank": None, "k_obmp": pl.get("k_obmp"), "outlier_repr": "bitmap",
                 "k_fp4_mapscale": pl.get("k_fp4_mapscale"), "k_fp4_mapcenter": pl.get("k_fp4_mapcenter"),
                 "v_main": pl["v_main"], "v_scale": pl["v_scale"], "v_zp": pl["v_zp"],
@@ -161,6 +164,7 @@ class CanonicalKVStore:
                 "page_size": self.ps, "outliers_per_vector": self.k, "k_format": "i2f4", "v_format": "int2",
                 "head_dim": self.D, "n_kv_heads": self.H, "kv_outlier_map": bool(p.kv_outlier_map),
                 "kv_int8_scale": True}
+        return dict(self._planes_full)
 
     def tail_bf16(self):
         """bf16 residual rows (sink, then everything from the boundary on): ``(k_tail, v_tail, n_rows)`` with
@@ -176,10 +180,9 @@ class CanonicalKVStore:
     def decode_inputs(self) -> dict:
         """Argument bundle of the decode call at the current state; lengths stay on the device."""
         p = self.pool
-        return {"planes": self.decode_planes_full(), "k_tail": p.k_tail[:1], "v_tail": p.v_tail[:1],
-                "b_tail_len": p.b_tail[:1], "b_seq_len": p.b_seq[:1], "packed_start_offset": 0,
-                "max_seq_len": max(1, self.window.packed_len(self.max_seq_len)),
-                "max_tail_len": p.max_tail_len}
+        kt, vt, b_tail, b_seq, _, _ = p._row_views(1)
+        return {"planes": self.decode_planes_full(), "k_tail": kt, "v_tail": vt, "b_tail_len": b_tail, "b_seq_len": b_seq,
+                "packed_start_offset": 0, "max_seq_len": max(1, p.max_packed_len), "max_tail_len": p.max_tail_len}
 
 
 __all__ = ["CanonicalKVStore"]

@@ -470,8 +470,19 @@ bool read_pool(PyObject *pool, ommx_kv_pool *p, at::Device *dev) {
     return r.ok;
 }
 
-// kv_append(pool, batch, advance, K, V, slots, write_pos, outputs): K, V [B, H, D] bf16 or None; slots / write_pos index
-// tensors the caller has checked, or None (slots: the pool's selected ones)
+// New rows as the store kernels take them: bf16 on the pool's device, [B, H, D] or for one row [H, D], last dim contiguous
+bool new_rows(const Tensor &K, const Tensor &V, const ommx_kv_pool &p, const at::Device &dev, int64_t batch, int64_t *sb, int64_t *sh) {
+    const int64_t d = K.dim();
+    if ((d != 3 && !(d == 2 && batch == 1)) || V.sizes() != K.sizes() || V.strides() != K.strides()) return false;
+    if (K.scalar_type() != at::kBFloat16 || V.scalar_type() != at::kBFloat16 || K.device() != dev || V.device() != dev || K.stride(d - 1) != 1) return false;
+    if (K.size(d - 1) != p.planes.head_dim || K.size(d - 2) != p.planes.n_kv_heads || (d == 3 && K.size(0) != batch)) return false;
+    *sb = d == 3 ? K.stride(0) : 0;
+    *sh = K.stride(d - 2);
+    return true;
+}
+
+// kv_append(pool, batch, advance, K, V, slots, write_pos, outputs): K, V the new rows or None; slots / write_pos index tensors the
+// caller has checked, or None (slots: the pool's selected ones).  None: K / V need the caller's conversions first.
 PyObject *py_kv_append(PyObject *, PyObject *const *a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "kv_append: wrong argument count"); return nullptr; }
@@ -484,9 +495,9 @@ PyObject *py_kv_append(PyObject *, PyObject *const *a, Py_ssize_t n) {
     bool outputs;
     if (!as_long(a[1], &batch) || !as_long(a[2], &advance) || !as_bool(a[7], &outputs)) { PyErr_SetString(PyExc_TypeError, "kv_append: batch, advance, outputs"); return nullptr; }
     const Tensor *K = as_tensor(a[3]), *V = as_tensor(a[4]), *slots = as_tensor(a[5]), *wpos = as_tensor(a[6]);
-    if (K && V) {
+    if (advance) {
+        NEED(K && V && new_rows(*K, *V, d.pool, dev, batch, &d.new_stride_b, &d.new_stride_h));
         d.k_new = K->data_ptr(); d.v_new = V->data_ptr();
-        d.new_stride_b = K->stride(0); d.new_stride_h = K->stride(1);
     }
     Tensor sel;
     if (!slots && !wpos) { sel = r.tensor(N.sel); d.slots = ptr(sel); }
@@ -502,6 +513,26 @@ PyObject *py_kv_append(PyObject *, PyObject *const *a, Py_ssize_t n) {
     d.status = (int32_t *)ptr(r.tensor(N.status));
     if (!r.ok) return nullptr;
     return PyLong_FromLong(launch(dev, [&](void *stream) { return ommx_b200_kv_append_decode(&d, stream); }));
+    END_HANDLE_TH_ERRORS
+}
+
+// kv_append_block(pool, slot, K, V): prefill of one slot; None: K / V need the caller's conversions first
+PyObject *py_kv_append_block(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 4) { PyErr_SetString(PyExc_TypeError, "kv_append_block: wrong argument count"); return nullptr; }
+    ommx_kv_pool p;
+    memset(&p, 0, sizeof(p));
+    at::Device dev(at::kCUDA);
+    if (!read_pool(a[0], &p, &dev)) return nullptr;
+    PoolReader r{a[0]};
+    const Tensor *K = as_tensor(a[2]), *V = as_tensor(a[3]);
+    int64_t slot, st, sh;
+    NEED(K && V && as_long(a[1], &slot) && K->dim() == 3 && new_rows(*K, *V, p, dev, K->size(0), &st, &sh));
+    int32_t *status = (int32_t *)ptr(r.tensor(N.status));
+    if (!r.ok) return nullptr;
+    return PyLong_FromLong(launch(dev, [&](void *stream) {
+        return ommx_b200_kv_append_block(&p, (int32_t)slot, K->data_ptr(), V->data_ptr(), st, sh, (int32_t)K->size(0), status, stream);
+    }));
     END_HANDLE_TH_ERRORS
 }
 
@@ -541,6 +572,7 @@ PyMethodDef METHODS[] = {
     {"pack_into", (PyCFunction)(void (*)())py_pack_into, METH_FASTCALL, "quantize and pack into given planes; None when an argument needs explaining"},
     {"pack_block", (PyCFunction)(void (*)())py_pack_block, METH_FASTCALL, "quantize and pack into fresh planes"},
     {"kv_append", (PyCFunction)(void (*)())py_kv_append, METH_FASTCALL, "decode-step store of a pool"},
+    {"kv_append_block", (PyCFunction)(void (*)())py_kv_append_block, METH_FASTCALL, "prefill of one slot of a pool"},
     {"kv_gather_tail", (PyCFunction)(void (*)())py_kv_gather_tail, METH_FASTCALL, "residual rows by position"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef MODULE = {PyModuleDef_HEAD_INIT, "_host", "torch tensors -> the C ABI of libommx_b200.so", -1, METHODS, nullptr, nullptr, nullptr, nullptr};

@@ -1357,6 +1357,31 @@ static int launch_store(const StoreParams &sp, const PackKParams &kp, const Pack
     return 0;
 }
 
+// Prefill: the rows a fresh sequence keeps (sink rows, then token `lo` on) go to their ring rows, and its length is set.
+// grid (rows), a block copies one K and one V row.
+struct FillParams {
+    const __nv_bfloat16 *k, *v;
+    int64_t st, sh;
+    __nv_bfloat16 *k_hist, *v_hist;    // the sequence's ring
+    int32_t H, D, sink, ring_cap, n_sink, lo, T, vec;
+    int32_t *seq_len;
+};
+__global__ void __launch_bounds__(256) kv_fill_ring_kernel(FillParams p) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *p.seq_len = p.T;
+    const int tok = (int)blockIdx.x < p.n_sink ? blockIdx.x : p.lo + ((int)blockIdx.x - p.n_sink);
+    if (tok >= p.T) return;
+    const int row = tok < p.sink ? tok : p.sink + (tok - p.sink) % (p.ring_cap - p.sink);
+    const int n = p.H * p.D / (p.vec ? 8 : 1), per = p.vec ? 8 : 1;
+    for (int x = threadIdx.x; x < 2 * n; x += blockDim.x) {
+        const bool is_v = x >= n;
+        const int at = (is_v ? x - n : x) * per, h = at / p.D, c = at - h * p.D;
+        const __nv_bfloat16 *src = (is_v ? p.v : p.k) + (int64_t)tok * p.st + (int64_t)h * p.sh + c;
+        __nv_bfloat16 *dst = (is_v ? p.v_hist : p.k_hist) + (int64_t)row * p.H * p.D + at;
+        if (p.vec) *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(src);
+        else *dst = *src;
+    }
+}
+
 static int launch_append(const ommx_kv_append_args *a, cudaStream_t st) {
     const ommx_kv_pool &pool = a->pool;
     const ommx_kv_planes &pl = pool.planes;
@@ -1610,4 +1635,49 @@ extern "C" int ommx_b200_kv_gather_tail(const ommx_kv_pool *pool, const void *se
                                         int32_t index_is_int64, int32_t batch, int32_t rows,
                                         void *k_tail, void *v_tail, int32_t *status, void *stream) {
     return ommx_b200_kv_gather_inputs(pool, sel, tail_idx, index_is_int64, batch, rows, k_tail, v_tail, nullptr, nullptr, status, stream);
+}
+
+extern "C" int ommx_b200_kv_append_block(const ommx_kv_pool *pool, int32_t slot, const void *k, const void *v, int64_t stride_token,
+                                         int64_t stride_head, int32_t num_tokens, int32_t *status, void *stream) {
+    using namespace ommx;
+    if (!pool || !pool->k_hist || !pool->v_hist || !pool->seq_len || !pool->req_to_token || !pool->req_to_group)
+        return fail(OMMX_E_ARG, "kv_append_block: ring, seq_len and the two tables must not be null");
+    if (slot < 0 || slot >= pool->num_seqs || num_tokens < 0 || (num_tokens > 0 && (!k || !v)))
+        return fail(OMMX_E_ARG, "kv_append_block: slot=%d of %d, %d tokens", slot, pool->num_seqs, num_tokens);
+    const ommx_kv_planes &pl = pool->planes;
+    const int sink = pool->sink_tokens, spare = num_tokens - sink - pool->recent_window;
+    const int groups = spare > 0 ? spare / 32 : 0, boundary = spare > 0 ? sink + 32 * groups : (sink < num_tokens ? sink : num_tokens);
+    if (pool->ring_cap - sink < pool->recent_window + 64)
+        return fail(OMMX_E_ARG, "kv_append_block: ring_cap=%d must hold sink + recent + 64 rows", pool->ring_cap);
+    if (pl.page_size <= 0 || 32 % pl.page_size != 0) return fail(OMMX_E_ARG, "kv_append_block: page_size=%d must divide 32", pl.page_size);
+    if (groups > pool->groups_per_seq || groups * (32 / pl.page_size) > pool->pages_per_seq)
+        return fail(OMMX_E_ARG, "kv_append_block: %d tokens do not fit the sequence's tables", num_tokens);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (groups > 0) {
+        ommx_pack_args a;
+        memset(&a, 0, sizeof(a));
+        a.k = (const __nv_bfloat16 *)k + (int64_t)sink * stride_token;
+        a.v = (const __nv_bfloat16 *)v + (int64_t)sink * stride_token;
+        a.in_dtype = OMMX_DT_BF16; a.num_tokens = 32 * groups; a.stride_token = stride_token; a.stride_head = stride_head;
+        a.dst_pages = pool->req_to_token + (int64_t)slot * pool->pages_per_seq;
+        a.dst_groups = pool->req_to_group + (int64_t)slot * pool->groups_per_seq;
+        a.outlier_select = 1; a.use_pow2 = 1; a.planes = pl; a.status = status;
+        if (int rc = ommx_b200_pack_kv(&a, stream)) return rc;
+    }
+    FillParams f;
+    const int64_t ring = (int64_t)slot * pool->ring_cap * pl.n_kv_heads * pl.head_dim;
+    f.k = (const __nv_bfloat16 *)k; f.v = (const __nv_bfloat16 *)v; f.st = stride_token; f.sh = stride_head;
+    f.k_hist = (__nv_bfloat16 *)pool->k_hist + ring; f.v_hist = (__nv_bfloat16 *)pool->v_hist + ring;
+    f.H = pl.n_kv_heads; f.D = pl.head_dim; f.sink = sink; f.ring_cap = pool->ring_cap;
+    f.n_sink = sink < num_tokens ? sink : num_tokens;
+    f.lo = boundary - 32 > sink ? boundary - 32 : sink;      // the newest packed group stays in the ring too
+    f.T = num_tokens;
+    const uintptr_t all = (uintptr_t)k | (uintptr_t)v | (uintptr_t)f.k_hist | (uintptr_t)f.v_hist;
+    f.vec = all % 16 == 0 && stride_token % 8 == 0 && stride_head % 8 == 0 && f.D % 8 == 0;
+    f.seq_len = pool->seq_len + slot;
+    const int rows = f.n_sink + (num_tokens > f.lo ? num_tokens - f.lo : 0);
+    kv_fill_ring_kernel<<<rows > 0 ? rows : 1, 256, 0, st>>>(f);
+    OMMX_CUDA_TRY(cudaGetLastError());
+    count_launch();
+    return 0;
 }
