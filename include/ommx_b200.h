@@ -105,6 +105,9 @@ typedef struct ommx_pack_args {
 
 int ommx_b200_pack_kv(const ommx_pack_args *args, void *stream);
 
+/* pages[i] = i, groups[i] = i, *status = 0 (optional): the tables of a freshly packed block, in one launch. */
+int ommx_b200_identity_tables(int32_t *pages, int32_t n_pages, int32_t *groups, int32_t n_groups, int32_t *status, void *stream);
+
 /*
  * Re-encode an outlier-index plane of `frames` (group, head, channel) frames with k outliers each between the
  * flat bitmask (4 bytes per frame) and relidx7 (ceil(7k/8) bytes per frame): to_relidx7 = 1 bitmask -> relidx7,

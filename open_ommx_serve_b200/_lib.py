@@ -84,6 +84,7 @@ class KVAppendArgs(C.Structure):
 #: every symbol include/ommx_b200.h declares: name -> (restype, argtypes)
 SYMBOLS = {
     "ommx_b200_pack_kv": (C.c_int, [C.POINTER(PackArgs), C.c_void_p]),
+    "ommx_b200_identity_tables": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]),
     "ommx_b200_outlier_index_convert": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),
     "ommx_b200_decode": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     "ommx_b200_decode_stage1": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),

@@ -84,6 +84,7 @@ struct PlaneSet {
     const Tensor *k_base, *k_scale, *k_zp, *k_idx, *k_oval, *k_ms, *k_mc, *v_main, *v_scale, *v_zp;
 };
 void *ptr(const Tensor *t) { return t ? t->data_ptr() : nullptr; }
+void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 bool fill_planes(const PlaneSet &s, int64_t k, bool use_map, bool relidx7, ommx_kv_planes *p) {
     for (const Tensor *t : {s.k_base, s.k_scale, s.k_zp, s.v_main, s.v_scale, s.v_zp})
@@ -389,8 +390,12 @@ PyObject *py_pack_block(PyObject *, PyObject *const *a, Py_ssize_t n) {
     auto opt = [](const Tensor &t) { return t.defined() ? &t : nullptr; };
     const PlaneSet s{&k_base, &k_scale, &k_zp, opt(k_obmp), opt(k_oval), opt(k_ms), opt(k_mc), &v_main, &v_scale, &v_zp};
     Tensor status;
-    if (check) status = at::zeros({1}, ints);
-    int rc = 0;
+    if (check) status = at::empty({1}, ints);
+    Tensor r2t = at::empty({1, pages}, ints), r2g = at::empty({1, G}, ints);
+    int rc = launch(K->device(), [&](void *stream) {
+        return ommx_b200_identity_tables((int32_t *)r2t.data_ptr(), (int32_t)pages, (int32_t *)r2g.data_ptr(), (int32_t)G, (int32_t *)ptr(status), stream);
+    });
+    if (rc != 0) return PyLong_FromLong(rc);
     NEED(pack_planes(*K, *V, s, nullptr, nullptr, k, is_signed, use_pow2, use_map, check ? (int32_t *)status.data_ptr() : nullptr, &rc));
     if (rc == 0 && relidx7 && k > 0) {
         // same outlier set, other index encoding: k ascending 7-bit positions per frame (the value plane is shared)
@@ -401,7 +406,6 @@ PyObject *py_pack_block(PyObject *, PyObject *const *a, Py_ssize_t n) {
         k_obmp = Tensor();
     }
     if (rc != 0) return PyLong_FromLong(rc);
-    Tensor r2t = at::arange(pages, ints).reshape({1, pages}), r2g = at::arange(G, ints).reshape({1, G});
     int64_t bits = 0;
     if (check) bits = read_int(status);
     PyObject *d = PyDict_New();
@@ -445,7 +449,7 @@ struct PoolReader {
         return r;
     }
 };
-void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
+
 
 // the pool descriptor; its tensors stay referenced by the pool object the caller holds
 bool read_pool(PyObject *pool, ommx_kv_pool *p, at::Device *dev) {

@@ -1681,3 +1681,23 @@ extern "C" int ommx_b200_kv_append_block(const ommx_kv_pool *pool, int32_t slot,
     count_launch();
     return 0;
 }
+
+namespace ommx {
+__global__ void identity_tables_kernel(int32_t *pages, int n_pages, int32_t *groups, int n_groups, int32_t *status) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_pages) pages[i] = i;
+    if (i < n_groups) groups[i] = i;
+    if (i == 0 && status) *status = 0;
+}
+}  // namespace ommx
+
+extern "C" int ommx_b200_identity_tables(int32_t *pages, int32_t n_pages, int32_t *groups, int32_t n_groups, int32_t *status, void *stream) {
+    using namespace ommx;
+    if (n_pages < 0 || n_groups < 0 || (n_pages > 0 && !pages) || (n_groups > 0 && !groups))
+        return fail(OMMX_E_ARG, "identity_tables: %d pages, %d groups", n_pages, n_groups);
+    const int n = n_pages > n_groups ? n_pages : n_groups;
+    identity_tables_kernel<<<n > 0 ? (n + 255) / 256 : 1, 256, 0, (cudaStream_t)stream>>>(pages, n_pages, groups, n_groups, status);
+    OMMX_CUDA_TRY(cudaGetLastError());
+    count_launch();
+    return 0;
+}
