@@ -625,61 +625,29 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             return false;
         }
         const int lg = (it - pc.it0) * GS + gsel;                 // local group of this unit
-        // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
-        // run up to NS groups ahead and the tiles of one unit are built by different warps, so
-        // "tile k was read" events rotate over NS barriers per unit (barrier k % NS, phase
-        // k / NS): the newest event a waiter can be missing is then always the one it waits
-        // for, never an older phase of the same parity.  A unit without a group in this stage goes
-        // through the same hand-overs with nothing in them.
-        if (it > 0 && !mbar_wait(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it - 1, NS)), ring_phase(it - 1, NS), wait_limit)) {
-            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
-            return false;
-        }
-        if (lg < pc.ng && !(p.abl & ABL_NO_COMPUTE)) {
-            uint8_t *gb = s_stage + (size_t)s * p.stage_bytes + (size_t)gsel * p.gb_bytes;
-            const int d0 = 64 * hf + 2 * lane;                   // first of this lane's two channels
-            bool clamped_any = false;
-            const bool splice = k_out > 0 && !no_outlier;
-            // ---- first the rows the code MMAs and the softmax read (K factors, V factors and zero-points): they are
-            //      cheap, and the MMA warp starts on them while the deltas are scattered ----
-            const uint32_t e2 = *reinterpret_cast<const uint16_t *>(gb + p.o_ks + h * 128 + d0);
-            const uint32_t z2 = *reinterpret_cast<const uint32_t *>(gb + p.o_kz + h * 256 + 2 * d0);
-            {
-                bool cl0, cl1;
-                const uint32_t f0 = pow2_f16_bits(max((int)(int8_t)e2, -126), cl0), f1 = pow2_f16_bits(max((int)(int8_t)(e2 >> 8), -126), cl1);
-                clamped_any = cl0 || cl1;
-                const uint32_t kf = hmul2_f16(f0 | (f1 << 16), slot_scale);                // * 4^-slot: exact, subnormals included
-                uint8_t *row = tile + ROW_KF * DT_STRIDE + 128 * hf + 64 * (da >> 1) + 16 * dj + 8 * (da & 1) + 2 * dh;
-                *reinterpret_cast<uint16_t *>(row) = (uint16_t)kf;
-                *reinterpret_cast<uint16_t *>(row + 4) = (uint16_t)(kf >> 16);
-            }
-            {   // V side: lane = (pair of tokens, scale group): power-of-two factors and zero-points of the two tokens
-                const int copy = it & 1;
-                const int tk = 16 * hf + 2 * (lane & 7), cg = lane >> 3;
-                uint32_t v0 = 0x80u, v1 = 0x80u, y0 = 0u, y1 = 0u;   // exponent -128 -> factor 0
-                const uint8_t *vs = gb + p.o_vs + (tk * H + h) * 4 + cg, *vz = gb + p.o_vz + (tk * H + h) * 8 + 2 * cg;
-                if (32 * lg + tk < pc.ntok) { v0 = vs[0]; y0 = *reinterpret_cast<const uint16_t *>(vz); }
-                if (32 * lg + tk + 1 < pc.ntok) { v1 = vs[4 * H]; y1 = *reinterpret_cast<const uint16_t *>(vz + 8 * H); }
-                bool cl0, cl1;
-                const uint32_t f0 = pow2_f16_bits((int)(int8_t)v0, cl0), f1 = pow2_f16_bits((int)(int8_t)v1, cl1);
-                clamped_any = clamped_any || cl0 || cl1;
-                *reinterpret_cast<uint32_t *>(tile + (ROW_VF + copy) * DT_STRIDE + 64 * cg + 16 * (lane & 3) + 8 * hf + 4 * ((lane >> 2) & 1)) = f0 | (f1 << 16);
-                *reinterpret_cast<uint32_t *>(tile + (ROW_ZT + copy) * DT_STRIDE + 2 * tk + ZT_STRIDE * cg) = pack_f16x2_sat(bf16_bits_to_f32(y0), bf16_bits_to_f32(y1));
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_trows + 8 * unit);
-            // ---- then the outlier deltas of this half's columns ----
+        const bool active = lg < pc.ng && !(p.abl & ABL_NO_COMPUTE);
+        const uint8_t *gb = s_stage + (size_t)s * p.stage_bytes + (size_t)gsel * p.gb_bytes;
+        const int d0 = 64 * hf + 2 * lane;                       // first of this lane's two channels
+        const bool splice = k_out > 0 && !no_outlier;
+        // ---- everything that only reads the stage comes before the wait for the tile, which the MMA warps make a decode warp
+        //      wait for (a sixth of its time): the parameters of both channels, the K and V factors, V zero-points ----
+        bool clamped_any = false;
+        uint32_t e2 = 0, z2 = 0, kf = 0, vf = 0, zt = 0, ms2 = 0, mc2 = 0;
+        uint2 bm2 = make_uint2(0u, 0u);
+        uint32_t st[2] = {0, 0}, sth[2] = {0, 0};                // nibble stream of each channel: outliers 0..7, 8..15
+        const int vtk = 16 * hf + 2 * (lane & 7), vcg = lane >> 3;   // V side: lane = (pair of tokens, scale group)
+        if (active) {
+            e2 = *reinterpret_cast<const uint16_t *>(gb + p.o_ks + h * 128 + d0);
+            z2 = *reinterpret_cast<const uint32_t *>(gb + p.o_kz + h * 256 + 2 * d0);
+            uint32_t v0 = 0x80u, v1 = 0x80u, y0 = 0u, y1 = 0u;   // exponent -128 -> factor 0
+            const uint8_t *vs = gb + p.o_vs + (vtk * H + h) * 4 + vcg, *vz = gb + p.o_vz + (vtk * H + h) * 8 + 2 * vcg;
+            if (32 * lg + vtk < pc.ntok) { v0 = vs[0]; y0 = *reinterpret_cast<const uint16_t *>(vz); }
+            if (32 * lg + vtk + 1 < pc.ntok) { v1 = vs[4 * H]; y1 = *reinterpret_cast<const uint16_t *>(vz + 8 * H); }
             if (splice) {
-                // clear this half's columns of token rows 0..31 (128 bytes per row)
-#pragma unroll
-                for (int k2 = 0; k2 < 8; ++k2)
-                    *reinterpret_cast<uint4 *>(tile + (4 * k2 + (lane >> 3)) * DT_STRIDE + 128 * hf + 16 * (lane & 7)) = make_uint4(0, 0, 0, 0);
-                uint32_t ms2 = 0, mc2 = 0;
                 if (p.use_map) {
                     ms2 = *reinterpret_cast<const uint32_t *>(gb + p.o_ms + h * 256 + 2 * d0);
                     mc2 = *reinterpret_cast<const uint32_t *>(gb + p.o_mc + h * 256 + 2 * d0);
                 }
-                uint2 bm2;
                 if (!p.idx7) {
                     bm2 = *reinterpret_cast<const uint2 *>(gb + p.o_bm + h * 512 + 4 * d0);
                 } else {
@@ -702,7 +670,6 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     }
                     bm2 = make_uint2(m2[0], m2[1]);
                 }
-                uint32_t st[2] = {0, 0}, sth[2] = {0, 0};            // nibble stream of each channel: outliers 0..7, 8..15
                 const int nb = KOUT >= 0 ? (KOUT + 1) / 2 : p.nb;
                 const uint8_t *ov = gb + p.o_ov + (h * 128 + d0) * nb;          // 2*nb bytes, 2-byte aligned
                 if (nb == 3) {
@@ -732,6 +699,42 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     const uint32_t w = *reinterpret_cast<const uint16_t *>(ov);
                     st[0] = w & 0xFFu; st[1] = w >> 8;
                 }
+            }
+            bool cl0, cl1, cl2, cl3;
+            const uint32_t k0 = pow2_f16_bits(max((int)(int8_t)e2, -126), cl0), k1 = pow2_f16_bits(max((int)(int8_t)(e2 >> 8), -126), cl1);
+            kf = hmul2_f16(k0 | (k1 << 16), slot_scale);         // * 4^-slot: exact, subnormals included
+            const uint32_t f0 = pow2_f16_bits((int)(int8_t)v0, cl2), f1 = pow2_f16_bits((int)(int8_t)v1, cl3);
+            vf = f0 | (f1 << 16);
+            zt = pack_f16x2_sat(bf16_bits_to_f32(y0), bf16_bits_to_f32(y1));
+            clamped_any = cl0 || cl1 || cl2 || cl3;
+        }
+        // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
+        // run up to NS groups ahead and the tiles of one unit are built by different warps, so
+        // "tile k was read" events rotate over NS barriers per unit (barrier k % NS, phase
+        // k / NS): the newest event a waiter can be missing is then always the one it waits
+        // for, never an older phase of the same parity.  A unit without a group in this stage goes
+        // through the same hand-overs with nothing in them.
+        if (it > 0 && !mbar_wait(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it - 1, NS)), ring_phase(it - 1, NS), wait_limit)) {
+            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
+            return false;
+        }
+        if (active) {
+            // ---- first the rows the code MMAs and the softmax read (K factors, V factors and zero-points): the MMA warp
+            //      starts on them while the deltas are scattered ----
+            uint8_t *row = tile + ROW_KF * DT_STRIDE + 128 * hf + 64 * (da >> 1) + 16 * dj + 8 * (da & 1) + 2 * dh;
+            *reinterpret_cast<uint16_t *>(row) = (uint16_t)kf;
+            *reinterpret_cast<uint16_t *>(row + 4) = (uint16_t)(kf >> 16);
+            const int copy = it & 1;
+            *reinterpret_cast<uint32_t *>(tile + (ROW_VF + copy) * DT_STRIDE + 64 * vcg + 16 * (lane & 3) + 8 * hf + 4 * ((lane >> 2) & 1)) = vf;
+            *reinterpret_cast<uint32_t *>(tile + (ROW_ZT + copy) * DT_STRIDE + 2 * vtk + ZT_STRIDE * vcg) = zt;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_trows + 8 * unit);
+            // ---- then the outlier deltas of this half's columns ----
+            if (splice) {
+                // clear this half's columns of token rows 0..31 (128 bytes per row)
+#pragma unroll
+                for (int k2 = 0; k2 < 8; ++k2)
+                    *reinterpret_cast<uint4 *>(tile + (4 * k2 + (lane >> 3)) * DT_STRIDE + 128 * hf + 16 * (lane & 7)) = make_uint4(0, 0, 0, 0);
                 __syncwarp();                                        // the cleared rows before any delta lands in them
                 const uint32_t bmv[2] = {bm2.x, bm2.y};
                 // The code byte holding this lane's channels, row pz: byte pz*TS + h*32 + d0/4 of the (1 KB aligned)
@@ -965,19 +968,6 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     kw[nt].y = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 16 + 4 * j), SWZ));
                 }
             }
-            // q.zp of heads 2j and 2j+1: exact bf16 products of the raw query with the zero-points, summed in fp32, every row
-            // of the A operand being the zero-point row.  It needs no tile, so it runs while the tile is built.
-            float Z0[4] = {0.f, 0.f, 0.f, 0.f}, Z1[4] = {0.f, 0.f, 0.f, 0.f};
-            {
-                const uint8_t *zrow = gb + p.o_kz + h * 256 + 16 * j;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const uint4 z = *reinterpret_cast<const uint4 *>(zrow + 64 * v);
-                    mma_bf16(Z0, z.x, z.x, z.y, z.y, QR[4 * v], QR[4 * v + 1]);
-                    mma_bf16(Z1, z.z, z.z, z.w, z.w, QR[4 * v + 2], QR[4 * v + 3]);
-                }
-            }
-            const float Sz[2] = {(Z0[0] + Z1[0]) * p.sm_scale, (Z0[1] + Z1[1]) * p.sm_scale};
             // The unit's sidecar tile arrives in two steps: first the factor and zero-point rows, then the outlier
             // deltas.  The code MMAs run on the first, while the decode warps still scatter the deltas.
             if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
@@ -1003,6 +993,19 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     }
                 }
             }
+            // q.zp of heads 2j and 2j+1: exact bf16 products of the raw query with the zero-points, summed in fp32, every row
+            // of the A operand being the zero-point row.  It needs no tile, so it stands where this warp may have to wait for the deltas.
+            float Z0[4] = {0.f, 0.f, 0.f, 0.f}, Z1[4] = {0.f, 0.f, 0.f, 0.f};
+            {
+                const uint8_t *zrow = gb + p.o_kz + h * 256 + 16 * j;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const uint4 z = *reinterpret_cast<const uint4 *>(zrow + 64 * v);
+                    mma_bf16(Z0, z.x, z.x, z.y, z.y, QR[4 * v], QR[4 * v + 1]);
+                    mma_bf16(Z1, z.z, z.z, z.w, z.w, QR[4 * v + 2], QR[4 * v + 3]);
+                }
+            }
+            const float Sz[2] = {(Z0[0] + Z1[0]) * p.sm_scale, (Z0[1] + Z1[1]) * p.sm_scale};
             if (has_delta) {
                 if (!mbar_wait(bar_tfull + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
                     gave_up = true;
