@@ -17,8 +17,9 @@ from concurrent.futures import ThreadPoolExecutor
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libommx_b200.so")
-SOURCES = ("ommx_capi.cu", "ommx_pack.cu", "ommx_decode.cu")
-HEADERS = ("ommx_common.cuh", "ommx_decode_tc.cuh", "ommx_tables.inc", os.path.join("..", "..", "include", "ommx_b200.h"))
+SOURCES = ("ommx_stage1_h8.cu", "ommx_stage1_h4.cu", "ommx_stage1_h2.cu", "ommx_stage1_h1.cu", "ommx_decode.cu", "ommx_pack.cu",
+           "ommx_capi.cu")
+HEADERS = ("ommx_common.cuh", "ommx_stage1.cuh", "ommx_decode_tc.cuh", "ommx_tables.inc", os.path.join("..", "..", "include", "ommx_b200.h"))
 OBJ = os.path.join(PKG, "build")
 HOST_LIB = os.path.join(PKG, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "ommx_host.cpp")

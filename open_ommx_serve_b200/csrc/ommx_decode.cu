@@ -25,1184 +25,9 @@
 // query with the zero-points (paged_decode.py:1754-1770), fp32 accumulation, V as exact code*2^e
 // products with the zero-point bias summed apart.  One point differs inside the gate: P is rounded
 // to fp16 (11 bits) instead of bf16.
-#include "ommx_common.cuh"
-#include <cuda.h>                       // CUtensorMap (types only; the encoder is looked up at run time)
-#include <mutex>
-#include <stdlib.h>
-#include <string.h>
+#include "ommx_stage1.cuh"
 
 namespace ommx {
-
-constexpr int HD = 128;                 // head_dim this build serves
-constexpr int NCW = 8;                  // (group, head) units in flight per CTA, one MMA warp each
-// Two warp layouts.  Narrow (4 or 8 local kv heads: 14 or 28 copies per ring stage): 15 decode warps + 1 producer warp,
-// which also builds the last tile half once its copies are out.  Wide (1 or 2 local kv heads: a stage is 8 or 4 groups,
-// 112 or 56 small copies): 16 decode warps + 4 producer warps, because one warp issues a bulk copy only every ~60 cycles
-// and the issues of different warps overlap (112 copies: 6400 cycles from one warp, 2000 from four).
-template <int H> struct WarpLayout {
-    static constexpr bool WIDE = H <= 2;
-    static constexpr int NDW = WIDE ? 16 : 15;            // decode warps (stateless sidecar builders, items dealt round-robin)
-    static constexpr int NPW = WIDE ? 4 : 1;              // producer warps
-    static constexpr int PRODUCER_WARP = NCW + NDW;       // the first of them
-    static constexpr int THREADS = (NCW + NDW + NPW) * 32;
-};
-// Register budget per role (setmaxnreg, warpgroup granularity).  Only what the CTA was launched with
-// can be moved around: 768 threads x 80 = 61440 = 256*128 (MMA) + 512*56 (decode + producer).  The
-// launch refuses to run if the compiled kernel holds fewer registers than the roles ask for, because
-// setmaxnreg.inc would then wait forever.
-#define OMMX_REGS_MMA "128"
-#define OMMX_REGS_DECODE "56"
-#define OMMX_REGS_PRODUCER "24"
-constexpr int REGS_MMA = 128, REGS_DECODE = 56, REGS_PRODUCER = 24;
-constexpr int MAX_STAGES = 4;           // ring depth (3 when the planes of a stage are large)
-constexpr int DT_STRIDE = 272;          // bytes per sidecar-tile row (256 data + 16 pad)
-constexpr int ROW_KF = 32;              // K scale factors 2^(e+4) * 4^-slot, fp16, in code-fragment order
-constexpr int ROW_VF = 33;              // V scale factors, fp16, fragment order (rows 33, 34: two copies)
-constexpr int ROW_ZT = 35;              // V zero-points [scale group][token], fp16 (rows 35, 36: two copies)
-constexpr int ZT_STRIDE = 68;           // bytes from one scale group's zero-points to the next (64 + a bank)
-constexpr int DT_ROWS = 37;             // rows 0..31: outlier deltas [token][channel in fragment order], fp16
-constexpr int DT_BYTES = DT_ROWS * DT_STRIDE;
-constexpr int MAX_SPLIT_GROUPS = 512;   // groups of the longest split that the entry points accept (16K tokens)
-constexpr int MAX_SPLIT_PAGES = 1024;
-constexpr int MAX_PIECES = 256;         // pieces of sequences one CTA can work on (32 bytes of shared memory each)
-constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;   // about a second of SM clock: the wait has failed
-
-struct S1Params {
-    const __nv_bfloat16 *q;
-    int64_t q_sb, q_sh;
-    int32_t B, Hq, H, gqa, q_vec_ok;     // q_vec_ok: eight adjacent q elements may be fetched as one 16-byte word
-    const uint8_t *k_base, *v_main, *v_scale, *v_zp, *k_scale, *k_zp, *k_ms, *k_mc, *k_obmp, *k_oval;
-    int32_t ps, ppg, num_pages, num_slots, k_out, nb, use_map;
-    int32_t nbi;                         // bytes of outlier index per channel: 4 (flat bitmask) or ceil(7k/8) (relidx7, idx7 = 1)
-    int32_t idx7;
-    const int32_t *b_seq_len;
-    const void *r2t, *r2g;
-    int32_t tbl64;
-    int64_t r2t_sb, r2g_sb;
-    float *al;
-    int64_t al_sb, al_sh, al_ss;
-    int32_t S, seg_group_base;
-    int32_t ncta, waves;                 // CTAs of the launch (one per SM at most), rounds of them that B * S splits would take
-    float sm_scale, logit_cap;
-    int32_t *status;
-    int32_t abl;
-    // shared-memory layout of one group block (bytes)
-    int32_t GS, gb_bytes, stage_bytes, nstages, hshift;
-    int32_t o_vm, o_vs, o_vz, o_ks, o_kz, o_ms, o_mc, o_bm, o_ov;
-    // tensor maps of the two code planes as [bytes/128][128] uint8 with 128-byte swizzle
-    uint32_t swz;                        // 0x70 when the maps are in use, else 0
-    int32_t rows_per_page;               // 128-byte lines per page
-    alignas(64) CUtensorMap tmap_k;
-    alignas(64) CUtensorMap tmap_v;
-};
-
-// One bulk copy of a stage: source plane, bytes, destination inside the stage, and which table entry
-// (page id or group slot) selects the source block.
-struct __align__(16) CopyDesc {
-    const uint8_t *src;                  // plane base, or nullptr + kind for a tensor-map copy
-    uint32_t unit, dst;
-    int32_t tbase, tmul, gi, tok0;       // gi: group in stage (bits 0..7) | kind << 8
-};                                       // kind 0 bulk copy, 1 k_base through tmap_k, 2 v_main through tmap_v
-// a stage holds at most 8 groups x (4 planes x 4 pages + 6 group planes) = 176 copies (1 kv head, 8-token pages)
-
-// ---- PTX wrappers --------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: returns false (and the caller raises OMMX_ST_TIMEOUT) instead of spinning forever.
-// try_wait already parks the warp in hardware for a short while.  The limit is counted on the SM
-// clock (cheap to read); nanosleep or the global timer in this loop would put their own latency
-// on every producer/consumer hand-off.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long limit = WAIT_LIMIT_CYCLES) {
-    long long t_end = 0;
-#pragma unroll 1
-    for (uint32_t i = 1; !mbar_try_wait(bar, parity); ++i) {
-        if ((i & 63u) == 0) {
-            const long long now = clock64();
-            if (t_end == 0) t_end = now + limit;
-            else if (now > t_end) return false;
-        }
-    }
-    return true;
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                        uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// two 16x16 byte matrices (rows from lanes 0-15 and 16-31), transposed: r[2m], r[2m+1] = rows 4j..4j+3 of columns g and
-// g + 8 of matrix m (lane = 4g + j)
-__device__ __forceinline__ void ldsm_b8_trans_x2(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t &r0, uint32_t &r1) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-// transpose an 8x8 matrix of 16-bit elements held one row pair per lane (the accumulator layout)
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
-    uint32_t r;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
-    return r;
-}
-__device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-__device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {       // clamped to the finite range
-    uint32_t r;
-    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-__device__ __forceinline__ uint32_t hmul2_f16(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// The 2-bit code planes are staged with the TMA's 128-byte swizzle (16-byte chunk index XOR line
-// index mod 8) when a page is a whole number of 1 KB swizzle atoms: a head's 32-byte code row then
-// lands in a different bank window on each token row instead of the same one.  `o` is the linear byte
-// offset inside a 1 KB aligned region; swz is 0x70 (swizzled) or 0 (plain bulk copies).
-__device__ __forceinline__ uint32_t swz128(uint32_t o, uint32_t swz) { return o ^ ((o >> 3) & swz); }
-
-__device__ __forceinline__ void tma_2d_g2s(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-
-__device__ __forceinline__ int64_t load_index(const void *tbl, int is64, int64_t i) {
-    return is64 ? reinterpret_cast<const int64_t *>(tbl)[i] : (int64_t) reinterpret_cast<const int32_t *>(tbl)[i];
-}
-
-// =================================================================================================
-// Stage 1
-// =================================================================================================
-// Ablation bits (differential timing only, they break parity; mirror of the reference's
-// OMMX_ABL_* knobs, paged_decode.py:3267-3279): 1 = skip the outlier splice, 2 = skip V dequant
-// and P.V, 4 = skip the K code dequant and its MMAs.
-constexpr int ABL_NO_OUTLIER = 1, ABL_NO_V = 2, ABL_NO_K = 4, ABL_NO_COMPUTE = 8;   // 8: stream the planes only
-// 16 (tests of the give-up path only): waits give up after about 2 ms and the producer announces the bytes of its
-// second ring fill without issuing the copies, so that every role runs out of patience and leaves through the epilogue
-constexpr int ABL_TEST_STALL = 16;
-constexpr long long TEST_WAIT_LIMIT_CYCLES = 4000000ll;
-
-// fp16 bits of 2^(e + FBIAS).  Exponents below -18 give 0 (such a scale step is under 2^-18 and the
-// term it multiplies is dropped); exponents above 11 are clamped and reported.
-constexpr int FBIAS = 4;
-__device__ __forceinline__ uint32_t pow2_f16_bits(int e, bool &clamped) {
-    int u = e + 15 + FBIAS;
-    clamped = u > 30;
-    u = min(u, 30);
-    return u < 1 ? 0u : (uint32_t)u << 10;
-}
-// the reference rounds an outlier's delta to bf16; keep that rounding point, then store it as fp16
-// (exact: 8 significant bits fit in 11)
-__device__ __forceinline__ uint32_t f16x2_of_bf16_rounded(float lo, float hi) {
-    uint32_t b;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b) : "f"(hi), "f"(lo));
-    return pack_f16x2_sat(__uint_as_float(b << 16), __uint_as_float(b & 0xFFFF0000u));
-}
-// the FP4 levels of four outliers (16 bits of the nibble stream) as the upper bytes of their fp16 values; the lower
-// bytes are zero.  A nibble is the byte selector of the magnitude table; its sign bit, which as a selector bit replicates
-// a byte's sign, turns 0x80 into 0xFF in a second lookup.
-__device__ __forceinline__ uint32_t fp4_levels_hi(uint32_t nibbles) {
-    const uint32_t mag = __byte_perm(0x3E3C3800u, 0x46444240u, nibbles & 0x7777u);
-    uint32_t sgn;
-    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(sgn) : "r"(0x80808080u), "r"(nibbles));
-    return mag | ((sgn << 7) & 0x80808080u);
-}
-__device__ __forceinline__ uint32_t f16_bits_sat(float x) {
-    uint16_t r;
-    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(r) : "f"(x));
-    return (uint32_t)r;
-}
-// field i (0..7) of the lower and upper 8 codes of a 32-bit code word, as two fp16 subnormals
-// code * 4^slot * 2^-24 with slot = i (i < 5) or i - 5: no arithmetic beyond the AND
-__device__ __forceinline__ uint32_t code_pair(uint32_t w, int i) {
-    return i < 5 ? (w & (0x00030003u << (2 * i))) : ((w >> 10) & (0x00030003u << (2 * (i - 5))));
-}
-__device__ __forceinline__ int code_slot(int i) { return i < 5 ? i : i - 5; }
-
-// stage index and phase parity of ring use number `it` (ring depth ns: 4 unless the planes are large)
-__device__ __forceinline__ int ring_slot(int it, int ns) { return ns == 4 ? (it & 3) : it % ns; }
-__device__ __forceinline__ uint32_t ring_phase(int it, int ns) { return (uint32_t)(ns == 4 ? (it >> 2) : it / ns) & 1u; }
-
-// ---- how the groups of a launch are shared out over its CTAs ------------------------------------------
-// The packed groups of all sequences form one running list, and CTA i takes groups [i * per, (i + 1) * per) of it, whatever
-// sequences they belong to: every CTA has the same work up to one group, also when the lengths are ragged (32 sequences of
-// 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us around its steady state).  A piece of
-// a sequence writes its partial result to workspace slot (its CTA - the first CTA of the sequence), and the caller's
-// workspace has S slots per sequence, which bounds `per` from below.  Where that bound makes the shares longer than S equal
-// splits per sequence dealt out one by one would be, those are taken instead (per = 0): item x is split x % S of sequence x / S.
-struct SharePlan {
-    int per, total;                      // groups per CTA (0: equal splits per sequence), groups of all sequences
-};
-__device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
-__device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, int ncta, int waves) {
-    SharePlan s;
-    s.total = total;
-    s.per = max(1, (total + ncta - 1) / ncta);
-    const int equal = (longest + S - 1) / S;
-    if (B == 1) {
-        s.per = max(s.per, equal);                             // a lone sequence starts at a CTA's beginning: exactly ceil(n / per) slots
-    } else {
-        if (S >= 2) s.per = max(s.per, (longest - 2) / (S - 1) + 1);   // anywhere else it touches up to (n - 2) / per + 2 CTAs
-        if (S < 2 || (waves <= MAX_PIECES && waves * equal <= s.per)) s.per = 0;
-    }
-    return s;
-}
-// called by whole warps; every lane gets the same answer
-__device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, int ncta, int waves, int lane) {
-    int n = 0, mx = 0;
-    if (B == 1) {
-        n = mx = groups_of(b_seq_len[0]);
-    } else {
-        for (int i = lane; i < B; i += 32) {
-            const int g = groups_of(b_seq_len[i]);
-            n += g;
-            mx = max(mx, g);
-        }
-        n = __reduce_add_sync(0xFFFFFFFFu, n);
-        mx = __reduce_max_sync(0xFFFFFFFFu, mx);
-    }
-    return share_plan_of(n, mx, B, S, ncta, waves);
-}
-
-// One piece of work of a CTA: consecutive groups of one sequence.  `it` counts the CTA's ring stages across its pieces, so that
-// the ring never drains between two of them.  One warp lists the pieces in shared memory; the roles walk that list, because
-// the walk's own state costs a decode warp (56 registers) 9 % of its speed in spills.
-struct alignas(16) Piece {
-    int b, slot, g0, ng;                 // sequence, workspace slot, first group in the sequence, groups
-    int ntok, it0, it1, more;            // tokens, ring iterations [it0, it1), whether another piece follows
-};
-struct PieceWalk {
-    int pos, end;                        // running list: first group of the piece, end of this CTA's share; splits: item, items
-};
-template <int GS>
-__device__ __forceinline__ void piece_range(Piece &c, int seq, int g0, int ng) {
-    c.g0 = g0;
-    c.ng = ng;
-    c.ntok = min(seq - 32 * g0, 32 * ng);
-    c.it1 = c.it0 + (ng + GS - 1) / GS;
-}
-// equal splits: the first item at or after w.pos that has groups
-template <int GS> __device__ __forceinline__ bool piece_of_splits(Piece &c, PieceWalk &w, const S1Params &p) {
-    for (; w.pos < w.end; w.pos += p.ncta) {
-        c.b = w.pos / p.S;
-        c.slot = w.pos - c.b * p.S;
-        const int seq = p.b_seq_len[c.b], n = groups_of(seq), per = (n + p.S - 1) / p.S, g0 = c.slot * per;
-        if (g0 < n) {
-            piece_range<GS>(c, seq, g0, min(per, n - g0));
-            return true;
-        }
-    }
-    return false;
-}
-template <int GS> __device__ __forceinline__ bool first_piece(Piece &c, PieceWalk &w, const S1Params &p, const SharePlan &plan, int cta, int lane) {
-    c.it0 = 0;
-    if (plan.per == 0) {
-        w.pos = cta;
-        w.end = p.B * p.S;
-        return piece_of_splits<GS>(c, w, p);
-    }
-    w.pos = cta * plan.per;
-    w.end = min(w.pos + plan.per, plan.total);
-    if (w.pos >= w.end) return false;
-    int off = 0, seq, n;                                       // groups before the sequence that holds w.pos
-    if (p.B == 1) {
-        c.b = 0;
-        seq = p.b_seq_len[0];
-        n = groups_of(seq);
-    } else {
-        for (int base = 0;; base += 32) {
-            const int len = base + lane < p.B ? p.b_seq_len[base + lane] : 0;
-            const int g = groups_of(len);
-            int x = g;                                         // inclusive sums over the lanes
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-                if (lane >= o) x += y;
-            }
-            const uint32_t past = __ballot_sync(0xFFFFFFFFu, off + x > w.pos);
-            if (past) {
-                const int l = __ffs(past) - 1;
-                c.b = base + l;
-                seq = __shfl_sync(0xFFFFFFFFu, len, l);
-                n = __shfl_sync(0xFFFFFFFFu, g, l);
-                off += __shfl_sync(0xFFFFFFFFu, x, l) - n;
-                break;
-            }
-            off += __shfl_sync(0xFFFFFFFFu, x, 31);
-        }
-    }
-    c.slot = cta - off / plan.per;
-    const int g0 = w.pos - off, ng = min(n - g0, w.end - w.pos);
-    piece_range<GS>(c, seq, g0, ng);
-    return true;
-}
-template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk &w, const S1Params &p, const SharePlan &plan) {
-    c.it0 = c.it1;
-    if (plan.per == 0) {
-        w.pos += p.ncta;
-        return piece_of_splits<GS>(c, w, p);
-    }
-    w.pos += c.ng;
-    if (w.pos >= w.end) return false;
-    int seq;
-    do seq = p.b_seq_len[++c.b];                               // the share has groups left, so a later sequence has some
-    while (seq <= 0);
-    const int n = groups_of(seq), ng = min(n, w.end - w.pos);
-    c.slot = 0;                                                // it begins inside this CTA's share
-    piece_range<GS>(c, seq, 0, ng);
-    return true;
-}
-
-// KOUT: outliers per K vector known at compile time (static, unrolled splice) or -1 (runtime).
-//
-// Every MMA is m16n8k16 fp16 with the 2-bit codes as the A operand: a code field masked in place is an
-// fp16 subnormal, code * 4^slot * 2^-24, exact and without an offset.  N = 8 columns are the query heads
-// of the kv head (GQA <= 8).
-//   logits   S^T[token][head]  = codes[token][ch] . (q * 2^e_k)[ch][head]      (2 m-tiles x 8 k-steps)
-//                              + delta[token][ch] . q[ch][head]                (sidecar tile, same shape)
-//                              + zp[ch] . q[ch][head]                          (one row, broadcast)
-//   output   O^T[ch][head]     = codes^T[ch][token] . (P * 2^e_v)[token][head] (8 m-tiles x 2 k-steps, the
-//                                16 rows of an m-tile lie in one V scale group)
-//                              + vz^T[group][token] . P[token][head]
-// The power-of-two factors, zero-points and deltas of a unit are laid out for these fragments by the
-// decode warps (the sidecar tile), so the MMA warps multiply and accumulate and do little else.
-template <int KOUT, int H>
-__global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kernel(const __grid_constant__ S1Params p) {
-    constexpr bool WIDE = WarpLayout<H>::WIDE;
-    constexpr int NDW = WarpLayout<H>::NDW, NPW = WarpLayout<H>::NPW, PRODUCER_WARP = WarpLayout<H>::PRODUCER_WARP;
-    constexpr int S1_THREADS = WarpLayout<H>::THREADS;
-    constexpr int GS = NCW / H;                                     // groups per ring stage
-    constexpr int TS = H * 32;                                      // bytes per token row (all heads)
-    constexpr uint32_t SWZ = H >= 4 ? 0x70u : 0u;                   // the code planes are staged through swizzled tensor maps
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // swizzle atoms are 1 KB: align the ring by hand (the launch adds 1 KB of slack)
-    uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int cta = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int NS = p.nstages;
-    const int k_out = KOUT >= 0 ? KOUT : p.k_out;
-    const long long wait_limit = (p.abl & ABL_TEST_STALL) ? TEST_WAIT_LIMIT_CYCLES : WAIT_LIMIT_CYCLES;
-
-    // ---- shared memory carve-up ----
-    uint8_t *s_stage = smem;                                            // nstages * stage_bytes
-    uint8_t *s_tiles = s_stage + NS * p.stage_bytes;                    // NCW * DT_BYTES
-    float *s_lut = reinterpret_cast<float *>(s_tiles + NCW * DT_BYTES);
-    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_lut + 16);         // full[], empty[], tile_full[NCW], tile_empty[NCW][], tile_rows[NCW]
-    CopyDesc *s_desc = reinterpret_cast<CopyDesc *>(s_bar + 2 * MAX_STAGES + (2 + MAX_STAGES) * NCW);
-    const uint32_t bar_full = smem_u32(s_bar), bar_empty = smem_u32(s_bar + MAX_STAGES);
-    const uint32_t bar_tfull = smem_u32(s_bar + 2 * MAX_STAGES), bar_tempty = smem_u32(s_bar + 2 * MAX_STAGES + NCW);
-    const uint32_t bar_trows = smem_u32(s_bar + 2 * MAX_STAGES + (1 + MAX_STAGES) * NCW);
-
-    // ---- prologue: LUT, barriers and copy descriptors.  None of it depends on an earlier kernel, so it runs while the
-    //      kernel before this one in the stream drains (the grid may start then, see the wait below). ----
-    // the first tensor-map copy otherwise pays for fetching its descriptor
-    if (SWZ != 0 && threadIdx.x == S1_THREADS - 32) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_k)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_v)) : "memory");
-    }
-    if (threadIdx.x < 16) {
-        const int c = threadIdx.x;
-        const int mi = ((c >> 1) & 3) * 2 + (c & 1);                    // exp*2 + mant
-        const float mag = mi == 0 ? 0.f : (mi == 1 ? .5f : (float)(2 + (mi & 1)) * (float)(1 << (mi >> 1)) * 0.25f);
-        s_lut[c] = (c & 8) ? -mag : mag;
-    }
-    {
-        // one barrier per thread (56 of them: a single thread's serial inits were a microsecond of every launch)
-        const int t = (int)threadIdx.x - 32;
-        constexpr int NB_RING = 2 * MAX_STAGES, NB_ALL = NB_RING + (2 + MAX_STAGES) * NCW;
-        if (t >= 0 && t < NB_ALL) {
-            uint32_t count;
-            if (t < MAX_STAGES) count = NPW;                                   // full[]: each producer warp announces its own copies
-            else if (t < NB_RING) count = 3 * NCW;                             // empty[]: 8 MMA warps + 16 tile halves
-            else if (t < NB_RING + NCW) count = 2;                             // tile_full[]: the two halves' deltas scattered
-            else if (t < NB_RING + NCW + MAX_STAGES * NCW) count = 1;          // tile_empty[][]
-            else count = 2;                                                    // tile_rows[]: the two halves' rows written
-            mbar_init(bar_full + 8 * t, count);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-    }
-    const int cpg = 4 * p.ppg + 6;                                      // copies per group
-    const int ncopies = GS * cpg;
-    {
-        // Copy roles (group-in-stage, plane) are tabulated once; the producer's loop body is then one
-        // descriptor load, one multiply-add and one copy per role, with no divergent paths, because that
-        // single warp's issue latency bounds how fast stages refill.
-        const uint32_t page_b = (uint32_t)p.ps * H;                     // (token, head) rows per page
-        const int c = (int)threadIdx.x - 64;                            // threads 64.. build one descriptor each
-        if (c >= 0 && c < ncopies) {
-            CopyDesc d;
-            d.src = nullptr; d.unit = 0; d.dst = 0; d.tbase = 0; d.tmul = 0; d.gi = 0; d.tok0 = 0;
-            const int gi = c / cpg, ci = c - gi * cpg;
-            d.gi = gi;
-            const uint32_t gbo = (uint32_t)gi * p.gb_bytes;
-            if (ci < 4 * p.ppg) {
-                const int pg = ci >> 2, plane = ci & 3;
-                const uint32_t w = plane < 2 ? 32u : (plane == 2 ? 4u : 8u);
-                d.src = plane == 0 ? p.k_base : (plane == 1 ? p.v_main : (plane == 2 ? p.v_scale : p.v_zp));
-                d.unit = page_b * w;
-                d.dst = gbo + (plane == 0 ? 0u : (plane == 1 ? (uint32_t)p.o_vm : (plane == 2 ? (uint32_t)p.o_vs : (uint32_t)p.o_vz)))
-                      + (uint32_t)pg * page_b * w;
-                d.tbase = pg; d.tmul = p.ppg; d.tok0 = pg * p.ps;
-                if (SWZ != 0 && plane < 2) d.gi |= (plane + 1) << 8;
-            } else {
-                const int gp = ci - 4 * p.ppg;
-                const bool on = gp < 2 || (k_out > 0 && (gp >= 4 || p.use_map));
-                if (on) {
-                    const uint32_t w = gp == 0 ? 128u : (gp == 4 ? 128u * p.nbi : (gp == 5 ? 128u * p.nb : 256u));
-                    d.src = gp == 0 ? p.k_scale : (gp == 1 ? p.k_zp : (gp == 2 ? p.k_ms : (gp == 3 ? p.k_mc : (gp == 4 ? p.k_obmp : p.k_oval))));
-                    d.unit = (uint32_t)H * w;
-                    d.dst = gbo + (uint32_t)(gp == 0 ? p.o_ks : (gp == 1 ? p.o_kz : (gp == 2 ? p.o_ms : (gp == 3 ? p.o_mc : (gp == 4 ? p.o_bm : p.o_ov)))));
-                    d.tbase = 0; d.tmul = 0;                            // tmul 0: the index is a group slot
-                }
-            }
-            s_desc[c] = d;
-        }
-    }
-    __syncthreads();
-    // Nothing an earlier kernel may have written - lengths, tables, the query, the planes, the split workspace a
-    // previous layer's combine still reads - is touched before this returns.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // Stage 2 is launched as a programmatic dependent: it may start its own prologue (residual-row
-    // logits, which do not depend on this kernel but may depend on the one before it: hence after the wait)
-    // as soon as SM resources free up, and waits for this grid to finish before it reads the split partials.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
-    Piece pc;
-    PieceWalk walk;
-    const SharePlan plan = share_plan(p.b_seq_len, p.B, p.S, p.ncta, p.waves, lane);
-    if (!first_piece<GS>(pc, walk, p, plan, cta, lane)) return;
-
-    const int g = lane >> 2, j = lane & 3;
-    const float LOG2E = 1.4426950408889634f;
-    const bool no_outlier = (p.abl & ABL_NO_OUTLIER) != 0;
-
-    // ---- one stage of the ring: look up its page ids and group slots, announce its bytes, issue its copies (producer
-    //      warps).  The lookup of a stage runs while the stage before it is still on its way, so that no copy waits for its
-    //      table entry; each lane leaves what it finds in s_idx for itself. ----
-    Piece *s_piece = reinterpret_cast<Piece *>(s_desc + ncopies);
-    int32_t *s_idx = reinterpret_cast<int32_t *>(s_piece + MAX_PIECES);
-    auto whole_stage = [&](const Piece &q, int it) { return 32 * GS * (it + 1 - q.it0) <= q.ntok; };
-    auto copy_on = [&](const CopyDesc &d, const Piece &q, int it) __attribute__((always_inline)) {
-        const int lg = (it - q.it0) * GS + (d.gi & 0xFF);
-        return d.unit != 0 && lg < q.ng && 32 * lg + d.tok0 < q.ntok;
-    };
-    auto lookup_stage = [&](const Piece &q, int it, int nshare, int share) __attribute__((always_inline)) {
-        const int64_t g0 = (int64_t)p.seg_group_base + q.g0 + (it - q.it0) * GS;
-#pragma unroll 1
-        for (int ci = lane * nshare + share; ci < ncopies; ci += 32 * nshare) {
-            const CopyDesc d = s_desc[ci];
-            if (!copy_on(d, q, it)) continue;
-            const bool page = d.tmul != 0;                          // tmul 0: the index is a group slot
-            const int64_t at = page ? (int64_t)q.b * p.r2t_sb + (g0 + (d.gi & 0xFF)) * d.tmul + d.tbase : (int64_t)q.b * p.r2g_sb + g0 + (d.gi & 0xFF);
-            int64_t x = load_index(page ? p.r2t : p.r2g, p.tbl64, at);
-            if (x < 0 || x >= (page ? p.num_pages : p.num_slots)) { or_status(p.status, page ? OMMX_ST_BAD_PAGE : OMMX_ST_BAD_GROUP); x = 0; }
-            s_idx[ci] = (int)x;
-        }
-    };
-    // `nshare` warps split the copies of a stage, this one taking share `share`; with `announce_all` it announces the bytes
-    // of all of them (the others then announce nothing), else its own.
-    // (A copy of another warp may land before the announcement: the phase cannot complete without the announcing arrival,
-    // and the transaction count may run negative meanwhile.)
-    auto stage_bytes_of = [&](const Piece &q, int it, bool whole, int first, int step) __attribute__((always_inline)) {
-        uint32_t mine = 0;
-#pragma unroll 1
-        for (int ci = first; ci < ncopies; ci += step) {
-            const CopyDesc d = s_desc[ci];
-            if (whole || copy_on(d, q, it)) mine += d.unit;
-        }
-        return __reduce_add_sync(0xFFFFFFFFu, mine);
-    };
-    auto issue_stage = [&](const Piece &q, int it, int nshare, int share, uint32_t announce) __attribute__((always_inline)) {
-        const int s = ring_slot(it, NS);
-        if (announce) {
-            if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, announce);
-            __syncwarp();
-        }
-        const uint32_t sbase = smem_u32(s_stage + (size_t)s * p.stage_bytes);
-#pragma unroll 1
-        for (int ci = lane * nshare + share; ci < ncopies; ci += 32 * nshare) {
-            const CopyDesc d = s_desc[ci];
-            const int kind = d.gi >> 8;
-            if (copy_on(d, q, it) && !((p.abl & ABL_TEST_STALL) && it == 1)) {
-                const int idx = s_idx[ci];
-                if (kind == 0) bulk_g2s(sbase + d.dst, d.src + (int64_t)idx * d.unit, d.unit, bar_full + 8 * s);
-                else tma_2d_g2s(sbase + d.dst, kind == 1 ? &p.tmap_k : &p.tmap_v, 0, idx * p.rows_per_page, bar_full + 8 * s);
-            }
-        }
-    };
-    // The first ring fill is on every CTA's critical path: it goes out before the register budgets are resized.
-    // A warp issues a bulk copy only about every 60 cycles and different warps overlap, so in the narrow layout the three
-    // decode warps of the producer's warpgroup (idle until the data lands) take a quarter of the first fill each.
-    if (warp >= PRODUCER_WARP - (WIDE ? 0 : 3)) {
-        constexpr int W0 = PRODUCER_WARP - (WIDE ? 0 : 3);
-        lookup_stage(pc, 0, 4, warp - W0);
-        const uint32_t bytes = WIDE ? stage_bytes_of(pc, 0, false, lane * NPW + warp - W0, 32 * NPW)
-                                    : (warp == PRODUCER_WARP ? stage_bytes_of(pc, 0, false, lane, 32) : 0u);
-        issue_stage(pc, 0, 4, warp - W0, bytes);
-    }
-
-    if (warp == PRODUCER_WARP) {
-        int n = 0;
-        for (bool more = true; more; ++n) {
-            Piece cur = pc;
-            more = next_piece<GS>(pc, walk, p, plan);
-            if (more && n + 1 == MAX_PIECES) {                       // the host sizes the grid so that this cannot be
-                if (lane == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
-                more = false;
-            }
-            cur.more = more;
-            if (lane == 0) s_piece[n] = cur;
-        }
-    }
-    __syncthreads();
-    int pi = 0;
-    pc = s_piece[0];
-    auto step_piece = [&]() __attribute__((always_inline)) {
-        if (!pc.more) return false;
-        pc = s_piece[++pi];
-        return true;
-    };
-
-    // ---- one work item of the decode role: half hf of the sidecar tile of (iteration it, unit) ----
-    // Channel 64 w + 16 j + 8 x + i (i = 0..7) sits in member x of the pair in register 8 w + i of lane group j in the MMAs
-    // below, i.e. in column byte 128 w + 16 i + 4 j + 2 x of the delta rows.  This half has w = hf, this lane channels
-    // 2 lane and 2 lane + 1 of it: j = dj, x = dh, i = 2 da and 2 da + 1.
-    const int da = lane & 3, dh = (lane >> 2) & 1, dj = lane >> 3;
-    // 4^-slot of those two channels' code fields, fp16
-    const uint32_t slot_scale = da == 0 ? 0x34003C00u : (da == 1 ? 0x24002C00u : (da == 2 ? 0x3C001C00u : 0x2C003400u));
-    // Build the sidecar tile of a unit between two uses by its MMA warp.  A tile is built in two
-    // halves by two warps at once, because the MMA warp of the unit waits for it: half hf takes 64 of the
-    // K channels (delta columns, scale factors) and V tokens 16hf..16hf+15 (factors, zero-points).
-    // Returns false when a bounded wait ran out.
-    auto decode_item = [&](const Piece &pc, const int n) __attribute__((always_inline)) -> bool {
-        const int it = n / (2 * NCW), unit = (n >> 1) % NCW, hf = n & 1;
-        const int h = unit % H, gsel = unit / H;
-        uint8_t *tile = s_tiles + unit * DT_BYTES;
-        const int s = ring_slot(it, NS);
-        const uint32_t ph = ring_phase(it, NS);
-        if (!mbar_wait(bar_full + 8 * s, ph, wait_limit)) {
-            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
-            return false;
-        }
-        const int lg = (it - pc.it0) * GS + gsel;                 // local group of this unit
-        const bool active = lg < pc.ng && !(p.abl & ABL_NO_COMPUTE);
-        const uint8_t *gb = s_stage + (size_t)s * p.stage_bytes + (size_t)gsel * p.gb_bytes;
-        const int d0 = 64 * hf + 2 * lane;                       // first of this lane's two channels
-        const bool splice = k_out > 0 && !no_outlier;
-        // ---- everything that only reads the stage comes before the wait for the tile, which the MMA warps make a decode warp
-        //      wait for (a sixth of its time): the parameters of both channels, the K and V factors, V zero-points ----
-        bool clamped_any = false;
-        uint32_t e2 = 0, z2 = 0, kf = 0, vf = 0, zt = 0, ms2 = 0, mc2 = 0;
-        uint2 bm2 = make_uint2(0u, 0u);
-        uint32_t st[2] = {0, 0}, sth[2] = {0, 0};                // nibble stream of each channel: outliers 0..7, 8..15
-        const int vtk = 16 * hf + 2 * (lane & 7), vcg = lane >> 3;   // V side: lane = (pair of tokens, scale group)
-        if (active) {
-            e2 = *reinterpret_cast<const uint16_t *>(gb + p.o_ks + h * 128 + d0);
-            z2 = *reinterpret_cast<const uint32_t *>(gb + p.o_kz + h * 256 + 2 * d0);
-            uint32_t v0 = 0x80u, v1 = 0x80u, y0 = 0u, y1 = 0u;   // exponent -128 -> factor 0
-            const uint8_t *vs = gb + p.o_vs + (vtk * H + h) * 4 + vcg, *vz = gb + p.o_vz + (vtk * H + h) * 8 + 2 * vcg;
-            if (32 * lg + vtk < pc.ntok) { v0 = vs[0]; y0 = *reinterpret_cast<const uint16_t *>(vz); }
-            if (32 * lg + vtk + 1 < pc.ntok) { v1 = vs[4 * H]; y1 = *reinterpret_cast<const uint16_t *>(vz + 8 * H); }
-            if (splice) {
-                if (p.use_map) {
-                    ms2 = *reinterpret_cast<const uint32_t *>(gb + p.o_ms + h * 256 + 2 * d0);
-                    mc2 = *reinterpret_cast<const uint32_t *>(gb + p.o_mc + h * 256 + 2 * d0);
-                }
-                if (!p.idx7) {
-                    bm2 = *reinterpret_cast<const uint2 *>(gb + p.o_bm + h * 512 + 4 * d0);
-                } else {
-                    // relidx7 (attention/codec.py:91-130 of the reference): k ascending token positions, 7 bits each,
-                    // LSB first; the outlier set as a bitmask again, the value stream is shared with that encoding
-                    uint32_t m2[2];
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const uint8_t *ip = gb + p.o_bm + (h * 128 + d0 + c) * p.nbi;
-                        uint32_t w[5] = {0u, 0u, 0u, 0u, 0u};
-                        for (int i = 0; i < p.nbi; ++i) w[i >> 2] |= (uint32_t)ip[i] << (8 * (i & 3));
-                        uint32_t bits = 0u;
-                        for (int r = 0; r < k_out; ++r) {
-                            const int bp = 7 * r;
-                            const uint32_t f = __funnelshift_r(w[bp >> 5], w[(bp >> 5) + 1], bp & 31) & 0x7Fu;
-                            if (f > 31u) or_status(p.status, OMMX_ST_BAD_GROUP);
-                            else bits |= 1u << f;
-                        }
-                        m2[c] = bits;
-                    }
-                    bm2 = make_uint2(m2[0], m2[1]);
-                }
-                const int nb = KOUT >= 0 ? (KOUT + 1) / 2 : p.nb;
-                const uint8_t *ov = gb + p.o_ov + (h * 128 + d0) * nb;          // 2*nb bytes, 2-byte aligned
-                if (nb == 3) {
-                    const uint32_t w0 = reinterpret_cast<const uint16_t *>(ov)[0], w1 = reinterpret_cast<const uint16_t *>(ov)[1],
-                                   w2 = reinterpret_cast<const uint16_t *>(ov)[2];
-                    st[0] = w0 | ((w1 & 0xFFu) << 16);
-                    st[1] = (w1 >> 8) | (w2 << 8);
-                } else if (nb == 4) {
-                    const uint2 w = *reinterpret_cast<const uint2 *>(ov);
-                    st[0] = w.x; st[1] = w.y;
-                } else if (nb == 2) {
-                    const uint32_t w = *reinterpret_cast<const uint32_t *>(ov);
-                    st[0] = w & 0xFFFFu; st[1] = w >> 16;
-                } else if (nb > 4) {
-                    // 9..16 outliers: the two channels' streams are 2*nb bytes back to back; read them as
-                    // 16-bit pieces into a 128-bit little-endian window and cut it at bit 8*nb
-                    uint32_t w[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (i < nb) w[i >> 1] |= (uint32_t) reinterpret_cast<const uint16_t *>(ov)[i] << (16 * (i & 1));
-                    const int sh = nb > 4 ? 8 * (nb - 4) : 8;        // 8..32 bits of a stream lie above its first word
-                    const uint32_t hmask = sh == 32 ? 0xFFFFFFFFu : ((1u << sh) - 1u);
-                    st[0] = w[0]; sth[0] = w[1] & hmask;
-                    if (sh == 32) { st[1] = w[2]; sth[1] = w[3]; }
-                    else { st[1] = __funnelshift_r(w[1], w[2], sh); sth[1] = __funnelshift_r(w[2], w[3], sh) & hmask; }
-                } else {
-                    const uint32_t w = *reinterpret_cast<const uint16_t *>(ov);
-                    st[0] = w & 0xFFu; st[1] = w >> 8;
-                }
-            }
-            bool cl0, cl1, cl2, cl3;
-            const uint32_t k0 = pow2_f16_bits(max((int)(int8_t)e2, -126), cl0), k1 = pow2_f16_bits(max((int)(int8_t)(e2 >> 8), -126), cl1);
-            kf = hmul2_f16(k0 | (k1 << 16), slot_scale);         // * 4^-slot: exact, subnormals included
-            const uint32_t f0 = pow2_f16_bits((int)(int8_t)v0, cl2), f1 = pow2_f16_bits((int)(int8_t)v1, cl3);
-            vf = f0 | (f1 << 16);
-            zt = pack_f16x2_sat(bf16_bits_to_f32(y0), bf16_bits_to_f32(y1));
-            clamped_any = cl0 || cl1 || cl2 || cl3;
-        }
-        // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
-        // run up to NS groups ahead and the tiles of one unit are built by different warps, so
-        // "tile k was read" events rotate over NS barriers per unit (barrier k % NS, phase
-        // k / NS): the newest event a waiter can be missing is then always the one it waits
-        // for, never an older phase of the same parity.  A unit without a group in this stage goes
-        // through the same hand-overs with nothing in them.
-        if (it > 0 && !mbar_wait(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it - 1, NS)), ring_phase(it - 1, NS), wait_limit)) {
-            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
-            return false;
-        }
-        if (active) {
-            // ---- first the rows the code MMAs and the softmax read (K factors, V factors and zero-points): the MMA warp
-            //      starts on them while the deltas are scattered ----
-            uint8_t *row = tile + ROW_KF * DT_STRIDE + 128 * hf + 64 * (da >> 1) + 16 * dj + 8 * (da & 1) + 2 * dh;
-            *reinterpret_cast<uint16_t *>(row) = (uint16_t)kf;
-            *reinterpret_cast<uint16_t *>(row + 4) = (uint16_t)(kf >> 16);
-            const int copy = it & 1;
-            *reinterpret_cast<uint32_t *>(tile + (ROW_VF + copy) * DT_STRIDE + 64 * vcg + 16 * (lane & 3) + 8 * hf + 4 * ((lane >> 2) & 1)) = vf;
-            *reinterpret_cast<uint32_t *>(tile + (ROW_ZT + copy) * DT_STRIDE + 2 * vtk + ZT_STRIDE * vcg) = zt;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_trows + 8 * unit);
-            // ---- then the outlier deltas of this half's columns ----
-            if (splice) {
-                // clear this half's columns of token rows 0..31 (128 bytes per row)
-#pragma unroll
-                for (int k2 = 0; k2 < 8; ++k2)
-                    *reinterpret_cast<uint4 *>(tile + (4 * k2 + (lane >> 3)) * DT_STRIDE + 128 * hf + 16 * (lane & 7)) = make_uint4(0, 0, 0, 0);
-                __syncwarp();                                        // the cleared rows before any delta lands in them
-                const uint32_t bmv[2] = {bm2.x, bm2.y};
-                // The code byte holding this lane's channels, row pz: byte pz*TS + h*32 + d0/4 of the (1 KB aligned)
-                // k_base block, with the 16-byte chunk bits XOR-ed by the row's swizzle term.  h*32 + d0/4 splits
-                // into a part above bit 7 (added to the row) and a part below (the XOR operand, swizzle term of the former
-                // included).
-                const uint8_t *k_hi = gb + (h >> 2) * 128;
-                const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2)) ^ (((uint32_t)(h >> 2) * 16u) & SWZ);
-                auto code_byte = [&](uint32_t pz) -> uint32_t {
-                    return k_hi[pz * TS + (k_lo ^ (((pz * TS) >> 3) & SWZ))];
-                };
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int e = max((int)(int8_t)(e2 >> (8 * c)), -126);
-                    const float sc = __uint_as_float((uint32_t)(e + 127) << 23);
-                    const float zp = bf16_bits_to_f32(c ? (z2 >> 16) : (z2 & 0xFFFFu));
-                    // delta between the outlier value and the base value it replaces: lvl * A + Bc - code * sc
-                    float A = sc, Bc = 0.f;                     // shared map: lvl*s + zp - (code*s + zp)
-                    if (p.use_map) {
-                        const float ms = bf16_bits_to_f32(c ? (ms2 >> 16) : (ms2 & 0xFFFFu));
-                        const float mc = bf16_bits_to_f32(c ? (mc2 >> 16) : (mc2 & 0xFFFFu));
-                        A = __fdividef(1.f, ms);
-                        Bc = mc - zp;
-                    }
-                    uint32_t bits = bmv[c];
-                    const uint32_t stream = st[c], stream_hi = sth[c];
-                    (void)stream_hi;
-                    const int fsh = 2 * ((d0 & 3) + c);          // bit position of the channel's code in its byte
-                    uint8_t *col = tile + 128 * hf + 32 * da + 16 * c + 4 * dj + 2 * dh;
-                    if constexpr (KOUT > 0 && KOUT % 2 == 0) {
-                        if (__popc(bits) == KOUT) {
-                            // The code enters as the fraction of 1 + code/4, whose bits an AND and an OR make, so that 4 * sc moves to
-                            // the constant: lvl * A + (Bc + 4 sc) - (1 + code/4) * 4 sc.
-                            const float Bq = fmaf(4.f, sc, Bc), Sq = -4.f * sc;
-                            const int sh = 21 - fsh;              // moves the code to the top of the mantissa
-                            // Two passes: all gathers (bit walk, base-code byte) first, then the arithmetic and the
-                            // stores.  In one pass every load would have to follow the previous outlier's store in
-                            // program order (shared memory may alias), i.e. KOUT load round trips in a row.
-                            uint32_t pzs[KOUT], cbs[KOUT];
-#pragma unroll
-                            for (int r = KOUT - 1; r >= 0; --r) {
-                                const uint32_t pz = 31 - __clz(bits);
-                                bits ^= 1u << pz;
-                                pzs[r] = pz;
-                                cbs[r] = code_byte(pz);
-                            }
-#pragma unroll
-                            for (int r = 0; r < KOUT; r += 2) {
-                                const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
-                                const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
-                                const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
-                                const float v0 = __uint_as_float(((cbs[r] << sh) & 0x600000u) | 0x3F800000u);
-                                const float v1 = __uint_as_float(((cbs[r + 1] << sh) & 0x600000u) | 0x3F800000u);
-                                const uint32_t X = f16x2_of_bf16_rounded(fmaf(v0, Sq, fmaf(lvf.x, A, Bq)), fmaf(v1, Sq, fmaf(lvf.y, A, Bq)));
-                                *reinterpret_cast<uint16_t *>(col + pzs[r] * DT_STRIDE) = (uint16_t)X;
-                                *reinterpret_cast<uint16_t *>(col + pzs[r + 1] * DT_STRIDE) = (uint16_t)(X >> 16);
-                            }
-                        } else {
-                            or_status(p.status, OMMX_ST_BAD_GROUP);   // bitmask and value stream disagree
-                        }
-                    } else {
-                        // any other k: one pass at run time
-                        int r = __popc(bits) - 1;
-                        while (bits) {
-                            const uint32_t pz = 31 - __clz(bits);
-                            bits ^= 1u << pz;
-                            const uint32_t nib = ((r < 8 ? stream : stream_hi) >> (4 * (r & 7))) & 0xFu;
-                            --r;
-                            const float cf = (float)((code_byte(pz) >> fsh) & 3u);
-                            const float X = fmaf(cf, -sc, fmaf(s_lut[nib], A, Bc));
-                            *reinterpret_cast<uint16_t *>(col + pz * DT_STRIDE) = (uint16_t)f16x2_of_bf16_rounded(X, X);
-                        }
-                    }
-                }
-            }
-            if (clamped_any) or_status(p.status, OMMX_ST_SCALE_RANGE);
-        } else if (lane == 0) {
-            mbar_arrive(bar_trows + 8 * unit);
-        }
-        __syncwarp();
-        if (lane == 0) {
-            mbar_arrive(bar_tfull + 8 * unit);
-            mbar_arrive(bar_empty + 8 * s);
-        }
-        return true;
-    };
-
-    // ---- roles; each branch starts by resizing its warpgroups' register budget and never rejoins ----
-    if constexpr (WIDE) {
-        if (warp >= PRODUCER_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_PRODUCER ";");
-        else if (warp >= NCW) asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_DECODE ";");
-    } else {
-        if (warp >= NCW) asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_DECODE ";");
-    }
-    bool producer_alive = true;
-    if (warp >= PRODUCER_WARP) {
-        // =========================== producer warp(s) ===========================
-        const int pw = warp - PRODUCER_WARP;
-        const uint32_t full_bytes = stage_bytes_of(pc, 0, true, lane * NPW + pw, 32 * NPW);   // this warp's share of a stage of whole groups
-        for (int it = 1;; ++it) {
-            if (it >= pc.it1 && !step_piece()) break;
-            lookup_stage(pc, it, NPW, pw);
-            const uint32_t bytes = whole_stage(pc, it) ? full_bytes : stage_bytes_of(pc, it, false, lane * NPW + pw, 32 * NPW);
-            // the first NS fills find their slots fresh
-            if (it >= NS && !mbar_wait(bar_empty + 8 * ring_slot(it, NS), ring_phase(it, NS) ^ 1, wait_limit)) {
-                if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
-                producer_alive = false;
-                break;
-            }
-            issue_stage(pc, it, NPW, pw, bytes);
-        }
-        if constexpr (WIDE) return;
-        // Narrow layout: with every stage on its way this warp has nothing left to do, while the 15 decode warps share
-        // 16 items per iteration: it joins them below for the very last item, so that the last iteration's 16 halves are
-        // built side by side.
-    }
-
-    // =========================== decode + MMA warps ===========================
-    // MMA warp w owns unit w = (group-in-stage, kv head) and its softmax state.  The decode warps are
-    // stateless: work item number n goes to decode warp n % NDW (narrow layout: except the last one, the producer's).
-    if (warp >= NCW) {
-        // =========================== decode warps (narrow layout: and the producer, once it is done) ===========================
-        const int dw = warp - NCW;
-        const bool is_producer = !WIDE && warp == PRODUCER_WARP;
-        if (!is_producer) {
-            if (dw < NCW) {           // the first to touch tile dw clears it once (unused rows stay zero)
-                uint8_t *t0p = s_tiles + dw * DT_BYTES;
-                for (int i = lane; i < DT_BYTES / 4; i += 32) reinterpret_cast<uint32_t *>(t0p)[i] = 0u;
-            }
-            // every tile is cleared before any half of it is written; the narrow layout's producer learns of it without
-            // being waited for
-            asm volatile("bar.sync 1, %0;" ::"n"(NDW * 32) : "memory");
-            if constexpr (!WIDE) asm volatile("bar.arrive 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
-        } else {
-            asm volatile("bar.sync 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
-            if (!producer_alive || pc.more) return;
-        }
-        // the producer takes the very last item, when this CTA's pieces end with one that is known to be the last
-        for (int n = is_producer ? pc.it1 * 2 * NCW - 1 : dw;; n += NDW) {
-            const int it = n / (2 * NCW);
-            while (it >= pc.it1)
-                if (!step_piece()) return;
-            if (!WIDE && !is_producer && !pc.more && n == pc.it1 * 2 * NCW - 1) return;
-            if (!decode_item(pc, n)) return;
-        }
-    }
-
-    // =========================== MMA warps ===========================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 " OMMX_REGS_MMA ";");
-    const int unit = warp;
-    const int h = unit % H, gsel = unit / H;
-    const uint8_t *tile = s_tiles + unit * DT_BYTES;
-    const uint32_t tile_s = smem_u32(tile);
-    // Column n = g of every MMA is query head g of this kv head.
-    const bool head_ok = g < p.gqa;
-    // per-lane fragment addresses inside the sidecar tile
-    const uint32_t a_delta = tile_s + ((lane & 7) + 8 * ((lane >> 3) & 1)) * DT_STRIDE + 16 * (lane >> 4);
-    const uint8_t *p_kf = tile + ROW_KF * DT_STRIDE + 16 * j;       // 16-byte piece q2 of lane group j at 64 q2 + 16 j: one line for all four
-    // V codes: row r of a 16x16 byte matrix is token sigma(r) = 2 (r / 4) + (r / 2) % 2 + 8 (r % 2) of its 16, so that the four
-    // bytes a lane receives are tokens 2j, 8 + 2j, 2j + 1, 9 + 2j: bytes 0 and 2 sit in the two halves of a register as they
-    // are, bytes 1 and 3 after a shift.
-    const uint32_t v_off = swz128((uint32_t)((2 * ((lane & 15) >> 2) + ((lane >> 1) & 1) + 8 * (lane & 1)) * TS + h * 32 + 16 * (lane >> 4)), SWZ);
-    static_assert(SWZ == 0 || (16 * TS) % 1024 == 0, "the second half of the tokens has the same swizzle");
-    const bool do_k = !(p.abl & ABL_NO_K), do_v = !(p.abl & ABL_NO_V);
-    const bool has_delta = !(k_out == 0 || no_outlier);
-
-    bool gave_up = false;                        // a wait ran out: no more groups, but every piece still goes through its epilogue
-    do {
-    // B fragments of q.  QR: raw bf16, registers 4v..4v+3 hold channels 32v + 8j .. + 7 (zero-point MMAs).  QP: fp16 of
-    // bf16(q * sm_scale), register r = 8w + i holds channels (64w + 16j + i, + 8), the pair a code word yields in one AND (code
-    // and delta MMAs).
-    uint32_t QR[16], QP[16];
-    {
-        const uint16_t *qrow = reinterpret_cast<const uint16_t *>(p.q + (int64_t)pc.b * p.q_sb + (int64_t)(h * p.gqa + (head_ok ? g : 0)) * p.q_sh);
-        auto eight = [&](const uint16_t *q8, uint32_t (&w)[4]) __attribute__((always_inline)) {
-            if (p.q_vec_ok) {
-                const uint4 t = __ldg(reinterpret_cast<const uint4 *>(q8));
-                w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
-            } else {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) w[v] = (uint32_t)__ldg(q8 + 2 * v) | ((uint32_t)__ldg(q8 + 2 * v + 1) << 16);
-            }
-        };
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            uint32_t w[4];
-            eight(qrow + 32 * v + 8 * j, w);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) QR[4 * v + i] = head_ok ? w[i] : 0u;
-        }
-        auto scaled = [&](uint32_t b16) { return bf16_round_f32(bf16_bits_to_f32(b16 & 0xFFFFu) * p.sm_scale); };
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-            uint32_t lo[4], hi[4];
-            eight(qrow + 64 * w + 16 * j, lo);
-            eight(qrow + 64 * w + 16 * j + 8, hi);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                QP[8 * w + i] = head_ok ? pack_f16x2(scaled(lo[i >> 1] >> (16 * (i & 1))), scaled(hi[i >> 1] >> (16 * (i & 1)))) : 0u;
-        }
-    }
-    // ---- online softmax state of heads 2j and 2j+1 (the two columns this lane holds) ----
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-    // acc[2*cg + u]: rows = channels 32cg + 4g + u (regs 0,1) and 32cg + 4g + 2 + u (regs 2,3), columns = heads
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f; }
-    float accz[4] = {0.f, 0.f, 0.f, 0.f};        // rows = V scale groups: sum_t vz[t][cg] * P[t][head]
-
-    for (int it = pc.it0; it < pc.it1 && !gave_up; ++it) {
-        const int s = ring_slot(it, NS);
-        const uint32_t ph = ring_phase(it, NS);
-        const int lg = (it - pc.it0) * GS + gsel;                    // local group of this warp
-        const bool active = lg < pc.ng && !(p.abl & ABL_NO_COMPUTE);
-        if (!mbar_wait(bar_full + 8 * s, ph, wait_limit)) {
-            gave_up = true;
-            break;
-        }
-        if (active) {
-            uint8_t *gb = s_stage + (size_t)s * p.stage_bytes + (size_t)gsel * p.gb_bytes;
-            const uint32_t v_addr = smem_u32(gb + p.o_vm) + v_off;  // v_main region of the group (1 KB aligned)
-
-            // ======================= logits =======================
-            // code words of this lane's four token rows (tokens 8*nt + g), channels 16j..16j+15 of either half
-            uint2 kw[4];
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                kw[nt] = make_uint2(0u, 0u);
-                if (do_k) {
-                    kw[nt].x = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 4 * j), SWZ));
-                    kw[nt].y = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 16 + 4 * j), SWZ));
-                }
-            }
-            // The unit's sidecar tile arrives in two steps: first the factor and zero-point rows, then the outlier
-            // deltas.  The code MMAs run on the first, while the decode warps still scatter the deltas.
-            if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
-                gave_up = true;
-                break;
-            }
-            float Sc[2][4], Sd[2][4];
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) { Sc[mt][0] = Sc[mt][1] = Sc[mt][2] = Sc[mt][3] = 0.f; Sd[mt][0] = Sd[mt][1] = Sd[mt][2] = Sd[mt][3] = 0.f; }
-            // Two accumulators take turns, so that neighbours in the instruction stream never wait on each other
-            // (the asm statements keep their order, so the order written here is the order issued).
-#pragma unroll
-            for (int q2 = 0; q2 < 4; ++q2) {
-                const uint4 f = *reinterpret_cast<const uint4 *>(p_kf + 64 * q2);      // two k-steps' factor pairs
-#pragma unroll
-                for (int q = 2 * q2; q < 2 * q2 + 2; ++q) {
-                    const int wi = q >> 2, i0 = 2 * (q & 3);
-                    const uint32_t b0 = hmul2_f16(QP[2 * q], q & 1 ? f.z : f.x), b1 = hmul2_f16(QP[2 * q + 1], q & 1 ? f.w : f.y);
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) {
-                        const uint32_t wlo = wi ? kw[2 * mt].y : kw[2 * mt].x, whi = wi ? kw[2 * mt + 1].y : kw[2 * mt + 1].x;
-                        mma_f16(Sc[mt], code_pair(wlo, i0), code_pair(whi, i0), code_pair(wlo, i0 + 1), code_pair(whi, i0 + 1), b0, b1);
-                    }
-                }
-            }
-            // q.zp of heads 2j and 2j+1: exact bf16 products of the raw query with the zero-points, summed in fp32, every row
-            // of the A operand being the zero-point row.  It needs no tile, so it stands where this warp may have to wait for the deltas.
-            float Z0[4] = {0.f, 0.f, 0.f, 0.f}, Z1[4] = {0.f, 0.f, 0.f, 0.f};
-            {
-                const uint8_t *zrow = gb + p.o_kz + h * 256 + 16 * j;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const uint4 z = *reinterpret_cast<const uint4 *>(zrow + 64 * v);
-                    mma_bf16(Z0, z.x, z.x, z.y, z.y, QR[4 * v], QR[4 * v + 1]);
-                    mma_bf16(Z1, z.z, z.z, z.w, z.w, QR[4 * v + 2], QR[4 * v + 3]);
-                }
-            }
-            const float Sz[2] = {(Z0[0] + Z1[0]) * p.sm_scale, (Z0[1] + Z1[1]) * p.sm_scale};
-            if (has_delta) {
-                if (!mbar_wait(bar_tfull + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
-                    gave_up = true;
-                    break;
-                }
-                uint32_t d0f[4], d1f[4];                         // delta fragments of m-tile 0 / 1
-                ldsm_x4(a_delta, d0f[0], d0f[1], d0f[2], d0f[3]);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    ldsm_x4(a_delta + 16 * DT_STRIDE + 32 * q, d1f[0], d1f[1], d1f[2], d1f[3]);
-                    mma_f16(Sd[0], d0f[0], d0f[1], d0f[2], d0f[3], QP[2 * q], QP[2 * q + 1]);
-                    if (q < 7) ldsm_x4(a_delta + 32 * (q + 1), d0f[0], d0f[1], d0f[2], d0f[3]);
-                    mma_f16(Sd[1], d1f[0], d1f[1], d1f[2], d1f[3], QP[2 * q], QP[2 * q + 1]);
-                }
-            }
-            __syncwarp();
-            // the next tile may be built (where warps merge below, they do it in their tiles: not before that)
-            if (lane == 0 && (GS == 1 || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
-
-            // ======================= online softmax =======================
-            // x[mt][r]: token 16mt + g + 8(r>>1), head 2j + (r&1)
-            float x[2][4];
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) x[mt][r] = fmaf(Sc[mt][r], 1048576.f, Sd[mt][r] + Sz[r & 1]);
-            if (p.logit_cap > 0.f) {
-#pragma unroll
-                for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) x[mt][r] = p.logit_cap * tanhf(x[mt][r] / p.logit_cap);
-            }
-            const int tok_base = 32 * lg;
-            if (tok_base + 32 > pc.ntok) {
-#pragma unroll
-                for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                    for (int r = 0; r < 4; ++r)
-                        if (tok_base + 16 * mt + g + 8 * (r >> 1) >= pc.ntok) x[mt][r] = -INFINITY;
-            }
-            float corr[2], mneg[2];
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                float mloc = fmaxf(fmaxf(x[0][hh], x[0][2 + hh]), fmaxf(x[1][hh], x[1][2 + hh]));
-                mloc = fmaxf(mloc, __shfl_xor_sync(0xFFFFFFFFu, mloc, 4));
-                mloc = fmaxf(mloc, __shfl_xor_sync(0xFFFFFFFFu, mloc, 8));
-                mloc = fmaxf(mloc, __shfl_xor_sync(0xFFFFFFFFu, mloc, 16));
-                const float m_new = fmaxf(m_run[hh], mloc);
-                const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-                corr[hh] = fast_exp2((m_run[hh] - m_use) * LOG2E);   // m_run = -inf -> 0
-                mneg[hh] = -m_use * LOG2E;
-                m_run[hh] = m_new;
-            }
-            float pr[2][4];
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) pr[mt][r] = fast_exp2(fmaf(x[mt][r], LOG2E, mneg[r & 1]));
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-                l_run[hh] = l_run[hh] * corr[hh] + ((pr[0][hh] + pr[0][2 + hh]) + (pr[1][hh] + pr[1][2 + hh]));   // this lane's tokens only
-            if (__any_sync(0xFFFFFFFFu, corr[0] != 1.0f || corr[1] != 1.0f)) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) { acc[i][0] *= corr[0]; acc[i][1] *= corr[1]; acc[i][2] *= corr[0]; acc[i][3] *= corr[1]; }
-                accz[0] *= corr[0]; accz[1] *= corr[1];
-            }
-            // P^T as B fragments: transpose each 8x8 (token, head) block; T[ks][b] = tokens 16ks + 8b + 2j, +1 of head g
-            uint32_t T[2][2];
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                T[mt][0] = movmatrix_trans(pack_f16x2(pr[mt][0], pr[mt][1]));
-                T[mt][1] = movmatrix_trans(pack_f16x2(pr[mt][2], pr[mt][3]));
-            }
-
-            // ======================= P.V =======================
-            if (do_v) {
-                const int copy = it & 1;
-                uint32_t VF[16];                                     // factor pairs, index 4cg + 2ks + b
-                {
-                    const uint8_t *p_vf = tile + (ROW_VF + copy) * DT_STRIDE + 16 * j;
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        const uint4 t = *reinterpret_cast<const uint4 *>(p_vf + 64 * v);
-                        VF[4 * v] = t.x; VF[4 * v + 1] = t.y; VF[4 * v + 2] = t.z; VF[4 * v + 3] = t.w;
-                    }
-                }
-                const uint8_t *p_zt = tile + (ROW_ZT + copy) * DT_STRIDE + ZT_STRIDE * (g & 3) + 4 * j;
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {
-                    uint32_t vc[4];                                  // by scale group: channels 32cg + 4g .. + 3 of four tokens, a byte each
-                    ldsm_b8_trans_x2(v_addr + 16 * TS * ks, vc);
-#pragma unroll
-                    for (int cg = 0; cg < 4; ++cg) {
-                        const uint32_t w01 = vc[cg], w89 = vc[cg] >> 8;
-                        const uint32_t pb0 = hmul2_f16(T[ks][0], VF[4 * cg + 2 * ks]), pb1 = hmul2_f16(T[ks][1], VF[4 * cg + 2 * ks + 1]);
-#pragma unroll
-                        for (int u = 0; u < 2; ++u)
-                            mma_f16(acc[2 * cg + u], w01 & (0x00030003u << (2 * u)), w01 & (0x00030003u << (2 * u + 4)),
-                                    w89 & (0x00030003u << (2 * u)), w89 & (0x00030003u << (2 * u + 4)), pb0, pb1);
-                    }
-                    uint32_t za0 = 0u, za2 = 0u;
-                    if (g < 4) {
-                        za0 = *reinterpret_cast<const uint32_t *>(p_zt + 32 * ks);
-                        za2 = *reinterpret_cast<const uint32_t *>(p_zt + 32 * ks + 16);
-                    }
-                    mma_f16(accz, za0, 0u, za2, 0u, T[ks][0], T[ks][1]);
-                }
-            }
-        } else {
-            if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
-                gave_up = true;
-                break;
-            }
-            if (lane == 0 && (GS == 1 || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
-        }
-        // release the stage
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_empty + 8 * s);
-    }
-    if (gave_up) {
-        if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
-        m_run[0] = m_run[1] = -INFINITY; l_run[0] = l_run[1] = 0.f;
-    }
-
-    // ---- epilogue: this lane holds 16 channels of heads 2j and 2j+1; merge warps that share a head ----
-    float l_tot[2];
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-        float l = l_run[hh];
-        l += __shfl_xor_sync(0xFFFFFFFFu, l, 4);
-        l += __shfl_xor_sync(0xFFFFFFFFu, l, 8);
-        l += __shfl_xor_sync(0xFFFFFFFFu, l, 16);
-        l_tot[hh] = l;
-    }
-    // outv[hh][4cg + c]: channel 32cg + 4g + c of head 2j + hh, un-normalised
-    float outv[2][16];
-#pragma unroll
-    for (int cg = 0; cg < 4; ++cg) {
-        const float bz0 = __shfl_sync(0xFFFFFFFFu, accz[0], 4 * cg + j);
-        const float bz1 = __shfl_sync(0xFFFFFFFFu, accz[1], 4 * cg + j);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int u = c & 1, v = c >> 1;
-            const float f = 1048576.f / (float)(1 << (2 * c));       // 2^(24 - FBIAS) * 4^-slot
-            outv[0][4 * cg + c] = fmaf(acc[2 * cg + u][2 * v], f, bz0);
-            outv[1][4 * cg + c] = fmaf(acc[2 * cg + u][2 * v + 1], f, bz1);
-        }
-    }
-
-    // Several groups per stage (fewer than 8 local kv heads): the warps that share a head merge, each through the delta rows
-    // of its own tile, which nobody builds again before it is handed back below.  With 8 heads every warp owns its head and
-    // writes straight away.
-    static_assert(32 * 36 * 4 <= 32 * DT_STRIDE, "the merge fits the delta rows of a tile");
-    if (GS > 1) {
-        if (gsel > 0) {
-            float *my = reinterpret_cast<float *>(s_tiles + unit * DT_BYTES) + lane * 36;
-            my[0] = m_run[0]; my[1] = m_run[1]; my[2] = l_tot[0]; my[3] = l_tot[1];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) { my[4 + i] = outv[0][i]; my[20 + i] = outv[1][i]; }
-        }
-        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
-    }
-    if (gsel == 0) {
-        for (int o = 1; o < GS; ++o) {
-            const float *ot = reinterpret_cast<const float *>(s_tiles + (o * H + h) * DT_BYTES) + lane * 36;
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const float m2 = ot[hh], l2 = ot[2 + hh];
-                const float mn = fmaxf(m_run[hh], m2);
-                const float mu = (mn == -INFINITY) ? 0.f : mn;
-                const float c1 = fast_exp2((m_run[hh] - mu) * LOG2E), c2 = fast_exp2((m2 - mu) * LOG2E);
-                l_tot[hh] = l_tot[hh] * c1 + l2 * c2;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) outv[hh][i] = outv[hh][i] * c1 + ot[4 + 16 * hh + i] * c2;
-                m_run[hh] = mn;
-            }
-        }
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int head = 2 * j + hh;
-            if (head < p.gqa) {
-                const float inv = l_tot[hh] > 0.f ? 1.f / l_tot[hh] : 0.f;
-                float *dst = p.al + (int64_t)pc.b * p.al_sb + (int64_t)(h * p.gqa + head) * p.al_sh + (int64_t)pc.slot * p.al_ss;
-#pragma unroll
-                for (int cg = 0; cg < 4; ++cg)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) dst[32 * cg + 4 * g + c] = outv[hh][4 * cg + c] * inv;
-                if (g == 0) dst[HD] = l_tot[hh] > 0.f ? m_run[hh] + logf(l_tot[hh]) : -INFINITY;
-            }
-        }
-    }
-    if (GS > 1) {
-        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
-        if (lane == 0) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(pc.it1 - 1, NS)));
-    }
-    } while (step_piece());
-}
 
 // =================================================================================================
 // Stage 2: bf16 sink/recent rows + log-sum-exp combine (reference: paged_decode.py:2366-2500)
@@ -1631,40 +456,6 @@ static size_t stage1_smem(const S1Params &p) {
            + (size_t)p.GS * (4 * p.ppg + 6) * (sizeof(CopyDesc) + 4) + MAX_PIECES * sizeof(Piece);   // copy roles, their table entries, pieces
 }
 
-// Launch as a programmatic dependent of whatever precedes it in the stream: the grid may be placed while that
-// kernel drains, and the kernel itself waits (griddepcontrol.wait) before it reads or writes global memory.
-template <typename Kernel, typename Params>
-static cudaError_t launch_overlapping_previous(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const Params &p) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
-constexpr int MAX_DEVICES = 64;
-static int current_device(int *dev) {
-    OMMX_CUDA_TRY(cudaGetDevice(dev));
-    if (*dev < 0 || *dev >= MAX_DEVICES) return fail(OMMX_E_UNSUPPORTED, "device ordinal %d (this build tracks %d devices)", *dev, MAX_DEVICES);
-    return 0;
-}
-
-static int sm_count_of(int dev) {
-    static std::atomic<int> counts[MAX_DEVICES];
-    int n = counts[dev].load(std::memory_order_acquire);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = 148; }
-        counts[dev].store(n, std::memory_order_release);
-    }
-    return n;
-}
-
 // CTAs of a stage-1 launch: one per SM, or one per group where there are fewer groups than SMs; and the rounds of them
 // that equal splits would take (capped: past the cap they are never the choice)
 static int stage1_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
@@ -1677,44 +468,6 @@ static int stage1_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
     *ncta = (int)max(min((long long)sm_count_of(dev), max(groups, 1ll)), least);
     *waves = (int)min((splits + *ncta - 1) / *ncta, 1024ll);
     return 0;
-}
-
-template <int KOUT, int H>
-static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
-    using L = WarpLayout<H>;
-    // function attributes belong to (kernel instantiation, device): one entry per device ordinal
-    static std::atomic<size_t> attr_smem[MAX_DEVICES];
-    static std::atomic<int> regs_state[MAX_DEVICES];   // 0 unknown, 1 enough, 2 too few
-    int dev = 0;
-    if (int rc = current_device(&dev)) return rc;
-    int regs_ok = regs_state[dev].load(std::memory_order_acquire);
-    if (regs_ok == 0) {
-        cudaFuncAttributes fa;
-        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, H>));
-        // setmaxnreg.inc must find the registers the other roles gave back
-        const int need = NCW * 32 * REGS_MMA + (L::WIDE ? L::NDW * 32 * REGS_DECODE + L::NPW * 32 * REGS_PRODUCER
-                                                        : (L::THREADS - NCW * 32) * REGS_DECODE);
-        regs_ok = fa.numRegs * L::THREADS >= need ? 1 : 2;
-        regs_state[dev].store(regs_ok, std::memory_order_release);
-    }
-    if (regs_ok != 1) return fail(OMMX_E_CUDA, "stage 1 was compiled with fewer registers than its warp roles need");
-    if (smem > attr_smem[dev].load(std::memory_order_acquire)) {
-        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_kernel<KOUT, H>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_smem[dev].store(smem, std::memory_order_release);
-    }
-    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H>, dim3(p.ncta), L::THREADS, smem, st, p));
-    count_launch();
-    return 0;
-}
-template <int KOUT>
-static int launch_s1_heads(const S1Params &p, size_t smem, cudaStream_t st) {
-    switch (p.H) {
-        case 8: return launch_s1<KOUT, 8>(p, smem, st);
-        case 4: return launch_s1<KOUT, 4>(p, smem, st);
-        case 2: return launch_s1<KOUT, 2>(p, smem, st);
-        default: return launch_s1<KOUT, 1>(p, smem, st);
-    }
 }
 
 }  // namespace ommx
@@ -1818,14 +571,11 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
     const size_t smem = stage1_smem(p);
     if (smem > 232448) return fail(OMMX_E_UNSUPPORTED, "stage 1 planes of one group do not fit shared memory");
     if (int rc = stage1_ctas(a, &p.ncta, &p.waves)) return rc;
-    switch (p.k_out) {                       // the serving recipes get the unrolled two-pass splice
-        case 0: return launch_s1_heads<0>(p, smem, st);
-        case 2: return launch_s1_heads<2>(p, smem, st);
-        case 4: return launch_s1_heads<4>(p, smem, st);
-        case 6: return launch_s1_heads<6>(p, smem, st);
-        case 8: return launch_s1_heads<8>(p, smem, st);
-        case 12: return launch_s1_heads<12>(p, smem, st);
-        default: return launch_s1_heads<-1>(p, smem, st);
+    switch (p.H) {
+        case 8: return launch_stage1_h8(p, smem, st);
+        case 4: return launch_stage1_h4(p, smem, st);
+        case 2: return launch_stage1_h2(p, smem, st);
+        default: return launch_stage1_h1(p, smem, st);
     }
 }
 
