@@ -1,22 +1,22 @@
 // Paged decode attention over OMMX-quantized KV planes for sm_100a: split-KV stage 1, stage 2
 // (log-sum-exp combine with the bf16 sink/recent rows fused in) and the partial-state merge.
 //
-// Stage 1 replaces _canonical_splitkv_stage1 (ommx_gpu_serve/attention/paged_decode.py:1255-2284
-// of the reference).  One CTA serves one (split, sequence) pair and ALL local kv heads of its
-// token range, so every page row it touches is a full contiguous line:
+// Stage 1 (ommx_stage1.cuh) replaces _canonical_splitkv_stage1 (ommx_gpu_serve/attention/paged_decode.py:1255-2284
+// of the reference).  The groups of all sequences form one running list of which every CTA takes an
+// equal share, for ALL local kv heads, so every page row it touches is a full contiguous line:
 //
 //   producer warp   streams whole pages / group-slot planes into a shared-memory ring: the two
 //                   code planes through swizzled tensor maps, the small planes with 1-D bulk
-//                   copies, completion through mbarrier transaction counts; page ids, group
-//                   slots and the copy roles of a stage are tabulated in shared memory once.
+//                   copies, completion through mbarrier transaction counts; page ids and group
+//                   slots are read one ring stage ahead.
 //   15 decode warps build, two per (group, kv head) unit, the unit's sidecar tile: outlier
 //                   deltas (bit walk with clz, FP4 nibble, base code byte) as fp16
-//                   [token][channel], the fp32 q.zp dot products of the unit's query heads, and the
-//                   power-of-two K and V scale factors laid out in MMA-fragment order.
+//                   [token][channel], and the power-of-two K and V scale factors laid out in
+//                   MMA-fragment order.
 //   8 MMA warps     own one unit per stage and a private online-softmax state.  All MMAs are
 //                   m16n8k16 fp16 with the 2-bit codes as the A operand - a code field masked in
 //                   place is the fp16 subnormal code * 4^slot * 2^-24, exact and offset-free - and
-//                   the query heads as the 8 columns: logits = codes.(q*2^e) + delta.q + (q.zp from the sidecar),
+//                   the query heads as the 8 columns: logits = codes.(q*2^e) + delta.q + q.zp,
 //                   softmax over token rows, P transposed with movmatrix, output =
 //                   codes^T.(P*2^e_v) + vz^T.P.
 //

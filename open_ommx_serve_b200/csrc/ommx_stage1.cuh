@@ -242,7 +242,8 @@ __device__ __forceinline__ uint32_t ring_phase(int it, int ns) { return (uint32_
 // ---- how the groups of a launch are shared out over its CTAs ------------------------------------------
 // The packed groups of all sequences form one running list, and CTA i takes groups [i * per, (i + 1) * per) of it, whatever
 // sequences they belong to: every CTA has the same work up to one group, also when the lengths are ragged (32 sequences of
-// 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us around its steady state).  A piece of
+// 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us around its steady state: 560 us of
+// store and decode against 363 us).  A piece of
 // a sequence writes its partial result to workspace slot (its CTA - the first CTA of the sequence), and the caller's
 // workspace has S slots per sequence, which bounds `per` from below.  Where that bound makes the shares longer than S equal
 // splits per sequence dealt out one by one would be, those are taken instead (per = 0): item x is split x % S of sequence x / S.
@@ -381,12 +382,19 @@ template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk
 //                                16 rows of an m-tile lie in one V scale group)
 //                              + vz^T[group][token] . P[token][head]
 // The power-of-two factors, zero-points and deltas of a unit are laid out for these fragments by the
-// decode warps (the sidecar tile), so the MMA warps multiply and accumulate and do little else.
+// decode warps (the sidecar tile), so the MMA warps multiply and accumulate and do little else; what they
+// still compute themselves, q.zp, fits into their wait for the deltas.
+//
+// Bound by the dependent chain of an MMA warp (about 5000 cycles for a group of a head: code MMAs, delta MMAs, softmax,
+// P.V) with the decode warps that feed it close behind; the register file (8 x 128 + 16 x 56 a lane) holds no second unit
+// in flight, and memory is at a quarter of its rate.  Measured, this stage alone, before the running list, the cheaper unit
+// and PLAIN -> with them: 64K tokens x 8 heads 50.2 -> 40.8 us; 8 x 32K 184 -> 143.9 us; 32 sequences of 1K to 32K in
+// splits of 512 with the store and stage 2 around it 560 -> 328 us.
 //
 // PLAIN: the recipe that is served - bitmask index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
-// form keeps them at run time; its tests and address arithmetic inside the unit cost it 6 % (70B heads 8 x 32K: 160.6 us
-// against 151.3 us).
+// form keeps them at run time; its tests and address arithmetic inside the unit cost it 10 % (70B heads 8 x 32K: 160.6 us
+// against 143.9 us).
 template <int KOUT, int H> struct PlainLayout {
     static constexpr int NB = KOUT > 0 ? (KOUT + 1) / 2 : 0;
     static constexpr int VM = H * 1024, VS = H * 2048, VZ = VS + H * 128, KS = VZ + H * 256, KZ = KS + H * 128, MS = KZ + H * 256, MC = MS + H * 256,

@@ -107,6 +107,20 @@ def test_decode_batch32_ragged_partition_512():
     _run_and_check(case, num_kv_splits=(max(case.packed) + 511) // 512)
 
 
+@pytest.mark.parametrize("lens,H,splits", [
+    ([40, 2088, 8, 72, 40, 1064, 104, 40], 8, 148),        # one group per CTA, sequences without groups at the ends and between
+    ([72 + 32 * (i % 5) for i in range(40)], 4, 4),        # 40 short sequences, several to a CTA; stage 2 with 640 rows
+    ([72 + 32 * (i % 3) for i in range(160)], 2, 2),       # more sequences than CTAs
+    ([4136, 40, 72, 2088, 104], 1, 16),                    # the wide layout, one head
+    ([5000, 72, 72, 72, 72, 72, 72, 72, 72], 8, 3),        # the longest sequence bounds the share (workspace slots); 288 rows
+    ([1000, 40, 600], 8, 1),                               # one slot per sequence: equal splits
+    ([1064] * 16, 8, 9),                                   # equal lengths that fill the waves of CTAs: equal splits
+])
+def test_decode_groups_shared_over_the_ctas(lens, H, splits):
+    """Where a CTA's share begins and ends inside sequences, and every block size of stage 2."""
+    _run_and_check(Case(lens, H=H, Hq=4 * H, seed=17), num_kv_splits=splits)
+
+
 def test_decode_tail_only_and_empty():
     case = Case([30, 8, 71], seed=2)                 # nothing quantized anywhere
     o, lse = case.run()

@@ -86,6 +86,42 @@ def test_incremental_store_equals_bulk_pack(k, page_size):
             _check_against_history(pool, hist_k, hist_v, k=k, page_size=page_size)
 
 
+@pytest.mark.parametrize("D,H,sink,recent,lens", [
+    (128, 1, 8, 1, [7, 8, 9, 40, 41, 72]),       # lengths around the sink and the first group's boundary
+    (64, 3, 0, 33, [1, 64, 65, 66, 97]),         # no sink, an odd window, two warps' worth of channels
+    (128, 2, 8, 0, [8, 39, 40, 41]),             # no recent rows: the separate kernels
+    (96, 2, 4, 32, [3, 67, 68, 69]),             # channels that are not whole 64-channel units: the separate kernels
+])
+def test_store_step_and_prefill_at_the_window_edges(D, H, sink, recent, lens):
+    from open_ommx_serve_b200.attention.kv_pool import MultiSeqKVPool
+    from open_ommx_serve_b200.attention.kv_window import WindowSpec
+    pool = MultiSeqKVPool(D, H, len(lens), 256, window=WindowSpec(sink, recent, 32, 16), device="cuda")
+    hist = [list(gaussian_kv(300 + r, T, H, D)) for r, T in enumerate(lens)]
+    for r, (K, V) in enumerate(hist):
+        pool.append_block(r, K.cuda().bfloat16(), V.cuda().bfloat16())
+    g = torch.Generator().manual_seed(9)
+    for step in range(35):
+        new = torch.randn(2, len(lens), H, D, generator=g).bfloat16()
+        pool.append_decode_device(new[0].cuda(), new[1].cuda(), len(lens))
+        for r, kv in enumerate(hist):
+            for i in (0, 1):
+                kv[i] = torch.cat([kv[i], new[i, r:r + 1].float()])
+        if step not in (0, 1, 31, 34):
+            continue
+        assert int(pool.status.item()) == 0
+        for r, (K, V) in enumerate(hist):
+            T = K.shape[0]
+            edge = O.packed_boundary(T, sink, recent)
+            packed = max(0, edge - sink)
+            rows = list(range(min(sink, T))) + list(range(edge, T))
+            assert int(pool.b_seq[r]) == packed and int(pool.b_tail[r]) == len(rows), (step, r)
+            assert torch.equal(pool.k_tail[r, :len(rows)].cpu(), K[rows].bfloat16()), (step, r)
+            assert torch.equal(pool.v_tail[r, :len(rows)].cpu(), V[rows].bfloat16()), (step, r)
+            if packed:
+                want = O.pack_kv(K[sink:edge].numpy(), V[sink:edge].numpy(), outliers_per_vector=6, page_size=16)
+                assert_planes_equal(_seq_planes(pool, r, packed // 32), want, ctx=f"step {step} req {r}: ")
+
+
 def test_store_feeds_decode_without_host_state():
     """append_decode_device -> decode_inputs_device -> the decode kernels, with nothing in between."""
     from open_ommx_serve_b200 import ommx_paged_decode_attention_canonical
