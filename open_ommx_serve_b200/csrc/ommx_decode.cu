@@ -478,14 +478,14 @@ namespace ommx {
 // is the faster of the two (53 us against 142 us per 64K-context layer).  OMMX_B200_STAGE1=tc selects the tensor-core
 // kernel (decode_stage1_tc_kernel) where its shared-memory plan fits - 4 or 8 local kv heads with GQA <= 4, fewer
 // heads at any GQA <= 8 - and no differential-timing knob is set; it produces the same results within the path's
-// tolerance and is kept for further work on its pipeline.  The variable is read per call.
+// tolerance and is kept for further work on its pipeline.  The variable is read once per call (`tc` below).
 static bool tensor_core_stage1() {
     const char *e = getenv("OMMX_B200_STAGE1");
     return e && !strcmp(e, "tc");
 }
-// Its shared memory for this call, or 0 where the default kernel serves
+// Its shared memory for this call (when it is asked for), or 0 where the default kernel serves
 static size_t tensor_core_plan(const ommx_decode_args *a, const S1Params &p, TcParams *T) {
-    if (!tensor_core_stage1() || p.abl != 0 || p.gqa > 8 || p.idx7) return 0;
+    if (p.abl != 0 || p.gqa > 8 || p.idx7) return 0;
     T->s = p;
     T->s.GS = 1;
     T->s.stage_bytes = p.gb_bytes;
@@ -543,8 +543,8 @@ static int fill_stage1(const ommx_decode_args *a, S1Params &p) {
 
 // CTAs that stage 1 shares the groups over, 0 where it makes equal splits per sequence (the tensor-core kernel): stage 2
 // works out the same workspace slots from it
-static int shared_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
-    if (tensor_core_stage1()) {
+static int shared_ctas(const ommx_decode_args *a, bool tc, int *ncta, int *waves) {
+    if (tc) {
         S1Params p;
         TcParams T;
         if (int rc = fill_stage1(a, p)) return rc;
@@ -553,11 +553,11 @@ static int shared_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
     return stage1_ctas(a, ncta, waves);
 }
 
-static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
+static int launch_stage1(const ommx_decode_args *a, cudaStream_t st, bool tc) {
     if (a->max_seq_len <= 0) return 0;                                   // tail-only decode
     S1Params p;
     if (int rc = fill_stage1(a, p)) return rc;
-    if (tensor_core_stage1()) {
+    if (tc) {
         TcParams T;
         if (const size_t tsmem = tensor_core_plan(a, p, &T)) {
             dim3 tgrid(a->num_kv_splits, a->batch);
@@ -581,7 +581,7 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st) {
 
 // `after_stage1`: the previous kernel in the stream is this call's own stage 1, so stage 2 may be
 // launched as its programmatic dependent.
-static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool after_stage1 = false) {
+static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bool after_stage1) {
     const ommx_kv_planes &pl = a->planes;
     S2Params p;
     p.q = (const __nv_bfloat16 *)a->q; p.q_sb = a->q_stride_b; p.q_sh = a->q_stride_h;
@@ -594,7 +594,7 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool after_
     p.S = a->max_seq_len > 0 ? a->num_kv_splits : 0;
     p.B = a->batch; p.ncta = p.waves = 0;
     if (p.S > 0)
-        if (int rc = shared_ctas(a, &p.ncta, &p.waves)) return rc;
+        if (int rc = shared_ctas(a, tc, &p.ncta, &p.waves)) return rc;
     p.o = a->o; p.o_bf16 = (a->o_dtype == OMMX_DT_BF16); p.o_sb = a->o_stride_b; p.o_sh = a->o_stride_h;
     p.lse = a->lse; p.lse_sb = a->lse_stride_b;
     p.sm_scale = a->sm_scale; p.logit_cap = a->logit_cap;
@@ -676,19 +676,20 @@ extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, 
 extern "C" int ommx_b200_decode_stage1(const ommx_decode_args *a, void *stream) {
     int rc = ommx::validate_decode(a);
     if (rc) return rc;
-    return ommx::launch_stage1(a, (cudaStream_t)stream);
+    return ommx::launch_stage1(a, (cudaStream_t)stream, ommx::tensor_core_stage1());
 }
 extern "C" int ommx_b200_decode_stage2(const ommx_decode_args *a, void *stream) {
     int rc = ommx::validate_decode(a);
     if (rc) return rc;
-    return ommx::launch_stage2(a, (cudaStream_t)stream);
+    return ommx::launch_stage2(a, (cudaStream_t)stream, ommx::tensor_core_stage1(), false);
 }
 extern "C" int ommx_b200_decode(const ommx_decode_args *a, void *stream) {
     int rc = ommx::validate_decode(a);
     if (rc) return rc;
-    rc = ommx::launch_stage1(a, (cudaStream_t)stream);
+    const bool tc = ommx::tensor_core_stage1();
+    rc = ommx::launch_stage1(a, (cudaStream_t)stream, tc);
     if (rc) return rc;
-    return ommx::launch_stage2(a, (cudaStream_t)stream, true);
+    return ommx::launch_stage2(a, (cudaStream_t)stream, tc, true);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -743,9 +744,10 @@ extern "C" int ommx_b200_decode_static_ws(const ommx_decode_args *a, void *strea
     b.al_stride_b = (int64_t)a->n_q_heads * b.al_stride_h;
     rc = validate_decode(&b);
     if (rc) return rc;
-    rc = launch_stage1(&b, (cudaStream_t)stream);
+    const bool tc = tensor_core_stage1();
+    rc = launch_stage1(&b, (cudaStream_t)stream, tc);
     if (rc) return rc;
-    return launch_stage2(&b, (cudaStream_t)stream, true);
+    return launch_stage2(&b, (cudaStream_t)stream, tc, true);
 }
 
 extern "C" int ommx_b200_merge_states(const float *o_parts, const float *lse_parts, const int32_t *valid_lens,

@@ -11,11 +11,13 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Device.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <cctype>
 #include <cstdlib>
@@ -71,6 +73,17 @@ bool env_on(const char *name) {
         if (n == strlen(off) && strncasecmp(v, off, n) == 0) return false;
     return true;
 }
+
+// Whether any switch of this package is set: one pass over the environment where a getenv per switch takes one each (nine
+// of them were 1.5 us of a decode call under 135 variables).
+bool any_switch() {
+    for (char **e = environ; e && *e; ++e)
+        if (strncmp(*e, "OMMX", 4) == 0) return true;
+    return false;
+}
+
+// a fresh tensor without the dispatcher's round (pack_block makes twelve)
+Tensor fresh(at::IntArrayRef size, const at::TensorOptions &o) { return at::detail::empty_cuda(size, o); }
 
 struct Names {                                        // interned dictionary keys and attribute names
     PyObject *k_base, *k_scale, *k_zp, *k_obmp, *k_oval, *k_fp4_mapscale, *k_fp4_mapcenter, *v_main, *v_scale, *v_zp;
@@ -170,8 +183,9 @@ PyObject *py_decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
     const char *fmt = PyUnicode_AsUTF8(a[K_FORMAT]);
     if (!fmt) return nullptr;
     NEED(strcasecmp(fmt, "i2f4") == 0 || strcasecmp(fmt, "itf4") == 0);
-    combinadic = combinadic || env_on("OMMX_VLLM_KV_COMBINADIC_READ");
-    bitmap = bitmap || env_on("OMMX_VLLM_KV_BITMAP_READ");
+    const bool switches = any_switch();
+    combinadic = combinadic || (switches && env_on("OMMX_VLLM_KV_COMBINADIC_READ"));
+    bitmap = bitmap || (switches && env_on("OMMX_VLLM_KV_BITMAP_READ"));
     const bool relidx7 = k > 0 && !bitmap;
     NEED(!(bitmap && combinadic) && !(relidx7 && combinadic) && k <= 16);
     NEED(start_offset >= 0 && start_offset < page_size && seg_base >= 0 && seg_base <= INT32_MAX);
@@ -228,7 +242,7 @@ PyObject *py_decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
     if (a[SPLITS] != Py_None) {
         NEED(as_long(a[SPLITS], &splits));
     } else {
-        const char *forced = getenv("OMMX_ATTN_NUM_KV_SPLITS");
+        const char *forced = switches ? getenv("OMMX_ATTN_NUM_KV_SPLITS") : nullptr;
         while (forced && isspace((unsigned char)*forced)) ++forced;
         if (forced && *forced) {
             PyObject *mod = PyImport_ImportModule("open_ommx_serve_b200.attention.paged_decode");   // its strict reader
@@ -250,7 +264,7 @@ PyObject *py_decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
         const Tensor *al = as_tensor(a[ATTN_LOGITS]);
         if (!al) {
             NEED(a[ATTN_LOGITS] == Py_None);
-            own_logits = at::empty({batch, heads, splits + 1, D + 1}, q->options().dtype(at::kFloat));
+            own_logits = fresh({batch, heads, splits + 1, D + 1}, q->options().dtype(at::kFloat));
             al = &own_logits;
         }
         NEED(al->scalar_type() == at::kFloat && al->device() == dev && al->dim() == 4 && al->size(0) >= batch && al->size(1) >= heads);
@@ -283,7 +297,7 @@ PyObject *py_decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
         d.status = (int32_t *)st->data_ptr();
     }
     // differential-timing knobs: the caller records them, so a leaked export cannot pass as served
-    for (size_t i = 0; i < sizeof(ABL_FLAGS) / sizeof(ABL_FLAGS[0]); ++i)
+    for (size_t i = 0; switches && i < sizeof(ABL_FLAGS) / sizeof(ABL_FLAGS[0]); ++i)
         if (env_on(ABL_FLAGS[i])) d.abl_flags |= 1 << i;
     if (a[HEAD_GATHER] != Py_None) {
         NEED(stage != 1);
@@ -378,20 +392,20 @@ PyObject *py_pack_block(PyObject *, PyObject *const *a, Py_ssize_t n) {
     const auto bytes = K->options().dtype(at::kByte), ints = K->options().dtype(at::kInt);
     const auto scale = K->options().dtype(kind == OMMX_SCALE_INT8_EXP ? at::kChar : (kind == OMMX_SCALE_BF16 ? at::kBFloat16 : at::kFloat));
     const auto zp = K->options().dtype(kind == OMMX_SCALE_F32 ? at::kFloat : at::kBFloat16);
-    Tensor k_base = at::empty({pages, ps, H, D / 4}, bytes), v_main = at::empty({pages, ps, H, D / 4}, bytes);
-    Tensor k_scale = at::empty({G, H, D}, scale), k_zp = at::empty({G, H, D}, zp);
-    Tensor v_scale = at::empty({pages, ps, H, D / 32}, scale), v_zp = at::empty({pages, ps, H, D / 32}, zp);
+    Tensor k_base = fresh({pages, ps, H, D / 4}, bytes), v_main = fresh({pages, ps, H, D / 4}, bytes);
+    Tensor k_scale = fresh({G, H, D}, scale), k_zp = fresh({G, H, D}, zp);
+    Tensor v_scale = fresh({pages, ps, H, D / 32}, scale), v_zp = fresh({pages, ps, H, D / 32}, zp);
     Tensor k_obmp, k_oval, k_ms, k_mc, k_oidx;
     if (k > 0) {
-        k_obmp = at::empty({G, H, D, 4}, bytes);
-        k_oval = at::empty({G, H, D, (k + 1) / 2}, bytes);
-        if (use_map) { k_ms = at::empty({G, H, D}, zp); k_mc = at::empty({G, H, D}, zp); }
+        k_obmp = fresh({G, H, D, 4}, bytes);
+        k_oval = fresh({G, H, D, (k + 1) / 2}, bytes);
+        if (use_map) { k_ms = fresh({G, H, D}, zp); k_mc = fresh({G, H, D}, zp); }
     }
     auto opt = [](const Tensor &t) { return t.defined() ? &t : nullptr; };
     const PlaneSet s{&k_base, &k_scale, &k_zp, opt(k_obmp), opt(k_oval), opt(k_ms), opt(k_mc), &v_main, &v_scale, &v_zp};
     Tensor status;
-    if (check) status = at::empty({1}, ints);
-    Tensor r2t = at::empty({1, pages}, ints), r2g = at::empty({1, G}, ints);
+    if (check) status = fresh({1}, ints);
+    Tensor r2t = fresh({1, pages}, ints), r2g = fresh({1, G}, ints);
     int rc = launch(K->device(), [&](void *stream) {
         return ommx_b200_identity_tables((int32_t *)r2t.data_ptr(), (int32_t)pages, (int32_t *)r2g.data_ptr(), (int32_t)G, (int32_t *)ptr(status), stream);
     });
@@ -399,16 +413,15 @@ PyObject *py_pack_block(PyObject *, PyObject *const *a, Py_ssize_t n) {
     NEED(pack_planes(*K, *V, s, nullptr, nullptr, k, is_signed, use_pow2, use_map, check ? (int32_t *)status.data_ptr() : nullptr, &rc));
     if (rc == 0 && relidx7 && k > 0) {
         // same outlier set, other index encoding: k ascending 7-bit positions per frame (the value plane is shared)
-        k_oidx = at::empty({G, H, D, (7 * k + 7) / 8}, bytes);
+        k_oidx = fresh({G, H, D, (7 * k + 7) / 8}, bytes);
         rc = launch(K->device(), [&](void *stream) {
             return ommx_b200_outlier_index_convert(k_obmp.data_ptr(), k_oidx.data_ptr(), G * H * D, (int32_t)k, 1, nullptr, stream);
         });
         k_obmp = Tensor();
     }
     if (rc != 0) return PyLong_FromLong(rc);
-    int64_t bits = 0;
-    if (check) bits = read_int(status);
-    PyObject *d = PyDict_New();
+    THPObjectPtr d(PyDict_New());                          // made while the GPU packs; the status is read last
+    if (!d) return nullptr;
     struct { const char *name; const Tensor *t; } out[] = {
         {"k_base", &k_base}, {"k_scale", &k_scale}, {"k_zp", &k_zp}, {"k_oidx", &k_oidx}, {"k_crank", nullptr}, {"k_obmp", &k_obmp}, {"k_oval", &k_oval},
         {"k_fp4_mapscale", &k_ms}, {"k_fp4_mapcenter", &k_mc}, {"v_main", &v_main}, {"v_scale", &v_scale}, {"v_zp", &v_zp},
@@ -416,13 +429,15 @@ PyObject *py_pack_block(PyObject *, PyObject *const *a, Py_ssize_t n) {
     for (auto &e : out) {
         if (e.t && e.t->defined()) {
             PyObject *w = THPVariable_Wrap(*e.t);
-            PyDict_SetItemString(d, e.name, w);
+            PyDict_SetItemString(d.get(), e.name, w);
             Py_XDECREF(w);
         } else {
-            PyDict_SetItemString(d, e.name, Py_None);
+            PyDict_SetItemString(d.get(), e.name, Py_None);
         }
     }
-    return Py_BuildValue("(NL)", d, (long long)bits);
+    int64_t bits = 0;
+    if (check) bits = read_int(status);
+    return Py_BuildValue("(NL)", d.release(), (long long)bits);
     END_HANDLE_TH_ERRORS
 }
 
