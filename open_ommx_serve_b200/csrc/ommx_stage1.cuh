@@ -235,6 +235,39 @@ __device__ __forceinline__ uint32_t code_pair(uint32_t w, int i) {
 }
 __device__ __forceinline__ int code_slot(int i) { return i < 5 ? i : i - 5; }
 
+// Bit planes of the 2-bit codes of 64 channels x 32 tokens, the codes of a channel pair to a lane: w[0], w[1] are the low and the
+// high code bit of its first channel, w[2], w[3] of its second, token = bit.  `addr` is the lane's row for the ldmatrix below:
+// the 16 bytes of token 8 (lane / 4 % 4) + 4 (lane / 16) + lane % 4.  Lane 4g + j gets byte column g (j < 2) or g + 8, channels
+// 2 (j & 1) and one more of it.
+__device__ __forceinline__ void code_bit_planes(uint32_t addr, int lane, uint32_t (&w)[4]) {
+    const bool right = lane & 2, odd = lane & 1;
+    uint32_t r[4];
+    ldsm_b8_trans_x2(addr, r);                               // r[2m + c]: tokens of quad j of matrix m, column g + 8c
+    uint32_t own[2], oth[2];                                 // this lane's column: quads j and j ^ 2
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        own[m] = right ? r[2 * m + 1] : r[2 * m];
+        oth[m] = __shfl_xor_sync(0xFFFFFFFFu, right ? r[2 * m] : r[2 * m + 1], 2);
+    }
+    // nibbles: both matrices' tokens side by side, the lower or upper channel pair; the other pair goes to the neighbour
+    const uint32_t LO = 0x0F0F0F0Fu;
+    const uint32_t a = (own[0] & LO) | ((own[1] << 4) & ~LO), b = ((own[0] >> 4) & LO) | (own[1] & ~LO);
+    const uint32_t c = (oth[0] & LO) | ((oth[1] << 4) & ~LO), d = ((oth[0] >> 4) & LO) | (oth[1] & ~LO);
+    const uint32_t q0 = odd ? b : a, q2 = odd ? d : c;                                            // quads j, j ^ 2
+    const uint32_t q1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? a : b, 1), q3 = __shfl_xor_sync(0xFFFFFFFFu, odd ? c : d, 1);   // j ^ 1, j ^ 3
+    // quads in order in the bytes, the token inside its quad to the register
+    const uint32_t s01 = odd ? 0x1504u : 0x5140u, s23 = odd ? 0x3726u : 0x7362u;
+    const uint32_t e01 = __byte_perm(q0, q1, s01), e23 = __byte_perm(q0, q1, s23), f01 = __byte_perm(q2, q3, s01), f23 = __byte_perm(q2, q3, s23);
+    const uint32_t h0 = right ? 0x1054u : 0x5410u, h1 = right ? 0x3276u : 0x7632u;
+    const uint32_t a0 = __byte_perm(e01, f01, h0), a1 = __byte_perm(e01, f01, h1), a2 = __byte_perm(e23, f23, h0), a3 = __byte_perm(e23, f23, h1);
+    // a_k, nibble n, bit i -> w_i, nibble n, bit k
+    const uint32_t P = 0x33333333u, Q = 0x55555555u;
+    const uint32_t b0 = (a0 & P) | ((a2 << 2) & ~P), b2 = ((a0 >> 2) & P) | (a2 & ~P);
+    const uint32_t b1 = (a1 & P) | ((a3 << 2) & ~P), b3 = ((a1 >> 2) & P) | (a3 & ~P);
+    w[0] = (b0 & Q) | ((b1 << 1) & ~Q); w[1] = ((b0 >> 1) & Q) | (b1 & ~Q);
+    w[2] = (b2 & Q) | ((b3 << 1) & ~Q); w[3] = ((b2 >> 1) & Q) | (b3 & ~Q);
+}
+
 // stage index and phase parity of ring use number `it` (ring depth ns: 4 unless the planes are large)
 __device__ __forceinline__ int ring_slot(int it, int ns) { return ns == 4 ? (it & 3) : it % ns; }
 __device__ __forceinline__ uint32_t ring_phase(int it, int ns) { return (uint32_t)(ns == 4 ? (it >> 2) : it / ns) & 1u; }
@@ -611,8 +644,10 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     // ---- one work item of the decode role: half hf of the sidecar tile of (iteration it, unit) ----
     // Channel 64 w + 16 j + 8 x + i (i = 0..7) sits in member x of the pair in register 8 w + i of lane group j in the MMAs
     // below, i.e. in column byte 128 w + 16 i + 4 j + 2 x of the delta rows.  This half has w = hf, this lane channels
-    // 2 lane and 2 lane + 1 of it: j = dj, x = dh, i = 2 da and 2 da + 1.
-    const int da = lane & 3, dh = (lane >> 2) & 1, dj = lane >> 3;
+    // 2 cp and 2 cp + 1 of it (the pair that code_bit_planes gives it): j = dj, x = dh, i = 2 da and 2 da + 1.
+    const int cp = 8 * (lane & 2) + 2 * (lane >> 2) + (lane & 1);
+    const int da = cp & 3, dh = (cp >> 2) & 1, dj = cp >> 3;
+    const int lm_tok = 8 * ((lane >> 2) & 3) + 4 * (lane >> 4) + (lane & 3);
     // 4^-slot of those two channels' code fields, fp16
     const uint32_t slot_scale = da == 0 ? 0x34003C00u : (da == 1 ? 0x24002C00u : (da == 2 ? 0x3C001C00u : 0x2C003400u));
     // Build the sidecar tile of a unit between two uses by its MMA warp.  A tile is built in two
@@ -632,13 +667,23 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const int lg = (it - pc.it0) * GS + gsel;                 // local group of this unit
         const bool active = lg < pc.ng && !(abl & ABL_NO_COMPUTE);
         const uint8_t *gb = s_stage + (size_t)s * stage_bytes + (size_t)gsel * gb_bytes;
-        const int d0 = 64 * hf + 2 * lane;                       // first of this lane's two channels
+        const int d0 = 64 * hf + 2 * cp;                         // first of this lane's two channels
         const bool splice = k_out > 0 && !no_outlier;
         // ---- everything that only reads the stage comes before the wait for the tile, which the MMA warps make a decode warp
         //      wait for (a sixth of its time): the parameters of both channels, the K and V factors, V zero-points ----
         bool clamped_any = false;
         uint32_t e2 = 0, z2 = 0, kf = 0, vf = 0, zt = 0, ms2 = 0, mc2 = 0;
         uint2 bm2 = make_uint2(0u, 0u);
+        // From 6 outliers on the base codes are looked up in bit planes in registers: a gather per outlier costs 3 to 4 conflicting
+        // shared-memory wavefronts, the planes of 64 channels about 50 instructions.  64K x 8 heads, stage 1: k = 12 53.8 -> 50.2 us,
+        // k = 8 43.3 -> 42.7, k = 6 40.3 -> 40.0; k = 4 37.2 -> 37.4 and k = 2 34.7 -> 35.5, which therefore gather.
+        constexpr bool PLANES = KOUT >= 6 && KOUT % 2 == 0;
+        uint32_t cw[4] = {0, 0, 0, 0};                           // bit planes of both channels' codes
+        // Row pz of the code bytes of the channels at byte o of the head: byte pz*TS + h*32 + o of the (1 KB aligned) k_base
+        // block, with the 16-byte chunk bits XOR-ed by the row's swizzle term.  h*32 + o splits into a part above
+        // bit 7 (added to the row) and a part below (the XOR operand, swizzle term of the former included).
+        const uint8_t *k_hi = gb + (h >> 2) * 128;
+        const uint32_t k_sw = ((uint32_t)(h >> 2) * 16u) & SWZ;
         uint32_t st[2] = {0, 0}, sth[2] = {0, 0};                // nibble stream of each channel: outliers 0..7, 8..15
         const int vtk = 16 * hf + 2 * (lane & 7), vcg = lane >> 3;   // V side: lane = (pair of tokens, scale group)
         if (active) {
@@ -705,6 +750,8 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     st[0] = w & 0xFFu; st[1] = w >> 8;
                 }
             }
+            if constexpr (PLANES)
+                if (splice) code_bit_planes(smem_u32(k_hi + lm_tok * TS) + (((h & 3) * 32 + 16 * hf) ^ k_sw ^ (((uint32_t)(lm_tok * TS) >> 3) & SWZ)), lane, cw);
             bool cl0, cl1, cl2, cl3;
             const uint32_t k0 = pow2_f16_bits(max((int)(int8_t)e2, -126), cl0), k1 = pow2_f16_bits(max((int)(int8_t)(e2 >> 8), -126), cl1);
             kf = hmul2_f16(k0 | (k1 << 16), slot_scale);         // * 4^-slot: exact, subnormals included
@@ -742,12 +789,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     *reinterpret_cast<uint4 *>(tile + (4 * k2 + (lane >> 3)) * DT_STRIDE + 128 * hf + 16 * (lane & 7)) = make_uint4(0, 0, 0, 0);
                 __syncwarp();                                        // the cleared rows before any delta lands in them
                 const uint32_t bmv[2] = {bm2.x, bm2.y};
-                // The code byte holding this lane's channels, row pz: byte pz*TS + h*32 + d0/4 of the (1 KB aligned)
-                // k_base block, with the 16-byte chunk bits XOR-ed by the row's swizzle term.  h*32 + d0/4 splits
-                // into a part above bit 7 (added to the row) and a part below (the XOR operand, swizzle term of the former
-                // included).
-                const uint8_t *k_hi = gb + (h >> 2) * 128;
-                const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2)) ^ (((uint32_t)(h >> 2) * 16u) & SWZ);
+                const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2)) ^ k_sw;
                 auto code_byte = [&](uint32_t pz) -> uint32_t {
                     return k_hi[pz * TS + (k_lo ^ (((pz * TS) >> 3) & SWZ))];
                 };
@@ -771,31 +813,53 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     uint8_t *col = tile + 128 * hf + 32 * da + 16 * c + 4 * dj + 2 * dh;
                     if constexpr (KOUT > 0 && KOUT % 2 == 0) {
                         if (__popc(bits) == KOUT) {
-                            // The code enters as the fraction of 1 + code/4, whose bits an AND and an OR make, so that 4 * sc moves to
-                            // the constant: lvl * A + (Bc + 4 sc) - (1 + code/4) * 4 sc.
-                            const float Bq = fmaf(4.f, sc, Bc), Sq = -4.f * sc;
-                            const int sh = 21 - fsh;              // moves the code to the top of the mantissa
-                            // Two passes: all gathers (bit walk, base-code byte) first, then the arithmetic and the
-                            // stores.  In one pass every load would have to follow the previous outlier's store in
-                            // program order (shared memory may alias), i.e. KOUT load round trips in a row.
-                            uint32_t pzs[KOUT], cbs[KOUT];
+                            if constexpr (PLANES) {
+                                const float sc2 = 2.f * sc;
 #pragma unroll
-                            for (int r = KOUT - 1; r >= 0; --r) {
-                                const uint32_t pz = 31 - __clz(bits);
-                                bits ^= 1u << pz;
-                                pzs[r] = pz;
-                                cbs[r] = code_byte(pz);
-                            }
+                                for (int r = KOUT - 2; r >= 0; r -= 2) {
+                                    const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
+                                    const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
+                                    const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
+                                    const uint32_t p1 = 31 - __clz(bits), m1 = 1u << p1;
+                                    bits ^= m1;
+                                    const uint32_t p0 = 31 - __clz(bits), m0 = 1u << p0;
+                                    bits ^= m0;
+                                    float x0 = fmaf(lvf.x, A, Bc), x1 = fmaf(lvf.y, A, Bc);
+                                    if (cw[2 * c] & m0) x0 -= sc;
+                                    if (cw[2 * c + 1] & m0) x0 -= sc2;
+                                    if (cw[2 * c] & m1) x1 -= sc;
+                                    if (cw[2 * c + 1] & m1) x1 -= sc2;
+                                    const uint32_t X = f16x2_of_bf16_rounded(x0, x1);
+                                    *reinterpret_cast<uint16_t *>(col + p0 * DT_STRIDE) = (uint16_t)X;
+                                    *reinterpret_cast<uint16_t *>(col + p1 * DT_STRIDE) = (uint16_t)(X >> 16);
+                                }
+                            } else {
+                                // The code enters as the fraction of 1 + code/4, whose bits an AND and an OR make, so that 4 * sc moves to
+                                // the constant: lvl * A + (Bc + 4 sc) - (1 + code/4) * 4 sc.
+                                const float Bq = fmaf(4.f, sc, Bc), Sq = -4.f * sc;
+                                const int sh = 21 - fsh;              // moves the code to the top of the mantissa
+                                // Two passes: all gathers (bit walk, base-code byte) first, then the arithmetic and the
+                                // stores.  In one pass every load would have to follow the previous outlier's store in
+                                // program order (shared memory may alias), i.e. KOUT load round trips in a row.
+                                uint32_t pzs[KOUT], cbs[KOUT];
 #pragma unroll
-                            for (int r = 0; r < KOUT; r += 2) {
-                                const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
-                                const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
-                                const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
-                                const float v0 = __uint_as_float(((cbs[r] << sh) & 0x600000u) | 0x3F800000u);
-                                const float v1 = __uint_as_float(((cbs[r + 1] << sh) & 0x600000u) | 0x3F800000u);
-                                const uint32_t X = f16x2_of_bf16_rounded(fmaf(v0, Sq, fmaf(lvf.x, A, Bq)), fmaf(v1, Sq, fmaf(lvf.y, A, Bq)));
-                                *reinterpret_cast<uint16_t *>(col + pzs[r] * DT_STRIDE) = (uint16_t)X;
-                                *reinterpret_cast<uint16_t *>(col + pzs[r + 1] * DT_STRIDE) = (uint16_t)(X >> 16);
+                                for (int r = KOUT - 1; r >= 0; --r) {
+                                    const uint32_t pz = 31 - __clz(bits);
+                                    bits ^= 1u << pz;
+                                    pzs[r] = pz;
+                                    cbs[r] = code_byte(pz);
+                                }
+#pragma unroll
+                                for (int r = 0; r < KOUT; r += 2) {
+                                    const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
+                                    const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
+                                    const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
+                                    const float v0 = __uint_as_float(((cbs[r] << sh) & 0x600000u) | 0x3F800000u);
+                                    const float v1 = __uint_as_float(((cbs[r + 1] << sh) & 0x600000u) | 0x3F800000u);
+                                    const uint32_t X = f16x2_of_bf16_rounded(fmaf(v0, Sq, fmaf(lvf.x, A, Bq)), fmaf(v1, Sq, fmaf(lvf.y, A, Bq)));
+                                    *reinterpret_cast<uint16_t *>(col + pzs[r] * DT_STRIDE) = (uint16_t)X;
+                                    *reinterpret_cast<uint16_t *>(col + pzs[r + 1] * DT_STRIDE) = (uint16_t)(X >> 16);
+                                }
                             }
                         } else {
                             or_status(p.status, OMMX_ST_BAD_GROUP);   // bitmask and value stream disagree
