@@ -39,7 +39,7 @@ struct S2Params {
     const __nv_bfloat16 *k_tail, *v_tail;
     int64_t t_sb, t_st, t_sh;
     const int32_t *b_tail_len, *b_seq_len;
-    int32_t max_tail;
+    int32_t max_tail, v_vec_ok;          // v_vec_ok: four adjacent V elements may be fetched as one 8-byte word
     const float *al;
     int64_t al_sb, al_sh, al_ss;
     int32_t S, B, ncta, waves;           // ncta: CTAs stage 1 shared the groups over (0: equal splits per sequence)
@@ -57,22 +57,24 @@ struct S2Params {
     int32_t *status;
 };
 
+typedef void (*Stage2Kernel)(S2Params);
 constexpr int S2_MAX_TAIL = 256;
 constexpr int S2_MAX_SPLITS = 1024;
 
 // One CTA per (query head, sequence).  Warps stripe over the bf16 residual rows for the logits,
 // then over the splits for the combine; every loop keeps many independent loads in flight,
 // because this kernel is pure latency (a few hundred KB through L2).
-// Three sizes, by what the rows of the grid need to run side by side (chosen in launch_stage2).  16 warps: one CTA per SM, all
-// of a row's loads are one round trip.  8 warps: three per SM.  4 warps: six per SM.  1024 rows (batch 32, 32 heads) took 31 us
-// with 16 warps and take 15 with 4; 512 rows 18 -> 8.7; 256 rows 9.8 -> 6.8 (8 warps).
-template <int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : (NW == 8 ? 3 : 6)) decode_stage2_kernel(const S2Params p) {
-    __shared__ float s_q[HD];
-    __shared__ float s_logit[S2_MAX_TAIL];
+// Four sizes (NW warps, PER_SM blocks to an SM), by what the rows of the grid need to run side by side (chosen in
+// launch_stage2): the more registers a row can have, the more of its loads are in flight at once, but a second round of blocks
+// costs more than that gains.  What it adds to a layer behind stage 1, against one row to 16 / 8 / 4 warps with a load
+// round for every six residual rows: 32 rows 4.3 -> 3.6 us, 256 rows 6.3 -> 3.9, 512 rows 10.3 -> 5.7, 1024 rows 16.7 -> 9.1,
+// 2048 rows 22.0 -> 11.9.  Spills undo it (80 registers at <8, 3>: 6.2 us for 256 rows).
+template <int NW, int PER_SM>
+__global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2Params p) {
+    __shared__ __align__(16) float s_q[HD];
     __shared__ float s_w[NW];
     __shared__ float s_red[NW];
-    __shared__ float s_acc[NW][HD];
+    __shared__ __align__(16) float s_acc[NW][HD];
     // the next kernel in the stream (the following layer's stage 1) may be placed as SMs free up; it waits for
     // this grid to finish before it touches memory
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -112,65 +114,99 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : (NW == 8 ? 3 : 6)) dec
     }
     const float *base = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh;
 
-    constexpr int PRE_T = NW == 16 ? 5 : 6, PRE_S = NW == 16 ? 10 : 5;   // rows / splits per warp held in registers
-    // ---- bf16 residual rows: logits of this q head (independent of stage 1) ----
-    // The K rows of this warp (rows warp, warp+16, ...) are requested together, before the query is in shared memory:
-    // this part runs after stage 1 whenever stage 1 fills every SM, so each round trip saved is a round trip per layer.
+    constexpr int PRE_S = NW == 16 ? 10 : 5;                              // splits per warp held in registers
+    // ---- bf16 residual rows of this q head: they do not depend on stage 1, so everything about them happens before its end is
+    //      waited for ----
+    // A warp takes rows warp, warp + NW, ..., four of them at a time for the logits: eight lanes to a row, three exchanges
+    // for four rows, and KB such batches in flight at once, K and V together: the rows a window usually has (8 + 32 + up to 31) in
+    // one turn of the loop, in two where seven blocks share an SM's registers.
+    constexpr int KB = NW == 16 ? 2 : (PER_SM == 4 ? 5 : 3);
+    float m_t = -INFINITY, den_t = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;    // v: channels 4 lane .. 4 lane + 3
     if (tail > 0) {
-        const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh;
-        uint2 kpre[PRE_T];
-        auto load_k = [&](int r0) __attribute__((always_inline)) {
-#pragma unroll
-            for (int k = 0; k < PRE_T; ++k) {
-                const int r = r0 + k * NW;
-                kpre[k] = make_uint2(0u, 0u);
-                if (r < tail) kpre[k] = *reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 4 * lane);
-            }
-        };
-        load_k(warp);
-        if (tid < D) s_q[tid] = __bfloat162float(p.q[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid]);
-        __syncthreads();
-        const float q0 = s_q[4 * lane], q1 = s_q[4 * lane + 1], q2 = s_q[4 * lane + 2], q3 = s_q[4 * lane + 3];
-        auto logit_of = [&](const uint2 kv) {
-            float d = q0 * bf16_bits_to_f32(kv.x & 0xFFFFu) + q1 * bf16_bits_to_f32(kv.x >> 16)
-                    + q2 * bf16_bits_to_f32(kv.y & 0xFFFFu) + q3 * bf16_bits_to_f32(kv.y >> 16);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, o);
-            float x = d * p.sm_scale;
-            if (p.logit_cap > 0.f) x = p.logit_cap * tanhf(x / p.logit_cap);
-            return x;
-        };
+        const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * (lane & 7);
+        const __nv_bfloat16 *vt = p.v_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * lane;
 #pragma unroll 1
-        for (int r0 = warp; r0 < tail; r0 += PRE_T * NW) {
-            if (r0 != warp) load_k(r0);
+        for (int r0 = warp; r0 - warp < tail; r0 += NW * 4 * KB) {
+            uint2 kx[KB][4], vx[4 * KB];                                 // K: channels 4 (lane % 8) + 32 i of row lane / 8 of the batch
 #pragma unroll
-            for (int k = 0; k < PRE_T; ++k) {
-                const int r = r0 + k * NW;
-                if (r < tail) {                                          // warp-uniform
-                    const float x = logit_of(kpre[k]);
-                    if (lane == 0) s_logit[r] = x;
+            for (int k = 0; k < KB; ++k) {
+                const int r = r0 + NW * (4 * k + (lane >> 3));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    kx[k][i] = make_uint2(0u, 0u);
+                    if (r < tail) kx[k][i] = *reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 32 * i);
                 }
             }
-        }
-    }
-    // residual V rows of this warp (rows warp, warp+16, ...), requested before the wait below: they do not depend on stage 1
-    const __nv_bfloat16 *vt = p.v_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh;
-    uint32_t vpre[PRE_T][4];                                             // raw bf16 bits: turned into floats where they are used
+            auto load_v = [&](int k) __attribute__((always_inline)) {
+                const int r = r0 + NW * k;
+                vx[k] = make_uint2(0u, 0u);
+                if (r < tail) {
+                    const __nv_bfloat16 *row = vt + (int64_t)r * p.t_st;
+                    if (p.v_vec_ok) vx[k] = *reinterpret_cast<const uint2 *>(row);
+                    else {
+                        const uint16_t *e = reinterpret_cast<const uint16_t *>(row);
+                        vx[k] = make_uint2(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16));
+                    }
+                }
+            };
+            constexpr int V_FIRST = PER_SM == 1 ? 4 * KB : (PER_SM <= 4 ? 2 * KB : KB);   // the registers of the K rows hold the others
 #pragma unroll
-    for (int k = 0; k < PRE_T; ++k) {
-        const int r = warp + k * NW;
-        vpre[k][0] = vpre[k][1] = vpre[k][2] = vpre[k][3] = 0u;
-        if (r < tail) {
-            const uint16_t *row = reinterpret_cast<const uint16_t *>(vt + (int64_t)r * p.t_st);
-            vpre[k][0] = row[lane]; vpre[k][1] = row[lane + 32]; vpre[k][2] = row[lane + 64]; vpre[k][3] = row[lane + 96];
+            for (int k = 0; k < V_FIRST; ++k) load_v(k);
+            if (r0 == warp) {
+                if (tid < D) s_q[tid] = __bfloat162float(p.q[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid]);
+                __syncthreads();
+            }
+            float x[KB], mx = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < KB; ++k) x[k] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 q = *reinterpret_cast<const float4 *>(s_q + 4 * (lane & 7) + 32 * i);
+#pragma unroll
+                for (int k = 0; k < KB; ++k)
+                    x[k] += q.x * bf16_bits_to_f32(kx[k][i].x & 0xFFFFu) + q.y * bf16_bits_to_f32(kx[k][i].x >> 16)
+                          + q.z * bf16_bits_to_f32(kx[k][i].y & 0xFFFFu) + q.w * bf16_bits_to_f32(kx[k][i].y >> 16);
+            }
+#pragma unroll
+            for (int k = V_FIRST; k < 4 * KB; ++k) load_v(k);
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) x[k] += __shfl_xor_sync(0xFFFFFFFFu, x[k], o);
+                x[k] *= p.sm_scale;
+                if (p.logit_cap > 0.f) x[k] = p.logit_cap * tanhf(x[k] / p.logit_cap);
+                if (r0 + NW * (4 * k + (lane >> 3)) >= tail) x[k] = -INFINITY;
+                mx = fmaxf(mx, x[k]);
+            }
+            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 16));
+            const float m_new = fmaxf(m_t, mx), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_t - m_use);
+            m_t = m_new;
+            den_t *= corr; v0 *= corr; v1 *= corr; v2 *= corr; v3 *= corr;
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+                x[k] = __expf(x[k] - m_use);                             // 0 for the rows past the end
+                den_t += x[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4 * KB; ++k) {
+                const float w = __shfl_sync(0xFFFFFFFFu, x[k >> 2], 8 * (k & 3));
+                v0 += w * bf16_bits_to_f32(vx[k].x & 0xFFFFu); v1 += w * bf16_bits_to_f32(vx[k].x >> 16);
+                v2 += w * bf16_bits_to_f32(vx[k].y & 0xFFFFu); v3 += w * bf16_bits_to_f32(vx[k].y >> 16);
+            }
         }
+        den_t += __shfl_xor_sync(0xFFFFFFFFu, den_t, 8);
+        den_t += __shfl_xor_sync(0xFFFFFFFFu, den_t, 16);
     }
+    // the channels lane + 32 i, as the rows of the splits are read
+    *reinterpret_cast<float4 *>(&s_acc[warp][4 * lane]) = make_float4(v0, v1, v2, v3);
+    __syncwarp();
+    float a0 = s_acc[warp][lane], a1 = s_acc[warp][lane + 32], a2 = s_acc[warp][lane + 64], a3 = s_acc[warp][lane + 96];
     // ---- everything below reads what stage 1 wrote: wait for that grid (no-op without a
     //      programmatic launch) ----
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // Every warp folds its own splits (warp, warp+16, ...) and its own residual rows into a private softmax state -
-    // maximum, sum of weights, weighted rows - with no exchange: the lse of a split is read by all lanes at once (one
-    // address), the residual logits of rows warp, warp+16, ... were written by this very warp.  The 16 states are
+    // Every warp folds its own splits (warp, warp + NW, ...) into its softmax state of the residual rows - maximum, sum of
+    // weights, weighted rows - with no exchange: the lse of a split is read by all lanes at once (one address).  The NW states are
     // merged once at the end.  The split rows are requested together with the lse values, not after the weights are
     // known: the kernel is a chain of global round trips and this takes one link out of it.
     float spre[PRE_S][4], lpre[PRE_S];
@@ -185,15 +221,15 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : (NW == 8 ? 3 : 6)) dec
             lpre[k] = row[D];
         }
     }
-    __syncwarp();                                                        // s_logit rows of this warp (lane 0 wrote them)
-    float m_w = -INFINITY;
+    float m_w = m_t;
 #pragma unroll
     for (int k = 0; k < PRE_S; ++k) m_w = fmaxf(m_w, lpre[k]);
     for (int s = warp + PRE_S * NW; s < nsplit; s += NW) m_w = fmaxf(m_w, base[(int64_t)s * p.al_ss + D]);
-    for (int r = warp; r < tail; r += NW) m_w = fmaxf(m_w, s_logit[r]);
     const float m_safe = (m_w == -INFINITY) ? 0.f : m_w;
     // weighted sum: lane owns channels lane + 32*i
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, den_w = 0.f;
+    const float f_t = __expf(m_t - m_safe);                              // 0 without residual rows
+    float den_w = den_t * f_t;
+    a0 *= f_t; a1 *= f_t; a2 *= f_t; a3 *= f_t;
 #pragma unroll
     for (int k = 0; k < PRE_S; ++k) {
         const float w = __expf(lpre[k] - m_safe);                        // exp(-inf) = 0 for the slots past nsplit
@@ -207,31 +243,11 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : (NW == 8 ? 3 : 6)) dec
         den_w += w;
         a0 += w * row[lane]; a1 += w * row[lane + 32]; a2 += w * row[lane + 64]; a3 += w * row[lane + 96];
     }
-    if (tail > 0) {
-#pragma unroll
-        for (int k = 0; k < PRE_T; ++k) {
-            const int r = warp + k * NW;
-            if (r < tail) {
-                const float w = __expf(s_logit[r] - m_safe);
-                den_w += w;
-                a0 += w * bf16_bits_to_f32(vpre[k][0]); a1 += w * bf16_bits_to_f32(vpre[k][1]);
-                a2 += w * bf16_bits_to_f32(vpre[k][2]); a3 += w * bf16_bits_to_f32(vpre[k][3]);
-            }
-        }
-#pragma unroll 4
-        for (int r = warp + PRE_T * NW; r < tail; r += NW) {
-            const __nv_bfloat16 *row = vt + (int64_t)r * p.t_st;
-            const float w = __expf(s_logit[r] - m_safe);
-            den_w += w;
-            a0 += w * __bfloat162float(row[lane]); a1 += w * __bfloat162float(row[lane + 32]);
-            a2 += w * __bfloat162float(row[lane + 64]); a3 += w * __bfloat162float(row[lane + 96]);
-        }
-    }
     s_acc[warp][lane] = a0; s_acc[warp][lane + 32] = a1;
     s_acc[warp][lane + 64] = a2; s_acc[warp][lane + 96] = a3;
     if (lane == 0) { s_red[warp] = m_w; s_w[warp] = den_w; }
     __syncthreads();
-    // ---- merge of the 16 states ----
+    // ---- merge of the NW states ----
     float out = 0.f;
     if (tid < D) {
         float g_max = s_red[0];
@@ -590,6 +606,7 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
     p.t_sb = a->tail_stride_b; p.t_st = a->tail_stride_t; p.t_sh = a->tail_stride_h;
     p.b_tail_len = a->max_tail_len > 0 ? a->b_tail_len : nullptr; p.b_seq_len = a->b_seq_len;
     p.max_tail = a->max_tail_len;
+    p.v_vec_ok = (((uintptr_t)a->v_tail & 7) == 0 && a->tail_stride_b % 4 == 0 && a->tail_stride_t % 4 == 0 && a->tail_stride_h % 4 == 0) ? 1 : 0;
     p.al = a->attn_logits; p.al_sb = a->al_stride_b; p.al_sh = a->al_stride_h; p.al_ss = a->al_stride_s;
     p.S = a->max_seq_len > 0 ? a->num_kv_splits : 0;
     p.B = a->batch; p.ncta = p.waves = 0;
@@ -606,21 +623,24 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
         p.g_world = g->world; p.g_rank = g->rank; p.g_recv = g->recv; p.g_out = g->out; p.g_state = g->state;
     }
     int warps;
+    Stage2Kernel kernel;
     {
         // Stage 1 runs with the largest shared-memory carve-out; asking for the same split here spares the SMs a
         // reconfiguration between the two kernels of every layer.
+        static const Stage2Kernel all[] = {decode_stage2_kernel<16, 1>, decode_stage2_kernel<8, 2>, decode_stage2_kernel<4, 4>, decode_stage2_kernel<4, 7>};
         static std::atomic<int> carve_set[MAX_DEVICES];
         int dev = 0;
         if (int rc = current_device(&dev)) return rc;
         if (carve_set[dev].load(std::memory_order_acquire) == 0) {
-            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel<16>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel<8>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-            OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage2_kernel<4>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+            for (Stage2Kernel k : all)
+                OMMX_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
             carve_set[dev].store(1, std::memory_order_release);
         }
-        // the largest CTAs of which all rows still run at once; past three rows per SM the small ones win even in several rounds
-        const long long rows = (long long)a->n_q_heads * a->batch;
-        warps = rows <= sm_count_of(dev) ? 16 : (rows <= 3 * sm_count_of(dev) ? 8 : 4);
+        // the largest CTAs of which all rows still run at once
+        const long long rows = (long long)a->n_q_heads * a->batch, sms = sm_count_of(dev);
+        const int size = rows <= sms ? 0 : (rows <= 2 * sms ? 1 : (rows <= 4 * sms ? 2 : 3));
+        kernel = all[size];
+        warps = size == 0 ? 16 : (size == 1 ? 8 : 4);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a->n_q_heads, a->batch);
@@ -632,8 +652,7 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
     attr[0].val.programmaticStreamSerializationAllowed = 1;   // overlap this kernel's prologue with stage 1's tail
     cfg.attrs = attr;
     cfg.numAttrs = (after_stage1 && a->max_seq_len > 0) ? 1 : 0;
-    OMMX_CUDA_TRY(warps == 16 ? cudaLaunchKernelEx(&cfg, decode_stage2_kernel<16>, p)
-                              : (warps == 8 ? cudaLaunchKernelEx(&cfg, decode_stage2_kernel<8>, p) : cudaLaunchKernelEx(&cfg, decode_stage2_kernel<4>, p)));
+    OMMX_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
     count_launch();
     return 0;
 }

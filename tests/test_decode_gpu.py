@@ -121,6 +121,16 @@ def test_decode_groups_shared_over_the_ctas(lens, H, splits):
     _run_and_check(Case(lens, H=H, Hq=4 * H, seed=17), num_kv_splits=splits)
 
 
+@pytest.mark.parametrize("Hq,aligned", [(8, True), (16, True), (32, True), (64, True), (8, False), (64, False)])
+def test_decode_residual_row_counts(Hq, aligned):
+    """Residual rows around the batches and turns of stage 2's loop, in each of its block sizes."""
+    case = Case([1, 4, 5, 48, 49, 80, 81, 128, 129, 256, 1400], Hq=Hq, seed=19, recent=216)
+    if not aligned:
+        v = torch.empty(case.v_tail.numel() + 1, dtype=torch.bfloat16, device="cuda")[1:].view(case.v_tail.shape)
+        case.v_tail = v.copy_(case.v_tail)
+    _run_and_check(case, num_kv_splits=5)
+
+
 def test_decode_tail_only_and_empty():
     case = Case([30, 8, 71], seed=2)                 # nothing quantized anywhere
     o, lse = case.run()
