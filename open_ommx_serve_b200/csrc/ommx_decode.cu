@@ -467,10 +467,7 @@ static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes,
     return true;
 }
 
-static size_t stage1_smem(const S1Params &p) {
-    return 1024 + (size_t)p.nstages * p.stage_bytes + (size_t)NCW * DT_BYTES + 64 + (2 * MAX_STAGES + (2 + MAX_STAGES) * NCW) * 8
-           + (size_t)p.GS * (4 * p.ppg + 6) * (sizeof(CopyDesc) + 4) + MAX_PIECES * sizeof(Piece);   // copy roles, their table entries, pieces
-}
+static size_t stage1_smem(const S1Params &p) { return stage1_smem(p.nstages, p.stage_bytes, p.GS, p.ppg); }
 
 // CTAs of a stage-1 launch: one per SM, or one per group where there are fewer groups than SMs; and the rounds of them
 // that equal splits would take (capped: past the cap they are never the choice)
@@ -583,9 +580,9 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st, bool tc) {
     }
     // deepest ring that fits the 227 KB a CTA may use
     p.nstages = MAX_STAGES;
-    while (p.nstages > 2 && stage1_smem(p) > 232448) --p.nstages;
+    while (p.nstages > 2 && stage1_smem(p) > SMEM_LIMIT) --p.nstages;
     const size_t smem = stage1_smem(p);
-    if (smem > 232448) return fail(OMMX_E_UNSUPPORTED, "stage 1 planes of one group do not fit shared memory");
+    if (smem > SMEM_LIMIT) return fail(OMMX_E_UNSUPPORTED, "stage 1 planes of one group do not fit shared memory");
     if (int rc = stage1_ctas(a, &p.ncta, &p.waves)) return rc;
     switch (p.H) {
         case 8: return launch_stage1_h8(p, smem, st);

@@ -40,7 +40,7 @@ constexpr int DT_ROWS = 37;             // rows 0..31: outlier deltas [token][ch
 constexpr int DT_BYTES = DT_ROWS * DT_STRIDE;
 constexpr int MAX_SPLIT_GROUPS = 512;   // groups of the longest split that the entry points accept (16K tokens)
 constexpr int MAX_SPLIT_PAGES = 1024;
-constexpr int MAX_PIECES = 256;         // pieces of sequences one CTA can work on (32 bytes of shared memory each)
+constexpr int MAX_PIECES = 128;         // pieces of sequences one CTA can work on (32 bytes of shared memory each)
 constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;   // about a second of SM clock: the wait has failed
 
 struct S1Params {
@@ -272,6 +272,18 @@ __device__ __forceinline__ void code_bit_planes(uint32_t addr, int lane, uint32_
 __device__ __forceinline__ int ring_slot(int it, int ns) { return ns == 4 ? (it & 3) : it % ns; }
 __device__ __forceinline__ uint32_t ring_phase(int it, int ns) { return (uint32_t)(ns == 4 ? (it >> 2) : it / ns) & 1u; }
 
+// the bits of a pair's position stream (two streams of `bytes` bytes, k positions each) that only positions past 31 set
+struct PositionBits { uint32_t word[8]; };
+__host__ __device__ constexpr PositionBits past_31_bits(int k, int bytes) {
+    PositionBits m = {};
+    for (int i = 0; i < 2 * k; ++i)
+        for (int b = 5; b < 7; ++b) {
+            const int at = (i < k ? 0 : 8 * bytes) + 7 * (i % k) + b;
+            m.word[at >> 5] |= 1u << (at & 31);
+        }
+    return m;
+}
+
 // ---- how the groups of a launch are shared out over its CTAs ------------------------------------------
 // The packed groups of all sequences form one running list, and CTA i takes groups [i * per, (i + 1) * per) of it, whatever
 // sequences they belong to: every CTA has the same work up to one group, also when the lengths are ragged (32 sequences of
@@ -403,6 +415,11 @@ template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk
     return true;
 }
 
+constexpr size_t SMEM_LIMIT = 232448;   // what a CTA may ask for
+constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_per_group) {       // last line: copy roles, their table entries, pieces
+    return 1024 + (size_t)stages * stage_bytes + (size_t)NCW * DT_BYTES + 64 + (2 * MAX_STAGES + (2 + MAX_STAGES) * NCW) * 8
+           + (size_t)groups * (4 * pages_per_group + 6) * (sizeof(CopyDesc) + 4) + MAX_PIECES * sizeof(Piece);
+}
 // KOUT: outliers per K vector known at compile time (static, unrolled splice) or -1 (runtime).
 //
 // Every MMA is m16n8k16 fp16 with the 2-bit codes as the A operand: a code field masked in place is an
@@ -424,19 +441,22 @@ template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk
 // and PLAIN -> with them: 64K tokens x 8 heads 50.2 -> 40.8 us; 8 x 32K 184 -> 143.9 us; 32 sequences of 1K to 32K in
 // splits of 512 with the store and stage 2 around it 560 -> 328 us.
 //
-// PLAIN: the recipe that is served - bitmask index, outlier map, no logit cap, no differential-timing knob, a page layout that
+// PLAIN: the recipes that are served - bitmask or relidx7 index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
 // form keeps them at run time; its tests and address arithmetic inside the unit cost it 10 % (70B heads 8 x 32K: 160.6 us
 // against 143.9 us).
-template <int KOUT, int H> struct PlainLayout {
-    static constexpr int NB = KOUT > 0 ? (KOUT + 1) / 2 : 0;
+// IDX7 (plain form only): relidx7 positions instead of bitmasks, turned into masks by three instructions a position.  At run time, byte
+// by byte, they took longer than the rest of the tile: 64K x 8 heads, both stages, k = 6 66.3 -> 45.9 us, k = 12 94.9 -> 58.7.
+template <int KOUT, int H, bool IDX7> struct PlainLayout {
+    static constexpr int NB = KOUT > 0 ? (KOUT + 1) / 2 : 0, NBI = IDX7 ? (7 * KOUT + 7) / 8 : 4;
     static constexpr int VM = H * 1024, VS = H * 2048, VZ = VS + H * 128, KS = VZ + H * 256, KZ = KS + H * 128, MS = KZ + H * 256, MC = MS + H * 256,
-                         BM = MC + H * 256, OV = BM + H * 512;
+                         BM = MC + H * 256, OV = BM + H * 128 * NBI;
     static constexpr int ROUND = H >= 4 ? 1024 : 128;
     static constexpr int GB = (OV + H * 128 * NB + ROUND - 1) / ROUND * ROUND;
-    static constexpr int STAGES = KOUT <= 8 ? 4 : 3;
+    static constexpr int STAGES = stage1_smem(4, NCW / H * GB, NCW / H, 2) <= SMEM_LIMIT ? 4 : 3;   // with 16-token pages
+    static_assert(stage1_smem(STAGES, NCW / H * GB, NCW / H, 2) <= SMEM_LIMIT, "the ring fits");
 };
-template <int KOUT, int H, bool PLAIN>
+template <int KOUT, int H, bool PLAIN, bool IDX7>
 __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kernel(const __grid_constant__ S1Params p) {
     constexpr bool WIDE = WarpLayout<H>::WIDE;
     constexpr int NDW = WarpLayout<H>::NDW, NPW = WarpLayout<H>::NPW, PRODUCER_WARP = WarpLayout<H>::PRODUCER_WARP;
@@ -450,14 +470,14 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     const int cta = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     static_assert(!PLAIN || KOUT >= 0, "the plain form knows its outlier count");
-    typedef PlainLayout<KOUT, H> L;
+    typedef PlainLayout<KOUT, H, IDX7> L;
     const int NS = PLAIN ? L::STAGES : p.nstages;
     const int gb_bytes = PLAIN ? L::GB : p.gb_bytes, stage_bytes = PLAIN ? GS * L::GB : p.stage_bytes;
     const int o_vm = PLAIN ? L::VM : p.o_vm, o_vs = PLAIN ? L::VS : p.o_vs, o_vz = PLAIN ? L::VZ : p.o_vz, o_ks = PLAIN ? L::KS : p.o_ks,
               o_kz = PLAIN ? L::KZ : p.o_kz, o_ms = PLAIN ? L::MS : p.o_ms, o_mc = PLAIN ? L::MC : p.o_mc, o_bm = PLAIN ? L::BM : p.o_bm,
               o_ov = PLAIN ? L::OV : p.o_ov;
     const int abl = PLAIN ? 0 : p.abl;
-    const bool use_map = PLAIN || p.use_map, idx7 = !PLAIN && p.idx7;
+    const bool use_map = PLAIN || p.use_map, idx7 = PLAIN ? IDX7 : p.idx7;
     const int k_out = KOUT >= 0 ? KOUT : p.k_out;
     const long long wait_limit = (abl & ABL_TEST_STALL) ? TEST_WAIT_LIMIT_CYCLES : WAIT_LIMIT_CYCLES;
 
@@ -703,20 +723,45 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 } else {
                     // relidx7 (attention/codec.py:91-130 of the reference): k ascending token positions, 7 bits each,
                     // LSB first; the outlier set as a bitmask again, the value stream is shared with that encoding
-                    uint32_t m2[2];
+                    uint32_t m2[2] = {0u, 0u};
+                    if constexpr (KOUT > 0) {
+                        // both channels' streams are 2 * NBI bytes back to back, 4-byte aligned where that is whole words
+                        constexpr int NBI = (7 * KOUT + 7) / 8, NW = (2 * NBI + 3) / 4;
+                        constexpr PositionBits PAST = past_31_bits(KOUT, NBI);
+                        const uint8_t *ip = gb + o_bm + (h * 128 + d0) * NBI;
+                        uint32_t w[NW + 1] = {}, past = 0u;
+                        if constexpr (NBI % 2 == 0) {
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const uint8_t *ip = gb + o_bm + (h * 128 + d0 + c) * p.nbi;
-                        uint32_t w[5] = {0u, 0u, 0u, 0u, 0u};
-                        for (int i = 0; i < p.nbi; ++i) w[i >> 2] |= (uint32_t)ip[i] << (8 * (i & 3));
-                        uint32_t bits = 0u;
-                        for (int r = 0; r < k_out; ++r) {
-                            const int bp = 7 * r;
-                            const uint32_t f = __funnelshift_r(w[bp >> 5], w[(bp >> 5) + 1], bp & 31) & 0x7Fu;
-                            if (f > 31u) or_status(p.status, OMMX_ST_BAD_GROUP);
-                            else bits |= 1u << f;
+                            for (int i = 0; i < NW; ++i) w[i] = reinterpret_cast<const uint32_t *>(ip)[i];
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < NBI; ++i) w[i >> 1] |= (uint32_t)reinterpret_cast<const uint16_t *>(ip)[i] << (16 * (i & 1));
                         }
-                        m2[c] = bits;
+#pragma unroll
+                        for (int i = 0; i < NW; ++i) past |= w[i] & PAST.word[i];
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+#pragma unroll
+                            for (int r = 0; r < KOUT; ++r) {
+                                const int bp = 8 * NBI * c + 7 * r;
+                                m2[c] |= __funnelshift_l(0u, 1u, __funnelshift_r(w[bp >> 5], w[(bp >> 5) + 1], bp & 31));   // 1 << its low five bits
+                            }
+                        if (past) m2[0] = m2[1] = 0u;                    // reported below: no mask of k bits
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const uint8_t *ip = gb + o_bm + (h * 128 + d0 + c) * p.nbi;
+                            uint32_t w[5] = {0u, 0u, 0u, 0u, 0u};
+                            for (int i = 0; i < p.nbi; ++i) w[i >> 2] |= (uint32_t)ip[i] << (8 * (i & 3));
+                            uint32_t bits = 0u;
+                            for (int r = 0; r < k_out; ++r) {
+                                const int bp = 7 * r;
+                                const uint32_t f = __funnelshift_r(w[bp >> 5], w[(bp >> 5) + 1], bp & 31) & 0x7Fu;
+                                if (f > 31u) or_status(p.status, OMMX_ST_BAD_GROUP);
+                                else bits |= 1u << f;
+                            }
+                            m2[c] = bits;
+                        }
                     }
                     bm2 = make_uint2(m2[0], m2[1]);
                 }
@@ -1307,7 +1352,7 @@ static int sm_count_of(int dev) {
     return n;
 }
 
-template <int KOUT, int H, bool PLAIN>
+template <int KOUT, int H, bool PLAIN, bool IDX7>
 static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     using L = WarpLayout<H>;
     // function attributes belong to (kernel instantiation, device): one entry per device ordinal
@@ -1318,7 +1363,7 @@ static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     int regs_ok = regs_state[dev].load(std::memory_order_acquire);
     if (regs_ok == 0) {
         cudaFuncAttributes fa;
-        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, H, PLAIN>));
+        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, H, PLAIN, IDX7>));
         // setmaxnreg.inc must find the registers the other roles gave back
         const int need = NCW * 32 * REGS_MMA + (L::WIDE ? L::NDW * 32 * REGS_DECODE + L::NPW * 32 * REGS_PRODUCER
                                                         : (L::THREADS - NCW * 32) * REGS_DECODE);
@@ -1327,35 +1372,38 @@ static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     }
     if (regs_ok != 1) return fail(OMMX_E_CUDA, "stage 1 was compiled with fewer registers than its warp roles need");
     if (smem > attr_smem[dev].load(std::memory_order_acquire)) {
-        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_kernel<KOUT, H, PLAIN>,
+        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_smem[dev].store(smem, std::memory_order_release);
     }
-    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H, PLAIN>, dim3(p.ncta), L::THREADS, smem, st, p));
+    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>, dim3(p.ncta), L::THREADS, smem, st, p));
     count_launch();
     return 0;
 }
-// The outlier counts of the serving recipes get the unrolled two-pass splice.
-template <int H, bool PLAIN>
-static int launch_s1_counts(const S1Params &p, size_t smem, cudaStream_t st) {
-    switch (p.k_out) {
-        case 0: return launch_s1<0, H, PLAIN>(p, smem, st);
-        case 2: return launch_s1<2, H, PLAIN>(p, smem, st);
-        case 4: return launch_s1<4, H, PLAIN>(p, smem, st);
-        case 6: return launch_s1<6, H, PLAIN>(p, smem, st);
-        case 8: return launch_s1<8, H, PLAIN>(p, smem, st);
-        case 12: return launch_s1<12, H, PLAIN>(p, smem, st);
-        default:
-            if constexpr (PLAIN) return fail(OMMX_E_UNSUPPORTED, "stage 1: outliers_per_vector=%d has no plain form", p.k_out);
-            else return launch_s1<-1, H, false>(p, smem, st);
+// The plain form where the recipe and the ring depth are its own, else the general one.
+template <int KOUT, int H>
+static int launch_s1_forms(const S1Params &p, size_t smem, cudaStream_t st) {
+    if constexpr (KOUT >= 0) {
+        if (p.abl == 0 && (KOUT == 0 || p.use_map) && p.logit_cap <= 0.f) {
+            if (!p.idx7 && p.nstages >= PlainLayout<KOUT, H, false>::STAGES) return launch_s1<KOUT, H, true, false>(p, smem, st);
+            if constexpr (KOUT > 0)
+                if (p.idx7 && p.nstages >= PlainLayout<KOUT, H, true>::STAGES) return launch_s1<KOUT, H, true, true>(p, smem, st);
+        }
     }
+    return launch_s1<KOUT, H, false, false>(p, smem, st);
 }
+// The outlier counts of the serving recipes get the unrolled two-pass splice.
 template <int H>
 static int launch_s1_heads(const S1Params &p, size_t smem, cudaStream_t st) {
-    const int k = p.k_out;
-    const bool counted = k == 0 || k == 2 || k == 4 || k == 6 || k == 8 || k == 12;
-    const bool plain = counted && p.abl == 0 && !p.idx7 && (k == 0 || p.use_map) && p.logit_cap <= 0.f && p.nstages == (k <= 8 ? 4 : 3);
-    return plain ? launch_s1_counts<H, true>(p, smem, st) : launch_s1_counts<H, false>(p, smem, st);
+    switch (p.k_out) {
+        case 0: return launch_s1_forms<0, H>(p, smem, st);
+        case 2: return launch_s1_forms<2, H>(p, smem, st);
+        case 4: return launch_s1_forms<4, H>(p, smem, st);
+        case 6: return launch_s1_forms<6, H>(p, smem, st);
+        case 8: return launch_s1_forms<8, H>(p, smem, st);
+        case 12: return launch_s1_forms<12, H>(p, smem, st);
+        default: return launch_s1_forms<-1, H>(p, smem, st);
+    }
 }
 
 // one per translation unit

@@ -74,3 +74,34 @@ def test_decode_relidx7_planes_equal_bitmask_planes(k, H, Hq):
         kv_int8_scale=True, num_kv_splits=9, max_seq_len=max(case.packed), max_tail_len=max(case.tails))
     torch.cuda.synchronize()
     assert torch.equal(o, o_bm) and torch.equal(lse, lse_bm)
+
+
+@pytest.mark.parametrize("k,H,page_size", [(2, 8, 16), (8, 8, 16), (12, 8, 16), (8, 4, 8), (12, 2, 16), (6, 1, 32), (8, 1, 8)])
+def test_decode_relidx7_outlier_counts_and_bad_position(k, H, page_size):
+    """Every unrolled count, streams that do and do not end on a word, both ring depths; a position past 31 is reported."""
+    from open_ommx_serve_b200 import _lib
+    from open_ommx_serve_b200.attention.paged_decode import ommx_paged_decode_attention_canonical
+    case = Case([2400, 72, 500], H=H, Hq=4 * H, seed=k + H, k=k, page_size=page_size)
+    o_bm, lse_bm = case.run(num_kv_splits=7)
+    obmp = case.pooled_np["k_obmp"]
+    words = obmp.reshape(-1, 4).copy().view(np.uint32)[:, 0]
+    used = np.array([bin(int(w)).count("1") == k for w in words])
+    flat = np.zeros((words.shape[0], (7 * k + 7) // 8), dtype=np.uint8)
+    flat[used] = O.relidx7_from_bitmask(obmp.reshape(-1, 4)[used], k)
+    p = case.planes
+    for bad in (False, True):
+        if bad:
+            flat[np.flatnonzero(used)[5], 0] |= 0x20
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        o, lse = torch.zeros_like(o_bm), torch.zeros_like(lse_bm)
+        ommx_paged_decode_attention_canonical(
+            case.q_dev, p["k_base"], p["k_scale"], p["k_zp"], torch.from_numpy(flat.reshape(obmp.shape[:-1] + (flat.shape[1],))).cuda(),
+            p["k_oval"], p["v_main"], p["v_scale"], p["v_zp"], case.k_tail, case.v_tail, case.b_tail_len, o, lse, case.req_to_token,
+            case.req_to_group, case.b_seq_len, sm_scale=case.sm_scale, page_size=page_size, k_outliers_per_vector=k,
+            k_fp4_mapscale=p["k_fp4_mapscale"], k_fp4_mapcenter=p["k_fp4_mapcenter"], kv_outlier_map=True, kv_int8_scale=True,
+            num_kv_splits=7, max_seq_len=max(case.packed), max_tail_len=max(case.tails), status=status)
+        torch.cuda.synchronize()
+        if bad:
+            assert int(status) == _lib.ST_BAD_GROUP and torch.isfinite(o).all()
+        else:
+            assert int(status) == 0 and torch.equal(o, o_bm) and torch.equal(lse, lse_bm)
