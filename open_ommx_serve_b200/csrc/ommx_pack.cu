@@ -249,6 +249,23 @@ __global__ void __launch_bounds__(PACK_WARPS * 32) pack_k_kernel(PackKParams p) 
     }
 }
 
+// Drops the highest tokens of `eq` from `picks` until `keep` picks are left
+__device__ __forceinline__ uint32_t drop_ties(uint32_t picks, uint32_t eq, int keep) {
+    for (int over = __popc(picks) - keep; over > 0; --over) {
+        const uint32_t bit = 0x80000000u >> __clz(eq);
+        picks ^= bit;
+        eq ^= bit;
+    }
+    return picks;
+}
+
+// a >= b afterwards
+__device__ __forceinline__ void order2(float &a, float &b) {
+    const float hi = fmaxf(a, b);
+    b = fminf(a, b);
+    a = hi;
+}
+
 // ---------------------------------------------------------------------------------------------
 // K kernel, lane-per-channel form, for the signed selection rule with a compile-time (KT, KB) =
 // (picks from the top, picks from the bottom).  One warp per (32-token group, kv head, 32-channel
@@ -349,6 +366,81 @@ __global__ void __launch_bounds__(PACK_WARPS * 32) pack_k_lane_kernel(PackKParam
         // an infinity or a NaN is the largest (smallest) key of its sign: the two ends of the order tell
         bad = top[0] >= 0xFF800000u || bot[0] < 0x00800000u;
         rounds = __any_sync(0xFFFFFFFFu, __popc(omask) != K || bad);
+    } else {
+        // The M largest and M smallest of the 32 values by a sorting network (248 min / max at M = 4; the rounds below took some 900
+        // instructions), the picks by two comparisons a token, ties by the stable-sort rule, as pack_k_pair does for 16-bit values.
+        // 8192 tokens x 8 heads, K + V: 61.5 -> 53.6 us.
+        rounds = false;
+        constexpr int M = KT >= KB ? KT + 1 : KB + 1;
+        float top[M <= 4 ? 4 : M], bot[M <= 4 ? 4 : M], zero = 0.f;
+        if constexpr (M == 1) {
+            top[0] = bot[0] = x[0];
+#pragma unroll
+            for (int t = 1; t < 32; ++t) { top[0] = fmaxf(top[0], x[t]); bot[0] = fminf(bot[0], x[t]); }
+        } else if constexpr (M <= 4) {
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                float s0 = x[4 * b], s1 = x[4 * b + 1], s2 = x[4 * b + 2], s3 = x[4 * b + 3];
+                order2(s0, s1); order2(s2, s3); order2(s0, s2); order2(s1, s3); order2(s1, s2);
+                if (b == 0) {
+                    top[0] = s0; top[1] = s1; top[2] = s2; top[3] = s3;
+                    bot[0] = s3; bot[1] = s2; bot[2] = s1; bot[3] = s0;
+                } else {
+                    // the larger (smaller) halves of two sorted fours are bitonic: two rounds sort them
+                    top[0] = fmaxf(top[0], s3); top[1] = fmaxf(top[1], s2); top[2] = fmaxf(top[2], s1); top[3] = fmaxf(top[3], s0);
+                    order2(top[0], top[2]); order2(top[1], top[3]); order2(top[0], top[1]); order2(top[2], top[3]);
+                    bot[0] = fminf(bot[0], s0); bot[1] = fminf(bot[1], s1); bot[2] = fminf(bot[2], s2); bot[3] = fminf(bot[3], s3);
+                    order2(bot[2], bot[0]); order2(bot[3], bot[1]); order2(bot[1], bot[0]); order2(bot[3], bot[2]);
+                }
+            }
+        } else {
+            // five of each: insertion, from infinities that every value pushes out
+#pragma unroll
+            for (int i = 0; i < M; ++i) { top[i] = -INFINITY; bot[i] = INFINITY; }
+#pragma unroll
+            for (int t = 0; t < 32; ++t) {
+                float c = x[t], d = c;
+#pragma unroll
+                for (int i = 0; i < M; ++i) { order2(top[i], c); order2(d, bot[i]); }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 32; ++t) zero = fmaf(x[t], 0.f, zero);       // NaN once a value is not finite
+        bad = zero != 0.f;
+        if constexpr (K > 0) {
+            const float thr_t = top[KT > 0 ? KT - 1 : 0], thr_b = bot[KB > 0 ? KB - 1 : 0];
+#pragma unroll
+            for (int t = 0; t < 32; ++t)
+                if (x[t] >= thr_t || x[t] <= thr_b) omask |= 1u << t;
+            if (__any_sync(0xFFFFFFFFu, __popc(omask) != K && !bad)) {
+                // more tokens at a threshold than picks left: the lowest of them are taken, the bottom picks among what the
+                // top picks left
+                uint32_t tm = 0, te = 0, bm = 0, be = 0;
+#pragma unroll
+                for (int t = 0; t < 32; ++t) {
+                    if (x[t] >= thr_t) tm |= 1u << t;
+                    if (x[t] == thr_t) te |= 1u << t;
+                    if (x[t] <= thr_b) bm |= 1u << t;
+                    if (x[t] == thr_b) be |= 1u << t;
+                }
+                if (!bad) {
+                    tm = drop_ties(tm, te, KT);
+                    bm &= ~tm;
+                    bm = drop_ties(bm, be & bm, KB);
+                    omask = tm | bm;
+                }
+            }
+            if (bad) omask = (1u << K) - 1u;                             // refused input: any K tokens
+            uint32_t m = omask;
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                pick_tok[r] = __ffs(m) - 1;
+                m &= m - 1u;
+                pick_key[r] = f32_key(load_as_f32(col + (int64_t)pick_tok[r] * p.stride_token));
+            }
+        }
+        kmax = f32_key(top[KT]);
+        kmin = f32_key(bot[KB]);
     }
     if (rounds) {
         uint32_t cand[32];                    // order keys; 0 marks a picked token (no finite value has key 0)
@@ -598,6 +690,13 @@ __global__ void __launch_bounds__(128) pack_v_kernel(PackVParams p) {
                 x[8 * v + 2 * i + 1] = bits16_as_f32<T>(ww[i] >> 16);
             }
         }
+    } else if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
+        // 128 contiguous bytes: eight 16-byte loads (8192 tokens x 8 heads, K + V: 53.6 -> 32.2 us)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+            const float4 w = reinterpret_cast<const float4 *>(row)[v];
+            x[4 * v] = w.x; x[4 * v + 1] = w.y; x[4 * v + 2] = w.z; x[4 * v + 3] = w.w;
+        }
     } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = load_as_f32(row + i);
@@ -693,16 +792,6 @@ __device__ __forceinline__ uint32_t fp4_code(float m) {
     const bool c1 = a >= (c2 ? c_fp4_thresh[5] : c_fp4_thresh[1]);
     const bool c0 = a >= (c2 ? (c1 ? c_fp4_thresh[6] : c_fp4_thresh[4]) : (c1 ? c_fp4_thresh[2] : c_fp4_thresh[0]));
     return (m < 0.f ? 8u : 0u) | (c2 ? 4u : 0u) | (c1 ? 2u : 0u) | (c0 ? 1u : 0u);
-}
-
-// Drops the highest tokens of `eq` from `picks` until `keep` picks are left
-__device__ __forceinline__ uint32_t drop_ties(uint32_t picks, uint32_t eq, int keep) {
-    for (int over = __popc(picks) - keep; over > 0; --over) {
-        const uint32_t bit = 0x80000000u >> __clz(eq);
-        picks ^= bit;
-        eq ^= bit;
-    }
-    return picks;
 }
 
 // col: this lane's channels 2 lane, 2 lane + 1 in row 0; the unit's destination group slot, page of every token and head

@@ -169,3 +169,24 @@ def test_pack_16_bit_inputs_with_ties(k, D, H):
             want = O.pack_kv(Kd.float().numpy(), Vd.float().numpy(), outliers_per_vector=k, use_pow2=pow2, kv_outlier_map=omap,
                              kv_int8_scale=pow2)
             assert_planes_equal(_gpu_pack(Kd, Vd, k=k, pow2=pow2, omap=omap), want, ctx=f"{dtype} pow2={pow2} map={omap}:")
+
+
+@pytest.mark.parametrize("k", [0, 2, 4, 6, 8])
+@pytest.mark.parametrize("D,H", [(96, 1), (128, 3)])
+def test_pack_fp32_inputs_with_ties(k, D, H):
+    """The same groups in fp32, with values that 16 bits cannot tell apart and infinities that are reported."""
+    g = torch.Generator().manual_seed(800 + k)
+    K, V = gaussian_kv(80 + k, 192, H, D, mag=30.0, bf16=False)
+    levels = torch.tensor([-2.0, -0.5, -0.25, 0.0, 1.0, 1.0 + 2.0 ** -23])
+    K[32:64] = levels[torch.randint(0, 6, (32, H, D), generator=g)]
+    K[64:96] = levels[torch.randint(4, 6, (32, H, D), generator=g)]
+    K[96:128] = torch.where(torch.rand(32, H, D, generator=g) < 0.5, torch.tensor(0.0), torch.tensor(3.0))
+    K[128:160] = torch.randn(1, H, D, generator=g)
+    for pow2, omap in ((True, True), (True, False), (False, True)):
+        want = O.pack_kv(K.numpy(), V.numpy(), outliers_per_vector=k, use_pow2=pow2, kv_outlier_map=omap, kv_int8_scale=pow2)
+        assert_planes_equal(_gpu_pack(K, V, k=k, pow2=pow2, omap=omap), want, ctx=f"pow2={pow2} map={omap}:")
+    for value in (float("inf"), float("-inf"), float("nan")):
+        bad = K.clone()
+        bad[37, 0, 5] = value
+        with pytest.raises(ValueError):
+            _gpu_pack(bad, V, k=k)
