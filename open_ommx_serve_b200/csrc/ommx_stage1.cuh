@@ -435,11 +435,12 @@ constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_
 // decode warps (the sidecar tile), so the MMA warps multiply and accumulate and do little else; what they
 // still compute themselves, q.zp, fits into their wait for the deltas.
 //
-// Bound by the dependent chain of an MMA warp (about 5000 cycles for a group of a head: code MMAs, delta MMAs, softmax,
-// P.V) with the decode warps that feed it close behind; the register file (8 x 128 + 16 x 56 a lane) holds no second unit
-// in flight, and memory is at a quarter of its rate.  Measured, this stage alone, before the running list, the cheaper unit
-// and PLAIN -> with them: 64K tokens x 8 heads 50.2 -> 40.8 us; 8 x 32K 184 -> 143.9 us; 32 sequences of 1K to 32K in
-// splits of 512 with the store and stage 2 around it 560 -> 328 us.
+// Bound by instruction issue and the logic pipe, which both roles share (leaving out any part of either saves its share), and in the
+// chain view by an MMA warp's unit: about 4600 cycles of code MMAs, delta MMAs, softmax and P.V in a row, with the decode warps
+// that feed it close behind; the register file (8 x 128 + 16 x 56 a lane) holds no second unit in flight, and memory is at a
+// quarter of its rate.  Measured, this stage alone, before the running list, the cheaper unit and PLAIN -> with them: 64K tokens x 8
+// heads 50.2 -> 40.1 us; 8 x 32K 184 -> 142.5 us; 32 sequences of 1K to 32K in splits of 512 with the store and stage 2 around it
+// 560 -> 318 us.
 //
 // PLAIN: the recipes that are served - bitmask or relidx7 index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
