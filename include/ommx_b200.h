@@ -319,6 +319,13 @@ int ommx_b200_merge_states(const float *o_parts, const float *lse_parts, const i
 int ommx_b200_host_pow2_exponent(float x);
 int ommx_b200_host_fp4_encode(float m);
 
+/* Host-side twin of the plan by which both decode stages share the packed groups of a batch out over CTAs (no GPU needed;
+ * b_seq_len is host memory here).  *ctas: CTAs of the stage-1 launch; *groups_per_cta: consecutive groups of the running list
+ * each of them takes, 0 = equal splits per sequence, dealt out one by one.  Returns how many pieces of sequences a CTA can
+ * list, which no plan exceeds, or a negative code. */
+int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len,
+                              int32_t sm_count, int32_t *ctas, int32_t *groups_per_cta);
+
 int ommx_b200_abi_version(void);
 const char *ommx_b200_last_error(void);   /* thread-local text of the last negative return */
 /* Kernels launched by this library since load (or since the last reset), for launch evidence;

@@ -107,6 +107,8 @@ SYMBOLS = {
                                          C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ommx_b200_host_pow2_exponent": (C.c_int, [C.c_float]),
     "ommx_b200_host_fp4_encode": (C.c_int, [C.c_float]),
+    "ommx_b200_host_share_plan": (C.c_int, [C.POINTER(C.c_int32), C.c_int32, C.c_int32, C.c_int32, C.c_int32,
+                                            C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "ommx_b200_abi_version": (C.c_int, []),
     "ommx_b200_last_error": (C.c_char_p, []),
     "ommx_b200_launch_count": (C.c_int64, []),

@@ -469,17 +469,10 @@ static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes,
 
 static size_t stage1_smem(const S1Params &p) { return stage1_smem(p.nstages, p.stage_bytes, p.GS, p.ppg); }
 
-// CTAs of a stage-1 launch: one per SM, or one per group where there are fewer groups than SMs; and the rounds of them
-// that equal splits would take (capped: past the cap they are never the choice)
 static int stage1_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
-    const long long groups = (long long)a->batch * ((a->max_seq_len + 31) / 32);
-    // (a CTA lists at most MAX_PIECES pieces: more CTAs than SMs for thousands of short sequences)
-    const long long splits = (long long)a->batch * a->num_kv_splits;
-    const long long least = (min((long long)a->batch, groups) > MAX_PIECES ? (max(groups, splits) + MAX_PIECES - 1) / MAX_PIECES : 1);
-    *ncta = (int)max(min((long long)sm_count_of(dev), max(groups, 1ll)), least);
-    *waves = (int)min((splits + *ncta - 1) / *ncta, 1024ll);
+    stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, sm_count_of(dev), ncta, waves);
     return 0;
 }
 
@@ -687,6 +680,21 @@ extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, 
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
     return max(1, best);
+}
+
+extern "C" int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
+                                         int32_t *ctas, int32_t *groups_per_cta) {
+    using namespace ommx;
+    if (!b_seq_len || !ctas || !groups_per_cta || batch < 1 || num_kv_splits < 1 || sm_count < 1)
+        return fail(OMMX_E_ARG, "host_share_plan: batch=%d num_kv_splits=%d sm_count=%d", batch, num_kv_splits, sm_count);
+    int total = 0, longest = 0, waves = 0;
+    for (int i = 0; i < batch; ++i) {
+        total += groups_of(b_seq_len[i]);
+        longest = max(longest, groups_of(b_seq_len[i]));
+    }
+    stage1_grid(batch, num_kv_splits, max_seq_len, sm_count, ctas, &waves);
+    *groups_per_cta = share_plan_of(total, longest, batch, num_kv_splits, *ctas, waves).per;
+    return MAX_PIECES;
 }
 
 extern "C" int ommx_b200_decode_stage1(const ommx_decode_args *a, void *stream) {

@@ -286,17 +286,19 @@ __host__ __device__ constexpr PositionBits past_31_bits(int k, int bytes) {
 
 // ---- how the groups of a launch are shared out over its CTAs ------------------------------------------
 // The packed groups of all sequences form one running list, and CTA i takes groups [i * per, (i + 1) * per) of it, whatever
-// sequences they belong to: every CTA has the same work up to one group, also when the lengths are ragged (32 sequences of
-// 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us around its steady state: 560 us of
-// store and decode against 363 us).  A piece of
-// a sequence writes its partial result to workspace slot (its CTA - the first CTA of the sequence), and the caller's
-// workspace has S slots per sequence, which bounds `per` from below.  Where that bound makes the shares longer than S equal
-// splits per sequence dealt out one by one would be, those are taken instead (per = 0): item x is split x % S of sequence x / S.
+// sequences they belong to (32 sequences of 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us
+// around its steady state: 560 us of store and decode against 318 us).  A piece of a sequence writes its partial result to
+// workspace slot (its CTA - the first CTA of the sequence), and the caller's workspace has S slots per sequence, which bounds `per`
+// from below: shares are even up to one group where S is generous, and longer, up to the longest sequence over S - 1, where it is not.
+// Equal splits per sequence, dealt out one by one (per = 0: item x is split x % S of sequence x / S), are taken instead
+//   * where that bound makes the shares longer than S of them per sequence would be, and
+//   * where a share could hold more sequences than a CTA lists (MAX_PIECES).  Of equal splits a CTA never has more than that:
+//     stage1_grid makes a CTA for every MAX_PIECES of them as soon as there are that many sequences.
 struct SharePlan {
     int per, total;                      // groups per CTA (0: equal splits per sequence), groups of all sequences
 };
-__device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
-__device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, int ncta, int waves) {
+__host__ __device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
+__host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, int ncta, int waves) {
     SharePlan s;
     s.total = total;
     s.per = max(1, (total + ncta - 1) / ncta);
@@ -305,9 +307,17 @@ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B
         s.per = max(s.per, equal);                             // a lone sequence starts at a CTA's beginning: exactly ceil(n / per) slots
     } else {
         if (S >= 2) s.per = max(s.per, (longest - 2) / (S - 1) + 1);   // anywhere else it touches up to (n - 2) / per + 2 CTAs
-        if (S < 2 || (waves <= MAX_PIECES && waves * equal <= s.per)) s.per = 0;
+        if (S < 2 || min(s.per, B) > MAX_PIECES || (waves <= MAX_PIECES && waves * equal <= s.per)) s.per = 0;
     }
     return s;
+}
+// CTAs of a launch - one per SM, or one per group where there are fewer; above MAX_PIECES sequences at least one for every MAX_PIECES
+// groups or splits - and the rounds of them that equal splits would take (capped: past the cap they are never the choice)
+static inline void stage1_grid(int batch, int S, int max_seq_len, int sm_count, int *ncta, int *waves) {
+    const long long groups = (long long)batch * groups_of(max_seq_len), splits = (long long)batch * S;
+    const long long least = batch > MAX_PIECES ? (max(groups, splits) + MAX_PIECES - 1) / MAX_PIECES : 1;
+    *ncta = (int)max(min((long long)sm_count, max(groups, 1ll)), least);
+    *waves = (int)min((splits + *ncta - 1) / *ncta, 1024ll);
 }
 // called by whole warps; every lane gets the same answer
 __device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, int ncta, int waves, int lane) {
@@ -645,7 +655,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         for (bool more = true; more; ++n) {
             Piece cur = pc;
             more = next_piece<GS>(pc, walk, p, plan);
-            if (more && n + 1 == MAX_PIECES) {                       // the host sizes the grid so that this cannot be
+            if (more && n + 1 == MAX_PIECES) {                       // a bounds check: share_plan_of rules it out
                 if (lane == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
                 more = false;
             }

@@ -121,6 +121,16 @@ def test_decode_groups_shared_over_the_ctas(lens, H, splits):
     _run_and_check(Case(lens, H=H, Hq=4 * H, seed=17), num_kv_splits=splits)
 
 
+@pytest.mark.parametrize("H,at,splits", [(2, 0, None), (2, 199, None), (8, 100, 3)])
+def test_decode_many_short_sequences_beside_a_longer_one(H, at, splits):
+    """More sequences in an even share than a CTA can list: 199 of one group and one of 200."""
+    lens = [72] * 200
+    lens[at] = 40 + 200 * 32
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _run_and_check(Case(lens, H=H, Hq=4 * H, seed=23), num_kv_splits=splits, status=status)
+    assert int(status.item()) == 0
+
+
 @pytest.mark.parametrize("Hq,aligned", [(8, True), (16, True), (32, True), (64, True), (8, False), (64, False)])
 def test_decode_residual_row_counts(Hq, aligned):
     """Residual rows around the batches and turns of stage 2's loop, in each of its block sizes."""

@@ -1,0 +1,89 @@
+"""How stage 1 deals the groups of a batch to its CTAs and where stage 2 looks for the results: the plan of the library
+(host twin of what both kernels compute) held to what the kernels assume of it, over random lengths and split counts."""
+import ctypes as C
+import random
+
+import pytest
+
+from open_ommx_serve_b200 import _lib
+
+SMS = 148
+
+
+def plan(groups, splits, bound):
+    """``bound``: the call's max_seq_len in multiples of the longest sequence."""
+    lens = (C.c_int32 * len(groups))(*[32 * g for g in groups])
+    ctas, per = C.c_int32(), C.c_int32()
+    limit = _lib.load().ommx_b200_host_share_plan(lens, len(groups), splits, 32 * max(groups) * bound, SMS, C.byref(ctas), C.byref(per))
+    assert limit == 128
+    return limit, ctas.value, per.value
+
+
+def pieces_of(groups, splits, ctas, per):
+    """(cta, sequence, slot, first group, groups) of every piece, as stage 1 lists them."""
+    out = []
+    if per == 0:                                            # split x % S of sequence x / S, dealt out one by one
+        for x in range(len(groups) * splits):
+            b, s = divmod(x, splits)
+            size = -(-groups[b] // splits)
+            if s * size < groups[b]:
+                out.append((x % ctas, b, s, s * size, min(size, groups[b] - s * size)))
+        return out
+    at = 0
+    for b, n in enumerate(groups):
+        for cta in range(at // per, (at + n - 1) // per + 1 if n else at // per):
+            lo, hi = max(at, cta * per), min(at + n, (cta + 1) * per)
+            out.append((cta, b, cta - at // per, lo - at, hi - lo))
+        at += n
+    return out
+
+
+def check(groups, splits, bound=1):
+    limit, ctas, per = plan(groups, splits, bound)
+    pieces = pieces_of(groups, splits, ctas, per)
+    count, slots, covered, before = {}, {}, [0] * len(groups), 0
+    for cta, b, slot, first, n in pieces:
+        assert 0 <= cta < ctas and n > 0 and first == covered[b]           # every group once, in order
+        covered[b] += n
+        count[cta] = count.get(cta, 0) + 1
+        slots.setdefault(b, []).append(slot)
+    assert covered == list(groups)
+    assert max(count.values(), default=0) <= limit, (max(count.values()), per, ctas)
+    for b, n in enumerate(groups):                          # stage 2 reads slots 0 .. count - 1 of the caller's S
+        if n == 0:
+            want = 0
+        elif per == 0:
+            want = -(-n // -(-n // splits))
+        else:
+            want = (before + n - 1) // per - before // per + 1
+        assert slots.get(b, []) == list(range(want)) and want <= splits
+        before += n
+
+
+@pytest.mark.parametrize("long", [130, 200, 254, 300])
+@pytest.mark.parametrize("n", [200, 220, 300, 1000])
+@pytest.mark.parametrize("at", [0, 100, -1])
+def test_many_short_sequences_beside_a_longer_one(n, long, at):
+    """The share that the longest sequence asks for holds more short sequences than a CTA can list."""
+    groups = [1] * n
+    groups[at] = long
+    for splits in (2, 3, 5):
+        check(groups, splits)
+        check(groups, splits, 16)
+
+
+@pytest.mark.parametrize("seed", range(300))
+def test_every_group_is_dealt_once_and_found_again(seed):
+    rng = random.Random(seed)
+    batch = int(round(600 ** rng.random())) if rng.random() < 0.7 else rng.randint(129, 600)
+    hi = int(round(512 ** rng.random()))
+    kind = rng.randrange(3)
+    groups = [rng.randint(0 if kind else hi, hi) for _ in range(batch)]
+    if kind == 2:
+        groups = [rng.randint(0, 2) for _ in range(batch)]
+        groups[rng.randrange(batch)] = hi
+    if max(groups) == 0:
+        groups[0] = 1
+    auto = _lib.load().ommx_b200_auto_num_kv_splits(32 * max(groups), batch, 8)
+    for splits in {auto, 1, rng.randint(2, 8), int(round(1024 ** rng.random()))}:
+        check(groups, splits, rng.choice((1, 1, 2, 16)))
