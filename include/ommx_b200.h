@@ -156,7 +156,7 @@ typedef struct ommx_decode_args {
     int32_t batch, n_q_heads;
     int64_t q_stride_b, q_stride_h;
     ommx_kv_planes planes;
-    const void *k_tail, *v_tail;  /* bf16 [batch, T_tail_max, n_kv_heads, head_dim] */
+    const void *k_tail, *v_tail;  /* bf16 [batch, T_tail_max, n_kv_heads, head_dim]; every k_tail row 8-byte aligned */
     int64_t tail_stride_b, tail_stride_t, tail_stride_h;
     const int32_t *b_tail_len;    /* [batch] valid residual rows (0 allowed) */
     const int32_t *b_seq_len;     /* [batch] packed tokens */

@@ -136,7 +136,7 @@ def ommx_paged_decode_attention_canonical(
 
     Arguments and plane layout are the reference's (``paged_decode.py:2856-2902``): ``q``
     bf16 ``[B,Hq,D]``; page planes ``[pages, page_size, Hkv, .]``; group planes
-    ``[group_slots, Hkv, D, .]``; ``k_tail/v_tail`` bf16 ``[B, T_tail, Hkv, D]`` with
+    ``[group_slots, Hkv, D, .]``; ``k_tail/v_tail`` bf16 ``[B, T_tail, Hkv, D]`` (rows of ``k_tail`` 8-byte aligned) with
     ``b_tail_len`` valid rows; ``req_to_token`` / ``req_to_group`` int32 or int64 tables;
     ``b_seq_len`` packed token counts.  Pass ``max_seq_len``, ``max_tail_len`` and
     ``attn_logits`` (f32 ``[B,Hq,S+1,D+1]``) to avoid every host sync and allocation, which

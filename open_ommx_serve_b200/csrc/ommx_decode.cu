@@ -385,6 +385,11 @@ static int validate_decode(const ommx_decode_args *a) {
     if (a->max_tail_len > S2_MAX_TAIL) return fail(OMMX_E_UNSUPPORTED, "decode: max_tail_len=%d (max %d)", a->max_tail_len, S2_MAX_TAIL);
     if (a->max_tail_len > 0 && (!a->k_tail || !a->v_tail || !a->b_tail_len))
         return fail(OMMX_E_ARG, "decode: max_tail_len>0 needs k_tail, v_tail and b_tail_len");
+    // stage 2 reads K rows in 8-byte words; a stride that no index goes along may be anything
+    if (a->max_tail_len > 0 && (((uintptr_t)a->k_tail & 7) != 0 || (a->batch > 1 && a->tail_stride_b % 4 != 0) ||
+                                (a->max_tail_len > 1 && a->tail_stride_t % 4 != 0) || (pl.n_kv_heads > 1 && a->tail_stride_h % 4 != 0)))
+        return fail(OMMX_E_ARG, "decode: k_tail rows must start on 8-byte boundaries (base %% 8 = %d bytes, strides %lld, %lld, %lld elements)",
+                    (int)((uintptr_t)a->k_tail & 7), (long long)a->tail_stride_b, (long long)a->tail_stride_t, (long long)a->tail_stride_h);
     if (a->max_seq_len > 0) {
         if (!a->req_to_token || !a->req_to_group) return fail(OMMX_E_ARG, "decode: page / group tables are null");
         if (!pl.k_base || !pl.k_scale || !pl.k_zp || !pl.v_main || !pl.v_scale || !pl.v_zp)

@@ -66,6 +66,30 @@ def test_host_side_rejections():
         _lib.check(-1, "x")
 
 
+@pytest.mark.parametrize("entry", ["ommx_b200_decode", "ommx_b200_decode_stage2"])
+def test_decode_refuses_residual_k_rows_off_an_8_byte_boundary(entry):
+    """Stage 2 reads K rows in 8-byte words.  Every call here is refused on the host: the aligned ones at the next
+    check (no room for a row in the split workspace), so nothing is ever launched."""
+    def call(base=4096, strides=(8192, 1024, 128), batch=2, rows=4, heads=8):
+        d = _lib.DecodeArgs()
+        d.q = d.o = d.lse = d.attn_logits = d.b_seq_len = d.b_tail_len = 4096
+        d.q_dtype, d.o_dtype, d.batch, d.n_q_heads = _lib.OMMX_DT_BF16, _lib.OMMX_DT_F32, batch, heads
+        p = d.planes
+        p.n_kv_heads, p.head_dim, p.page_size, p.scale_kind = heads, 128, 16, _lib.OMMX_SCALE_INT8_EXP
+        d.num_kv_splits, d.max_seq_len, d.max_tail_len, d.al_stride_s = 1, 0, rows, 0
+        d.k_tail, d.v_tail = base, 4096
+        d.tail_stride_b, d.tail_stride_t, d.tail_stride_h = strides
+        assert getattr(_lib.load(), entry)(C.byref(d), None) == -1
+        return _lib.last_error()
+
+    for ok in (dict(), dict(base=4104), dict(strides=(8193, 1024, 128), batch=1), dict(strides=(8192, 1, 128), rows=1),
+               dict(strides=(8192, 1024, 1), heads=1), dict(strides=(8196, 1028, 132))):
+        assert "attn_logits" in call(**ok), ok
+    for bad in (dict(base=4098), dict(base=4100), dict(strides=(8193, 1024, 128)), dict(strides=(8192, 1026, 128)),
+                dict(strides=(8192, 1024, 130)), dict(base=4098, strides=(8192, 1024, 128), batch=1, rows=1, heads=1)):
+        assert "k_tail" in call(**bad), bad
+
+
 def test_min_splits_rule():
     lib = _lib.load()
     assert lib.ommx_b200_min_num_kv_splits(0, 16) == 1

@@ -281,6 +281,19 @@ def test_decode_refusals():
         case.run(seg_group_base=-1)
 
 
+def test_decode_refuses_a_shifted_residual_k_buffer():
+    """Its rows are read in 8-byte words; the V buffer may lie anywhere (test_decode_residual_row_counts)."""
+    case = Case([200], seed=1)
+    k = torch.empty(case.k_tail.numel() + 4, dtype=torch.bfloat16, device="cuda")
+    good = case.k_tail
+    for shift in (1, 2, 3):
+        case.k_tail = k[shift:shift + good.numel()].view(good.shape).copy_(good)
+        with pytest.raises(ValueError, match="k_tail"):
+            case.run()
+    case.k_tail = k[4:].view(good.shape).copy_(good)
+    _run_and_check(case)
+
+
 def test_store_then_decode_end_to_end():
     """CUDA store kernel feeding the CUDA decode kernels (no oracle-made planes in the loop)."""
     from open_ommx_serve_b200 import ommx_pack_kv_canonical_block
