@@ -7,9 +7,13 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import re
+import sys
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libommx_b200.so")
+HOST_PATH = os.path.join(PKG, "_host.so")
+HOST_MARK = b"ommx-host-built-for: "            # in front of the text that host_target() gave when the module was built
 
 OMMX_DT_F32, OMMX_DT_BF16, OMMX_DT_F16 = 0, 1, 2
 OMMX_SCALE_INT8_EXP, OMMX_SCALE_BF16, OMMX_SCALE_F32 = 0, 1, 2
@@ -119,13 +123,29 @@ _LIB = None
 _HOST = None
 
 
+def host_target() -> str:
+    """What _host.so has to be built for: it links torch's C++ internals, which change from one release to the next."""
+    import torch
+    return f"torch {torch.__version__}, python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
+def host_built_for(path: str = HOST_PATH) -> str:
+    """What the module at ``path`` was built for, read from the file without loading it ('' when it does not say)."""
+    with open(path, "rb") as f:
+        found = re.search(re.escape(HOST_MARK) + rb"([^\0]*)\0", f.read())
+    return found.group(1).decode("utf-8", "replace") if found else ""
+
+
 def host():
-    """The native half of the Python entry points (_host.so), loaded once; ``RuntimeError`` when it is not there."""
+    """The native half of the Python entry points (_host.so), loaded once; ``RuntimeError`` when it is not there or was
+    built for another torch or python (such a module may crash instead of failing to load)."""
     global _HOST
     if _HOST is None:
         load()
+        if os.path.exists(HOST_PATH) and host_built_for(HOST_PATH) != host_target():
+            raise RuntimeError(f"{HOST_PATH} was built for {host_built_for(HOST_PATH) or 'an unknown torch'}; this is {host_target()}: "
+                               "rebuild it with `python -m open_ommx_serve_b200.build`.")
         try:
-            import torch  # noqa: F401  (the module links torch's libraries)
             from . import _host
         except ImportError as e:
             raise RuntimeError(f"{PKG}/_host.so cannot be loaded ({e}): build it with `python -m "

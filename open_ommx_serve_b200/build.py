@@ -14,6 +14,8 @@ import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
+from ._lib import HOST_MARK, HOST_PATH, host_built_for, host_target
+
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libommx_b200.so")
@@ -21,7 +23,7 @@ SOURCES = ("ommx_stage1_h8.cu", "ommx_stage1_h4.cu", "ommx_stage1_h2.cu", "ommx_
            "ommx_capi.cu")
 HEADERS = ("ommx_common.cuh", "ommx_stage1.cuh", "ommx_decode_tc.cuh", "ommx_tables.inc", os.path.join("..", "..", "include", "ommx_b200.h"))
 OBJ = os.path.join(PKG, "build")
-HOST_LIB = os.path.join(PKG, "_host.so")
+HOST_LIB = HOST_PATH
 HOST_SOURCE = os.path.join(CSRC, "ommx_host.cpp")
 NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC")
 
@@ -49,14 +51,16 @@ def _run(cmd) -> str:
 
 
 def build_host(force: bool = False) -> str:
-    """Compile ``_host.so`` against the torch that this interpreter imports; returns its path."""
-    if not force and not _older(HOST_LIB, (HOST_SOURCE, os.path.join(PKG, "..", "include", "ommx_b200.h"))):
-        return HOST_LIB
+    """Compile ``_host.so`` against the torch that this interpreter imports, unless it is newer than its sources and was built
+    for this torch and python; returns its path."""
     import torch
+    target = host_target()
+    if not force and not _older(HOST_LIB, (HOST_SOURCE, os.path.join(PKG, "..", "include", "ommx_b200.h"))) and host_built_for(HOST_LIB) == target:
+        return HOST_LIB
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     _run([os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC",
-          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DOMMX_HOST_BUILT_FOR="{HOST_MARK.decode()}{target}"',
           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
           f"-I{cuda}/include", "-o", HOST_LIB, HOST_SOURCE, f"-L{PKG}", "-l:" + os.path.basename(LIB),
           f"-L{root}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])

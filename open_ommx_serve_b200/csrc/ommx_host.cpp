@@ -26,6 +26,9 @@
 
 #include "../../include/ommx_b200.h"
 
+// the torch and python this module is built for; the loader reads it from the file before it loads the module
+extern "C" __attribute__((used, visibility("default"))) const char ommx_host_built_for[] = OMMX_HOST_BUILT_FOR;
+
 namespace {
 
 using at::Tensor;
