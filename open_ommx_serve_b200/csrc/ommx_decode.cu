@@ -502,7 +502,7 @@ static size_t tensor_core_plan(const ommx_decode_args *a, const S1Params &p, TcP
     T->s.stage_bytes = p.gb_bytes;
     const int per_max = ((a->max_seq_len + a->num_kv_splits - 1) / a->num_kv_splits + 31) / 32;   // groups of the longest split
     const size_t smem = tc_layout(*T, p.gqa <= 4 ? 4 : 8, per_max + 1);
-    return smem <= 232448 ? smem : 0;
+    return smem <= SMEM_LIMIT ? smem : 0;
 }
 
 static int fill_stage1(const ommx_decode_args *a, S1Params &p) {

@@ -873,13 +873,10 @@ static size_t tc_layout(TcParams &P, int gqap, int max_groups_per_split) {
 
 template <int GQAP, bool NB8>
 static int launch_tc(const TcParams &P, dim3 grid, size_t smem, cudaStream_t st) {
-    static std::atomic<size_t> attr_smem[MAX_DEVICES];
+    static std::atomic<int> smem_set[MAX_DEVICES];
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
-    if (smem > attr_smem[dev].load(std::memory_order_acquire)) {
-        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_tc_kernel<GQAP, NB8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_smem[dev].store(smem, std::memory_order_release);
-    }
+    if (int rc = allow_full_smem(decode_stage1_tc_kernel<GQAP, NB8>, smem_set, dev)) return rc;
     static std::atomic<int> regs_state[MAX_DEVICES];   // 0 unknown, 1 enough, 2 too few
     int regs_ok = regs_state[dev].load(std::memory_order_acquire);
     if (regs_ok == 0) {

@@ -1363,11 +1363,21 @@ static int sm_count_of(int dev) {
     return n;
 }
 
+// Lets `kernel` be launched with up to SMEM_LIMIT of dynamic shared memory; `done` holds what has been done on each device.  Always
+// the limit, not what the call needs: of two threads whose first calls need different sizes, the smaller could come last.
+template <typename Kernel> static int allow_full_smem(Kernel kernel, std::atomic<int> (&done)[MAX_DEVICES], int dev) {
+    if (done[dev].load(std::memory_order_acquire) == 0) {
+        OMMX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT));
+        done[dev].store(1, std::memory_order_release);
+    }
+    return 0;
+}
+
 template <int KOUT, int H, bool PLAIN, bool IDX7>
 static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     using L = WarpLayout<H>;
     // function attributes belong to (kernel instantiation, device): one entry per device ordinal
-    static std::atomic<size_t> attr_smem[MAX_DEVICES];
+    static std::atomic<int> smem_set[MAX_DEVICES];
     static std::atomic<int> regs_state[MAX_DEVICES];   // 0 unknown, 1 enough, 2 too few
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
@@ -1382,11 +1392,7 @@ static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
         regs_state[dev].store(regs_ok, std::memory_order_release);
     }
     if (regs_ok != 1) return fail(OMMX_E_CUDA, "stage 1 was compiled with fewer registers than its warp roles need");
-    if (smem > attr_smem[dev].load(std::memory_order_acquire)) {
-        OMMX_CUDA_TRY(cudaFuncSetAttribute(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_smem[dev].store(smem, std::memory_order_release);
-    }
+    if (int rc = allow_full_smem(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>, smem_set, dev)) return rc;
     OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>, dim3(p.ncta), L::THREADS, smem, st, p));
     count_launch();
     return 0;
