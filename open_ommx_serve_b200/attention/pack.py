@@ -133,12 +133,19 @@ def ommx_pack_kv_into(K, V, planes: dict, *, dst_pages=None, dst_groups=None,
     rc = _lib.host().pack_into(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, use_pow2,
                                kv_outlier_map, status)
     if rc is None:
-        _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, kv_outlier_map)
+        _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, kv_outlier_map, status)
     if rc:
         _lib.check(rc, "ommx_b200_pack_kv")
 
 
-def _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, kv_outlier_map):
+def refuse_host_tensors(**tensors) -> None:
+    """``ValueError`` for a tensor that a kernel cannot reach: on the host and not pinned."""
+    for name, t in tensors.items():
+        if isinstance(t, torch.Tensor) and not t.is_cuda and not t.is_pinned():
+            raise ValueError(f"{name} is on {t.device}: it must be a CUDA tensor")
+
+
+def _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, outlier_select, kv_outlier_map, status):
     """The exception for arguments the host module declined: the same conditions, one by one.  Always raises."""
     if not K.is_cuda:
         raise RuntimeError("ommx_pack_kv_into needs CUDA tensors (no CPU path)")
@@ -152,6 +159,7 @@ def _explain_refusal(K, V, planes, dst_pages, dst_groups, outliers_per_vector, o
     for name, t in (("dst_pages", dst_pages), ("dst_groups", dst_groups)):
         if t is not None and (t.dtype != torch.int32 or not t.is_cuda or not t.is_contiguous()):
             raise ValueError(f"{name} must be a contiguous int32 CUDA tensor")
+    refuse_host_tensors(V=V, status=status, **{name: t for name, t in planes.items() if isinstance(t, torch.Tensor)})
     p = planes_struct(planes, k=int(outliers_per_vector), outlier_map=bool(kv_outlier_map))
     if p.n_kv_heads != int(K.shape[1]) or p.head_dim != int(K.shape[2]):
         raise ValueError("K/V geometry does not match the destination planes")

@@ -21,7 +21,7 @@ from typing import Any, Optional
 import torch
 
 from .. import _lib
-from .pack import planes_struct
+from .pack import planes_struct, refuse_host_tensors
 
 _LAUNCHES = {"stage1": 0, "bitmap": 0, "abl": 0}
 _HOST = None                                   # the native half of the launcher, loaded at the first call
@@ -169,7 +169,7 @@ def ommx_paged_decode_attention_canonical(
             k_fp4_mapscale=k_fp4_mapscale, k_fp4_mapcenter=k_fp4_mapcenter, kv_outlier_map=kv_outlier_map,
             num_kv_splits=num_kv_splits, max_seq_len=max_seq_len, max_tail_len=max_tail_len, attn_logits=attn_logits,
             packed_start_offset=packed_start_offset, seg_group_base=seg_group_base, _stage=_stage,
-            static_workspace=static_workspace, head_gather=head_gather)
+            static_workspace=static_workspace, head_gather=head_gather, status=status)
     if ran < 0:
         _lib.check(ran, "ommx_b200_decode_static_ws" if static_workspace else "ommx_b200_decode")
     if ran:
@@ -188,7 +188,7 @@ def _load_host():
 def _explain_refusal(q, k_base, k_scale, k_zp, k_oidx, k_oval, v_main, v_scale, v_zp, k_tail, v_tail, b_tail_len, o, lse,
                      req_to_token, req_to_group, b_seq_len, *, page_size, k_outliers_per_vector, k_format, combinadic_read,
                      bitmap_read, k_obmp, k_fp4_mapscale, k_fp4_mapcenter, kv_outlier_map, num_kv_splits, max_seq_len,
-                     max_tail_len, attn_logits, packed_start_offset, seg_group_base, _stage, static_workspace, head_gather):
+                     max_tail_len, attn_logits, packed_start_offset, seg_group_base, _stage, static_workspace, head_gather, status):
     """The exception for arguments the host module declined: the same conditions, one by one.  Always raises."""
     if not q.is_cuda:
         raise RuntimeError("ommx_paged_decode_attention_canonical needs CUDA tensors (no CPU path)")
@@ -292,12 +292,14 @@ def _explain_refusal(q, k_base, k_scale, k_zp, k_oidx, k_oval, v_main, v_scale, 
     if b_seq_len.dtype != torch.int32 or (b_tail_len is not None and b_tail_len.dtype != torch.int32):
         raise ValueError("b_seq_len / b_tail_len must be int32")
 
-    planes_struct({"k_base": k_base, "k_scale": k_scale, "k_zp": k_zp, "k_obmp": k_obmp if (k > 0 and bitmap_read) else None,
-                   "k_oidx": k_oidx if relidx7_read else None,
-                   "k_oval": k_oval if k > 0 else None,
-                   "k_fp4_mapscale": k_fp4_mapscale if use_map else None,
-                   "k_fp4_mapcenter": k_fp4_mapcenter if use_map else None,
-                   "v_main": v_main, "v_scale": v_scale, "v_zp": v_zp}, k=k, outlier_map=use_map, relidx7=relidx7_read)
+    planes = {"k_base": k_base, "k_scale": k_scale, "k_zp": k_zp, "k_obmp": k_obmp if (k > 0 and bitmap_read) else None,
+              "k_oidx": k_oidx if relidx7_read else None,
+              "k_oval": k_oval if k > 0 else None,
+              "k_fp4_mapscale": k_fp4_mapscale if use_map else None,
+              "k_fp4_mapcenter": k_fp4_mapcenter if use_map else None,
+              "v_main": v_main, "v_scale": v_scale, "v_zp": v_zp}
+    refuse_host_tensors(status=status, **planes)
+    planes_struct(planes, k=k, outlier_map=use_map, relidx7=relidx7_read)
     if max_tail > 0:
         if k_tail is None or v_tail is None or b_tail_len is None:
             raise ValueError("max_tail_len > 0 needs k_tail, v_tail and b_tail_len")
@@ -332,6 +334,7 @@ def merge_attention_states(o_parts, lse_parts, *, valid_lens=None, out=None, lse
                          f"{tuple(lse_parts.shape)} vs {tuple(o_parts.shape[:2])}.")
     if not o_parts.is_cuda:
         raise RuntimeError("merge_attention_states needs CUDA tensors (no CPU path)")
+    refuse_host_tensors(lse_parts=lse_parts)
     P, R, D = (int(s) for s in o_parts.shape)
     op = o_parts.contiguous().to(torch.float32)
     lp = lse_parts.contiguous().to(torch.float32)

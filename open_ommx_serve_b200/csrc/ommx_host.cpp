@@ -101,12 +101,14 @@ struct PlaneSet {
 };
 void *ptr(const Tensor *t) { return t ? t->data_ptr() : nullptr; }
 void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
+// memory a kernel may touch: a plain host tensor is declined, not handed to the GPU
+bool reachable(const Tensor *t) { return !t || t->is_cuda() || t->is_pinned(); }
 
 bool fill_planes(const PlaneSet &s, int64_t k, bool use_map, bool relidx7, ommx_kv_planes *p) {
     for (const Tensor *t : {s.k_base, s.k_scale, s.k_zp, s.v_main, s.v_scale, s.v_zp})
-        if (!t || !t->is_contiguous()) return false;
+        if (!t || !t->is_contiguous() || !reachable(t)) return false;
     for (const Tensor *t : {s.k_idx, s.k_oval, s.k_ms, s.k_mc})
-        if (t && !t->is_contiguous()) return false;
+        if (t && (!t->is_contiguous() || !reachable(t))) return false;
     if (s.k_base->dim() != 4 || s.k_scale->dim() < 1) return false;
     const auto kind = s.k_scale->scalar_type();
     if (kind == at::kChar) p->scale_kind = OMMX_SCALE_INT8_EXP;
@@ -296,7 +298,7 @@ PyObject *py_decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
     d.sm_scale = (float)sm_scale; d.logit_cap = (float)logit_cap;
     if (a[STATUS] != Py_None) {
         const Tensor *st = as_tensor(a[STATUS]);
-        NEED(st);
+        NEED(st && reachable(st));
         d.status = (int32_t *)st->data_ptr();
     }
     // differential-timing knobs: the caller records them, so a leaked export cannot pass as served
@@ -341,7 +343,7 @@ bool index_table(PyObject *o, const int32_t **out) {
 bool pack_planes(const Tensor &K0, const Tensor &V0, const PlaneSet &s, const int32_t *pages, const int32_t *groups, int64_t k,
                  bool is_signed, bool use_pow2, bool use_map, int32_t *status, int *rc) {
     Tensor K = K0, V = V0;
-    if (K.dim() != 3 || K.sizes() != V.sizes() || K.scalar_type() != V.scalar_type() || !K.is_cuda()) return false;
+    if (K.dim() != 3 || K.sizes() != V.sizes() || K.scalar_type() != V.scalar_type() || !K.is_cuda() || !reachable(&V)) return false;
     if (K.stride(2) != 1 || V.stride(2) != 1 || K.strides() != V.strides()) { K = K.contiguous(); V = V.contiguous(); }
     ommx_pack_args a;
     memset(&a, 0, sizeof(a));
@@ -368,7 +370,7 @@ PyObject *py_pack_into(PyObject *, PyObject *const *a, Py_ssize_t n) {
     int64_t k;
     bool use_pow2, use_map;
     NEED(K && V && read_plane_dict(a[2], &s) && index_table(a[3], &pages) && index_table(a[4], &groups) && as_long(a[5], &k));
-    NEED(PyUnicode_Check(a[6]) && as_bool(a[7], &use_pow2) && as_bool(a[8], &use_map) && (st || a[9] == Py_None));
+    NEED(PyUnicode_Check(a[6]) && as_bool(a[7], &use_pow2) && as_bool(a[8], &use_map) && (st || a[9] == Py_None) && reachable(st));
     const char *sel = PyUnicode_AsUTF8(a[6]);
     if (!sel) return nullptr;
     const bool is_signed = strcasecmp(sel, "signed") == 0;
@@ -571,6 +573,8 @@ PyObject *py_kv_gather_tail(PyObject *, PyObject *const *a, Py_ssize_t n) {
     const Tensor *sel = as_tensor(a[1]), *idx = as_tensor(a[2]), *kt = as_tensor(a[3]), *vt = as_tensor(a[4]);
     bool tables;
     if (!idx || !kt || !vt || !as_bool(a[5], &tables)) { PyErr_SetString(PyExc_TypeError, "kv_gather_tail: tensors expected"); return nullptr; }
+    for (const Tensor *t : {sel, idx, kt, vt})
+        if (!reachable(t)) { PyErr_SetString(PyExc_ValueError, "kv_gather_tail: sel, tail indices and residual buffers must be CUDA tensors"); return nullptr; }
     const Tensor sel_c = sel ? sel->contiguous() : Tensor(), idx_c = idx->contiguous();
     int32_t *status = (int32_t *)ptr(r.tensor(N.status));
     if (!r.ok) return nullptr;
