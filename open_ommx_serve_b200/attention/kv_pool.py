@@ -355,6 +355,8 @@ class MultiSeqKVPool:
         B, T = int(tidx.shape[0]), int(tidx.shape[1])
         if tidx.dtype not in (torch.int32, torch.int64) or (sel is not None and sel.dtype != tidx.dtype):
             raise ValueError("sel / tail index tensors must both be int32 or both int64")
+        if sel is not None and int(sel.numel()) < B:
+            raise ValueError(f"sel names {int(sel.numel())} slots for {B} rows of tail indices")
         if tuple(kt.shape) != (B, T, self.H, self.D) or not kt.is_contiguous() or not vt.is_contiguous() or tuple(vt.shape) != tuple(kt.shape):
             raise ValueError(f"k_tail / v_tail must be contiguous [{B}, {T}, {self.H}, {self.D}]")
         got = _lib.host().kv_gather_tail(self, sel, tidx, kt, vt, with_tables)

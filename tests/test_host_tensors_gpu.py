@@ -1,4 +1,5 @@
-"""A tensor in plain host memory where a kernel would read or write it is refused before anything is launched."""
+"""Tensors that a kernel would read or write outside what is there - in plain host memory, or too few - are refused before
+anything is launched."""
 import pytest
 import torch
 
@@ -51,6 +52,19 @@ def test_gather_refuses_indices_and_buffers_on_the_host(which):
     args = [t if i == which else t.cuda() for i, t in enumerate(args)]
     with pytest.raises(ValueError, match="CUDA"):
         pool._gather_tail(*args)
+
+
+def test_gather_refuses_a_selection_that_is_too_short():
+    """One entry of ``sel`` is read for every row of tail indices."""
+    from open_ommx_serve_b200.attention.kv_pool import MultiSeqKVPool
+    pool = MultiSeqKVPool(128, 2, 4, 256)
+    buf = torch.zeros(2, 8, 2, 128, dtype=torch.bfloat16, device="cuda")
+    lens = torch.zeros(2, dtype=torch.int32, device="cuda")
+    tidx = torch.zeros(2, 8, dtype=torch.int64, device="cuda")
+    with pytest.raises(ValueError, match="1 slots for 2 rows"):
+        pool.decode_inputs_captured(torch.arange(1, device="cuda"), lens, lens, tidx, buf, buf.clone(), 0)
+    for n in (2, 3):                                       # a longer one's first entries count
+        pool.decode_inputs_captured(torch.arange(n, device="cuda"), lens, lens, tidx, buf, buf.clone(), 0)
 
 
 def test_merge_refuses_lse_on_the_host():
