@@ -259,11 +259,52 @@ __device__ __forceinline__ uint32_t drop_ties(uint32_t picks, uint32_t eq, int k
     return picks;
 }
 
-// a >= b afterwards
-__device__ __forceinline__ void order2(float &a, float &b) {
-    const float hi = fmaxf(a, b);
-    b = fminf(a, b);
+// The M largest (descending) and M smallest (ascending) of 32 values x(0) .. x(31), by a sorting network for M <= 4: blocks of four are
+// sorted, then merged (248 min / max at M = 4).  V is float, or a pair of 16-bit values, whose halves are two channels and on whose
+// min and max a NaN wins.  lowest / highest: what every value displaces.
+__device__ __forceinline__ float v_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ float v_min(float a, float b) { return fminf(a, b); }
+template <typename V> __device__ __forceinline__ V v_max(V a, V b) { return __hmax2_nan(a, b); }
+template <typename V> __device__ __forceinline__ V v_min(V a, V b) { return __hmin2_nan(a, b); }
+template <typename V> __device__ __forceinline__ void order2(V &a, V &b) {       // a >= b afterwards
+    const V hi = v_max(a, b);
+    b = v_min(a, b);
     a = hi;
+}
+template <int M, int N, typename V, typename Fn>
+__device__ __forceinline__ void extremes_of_32(Fn x, V (&top)[N], V (&bot)[N], V lowest, V highest) {
+    static_assert(N >= 4 && N >= M, "a block of four is sorted in place");
+    if constexpr (M == 1) {
+        top[0] = bot[0] = x(0);
+#pragma unroll
+        for (int t = 1; t < 32; ++t) { top[0] = v_max(top[0], x(t)); bot[0] = v_min(bot[0], x(t)); }
+    } else if constexpr (M <= 4) {
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            V s0 = x(4 * b), s1 = x(4 * b + 1), s2 = x(4 * b + 2), s3 = x(4 * b + 3);
+            order2(s0, s1); order2(s2, s3); order2(s0, s2); order2(s1, s3); order2(s1, s2);
+            if (b == 0) {
+                top[0] = s0; top[1] = s1; top[2] = s2; top[3] = s3;
+                bot[0] = s3; bot[1] = s2; bot[2] = s1; bot[3] = s0;
+            } else {
+                // the larger (smaller) halves of two sorted fours are bitonic: two rounds sort them
+                top[0] = v_max(top[0], s3); top[1] = v_max(top[1], s2); top[2] = v_max(top[2], s1); top[3] = v_max(top[3], s0);
+                order2(top[0], top[2]); order2(top[1], top[3]); order2(top[0], top[1]); order2(top[2], top[3]);
+                bot[0] = v_min(bot[0], s0); bot[1] = v_min(bot[1], s1); bot[2] = v_min(bot[2], s2); bot[3] = v_min(bot[3], s3);
+                order2(bot[2], bot[0]); order2(bot[3], bot[1]); order2(bot[1], bot[0]); order2(bot[3], bot[2]);
+            }
+        }
+    } else {
+        // five of each: insertion
+#pragma unroll
+        for (int i = 0; i < M; ++i) { top[i] = lowest; bot[i] = highest; }
+#pragma unroll
+        for (int t = 0; t < 32; ++t) {
+            V c = x(t), d = c;
+#pragma unroll
+            for (int i = 0; i < M; ++i) { order2(top[i], c); order2(d, bot[i]); }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -367,43 +408,12 @@ __global__ void __launch_bounds__(PACK_WARPS * 32) pack_k_lane_kernel(PackKParam
         bad = top[0] >= 0xFF800000u || bot[0] < 0x00800000u;
         rounds = __any_sync(0xFFFFFFFFu, __popc(omask) != K || bad);
     } else {
-        // The M largest and M smallest of the 32 values by a sorting network (248 min / max at M = 4; the rounds below took some 900
-        // instructions), the picks by two comparisons a token, ties by the stable-sort rule, as pack_k_pair does for 16-bit values.
-        // 8192 tokens x 8 heads, K + V: 61.5 -> 53.6 us.
+        // The extremes by the sorting network (the rounds below took some 900 instructions), the picks by two comparisons a token, ties
+        // by the stable-sort rule, as pack_k_pair does for 16-bit values.  8192 tokens x 8 heads, K + V: 61.5 -> 53.6 us.
         rounds = false;
         constexpr int M = KT >= KB ? KT + 1 : KB + 1;
         float top[M <= 4 ? 4 : M], bot[M <= 4 ? 4 : M], zero = 0.f;
-        if constexpr (M == 1) {
-            top[0] = bot[0] = x[0];
-#pragma unroll
-            for (int t = 1; t < 32; ++t) { top[0] = fmaxf(top[0], x[t]); bot[0] = fminf(bot[0], x[t]); }
-        } else if constexpr (M <= 4) {
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                float s0 = x[4 * b], s1 = x[4 * b + 1], s2 = x[4 * b + 2], s3 = x[4 * b + 3];
-                order2(s0, s1); order2(s2, s3); order2(s0, s2); order2(s1, s3); order2(s1, s2);
-                if (b == 0) {
-                    top[0] = s0; top[1] = s1; top[2] = s2; top[3] = s3;
-                    bot[0] = s3; bot[1] = s2; bot[2] = s1; bot[3] = s0;
-                } else {
-                    // the larger (smaller) halves of two sorted fours are bitonic: two rounds sort them
-                    top[0] = fmaxf(top[0], s3); top[1] = fmaxf(top[1], s2); top[2] = fmaxf(top[2], s1); top[3] = fmaxf(top[3], s0);
-                    order2(top[0], top[2]); order2(top[1], top[3]); order2(top[0], top[1]); order2(top[2], top[3]);
-                    bot[0] = fminf(bot[0], s0); bot[1] = fminf(bot[1], s1); bot[2] = fminf(bot[2], s2); bot[3] = fminf(bot[3], s3);
-                    order2(bot[2], bot[0]); order2(bot[3], bot[1]); order2(bot[1], bot[0]); order2(bot[3], bot[2]);
-                }
-            }
-        } else {
-            // five of each: insertion, from infinities that every value pushes out
-#pragma unroll
-            for (int i = 0; i < M; ++i) { top[i] = -INFINITY; bot[i] = INFINITY; }
-#pragma unroll
-            for (int t = 0; t < 32; ++t) {
-                float c = x[t], d = c;
-#pragma unroll
-                for (int i = 0; i < M; ++i) { order2(top[i], c); order2(d, bot[i]); }
-            }
-        }
+        extremes_of_32<M>([&](int t) { return x[t]; }, top, bot, -INFINITY, INFINITY);
 #pragma unroll
         for (int t = 0; t < 32; ++t) zero = fmaf(x[t], 0.f, zero);       // NaN once a value is not finite
         bad = zero != 0.f;
@@ -767,12 +777,6 @@ template <> struct Pair16<__half> {
 };
 template <typename V> __device__ __forceinline__ V as_pair(uint32_t w) { return *reinterpret_cast<const V *>(&w); }
 template <typename V> __device__ __forceinline__ uint32_t pair_bits(V v) { return *reinterpret_cast<const uint32_t *>(&v); }
-// a >= b afterwards, NaN goes everywhere
-template <typename V> __device__ __forceinline__ void order2(V &a, V &b) {
-    const V hi = __hmax2_nan(a, b);
-    b = __hmin2_nan(a, b);
-    a = hi;
-}
 // one 16-bit value of half c of a pair of words
 __device__ __forceinline__ bool half_is_special(uint32_t w, uint32_t exp) {
     return (w & exp) == exp || ((w >> 16) & exp) == exp;
@@ -809,37 +813,7 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
     // ---- the M largest, descending, and the M smallest, ascending ----
     constexpr int M = KT >= KB ? KT + 1 : KB + 1;
     V top[M <= 4 ? 4 : M], bot[M <= 4 ? 4 : M];
-    if constexpr (M == 1) {
-        top[0] = bot[0] = as_pair<V>(w[0]);
-#pragma unroll
-        for (int t = 1; t < 32; ++t) { top[0] = __hmax2_nan(top[0], as_pair<V>(w[t])); bot[0] = __hmin2_nan(bot[0], as_pair<V>(w[t])); }
-    } else if constexpr (M <= 4) {
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            V s0 = as_pair<V>(w[4 * b]), s1 = as_pair<V>(w[4 * b + 1]), s2 = as_pair<V>(w[4 * b + 2]), s3 = as_pair<V>(w[4 * b + 3]);
-            order2(s0, s1); order2(s2, s3); order2(s0, s2); order2(s1, s3); order2(s1, s2);
-            if (b == 0) {
-                top[0] = s0; top[1] = s1; top[2] = s2; top[3] = s3;
-                bot[0] = s3; bot[1] = s2; bot[2] = s1; bot[3] = s0;
-            } else {
-                // the larger (smaller) halves of two sorted fours are bitonic: two rounds sort them
-                top[0] = __hmax2_nan(top[0], s3); top[1] = __hmax2_nan(top[1], s2); top[2] = __hmax2_nan(top[2], s1); top[3] = __hmax2_nan(top[3], s0);
-                order2(top[0], top[2]); order2(top[1], top[3]); order2(top[0], top[1]); order2(top[2], top[3]);
-                bot[0] = __hmin2_nan(bot[0], s0); bot[1] = __hmin2_nan(bot[1], s1); bot[2] = __hmin2_nan(bot[2], s2); bot[3] = __hmin2_nan(bot[3], s3);
-                order2(bot[2], bot[0]); order2(bot[3], bot[1]); order2(bot[1], bot[0]); order2(bot[3], bot[2]);
-            }
-        }
-    } else {
-        // five of each: insertion, from infinities that every value pushes out
-#pragma unroll
-        for (int i = 0; i < M; ++i) { top[i] = as_pair<V>(P::EXP | (P::EXP << 16) | 0x80008000u); bot[i] = as_pair<V>(P::EXP | (P::EXP << 16)); }
-#pragma unroll
-        for (int t = 0; t < 32; ++t) {
-            V c = as_pair<V>(w[t]), d = c;
-#pragma unroll
-            for (int i = 0; i < M; ++i) { order2(top[i], c); order2(d, bot[i]); }
-        }
-    }
+    extremes_of_32<M>([&](int t) { return as_pair<V>(w[t]); }, top, bot, as_pair<V>(P::EXP | (P::EXP << 16) | 0x80008000u), as_pair<V>(P::EXP | (P::EXP << 16)));
     bool bad = half_is_special(pair_bits(top[0]), P::EXP) || half_is_special(pair_bits(bot[0]), P::EXP);
 
     // ---- which tokens are picked ----
