@@ -527,7 +527,6 @@ static int fill_stage1(const ommx_decode_args *a, S1Params &p) {
     p.sm_scale = a->sm_scale; p.logit_cap = a->logit_cap; p.status = a->status;
     const int H = p.H;
     p.GS = NCW / H;
-    p.hshift = H == 8 ? 3 : (H == 4 ? 2 : (H == 2 ? 1 : 0));
     p.o_vm = H * 1024; p.o_vs = H * 2048; p.o_vz = p.o_vs + H * 128; p.o_ks = p.o_vz + H * 256;
     p.o_kz = p.o_ks + H * 128; p.o_ms = p.o_kz + H * 256; p.o_mc = p.o_ms + H * 256; p.o_bm = p.o_mc + H * 256;
     p.o_ov = (p.o_bm + H * 128 * p.nbi + 15) / 16 * 16;

@@ -63,7 +63,7 @@ struct S1Params {
     int32_t *status;
     int32_t abl;
     // shared-memory layout of one group block (bytes)
-    int32_t GS, gb_bytes, stage_bytes, nstages, hshift;
+    int32_t GS, gb_bytes, stage_bytes, nstages;
     int32_t o_vm, o_vs, o_vz, o_ks, o_kz, o_ms, o_mc, o_bm, o_ov;
     // tensor maps of the two code planes as [bytes/128][128] uint8 with 128-byte swizzle
     uint32_t swz;                        // 0x70 when the maps are in use, else 0
