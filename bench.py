@@ -795,7 +795,7 @@ def workload_prefill_pack(args, device, flush, peak, tokens=8192):
     return {"config": {"workload": f"bulk quantize + pack of {tokens} tokens x {HKV} kv heads (bf16 K and V in, packed planes out, "
                                    f"{PAGE}-token pages through a random page table); {n_sets} chunks per step, L2 flushed between steps"},
             "us_per_chunk": us, "hbm_gbs": ach,
-            "roofline": {"bound": "hbm", "kernel": "pack_k_lane_kernel + pack_v_kernel", "achieved": ach, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "pack16_kernel", "achieved": ach, "peak": peak,
                          "unit": "GB/s", "frac": ach / peak, "algorithmic_bytes_per_chunk": nbytes}}
 
 

@@ -34,7 +34,7 @@ extern "C" {
 #define OMMX_ST_BAD_GROUP    2     /* group slot outside [0, num_group_slots) - access skipped */
 #define OMMX_ST_NONFINITE    4     /* packer saw NaN/Inf in K or V */
 #define OMMX_ST_TIMEOUT      8     /* a bounded wait inside a kernel ran out */
-#define OMMX_ST_BAD_LENGTH  16     /* b_seq_len needs more groups per split than a CTA can index */
+#define OMMX_ST_BAD_LENGTH  16     /* a length past what its tables, its residual buffer or a CTA's split can hold */
 #define OMMX_ST_SCALE_RANGE 32     /* a K or V scale exponent above 11 was clamped in decode (scale step > 2048) */
 
 /* element types of q / o / k,v inputs */
@@ -125,8 +125,9 @@ int ommx_b200_outlier_index_convert(const void *src, void *dst, int64_t frames, 
  * (:1255), stage 2 = _canonical_lse_merge with the bf16 sink/recent rows fused in (:2366).
  * Writes o / lse in place.  attn_logits is the caller's split workspace
  * f32 [batch, n_q_heads, num_kv_splits+1, head_dim+1] (lane head_dim = log-sum-exp).
- * b_seq_len holds PACKED token counts; split s covers tokens [s*per, min((s+1)*per, seq)) with
- * per = ceil(ceil(seq/num_kv_splits)/32)*32, exactly as the reference.
+ * b_seq_len holds PACKED token counts.  num_kv_splits is the number of workspace slots of a sequence: its 32-token groups are
+ * worked on in at most that many pieces.  Where they are cut follows from all lengths of the batch, on the device, so that the
+ * CTAs have even shares (ommx_b200_host_share_plan); the reference cuts every sequence into num_kv_splits equal ones.
  */
 /*
  * Head-output exchange fused into stage 2, for kv heads sharded over the GPUs of one node (the split vLLM
@@ -172,7 +173,7 @@ typedef struct ommx_decode_args {
     float *attn_logits;
     int64_t al_stride_b, al_stride_h, al_stride_s;
     int32_t num_kv_splits;
-    int32_t max_seq_len;          /* upper bound of b_seq_len (sizes nothing on device; checked) */
+    int32_t max_seq_len;          /* upper bound of b_seq_len: sizes the grid, checked against num_kv_splits */
     int32_t max_tail_len;
     int32_t seg_group_base;       /* first group of the attended segment (0 = whole sequence) */
     int32_t packed_start_offset;  /* must be 0 */
@@ -287,11 +288,6 @@ int ommx_b200_kv_gather_inputs(const ommx_kv_pool *pool, const void *sel, const 
                                int32_t *r2t_out, int32_t *r2g_out, int32_t *status, void *stream);
 
 /*
- * Split count this library prefers for (max context, batch, local kv heads) on the current
- * device.  Replaces _auto_num_kv_splits (attention/paged_decode.py:409-461), which callers
- * use to size attn_logits once.
- */
-/*
  * Device memory that other processes of the node can map (CUDA IPC), for ommx_head_gather.  `alloc` returns a
  * zero-filled allocation and its 64-byte handle; `open` maps another process's allocation into this one (peer
  * access over NVLink) and `close` unmaps it; `free` releases an own allocation.  Call them outside stream capture.
@@ -301,6 +297,11 @@ int ommx_b200_peer_open(const void *handle64, void **ptr);
 int ommx_b200_peer_close(void *ptr);
 int ommx_b200_peer_free(void *ptr);
 
+/*
+ * Split count this library prefers for (max context, batch, local kv heads) on the current
+ * device.  Replaces _auto_num_kv_splits (attention/paged_decode.py:409-461), which callers
+ * use to size attn_logits once.
+ */
 int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, int32_t n_kv_heads);
 /* Smallest split count ommx_b200_decode accepts for a context of max_seq_len packed tokens. */
 int ommx_b200_min_num_kv_splits(int32_t max_seq_len, int32_t page_size);

@@ -21,7 +21,7 @@ OMMX_OIDX_BITMASK, OMMX_OIDX_RELIDX7 = 0, 1
 ST_BAD_PAGE, ST_BAD_GROUP, ST_NONFINITE, ST_TIMEOUT, ST_BAD_LENGTH, ST_SCALE_RANGE = 1, 2, 4, 8, 16, 32
 STATUS_NAMES = {ST_BAD_PAGE: "page id out of range", ST_BAD_GROUP: "group slot out of range",
                 ST_NONFINITE: "non-finite K/V value", ST_TIMEOUT: "a bounded device wait ran out",
-                ST_BAD_LENGTH: "a split holds more groups than one CTA can index",
+                ST_BAD_LENGTH: "a length past what its tables, its residual buffer or a CTA's split can hold",
                 ST_SCALE_RANGE: "a scale exponent above 11 was clamped"}
 
 

@@ -83,10 +83,11 @@ def _env_int(name: str, default: int, *, allow_zero: bool = False) -> int:
 
 
 def _auto_num_kv_splits(seq_len: int, batch_size: int, device: Any = None, kv_heads: int = 8) -> int:
-    """Split count for (max context, batch): sized so that batch x splits fills the 148 SMs.
+    """Split count for (max context, batch): sized so that equal splits of sequences of that length fill the SMs.
 
-    One CTA serves one (split, sequence) with all local kv heads, so ``kv_heads`` does not
-    enter.  ``OMMX_ATTN_NUM_KV_SPLITS`` overrides, as in the reference.
+    It sizes the split workspace; how the groups are dealt to CTAs is decided on the device, more evenly with more slots where the
+    lengths differ.  A CTA works for all local kv heads, so ``kv_heads`` does not enter.  ``OMMX_ATTN_NUM_KV_SPLITS`` overrides,
+    as in the reference.
     """
     if str(os.environ.get("OMMX_ATTN_NUM_KV_SPLITS") or "").strip():
         return _env_int("OMMX_ATTN_NUM_KV_SPLITS", 1)

@@ -2,8 +2,8 @@
 // (log-sum-exp combine with the bf16 sink/recent rows fused in) and the partial-state merge.
 //
 // Stage 1 (ommx_stage1.cuh) replaces _canonical_splitkv_stage1 (ommx_gpu_serve/attention/paged_decode.py:1255-2284
-// of the reference).  The groups of all sequences form one running list of which every CTA takes an
-// equal share, for ALL local kv heads, so every page row it touches is a full contiguous line:
+// of the reference).  The groups of all sequences form one running list of which every CTA takes a
+// contiguous share, for ALL local kv heads, so every page row it touches is a full contiguous line:
 //
 //   producer warp   streams whole pages / group-slot planes into a shared-memory ring: the two
 //                   code planes through swizzled tensor maps, the small planes with 1-D bulk
@@ -486,7 +486,7 @@ static int stage1_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
 namespace ommx {
 
 // Which stage-1 kernel serves a call.  The register-operand kernel (decode_stage1_kernel) is the default: on B200 it
-// is the faster of the two (53 us against 142 us per 64K-context layer).  OMMX_B200_STAGE1=tc selects the tensor-core
+// is the faster of the two (40 us against 98 us for 64K tokens x 8 heads).  OMMX_B200_STAGE1=tc selects the tensor-core
 // kernel (decode_stage1_tc_kernel) where its shared-memory plan fits - 4 or 8 local kv heads with GQA <= 4, fewer
 // heads at any GQA <= 8 - and no differential-timing knob is set; it produces the same results within the path's
 // tolerance and is kept for further work on its pipeline.  The variable is read once per call (`tc` below).
@@ -668,10 +668,10 @@ extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, 
     int dev = 0, sm_count = 148;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < ommx::MAX_DEVICES) sm_count = ommx::sm_count_of(dev);
     else (void)cudaGetLastError();
-    // One CTA runs per SM, so a launch takes (waves of CTAs) x (groups per CTA + what a CTA costs before and after its
-    // steady state, about three groups' worth).  Pick the split count that minimises it: 148 at batch 1, and e.g. 18
-    // rather than 19 at batch 8, where 152 CTAs would leave a second wave of four.  Ties go to fewer splits (less for
-    // stage 2 to combine).
+    // For sequences of one length in equal splits: one CTA runs per SM, so a launch takes (waves of CTAs) x (groups per CTA +
+    // what a CTA costs before and after its steady state, about three groups' worth).  Pick the split count that minimises it:
+    // 147 or 148 at batch 1, and e.g. 18 rather than 19 at batch 8, where 152 CTAs would leave a second wave of four.  Ties go to
+    // fewer splits (less for stage 2 to combine).  A ragged batch is shared out more evenly with more slots (share_plan_of).
     const int groups = max(1, (max_seq_len + 31) / 32);
     const int b = max(1, batch);
     const int s_min = ommx_b200_min_num_kv_splits(max_seq_len, 16);

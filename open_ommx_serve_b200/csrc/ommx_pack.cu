@@ -758,8 +758,10 @@ __global__ void __launch_bounds__(128) pack_v_kernel(PackVParams p) {
 // KT-th (KB-th) value, and where equal values leave too many, the highest tokens go - the stable-sort rule.  The values behind the
 // picks are the base range.  Codes are two FMAs and one shifted add per value: (x - zp) / 4s saturated to [0, 1] in one FMA (one
 // rounding, the same as the subtraction's, because s is a power of two), times 4 onto 1.5 * 2^23, which rounds to nearest even.
-// Bound by the ALU pipe (min / max, compare and logic run at half the FMA rate).  Measured, K + V: 8192 tokens x 8 heads (42 MB)
-// 34.8 -> 17.2 us, 2.5 TB/s; 32768 tokens 122 -> 61 us; 1024 tokens 9.3 -> 5.5 us.
+// Bound by no single pipe: while the SMs are busy the ALU pipe (min / max, compare and logic run at half the FMA rate) is 60 % and the
+// issue slots are 63 % taken, DRAM 21 %; the rest is waiting for instructions to be fetched (straight-line code), for first loads
+// and for fixed-latency results, and the last of three waves leaves SMs idle for a fifth of the launch.  Measured, K + V: 8192 tokens x
+// 8 heads (42 MB) 38.9 -> 18.9 us, 2.2 TB/s; 32768 tokens 122 -> 61 us; 1024 tokens 9.3 -> 5.5 us.
 // The scale, map and FP4 steps are those of pack_k_kernel, operation for operation.
 // ---------------------------------------------------------------------------------------------
 template <typename T> struct Pair16;
@@ -1303,8 +1305,10 @@ __global__ void __launch_bounds__(256) kv_gather_tail_kernel(GatherParams p) {
 //     the new one overwrites in the ring left the group's 32 rows long ago (the ring holds recent + 32 at least);
 //   * the residual rows that are handed to the decode call come from the ring, except the new one, which comes from its source;
 //   * the length is advanced once every CTA of the row's cluster has read it (a cluster barrier).
-// Bound by latency: one chain slot -> length -> rows.  Measured: 17 -> 4 us at batch 1, 8 heads.  Needs recent >= 1, whole 64-channel units and 16-byte pieces;
-// launch_append keeps the separate kernels for anything else.
+// Bound by latency, one chain slot -> length -> rows: at batch 32 the issue slots are 26 % and DRAM 10 % busy, and waiting for loads is
+// the largest stall.  A step in which a quarter of the rows complete a group takes twice one in which none does (18.3 and 9.1 us, cold).
+// Measured: 17 -> 4 us at batch 1, 8 heads.  Needs recent >= 1, whole 64-channel units and 16-byte pieces; launch_append keeps the
+// separate kernels for anything else.
 // ---------------------------------------------------------------------------------------------
 constexpr int STORE_CTAS = 8, STORE_THREADS = 256;
 template <int KT, int KB>

@@ -289,11 +289,17 @@ __host__ __device__ constexpr PositionBits past_31_bits(int k, int bytes) {
 // sequences they belong to (32 sequences of 1K..32K tokens in splits of 512 were 2048 CTAs in waves of 148, each with 7 to 9 us
 // around its steady state: 560 us of store and decode against 318 us).  A piece of a sequence writes its partial result to
 // workspace slot (its CTA - the first CTA of the sequence), and the caller's workspace has S slots per sequence, which bounds `per`
-// from below: shares are even up to one group where S is generous, and longer, up to the longest sequence over S - 1, where it is not.
+// from below: shares are even up to one group where S is generous, and longer, up to the longest sequence over S - 1, where it is not
+// (8 sequences of 4K..32K tokens, both stages: 86 us with 64 slots, 145 us with the 18 of ommx_b200_auto_num_kv_splits).
 // Equal splits per sequence, dealt out one by one (per = 0: item x is split x % S of sequence x / S), are taken instead
 //   * where that bound makes the shares longer than S of them per sequence would be, and
 //   * where a share could hold more sequences than a CTA lists (MAX_PIECES).  Of equal splits a CTA never has more than that:
-//     stage1_grid makes a CTA for every MAX_PIECES of them as soon as there are that many sequences.
+//     stage1_grid makes a CTA for every MAX_PIECES of them as soon as there are that many sequences.  The line is drawn where any
+//     lengths are safe; where none are short the list would have been, and is faster or slower (2 kv heads, S = 2: 187 sequences of
+//     68..136 groups 115 us by the list, 173 by splits; 204 of 119..238 groups 341 and 226).  A line drawn from the shortest sequence
+//     costs every batch: one more reduction ahead of the stages made the long cases 3 to 4 % slower.
+// Where pieces begin depends on the plan, and with it the running maximum against which P is rounded to fp16: another split
+// count or batch moves a result by about 5e-5 of its norm, the same call repeats its bits.
 struct SharePlan {
     int per, total;                      // groups per CTA (0: equal splits per sequence), groups of all sequences
 };
