@@ -121,11 +121,12 @@ def test_decode_groups_shared_over_the_ctas(lens, H, splits):
     _run_and_check(Case(lens, H=H, Hq=4 * H, seed=17), num_kv_splits=splits)
 
 
-@pytest.mark.parametrize("H,at,splits", [(2, 0, None), (2, 199, None), (8, 100, 3)])
-def test_decode_many_short_sequences_beside_a_longer_one(H, at, splits):
-    """More sequences in an even share than a CTA can list: 199 of one group and one of 200."""
-    lens = [72] * 200
-    lens[at] = 40 + 200 * 32
+@pytest.mark.parametrize("H,n,long,at,splits", [(2, 200, 200, 0, None), (2, 200, 200, 199, None), (8, 200, 200, 100, 3),
+                                                (2, 300, 129, 299, 2)])        # the last: a CTA lists as many as it can
+def test_decode_many_short_sequences_beside_a_longer_one(H, n, long, at, splits):
+    """More sequences in an even share than a CTA can list: all of one group but one."""
+    lens = [72] * n
+    lens[at] = 40 + long * 32
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     _run_and_check(Case(lens, H=H, Hq=4 * H, seed=23), num_kv_splits=splits, status=status)
     assert int(status.item()) == 0

@@ -60,7 +60,7 @@ def check(groups, splits, bound=1):
         before += n
 
 
-@pytest.mark.parametrize("long", [130, 200, 254, 300])
+@pytest.mark.parametrize("long", [129, 130, 200, 254, 300])
 @pytest.mark.parametrize("n", [200, 220, 300, 1000])
 @pytest.mark.parametrize("at", [0, 100, -1])
 def test_many_short_sequences_beside_a_longer_one(n, long, at):
@@ -70,6 +70,13 @@ def test_many_short_sequences_beside_a_longer_one(n, long, at):
     for splits in (2, 3, 5):
         check(groups, splits)
         check(groups, splits, 16)
+
+
+def test_a_share_of_as_many_sequences_as_a_cta_lists_is_kept():
+    groups = [1] * 299 + [129]
+    limit, ctas, per = plan(groups, 2, 1)
+    pieces = pieces_of(groups, 2, ctas, per)
+    assert per == limit and sum(1 for p in pieces if p[0] == 0) == limit
 
 
 @pytest.mark.parametrize("seed", range(300))
