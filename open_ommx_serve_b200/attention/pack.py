@@ -189,7 +189,8 @@ def ommx_pack_kv_canonical_block(
     tensors are copied to ``device`` (default: the current CUDA device) first.  The returned
     dict has the reference's keys (``attention/pack.py:628-655``).  Served here: the flat
     bitmask and the relidx7 outlier index (``outlier_repr='bitmap'`` / ``'relidx7'``, k <= 16),
-    32-token / 32-channel groups, INT2 V.
+    32-token / 32-channel groups, INT2 V.  With int8 scales (``use_pow2`` and ``kv_int8_scale``) zero-points and
+    map planes are bfloat16 whatever ``scale_dtype`` says.
     Anything else raises ``NotImplementedError`` - there is no slower fallback.
     ``check_finite`` reads one status word back (a host sync, as the reference's own finite
     check is) and raises ``ValueError`` on NaN/Inf input.
