@@ -10,12 +10,13 @@
 //                   copies, completion through mbarrier transaction counts; page ids and group
 //                   slots are read one ring stage ahead.
 //   15 decode warps build, two per (group, kv head) unit, the unit's sidecar tile: outlier
-//                   deltas (bit walk with clz, FP4 nibble, base code byte) as fp16
+//                   deltas (bit walk, FP4 nibble, base code) as bf16
 //                   [token][channel], and the power-of-two K and V scale factors laid out in
 //                   MMA-fragment order.
 //   8 MMA warps     own one unit per stage and a private online-softmax state.  All MMAs are
-//                   m16n8k16 fp16 with the 2-bit codes as the A operand - a code field masked in
-//                   place is the fp16 subnormal code * 4^slot * 2^-24, exact and offset-free - and
+//                   m16n8k16 with the 2-bit codes as the A operand - a code field masked in
+//                   place is a subnormal, exact and offset-free, in bf16 for the logits and in
+//                   fp16 for the output - and
 //                   the query heads as the 8 columns: logits = codes.(q*2^e) + delta.q + q.zp,
 //                   softmax over token rows, P transposed with movmatrix, output =
 //                   codes^T.(P*2^e_v) + vz^T.P.

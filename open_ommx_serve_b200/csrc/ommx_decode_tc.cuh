@@ -132,6 +132,11 @@ __device__ __forceinline__ bool mbar_try_wait_ns(uint32_t bar, uint32_t parity, 
     return ok != 0;
 }
 __device__ __forceinline__ uint32_t dup16(uint32_t h) { return h | (h << 16); }
+// field i (0..7) of the lower and upper 8 codes of a 32-bit code word, as two fp16 subnormals
+// code * 4^slot * 2^-24 with slot = i (i < 5) or i - 5: no arithmetic beyond the AND
+__device__ __forceinline__ uint32_t code_pair(uint32_t w, int i) {
+    return i < 5 ? (w & (0x00030003u << (2 * i))) : ((w >> 10) & (0x00030003u << (2 * (i - 5))));
+}
 // fp16 bits of 2^(e + bias): 0 below the subnormal range of interest (e + bias < -14), clamped at 2^15
 __device__ __forceinline__ uint32_t tc_pow2_f16(int e, int bias, bool &clamped, int limit = 30) {
     int u = e + 15 + bias;

@@ -32,11 +32,9 @@ template <int H> struct WarpLayout {
 constexpr int REGS_MMA = 128, REGS_DECODE = 56, REGS_PRODUCER = 24;
 constexpr int MAX_STAGES = 4;           // ring depth (3 when the planes of a stage are large)
 constexpr int DT_STRIDE = 272;          // bytes per sidecar-tile row (256 data + 16 pad)
-constexpr int ROW_KF = 32;              // K scale factors 2^(e+4) * 4^-slot, fp16, in code-fragment order
+constexpr int ROW_KF = 32;              // K scale factors 2^(e + KF_BIAS) * 4^-slot, bf16, in code-fragment order
 constexpr int ROW_VF = 33;              // V scale factors, fp16, fragment order (rows 33, 34: two copies)
-constexpr int ROW_ZT = 35;              // V zero-points [scale group][token], fp16 (rows 35, 36: two copies)
-constexpr int ZT_STRIDE = 68;           // bytes from one scale group's zero-points to the next (64 + a bank)
-constexpr int DT_ROWS = 37;             // rows 0..31: outlier deltas [token][channel in fragment order], fp16
+constexpr int DT_ROWS = 35;             // rows 0..31: outlier deltas [token][channel in fragment order], bf16
 constexpr int DT_BYTES = DT_ROWS * DT_STRIDE;
 constexpr int MAX_SPLIT_GROUPS = 512;   // groups of the longest split that the entry points accept (16K tokens)
 constexpr int MAX_SPLIT_PAGES = 1024;
@@ -141,8 +139,9 @@ __device__ __forceinline__ void ldsm_b8_trans_x2(uint32_t addr, uint32_t (&r)[4]
     asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t &r0, uint32_t &r1) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
 }
 // transpose an 8x8 matrix of 16-bit elements held one row pair per lane (the accumulator layout)
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
@@ -160,6 +159,16 @@ __device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {       /
     asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
 __device__ __forceinline__ uint32_t hmul2_f16(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
@@ -169,6 +178,18 @@ __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+__device__ __forceinline__ uint32_t top_bit(uint32_t x) {                      // index of the highest set bit
+    uint32_t r;
+    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
+__device__ __forceinline__ void sub_if_bit(float &x, uint32_t word, uint32_t bit, float y) {   // one logic instruction and a predicated add
+    asm("{\n .reg .pred q;\n .reg .b32 t;\n and.b32 t, %1, %2;\n setp.ne.u32 q, t, 0;\n @q sub.f32 %0, %0, %3;\n}\n" : "+f"(x) : "r"(word), "r"(bit), "f"(y));
+}
+__device__ __forceinline__ void sts_u16x2(uint32_t a0, uint32_t a1, uint32_t x) {              // the halves of x to two places
+    asm volatile("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %2;\n st.shared.b16 [%0], l;\n st.shared.b16 [%1], h;\n}\n" ::"r"(a0), "r"(a1), "r"(x) : "memory");
 }
 
 // The 2-bit code planes are staged with the TMA's 128-byte swizzle (16-byte chunk index XOR line
@@ -198,22 +219,14 @@ constexpr int ABL_NO_OUTLIER = 1, ABL_NO_V = 2, ABL_NO_K = 4, ABL_NO_COMPUTE = 8
 constexpr int ABL_TEST_STALL = 16;
 constexpr long long TEST_WAIT_LIMIT_CYCLES = 4000000ll;
 
-// fp16 bits of 2^(e + FBIAS).  Exponents below -18 give 0 (such a scale step is under 2^-18 and the
-// term it multiplies is dropped); exponents above 11 are clamped and reported.
+// V scale factors are fp16, 2^(e + FBIAS): exponents below -18 give 0 (such a scale step is under 2^-18 and the term it multiplies
+// is dropped), exponents above 11 are clamped and reported.  K scale factors are bf16, 2^(e + KF_BIAS), clamped alike.
 constexpr int FBIAS = 4;
-__device__ __forceinline__ uint32_t pow2_f16_bits(int e, bool &clamped) {
-    int u = e + 15 + FBIAS;
-    clamped = u > 30;
-    u = min(u, 30);
-    return u < 1 ? 0u : (uint32_t)u << 10;
-}
-// the reference rounds an outlier's delta to bf16; keep that rounding point, then store it as fp16
-// (exact: 8 significant bits fit in 11)
-__device__ __forceinline__ uint32_t f16x2_of_bf16_rounded(float lo, float hi) {
-    uint32_t b;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b) : "f"(hi), "f"(lo));
-    return pack_f16x2_sat(__uint_as_float(b << 16), __uint_as_float(b & 0xFFFF0000u));
-}
+constexpr int KF_BIAS = 70;
+constexpr int E_TOP = 11 + 128;
+constexpr float LAG = 2.f;              // how far a logit may be ahead of the maximum that P is taken against (natural log)
+constexpr float KF_UNDO = 9223372036854775808.f;      // 2^(133 - KF_BIAS): a code field in place is code * 4^slot * 2^-133
+__host__ __device__ constexpr uint32_t half2_const(int lo, int hi) { return ((uint32_t)lo & 0xFFFFu) | ((uint32_t)hi << 16); }
 // the FP4 levels of four outliers (16 bits of the nibble stream) as the upper bytes of their fp16 values; the lower
 // bytes are zero.  A nibble is the byte selector of the magnitude table; its sign bit, which as a selector bit replicates
 // a byte's sign, turns 0x80 into 0xFF in a second lookup.
@@ -228,13 +241,9 @@ __device__ __forceinline__ uint32_t f16_bits_sat(float x) {
     asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(r) : "f"(x));
     return (uint32_t)r;
 }
-// field i (0..7) of the lower and upper 8 codes of a 32-bit code word, as two fp16 subnormals
-// code * 4^slot * 2^-24 with slot = i (i < 5) or i - 5: no arithmetic beyond the AND
-__device__ __forceinline__ uint32_t code_pair(uint32_t w, int i) {
-    return i < 5 ? (w & (0x00030003u << (2 * i))) : ((w >> 10) & (0x00030003u << (2 * (i - 5))));
-}
-__device__ __forceinline__ int code_slot(int i) { return i < 5 ? i : i - 5; }
-
+// field i (0..7) of the lower and upper 8 codes of a 32-bit code word, as two bf16 subnormals code * 4^slot * 2^-133 with
+// slot = i % 4 (7 mantissa bits and the lowest exponent bit: linear up to there): no arithmetic beyond the AND
+__device__ __forceinline__ uint32_t code_pair_bf16(uint32_t w, int i) { return (i < 4 ? w : w >> 8) & (0x00030003u << (2 * (i & 3))); }
 // Bit planes of the 2-bit codes of 64 channels x 32 tokens, the codes of a channel pair to a lane: w[0], w[1] are the low and the
 // high code bit of its first channel, w[2], w[3] of its second, token = bit.  `addr` is the lane's row for the ldmatrix below:
 // the 16 bytes of token 8 (lane / 4 % 4) + 4 (lane / 16) + lane % 4.  Lane 4g + j gets byte column g (j < 2) or g + 8, channels
@@ -438,25 +447,31 @@ constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_
 }
 // KOUT: outliers per K vector known at compile time (static, unrolled splice) or -1 (runtime).
 //
-// Every MMA is m16n8k16 fp16 with the 2-bit codes as the A operand: a code field masked in place is an
-// fp16 subnormal, code * 4^slot * 2^-24, exact and without an offset.  N = 8 columns are the query heads
-// of the kv head (GQA <= 8).
+// Every MMA is m16n8k16.  Logits in bf16: a 2-bit code field masked in place is a bf16 subnormal, code * 4^slot * 2^-133, exact and
+// without an offset (subnormal operands run at full rate), and q, the factors 2^e and the deltas are bf16 as they are, so no
+// product is rounded.  Output in fp16, whose subnormals hold a code field too (code * 4^slot * 2^-24) and whose 11 bits P needs.
+// N = 8 columns are the query heads of the kv head (GQA <= 8).
 //   logits   S^T[token][head]  = codes[token][ch] . (q * 2^e_k)[ch][head]      (2 m-tiles x 8 k-steps)
 //                              + delta[token][ch] . q[ch][head]                (sidecar tile, same shape)
 //                              + zp[ch] . q[ch][head]                          (one row, broadcast)
 //   output   O^T[ch][head]     = codes^T[ch][token] . (P * 2^e_v)[token][head] (8 m-tiles x 2 k-steps, the
 //                                16 rows of an m-tile lie in one V scale group)
 //                              + vz^T[group][token] . P[token][head]
-// The power-of-two factors, zero-points and deltas of a unit are laid out for these fragments by the
-// decode warps (the sidecar tile), so the MMA warps multiply and accumulate and do little else; what they
-// still compute themselves, q.zp, fits into their wait for the deltas.
+// The power-of-two factors and deltas of a unit are laid out for these fragments by the decode warps (the sidecar tile), so the MMA
+// warps multiply and accumulate and do little else; q.zp, which they compute themselves, fits into their wait for the deltas, and the
+// V zero-points come straight out of the staged plane by a transposed ldmatrix.
 //
-// Bound by instruction issue and the logic pipe, which both roles share (leaving out any part of either saves its share), and in the
-// chain view by an MMA warp's unit: about 4600 cycles of code MMAs, delta MMAs, softmax and P.V in a row, with the decode warps
-// that feed it close behind; the register file (8 x 128 + 16 x 56 a lane) holds no second unit in flight, and memory is at a
-// quarter of its rate.  Measured, this stage alone, before the running list, the cheaper unit and PLAIN -> with them: 64K tokens x 8
-// heads 50.2 -> 40.1 us; 8 x 32K 184 -> 142.5 us; 32 sequences of 1K to 32K in splits of 512 with the store and stage 2 around it
-// 560 -> 318 us.
+// Bound by issue slots, the logic pipe and shared-memory wavefronts (397 of them per unit, three quarters of what the pipe can
+// do in the steady state), which both roles share: leaving out any part of either saves its share, and the MMA warps' chain of code
+// MMAs, delta MMAs, softmax and P.V stands close behind.  The register file (8 x 128 + 16 x 56 a lane) holds no second unit in
+// flight, and memory is at a third of its rate.  Logits in bf16 (the deltas need no second conversion), one packed min-max-add per
+// factor pair, V factors by one warp with lane = token and zero-points without staging, code words by ldmatrix, zero-point words
+// used as loaded, and a maximum that follows lazily, before -> with them, this stage and stage 2: 64K x 8 heads 44.8 -> 41.8 us;
+// 8 x 32K, 70B heads 148.7 -> 136.7; 32 sequences of 1K to 32K in splits of 512 with the store 318 -> 294.
+// Tried and slower (64K / 70B): 16 warps that each build and use their own half tile, no hand-overs (47.2 / 162 us, latency-bound
+// at four warps a scheduler); 16 delta warps with their own MMAs beside 8 output warps (46.1 / 167); tile rows zeroed by an
+// out-of-range tensor-map load (83 / 289); FP4 levels by the conversion instruction and a shorter wait loop (53 fewer of 1532
+// instructions per unit, same time).
 //
 // PLAIN: the recipes that are served - bitmask or relidx7 index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
@@ -685,12 +700,11 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     const int cp = 8 * (lane & 2) + 2 * (lane >> 2) + (lane & 1);
     const int da = cp & 3, dh = (cp >> 2) & 1, dj = cp >> 3;
     const int lm_tok = 8 * ((lane >> 2) & 3) + 4 * (lane >> 4) + (lane & 3);
-    // 4^-slot of those two channels' code fields, fp16
-    const uint32_t slot_scale = da == 0 ? 0x34003C00u : (da == 1 ? 0x24002C00u : (da == 2 ? 0x3C001C00u : 0x2C003400u));
     // Build the sidecar tile of a unit between two uses by its MMA warp.  A tile is built in two
     // halves by two warps at once, because the MMA warp of the unit waits for it: half hf takes 64 of the
     // K channels (delta columns, scale factors) and V tokens 16hf..16hf+15 (factors, zero-points).
     // Returns false when a bounded wait ran out.
+    uint32_t e_max = 0;                                          // largest scale exponents seen, biased by 128, two halves
     auto decode_item = [&](const Piece &pc, const int n) __attribute__((always_inline)) -> bool {
         const int it = n / (2 * NCW), unit = (n >> 1) % NCW, hf = n & 1;
         const int h = unit % H, gsel = unit / H;
@@ -708,8 +722,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const bool splice = k_out > 0 && !no_outlier;
         // ---- everything that only reads the stage comes before the wait for the tile, which the MMA warps make a decode warp
         //      wait for (a sixth of its time): the parameters of both channels, the K and V factors, V zero-points ----
-        bool clamped_any = false;
-        uint32_t e2 = 0, z2 = 0, kf = 0, vf = 0, zt = 0, ms2 = 0, mc2 = 0;
+        uint32_t e2 = 0, z2 = 0, kf = 0, f02 = 0, f13 = 0, ms2 = 0, mc2 = 0;
         uint2 bm2 = make_uint2(0u, 0u);
         // From 6 outliers on the base codes are looked up in bit planes in registers: a gather per outlier costs 3 to 4 conflicting
         // shared-memory wavefronts, the planes of 64 channels about 50 instructions.  64K x 8 heads, stage 1: k = 12 53.8 -> 50.2 us,
@@ -722,14 +735,25 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const uint8_t *k_hi = gb + (h >> 2) * 128;
         const uint32_t k_sw = ((uint32_t)(h >> 2) * 16u) & SWZ;
         uint32_t st[2] = {0, 0}, sth[2] = {0, 0};                // nibble stream of each channel: outliers 0..7, 8..15
-        const int vtk = 16 * hf + 2 * (lane & 7), vcg = lane >> 3;   // V side: lane = (pair of tokens, scale group)
         if (active) {
             e2 = *reinterpret_cast<const uint16_t *>(gb + o_ks + h * 128 + d0);
             z2 = *reinterpret_cast<const uint32_t *>(gb + o_kz + h * 256 + 2 * d0);
-            uint32_t v0 = 0x80u, v1 = 0x80u, y0 = 0u, y1 = 0u;   // exponent -128 -> factor 0
-            const uint8_t *vs = gb + o_vs + (vtk * H + h) * 4 + vcg, *vz = gb + o_vz + (vtk * H + h) * 8 + 2 * vcg;
-            if (32 * lg + vtk < pc.ntok) { v0 = vs[0]; y0 = *reinterpret_cast<const uint16_t *>(vz); }
-            if (32 * lg + vtk + 1 < pc.ntok) { v1 = vs[4 * H]; y1 = *reinterpret_cast<const uint16_t *>(vz + 8 * H); }
+            {
+                // K scale factors 2^(e + KF_BIAS) * 4^-slot of the two channels, bf16
+                const uint32_t eb = __byte_perm(e2 ^ 0x8080u, 0u, 0x4140u);                       // e + 128, two halves
+                e_max = __vmaxs2(e_max, eb);
+                const uint32_t off = da & 1 ? half2_const(KF_BIAS - 5, KF_BIAS - 7) : half2_const(KF_BIAS - 1, KF_BIAS - 3);
+                const uint32_t top = da & 1 ? half2_const(E_TOP + KF_BIAS - 5, E_TOP + KF_BIAS - 7) : half2_const(E_TOP + KF_BIAS - 1, E_TOP + KF_BIAS - 3);
+                kf = __viaddmin_s16x2(eb, off, top) << 7;
+            }
+            if (hf == 0) {
+                // V scale factors 2^(e + FBIAS), fp16, of the four scale groups; lane = token
+                const uint32_t w = 32 * lg + lane < pc.ntok ? *reinterpret_cast<const uint32_t *>(gb + o_vs + (lane * H + h) * 4) ^ 0x80808080u : 0u;
+                const uint32_t e02 = w & 0x00FF00FFu, e13 = (w >> 8) & 0x00FF00FFu;               // e + 128, groups 0, 2 and 1, 3
+                e_max = __vimax3_s16x2(e_max, e02, e13);
+                f02 = __viaddmin_s16x2_relu(e02, half2_const(FBIAS + 15 - 128, FBIAS + 15 - 128), half2_const(30, 30)) << 10;
+                f13 = __viaddmin_s16x2_relu(e13, half2_const(FBIAS + 15 - 128, FBIAS + 15 - 128), half2_const(30, 30)) << 10;
+            }
             if (splice) {
                 if (use_map) {
                     ms2 = *reinterpret_cast<const uint32_t *>(gb + o_ms + h * 256 + 2 * d0);
@@ -814,13 +838,6 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             }
             if constexpr (PLANES)
                 if (splice) code_bit_planes(smem_u32(k_hi + lm_tok * TS) + (((h & 3) * 32 + 16 * hf) ^ k_sw ^ (((uint32_t)(lm_tok * TS) >> 3) & SWZ)), lane, cw);
-            bool cl0, cl1, cl2, cl3;
-            const uint32_t k0 = pow2_f16_bits(max((int)(int8_t)e2, -126), cl0), k1 = pow2_f16_bits(max((int)(int8_t)(e2 >> 8), -126), cl1);
-            kf = hmul2_f16(k0 | (k1 << 16), slot_scale);         // * 4^-slot: exact, subnormals included
-            const uint32_t f0 = pow2_f16_bits((int)(int8_t)v0, cl2), f1 = pow2_f16_bits((int)(int8_t)v1, cl3);
-            vf = f0 | (f1 << 16);
-            zt = pack_f16x2_sat(bf16_bits_to_f32(y0), bf16_bits_to_f32(y1));
-            clamped_any = cl0 || cl1 || cl2 || cl3;
         }
         // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
         // run up to NS groups ahead and the tiles of one unit are built by different warps, so
@@ -838,9 +855,13 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             uint8_t *row = tile + ROW_KF * DT_STRIDE + 128 * hf + 64 * (da >> 1) + 16 * dj + 8 * (da & 1) + 2 * dh;
             *reinterpret_cast<uint16_t *>(row) = (uint16_t)kf;
             *reinterpret_cast<uint16_t *>(row + 4) = (uint16_t)(kf >> 16);
-            const int copy = it & 1;
-            *reinterpret_cast<uint32_t *>(tile + (ROW_VF + copy) * DT_STRIDE + 64 * vcg + 16 * (lane & 3) + 8 * hf + 4 * ((lane >> 2) & 1)) = vf;
-            *reinterpret_cast<uint32_t *>(tile + (ROW_ZT + copy) * DT_STRIDE + 2 * vtk + ZT_STRIDE * vcg) = zt;
+            if (hf == 0) {
+                uint8_t *at = tile + (ROW_VF + (it & 1)) * DT_STRIDE + 16 * ((lane >> 1) & 3) + 8 * (lane >> 4) + 4 * ((lane >> 3) & 1) + 2 * (lane & 1);
+                *reinterpret_cast<uint16_t *>(at) = (uint16_t)f02;
+                *reinterpret_cast<uint16_t *>(at + 64) = (uint16_t)f13;
+                *reinterpret_cast<uint16_t *>(at + 128) = (uint16_t)(f02 >> 16);
+                *reinterpret_cast<uint16_t *>(at + 192) = (uint16_t)(f13 >> 16);
+            }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_trows + 8 * unit);
             // ---- then the outlier deltas of this half's columns ----
@@ -850,98 +871,108 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 for (int k2 = 0; k2 < 8; ++k2)
                     *reinterpret_cast<uint4 *>(tile + (4 * k2 + (lane >> 3)) * DT_STRIDE + 128 * hf + 16 * (lane & 7)) = make_uint4(0, 0, 0, 0);
                 __syncwarp();                                        // the cleared rows before any delta lands in them
-                const uint32_t bmv[2] = {bm2.x, bm2.y};
                 const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2)) ^ k_sw;
                 auto code_byte = [&](uint32_t pz) -> uint32_t {
                     return k_hi[pz * TS + (k_lo ^ (((pz * TS) >> 3) & SWZ))];
                 };
+                const uint32_t colp = smem_u32(tile) + 128 * hf + 32 * da + 4 * dj + 2 * dh;
+                uint32_t bmv[2] = {bm2.x, bm2.y};
+                float scale[2], lvlA[2], offs[2];                // delta of an outlier: lvl * lvlA + offs - code * scale
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
-                    const int e = max((int)(int8_t)(e2 >> (8 * c)), -126);
-                    const float sc = __uint_as_float((uint32_t)(e + 127) << 23);
-                    const float zp = bf16_bits_to_f32(c ? (z2 >> 16) : (z2 & 0xFFFFu));
-                    // delta between the outlier value and the base value it replaces: lvl * A + Bc - code * sc
-                    float A = sc, Bc = 0.f;                     // shared map: lvl*s + zp - (code*s + zp)
+                    scale[c] = __uint_as_float((uint32_t)(max((int)(int8_t)(e2 >> (8 * c)), -126) + 127) << 23);
+                    const float zp = __uint_as_float(c ? z2 & 0xFFFF0000u : z2 << 16);
+                    lvlA[c] = scale[c];                          // shared map: lvl*s + zp - (code*s + zp)
+                    offs[c] = 0.f;
                     if (use_map) {
-                        const float ms = bf16_bits_to_f32(c ? (ms2 >> 16) : (ms2 & 0xFFFFu));
-                        const float mc = bf16_bits_to_f32(c ? (mc2 >> 16) : (mc2 & 0xFFFFu));
-                        A = __fdividef(1.f, ms);
-                        Bc = mc - zp;
+                        lvlA[c] = __fdividef(1.f, __uint_as_float(c ? ms2 & 0xFFFF0000u : ms2 << 16));
+                        offs[c] = __uint_as_float(c ? mc2 & 0xFFFF0000u : mc2 << 16) - zp;
                     }
+                }
+                if constexpr (KOUT > 0 && KOUT % 2 == 0) {
+                    // a bitmask that disagrees with the value stream: reported, no deltas for that channel
+                    const bool bad0 = __popc(bmv[0]) != KOUT, bad1 = __popc(bmv[1]) != KOUT;
+                    if (__any_sync(0xFFFFFFFFu, bad0 || bad1)) {
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+                            if (c ? bad1 : bad0) {
+                                or_status(p.status, OMMX_ST_BAD_GROUP);
+                                bmv[c] = (1u << KOUT) - 1u;
+                                scale[c] = lvlA[c] = offs[c] = 0.f;
+                            }
+                    }
+                }
+                if constexpr (PLANES) {
+                    // both channels side by side: two bit walks in flight
+#pragma unroll
+                    for (int r = KOUT - 2; r >= 0; r -= 2)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const uint32_t nib = r < 8 ? (r & 4 ? st[c] >> 16 : st[c]) : (r & 4 ? sth[c] >> 16 : sth[c]);
+                            const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
+                            const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
+                            const uint32_t p1 = top_bit(bmv[c]), m1 = 1u << p1;
+                            bmv[c] ^= m1;
+                            const uint32_t p0 = top_bit(bmv[c]), m0 = 1u << p0;
+                            bmv[c] ^= m0;
+                            float x0 = fmaf(lvf.x, lvlA[c], offs[c]), x1 = fmaf(lvf.y, lvlA[c], offs[c]);
+                            sub_if_bit(x0, cw[2 * c], m0, scale[c]);
+                            sub_if_bit(x1, cw[2 * c], m1, scale[c]);
+                            sub_if_bit(x0, cw[2 * c + 1], m0, 2.f * scale[c]);
+                            sub_if_bit(x1, cw[2 * c + 1], m1, 2.f * scale[c]);
+                            sts_u16x2(colp + 16 * c + p0 * DT_STRIDE, colp + 16 * c + p1 * DT_STRIDE, pack_bf16x2(x0, x1));
+                        }
+                } else {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
                     uint32_t bits = bmv[c];
+                    const float sc = scale[c], A = lvlA[c], Bc = offs[c];
                     const uint32_t stream = st[c], stream_hi = sth[c];
                     (void)stream_hi;
                     const int fsh = 2 * ((d0 & 3) + c);          // bit position of the channel's code in its byte
-                    uint8_t *col = tile + 128 * hf + 32 * da + 16 * c + 4 * dj + 2 * dh;
+                    const uint32_t col = colp + 16 * c;
                     if constexpr (KOUT > 0 && KOUT % 2 == 0) {
-                        if (__popc(bits) == KOUT) {
-                            if constexpr (PLANES) {
-                                const float sc2 = 2.f * sc;
+                        // The code enters as the fraction of 1 + code/4, whose bits an AND and an OR make, so that 4 * sc moves to
+                        // the constant: lvl * A + (Bc + 4 sc) - (1 + code/4) * 4 sc.
+                        const float Bq = fmaf(4.f, sc, Bc), Sq = -4.f * sc;
+                        const int sh = 21 - fsh;                 // moves the code to the top of the mantissa
+                        // Two passes: all gathers (bit walk, base-code byte) first, then the arithmetic and the
+                        // stores.  In one pass every load would have to follow the previous outlier's store in
+                        // program order (shared memory may alias), i.e. KOUT load round trips in a row.
+                        uint32_t pzs[KOUT], cbs[KOUT];
 #pragma unroll
-                                for (int r = KOUT - 2; r >= 0; r -= 2) {
-                                    const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
-                                    const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
-                                    const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
-                                    const uint32_t p1 = 31 - __clz(bits), m1 = 1u << p1;
-                                    bits ^= m1;
-                                    const uint32_t p0 = 31 - __clz(bits), m0 = 1u << p0;
-                                    bits ^= m0;
-                                    float x0 = fmaf(lvf.x, A, Bc), x1 = fmaf(lvf.y, A, Bc);
-                                    if (cw[2 * c] & m0) x0 -= sc;
-                                    if (cw[2 * c + 1] & m0) x0 -= sc2;
-                                    if (cw[2 * c] & m1) x1 -= sc;
-                                    if (cw[2 * c + 1] & m1) x1 -= sc2;
-                                    const uint32_t X = f16x2_of_bf16_rounded(x0, x1);
-                                    *reinterpret_cast<uint16_t *>(col + p0 * DT_STRIDE) = (uint16_t)X;
-                                    *reinterpret_cast<uint16_t *>(col + p1 * DT_STRIDE) = (uint16_t)(X >> 16);
-                                }
-                            } else {
-                                // The code enters as the fraction of 1 + code/4, whose bits an AND and an OR make, so that 4 * sc moves to
-                                // the constant: lvl * A + (Bc + 4 sc) - (1 + code/4) * 4 sc.
-                                const float Bq = fmaf(4.f, sc, Bc), Sq = -4.f * sc;
-                                const int sh = 21 - fsh;              // moves the code to the top of the mantissa
-                                // Two passes: all gathers (bit walk, base-code byte) first, then the arithmetic and the
-                                // stores.  In one pass every load would have to follow the previous outlier's store in
-                                // program order (shared memory may alias), i.e. KOUT load round trips in a row.
-                                uint32_t pzs[KOUT], cbs[KOUT];
+                        for (int r = KOUT - 1; r >= 0; --r) {
+                            const uint32_t pz = top_bit(bits);
+                            bits ^= 1u << pz;
+                            pzs[r] = pz;
+                            cbs[r] = code_byte(pz);
+                        }
 #pragma unroll
-                                for (int r = KOUT - 1; r >= 0; --r) {
-                                    const uint32_t pz = 31 - __clz(bits);
-                                    bits ^= 1u << pz;
-                                    pzs[r] = pz;
-                                    cbs[r] = code_byte(pz);
-                                }
-#pragma unroll
-                                for (int r = 0; r < KOUT; r += 2) {
-                                    const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
-                                    const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
-                                    const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
-                                    const float v0 = __uint_as_float(((cbs[r] << sh) & 0x600000u) | 0x3F800000u);
-                                    const float v1 = __uint_as_float(((cbs[r + 1] << sh) & 0x600000u) | 0x3F800000u);
-                                    const uint32_t X = f16x2_of_bf16_rounded(fmaf(v0, Sq, fmaf(lvf.x, A, Bq)), fmaf(v1, Sq, fmaf(lvf.y, A, Bq)));
-                                    *reinterpret_cast<uint16_t *>(col + pzs[r] * DT_STRIDE) = (uint16_t)X;
-                                    *reinterpret_cast<uint16_t *>(col + pzs[r + 1] * DT_STRIDE) = (uint16_t)(X >> 16);
-                                }
-                            }
-                        } else {
-                            or_status(p.status, OMMX_ST_BAD_GROUP);   // bitmask and value stream disagree
+                        for (int r = 0; r < KOUT; r += 2) {
+                            const uint32_t nib = r < 8 ? (r & 4 ? stream >> 16 : stream) : (r & 4 ? stream_hi >> 16 : stream_hi);
+                            const uint32_t lv = __byte_perm(fp4_levels_hi(nib), 0u, r & 2 ? 0x3424u : 0x1404u);
+                            const float2 lvf = __half22float2(*reinterpret_cast<const __half2 *>(&lv));
+                            const float v0 = __uint_as_float(((cbs[r] << sh) & 0x600000u) | 0x3F800000u);
+                            const float v1 = __uint_as_float(((cbs[r + 1] << sh) & 0x600000u) | 0x3F800000u);
+                            sts_u16x2(col + pzs[r] * DT_STRIDE, col + pzs[r + 1] * DT_STRIDE,
+                                      pack_bf16x2(fmaf(v0, Sq, fmaf(lvf.x, A, Bq)), fmaf(v1, Sq, fmaf(lvf.y, A, Bq))));
                         }
                     } else {
                         // any other k: one pass at run time
                         int r = __popc(bits) - 1;
                         while (bits) {
-                            const uint32_t pz = 31 - __clz(bits);
+                            const uint32_t pz = top_bit(bits);
                             bits ^= 1u << pz;
                             const uint32_t nib = ((r < 8 ? stream : stream_hi) >> (4 * (r & 7))) & 0xFu;
                             --r;
                             const float cf = (float)((code_byte(pz) >> fsh) & 3u);
                             const float X = fmaf(cf, -sc, fmaf(s_lut[nib], A, Bc));
-                            *reinterpret_cast<uint16_t *>(col + pz * DT_STRIDE) = (uint16_t)f16x2_of_bf16_rounded(X, X);
+                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(col + pz * DT_STRIDE), "h"((uint16_t)pack_bf16x2(X, X)) : "memory");
                         }
                     }
                 }
+                }
             }
-            if (clamped_any) or_status(p.status, OMMX_ST_SCALE_RANGE);
         } else if (lane == 0) {
             mbar_arrive(bar_trows + 8 * unit);
         }
@@ -1006,11 +1037,13 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         // the producer takes the very last item, when this CTA's pieces end with one that is known to be the last
         for (int n = is_producer ? pc.it1 * 2 * NCW - 1 : dw;; n += NDW) {
             const int it = n / (2 * NCW);
-            while (it >= pc.it1)
-                if (!step_piece()) return;
-            if (!WIDE && !is_producer && !pc.more && n == pc.it1 * 2 * NCW - 1) return;
-            if (!decode_item(pc, n)) return;
+            bool more = true;
+            while (it >= pc.it1 && (more = step_piece())) {}
+            if (!more || (!WIDE && !is_producer && !pc.more && n == pc.it1 * 2 * NCW - 1) || !decode_item(pc, n)) break;
         }
+        // an exponent that the factors cannot hold was clamped
+        if ((int)(e_max & 0xFFFFu) > E_TOP || (int)(e_max >> 16) > E_TOP) or_status(p.status, OMMX_ST_SCALE_RANGE);
+        return;
     }
 
     // =========================== MMA warps ===========================
@@ -1019,7 +1052,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     const int h = unit % H, gsel = unit / H;
     const uint8_t *tile = s_tiles + unit * DT_BYTES;
     const uint32_t tile_s = smem_u32(tile);
-    // Column n = g of every MMA is query head g of this kv head.
+    // Column n = g of every MMA is query head g of this kv head.  Columns past the last head repeat head 0; nobody reads them.
     const bool head_ok = g < p.gqa;
     // per-lane fragment addresses inside the sidecar tile
     const uint32_t a_delta = tile_s + ((lane & 7) + 8 * ((lane >> 3) & 1)) * DT_STRIDE + 16 * (lane >> 4);
@@ -1029,14 +1062,16 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     // are, bytes 1 and 3 after a shift.
     const uint32_t v_off = swz128((uint32_t)((2 * ((lane & 15) >> 2) + ((lane >> 1) & 1) + 8 * (lane & 1)) * TS + h * 32 + 16 * (lane >> 4)), SWZ);
     static_assert(SWZ == 0 || (16 * TS) % 1024 == 0, "the second half of the tokens has the same swizzle");
+    // V zero-points come out of the plane as an A operand by a transposed load: two heads' four of a token are one 16-byte row
+    constexpr int ZROW = H > 1 ? 4 : 0;                             // rows of the odd head
+    const int zr = ZROW * (h & 1);
     const bool do_k = !(abl & ABL_NO_K), do_v = !(abl & ABL_NO_V);
     const bool has_delta = !(k_out == 0 || no_outlier);
 
     bool gave_up = false;                        // a wait ran out: no more groups, but every piece still goes through its epilogue
     do {
-    // B fragments of q.  QR: raw bf16, registers 4v..4v+3 hold channels 32v + 8j .. + 7 (zero-point MMAs).  QP: fp16 of
-    // bf16(q * sm_scale), register r = 8w + i holds channels (64w + 16j + i, + 8), the pair a code word yields in one AND (code
-    // and delta MMAs).
+    // B fragments of q, bf16.  QR: raw, registers 4v..4v+3 hold channels 32v + 8j .. + 7 (zero-point MMAs).  QP: q * sm_scale
+    // rounded, register r = 8w + i holds channels (64w + 16j + i, + 8), the pair a code word yields in one AND (code and delta MMAs).
     uint32_t QR[16], QP[16];
     {
         const uint16_t *qrow = reinterpret_cast<const uint16_t *>(p.q + (int64_t)pc.b * p.q_sb + (int64_t)(h * p.gqa + (head_ok ? g : 0)) * p.q_sh);
@@ -1054,9 +1089,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             uint32_t w[4];
             eight(qrow + 32 * v + 8 * j, w);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) QR[4 * v + i] = head_ok ? w[i] : 0u;
+            for (int i = 0; i < 4; ++i) QR[4 * v + i] = w[i];
         }
-        auto scaled = [&](uint32_t b16) { return bf16_round_f32(bf16_bits_to_f32(b16 & 0xFFFFu) * p.sm_scale); };
+        auto scaled = [&](uint32_t b16) { return bf16_bits_to_f32(b16 & 0xFFFFu) * p.sm_scale; };
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
             uint32_t lo[4], hi[4];
@@ -1064,7 +1099,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             eight(qrow + 64 * w + 16 * j + 8, hi);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                QP[8 * w + i] = head_ok ? pack_f16x2(scaled(lo[i >> 1] >> (16 * (i & 1))), scaled(hi[i >> 1] >> (16 * (i & 1)))) : 0u;
+                QP[8 * w + i] = pack_bf16x2(scaled(lo[i >> 1] >> (16 * (i & 1))), scaled(hi[i >> 1] >> (16 * (i & 1))));
         }
     }
     // ---- online softmax state of heads 2j and 2j+1 (the two columns this lane holds) ----
@@ -1073,7 +1108,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     float acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f; }
-    float accz[4] = {0.f, 0.f, 0.f, 0.f};        // rows = V scale groups: sum_t vz[t][cg] * P[t][head]
+    float accz[4] = {0.f, 0.f, 0.f, 0.f};        // rows = V scale groups (from row zr): sum_t vz[t][cg] * P[t][head]
 
     for (int it = pc.it0; it < pc.it1 && !gave_up; ++it) {
         const int s = ring_slot(it, NS);
@@ -1090,15 +1125,11 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
 
             // ======================= logits =======================
             // code words of this lane's four token rows (tokens 8*nt + g), channels 16j..16j+15 of either half
-            uint2 kw[4];
+            uint32_t kw[2][4] = {};
+            if (do_k)
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                kw[nt] = make_uint2(0u, 0u);
-                if (do_k) {
-                    kw[nt].x = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 4 * j), SWZ));
-                    kw[nt].y = *reinterpret_cast<const uint32_t *>(gb + swz128((uint32_t)((8 * nt + g) * TS + h * 32 + 16 + 4 * j), SWZ));
-                }
-            }
+                for (int w = 0; w < 2; ++w)
+                    ldsm_x4(smem_u32(gb) + swz128((uint32_t)(lane * TS + h * 32 + 16 * w), SWZ), kw[w][0], kw[w][1], kw[w][2], kw[w][3]);
             // The unit's sidecar tile arrives in two steps: first the factor and zero-point rows, then the outlier
             // deltas.  The code MMAs run on the first, while the decode warps still scatter the deltas.
             if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
@@ -1116,27 +1147,29 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
 #pragma unroll
                 for (int q = 2 * q2; q < 2 * q2 + 2; ++q) {
                     const int wi = q >> 2, i0 = 2 * (q & 3);
-                    const uint32_t b0 = hmul2_f16(QP[2 * q], q & 1 ? f.z : f.x), b1 = hmul2_f16(QP[2 * q + 1], q & 1 ? f.w : f.y);
+                    const uint32_t b0 = hmul2_bf16(QP[2 * q], q & 1 ? f.z : f.x), b1 = hmul2_bf16(QP[2 * q + 1], q & 1 ? f.w : f.y);
 #pragma unroll
                     for (int mt = 0; mt < 2; ++mt) {
-                        const uint32_t wlo = wi ? kw[2 * mt].y : kw[2 * mt].x, whi = wi ? kw[2 * mt + 1].y : kw[2 * mt + 1].x;
-                        mma_f16(Sc[mt], code_pair(wlo, i0), code_pair(whi, i0), code_pair(wlo, i0 + 1), code_pair(whi, i0 + 1), b0, b1);
+                        const uint32_t wlo = kw[wi][2 * mt], whi = kw[wi][2 * mt + 1];
+                        mma_bf16(Sc[mt], code_pair_bf16(wlo, i0), code_pair_bf16(whi, i0), code_pair_bf16(wlo, i0 + 1), code_pair_bf16(whi, i0 + 1), b0, b1);
                     }
                 }
             }
-            // q.zp of heads 2j and 2j+1: exact bf16 products of the raw query with the zero-points, summed in fp32, every row
-            // of the A operand being the zero-point row.  It needs no tile, so it stands where this warp may have to wait for the deltas.
+            // q.zp of heads 2j and 2j+1: exact bf16 products of the raw query with the zero-points, summed in fp32.  It needs no tile, so
+            // it stands where this warp may have to wait for the deltas.  The eight zero-points a lane loads stand in an A operand as
+            // they come, rows 0-7 holding words 0 and 2, rows 8-15 words 1 and 3: with the query's words 0 and 2 the first rows are
+            // of use, with 1 and 3 the others.
             float Z0[4] = {0.f, 0.f, 0.f, 0.f}, Z1[4] = {0.f, 0.f, 0.f, 0.f};
             {
                 const uint8_t *zrow = gb + o_kz + h * 256 + 16 * j;
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                     const uint4 z = *reinterpret_cast<const uint4 *>(zrow + 64 * v);
-                    mma_bf16(Z0, z.x, z.x, z.y, z.y, QR[4 * v], QR[4 * v + 1]);
-                    mma_bf16(Z1, z.z, z.z, z.w, z.w, QR[4 * v + 2], QR[4 * v + 3]);
+                    mma_bf16(Z0, z.x, z.y, z.z, z.w, QR[4 * v], QR[4 * v + 2]);
+                    mma_bf16(Z1, z.x, z.y, z.z, z.w, QR[4 * v + 1], QR[4 * v + 3]);
                 }
             }
-            const float Sz[2] = {(Z0[0] + Z1[0]) * p.sm_scale, (Z0[1] + Z1[1]) * p.sm_scale};
+            const float Sz[2] = {(Z0[0] + Z1[2]) * p.sm_scale, (Z0[1] + Z1[3]) * p.sm_scale};
             if (has_delta) {
                 if (!mbar_wait(bar_tfull + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
                     gave_up = true;
@@ -1147,9 +1180,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     ldsm_x4(a_delta + 16 * DT_STRIDE + 32 * q, d1f[0], d1f[1], d1f[2], d1f[3]);
-                    mma_f16(Sd[0], d0f[0], d0f[1], d0f[2], d0f[3], QP[2 * q], QP[2 * q + 1]);
+                    mma_bf16(Sd[0], d0f[0], d0f[1], d0f[2], d0f[3], QP[2 * q], QP[2 * q + 1]);
                     if (q < 7) ldsm_x4(a_delta + 32 * (q + 1), d0f[0], d0f[1], d0f[2], d0f[3]);
-                    mma_f16(Sd[1], d1f[0], d1f[1], d1f[2], d1f[3], QP[2 * q], QP[2 * q + 1]);
+                    mma_bf16(Sd[1], d1f[0], d1f[1], d1f[2], d1f[3], QP[2 * q], QP[2 * q + 1]);
                 }
             }
             __syncwarp();
@@ -1162,7 +1195,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-                for (int r = 0; r < 4; ++r) x[mt][r] = fmaf(Sc[mt][r], 1048576.f, Sd[mt][r] + Sz[r & 1]);
+                for (int r = 0; r < 4; ++r) x[mt][r] = fmaf(Sc[mt][r], KF_UNDO, Sd[mt][r] + Sz[r & 1]);
             if (!PLAIN && p.logit_cap > 0.f) {
 #pragma unroll
                 for (int mt = 0; mt < 2; ++mt)
@@ -1177,32 +1210,39 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     for (int r = 0; r < 4; ++r)
                         if (tok_base + 16 * mt + g + 8 * (r >> 1) >= pc.ntok) x[mt][r] = -INFINITY;
             }
-            float corr[2], mneg[2];
+            // The reference maximum follows only when a logit is more than LAG ahead of it, so that most units need neither the
+            // maximum over the lanes nor a rescaled accumulator; P is kept below 2^0 by the same distance.
+            bool ahead = false;
+            float mloc[2];
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                float mloc = fmaxf(fmaxf(x[0][hh], x[0][2 + hh]), fmaxf(x[1][hh], x[1][2 + hh]));
-                mloc = fmaxf(mloc, __shfl_xor_sync(0xFFFFFFFFu, mloc, 4));
-                mloc = fmaxf(mloc, __shfl_xor_sync(0xFFFFFFFFu, mloc, 8));
-                mloc = fmaxf(mloc, __shfl_xor_sync(0xFFFFFFFFu, mloc, 16));
-                const float m_new = fmaxf(m_run[hh], mloc);
-                const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-                corr[hh] = fast_exp2((m_run[hh] - m_use) * LOG2E);   // m_run = -inf -> 0
-                mneg[hh] = -m_use * LOG2E;
-                m_run[hh] = m_new;
+                mloc[hh] = fmaxf(fmaxf(x[0][hh], x[0][2 + hh]), fmaxf(x[1][hh], x[1][2 + hh]));
+                ahead = ahead || mloc[hh] > m_run[hh] + LAG;
             }
+            if (__any_sync(0xFFFFFFFFu, ahead)) {
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    mloc[hh] = fmaxf(mloc[hh], __shfl_xor_sync(0xFFFFFFFFu, mloc[hh], 4));
+                    mloc[hh] = fmaxf(mloc[hh], __shfl_xor_sync(0xFFFFFFFFu, mloc[hh], 8));
+                    mloc[hh] = fmaxf(mloc[hh], __shfl_xor_sync(0xFFFFFFFFu, mloc[hh], 16));
+                    const float m_new = fmaxf(m_run[hh], mloc[hh]);
+                    const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+                    const float corr = fast_exp2((m_run[hh] - m_use) * LOG2E);   // m_run = -inf -> 0
+                    m_run[hh] = m_new;
+                    l_run[hh] *= corr;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { acc[i][hh] *= corr; acc[i][2 + hh] *= corr; }
+                    accz[hh] *= corr;
+                }
+            }
+            const float mneg[2] = {m_run[0] == -INFINITY ? 0.f : -(m_run[0] + LAG) * LOG2E, m_run[1] == -INFINITY ? 0.f : -(m_run[1] + LAG) * LOG2E};
             float pr[2][4];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                 for (int r = 0; r < 4; ++r) pr[mt][r] = fast_exp2(fmaf(x[mt][r], LOG2E, mneg[r & 1]));
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-                l_run[hh] = l_run[hh] * corr[hh] + ((pr[0][hh] + pr[0][2 + hh]) + (pr[1][hh] + pr[1][2 + hh]));   // this lane's tokens only
-            if (__any_sync(0xFFFFFFFFu, corr[0] != 1.0f || corr[1] != 1.0f)) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) { acc[i][0] *= corr[0]; acc[i][1] *= corr[1]; acc[i][2] *= corr[0]; acc[i][3] *= corr[1]; }
-                accz[0] *= corr[0]; accz[1] *= corr[1];
-            }
+            for (int hh = 0; hh < 2; ++hh) l_run[hh] += (pr[0][hh] + pr[0][2 + hh]) + (pr[1][hh] + pr[1][2 + hh]);   // this lane's tokens only
             // P^T as B fragments: transpose each 8x8 (token, head) block; T[ks][b] = tokens 16ks + 8b + 2j, +1 of head g
             uint32_t T[2][2];
 #pragma unroll
@@ -1223,7 +1263,24 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                         VF[4 * v] = t.x; VF[4 * v + 1] = t.y; VF[4 * v + 2] = t.z; VF[4 * v + 3] = t.w;
                     }
                 }
-                const uint8_t *p_zt = tile + (ROW_ZT + copy) * DT_STRIDE + ZT_STRIDE * (g & 3) + 4 * j;
+                // zero-points: z[m] = tokens 8m + 2j, + 1 of row g
+                uint32_t z[4];
+                if constexpr (H > 1) {
+                    ldsm_x4_trans(smem_u32(gb + o_vz + (lane * H + (h & ~1)) * 8), z[0], z[1], z[2], z[3]);
+                } else {
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const uint16_t *vz = reinterpret_cast<const uint16_t *>(gb + o_vz + (8 * m + 2 * j) * 8) + (g & 3);
+                        z[m] = g < 4 ? (uint32_t)vz[0] | ((uint32_t)vz[4] << 16) : 0u;
+                    }
+                }
+                if (tok_base + 32 > pc.ntok) {                                     // what no token of this sequence wrote may be anything
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        if (8 * m + 2 * j + tok_base >= pc.ntok) z[m] = 0u;
+                        else if (8 * m + 2 * j + 1 + tok_base >= pc.ntok) z[m] &= 0xFFFFu;
+                    }
+                }
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
                     uint32_t vc[4];                                  // by scale group: channels 32cg + 4g .. + 3 of four tokens, a byte each
@@ -1237,12 +1294,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                             mma_f16(acc[2 * cg + u], w01 & (0x00030003u << (2 * u)), w01 & (0x00030003u << (2 * u + 4)),
                                     w89 & (0x00030003u << (2 * u)), w89 & (0x00030003u << (2 * u + 4)), pb0, pb1);
                     }
-                    uint32_t za0 = 0u, za2 = 0u;
-                    if (g < 4) {
-                        za0 = *reinterpret_cast<const uint32_t *>(p_zt + 32 * ks);
-                        za2 = *reinterpret_cast<const uint32_t *>(p_zt + 32 * ks + 16);
-                    }
-                    mma_f16(accz, za0, 0u, za2, 0u, T[ks][0], T[ks][1]);
+                    const uint32_t z0 = z[2 * ks], z1 = z[2 * ks + 1];
+                    mma_f16(accz, pack_f16x2_sat(bf16_bits_to_f32(z0), __uint_as_float(z0 & 0xFFFF0000u)), 0u,
+                            pack_f16x2_sat(bf16_bits_to_f32(z1), __uint_as_float(z1 & 0xFFFF0000u)), 0u, T[ks][0], T[ks][1]);
                 }
             }
         } else {
@@ -1275,8 +1329,8 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     float outv[2][16];
 #pragma unroll
     for (int cg = 0; cg < 4; ++cg) {
-        const float bz0 = __shfl_sync(0xFFFFFFFFu, accz[0], 4 * cg + j);
-        const float bz1 = __shfl_sync(0xFFFFFFFFu, accz[1], 4 * cg + j);
+        const float bz0 = __shfl_sync(0xFFFFFFFFu, accz[0], 4 * (zr + cg) + j);
+        const float bz1 = __shfl_sync(0xFFFFFFFFu, accz[1], 4 * (zr + cg) + j);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int u = c & 1, v = c >> 1;
@@ -1324,7 +1378,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 for (int cg = 0; cg < 4; ++cg)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) dst[32 * cg + 4 * g + c] = outv[hh][4 * cg + c] * inv;
-                if (g == 0) dst[HD] = l_tot[hh] > 0.f ? m_run[hh] + logf(l_tot[hh]) : -INFINITY;
+                if (g == 0) dst[HD] = l_tot[hh] > 0.f ? m_run[hh] + LAG + logf(l_tot[hh]) : -INFINITY;
             }
         }
     }

@@ -368,3 +368,44 @@ def test_bounded_waits_give_up_and_the_device_stays_usable(monkeypatch):
     assert int(status.item()) == 0
     want_o, want_lse = case.oracle_kernel_arith(num_kv_splits=4, split_pv=True)
     check_close(o2, want_o, ctx="after a timed-out call")
+
+
+@pytest.mark.parametrize("H,Hq", [(8, 32), (4, 16), (2, 8), (1, 8)])
+@pytest.mark.parametrize("left", [1, 17, 31])
+def test_decode_sequence_ends_inside_a_group(H, Hq, left):
+    """A last group of `left` tokens: what the planes hold past it (here NaN zero-points and the largest exponents) takes no part."""
+    case = Case([1000], H=H, Hq=Hq, seed=left, permute=False)
+    rec, seq = case.per_seq[0], case.packed[0] - 32 + left
+    case.b_seq_len[0] = seq
+    case.planes["v_zp"].view(-1, H, 4)[seq:case.packed[0]] = float("nan")
+    case.planes["v_scale"].view(-1, H, 4)[seq:case.packed[0]] = 127
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    groups = np.arange(case.packed[0] // 32)
+    tail = rec["tail_idx"]
+    want_o, want_lse, _ = O.decode_split_kv(case.q[0].float().numpy(), rec["planes"], rec["K"][tail].numpy(), rec["V"][tail].numpy(),
+                                            case.sm_scale, 1, seq=seq, req_to_group=groups, split_pv=True)
+    for splits in (1, 5):
+        o, lse = case.run(num_kv_splits=splits, status=status)
+        check_close(o[0], want_o, ctx=f"H={H} left={left} S={splits}")
+        np.testing.assert_allclose(lse[0].cpu().numpy(), want_lse, atol=2e-2, rtol=0)
+    assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("slope", [-3.0, 0.05, 1.9, 2.1, 9.0])
+def test_decode_logits_that_rise_from_group_to_group(slope, monkeypatch):
+    """The first head of every kv head meets logits that rise (or fall) by `slope` a group, around the distance at which the
+    running maximum follows; the others meet slopes of either sign."""
+    import helpers
+    seq, H, Hq, D, seed = 840, 4, 16, 128, 9
+    q = torch.randn(1, Hq, D, generator=torch.Generator().manual_seed(seed + 7)).bfloat16().float()[0, ::Hq // H]
+    step = slope / 32 * q / (q.pow(2).sum(-1, keepdim=True) * D ** -0.5)
+    plain = helpers.gaussian_kv
+
+    def rising(*a, **kw):
+        K, V = plain(*a, **kw)
+        return (K + torch.arange(K.shape[0])[:, None, None] * step).bfloat16().float(), V
+
+    monkeypatch.setattr(helpers, "gaussian_kv", rising)
+    case = Case([seq], H=H, Hq=Hq, seed=seed, mag=1.0)
+    for splits in (1, 3):
+        _run_and_check(case, num_kv_splits=splits, lse_atol_fp32=0.5)
