@@ -224,7 +224,7 @@ constexpr long long TEST_WAIT_LIMIT_CYCLES = 4000000ll;
 constexpr int FBIAS = 4;
 constexpr int KF_BIAS = 70;
 constexpr int E_TOP = 11 + 128;
-constexpr float LAG = 2.f;              // how far a logit may be ahead of the maximum that P is taken against (natural log)
+constexpr float LAG = 0.68f;            // how far a logit may be ahead of the maximum that P is taken against: e^LAG * 2^(11 + FBIAS) < 65504
 constexpr float KF_UNDO = 9223372036854775808.f;      // 2^(133 - KF_BIAS): a code field in place is code * 4^slot * 2^-133
 __host__ __device__ constexpr uint32_t half2_const(int lo, int hi) { return ((uint32_t)lo & 0xFFFFu) | ((uint32_t)hi << 16); }
 // the FP4 levels of four outliers (16 bits of the nibble stream) as the upper bytes of their fp16 values; the lower
@@ -1211,7 +1211,8 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                         if (tok_base + 16 * mt + g + 8 * (r >> 1) >= pc.ntok) x[mt][r] = -INFINITY;
             }
             // The reference maximum follows only when a logit is more than LAG ahead of it, so that most units need neither the
-            // maximum over the lanes nor a rescaled accumulator; P is kept below 2^0 by the same distance.
+            // maximum over the lanes nor a rescaled accumulator.  P may then be up to e^LAG, which the largest V factor just allows;
+            // against a maximum LAG further up, small P would lose bits (errors against 64-bit attention 2 to 4 % larger).
             bool ahead = false;
             float mloc[2];
 #pragma unroll
@@ -1235,7 +1236,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     accz[hh] *= corr;
                 }
             }
-            const float mneg[2] = {m_run[0] == -INFINITY ? 0.f : -(m_run[0] + LAG) * LOG2E, m_run[1] == -INFINITY ? 0.f : -(m_run[1] + LAG) * LOG2E};
+            const float mneg[2] = {m_run[0] == -INFINITY ? 0.f : -m_run[0] * LOG2E, m_run[1] == -INFINITY ? 0.f : -m_run[1] * LOG2E};
             float pr[2][4];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt)
@@ -1378,7 +1379,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 for (int cg = 0; cg < 4; ++cg)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) dst[32 * cg + 4 * g + c] = outv[hh][4 * cg + c] * inv;
-                if (g == 0) dst[HD] = l_tot[hh] > 0.f ? m_run[hh] + LAG + logf(l_tot[hh]) : -INFINITY;
+                if (g == 0) dst[HD] = l_tot[hh] > 0.f ? m_run[hh] + logf(l_tot[hh]) : -INFINITY;
             }
         }
     }
