@@ -127,7 +127,7 @@ int ommx_b200_outlier_index_convert(const void *src, void *dst, int64_t frames, 
  * f32 [batch, n_q_heads, num_kv_splits+1, head_dim+1] (lane head_dim = log-sum-exp).
  * b_seq_len holds PACKED token counts.  num_kv_splits is the number of workspace slots of a sequence: its 32-token groups are
  * worked on in at most that many pieces.  Where they are cut follows from all lengths of the batch, on the device, so that the
- * CTAs have even shares (ommx_b200_host_share_plan); the reference cuts every sequence into num_kv_splits equal ones.
+ * CTAs have even shares (ommx_b200_host_share_plan); where there are few slots, several CTAs work on a piece.  The reference cuts every sequence into num_kv_splits equal ones.
  */
 /*
  * Head-output exchange fused into stage 2, for kv heads sharded over the GPUs of one node (the split vLLM
@@ -321,9 +321,9 @@ int ommx_b200_host_pow2_exponent(float x);
 int ommx_b200_host_fp4_encode(float m);
 
 /* Host-side twin of the plan by which both decode stages share the packed groups of a batch out over CTAs (no GPU needed;
- * b_seq_len is host memory here).  *ctas: CTAs of the stage-1 launch; *groups_per_cta: consecutive groups of the running list
- * each of them takes, 0 = equal splits per sequence, dealt out one by one.  Returns how many pieces of sequences a CTA can
- * list, which no plan exceeds, or a negative code. */
+ * b_seq_len is host memory here).  *ctas: shares of the stage-1 launch, each the work of one CTA or of one cluster of CTAs where
+ * there are few slots; *groups_per_cta: consecutive groups of the running list in a share, 0 = equal splits per sequence, dealt
+ * out to the shares one by one.  Returns how many pieces of sequences a CTA can list, which no plan exceeds, or a negative code. */
 int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len,
                               int32_t sm_count, int32_t *ctas, int32_t *groups_per_cta);
 

@@ -43,7 +43,8 @@ struct S2Params {
     int32_t max_tail, v_vec_ok;          // v_vec_ok: four adjacent V elements may be fetched as one 8-byte word
     const float *al;
     int64_t al_sb, al_sh, al_ss;
-    int32_t S, B, ncta, waves;           // ncta: CTAs stage 1 shared the groups over (0: equal splits per sequence)
+    int32_t S, B;
+    Stage1Grid grid;                     // stage 1's launch; ncta = 0: equal splits per sequence
     void *o;
     int32_t o_bf16;
     int64_t o_sb, o_sh;
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     const int groups = groups_of(seq);
     int nsplit = 0;
     if (p.S > 0 && groups > 0) {
-        const int per = p.ncta > 0 ? share_plan_of(total, longest, p.B, p.S, p.ncta, p.waves).per : 0;
+        const int per = p.grid.ncta > 0 ? share_plan_of(total, longest, p.B, p.S, p.grid).per : 0;
         if (per == 0) {
             const int equal = (groups + p.S - 1) / p.S;
             nsplit = (groups + equal - 1) / equal;
@@ -475,10 +476,10 @@ static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes,
 
 static size_t stage1_smem(const S1Params &p) { return stage1_smem(p.nstages, p.stage_bytes, p.GS, p.ppg); }
 
-static int stage1_ctas(const ommx_decode_args *a, int *ncta, int *waves) {
+static int stage1_launch(const ommx_decode_args *a, Stage1Grid *grid) {
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
-    stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, sm_count_of(dev), ncta, waves);
+    *grid = stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, sm_count_of(dev));
     return 0;
 }
 
@@ -552,16 +553,16 @@ static int fill_stage1(const ommx_decode_args *a, S1Params &p) {
     return 0;
 }
 
-// CTAs that stage 1 shares the groups over, 0 where it makes equal splits per sequence (the tensor-core kernel): stage 2
-// works out the same workspace slots from it
-static int shared_ctas(const ommx_decode_args *a, bool tc, int *ncta, int *waves) {
+// Stage 1's launch, without CTAs where it makes equal splits per sequence (the tensor-core kernel): stage 2 works out the same
+// workspace slots from it
+static int shared_grid(const ommx_decode_args *a, bool tc, Stage1Grid *grid) {
     if (tc) {
         S1Params p;
         TcParams T;
         if (int rc = fill_stage1(a, p)) return rc;
-        if (tensor_core_plan(a, p, &T)) { *ncta = 0; return 0; }
+        if (tensor_core_plan(a, p, &T)) { *grid = Stage1Grid{0, 0, 1, 0}; return 0; }
     }
-    return stage1_ctas(a, ncta, waves);
+    return stage1_launch(a, grid);
 }
 
 static int launch_stage1(const ommx_decode_args *a, cudaStream_t st, bool tc) {
@@ -581,7 +582,7 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st, bool tc) {
     while (p.nstages > 2 && stage1_smem(p) > SMEM_LIMIT) --p.nstages;
     const size_t smem = stage1_smem(p);
     if (smem > SMEM_LIMIT) return fail(OMMX_E_UNSUPPORTED, "stage 1 planes of one group do not fit shared memory");
-    if (int rc = stage1_ctas(a, &p.ncta, &p.waves)) return rc;
+    if (int rc = stage1_launch(a, &p.grid)) return rc;
     switch (p.H) {
         case 8: return launch_stage1_h8(p, smem, st);
         case 4: return launch_stage1_h4(p, smem, st);
@@ -604,9 +605,9 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
     p.v_vec_ok = (((uintptr_t)a->v_tail & 7) == 0 && a->tail_stride_b % 4 == 0 && a->tail_stride_t % 4 == 0 && a->tail_stride_h % 4 == 0) ? 1 : 0;
     p.al = a->attn_logits; p.al_sb = a->al_stride_b; p.al_sh = a->al_stride_h; p.al_ss = a->al_stride_s;
     p.S = a->max_seq_len > 0 ? a->num_kv_splits : 0;
-    p.B = a->batch; p.ncta = p.waves = 0;
+    p.B = a->batch; p.grid = Stage1Grid{0, 0, 1, 0};
     if (p.S > 0)
-        if (int rc = shared_ctas(a, tc, &p.ncta, &p.waves)) return rc;
+        if (int rc = shared_grid(a, tc, &p.grid)) return rc;
     p.o = a->o; p.o_bf16 = (a->o_dtype == OMMX_DT_BF16); p.o_sb = a->o_stride_b; p.o_sh = a->o_stride_h;
     p.lse = a->lse; p.lse_sb = a->lse_stride_b;
     p.sm_scale = a->sm_scale; p.logit_cap = a->logit_cap;
@@ -692,13 +693,15 @@ extern "C" int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch
     using namespace ommx;
     if (!b_seq_len || !ctas || !groups_per_cta || batch < 1 || num_kv_splits < 1 || sm_count < 1)
         return fail(OMMX_E_ARG, "host_share_plan: batch=%d num_kv_splits=%d sm_count=%d", batch, num_kv_splits, sm_count);
-    int total = 0, longest = 0, waves = 0;
+    int total = 0, longest = 0;
     for (int i = 0; i < batch; ++i) {
         total += groups_of(b_seq_len[i]);
         longest = max(longest, groups_of(b_seq_len[i]));
     }
-    stage1_grid(batch, num_kv_splits, max_seq_len, sm_count, ctas, &waves);
-    *groups_per_cta = share_plan_of(total, longest, batch, num_kv_splits, *ctas, waves).per;
+    const Stage1Grid grid = stage1_grid(batch, num_kv_splits, max_seq_len, sm_count);
+    const SharePlan plan = share_plan_of(total, longest, batch, num_kv_splits, grid);
+    *ctas = plan.shares;
+    *groups_per_cta = plan.per;
     return MAX_PIECES;
 }
 

@@ -41,6 +41,9 @@ constexpr int MAX_SPLIT_PAGES = 1024;
 constexpr int MAX_PIECES = 128;         // pieces of sequences one CTA can work on (32 bytes of shared memory each)
 constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;   // about a second of SM clock: the wait has failed
 
+// The launch: CTAs (one per SM at most) in clusters of `cluster`; rounds of CTAs (clusters) that B * S splits would take
+struct Stage1Grid { int32_t ncta, waves, cluster, cluster_waves; };
+
 struct S1Params {
     const __nv_bfloat16 *q;
     int64_t q_sb, q_sh;
@@ -56,7 +59,7 @@ struct S1Params {
     float *al;
     int64_t al_sb, al_sh, al_ss;
     int32_t S, seg_group_base;
-    int32_t ncta, waves;                 // CTAs of the launch (one per SM at most), rounds of them that B * S splits would take
+    Stage1Grid grid;
     float sm_scale, logit_cap;
     int32_t *status;
     int32_t abl;
@@ -112,6 +115,36 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
         }
     }
     return true;
+}
+// ---- between the CTAs of a cluster: the address of a peer's shared memory, a release-arrive there, an acquire-wait here, a load ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t peer_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer_bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_peers(uint32_t bar, uint32_t parity, long long limit) {
+    const long long t_end = clock64() + limit;
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if (clock64() > t_end) return false;
+    }
+}
+__device__ __forceinline__ float lds_peer(uint32_t peer_addr) {
+    float x;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(peer_addr) : "memory");
+    return x;
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -309,13 +342,24 @@ __host__ __device__ constexpr PositionBits past_31_bits(int k, int bytes) {
 //     costs every batch: one more reduction ahead of the stages made the long cases 3 to 4 % slower.
 // Where pieces begin depends on the plan, and with it the running maximum against which P is rounded to fp16: another split
 // count or batch moves a result by about 5e-5 of its norm, the same call repeats its bits.
+//
+// Where S bounds the shares from below and leaves CTAs without one - few sequences in splits of 512 tokens, or a ragged batch at the
+// automatic count - a share (or split) is worked on by a whole cluster of CTAs: each piece is dealt out evenly to them, and for every
+// kv head one of them merges the others' softmax states through their shared memory before the one result goes to the piece's slot.
+// It is taken where the groups per CTA, the merge counted as one more, get fewer.  Measured, 8 kv heads, without / with the size taken
+// (2, 4, 8): 4K in 8 slots 42.2 / 18.5 us (28.6, 20.6, 18.1); 16K in 32 42.6 / 23.6 (28.9, 22.8, 24.8); 8 sequences of 700..2048 in 4
+// 43.1 / 25.0 (31.1, 24.1, 33.1); 4 of 4K..8K in 16 43.0 / 32.3 (31.5, 33.3, 37.5).  In brackets before the barrier that holds
+// a cluster's CTAs until all have read (0.4..0.9 us).
 struct SharePlan {
-    int per, total;                      // groups per CTA (0: equal splits per sequence), groups of all sequences
+    int per, total;                      // groups per share (0: equal splits per sequence), groups of all sequences
+    int ctas, shares;                    // CTAs to a share, shares
 };
 __host__ __device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
 __host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, int ncta, int waves) {
     SharePlan s;
     s.total = total;
+    s.ctas = 1;
+    s.shares = ncta;
     s.per = max(1, (total + ncta - 1) / ncta);
     const int equal = (longest + S - 1) / S;
     if (B == 1) {
@@ -326,16 +370,45 @@ __host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longe
     }
     return s;
 }
+__host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, const Stage1Grid &g) {
+    SharePlan a = share_plan_of(total, longest, B, S, g.ncta, g.waves);
+    if (g.cluster > 1) {
+        const int equal = (longest + S - 1) / S;
+        SharePlan c = share_plan_of(total, longest, B, S, g.ncta / g.cluster, g.cluster_waves);
+        c.ctas = g.cluster;
+        const int of_a = a.per > 0 ? a.per : g.waves * equal, of_c = c.per > 0 ? c.per : g.cluster_waves * equal;
+        if ((c.per > 0 || g.cluster_waves <= MAX_PIECES) && (of_c + g.cluster - 1) / g.cluster + 1 < of_a) return c;
+    }
+    return a;
+}
 // CTAs of a launch - one per SM, or one per group where there are fewer; above MAX_PIECES sequences at least one for every MAX_PIECES
 // groups or splits - and the rounds of them that equal splits would take (capped: past the cap they are never the choice)
-static inline void stage1_grid(int batch, int S, int max_seq_len, int sm_count, int *ncta, int *waves) {
-    const long long groups = (long long)batch * groups_of(max_seq_len), splits = (long long)batch * S;
+static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, int sm_count) {
+    const long long longest = groups_of(max_seq_len), groups = batch * longest, splits = (long long)batch * S;
     const long long least = batch > MAX_PIECES ? (max(groups, splits) + MAX_PIECES - 1) / MAX_PIECES : 1;
-    *ncta = (int)max(min((long long)sm_count, max(groups, 1ll)), least);
-    *waves = (int)min((splits + *ncta - 1) / *ncta, 1024ll);
+    Stage1Grid g;
+    g.ncta = (int)max(min((long long)sm_count, max(groups, 1ll)), least);
+    g.cluster = 1;
+    // The cluster size that leaves the fewest groups per CTA if all sequences are of the longest's length; share_plan_of then decides by
+    // the lengths.  Clusters of two fill the chip (74 at once on 148 SMs); of four 33 run at once, of eight 15.  A launch that cannot
+    // gain at equal lengths keeps the form without clusters: the exchange's code alone costs 4.5 % (8 x 32K: 133.9 -> 140.0 us), although
+    // a ragged batch would win by more (8 sequences of 4K..32K in 18 slots each: 133.5 -> 103.4).
+    if (batch <= MAX_PIECES && S > (batch > 1 ? 1 : 0) && sm_count >= 128) {     // counted on the whole chip only
+        const long long bound = batch == 1 ? (longest + S - 1) / S : (longest - 2) / (S - 1) + 1;
+        long long best = min(max((groups + sm_count - 1) / sm_count, bound), (splits + sm_count - 1) / sm_count * ((longest + S - 1) / S));
+        for (int c = 2; c <= 8; c *= 2) {
+            const long long at_once = c == 2 ? sm_count / 2 : (c == 4 ? sm_count * 2 / 9 : sm_count / 10), shares = max(1ll, min(at_once, groups));
+            const long long cost = (min(max((groups + shares - 1) / shares, bound), (splits + shares - 1) / shares * ((longest + S - 1) / S)) + c - 1) / c + 1;
+            if (cost < best) { best = cost; g.cluster = c; g.ncta = (int)shares * c; }
+        }
+    }
+    g.waves = (int)min((splits + g.ncta - 1) / g.ncta, 1024ll);
+    const int shares = g.ncta / g.cluster;
+    g.cluster_waves = (int)min((splits + shares - 1) / shares, 1024ll);
+    return g;
 }
 // called by whole warps; every lane gets the same answer
-__device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, int ncta, int waves, int lane) {
+template <bool CLUSTER> __device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, const Stage1Grid &g, int lane) {
     int n = 0, mx = 0;
     if (B == 1) {
         n = mx = groups_of(b_seq_len[0]);
@@ -348,7 +421,8 @@ __device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B,
         n = __reduce_add_sync(0xFFFFFFFFu, n);
         mx = __reduce_max_sync(0xFFFFFFFFu, mx);
     }
-    return share_plan_of(n, mx, B, S, ncta, waves);
+    if constexpr (CLUSTER) return share_plan_of(n, mx, B, S, g);
+    else return share_plan_of(n, mx, B, S, g.ncta, g.waves);
 }
 
 // One piece of work of a CTA: consecutive groups of one sequence.  `it` counts the CTA's ring stages across its pieces, so that
@@ -359,7 +433,7 @@ struct alignas(16) Piece {
     int ntok, it0, it1, more;            // tokens, ring iterations [it0, it1), whether another piece follows
 };
 struct PieceWalk {
-    int pos, end;                        // running list: first group of the piece, end of this CTA's share; splits: item, items
+    int pos, end, step;                  // running list: first group of the piece, end of this CTA's share; splits: item, items, items between two
 };
 template <int GS>
 __device__ __forceinline__ void piece_range(Piece &c, int seq, int g0, int ng) {
@@ -370,7 +444,7 @@ __device__ __forceinline__ void piece_range(Piece &c, int seq, int g0, int ng) {
 }
 // equal splits: the first item at or after w.pos that has groups
 template <int GS> __device__ __forceinline__ bool piece_of_splits(Piece &c, PieceWalk &w, const S1Params &p) {
-    for (; w.pos < w.end; w.pos += p.ncta) {
+    for (; w.pos < w.end; w.pos += w.step) {
         c.b = w.pos / p.S;
         c.slot = w.pos - c.b * p.S;
         const int seq = p.b_seq_len[c.b], n = groups_of(seq), per = (n + p.S - 1) / p.S, g0 = c.slot * per;
@@ -382,10 +456,11 @@ template <int GS> __device__ __forceinline__ bool piece_of_splits(Piece &c, Piec
     return false;
 }
 template <int GS> __device__ __forceinline__ bool first_piece(Piece &c, PieceWalk &w, const S1Params &p, const SharePlan &plan, int cta, int lane) {
-    c.it0 = 0;
+    c.it0 = 0;                                                 // cta: the share
     if (plan.per == 0) {
         w.pos = cta;
         w.end = p.B * p.S;
+        w.step = plan.shares;
         return piece_of_splits<GS>(c, w, p);
     }
     w.pos = cta * plan.per;
@@ -426,7 +501,7 @@ template <int GS> __device__ __forceinline__ bool first_piece(Piece &c, PieceWal
 template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk &w, const S1Params &p, const SharePlan &plan) {
     c.it0 = c.it1;
     if (plan.per == 0) {
-        w.pos += p.ncta;
+        w.pos += w.step;
         return piece_of_splits<GS>(c, w, p);
     }
     w.pos += c.ng;
@@ -440,9 +515,24 @@ template <int GS> __device__ __forceinline__ bool next_piece(Piece &c, PieceWalk
     return true;
 }
 
+// The part of a piece that CTA `rank` of the `n` that share it works on, its ring iterations from `it0` on; there may be nothing in it.
+// Which CTA gets the odd groups turns with the piece.
+template <int GS> __device__ __forceinline__ Piece part_of(const Piece &c, int rank, int n, int it0) {
+    Piece q = c;
+    if (n > 1) {
+        const int r = (rank + c.b + c.slot) % n, lo = c.ng * r / n;
+        q.g0 = c.g0 + lo;
+        q.ng = c.ng * (r + 1) / n - lo;
+        q.ntok = min(c.ntok - 32 * lo, 32 * q.ng);
+    }
+    q.it0 = it0;
+    q.it1 = it0 + (q.ng + GS - 1) / GS;
+    return q;
+}
+
 constexpr size_t SMEM_LIMIT = 232448;   // what a CTA may ask for
 constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_per_group) {       // last line: copy roles, their table entries, pieces
-    return 1024 + (size_t)stages * stage_bytes + (size_t)NCW * DT_BYTES + 64 + (2 * MAX_STAGES + (2 + MAX_STAGES) * NCW) * 8
+    return 1024 + (size_t)stages * stage_bytes + (size_t)NCW * DT_BYTES + 64 + (2 * MAX_STAGES + (2 + MAX_STAGES) * NCW + 3 * NCW) * 8
            + (size_t)groups * (4 * pages_per_group + 6) * (sizeof(CopyDesc) + 4) + MAX_PIECES * sizeof(Piece);
 }
 // KOUT: outliers per K vector known at compile time (static, unrolled splice) or -1 (runtime).
@@ -488,7 +578,7 @@ template <int KOUT, int H, bool IDX7> struct PlainLayout {
     static constexpr int STAGES = stage1_smem(4, NCW / H * GB, NCW / H, 2) <= SMEM_LIMIT ? 4 : 3;   // with 16-token pages
     static_assert(stage1_smem(STAGES, NCW / H * GB, NCW / H, 2) <= SMEM_LIMIT, "the ring fits");
 };
-template <int KOUT, int H, bool PLAIN, bool IDX7>
+template <int KOUT, int H, bool PLAIN, bool IDX7, bool CLUSTER>
 __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kernel(const __grid_constant__ S1Params p) {
     constexpr bool WIDE = WarpLayout<H>::WIDE;
     constexpr int NDW = WarpLayout<H>::NDW, NPW = WarpLayout<H>::NPW, PRODUCER_WARP = WarpLayout<H>::PRODUCER_WARP;
@@ -518,10 +608,13 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     uint8_t *s_tiles = s_stage + NS * stage_bytes;                    // NCW * DT_BYTES
     float *s_lut = reinterpret_cast<float *>(s_tiles + NCW * DT_BYTES);
     uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_lut + 16);         // full[], empty[], tile_full[NCW], tile_empty[NCW][], tile_rows[NCW]
-    CopyDesc *s_desc = reinterpret_cast<CopyDesc *>(s_bar + 2 * MAX_STAGES + (2 + MAX_STAGES) * NCW);
+    CopyDesc *s_desc = reinterpret_cast<CopyDesc *>(s_bar + 2 * MAX_STAGES + (5 + MAX_STAGES) * NCW);
     const uint32_t bar_full = smem_u32(s_bar), bar_empty = smem_u32(s_bar + MAX_STAGES);
     const uint32_t bar_tfull = smem_u32(s_bar + 2 * MAX_STAGES), bar_tempty = smem_u32(s_bar + 2 * MAX_STAGES + NCW);
     const uint32_t bar_trows = smem_u32(s_bar + 2 * MAX_STAGES + (1 + MAX_STAGES) * NCW);
+    // states of a head: handed in by the cluster's other CTAs, taken from this one; whether there is one (8 bytes a head)
+    const uint32_t bar_handed = bar_trows + 8 * NCW, bar_taken = bar_handed + 8 * NCW, s_there = bar_taken + 8 * NCW;
+    volatile int *s_ctas = reinterpret_cast<int *>(s_bar + 2 * MAX_STAGES + (4 + MAX_STAGES) * NCW) + 1;   // CTAs to a share (the odd word of s_there[0])
 
     // ---- prologue: LUT, barriers and copy descriptors.  None of it depends on an earlier kernel, so it runs while the
     //      kernel before this one in the stream drains (the grid may start then, see the wait below). ----
@@ -537,16 +630,18 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         s_lut[c] = (c & 8) ? -mag : mag;
     }
     {
-        // one barrier per thread (56 of them: a single thread's serial inits were a microsecond of every launch)
+        // one barrier per thread (72 of them: a single thread's serial inits were a microsecond of every launch)
         const int t = (int)threadIdx.x - 32;
-        constexpr int NB_RING = 2 * MAX_STAGES, NB_ALL = NB_RING + (2 + MAX_STAGES) * NCW;
+        constexpr int NB_RING = 2 * MAX_STAGES, NB_TILE = NB_RING + (2 + MAX_STAGES) * NCW, NB_ALL = NB_TILE + (CLUSTER ? 2 * NCW : 0);
         if (t >= 0 && t < NB_ALL) {
             uint32_t count;
             if (t < MAX_STAGES) count = NPW;                                   // full[]: each producer warp announces its own copies
             else if (t < NB_RING) count = 3 * NCW;                             // empty[]: 8 MMA warps + 16 tile halves
             else if (t < NB_RING + NCW) count = 2;                             // tile_full[]: the two halves' deltas scattered
             else if (t < NB_RING + NCW + MAX_STAGES * NCW) count = 1;          // tile_empty[][]
-            else count = 2;                                                    // tile_rows[]: the two halves' rows written
+            else if (t < NB_TILE) count = 2;                                   // tile_rows[]: the two halves' rows written
+            else if (t < NB_TILE + NCW) count = max(p.grid.cluster - 1, 1);    // handed[]: by every other CTA of the cluster
+            else count = 1;                                                    // taken[]
             mbar_init(bar_full + 8 * t, count);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -589,6 +684,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         }
     }
     __syncthreads();
+    if constexpr (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");         // this CTA's barriers are ready
     // Nothing an earlier kernel may have written - lengths, tables, the query, the planes, the split workspace a
     // previous layer's combine still reads - is touched before this returns.
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -599,8 +695,12 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
 
     Piece pc;
     PieceWalk walk;
-    const SharePlan plan = share_plan(p.b_seq_len, p.B, p.S, p.ncta, p.waves, lane);
-    if (!first_piece<GS>(pc, walk, p, plan, cta, lane)) return;
+    const SharePlan plan = share_plan<CLUSTER>(p.b_seq_len, p.B, p.S, p.grid, lane);
+    if (!first_piece<GS>(pc, walk, p, plan, CLUSTER ? cta / plan.ctas : cta, lane)) return;
+    auto my_part = [&](const Piece &c, int it0) __attribute__((always_inline)) {
+        if constexpr (CLUSTER) return part_of<GS>(c, cluster_rank(), plan.ctas, it0);
+        else return c;
+    };
 
     const int g = lane >> 2, j = lane & 3;
     const float LOG2E = 1.4426950408889634f;
@@ -665,16 +765,26 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     // decode warps of the producer's warpgroup (idle until the data lands) take a quarter of the first fill each.
     if (warp >= PRODUCER_WARP - (WIDE ? 0 : 3)) {
         constexpr int W0 = PRODUCER_WARP - (WIDE ? 0 : 3);
-        lookup_stage(pc, 0, 4, warp - W0);
-        const uint32_t bytes = WIDE ? stage_bytes_of(pc, 0, false, lane * NPW + warp - W0, 32 * NPW)
-                                    : (warp == PRODUCER_WARP ? stage_bytes_of(pc, 0, false, lane, 32) : 0u);
-        issue_stage(pc, 0, 4, warp - W0, bytes);
+        Piece q = my_part(pc, 0);
+        if (CLUSTER && q.ng == 0) {                                             // this CTA begins with a later piece, if any
+            Piece c = pc;
+            PieceWalk w = walk;
+            while (q.ng == 0 && next_piece<GS>(c, w, p, plan)) q = my_part(c, 0);
+        }
+        if (!CLUSTER || q.ng > 0) {
+            lookup_stage(q, 0, 4, warp - W0);
+            const uint32_t bytes = WIDE ? stage_bytes_of(q, 0, false, lane * NPW + warp - W0, 32 * NPW)
+                                        : (warp == PRODUCER_WARP ? stage_bytes_of(q, 0, false, lane, 32) : 0u);
+            issue_stage(q, 0, 4, warp - W0, bytes);
+        }
     }
 
     if (warp == PRODUCER_WARP) {
-        int n = 0;
+        if (CLUSTER && lane == 0) *s_ctas = plan.ctas;
+        int n = 0, at = 0;
         for (bool more = true; more; ++n) {
-            Piece cur = pc;
+            Piece cur = my_part(pc, at);
+            at = cur.it1;
             more = next_piece<GS>(pc, walk, p, plan);
             if (more && n + 1 == MAX_PIECES) {                       // a bounds check: share_plan_of rules it out
                 if (lane == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
@@ -685,6 +795,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         }
     }
     __syncthreads();
+    if constexpr (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     int pi = 0;
     pc = s_piece[0];
     auto step_piece = [&]() __attribute__((always_inline)) {
@@ -997,7 +1108,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const int pw = warp - PRODUCER_WARP;
         const uint32_t full_bytes = stage_bytes_of(pc, 0, true, lane * NPW + pw, 32 * NPW);   // this warp's share of a stage of whole groups
         for (int it = 1;; ++it) {
-            if (it >= pc.it1 && !step_piece()) break;
+            bool more = true;
+            while (it >= pc.it1 && (more = step_piece())) {}            // a shared piece may hold nothing for this CTA
+            if (!more) break;
             lookup_stage(pc, it, NPW, pw);
             const uint32_t bytes = whole_stage(pc, it) ? full_bytes : stage_bytes_of(pc, it, false, lane * NPW + pw, 32 * NPW);
             // the first NS fills find their slots fresh
@@ -1032,7 +1145,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             if constexpr (!WIDE) asm volatile("bar.arrive 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
         } else {
             asm volatile("bar.sync 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
-            if (!producer_alive || pc.more) return;
+            if (!producer_alive || pc.more || (CLUSTER && pc.it0 == pc.it1)) return;
         }
         // the producer takes the very last item, when this CTA's pieces end with one that is known to be the last
         for (int n = is_producer ? pc.it1 * 2 * NCW - 1 : dw;; n += NDW) {
@@ -1068,6 +1181,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     const bool do_k = !(abl & ABL_NO_K), do_v = !(abl & ABL_NO_V);
     const bool has_delta = !(k_out == 0 || no_outlier);
 
+    constexpr bool keep_last = GS > 1 || CLUSTER;                    // a piece's last tile serves to exchange states before it is handed back
     bool gave_up = false;                        // a wait ran out: no more groups, but every piece still goes through its epilogue
     do {
     // B fragments of q, bf16.  QR: raw, registers 4v..4v+3 hold channels 32v + 8j .. + 7 (zero-point MMAs).  QP: q * sm_scale
@@ -1187,7 +1301,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             }
             __syncwarp();
             // the next tile may be built (where warps merge below, they do it in their tiles: not before that)
-            if (lane == 0 && (GS == 1 || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
+            if (lane == 0 && (!keep_last || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
 
             // ======================= online softmax =======================
             // x[mt][r]: token 16mt + g + 8(r>>1), head 2j + (r&1)
@@ -1305,7 +1419,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 gave_up = true;
                 break;
             }
-            if (lane == 0 && (GS == 1 || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
+            if (lane == 0 && (!keep_last || it + 1 < pc.it1)) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(it, NS)));
         }
         // release the stage
         __syncwarp();
@@ -1341,34 +1455,71 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         }
     }
 
-    // Several groups per stage (fewer than 8 local kv heads): the warps that share a head merge, each through the delta rows
-    // of its own tile, which nobody builds again before it is handed back below.  With 8 heads every warp owns its head and
-    // writes straight away.
-    static_assert(32 * 36 * 4 <= 32 * DT_STRIDE, "the merge fits the delta rows of a tile");
-    if (GS > 1) {
-        if (gsel > 0) {
-            float *my = reinterpret_cast<float *>(s_tiles + unit * DT_BYTES) + lane * 36;
-            my[0] = m_run[0]; my[1] = m_run[1]; my[2] = l_tot[0]; my[3] = l_tot[1];
+    // softmax state (m2, l2, un-normalised rows `other(i)`) into this warp's
+    auto merge_state = [&](auto other) __attribute__((always_inline)) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) { my[4 + i] = outv[0][i]; my[20 + i] = outv[1][i]; }
+        for (int hh = 0; hh < 2; ++hh) {
+            const float m2 = other(hh), l2 = other(2 + hh);
+            const float mn = fmaxf(m_run[hh], m2);
+            const float mu = (mn == -INFINITY) ? 0.f : mn;
+            const float c1 = fast_exp2((m_run[hh] - mu) * LOG2E), c2 = fast_exp2((m2 - mu) * LOG2E);
+            l_tot[hh] = l_tot[hh] * c1 + l2 * c2;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) outv[hh][i] = outv[hh][i] * c1 + other(4 + 16 * hh + i) * c2;
+            m_run[hh] = mn;
+        }
+    };
+    auto store_state = [&]() __attribute__((always_inline)) {
+        float *my = reinterpret_cast<float *>(s_tiles + unit * DT_BYTES) + lane;
+        my[0] = m_run[0]; my[32] = m_run[1]; my[64] = l_tot[0]; my[96] = l_tot[1];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { my[32 * (4 + i)] = outv[0][i]; my[32 * (20 + i)] = outv[1][i]; }
+    };
+    // Several groups per stage (fewer than 8 local kv heads): the warps that share a head merge, each through the delta rows
+    // of its own tile, which nobody builds again before it is handed back below.  With 8 heads every warp owns its head.
+    static_assert(32 * 36 * 4 <= 32 * DT_STRIDE, "the merge fits the delta rows of a tile");
+    const bool mine = !CLUSTER || pc.it0 < pc.it1;                   // this CTA had groups of the piece
+    if (GS > 1 && mine) {
+        if (gsel > 0) store_state();
+        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
+        if (gsel == 0) {
+#pragma unroll 1
+            for (int o = 1; o < GS; ++o) {
+                const float *ot = reinterpret_cast<const float *>(s_tiles + (o * H + h) * DT_BYTES) + lane;
+                merge_state([&](int i) { return ot[32 * i]; });
+            }
         }
         asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
     }
-    if (gsel == 0) {
-        for (int o = 1; o < GS; ++o) {
-            const float *ot = reinterpret_cast<const float *>(s_tiles + (o * H + h) * DT_BYTES) + lane * 36;
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const float m2 = ot[hh], l2 = ot[2 + hh];
-                const float mn = fmaxf(m_run[hh], m2);
-                const float mu = (mn == -INFINITY) ? 0.f : mn;
-                const float c1 = fast_exp2((m_run[hh] - mu) * LOG2E), c2 = fast_exp2((m2 - mu) * LOG2E);
-                l_tot[hh] = l_tot[hh] * c1 + l2 * c2;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) outv[hh][i] = outv[hh][i] * c1 + ot[4 + 16 * hh + i] * c2;
-                m_run[hh] = mn;
+    bool write = gsel == 0;
+    if constexpr (CLUSTER)
+    if (gsel == 0 && *s_ctas > 1) {
+        // the CTAs that share the piece: head h is merged by CTA h % n_ctas
+        const int n_ctas = *s_ctas, rank = cluster_rank(), to = h % n_ctas;
+        const uint32_t there = s_there + 8 * h;
+        write = rank == to;
+        if (!write) {
+            if (mine) store_state();
+            if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(there), "r"((uint32_t)mine) : "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_peer(peer_smem(bar_handed + 8 * h, to));
+            if (!mbar_wait_peers(bar_taken + 8 * h, (uint32_t)pi & 1u, wait_limit)) gave_up = true;
+        } else {
+            if (!mbar_wait_peers(bar_handed + 8 * h, (uint32_t)pi & 1u, wait_limit)) gave_up = true;
+            const uint32_t tile_l = smem_u32(tile) + 4 * lane;
+#pragma unroll 1
+            for (int o = 1; o < n_ctas && !gave_up; ++o) {           // not all have stored theirs where the wait gave up
+                const uint32_t from = (rank + o) % n_ctas;
+                if (__float_as_uint(lds_peer(peer_smem(there, from))) == 0u) continue;
+                const uint32_t at = peer_smem(tile_l, from);
+                merge_state([&](int i) { return lds_peer(at + 128 * i); });
             }
+            __syncwarp();
+            if (lane < n_ctas && lane != rank) mbar_arrive_peer(peer_smem(bar_taken + 8 * h, lane));
         }
+        if (gave_up && lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
+    }
+    if (write) {
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             const int head = 2 * j + hh;
@@ -1383,27 +1534,30 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             }
         }
     }
-    if (GS > 1) {
-        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
-        if (lane == 0) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(pc.it1 - 1, NS)));
-    }
+    if (keep_last && mine && lane == 0) mbar_arrive(bar_tempty + 8 * (MAX_STAGES * unit + ring_slot(pc.it1 - 1, NS)));
     } while (step_piece());
+    // no CTA leaves while another of its cluster may still read its tiles or arrive on its barriers; warps that left count as arrived
+    if constexpr (CLUSTER)
+        if (*s_ctas > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Launch as a programmatic dependent of whatever precedes it in the stream: the grid may be placed while that
 // kernel drains, and the kernel itself waits (griddepcontrol.wait) before it reads or writes global memory.
 template <typename Kernel, typename Params>
-static cudaError_t launch_overlapping_previous(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const Params &p) {
+static cudaError_t launch_overlapping_previous(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const Params &p, int cluster = 1) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
@@ -1434,7 +1588,7 @@ template <typename Kernel> static int allow_full_smem(Kernel kernel, std::atomic
     return 0;
 }
 
-template <int KOUT, int H, bool PLAIN, bool IDX7>
+template <int KOUT, int H, bool PLAIN, bool IDX7, bool CLUSTER>
 static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     using L = WarpLayout<H>;
     // function attributes belong to (kernel instantiation, device): one entry per device ordinal
@@ -1445,7 +1599,7 @@ static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     int regs_ok = regs_state[dev].load(std::memory_order_acquire);
     if (regs_ok == 0) {
         cudaFuncAttributes fa;
-        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, H, PLAIN, IDX7>));
+        OMMX_CUDA_TRY(cudaFuncGetAttributes(&fa, decode_stage1_kernel<KOUT, H, PLAIN, IDX7, CLUSTER>));
         // setmaxnreg.inc must find the registers the other roles gave back
         const int need = NCW * 32 * REGS_MMA + (L::WIDE ? L::NDW * 32 * REGS_DECODE + L::NPW * 32 * REGS_PRODUCER
                                                         : (L::THREADS - NCW * 32) * REGS_DECODE);
@@ -1453,8 +1607,8 @@ static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
         regs_state[dev].store(regs_ok, std::memory_order_release);
     }
     if (regs_ok != 1) return fail(OMMX_E_CUDA, "stage 1 was compiled with fewer registers than its warp roles need");
-    if (int rc = allow_full_smem(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>, smem_set, dev)) return rc;
-    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H, PLAIN, IDX7>, dim3(p.ncta), L::THREADS, smem, st, p));
+    if (int rc = allow_full_smem(decode_stage1_kernel<KOUT, H, PLAIN, IDX7, CLUSTER>, smem_set, dev)) return rc;
+    OMMX_CUDA_TRY(launch_overlapping_previous(decode_stage1_kernel<KOUT, H, PLAIN, IDX7, CLUSTER>, dim3(p.grid.ncta), L::THREADS, smem, st, p, p.grid.cluster));
     count_launch();
     return 0;
 }
@@ -1463,12 +1617,12 @@ template <int KOUT, int H>
 static int launch_s1_forms(const S1Params &p, size_t smem, cudaStream_t st) {
     if constexpr (KOUT >= 0) {
         if (p.abl == 0 && (KOUT == 0 || p.use_map) && p.logit_cap <= 0.f) {
-            if (!p.idx7 && p.nstages >= PlainLayout<KOUT, H, false>::STAGES) return launch_s1<KOUT, H, true, false>(p, smem, st);
+            if (!p.idx7 && p.nstages >= PlainLayout<KOUT, H, false>::STAGES) return p.grid.cluster > 1 ? launch_s1<KOUT, H, true, false, true>(p, smem, st) : launch_s1<KOUT, H, true, false, false>(p, smem, st);
             if constexpr (KOUT > 0)
-                if (p.idx7 && p.nstages >= PlainLayout<KOUT, H, true>::STAGES) return launch_s1<KOUT, H, true, true>(p, smem, st);
+                if (p.idx7 && p.nstages >= PlainLayout<KOUT, H, true>::STAGES) return p.grid.cluster > 1 ? launch_s1<KOUT, H, true, true, true>(p, smem, st) : launch_s1<KOUT, H, true, true, false>(p, smem, st);
         }
     }
-    return launch_s1<KOUT, H, false, false>(p, smem, st);
+    return launch_s1<KOUT, H, false, false, true>(p, smem, st);
 }
 // The outlier counts of the serving recipes get the unrolled two-pass splice.
 template <int H>

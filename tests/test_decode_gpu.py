@@ -409,3 +409,24 @@ def test_decode_logits_that_rise_from_group_to_group(slope, monkeypatch):
     case = Case([seq], H=H, Hq=Hq, seed=seed, mag=1.0)
     for splits in (1, 3):
         _run_and_check(case, num_kv_splits=splits, lse_atol_fp32=0.5)
+
+
+@pytest.mark.parametrize("lens,H,splits,k", [
+    ([3960], 8, 8, 6), ([3960], 4, 8, 6), ([3960], 1, 4, 6), ([2000], 2, 2, 4),        # clusters of eight to a split
+    ([3000, 700, 1500, 40, 2048], 8, 4, 6), ([1000, 1000], 1, 2, 8),                   # several sequences, one without groups
+    ([104, 2088], 8, 2, 6), ([72, 72, 1064], 4, 1, 6),                                 # pieces of fewer groups than CTAs
+    ([16000], 8, 32, 2), ([5000, 5000], 2, 10, 6),                                     # clusters of four and two
+    ([9000, 300, 300, 72, 4000, 1000], 8, None, 6), ([6000, 200, 1500], 1, None, 12),  # ragged batches at the automatic count
+    ([3960], 8, 8, 3), ([2000, 500], 4, 2, 0),                                         # the general form; no outliers
+])
+def test_decode_pieces_shared_by_a_cluster(lens, H, splits, k):
+    """Few workspace slots for the CTAs there are: a cluster of CTAs works on a piece and merges its states into one slot."""
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    case = Case(lens, H=H, Hq=4 * H, seed=29, k=k)
+    o, lse = _run_and_check(case, num_kv_splits=splits, status=status)
+    assert int(status.item()) == 0
+    again, lse2 = case.run(num_kv_splits=splits)
+    assert torch.equal(o, again) and torch.equal(lse, lse2)
+    if splits and len(lens) == 1:                                                      # the same groups, a slot to each CTA
+        many, lse2 = case.run(num_kv_splits=148)
+        assert (o - many).abs().max().item() < 2e-3 and (lse - lse2).abs().max().item() < 2e-3
