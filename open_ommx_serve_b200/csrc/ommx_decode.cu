@@ -71,7 +71,8 @@ constexpr int S2_MAX_SPLITS = 1024;
 // costs more than that gains.  What it adds to a layer behind stage 1, against one row to 16 / 8 / 4 warps with a load
 // round for every six residual rows: 32 rows 4.3 -> 3.6 us, 256 rows 6.3 -> 3.9, 512 rows 10.3 -> 5.7, 1024 rows 16.7 -> 9.1,
 // 2048 rows 22.0 -> 11.9.  Spills undo it (80 registers at <8, 3>: 6.2 us for 256 rows).
-template <int NW, int PER_SM>
+// CLUSTER: stage 1 was launched in clusters.  Choosing between its two plans in every launch cost 0.1 us (32 layers at 4K 389 -> 392 us).
+template <int NW, int PER_SM, bool CLUSTER>
 __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2Params p) {
     __shared__ __align__(16) float s_q[HD];
     __shared__ float s_w[NW];
@@ -106,7 +107,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     const int groups = groups_of(seq);
     int nsplit = 0;
     if (p.S > 0 && groups > 0) {
-        const int per = p.grid.ncta > 0 ? share_plan_of(total, longest, p.B, p.S, p.grid).per : 0;
+        int per = 0;
+        if constexpr (CLUSTER) per = share_plan_of(total, longest, p.B, p.S, p.grid).per;
+        else if (p.grid.ncta > 0) per = share_plan_of(total, longest, p.B, p.S, p.grid.ncta, p.grid.waves).per;
         if (per == 0) {
             const int equal = (groups + p.S - 1) / p.S;
             nsplit = (groups + equal - 1) / equal;
@@ -623,7 +626,9 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
     {
         // Stage 1 runs with the largest shared-memory carve-out; asking for the same split here spares the SMs a
         // reconfiguration between the two kernels of every layer.
-        static const Stage2Kernel all[] = {decode_stage2_kernel<16, 1>, decode_stage2_kernel<8, 2>, decode_stage2_kernel<4, 4>, decode_stage2_kernel<4, 7>};
+        static const Stage2Kernel all[] = {decode_stage2_kernel<16, 1, false>, decode_stage2_kernel<8, 2, false>, decode_stage2_kernel<4, 4, false>,
+                                           decode_stage2_kernel<4, 7, false>, decode_stage2_kernel<16, 1, true>, decode_stage2_kernel<8, 2, true>,
+                                           decode_stage2_kernel<4, 4, true>, decode_stage2_kernel<4, 7, true>};
         static std::atomic<int> carve_set[MAX_DEVICES];
         int dev = 0;
         if (int rc = current_device(&dev)) return rc;
@@ -635,7 +640,7 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
         // the largest CTAs of which all rows still run at once
         const long long rows = (long long)a->n_q_heads * a->batch, sms = sm_count_of(dev);
         const int size = rows <= sms ? 0 : (rows <= 2 * sms ? 1 : (rows <= 4 * sms ? 2 : 3));
-        kernel = all[size];
+        kernel = all[size + (p.grid.cluster > 1 ? 4 : 0)];
         warps = size == 0 ? 16 : (size == 1 ? 8 : 4);
     }
     cudaLaunchConfig_t cfg = {};
