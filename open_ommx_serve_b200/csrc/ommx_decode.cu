@@ -491,7 +491,7 @@ static int stage1_launch(const ommx_decode_args *a, Stage1Grid *grid) {
 namespace ommx {
 
 // Which stage-1 kernel serves a call.  The register-operand kernel (decode_stage1_kernel) is the default: on B200 it
-// is the faster of the two (40 us against 98 us for 64K tokens x 8 heads).  OMMX_B200_STAGE1=tc selects the tensor-core
+// is the faster of the two (37 us against 98 us for 64K tokens x 8 heads).  OMMX_B200_STAGE1=tc selects the tensor-core
 // kernel (decode_stage1_tc_kernel) where its shared-memory plan fits - 4 or 8 local kv heads with GQA <= 4, fewer
 // heads at any GQA <= 8 - and no differential-timing knob is set; it produces the same results within the path's
 // tolerance and is kept for further work on its pipeline.  The variable is read once per call (`tc` below).

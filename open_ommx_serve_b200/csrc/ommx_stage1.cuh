@@ -343,8 +343,8 @@ __host__ __device__ constexpr PositionBits past_31_bits(int k, int bytes) {
 // Where pieces begin depends on the plan, and with it the running maximum against which P is rounded to fp16: another split
 // count or batch moves a result by about 5e-5 of its norm, the same call repeats its bits.
 //
-// Where S bounds the shares from below and leaves CTAs without one - few sequences in splits of 512 tokens, or a ragged batch at the
-// automatic count - a share (or split) is worked on by a whole cluster of CTAs: each piece is dealt out evenly to them, and for every
+// Where S bounds the shares from below and leaves CTAs without one - few sequences in splits of
+// 512 tokens - a share (or split) is worked on by a whole cluster of CTAs: each piece is dealt out evenly to them, and for every
 // kv head one of them merges the others' softmax states through their shared memory before the one result goes to the piece's slot.
 // It is taken where the groups per CTA, the merge counted as one more, get fewer.  Measured, 8 kv heads, without / with the size taken
 // (2, 4, 8): 4K in 8 slots 42.2 / 18.5 us (28.6, 20.6, 18.1); 16K in 32 42.6 / 23.6 (28.9, 22.8, 24.8); 8 sequences of 700..2048 in 4
@@ -551,13 +551,13 @@ constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_
 // warps multiply and accumulate and do little else; q.zp, which they compute themselves, fits into their wait for the deltas, and the
 // V zero-points come straight out of the staged plane by a transposed ldmatrix.
 //
-// Bound by issue slots, the logic pipe and shared-memory wavefronts (397 of them per unit, three quarters of what the pipe can
+// Bound by issue slots, the logic pipe and shared-memory wavefronts (397 of them per unit, near four fifths of what the pipe can
 // do in the steady state), which both roles share: leaving out any part of either saves its share, and the MMA warps' chain of code
 // MMAs, delta MMAs, softmax and P.V stands close behind.  The register file (8 x 128 + 16 x 56 a lane) holds no second unit in
 // flight, and memory is at a third of its rate.  Logits in bf16 (the deltas need no second conversion), one packed min-max-add per
 // factor pair, V factors by one warp with lane = token and zero-points without staging, code words by ldmatrix, zero-point words
 // used as loaded, and a maximum that follows lazily, before -> with them, this stage and stage 2: 64K x 8 heads 44.8 -> 41.8 us;
-// 8 x 32K, 70B heads 148.7 -> 136.7; 32 sequences of 1K to 32K in splits of 512 with the store 318 -> 294.
+// 8 x 32K, 70B heads 148.7 -> 136.4; 32 sequences of 1K to 32K in splits of 512 with the store 318 -> 291.5.
 // Tried and slower (64K / 70B): 16 warps that each build and use their own half tile, no hand-overs (47.2 / 162 us, latency-bound
 // at four warps a scheduler); 16 delta warps with their own MMAs beside 8 output warps (46.1 / 167); tile rows zeroed by an
 // out-of-range tensor-map load (83 / 289); FP4 levels by the conversion instruction and a shorter wait loop (53 fewer of 1532
