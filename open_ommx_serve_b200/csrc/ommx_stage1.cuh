@@ -1498,14 +1498,23 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const int n_ctas = *s_ctas, rank = cluster_rank(), to = h % n_ctas;
         const uint32_t there = s_there + 8 * h;
         write = rank == to;
-        if (!write) {
+        // A warp that has given up takes no further part: it neither waits nor arrives, so no barrier runs ahead of those who still
+        // do, each of which gives up once in turn (with arrivals but without waits the phases alias, and a launch may wait six limits
+        // instead of two).  The lanes agree on it, whichever of them saw the clock run out.
+        auto wait_peers = [&](uint32_t bar) __attribute__((always_inline)) {
+            if (__all_sync(0xFFFFFFFFu, mbar_wait_peers(bar, (uint32_t)pi & 1u, wait_limit))) return;
+            gave_up = true;
+            if (lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
+        };
+        if (gave_up) {
+        } else if (!write) {
             if (mine) store_state();
             if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(there), "r"((uint32_t)mine) : "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_peer(peer_smem(bar_handed + 8 * h, to));
-            if (!mbar_wait_peers(bar_taken + 8 * h, (uint32_t)pi & 1u, wait_limit)) gave_up = true;
+            wait_peers(bar_taken + 8 * h);
         } else {
-            if (!mbar_wait_peers(bar_handed + 8 * h, (uint32_t)pi & 1u, wait_limit)) gave_up = true;
+            wait_peers(bar_handed + 8 * h);
             const uint32_t tile_l = smem_u32(tile) + 4 * lane;
 #pragma unroll 1
             for (int o = 1; o < n_ctas && !gave_up; ++o) {           // not all have stored theirs where the wait gave up
@@ -1515,9 +1524,8 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 merge_state([&](int i) { return lds_peer(at + 128 * i); });
             }
             __syncwarp();
-            if (lane < n_ctas && lane != rank) mbar_arrive_peer(peer_smem(bar_taken + 8 * h, lane));
+            if (!gave_up && lane < n_ctas && lane != rank) mbar_arrive_peer(peer_smem(bar_taken + 8 * h, lane));
         }
-        if (gave_up && lane == 0) or_status(p.status, OMMX_ST_TIMEOUT);
     }
     if (write) {
 #pragma unroll

@@ -430,3 +430,29 @@ def test_decode_pieces_shared_by_a_cluster(lens, H, splits, k):
     if splits and len(lens) == 1:                                                      # the same groups, a slot to each CTA
         many, lse2 = case.run(num_kv_splits=148)
         assert (o - many).abs().max().item() < 2e-3 and (lse - lse2).abs().max().item() < 2e-3
+
+
+@pytest.mark.parametrize("H", [8, 1])
+def test_bounded_waits_of_a_cluster_do_not_add_up(monkeypatch, H):
+    """Sixty pieces to a cluster of four and a ring that stops in one of the first: a warp waits a limit out once for the ring or once
+    for its peers, not at every further piece.  Limits are 4 M cycles (about 2 ms) under the knob; two of them can follow one another,
+    and sixty pieces would take thirty and more."""
+    from open_ommx_serve_b200 import _lib
+    case = Case([72] * 60 + [2088], H=H, Hq=4 * H, seed=5)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ws = torch.empty(61, 4 * H, 3, 129, dtype=torch.float32, device="cuda")
+    want, want_lse = case.run(num_kv_splits=2, attn_logits=ws)
+    monkeypatch.setenv("OMMX_ABL_TEST_STALL", "1")
+    ends = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    for _ in range(2):                                               # the first also loads the form of the kernel that has the knob
+        ends[0].record()
+        o, lse = case.run(num_kv_splits=2, attn_logits=ws, status=status)
+        ends[1].record()
+    torch.cuda.synchronize()
+    assert int(status.item()) & _lib.ST_TIMEOUT
+    assert torch.isfinite(o).all()
+    assert ends[0].elapsed_time(ends[1]) < 20
+    monkeypatch.delenv("OMMX_ABL_TEST_STALL")
+    status.zero_()
+    again, again_lse = case.run(num_kv_splits=2, attn_logits=ws, status=status)
+    assert int(status.item()) == 0 and torch.equal(again, want) and torch.equal(again_lse, want_lse)
