@@ -122,3 +122,15 @@ def test_auto_split_count_fills_whole_waves():
         s = f(seq, b, 8)
         assert 1 <= s <= max(1, (seq + 31) // 32)
         assert s >= lib.ommx_b200_min_num_kv_splits(seq, 16)
+
+
+@pytest.mark.parametrize("heads", [1, 2, 4, 8])
+@pytest.mark.parametrize("plain", [0, 1])
+def test_stage1_has_a_form_without_clusters_for_every_recipe(heads, plain):
+    """Launches without clusters do not carry the code that exchanges states: decode_stage1_kernel<k, heads, plain, relidx7, cluster>
+    is compiled, which it is where a launch refers to it, both with and without."""
+    with open(_lib.LIB_PATH, "rb") as f:
+        image = f.read()
+    for k in ("0", "2", "4", "6", "8", "12") + (("n1",) if not plain else ()):
+        for cluster in (0, 1):
+            assert f"decode_stage1_kernelILi{k}ELi{heads}ELb{plain}ELb0ELb{cluster}EE".encode() in image, (k, cluster)
