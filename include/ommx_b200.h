@@ -22,7 +22,7 @@
 extern "C" {
 #endif
 
-#define OMMX_B200_ABI_VERSION 4
+#define OMMX_B200_ABI_VERSION 5
 
 /* host-side argument errors (return values) */
 #define OMMX_E_ARG          (-1)   /* null pointer, bad size, misaligned plane */
@@ -127,7 +127,8 @@ int ommx_b200_outlier_index_convert(const void *src, void *dst, int64_t frames, 
  * f32 [batch, n_q_heads, num_kv_splits+1, head_dim+1] (lane head_dim = log-sum-exp).
  * b_seq_len holds PACKED token counts.  num_kv_splits is the number of workspace slots of a sequence: its 32-token groups are
  * worked on in at most that many pieces.  Where they are cut follows from all lengths of the batch, on the device, so that the
- * CTAs have even shares (ommx_b200_host_share_plan); where there are few slots, several CTAs work on a piece.  The reference cuts every sequence into num_kv_splits equal ones.
+ * CTAs have even shares (ommx_b200_host_launch_plan); where there are few slots, several CTAs work on a piece.  The reference cuts
+ * every sequence into num_kv_splits equal ones.
  */
 /*
  * Head-output exchange fused into stage 2, for kv heads sharded over the GPUs of one node (the split vLLM
@@ -321,9 +322,21 @@ int ommx_b200_host_pow2_exponent(float x);
 int ommx_b200_host_fp4_encode(float m);
 
 /* Host-side twin of the plan by which both decode stages share the packed groups of a batch out over CTAs (no GPU needed;
- * b_seq_len is host memory here).  *ctas: shares of the stage-1 launch, each the work of one CTA or of one cluster of CTAs where
- * there are few slots; *groups_per_cta: consecutive groups of the running list in a share, 0 = equal splits per sequence, dealt
- * out to the shares one by one.  Returns how many pieces of sequences a CTA can list, which no plan exceeds, or a negative code. */
+ * b_seq_len is host memory here).  The launch is made from the sizes, max_seq_len among them, the shares from the lengths on the
+ * device: the CTAs [i * ctas_per_share, (i + 1) * ctas_per_share) work on share i together. */
+typedef struct ommx_launch_plan {
+    int32_t ctas, cluster;          /* CTAs of the stage-1 launch, CTAs to a cluster of it (1: no clusters) */
+    int32_t shares, ctas_per_share; /* shares the groups are dealt out to, CTAs to each: 1, or `cluster` where slots are few */
+    int32_t groups_per_share;       /* consecutive groups of the running list in a share; 0: equal splits per sequence, split x of
+                                       the batch in share x % shares */
+} ommx_launch_plan;
+/* clusters_at_once: how many clusters of 2, 4 and 8 CTAs, each with an SM to itself, run at once on that device (0: none of that
+ * size are launched); NULL: in proportion to a B200's.  Returns how many pieces of sequences a CTA can list, which no plan exceeds, or
+ * a negative code. */
+int ommx_b200_host_launch_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
+                               const int32_t *clusters_at_once, ommx_launch_plan *plan);
+/* The shares and groups_per_share of that plan.  Since version 5 *ctas counts shares: with few slots a share is the work of a
+ * cluster of CTAs (ommx_b200_host_launch_plan has its size). */
 int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len,
                               int32_t sm_count, int32_t *ctas, int32_t *groups_per_cta);
 

@@ -85,6 +85,10 @@ class KVAppendArgs(C.Structure):
                 ("write_pos", C.c_void_p), ("index_is_int64", C.c_int32)]
 
 
+class LaunchPlan(C.Structure):
+    _fields_ = [(name, C.c_int32) for name in ("ctas", "cluster", "shares", "ctas_per_share", "groups_per_share")]
+
+
 #: every symbol include/ommx_b200.h declares: name -> (restype, argtypes)
 SYMBOLS = {
     "ommx_b200_pack_kv": (C.c_int, [C.POINTER(PackArgs), C.c_void_p]),
@@ -111,6 +115,8 @@ SYMBOLS = {
                                          C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ommx_b200_host_pow2_exponent": (C.c_int, [C.c_float]),
     "ommx_b200_host_fp4_encode": (C.c_int, [C.c_float]),
+    "ommx_b200_host_launch_plan": (C.c_int, [C.POINTER(C.c_int32), C.c_int32, C.c_int32, C.c_int32, C.c_int32,
+                                             C.POINTER(C.c_int32), C.POINTER(LaunchPlan)]),
     "ommx_b200_host_share_plan": (C.c_int, [C.POINTER(C.c_int32), C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                             C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "ommx_b200_abi_version": (C.c_int, []),

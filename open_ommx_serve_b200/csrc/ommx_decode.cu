@@ -482,7 +482,7 @@ static size_t stage1_smem(const S1Params &p) { return stage1_smem(p.nstages, p.s
 static int stage1_launch(const ommx_decode_args *a, Stage1Grid *grid) {
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
-    *grid = stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, sm_count_of(dev));
+    *grid = stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, chip_of(sm_count_of(dev)));
     return 0;
 }
 
@@ -693,21 +693,38 @@ extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, 
     return max(1, best);
 }
 
-extern "C" int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
-                                         int32_t *ctas, int32_t *groups_per_cta) {
+extern "C" int ommx_b200_host_launch_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
+                                          const int32_t *clusters_at_once, ommx_launch_plan *out) {
     using namespace ommx;
-    if (!b_seq_len || !ctas || !groups_per_cta || batch < 1 || num_kv_splits < 1 || sm_count < 1)
-        return fail(OMMX_E_ARG, "host_share_plan: batch=%d num_kv_splits=%d sm_count=%d", batch, num_kv_splits, sm_count);
+    if (!b_seq_len || !out || batch < 1 || num_kv_splits < 1 || sm_count < 1)
+        return fail(OMMX_E_ARG, "host_launch_plan: batch=%d num_kv_splits=%d sm_count=%d", batch, num_kv_splits, sm_count);
+    Chip chip = chip_of(sm_count);
+    if (clusters_at_once)
+        for (int i = 0; i < 3; ++i) {
+            if (clusters_at_once[i] < 0 || clusters_at_once[i] > sm_count >> (i + 1))
+                return fail(OMMX_E_ARG, "host_launch_plan: %d clusters of %d CTAs on %d SMs", clusters_at_once[i], 2 << i, sm_count);
+            chip.clusters[i] = clusters_at_once[i];
+        }
     int total = 0, longest = 0;
     for (int i = 0; i < batch; ++i) {
         total += groups_of(b_seq_len[i]);
         longest = max(longest, groups_of(b_seq_len[i]));
     }
-    const Stage1Grid grid = stage1_grid(batch, num_kv_splits, max_seq_len, sm_count);
+    const Stage1Grid grid = stage1_grid(batch, num_kv_splits, max_seq_len, chip);
     const SharePlan plan = share_plan_of(total, longest, batch, num_kv_splits, grid);
-    *ctas = plan.shares;
-    *groups_per_cta = plan.per;
+    *out = ommx_launch_plan{grid.ncta, grid.cluster, plan.shares, plan.ctas, plan.per};
     return MAX_PIECES;
+}
+extern "C" int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
+                                         int32_t *ctas, int32_t *groups_per_cta) {
+    using namespace ommx;
+    if (!ctas || !groups_per_cta) return fail(OMMX_E_ARG, "host_share_plan: null output");
+    ommx_launch_plan plan;
+    const int limit = ommx_b200_host_launch_plan(b_seq_len, batch, num_kv_splits, max_seq_len, sm_count, nullptr, &plan);
+    if (limit < 0) return limit;
+    *ctas = plan.shares;
+    *groups_per_cta = plan.groups_per_share;
+    return limit;
 }
 
 extern "C" int ommx_b200_decode_stage1(const ommx_decode_args *a, void *stream) {

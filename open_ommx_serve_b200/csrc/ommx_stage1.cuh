@@ -43,6 +43,8 @@ constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;   // about a second of SM 
 
 // The launch: CTAs (one per SM at most) in clusters of `cluster`; rounds of CTAs (clusters) that B * S splits would take
 struct Stage1Grid { int32_t ncta, waves, cluster, cluster_waves; };
+// What it is made for: SMs, and how many clusters of 2, 4 and 8 CTAs of one SM each run at once
+struct Chip { int sms, clusters[3]; };
 
 struct S1Params {
     const __nv_bfloat16 *q;
@@ -381,9 +383,12 @@ __host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longe
     }
     return a;
 }
+// clusters that fit a chip of so many SMs, as its graphics processing clusters leave room for them on the 148 of a B200
+static inline Chip chip_of(int sm_count) { return Chip{sm_count, {sm_count / 2, sm_count * 2 / 9, sm_count / 10}}; }
 // CTAs of a launch - one per SM, or one per group where there are fewer; above MAX_PIECES sequences at least one for every MAX_PIECES
 // groups or splits - and the rounds of them that equal splits would take (capped: past the cap they are never the choice)
-static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, int sm_count) {
+static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, const Chip &chip) {
+    const int sm_count = chip.sms;
     const long long longest = groups_of(max_seq_len), groups = batch * longest, splits = (long long)batch * S;
     const long long least = batch > MAX_PIECES ? (max(groups, splits) + MAX_PIECES - 1) / MAX_PIECES : 1;
     Stage1Grid g;
@@ -397,7 +402,8 @@ static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, int sm_c
         const long long bound = batch == 1 ? (longest + S - 1) / S : (longest - 2) / (S - 1) + 1;
         long long best = min(max((groups + sm_count - 1) / sm_count, bound), (splits + sm_count - 1) / sm_count * ((longest + S - 1) / S));
         for (int c = 2; c <= 8; c *= 2) {
-            const long long at_once = c == 2 ? sm_count / 2 : (c == 4 ? sm_count * 2 / 9 : sm_count / 10), shares = max(1ll, min(at_once, groups));
+            const long long at_once = chip.clusters[c / 4], shares = max(1ll, min(at_once, groups));
+            if (at_once == 0) continue;
             const long long cost = (min(max((groups + shares - 1) / shares, bound), (splits + shares - 1) / shares * ((longest + S - 1) / S)) + c - 1) / c + 1;
             if (cost < best) { best = cost; g.cluster = c; g.ncta = (int)shares * c; }
         }

@@ -94,3 +94,38 @@ def test_every_group_is_dealt_once_and_found_again(seed):
     auto = _lib.load().ommx_b200_auto_num_kv_splits(32 * max(groups), batch, 8)
     for splits in {auto, 1, rng.randint(2, 8), int(round(1024 ** rng.random()))}:
         check(groups, splits, rng.choice((1, 1, 2, 16)))
+
+
+def launch(groups, splits, clusters=None, sms=SMS):
+    lens = (C.c_int32 * len(groups))(*[32 * g for g in groups])
+    out = _lib.LaunchPlan()
+    at_once = (C.c_int32 * 3)(*clusters) if clusters else None
+    rc = _lib.load().ommx_b200_host_launch_plan(lens, len(groups), splits, 32 * max(groups), sms, at_once, C.byref(out))
+    assert rc == 128, _lib.last_error()
+    return out
+
+
+@pytest.mark.parametrize("clusters", [None, (74, 33, 15), (74, 32, 0), (70, 0, 0), (0, 0, 0), (5, 3, 1)])
+@pytest.mark.parametrize("groups,splits", [([128], 8), ([512], 32), ([64, 20, 33, 40] * 2, 4), ([256, 130, 200, 180], 16), ([64] + [1] * 60, 2),
+                                           ([2048], 147), ([1024] * 8, 18)])
+def test_launch_and_shares_agree(groups, splits, clusters):
+    """The clusters of a launch run at once, a share is one CTA's or one whole cluster's, and every share has its CTAs."""
+    p = launch(groups, splits, clusters)
+    assert p.ctas % p.cluster == 0 and p.ctas_per_share in (1, p.cluster) and p.shares * p.ctas_per_share == p.ctas <= SMS
+    if p.cluster > 1:
+        assert p.ctas // p.cluster <= (clusters or (74, 33, 15))[p.cluster // 4]
+    if not clusters:
+        assert plan(groups, splits, 1)[1:] == (p.shares, p.groups_per_share)
+
+
+def test_few_slots_take_clusters_where_there_are_any():
+    assert launch([128], 8).cluster > 1 and launch([128], 8).ctas_per_share > 1
+    assert launch([2048], 147).cluster == 1
+    alone = launch([128], 8, (0, 0, 0))
+    assert (alone.ctas, alone.cluster, alone.shares, alone.ctas_per_share) == (128, 1, 128, 1)
+
+
+def test_launch_plan_refuses_more_clusters_than_sms():
+    lens = (C.c_int32 * 1)(32)
+    for bad in ((75, 0, 0), (0, 38, 0), (0, 0, 19), (-1, 0, 0)):
+        assert _lib.load().ommx_b200_host_launch_plan(lens, 1, 1, 32, SMS, (C.c_int32 * 3)(*bad), C.byref(_lib.LaunchPlan())) == -1
