@@ -25,7 +25,8 @@ HEADERS = ("ommx_common.cuh", "ommx_stage1.cuh", "ommx_decode_tc.cuh", "ommx_tab
 OBJ = os.path.join(PKG, "build")
 HOST_LIB = HOST_PATH
 HOST_SOURCE = os.path.join(CSRC, "ommx_host.cpp")
-NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC")
+NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
+              "--no-compress")               # a process's first decode call waits 7 ms longer for the kernels of a compressed file
 
 
 def _nvcc() -> str:
