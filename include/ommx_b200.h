@@ -331,7 +331,8 @@ typedef struct ommx_launch_plan {
                                        the batch in share x % shares */
 } ommx_launch_plan;
 /* clusters_at_once: how many clusters of 2, 4 and 8 CTAs, each with an SM to itself, run at once on that device (0: none of that
- * size are launched); NULL: in proportion to a B200's.  Returns how many pieces of sequences a CTA can list, which no plan exceeds, or
+ * size are launched); NULL: in proportion to a B200's.  sm_count 0: the current device and its own clusters, as a launch on it has
+ * them.  Returns how many pieces of sequences a CTA can list, which no plan exceeds, or
  * a negative code. */
 int ommx_b200_host_launch_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
                                const int32_t *clusters_at_once, ommx_launch_plan *plan);

@@ -479,10 +479,47 @@ static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes,
 
 static size_t stage1_smem(const S1Params &p) { return stage1_smem(p.nstages, p.stage_bytes, p.GS, p.ppg); }
 
-static int stage1_launch(const ommx_decode_args *a, Stage1Grid *grid) {
+// Never launched: a CTA of it takes a whole SM, as those of every form of stage 1 do, so as many clusters of it run at once, and
+// the question loads no form that the process may never launch.
+__global__ void whole_sm_kernel() {}
+static int clusters_at_once(int cluster, int *n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(WarpLayout<8>::THREADS);
+    cfg.dynamicSmemBytes = SMEM_LIMIT;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    OMMX_CUDA_TRY(cudaFuncSetAttribute(whole_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT));
+    OMMX_CUDA_TRY(cudaOccupancyMaxActiveClusters(n, whole_sm_kernel, &cfg));
+    return 0;
+}
+// The current device, asked once; where it does not say how many clusters of a size it runs, none are launched
+static int current_chip(Chip *chip) {
+    static std::atomic<uint64_t> known[MAX_DEVICES];   // 16 bits each: SMs, clusters of 2, 4 and 8
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
-    *grid = stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, chip_of(sm_count_of(dev)));
+    uint64_t word = known[dev].load(std::memory_order_acquire);
+    if (word == 0) {
+        word = (uint64_t)(sm_count_of(dev) & 0xFFFF);
+        for (int i = 0; i < 3; ++i) {
+            int n = 0;
+            if (clusters_at_once(2 << i, &n) != 0) { (void)cudaGetLastError(); n = 0; }
+            word |= (uint64_t)(n & 0xFFFF) << (16 * (i + 1));
+        }
+        known[dev].store(word, std::memory_order_release);
+    }
+    *chip = Chip{(int)(word & 0xFFFF), {(int)(word >> 16 & 0xFFFF), (int)(word >> 32 & 0xFFFF), (int)(word >> 48)}};
+    return 0;
+}
+
+static int stage1_launch(const ommx_decode_args *a, Stage1Grid *grid) {
+    Chip chip;
+    if (int rc = current_chip(&chip)) return rc;
+    *grid = stage1_grid(a->batch, a->num_kv_splits, a->max_seq_len, chip);
     return 0;
 }
 
@@ -696,10 +733,12 @@ extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, 
 extern "C" int ommx_b200_host_launch_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
                                           const int32_t *clusters_at_once, ommx_launch_plan *out) {
     using namespace ommx;
-    if (!b_seq_len || !out || batch < 1 || num_kv_splits < 1 || sm_count < 1)
+    if (!b_seq_len || !out || batch < 1 || num_kv_splits < 1 || sm_count < 0)
         return fail(OMMX_E_ARG, "host_launch_plan: batch=%d num_kv_splits=%d sm_count=%d", batch, num_kv_splits, sm_count);
     Chip chip = chip_of(sm_count);
-    if (clusters_at_once)
+    if (sm_count == 0)
+        if (int rc = current_chip(&chip)) return rc;
+    if (sm_count > 0 && clusters_at_once)
         for (int i = 0; i < 3; ++i) {
             if (clusters_at_once[i] < 0 || clusters_at_once[i] > sm_count >> (i + 1))
                 return fail(OMMX_E_ARG, "host_launch_plan: %d clusters of %d CTAs on %d SMs", clusters_at_once[i], 2 << i, sm_count);
@@ -718,7 +757,7 @@ extern "C" int ommx_b200_host_launch_plan(const int32_t *b_seq_len, int32_t batc
 extern "C" int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch, int32_t num_kv_splits, int32_t max_seq_len, int32_t sm_count,
                                          int32_t *ctas, int32_t *groups_per_cta) {
     using namespace ommx;
-    if (!ctas || !groups_per_cta) return fail(OMMX_E_ARG, "host_share_plan: null output");
+    if (!ctas || !groups_per_cta || sm_count < 1) return fail(OMMX_E_ARG, "host_share_plan: null output or sm_count=%d", sm_count);
     ommx_launch_plan plan;
     const int limit = ommx_b200_host_launch_plan(b_seq_len, batch, num_kv_splits, max_seq_len, sm_count, nullptr, &plan);
     if (limit < 0) return limit;

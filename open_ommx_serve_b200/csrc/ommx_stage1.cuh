@@ -383,8 +383,8 @@ __host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longe
     }
     return a;
 }
-// clusters that fit a chip of so many SMs, as its graphics processing clusters leave room for them on the 148 of a B200
-static inline Chip chip_of(int sm_count) { return Chip{sm_count, {sm_count / 2, sm_count * 2 / 9, sm_count / 10}}; }
+// Host code without a device takes a chip of so many SMs to be a B200, which runs 74, 33 and 15 clusters on 148 (a launch asks its device)
+static inline Chip chip_of(int sm_count) { return Chip{sm_count, {sm_count / 2, sm_count * 33 / 148, sm_count * 15 / 148}}; }
 // CTAs of a launch - one per SM, or one per group where there are fewer; above MAX_PIECES sequences at least one for every MAX_PIECES
 // groups or splits - and the rounds of them that equal splits would take (capped: past the cap they are never the choice)
 static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, const Chip &chip) {
@@ -395,10 +395,10 @@ static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, const Ch
     g.ncta = (int)max(min((long long)sm_count, max(groups, 1ll)), least);
     g.cluster = 1;
     // The cluster size that leaves the fewest groups per CTA if all sequences are of the longest's length; share_plan_of then decides by
-    // the lengths.  Clusters of two fill the chip (74 at once on 148 SMs); of four 33 run at once, of eight 15.  A launch that cannot
+    // the lengths.  No more clusters than run at once: on a B200's 148 SMs 74 of two, 33 of four, 15 of eight.  A launch that cannot
     // gain at equal lengths keeps the form without clusters: the exchange's code alone costs 4.5 % (8 x 32K: 133.9 -> 140.0 us), although
     // a ragged batch would win by more (8 sequences of 4K..32K in 18 slots each: 133.5 -> 103.4).
-    if (batch <= MAX_PIECES && S > (batch > 1 ? 1 : 0) && sm_count >= 128) {     // counted on the whole chip only
+    if (batch <= MAX_PIECES && S > (batch > 1 ? 1 : 0)) {
         const long long bound = batch == 1 ? (longest + S - 1) / S : (longest - 2) / (S - 1) + 1;
         long long best = min(max((groups + sm_count - 1) / sm_count, bound), (splits + sm_count - 1) / sm_count * ((longest + S - 1) / S));
         for (int c = 2; c <= 8; c *= 2) {

@@ -129,3 +129,42 @@ def test_launch_plan_refuses_more_clusters_than_sms():
     lens = (C.c_int32 * 1)(32)
     for bad in ((75, 0, 0), (0, 38, 0), (0, 0, 19), (-1, 0, 0)):
         assert _lib.load().ommx_b200_host_launch_plan(lens, 1, 1, 32, SMS, (C.c_int32 * 3)(*bad), C.byref(_lib.LaunchPlan())) == -1
+
+
+@pytest.mark.gpu
+def test_launches_count_on_the_clusters_that_this_device_runs():
+    """Against the driver's answer for a kernel of ours that takes a whole SM."""
+    import torch
+    from cuda.bindings import driver, nvrtc
+
+    def ok(result):
+        assert int(result[0]) == 0, result
+        return result[1:] if len(result) > 2 else (result[1] if len(result) > 1 else None)
+
+    torch.zeros(1, device="cuda")
+    prog = ok(nvrtc.nvrtcCreateProgram(b'extern "C" __global__ void alone(float *p) { extern __shared__ float s[]; if (p) p[0] = s[0]; }',
+                                       b"alone.cu", 0, [], []))
+    ok(nvrtc.nvrtcCompileProgram(prog, 1, [b"--gpu-architecture=sm_100a"]))
+    image = b" " * ok(nvrtc.nvrtcGetCUBINSize(prog))
+    ok(nvrtc.nvrtcGetCUBIN(prog, image))
+    fn = ok(driver.cuModuleGetFunction(ok(driver.cuModuleLoadData(image)), b"alone"))
+    smem = 200 * 1024
+    ok(driver.cuFuncSetAttribute(fn, driver.CUfunction_attribute.CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, smem))
+    at_once = []
+    for size in (2, 4, 8):
+        attr = driver.CUlaunchAttribute()
+        attr.id = driver.CUlaunchAttributeID.CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION
+        attr.value.clusterDim.x, attr.value.clusterDim.y, attr.value.clusterDim.z = size, 1, 1
+        cfg = driver.CUlaunchConfig()
+        cfg.gridDimX, cfg.gridDimY, cfg.gridDimZ = size, 1, 1
+        cfg.blockDimX, cfg.blockDimY, cfg.blockDimZ = 768, 1, 1
+        cfg.sharedMemBytes, cfg.attrs, cfg.numAttrs = smem, [attr], 1
+        at_once.append(ok(driver.cuOccupancyMaxActiveClusters(fn, cfg)))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    sizes = set()
+    for groups, splits in (([2048], 8), ([512], 32), ([64] + [1] * 60, 2), ([512], 72), ([2048], 147)):
+        here, want = launch(groups, splits, sms=0), launch(groups, splits, at_once, sms)
+        assert all(getattr(here, f) == getattr(want, f) for f, _ in _lib.LaunchPlan._fields_)
+        if here.cluster > 1 and here.ctas // here.cluster == at_once[here.cluster // 4]:
+            sizes.add(here.cluster)
+    assert sizes == {2, 4, 8}
