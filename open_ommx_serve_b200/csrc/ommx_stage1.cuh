@@ -334,7 +334,7 @@ __host__ __device__ constexpr PositionBits past_31_bits(int k, int bytes) {
 // around its steady state: 560 us of store and decode against 318 us).  A piece of a sequence writes its partial result to
 // workspace slot (its CTA - the first CTA of the sequence), and the caller's workspace has S slots per sequence, which bounds `per`
 // from below: shares are even up to one group where S is generous, and longer, up to the longest sequence over S - 1, where it is not
-// (8 sequences of 4K..32K tokens, both stages: 86 us with 64 slots, 145 us with the 18 of ommx_b200_auto_num_kv_splits).
+// (8 sequences of 4K..32K tokens, both stages: 96 us with 64 slots, 133 us with the 18 of ommx_b200_auto_num_kv_splits).
 // Equal splits per sequence, dealt out one by one (per = 0: item x is split x % S of sequence x / S), are taken instead
 //   * where that bound makes the shares longer than S of them per sequence would be, and
 //   * where a share could hold more sequences than a CTA lists (MAX_PIECES).  Of equal splits a CTA never has more than that:
@@ -557,22 +557,24 @@ constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_
 // warps multiply and accumulate and do little else; q.zp, which they compute themselves, fits into their wait for the deltas, and the
 // V zero-points come straight out of the staged plane by a transposed ldmatrix.
 //
-// Bound by issue slots, the logic pipe and shared-memory wavefronts (397 of them per unit, near four fifths of what the pipe can
-// do in the steady state), which both roles share: leaving out any part of either saves its share, and the MMA warps' chain of code
+// Bound by issue slots, the logic pipe and shared-memory wavefronts (399 of them and 1536 instructions per unit, near four fifths of
+// what pipe and slots can do in the steady state), which both roles share: leaving out any part of either saves its share, and the MMA warps' chain of code
 // MMAs, delta MMAs, softmax and P.V stands close behind.  The register file (8 x 128 + 16 x 56 a lane) holds no second unit in
-// flight, and memory is at a third of its rate.  Logits in bf16 (the deltas need no second conversion), one packed min-max-add per
+// flight, and memory is at 28 to 32 % of its rate.  Logits in bf16 (the deltas need no second conversion), one packed min-max-add per
 // factor pair, V factors by one warp with lane = token and zero-points without staging, code words by ldmatrix, zero-point words
 // used as loaded, and a maximum that follows lazily, before -> with them, this stage and stage 2: 64K x 8 heads 44.8 -> 41.8 us;
 // 8 x 32K, 70B heads 148.7 -> 136.4; 32 sequences of 1K to 32K in splits of 512 with the store 318 -> 291.5.
 // Tried and slower (64K / 70B): 16 warps that each build and use their own half tile, no hand-overs (47.2 / 162 us, latency-bound
 // at four warps a scheduler); 16 delta warps with their own MMAs beside 8 output warps (46.1 / 167); tile rows zeroed by an
-// out-of-range tensor-map load (83 / 289); FP4 levels by the conversion instruction and a shorter wait loop (53 fewer of 1532
+// out-of-range tensor-map load (83 / 289); FP4 levels by the conversion instruction and a shorter wait loop (53 fewer
 // instructions per unit, same time).
+// With one or two kv heads a unit costs more: 1966 and 1792 instructions and 507 and 498 wavefronts (176 and 178 of them bank conflicts,
+// 111 at eight heads), because a page of theirs is staged as it lies, without a swizzle, and a stage takes 112 or 56 copies.
 //
 // PLAIN: the recipes that are served - bitmask or relidx7 index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
-// form keeps them at run time; its tests and address arithmetic inside the unit cost it 10 % (70B heads 8 x 32K: 160.6 us
-// against 143.9 us).
+// form keeps them at run time; its tests and address arithmetic inside the unit cost it 12 to 15 % (both stages: 64K
+// 46.1 us against 41.0, 70B heads 8 x 32K 155.4 against 135.5; one and two kv heads 34.1 against 32.8 and 30.0 against 28.3).
 // IDX7 (plain form only): relidx7 positions instead of bitmasks, turned into masks by three instructions a position.  At run time, byte
 // by byte, they took longer than the rest of the tile: 64K x 8 heads, both stages, k = 6 66.3 -> 45.9 us, k = 12 94.9 -> 58.7.
 template <int KOUT, int H, bool IDX7> struct PlainLayout {
@@ -819,7 +821,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     const int lm_tok = 8 * ((lane >> 2) & 3) + 4 * (lane >> 4) + (lane & 3);
     // Build the sidecar tile of a unit between two uses by its MMA warp.  A tile is built in two
     // halves by two warps at once, because the MMA warp of the unit waits for it: half hf takes 64 of the
-    // K channels (delta columns, scale factors) and V tokens 16hf..16hf+15 (factors, zero-points).
+    // K channels (delta columns, scale factors), half 0 the V factors of all 32 tokens as well (lane = token).
     // Returns false when a bounded wait ran out.
     uint32_t e_max = 0;                                          // largest scale exponents seen, biased by 128, two halves
     auto decode_item = [&](const Piece &pc, const int n) __attribute__((always_inline)) -> bool {
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const int d0 = 64 * hf + 2 * cp;                         // first of this lane's two channels
         const bool splice = k_out > 0 && !no_outlier;
         // ---- everything that only reads the stage comes before the wait for the tile, which the MMA warps make a decode warp
-        //      wait for (a sixth of its time): the parameters of both channels, the K and V factors, V zero-points ----
+        //      wait for (a sixth of its time): the parameters of both channels, the K and V factors ----
         uint32_t e2 = 0, z2 = 0, kf = 0, f02 = 0, f13 = 0, ms2 = 0, mc2 = 0;
         uint2 bm2 = make_uint2(0u, 0u);
         // From 6 outliers on the base codes are looked up in bit planes in registers: a gather per outlier costs 3 to 4 conflicting
@@ -967,7 +969,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             return false;
         }
         if (active) {
-            // ---- first the rows the code MMAs and the softmax read (K factors, V factors and zero-points): the MMA warp
+            // ---- first the rows of factors (K for the code MMAs, V for P.V): the MMA warp
             //      starts on them while the deltas are scattered ----
             uint8_t *row = tile + ROW_KF * DT_STRIDE + 128 * hf + 64 * (da >> 1) + 16 * dj + 8 * (da & 1) + 2 * dh;
             *reinterpret_cast<uint16_t *>(row) = (uint16_t)kf;
@@ -1250,7 +1252,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
 #pragma unroll
                 for (int w = 0; w < 2; ++w)
                     ldsm_x4(smem_u32(gb) + swz128((uint32_t)(lane * TS + h * 32 + 16 * w), SWZ), kw[w][0], kw[w][1], kw[w][2], kw[w][3]);
-            // The unit's sidecar tile arrives in two steps: first the factor and zero-point rows, then the outlier
+            // The unit's sidecar tile arrives in two steps: first the rows of factors, then the outlier
             // deltas.  The code MMAs run on the first, while the decode warps still scatter the deltas.
             if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
                 gave_up = true;
