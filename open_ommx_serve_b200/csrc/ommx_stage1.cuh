@@ -1507,8 +1507,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         const uint32_t there = s_there + 8 * h;
         write = rank == to;
         // A warp that has given up takes no further part: it neither waits nor arrives, so no barrier runs ahead of those who still
-        // do, each of which gives up once in turn (with arrivals but without waits the phases alias, and a launch may wait six limits
-        // instead of two).  The lanes agree on it, whichever of them saw the clock run out.
+        // do, each of which gives up once in turn, and the launch ends within two or three limits.  With further waits it could take
+        // fifteen, with arrivals but no waits, whose phases alias, six (a model of the barriers over random pieces).  The lanes agree on
+        // it, whichever of them saw the clock run out.
         auto wait_peers = [&](uint32_t bar) __attribute__((always_inline)) {
             if (__all_sync(0xFFFFFFFFu, mbar_wait_peers(bar, (uint32_t)pi & 1u, wait_limit))) return;
             gave_up = true;
