@@ -415,7 +415,8 @@ def test_decode_logits_that_rise_from_group_to_group(slope, monkeypatch):
     ([3960], 8, 8, 6), ([3960], 4, 8, 6), ([3960], 1, 4, 6), ([2000], 2, 2, 4),        # clusters of eight to a split
     ([3000, 700, 1500, 40, 2048], 8, 4, 6), ([1000, 1000], 1, 2, 8),                   # several sequences, one without groups
     ([104, 2088], 8, 2, 6), ([72, 72, 1064], 4, 1, 6),                                 # pieces of fewer groups than CTAs
-    ([16000], 8, 32, 2), ([5000, 5000], 2, 10, 6),                                     # clusters of four and two
+    ([16000], 8, 32, 2), ([5000, 5000], 2, 10, 6),                                     # clusters of four; of eight, two sequences to a share
+    ([16000], 8, 72, 6), ([16000], 1, 72, 6),                                          # clusters of two
     ([9000, 300, 300, 72, 4000, 1000], 8, None, 6), ([6000, 200, 1500], 1, None, 12),  # ragged batches at the automatic count
     ([3960], 8, 8, 3), ([2000, 500], 4, 2, 0),                                         # the general form; no outliers
 ])
@@ -430,6 +431,19 @@ def test_decode_pieces_shared_by_a_cluster(lens, H, splits, k):
     if splits and len(lens) == 1:                                                      # the same groups, a slot to each CTA
         many, lse2 = case.run(num_kv_splits=148)
         assert (o - many).abs().max().item() < 2e-3 and (lse - lse2).abs().max().item() < 2e-3
+
+
+@pytest.mark.parametrize("lens,H", [([300], 8), ([300, 72, 40, 520], 8), ([1000], 1)])
+def test_decode_launch_in_clusters_for_lengths_that_want_none(lens, H):
+    """The launch is made from max_seq_len, the shares from the lengths: a captured graph meets both."""
+    from open_ommx_serve_b200 import _lib
+    case = Case(lens, H=H, Hq=4 * H, seed=41)
+    plan = _lib.LaunchPlan()
+    lengths = (_lib.C.c_int32 * len(lens))(*case.packed)
+    assert _lib.load().ommx_b200_host_launch_plan(lengths, len(lens), 32, 15968, 0, None, _lib.C.byref(plan)) > 0
+    assert plan.cluster > 1 and plan.ctas_per_share == 1
+    o, lse = _run_and_check(case, num_kv_splits=32, max_seq_len=15968)
+    assert torch.equal(o, case.run(num_kv_splits=32, max_seq_len=15968)[0])
 
 
 def test_bounded_waits_of_a_cluster_do_not_add_up(monkeypatch):
