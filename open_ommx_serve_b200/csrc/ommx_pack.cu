@@ -101,9 +101,21 @@ struct PackKParams {
 constexpr int PACK_WARPS = 4;
 constexpr int PACK_BLK = 16;                       // channels per warp: one 32-bit word of 2-bit codes per token
 
+// RN(x / 3): quotient from the rounded reciprocal, exact remainder by one FMA, corrected quotient (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000", 1990); equal to the division for every x >= 1e-8, infinity included.
+__host__ __device__ __forceinline__ float div_by_3(float x) {
+    constexpr float THIRD = 1.f / 3.f;
+#ifdef __CUDA_ARCH__
+    const float q = __fmul_rn(x, THIRD), r = __fmaf_rn(-3.f, q, x);
+    return r == r ? __fmaf_rn(r, THIRD, q) : q;
+#else
+    return x / 3.f;
+#endif
+}
+
 // scale -> (value after optional pow2 snap and storage rounding, exponent)
 __device__ __forceinline__ float snap_scale(float rng, int use_pow2, int scale_kind, int &e) {
-    float scale = __fdiv_rn(fmaxf(rng, 1e-8f), 3.0f);
+    float scale = div_by_3(fmaxf(rng, 1e-8f));
     e = 0;
     if (use_pow2) {
         e = pow2_exponent_tbl(fmaxf(scale, 1e-12f), c_pow2_cut);
@@ -259,6 +271,16 @@ __device__ __forceinline__ uint32_t drop_ties(uint32_t picks, uint32_t eq, int k
     return picks;
 }
 
+// the same for both channels of a pair; called by whole warps
+__device__ __forceinline__ void drop_ties_pair(uint32_t (&picks)[2], uint32_t eq0, uint32_t eq1, int keep, bool none) {
+    int over0 = none ? 0 : __popc(picks[0]) - keep, over1 = none ? 0 : __popc(picks[1]) - keep;
+    while (__any_sync(0xFFFFFFFFu, max(over0, over1) > 0)) {
+        const uint32_t b0 = over0 > 0 ? 0x80000000u >> __clz(eq0) : 0u, b1 = over1 > 0 ? 0x80000000u >> __clz(eq1) : 0u;
+        picks[0] ^= b0; eq0 ^= b0; --over0;
+        picks[1] ^= b1; eq1 ^= b1; --over1;
+    }
+}
+
 // The M largest (descending) and M smallest (ascending) of 32 values x(0) .. x(31), by a sorting network for M <= 4: blocks of four are
 // sorted, then merged (248 min / max at M = 4).  V is float, or a pair of 16-bit values, whose halves are two channels and on whose
 // min and max a NaN wins.  lowest / highest: what every value displaces.
@@ -280,17 +302,24 @@ __device__ __forceinline__ void extremes_of_32(Fn x, V (&top)[N], V (&bot)[N], V
         for (int t = 1; t < 32; ++t) { top[0] = v_max(top[0], x(t)); bot[0] = v_min(bot[0], x(t)); }
     } else if constexpr (M <= 4) {
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            V s0 = x(4 * b), s1 = x(4 * b + 1), s2 = x(4 * b + 2), s3 = x(4 * b + 3);
-            order2(s0, s1); order2(s2, s3); order2(s0, s2); order2(s1, s3); order2(s1, s2);
+        for (int b = 0; b < 4; ++b) {
+            V v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = x(8 * b + i);
+            // Batcher's odd-even merge of two sorted fours
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) { order2(v[i], v[i + 1]); order2(v[i + 2], v[i + 3]); order2(v[i], v[i + 2]); order2(v[i + 1], v[i + 3]); order2(v[i + 1], v[i + 2]); }
+            order2(v[0], v[4]); order2(v[1], v[5]); order2(v[2], v[6]); order2(v[3], v[7]);
+            order2(v[2], v[4]); order2(v[3], v[5]);
+            order2(v[1], v[2]); order2(v[3], v[4]); order2(v[5], v[6]);
             if (b == 0) {
-                top[0] = s0; top[1] = s1; top[2] = s2; top[3] = s3;
-                bot[0] = s3; bot[1] = s2; bot[2] = s1; bot[3] = s0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { top[i] = v[i]; bot[i] = v[7 - i]; }
             } else {
                 // the larger (smaller) halves of two sorted fours are bitonic: two rounds sort them
-                top[0] = v_max(top[0], s3); top[1] = v_max(top[1], s2); top[2] = v_max(top[2], s1); top[3] = v_max(top[3], s0);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { top[i] = v_max(top[i], v[3 - i]); bot[i] = v_min(bot[i], v[4 + i]); }
                 order2(top[0], top[2]); order2(top[1], top[3]); order2(top[0], top[1]); order2(top[2], top[3]);
-                bot[0] = v_min(bot[0], s0); bot[1] = v_min(bot[1], s1); bot[2] = v_min(bot[2], s2); bot[3] = v_min(bot[3], s3);
                 order2(bot[2], bot[0]); order2(bot[3], bot[1]); order2(bot[1], bot[0]); order2(bot[3], bot[2]);
             }
         }
@@ -753,15 +782,19 @@ __global__ void __launch_bounds__(128) pack_v_kernel(PackVParams p) {
 //
 // K: one warp per (32-token group, kv head, 64 channels), lane = two adjacent channels in the halves of a register, so that
 // selection runs on both at once: 16-bit values need no order keys, min and max of packed halves sort them directly.  The
-// KT + 1 largest and KB + 1 smallest values come from a sorting network (blocks of four sorted, then merged: 248
+// KT + 1 largest and KB + 1 smallest values come from a sorting network (blocks of eight sorted, then merged: 224
 // min/max per pair of channels, where insertion of 32-bit keys took 900), the picks are what is not below (above) the
 // KT-th (KB-th) value, and where equal values leave too many, the highest tokens go - the stable-sort rule.  The values behind the
 // picks are the base range.  Codes are two FMAs and one shifted add per value: (x - zp) / 4s saturated to [0, 1] in one FMA (one
 // rounding, the same as the subtraction's, because s is a power of two), times 4 onto 1.5 * 2^23, which rounds to nearest even.
-// Bound by no single pipe: while the SMs are busy the ALU pipe (min / max, compare and logic run at half the FMA rate) is 60 % and the
-// issue slots are 63 % taken, DRAM 21 %; the rest is waiting for instructions to be fetched (straight-line code), for first loads
-// and for fixed-latency results, and the last of three waves leaves SMs idle for a fifth of the launch.  Measured, K + V: 8192 tokens x
-// 8 heads (42 MB) 38.9 -> 18.9 us, 2.2 TB/s; 32768 tokens 122 -> 61 us; 1024 tokens 9.3 -> 5.5 us.
+// Bound by instructions: min / max, compares and logic run at half rate in one pipe, which is 69 % busy in a steady state of K (issue slots
+// 69 %), and what can goes to the multiply-add pipe instead (masks of compares summed with powers of two, rows by one wide
+// multiply-add, the two channels' codes joined before the saturated ones are put right).  A K warp is 1670 instructions, a V warp
+// 308; with plain divisions for the indices, a vote-free tie test by counts and blocks of four they were 1875 and 442.  Measured, K + V,
+// bf16, one after the other: 8192 tokens x 8 heads (42 MB) 17.2 -> 14.7 us, 32768 tokens 61.9 -> 52.6, 1024 tokens 6.2 -> 5.5, 512 tokens 5.0 -> 4.4.
+// Tried and slower (8192 tokens): V of a unit staged by its K warp (18.8 against 17.2), V rows prefetched into the L2 by the K warps (15.9 against
+// 14.7: their first loads are what the kernel waits for at first), two V pieces a thread (15.1; 32768 tokens 50.2 against 52.1), eight
+// CTAs to an SM with spills (15.0), six (15.9 against 15.4).
 // The scale, map and FP4 steps are those of pack_k_kernel, operation for operation.
 // ---------------------------------------------------------------------------------------------
 template <typename T> struct Pair16;
@@ -779,17 +812,33 @@ template <> struct Pair16<__half> {
 };
 template <typename V> __device__ __forceinline__ V as_pair(uint32_t w) { return *reinterpret_cast<const V *>(&w); }
 template <typename V> __device__ __forceinline__ uint32_t pair_bits(V v) { return *reinterpret_cast<const uint32_t *>(&v); }
-// one 16-bit value of half c of a pair of words
-__device__ __forceinline__ bool half_is_special(uint32_t w, uint32_t exp) {
-    return (w & exp) == exp || ((w >> 16) & exp) == exp;
+// whether any of the four 16-bit values has an exponent of all ones (exp): one more in its lowest bit then reaches the sign
+__device__ __forceinline__ bool any_special(uint32_t a, uint32_t b, uint32_t exp) {
+    const uint32_t one = (exp & (0u - exp)) * 0x00010001u;
+    return ((((a & 0x7FFF7FFFu) + one) | ((b & 0x7FFF7FFFu) + one)) & 0x80008000u) != 0u;
 }
+// A sum over 16 tokens t of masks (0xFFFF or 0 in either half) times 2^t, taken apart into the bits of the lower and of the upper halves.
+// Summing by multiply-adds keeps the logic pipe free, which the selection is bound by: with S = -L + (L - H) 2^16 mod 2^32 for bits L and H.
+__device__ __forceinline__ uint32_t summed_lo(uint32_t s) { return (0u - s) & 0xFFFFu; }
+__device__ __forceinline__ uint32_t summed_hi(uint32_t s) { return (summed_lo(s) - ((s + summed_lo(s)) >> 16)) & 0xFFFFu; }
 
 // The rows of a group: consecutive, or in a residual ring (row `wrap` on follow behind row 0 of the ring again)
 struct GroupRows {
-    int64_t stride;                    // elements from a row to the next
+    int32_t stride;                    // elements from a row to the next
     int wrap, back;                    // rows t >= wrap lie `back` rows earlier
     __device__ __forceinline__ int64_t at(int t) const { return (int64_t)(t < wrap ? t : t - back) * stride; }
+    // `p` moved on to row t, by one multiply-add rather than two additions of the logic pipe
+    template <typename E> __device__ __forceinline__ const E *from(const E *p, int t) const {
+        int64_t r;
+        asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(t < wrap ? t : t - back), "r"(stride * (int)sizeof(E)), "l"(p));
+        return reinterpret_cast<const E *>(r);
+    }
 };
+
+// nibbles 0..4 of two channels, where 4 (saturated) is code 3, to nibbles of two codes
+__device__ __forceinline__ uint32_t join_codes(uint32_t a, uint32_t b) {
+    return (a + 4u * b) - (((a >> 2) & 0x11111111u) | (b & 0x44444444u));
+}
 
 // FP4 E2M1 code by three comparisons
 __device__ __forceinline__ uint32_t fp4_code(float m) {
@@ -800,9 +849,10 @@ __device__ __forceinline__ uint32_t fp4_code(float m) {
     return (m < 0.f ? 8u : 0u) | (c2 ? 4u : 0u) | (c1 ? 2u : 0u) | (c0 ? 1u : 0u);
 }
 
-// col: this lane's channels 2 lane, 2 lane + 1 in row 0; the unit's destination group slot, page of every token and head
+// col: this lane's channels 2 lane, 2 lane + 1 in row 0; the unit's destination group slot and head, and of the lane's token the page and
+// the row in it.  Rows of planes are counted in 32 bits.
 template <typename T, int KT, int KB>
-__device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, const GroupRows &rows, int slot, int h, int blk, int page, int lane) {
+__device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, const GroupRows &rows, int slot, int h, int blk, int page, int in_page, int lane) {
     typedef Pair16<T> P;
     typedef typename P::V V;
     constexpr int K = KT + KB;
@@ -810,50 +860,44 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
     static_assert(K <= 8, "the nibble stream is kept in 32 bits");
     uint32_t w[32];
 #pragma unroll
-    for (int t = 0; t < 32; ++t) w[t] = *reinterpret_cast<const uint32_t *>(col + rows.at(t));
+    for (int t = 0; t < 32; ++t) w[t] = *reinterpret_cast<const uint32_t *>(rows.from(col, t));
 
     // ---- the M largest, descending, and the M smallest, ascending ----
     constexpr int M = KT >= KB ? KT + 1 : KB + 1;
     V top[M <= 4 ? 4 : M], bot[M <= 4 ? 4 : M];
     extremes_of_32<M>([&](int t) { return as_pair<V>(w[t]); }, top, bot, as_pair<V>(P::EXP | (P::EXP << 16) | 0x80008000u), as_pair<V>(P::EXP | (P::EXP << 16)));
-    bool bad = half_is_special(pair_bits(top[0]), P::EXP) || half_is_special(pair_bits(bot[0]), P::EXP);
+    bool bad = any_special(pair_bits(top[0]), pair_bits(bot[0]), P::EXP);
 
     // ---- which tokens are picked ----
     uint32_t omask[2] = {0u, 0u};
     if constexpr (K > 0) {
-        uint32_t t0 = 0, t1 = 0, b0 = 0, b1 = 0;                      // halves: the two channels, tokens 0..15 and 16..31
+        uint32_t t0 = 0, t1 = 0, b0 = 0, b1 = 0;                      // sums of masks of the two channels, tokens 0..15 and 16..31
         const V thr_t = top[KT > 0 ? KT - 1 : 0], thr_b = bot[KB > 0 ? KB - 1 : 0];
 #pragma unroll
         for (int t = 0; t < 16; ++t) {
-            const uint32_t bit = 0x00010001u << t;
-            t0 |= __hge2_mask(as_pair<V>(w[t]), thr_t) & bit;
-            t1 |= __hge2_mask(as_pair<V>(w[t + 16]), thr_t) & bit;
-            b0 |= __hle2_mask(as_pair<V>(w[t]), thr_b) & bit;
-            b1 |= __hle2_mask(as_pair<V>(w[t + 16]), thr_b) & bit;
+            t0 += __hge2_mask(as_pair<V>(w[t]), thr_t) * (1u << t);
+            t1 += __hge2_mask(as_pair<V>(w[t + 16]), thr_t) * (1u << t);
+            b0 += __hle2_mask(as_pair<V>(w[t]), thr_b) * (1u << t);
+            b1 += __hle2_mask(as_pair<V>(w[t + 16]), thr_b) * (1u << t);
         }
-        uint32_t tm[2] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632)};
-        uint32_t bm[2] = {__byte_perm(b0, b1, 0x5410), __byte_perm(b0, b1, 0x7632)};
-        const bool ties = __popc(tm[0]) != KT || __popc(tm[1]) != KT || __popc(bm[0] & ~tm[0]) != KB || __popc(bm[1] & ~tm[1]) != KB;
-        if (__any_sync(0xFFFFFFFFu, ties && !bad)) {
-            // more tokens at a threshold than picks left: the lowest of them are taken, the bottom picks among what the
-            // top picks left
+        uint32_t tm[2] = {summed_lo(t0) | (summed_lo(t1) << 16), summed_hi(t0) | (summed_hi(t1) << 16)};
+        uint32_t bm[2] = {summed_lo(b0) | (summed_lo(b1) << 16), summed_hi(b0) | (summed_hi(b1) << 16)};
+        // more tokens at a threshold than picks left: the value behind it is equal to it, or the two thresholds meet
+        const uint32_t ties = __heq2_mask(thr_t, top[KT]) | __heq2_mask(thr_b, bot[KB]) | __hle2_mask(thr_t, thr_b);
+        if (__any_sync(0xFFFFFFFFu, ties != 0u && !bad)) {
+            // the lowest tokens are taken, the bottom picks among what the top picks left
             uint32_t e0 = 0, e1 = 0, f0 = 0, f1 = 0;
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
-                const uint32_t bit = 0x00010001u << t;
-                e0 |= __heq2_mask(as_pair<V>(w[t]), thr_t) & bit;
-                e1 |= __heq2_mask(as_pair<V>(w[t + 16]), thr_t) & bit;
-                f0 |= __heq2_mask(as_pair<V>(w[t]), thr_b) & bit;
-                f1 |= __heq2_mask(as_pair<V>(w[t + 16]), thr_b) & bit;
+                e0 += __heq2_mask(as_pair<V>(w[t]), thr_t) * (1u << t);
+                e1 += __heq2_mask(as_pair<V>(w[t + 16]), thr_t) * (1u << t);
+                f0 += __heq2_mask(as_pair<V>(w[t]), thr_b) * (1u << t);
+                f1 += __heq2_mask(as_pair<V>(w[t + 16]), thr_b) * (1u << t);
             }
-            if (!bad) {
-                tm[0] = drop_ties(tm[0], __byte_perm(e0, e1, 0x5410), KT);
-                tm[1] = drop_ties(tm[1], __byte_perm(e0, e1, 0x7632), KT);
-                bm[0] &= ~tm[0];
-                bm[1] &= ~tm[1];
-                bm[0] = drop_ties(bm[0], __byte_perm(f0, f1, 0x5410) & bm[0], KB);
-                bm[1] = drop_ties(bm[1], __byte_perm(f0, f1, 0x7632) & bm[1], KB);
-            }
+            drop_ties_pair(tm, summed_lo(e0) | (summed_lo(e1) << 16), summed_hi(e0) | (summed_hi(e1) << 16), KT, bad);
+            bm[0] &= ~tm[0];
+            bm[1] &= ~tm[1];
+            drop_ties_pair(bm, (summed_lo(f0) | (summed_lo(f1) << 16)) & bm[0], (summed_hi(f0) | (summed_hi(f1) << 16)) & bm[1], KB, bad);
         }
         omask[0] = tm[0] | bm[0];
         omask[1] = tm[1] | bm[1];
@@ -866,7 +910,7 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
     const bool store_f32 = p.scale_kind == OMMX_SCALE_F32;
     int e[2];
     float scale[2], zp[2];
-    uint32_t cw[4] = {0u, 0u, 0u, 0u};                                 // nibble i of word j: token 8j + i, both channels' codes
+    uint32_t both[2][4], cw[4];                                        // nibble i of word j: token 8j + i; cw: both channels' codes
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const uint32_t kx = pair_bits(top[KT]), kn = pair_bits(bot[KB]);
@@ -889,7 +933,6 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
                     const float y = __saturatef(__fmaf_rn(c ? P::hi(x) : P::lo(x), inv4, off));
                     acc[j] += __float_as_uint(__fmaf_rn(y, 4.f, 12582912.f)) * (1u << (4 * i));
                 }
-                acc[j] -= (acc[j] >> 2) & 0x11111111u;                 // 4 (saturated) is code 3
             }
         } else {
             const bool by_mul = p.use_pow2 && e[c] >= -126 && e[c] <= 126;
@@ -906,8 +949,10 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
             }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) cw[j] |= acc[j] << (2 * c);
+        for (int j = 0; j < 4; ++j) both[c][j] = acc[j];
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) cw[j] = join_codes(both[0][j], both[1][j]);
 
     // ---- outlier values, read back in token order ----
     float ms[2] = {0.f, 0.f}, mc[2] = {0.f, 0.f};
@@ -921,7 +966,7 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
             for (int r = 0; r < K; ++r) {
                 const int t = __ffs(m) - 1;
                 m &= m - 1u;
-                raw[c][r] = *reinterpret_cast<const uint16_t *>(col + c + rows.at(t));
+                raw[c][r] = *reinterpret_cast<const uint16_t *>(rows.from(col + c, t));
             }
         }
 #pragma unroll
@@ -945,7 +990,7 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
 
     // ---- per-channel planes: two adjacent entries a lane ----
     if (slot >= 0) {
-        const int64_t off = ((int64_t)slot * p.H + h) * p.D + 64 * blk + 2 * lane;
+        const int64_t off = (int64_t)((uint64_t)(uint32_t)(slot * p.H + h) * (uint32_t)p.D + (uint32_t)(64 * blk + 2 * lane));
         auto put16 = [&](void *plane, float a, float b) {
             if (store_f32) *reinterpret_cast<float2 *>(reinterpret_cast<float *>(plane) + off) = make_float2(a, b);
             else *reinterpret_cast<uint32_t *>(reinterpret_cast<uint16_t *>(plane) + off) = f32_to_bf16_bits(a) | (f32_to_bf16_bits(b) << 16);
@@ -994,20 +1039,20 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
         g = __shfl_xor_sync(0xFFFFFFFFu, __byte_perm(a, b, up2 ? 0x6420u : 0x7531u), 2);
         a = __byte_perm(a, g, up2 ? 0x3514u : 0x5240u);
         b = __byte_perm(b, g, up2 ? 0x3716u : 0x7260u);
-        g = __shfl_xor_sync(0xFFFFFFFFu, up1 ? ((a & 0x0F0F0F0Fu) | ((b << 4) & 0xF0F0F0F0u)) : (((a >> 4) & 0x0F0F0F0Fu) | (b & 0xF0F0F0F0u)), 1);
-        a = up1 ? ((a & 0xF0F0F0F0u) | (g & 0x0F0F0F0Fu)) : ((a & 0x0F0F0F0Fu) | ((g << 4) & 0xF0F0F0F0u));
-        b = up1 ? ((b & 0xF0F0F0F0u) | ((g >> 4) & 0x0F0F0F0Fu)) : ((b & 0x0F0F0F0Fu) | (g & 0xF0F0F0F0u));
+        const uint32_t keep = up1 ? 0xF0F0F0F0u : 0x0F0F0F0Fu, sa = up1 ? 0u : 4u, sb = 4u - sa;
+        g = __shfl_xor_sync(0xFFFFFFFFu, ((a >> sa) & 0x0F0F0F0Fu) | ((b << sb) & 0xF0F0F0F0u), 1);
+        a = (a & keep) | ((g << sa) & ~keep);
+        b = (b & keep) | ((g >> sb) & ~keep);
     }
     // lane = token now: its 16 code bytes of these 64 channels
     if (page >= 0)
-        *reinterpret_cast<uint4 *>(p.k_base + (((int64_t)page * p.page_size + lane % p.page_size) * p.H + h) * (p.D / 4) + 16 * blk) =
+        *reinterpret_cast<uint4 *>(p.k_base + (uint64_t)(uint32_t)((page * p.page_size + in_page) * p.H + h) * (uint32_t)(p.D / 4) + 16 * blk) =
             make_uint4(cw[0], cw[1], cw[2], cw[3]);
 }
 
-// V: one thread per (token, kv head, 32 channels), 64 contiguous bytes at `row`; loc = destination (page row * H + head), negative:
-// not written
+// V: one thread per (token, kv head, 32 channels), 64 contiguous bytes at `row`; loc = destination (page row * H + head)
 template <typename T>
-__device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row, int64_t loc, int cg) {
+__device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row, uint32_t loc, bool write, int cg) {
     typedef Pair16<T> P;
     typedef typename P::V V;
     uint32_t w[16];
@@ -1020,7 +1065,7 @@ __device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row,
 #pragma unroll
     for (int i = 1; i < 16; ++i) { hi2 = __hmax2_nan(hi2, as_pair<V>(w[i])); lo2 = __hmin2_nan(lo2, as_pair<V>(w[i])); }
     const uint32_t hb = pair_bits(hi2), lb = pair_bits(lo2);
-    const bool bad = half_is_special(hb, P::EXP) || half_is_special(lb, P::EXP);
+    const bool bad = any_special(hb, lb, P::EXP);
     const float mx = fmaxf(P::lo(hb), P::hi(hb)), mn = fminf(P::lo(lb), P::hi(lb)) + 0.f;
     int e;
     const float scale = snap_scale(__fsub_rn(mx, mn), p.use_pow2, p.scale_kind, e);
@@ -1029,15 +1074,15 @@ __device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row,
     const float inv4 = __uint_as_float((uint32_t)(125 - e) << 23), off = -zp * inv4;        // see pack_k_pair
     uint32_t code[2] = {0u, 0u};
     if (p.use_pow2 && e >= -120 && e <= 120 && fabsf(off) < 1e38f) {
-        constexpr uint32_t MAGIC_SUM = 0x4B400000u * 0x55555555u;
+        constexpr uint32_t MAGIC_SUM = 0x4B400000u * 0x11111111u;
+        uint32_t acc[2][2] = {{0u - MAGIC_SUM, 0u - MAGIC_SUM}, {0u - MAGIC_SUM, 0u - MAGIC_SUM}};      // nibbles: even channels, odd ones
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-            const float x = i & 1 ? P::hi(w[i >> 1]) : P::lo(w[i >> 1]);
-            const float y = fminf(__saturatef(__fmaf_rn(x, inv4, off)), 0.75f);
-            code[i >> 4] += __float_as_uint(__fmaf_rn(y, 4.f, 12582912.f)) * (1u << (2 * (i & 15)));
+            const float y = __saturatef(__fmaf_rn(i & 1 ? P::hi(w[i >> 1]) : P::lo(w[i >> 1]), inv4, off));
+            acc[i >> 4][i & 1] += __float_as_uint(__fmaf_rn(y, 4.f, 12582912.f)) * (1u << (4 * ((i & 15) >> 1)));
         }
-        code[0] -= MAGIC_SUM;
-        code[1] -= MAGIC_SUM;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) code[v] = join_codes(acc[v][0], acc[v][1]);
     } else {
         const bool by_mul = p.use_pow2 && e >= -126 && e <= 126;
         const float inv = __uint_as_float((uint32_t)(by_mul ? 127 - e : 127) << 23);
@@ -1048,9 +1093,9 @@ __device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row,
         }
     }
     if (bad) or_status(p.status, OMMX_ST_NONFINITE);
-    if (loc < 0) return;
-    *reinterpret_cast<uint2 *>(p.v_main + loc * (p.D / 4) + cg * 8) = make_uint2(code[0], code[1]);
-    const int64_t at = loc * (p.D / 32) + cg;
+    if (!write) return;
+    const uint64_t at = (uint64_t)loc * (uint32_t)(p.D / 32) + (uint32_t)cg;
+    *reinterpret_cast<uint2 *>(p.v_main + 8 * at) = make_uint2(code[0], code[1]);
     if (p.scale_kind == OMMX_SCALE_INT8_EXP) reinterpret_cast<int8_t *>(p.v_scale)[at] = (int8_t)e;
     else if (p.scale_kind == OMMX_SCALE_BF16) reinterpret_cast<uint16_t *>(p.v_scale)[at] = (uint16_t)f32_to_bf16_bits(scale);
     else reinterpret_cast<float *>(p.v_scale)[at] = scale;
@@ -1058,35 +1103,53 @@ __device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row,
     else reinterpret_cast<uint16_t *>(p.v_zp)[at] = (uint16_t)f32_to_bf16_bits(zp);
 }
 
-// K and V of a block in one launch: the first `k_blocks` CTAs take K (the longer work), the rest V and fill the last wave.
+// n / d for n < 2^31 by one multiplication: mul = ceil(2^(31 + shift) / d) with 2^shift >= d (Granlund and Montgomery, "Division by
+// invariant integers using multiplication", 1994).  A thread takes five such quotients; as plain divisions, one of them 64 bits wide,
+// they were a third of a V thread's instructions.
+struct FastDiv {
+    uint32_t d, mul, shift;
+    __host__ __device__ __forceinline__ uint32_t quotient(uint32_t n) const {
+#ifdef __CUDA_ARCH__
+        return __umulhi(2u * n, mul) >> shift;
+#else
+        return (uint32_t)(((uint64_t)(2u * n) * mul) >> 32) >> shift;
+#endif
+    }
+};
+static FastDiv fast_div(uint32_t d) {
+    uint32_t shift = 0;
+    while ((1ull << shift) < d) ++shift;
+    return FastDiv{d, (uint32_t)(((1ull << (31 + shift)) + d - 1) / d), shift};
+}
+struct PackDivs { FastDiv heads, page, blocks, groups; };           // by H, page_size, D / 64, D / 32
+
+// K and V of a block in one launch: the first `k_blocks` CTAs take K (the longer work), the rest V and fill the last wave (in turn with
+// them, one or two K to a V, K ends late: 8192 tokens x 8 heads 17.2 -> 18.4 and 19.6 us).
+constexpr int PACK16_CTAS = 7;                     // to an SM: 72 registers a thread
 template <typename T, int KT, int KB>
-__global__ void __launch_bounds__(PACK_WARPS * 32, 7) pack16_kernel(const PackKParams kp, const PackVParams vp, int k_blocks) {
+__global__ void __launch_bounds__(PACK_WARPS * 32, PACK16_CTAS) pack16_kernel(const PackKParams kp, const PackVParams vp, const PackDivs by, uint32_t k_blocks) {
     const int lane = threadIdx.x & 31;
-    if ((int)blockIdx.x < k_blocks) {
-        const int nblk = kp.D / 64;
-        const int unit = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5);        // (group, head, 64-channel half)
-        if (unit >= kp.num_groups * kp.H * nblk) return;
-        const int blk = unit % nblk, gh = unit / nblk, g = gh / kp.H, h = gh - g * kp.H;
-        int slot = kp.dst_groups ? kp.dst_groups[g] : g;
-        const int tok = g * 32 + lane;
-        int page = tok / kp.page_size;
-        if (kp.dst_pages) page = kp.dst_pages[page];
+    if (blockIdx.x < k_blocks) {
+        const uint32_t unit = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5);   // (group, head, 64-channel half)
+        const uint32_t gh = by.blocks.quotient(unit), blk = unit - gh * by.blocks.d, g = by.heads.quotient(gh), h = gh - g * by.heads.d;
+        if (g >= (uint32_t)kp.num_groups) return;
+        int slot = kp.dst_groups ? kp.dst_groups[g] : (int)g;
+        const uint32_t tok = g * 32 + lane, p0 = by.page.quotient(tok);
+        int page = kp.dst_pages ? kp.dst_pages[p0] : (int)p0;
         if (slot < 0 || slot >= kp.num_group_slots) { if (lane == 0) or_status(kp.status, OMMX_ST_BAD_GROUP); slot = -1; }
         if (page < 0 || page >= kp.num_pages) { or_status(kp.status, OMMX_ST_BAD_PAGE); page = -1; }
         const T *col = reinterpret_cast<const T *>(kp.k) + (int64_t)(g * 32) * kp.stride_token + (int64_t)h * kp.stride_head + blk * 64 + 2 * lane;
-        pack_k_pair<T, KT, KB>(kp, col, GroupRows{kp.stride_token, 32, 0}, slot, h, blk, page, lane);
+        pack_k_pair<T, KT, KB>(kp, col, GroupRows{(int32_t)kp.stride_token, 32, 0}, slot, h, blk, page, tok - p0 * by.page.d, lane);
     } else {
-        const int ngv = vp.D / 32;
-        const int64_t idx = (int64_t)(blockIdx.x - k_blocks) * blockDim.x + threadIdx.x;
-        if (idx >= (int64_t)vp.num_tokens * vp.H * ngv) return;
-        const int cg = (int)(idx % ngv);
-        const int64_t th = idx / ngv;
-        const int t = (int)(th / vp.H), h = (int)(th - (int64_t)t * vp.H);
-        int page = t / vp.page_size;
-        if (vp.dst_pages) page = vp.dst_pages[page];
-        int64_t loc = ((int64_t)page * vp.page_size + t % vp.page_size) * vp.H + h;
-        if (page < 0 || page >= vp.num_pages) { or_status(vp.status, OMMX_ST_BAD_PAGE); loc = -1; }
-        pack_v_group<T>(vp, reinterpret_cast<const T *>(vp.v) + (int64_t)t * vp.stride_token + (int64_t)h * vp.stride_head + cg * 32, loc, cg);
+        const uint32_t idx = (blockIdx.x - k_blocks) * (PACK_WARPS * 32) + threadIdx.x;
+        const uint32_t th = by.groups.quotient(idx), cg = idx - th * by.groups.d, t = by.heads.quotient(th), h = th - t * by.heads.d;
+        if (t >= (uint32_t)vp.num_tokens) return;
+        const uint32_t p0 = by.page.quotient(t);
+        const int page = vp.dst_pages ? vp.dst_pages[p0] : (int)p0;
+        const bool write = page >= 0 && page < vp.num_pages;
+        if (!write) or_status(vp.status, OMMX_ST_BAD_PAGE);
+        pack_v_group<T>(vp, reinterpret_cast<const T *>(vp.v) + (int64_t)t * vp.stride_token + (int64_t)h * vp.stride_head + cg * 32,
+                        ((uint32_t)page * by.page.d + (t - p0 * by.page.d)) * by.heads.d + h, write, cg);
     }
 }
 
@@ -1112,21 +1175,25 @@ static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
     vp.v_main = (uint8_t *)pl.v_main; vp.v_scale = pl.v_scale; vp.v_zp = pl.v_zp; vp.status = a->status;
     const int64_t nthreads = (int64_t)a->num_tokens * pl.n_kv_heads * (pl.head_dim / 32);
     if constexpr (sizeof(T) == 2) {
-        // The serving form: channel pairs need whole 64-channel units and rows whose 16-byte pieces are aligned
+        // The serving form: channel pairs need whole 64-channel units and rows whose 16-byte pieces are aligned, and its counts are 32 bits
+        // wide (2^31 pieces of a V row are more than a device holds, unless rows of K and V alias)
         const uintptr_t all = (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)pl.k_base | (uintptr_t)pl.k_scale | (uintptr_t)pl.k_zp | (uintptr_t)pl.k_obmp |
                               (uintptr_t)pl.k_oval | (uintptr_t)pl.k_mapscale | (uintptr_t)pl.k_mapcenter;
         const int k = kp.k_out;
         if (kp.select_signed && kp.D % 64 == 0 && all % 16 == 0 && a->stride_token % 8 == 0 && a->stride_head % 8 == 0 &&
-            (k == 0 || k == 2 || k == 4 || k == 6 || k == 8)) {
+            a->stride_token >= 0 && a->stride_token < (1 << 25) &&
+            (k == 0 || k == 2 || k == 4 || k == 6 || k == 8) && nthreads < (1ll << 31) - 128 && (int64_t)pl.num_pages * pl.page_size * kp.H < (1ll << 32) &&
+            (int64_t)pl.num_group_slots * kp.H < (1ll << 32)) {
             if (nthreads == 0) return 0;
+            const PackDivs by{fast_div(kp.H), fast_div(kp.page_size), fast_div(kp.D / 64), fast_div(kp.D / 32)};
             const int k_blocks = (kp.num_groups * kp.H * (kp.D / 64) + PACK_WARPS - 1) / PACK_WARPS;
             const unsigned grid = (unsigned)(k_blocks + (nthreads + 127) / 128);
             switch (k) {
-                case 0: pack16_kernel<T, 0, 0><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
-                case 2: pack16_kernel<T, 1, 1><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
-                case 4: pack16_kernel<T, 2, 2><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
-                case 6: pack16_kernel<T, 3, 3><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
-                default: pack16_kernel<T, 4, 4><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, k_blocks); break;
+                case 0: pack16_kernel<T, 0, 0><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
+                case 2: pack16_kernel<T, 1, 1><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
+                case 4: pack16_kernel<T, 2, 2><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
+                case 6: pack16_kernel<T, 3, 3><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
+                default: pack16_kernel<T, 4, 4><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
             }
             OMMX_CUDA_TRY(cudaGetLastError());
             count_launch();
@@ -1393,16 +1460,16 @@ __global__ void __cluster_dims__(STORE_CTAS, 1, 1) __launch_bounds__(STORE_THREA
             if (page < 0 || page >= kp.num_pages) { or_status(p.status, OMMX_ST_BAD_PAGE); page = -1; }
             for (int unit = rank + STORE_CTAS * warp; unit < p.H * nblk; unit += STORE_CTAS * (STORE_THREADS / 64)) {
                 const int h = unit / nblk, blk = unit - h * nblk;
-                pack_k_pair<T, KT, KB>(kp, p.k_hist + base + h * p.D + 64 * blk + 2 * lane, rows, slot, h, blk, page, lane);
+                pack_k_pair<T, KT, KB>(kp, p.k_hist + base + h * p.D + 64 * blk + 2 * lane, rows, slot, h, blk, page, lane % kp.page_size, lane);
             }
         } else {
             const int ngv = p.D / 32;
             for (int x = rank * (STORE_THREADS / 2) + (int)threadIdx.x - STORE_THREADS / 2; x < 32 * p.H * ngv; x += STORE_CTAS * (STORE_THREADS / 2)) {
                 const int cg = x % ngv, th = x / ngv, h = th % p.H, t = th / p.H;
                 const int page = pages[(grp * 32 + t) / vp.page_size];
-                int64_t loc = ((int64_t)page * vp.page_size + t % vp.page_size) * p.H + h;
-                if (page < 0 || page >= vp.num_pages) { or_status(p.status, OMMX_ST_BAD_PAGE); loc = -1; }
-                pack_v_group<T>(vp, p.v_hist + base + rows.at(t) + h * p.D + cg * 32, loc, cg);
+                const bool write = page >= 0 && page < vp.num_pages;
+                if (!write) or_status(p.status, OMMX_ST_BAD_PAGE);
+                pack_v_group<T>(vp, p.v_hist + base + rows.at(t) + h * p.D + cg * 32, (uint32_t)(page * vp.page_size + t % vp.page_size) * p.H + h, write, cg);
             }
         }
     }

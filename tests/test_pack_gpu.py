@@ -190,3 +190,28 @@ def test_pack_fp32_inputs_with_ties(k, D, H):
         bad[37, 0, 5] = value
         with pytest.raises(ValueError):
             _gpu_pack(bad, V, k=k)
+
+
+@pytest.mark.parametrize("T,H,D,ps", [(32, 7, 64, 8), (96, 5, 192, 96), (224, 3, 128, 32), (2048, 11, 128, 16)])
+def test_pack_16_bit_geometries(T, H, D, ps):
+    """Counts that no power of two divides: heads, 64-channel units, pages of several groups; the last CTAs partly full."""
+    K, V = gaussian_kv(T + H, T, H, D)
+    want = O.pack_kv(K.numpy(), V.numpy(), page_size=ps)
+    assert_planes_equal(_gpu_pack(K.bfloat16(), V.bfloat16(), ps=ps), want, ctx=f"T={T} H={H} D={D} ps={ps}:")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_pack_16_bit_inputs_report_what_is_not_finite(dtype, value):
+    """In either half of a register, K and V; the largest finite value is not one of them."""
+    K, V = (x.to(dtype) for x in gaussian_kv(7, 64, 2, 128))
+    top = torch.finfo(dtype).max if dtype == torch.float16 else 1e38
+    for t, c in ((3, 6), (33, 127)):
+        for X in (K, V):
+            keep = X[t, 1, c].clone()
+            X[t, 1, c] = top
+            _gpu_pack(K, V)
+            X[t, 1, c] = value
+            with pytest.raises(ValueError):
+                _gpu_pack(K, V)
+            X[t, 1, c] = keep
