@@ -1124,10 +1124,14 @@ static FastDiv fast_div(uint32_t d) {
 struct PackDivs { FastDiv heads, page, blocks, groups; };           // by H, page_size, D / 64, D / 32
 
 // K and V of a block in one launch: the first `k_blocks` CTAs take K (the longer work), the rest V and fill the last wave (in turn with
-// them, one or two K to a V, K ends late: 8192 tokens x 8 heads 17.2 -> 18.4 and 19.6 us).
+// them, one or two K to a V, K ends late: 8192 tokens x 8 heads 17.2 -> 18.4 and 19.6 us).  let_next_in: a dependent launch may be placed as
+// soon as all CTAs are; where they take less than two waves on a B200's 148 SMs, it would fill the SMs unevenly (2048 tokens 7.3 -> 10.4 us, 4096
+// 9.6 -> 10.8; 6144 12.0 -> 11.8, 8192 14.5 -> 14.2).
 constexpr int PACK16_CTAS = 7;                     // to an SM: 72 registers a thread
 template <typename T, int KT, int KB>
-__global__ void __launch_bounds__(PACK_WARPS * 32, PACK16_CTAS) pack16_kernel(const PackKParams kp, const PackVParams vp, const PackDivs by, uint32_t k_blocks) {
+__global__ void __launch_bounds__(PACK_WARPS * 32, PACK16_CTAS) pack16_kernel(const PackKParams kp, const PackVParams vp, const PackDivs by, uint32_t k_blocks, int let_next_in) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");                 // placed while the kernel before it drains
+    if (let_next_in) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     if (blockIdx.x < k_blocks) {
         const uint32_t unit = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5);   // (group, head, 64-channel half)
@@ -1151,6 +1155,22 @@ __global__ void __launch_bounds__(PACK_WARPS * 32, PACK16_CTAS) pack16_kernel(co
         pack_v_group<T>(vp, reinterpret_cast<const T *>(vp.v) + (int64_t)t * vp.stride_token + (int64_t)h * vp.stride_head + cg * 32,
                         ((uint32_t)page * by.page.d + (t - p0 * by.page.d)) * by.heads.d + h, write, cg);
     }
+}
+
+// Launch as a programmatic dependent: the grid is placed while the kernel before it in the stream drains, and waits for that kernel's end
+// (griddepcontrol.wait) before it touches memory.  Packs one after the other, called from Python: 8192 tokens x 8 heads 16.4 -> 15.0 us, a
+// small one 6.15 -> 4.2; eight prompts of 1333 tokens and 32 steps, with the ring's rows behind each pack, 837 -> 815.
+template <typename... P> static cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, P... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <typename T>
@@ -1188,14 +1208,9 @@ static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
             const PackDivs by{fast_div(kp.H), fast_div(kp.page_size), fast_div(kp.D / 64), fast_div(kp.D / 32)};
             const int k_blocks = (kp.num_groups * kp.H * (kp.D / 64) + PACK_WARPS - 1) / PACK_WARPS;
             const unsigned grid = (unsigned)(k_blocks + (nthreads + 127) / 128);
-            switch (k) {
-                case 0: pack16_kernel<T, 0, 0><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
-                case 2: pack16_kernel<T, 1, 1><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
-                case 4: pack16_kernel<T, 2, 2><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
-                case 6: pack16_kernel<T, 3, 3><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
-                default: pack16_kernel<T, 4, 4><<<grid, PACK_WARPS * 32, 0, st>>>(kp, vp, by, k_blocks); break;
-            }
-            OMMX_CUDA_TRY(cudaGetLastError());
+            void (*const kernel)(PackKParams, PackVParams, PackDivs, uint32_t, int) =
+                k == 0 ? pack16_kernel<T, 0, 0> : (k == 2 ? pack16_kernel<T, 1, 1> : (k == 4 ? pack16_kernel<T, 2, 2> : (k == 6 ? pack16_kernel<T, 3, 3> : pack16_kernel<T, 4, 4>)));
+            OMMX_CUDA_TRY(launch_early(kernel, dim3(grid), PACK_WARPS * 32, st, kp, vp, by, (uint32_t)k_blocks, grid >= 2u * PACK16_CTAS * 148u ? 1 : 0));
             count_launch();
             return 0;
         }
@@ -1481,16 +1496,7 @@ __global__ void __cluster_dims__(STORE_CTAS, 1, 1) __launch_bounds__(STORE_THREA
 
 template <int KT, int KB>
 static int launch_store(const StoreParams &sp, const PackKParams &kp, const PackVParams &vp, int B, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(STORE_CTAS, B);
-    cfg.blockDim = dim3(STORE_THREADS);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // placed while the kernel before it drains, waits for it before any access
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    OMMX_CUDA_TRY(cudaLaunchKernelEx(&cfg, kv_store_kernel<KT, KB>, sp, kp, vp));
+    OMMX_CUDA_TRY(launch_early(kv_store_kernel<KT, KB>, dim3(STORE_CTAS, B), STORE_THREADS, st, sp, kp, vp));
     count_launch();
     return 0;
 }
@@ -1505,6 +1511,8 @@ struct FillParams {
     int32_t *seq_len;
 };
 __global__ void __launch_bounds__(256) kv_fill_ring_kernel(FillParams p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.seq_len = p.T;
     const int tok = (int)blockIdx.x < p.n_sink ? blockIdx.x : p.lo + ((int)blockIdx.x - p.n_sink);
     if (tok >= p.T) return;
@@ -1814,8 +1822,7 @@ extern "C" int ommx_b200_kv_append_block(const ommx_kv_pool *pool, int32_t slot,
     f.vec = all % 16 == 0 && stride_token % 8 == 0 && stride_head % 8 == 0 && f.D % 8 == 0;
     f.seq_len = pool->seq_len + slot;
     const int rows = f.n_sink + (num_tokens > f.lo ? num_tokens - f.lo : 0);
-    kv_fill_ring_kernel<<<rows > 0 ? rows : 1, 256, 0, st>>>(f);
-    OMMX_CUDA_TRY(cudaGetLastError());
+    OMMX_CUDA_TRY(launch_early(kv_fill_ring_kernel, dim3(rows > 0 ? rows : 1), 256, st, f));
     count_launch();
     return 0;
 }
