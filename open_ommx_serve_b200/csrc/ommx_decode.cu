@@ -437,16 +437,16 @@ static EncodeTiledFn encode_tiled_fn() {
     return st == 1 ? fn : nullptr;
 }
 
-// Plane viewed as [bytes/128][128] uint8, box = one page, 128-byte swizzle.  Returns false when the
-// map cannot be built.
-// Encoded maps are kept in a small table keyed by (base, bytes, box rows): a serving loop calls with the
+// box_rows > 0: the plane viewed as [bytes/128][128] uint8, box = one page, 128-byte swizzle.  box_rows = 0: the plane viewed as
+// [bytes/row_bytes][row_bytes], box = one row as it lies (for loads of four rows).  Returns false when the map cannot be built.
+// Encoded maps are kept in a small table keyed by (base, bytes, box): a serving loop calls with the
 // same planes every step and the driver call costs about a microsecond.
-static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes, int rows_per_page) {
+static bool make_map(CUtensorMap *m, const void *base, int64_t total_bytes, int row_bytes, int box_rows) {
     EncodeTiledFn fn = encode_tiled_fn();
-    if (fn == nullptr || total_bytes < 128 || rows_per_page < 8 || rows_per_page > 256) return false;
-    // 512 sets x 4 ways, keyed by (device, base, bytes, box rows) and compared in full; a set that is
-    // full evicts round-robin.  2048 entries hold the two code planes of a 1000-layer model.
-    struct Entry { const void *base; int64_t bytes; int rows, dev; CUtensorMap map; };
+    if (fn == nullptr || total_bytes < row_bytes || row_bytes % 16 != 0 || row_bytes > GATHER_ROW_MAX || box_rows > 256) return false;
+    // 512 sets x 4 ways, keyed by (device, base, bytes, box) and compared in full; a set that is
+    // full evicts round-robin.  2048 entries hold the two code planes of a 1000-layer model, all ten planes of 200 layers.
+    struct Entry { const void *base; int64_t bytes; int row, rows, dev; CUtensorMap map; };
     constexpr int SETS = 512, WAYS = 4;
     static Entry table[SETS][WAYS];
     static uint8_t next_way[SETS];
@@ -459,21 +459,35 @@ static bool make_code_map(CUtensorMap *m, const void *base, int64_t total_bytes,
         std::lock_guard<std::mutex> g(mu);
         for (int w = 0; w < WAYS; ++w) {
             const Entry &e = table[set][w];
-            if (e.base == base && e.bytes == total_bytes && e.rows == rows_per_page && e.dev == dev) { *m = e.map; return true; }
+            if (e.base == base && e.bytes == total_bytes && e.row == row_bytes && e.rows == box_rows && e.dev == dev) { *m = e.map; return true; }
         }
     }
-    cuuint64_t gdim[2] = {128, (cuuint64_t)(total_bytes / 128)};
-    cuuint64_t gstride[1] = {128};
-    cuuint32_t box[2] = {128, (cuuint32_t)rows_per_page};
+    // a box is at most 256 elements wide
+    const int element = row_bytes <= 256 ? 1 : (row_bytes <= 1024 ? 4 : 8);
+    const CUtensorMapDataType type = element == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : (element == 4 ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_INT64);
+    cuuint64_t gdim[2] = {(cuuint64_t)(row_bytes / element), (cuuint64_t)(total_bytes / row_bytes)};
+    cuuint64_t gstride[1] = {(cuuint64_t)row_bytes};
+    cuuint32_t box[2] = {(cuuint32_t)(row_bytes / element), (cuuint32_t)max(box_rows, 1)};
     cuuint32_t estr[2] = {1, 1};
-    if (fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), gdim, gstride, box, estr,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    if (fn(m, type, 2, const_cast<void *>(base), gdim, gstride, box, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, box_rows > 0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     std::lock_guard<std::mutex> g(mu);
     Entry &e = table[set][next_way[set]];
     next_way[set] = (uint8_t)((next_way[set] + 1) % WAYS);
-    e.base = base; e.bytes = total_bytes; e.rows = rows_per_page; e.dev = dev; e.map = *m;
+    e.base = base; e.bytes = total_bytes; e.row = row_bytes; e.rows = box_rows; e.dev = dev; e.map = *m;
+    return true;
+}
+
+bool make_row_maps(S1GatherParams &p, bool with_index) {
+    const uint8_t *base[10] = {p.k_base, p.v_main, p.v_scale, p.v_zp, p.k_scale, p.k_zp, p.k_ms, p.k_mc, p.k_obmp, p.k_oval};
+    const int page = p.ps * p.H, slot = 128 * p.H, page_split = gather_page_split(p.GS * p.ppg), slot_split = gather_slot_split(p.H);
+    const int bytes[10] = {32 * page, 32 * page, 4 * page, 8 * page, slot, 2 * slot, 2 * slot, 2 * slot, p.nbi * slot, p.nb * slot};
+    for (int i = p.H == 4 ? 2 : 0; i < (p.k_out > 0 ? 10 : 6); ++i)
+        if (i != 8 || with_index)
+            if (!make_map(&p.rows[i], base[i], (int64_t)bytes[i] * (i < 4 ? p.num_pages : p.num_slots), bytes[i] / (i < 4 ? page_split : slot_split), 0))
+                return false;
     return true;
 }
 
@@ -485,7 +499,7 @@ __global__ void whole_sm_kernel() {}
 static int clusters_at_once(int cluster, int *n) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster);
-    cfg.blockDim = dim3(WarpLayout<8>::THREADS);
+    cfg.blockDim = dim3(WarpLayout<8, false>::THREADS);
     cfg.dynamicSmemBytes = SMEM_LIMIT;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -581,14 +595,14 @@ static int fill_stage1(const ommx_decode_args *a, S1Params &p) {
     memset(&p.tmap_k, 0, sizeof(CUtensorMap));
     memset(&p.tmap_v, 0, sizeof(CUtensorMap));
     if (H >= 4) {                                                        // a page is whole 1 KB swizzle atoms
-        if (!make_code_map(&p.tmap_k, pl.k_base, (int64_t)pl.num_pages * page_bytes, p.rows_per_page) ||
-            !make_code_map(&p.tmap_v, pl.v_main, (int64_t)pl.num_pages * page_bytes, p.rows_per_page))
+        if (!make_map(&p.tmap_k, pl.k_base, (int64_t)pl.num_pages * page_bytes, 128, p.rows_per_page) ||
+            !make_map(&p.tmap_v, pl.v_main, (int64_t)pl.num_pages * page_bytes, 128, p.rows_per_page))
             return fail(OMMX_E_CUDA, "stage 1: the tensor maps of the code planes could not be encoded");
         p.swz = 0x70u;
     }
     const int round_to = p.swz ? 1024 : 128;
     p.gb_bytes = (p.gb_bytes + round_to - 1) / round_to * round_to;
-    p.stage_bytes = p.GS * p.gb_bytes;
+    p.stage_bytes = (p.GS * p.gb_bytes + 1023) / 1024 * 1024;
     p.abl = a->abl_flags;
     return 0;
 }

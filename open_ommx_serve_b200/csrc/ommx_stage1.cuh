@@ -6,17 +6,20 @@
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 
 namespace ommx {
 
 constexpr int HD = 128;                 // head_dim this build serves
 constexpr int NCW = 8;                  // (group, head) units in flight per CTA, one MMA warp each
-// Two warp layouts.  Narrow (4 or 8 local kv heads: 14 or 28 copies per ring stage): 15 decode warps + 1 producer warp,
-// which also builds the last tile half once its copies are out.  Wide (1 or 2 local kv heads: a stage is 8 or 4 groups,
-// 112 or 56 small copies): 16 decode warps + 4 producer warps, because one warp issues a bulk copy only every ~60 cycles
-// and the issues of different warps overlap (112 copies: 6400 cycles from one warp, 2000 from four).
-template <int H> struct WarpLayout {
-    static constexpr bool WIDE = H <= 2;
+// Two warp layouts.  Narrow (2, 4 or 8 local kv heads: 14 to 16 copies per ring stage): 15 decode warps + 1 producer warp,
+// which also builds the last tile half once its copies are out.  Wide (1 local kv head: a stage is 8 groups, 28 copies; in the
+// general form, which copies page by page and slot by slot, 112, and 56 with 2 heads): 16 decode warps + 4 producer warps, because
+// one warp issues a copy only every ~60 cycles on an idle SM, three times that beside the other roles, and the issues of different
+// warps overlap.  One producer keeps up with about 20 copies a stage: 8 x 32K, one head, four rows to a copy 31.8 us by one
+// producer and 31.0 by four; 128K, two heads, 14 copies 28.2 and 28.6.
+template <int H, bool GATHER> struct WarpLayout {
+    static constexpr bool WIDE = H == 1 || (H == 2 && !GATHER);
     static constexpr int NDW = WIDE ? 16 : 15;            // decode warps (stateless sidecar builders, items dealt round-robin)
     static constexpr int NPW = WIDE ? 4 : 1;              // producer warps
     static constexpr int PRODUCER_WARP = NCW + NDW;       // the first of them
@@ -74,6 +77,20 @@ struct S1Params {
     alignas(64) CUtensorMap tmap_k;
     alignas(64) CUtensorMap tmap_v;
 };
+// One to four kv heads, plain form: a stage holds several groups, so its copies are many and small, and issuing them is what a stage
+// waits for (they go out one by one, ~30 instructions each).  Its planes are laid out for all its groups at once, so that one
+// instruction fetches four pages or group slots (`tile::gather4`): 28, 14 and 16 copies at 1, 2 and 4 heads for 112, 56 and 28.  Both
+// stages, before -> now: 128K x 2 heads 28.8 -> 28.1 us, 256K 46.1 -> 44.2; 8 x 32K x 1 head 33.9 -> 30.6, 512K 51.7 -> 44.3; 128K x 4
+// heads 46.1 -> 43.5, 32K 19.5 (no change).  Rows of two heads lie as they come (conflicts: a token row is 64 bytes): by page with a
+// swizzle they need 26 copies, 28.8 us.  Eight heads have a group to a stage and nothing to fold.
+// These are the tensor maps of the planes as they are numbered below, a page or group slot to a row.
+struct S1GatherParams : S1Params {
+    CUtensorMap rows[10];
+};
+// the planes: 0 k_base, 1 v_main, 2 v_scale, 3 v_zp by page; 4 k_scale, 5 k_zp, 6 map scale, 7 map center, 8 outlier index, 9 outlier values by slot
+constexpr int GATHER_ROW_MAX = 2048;     // bytes of a row: 256 elements of 8 bytes
+__host__ __device__ constexpr int gather_slot_split(int heads) { return heads == 4 ? 2 : 1; }          // rows of a group slot
+__host__ __device__ constexpr int gather_page_split(int stage_pages) { return stage_pages < 4 ? 2 : 1; }   // of a page (planes 2 and 3)
 
 // One bulk copy of a stage: source plane, bytes, destination inside the stage, and which table entry
 // (page id or group slot) selects the source block.
@@ -81,7 +98,7 @@ struct __align__(16) CopyDesc {
     const uint8_t *src;                  // plane base, or nullptr + kind for a tensor-map copy
     uint32_t unit, dst;
     int32_t tbase, tmul, gi, tok0;       // gi: group in stage (bits 0..7) | kind << 8
-};                                       // kind 0 bulk copy, 1 k_base through tmap_k, 2 v_main through tmap_v
+};                                       // kind 0 bulk copy, 1 k_base through tmap_k, 2 v_main through tmap_v, 3 + n four rows of plane n
 // a stage holds at most 8 groups x (4 planes x 4 pages + 6 group planes) = 176 copies (1 kv head, 8-token pages)
 
 // ---- PTX wrappers --------------------------------------------------------------------------------
@@ -236,6 +253,12 @@ __device__ __forceinline__ uint32_t swz128(uint32_t o, uint32_t swz) { return o 
 __device__ __forceinline__ void tma_2d_g2s(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+
+// four rows of a plane, one after the other in shared memory
+__device__ __forceinline__ void tma_rows_g2s(uint32_t dst, const CUtensorMap *map, const int4 &row, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                 ::"r"(dst), "l"(map), "r"(0), "r"(row.x), "r"(row.y), "r"(row.z), "r"(row.w), "r"(bar) : "memory");
 }
 
 __device__ __forceinline__ int64_t load_index(const void *tbl, int is64, int64_t i) {
@@ -568,32 +591,48 @@ constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_
 // at four warps a scheduler); 16 delta warps with their own MMAs beside 8 output warps (46.1 / 167); tile rows zeroed by an
 // out-of-range tensor-map load (83 / 289); FP4 levels by the conversion instruction and a shorter wait loop (53 fewer
 // instructions per unit, same time).
-// With one or two kv heads a unit costs more: 1966 and 1792 instructions and 507 and 498 wavefronts (176 and 178 of them bank conflicts,
-// 111 at eight heads), because a page of theirs is staged as it lies, without a swizzle, and a stage takes 112 or 56 copies.
-//
 // PLAIN: the recipes that are served - bitmask or relidx7 index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
 // form keeps them at run time; its tests and address arithmetic inside the unit cost it 12 to 15 % (both stages: 64K
-// 46.1 us against 41.0, 70B heads 8 x 32K 155.4 against 135.5; one and two kv heads 34.1 against 32.8 and 30.0 against 28.3).
+// 46.1 us against 41.0, 70B heads 8 x 32K 155.4 against 135.5).
 // IDX7 (plain form only): relidx7 positions instead of bitmasks, turned into masks by three instructions a position.  At run time, byte
 // by byte, they took longer than the rest of the tile: 64K x 8 heads, both stages, k = 6 66.3 -> 45.9 us, k = 12 94.9 -> 58.7.
 template <int KOUT, int H, bool IDX7> struct PlainLayout {
+    static constexpr bool GATHER = H <= 4;
+    static constexpr int GS = NCW / H;
+    static constexpr int U = GATHER ? NCW : H;                       // units to a block
     static constexpr int NB = KOUT > 0 ? (KOUT + 1) / 2 : 0, NBI = IDX7 ? (7 * KOUT + 7) / 8 : 4;
-    static constexpr int VM = H * 1024, VS = H * 2048, VZ = VS + H * 128, KS = VZ + H * 256, KZ = KS + H * 128, MS = KZ + H * 256, MC = MS + H * 256,
-                         BM = MC + H * 256, OV = BM + H * 128 * NBI;
-    static constexpr int ROUND = H >= 4 ? 1024 : 128;
-    static constexpr int GB = (OV + H * 128 * NB + ROUND - 1) / ROUND * ROUND;
-    static constexpr int STAGES = stage1_smem(4, NCW / H * GB, NCW / H, 2) <= SMEM_LIMIT ? 4 : 3;   // with 16-token pages
-    static_assert(stage1_smem(STAGES, NCW / H * GB, NCW / H, 2) <= SMEM_LIMIT, "the ring fits");
+    static constexpr int VM = U * 1024, VS = U * 2048, VZ = VS + U * 128, KS = VZ + U * 256, KZ = KS + U * 128, MS = KZ + U * 256, MC = MS + U * 256,
+                         BM = MC + U * 256, OV = BM + U * 128 * NBI;
+    static constexpr int GB = (OV + U * 128 * NB + 1023) / 1024 * 1024;
+    static constexpr int STAGE = NCW / U * GB;
+    static constexpr int STAGES = stage1_smem(4, STAGE, GS, 2) <= SMEM_LIMIT ? 4 : 3;   // with 16-token pages
+    static_assert(stage1_smem(STAGES, STAGE, GS, 2) <= SMEM_LIMIT, "the ring fits");
+    // Copies of four rows.  A row is a group slot, half of one at four heads; for page planes a page, or half of one where a stage has
+    // two.  The code planes of four heads go by page, swizzled, as does slot by slot an outlier index whose rows would be too long.
+    static constexpr int CODE_ROWS = H == 4 ? 1 : 4, SLOT_SPLIT = gather_slot_split(H), SLOT_ROWS = GS * SLOT_SPLIT;
+    static constexpr bool ROWS_FIT = H * 128 * NBI / SLOT_SPLIT <= GATHER_ROW_MAX;
+    static constexpr int GROUP_COPIES = (KOUT == 0 ? 2 : 6) * (SLOT_ROWS / 4) + (ROWS_FIT ? 0 : GS - SLOT_ROWS / 4);
+    static __host__ __device__ constexpr int copies(int pages) {
+        return 2 * (pages / CODE_ROWS) + 2 * (pages * gather_page_split(pages) / 4) + GROUP_COPIES;
+    }
+};
+template <int H, bool PLAIN> struct Stage1Form {
+    static constexpr bool GATHER = PLAIN && H <= 4;
+    typedef WarpLayout<H, GATHER> Layout;
+    typedef std::conditional_t<GATHER, S1GatherParams, S1Params> Params;
 };
 template <int KOUT, int H, bool PLAIN, bool IDX7, bool CLUSTER>
-__global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kernel(const __grid_constant__ S1Params p) {
-    constexpr bool WIDE = WarpLayout<H>::WIDE;
-    constexpr int NDW = WarpLayout<H>::NDW, NPW = WarpLayout<H>::NPW, PRODUCER_WARP = WarpLayout<H>::PRODUCER_WARP;
-    constexpr int S1_THREADS = WarpLayout<H>::THREADS;
+__global__ void __launch_bounds__(Stage1Form<H, PLAIN>::Layout::THREADS, 1)
+decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Params p) {
+    constexpr bool GATHER = Stage1Form<H, PLAIN>::GATHER;
+    typedef typename Stage1Form<H, PLAIN>::Layout Warps;
+    constexpr bool WIDE = Warps::WIDE;
+    constexpr int NDW = Warps::NDW, NPW = Warps::NPW, PRODUCER_WARP = Warps::PRODUCER_WARP;
+    constexpr int S1_THREADS = Warps::THREADS;
     constexpr int GS = NCW / H;                                     // groups per ring stage
     constexpr int TS = H * 32;                                      // bytes per token row (all heads)
-    constexpr uint32_t SWZ = H >= 4 ? 0x70u : 0u;                   // the code planes are staged through swizzled tensor maps
+    constexpr uint32_t SWZ = H >= 4 ? 0x70u : 0u;    // the code planes are staged through swizzled tensor maps
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // swizzle atoms are 1 KB: align the ring by hand (the launch adds 1 KB of slack)
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -602,7 +641,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     static_assert(!PLAIN || KOUT >= 0, "the plain form knows its outlier count");
     typedef PlainLayout<KOUT, H, IDX7> L;
     const int NS = PLAIN ? L::STAGES : p.nstages;
-    const int gb_bytes = PLAIN ? L::GB : p.gb_bytes, stage_bytes = PLAIN ? GS * L::GB : p.stage_bytes;
+    const int gb_bytes = PLAIN ? L::GB : p.gb_bytes, stage_bytes = PLAIN ? L::STAGE : p.stage_bytes;
     const int o_vm = PLAIN ? L::VM : p.o_vm, o_vs = PLAIN ? L::VS : p.o_vs, o_vz = PLAIN ? L::VZ : p.o_vz, o_ks = PLAIN ? L::KS : p.o_ks,
               o_kz = PLAIN ? L::KZ : p.o_kz, o_ms = PLAIN ? L::MS : p.o_ms, o_mc = PLAIN ? L::MC : p.o_mc, o_bm = PLAIN ? L::BM : p.o_bm,
               o_ov = PLAIN ? L::OV : p.o_ov;
@@ -631,6 +670,11 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_k)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.tmap_v)) : "memory");
     }
+    if constexpr (GATHER) {
+        const int i = (int)threadIdx.x - (S1_THREADS - 32);
+        if (i >= (L::CODE_ROWS == 1 ? 2 : 0) && i < (KOUT > 0 ? 10 : 6) && (i != 8 || L::ROWS_FIT))
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.rows[i])) : "memory");
+    }
     if (threadIdx.x < 16) {
         const int c = threadIdx.x;
         const int mi = ((c >> 1) & 3) * 2 + (c & 1);                    // exp*2 + mant
@@ -655,8 +699,47 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         }
     }
     const int cpg = 4 * p.ppg + 6;                                      // copies per group
-    const int ncopies = GS * cpg;
-    {
+    const int ppg_log = __ffs(p.ppg) - 1, stage_pages = GS << ppg_log;
+    const int page_split = H == 4 ? gather_page_split(stage_pages) : 1, page_rows = stage_pages * page_split;
+    const int ncopies = GATHER ? L::copies(stage_pages) : GS * cpg;
+    if constexpr (GATHER) {
+        const int c = (int)threadIdx.x - 64;
+        const int n_code = 2 * (stage_pages / L::CODE_ROWS), n_page = n_code + 2 * (page_rows / 4);
+        if (c >= 0 && c < ncopies) {
+            int plane, row;                                             // its first row
+            if (c < n_code) {
+                plane = c >= n_code / 2;
+                row = L::CODE_ROWS * (c - plane * (n_code / 2));
+            } else if (c < n_page) {
+                plane = 2 + (c >= (n_code + n_page) / 2);
+                row = 4 * (c - (plane == 2 ? n_code : (n_code + n_page) / 2));
+            } else {
+                const int x = c - n_page;
+                constexpr int Q = L::SLOT_ROWS / 4, FIRST = 4 * Q;      // k_scale, k_zp, map scale, map center; then index, values
+                constexpr int Q8 = L::ROWS_FIT ? Q : GS;
+                plane = x < FIRST ? 4 + x / Q : (x < FIRST + Q8 ? 8 : 9);
+                row = plane < 8 ? 4 * (x % Q) : (plane == 8 ? (L::SLOT_ROWS / Q8) * (x - FIRST) : 4 * (x - FIRST - Q8));
+            }
+            const bool by_page = plane < 4, single = (plane < 2 && L::CODE_ROWS == 1) || (plane == 8 && !L::ROWS_FIT);
+            const int split = by_page ? (plane < 2 ? 1 : page_split) : L::SLOT_SPLIT;
+            const uint32_t bytes = (by_page ? (uint32_t)p.ps * H * (plane < 2 ? 32u : (plane == 2 ? 4u : 8u))     // of a row
+                                            : H * 128u * (plane == 4 ? 1u : (plane < 8 ? 2u : (plane == 8 ? (uint32_t)L::NBI : (uint32_t)L::NB)))) >> (split - 1);
+            const uint32_t at[10] = {0, L::VM, L::VS, L::VZ, L::KS, L::KZ, L::MS, L::MC, L::BM, L::OV};
+            uint32_t off = 0;
+#pragma unroll
+            for (int i = 1; i < 10; ++i) off = plane == i ? at[i] : off;
+            CopyDesc d;
+            d.src = p.k_obmp;                                           // of the one plane that may be copied slot by slot
+            d.unit = bytes * (single ? (plane == 8 ? L::SLOT_SPLIT : 1) : 4);
+            d.dst = off + row * bytes;
+            d.tbase = plane < 2 ? row * page_split : (by_page ? row : page_rows + row);
+            d.tmul = 0;
+            const int whole = row >> (split - 1), gi = by_page ? whole >> ppg_log : whole;   // page or slot, its group
+            d.tok0 = by_page ? (whole & (p.ppg - 1)) * p.ps : 0;
+            d.gi = gi | (single ? (plane < 2 ? plane + 1 : 0) : 3 + plane) << 8;
+            s_desc[c] = d;
+        }
+    } else {
         // Copy roles (group-in-stage, plane) are tabulated once; the producer's loop body is then one
         // descriptor load, one multiply-add and one copy per role, with no divergent paths, because that
         // single warp's issue latency bounds how fast stages refill.
@@ -717,8 +800,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     // ---- one stage of the ring: look up its page ids and group slots, announce its bytes, issue its copies (producer
     //      warps).  The lookup of a stage runs while the stage before it is still on its way, so that no copy waits for its
     //      table entry; each lane leaves what it finds in s_idx for itself. ----
-    Piece *s_piece = reinterpret_cast<Piece *>(s_desc + ncopies);
-    int32_t *s_idx = reinterpret_cast<int32_t *>(s_piece + MAX_PIECES);
+    Piece *s_piece = reinterpret_cast<Piece *>(s_desc + GS * cpg);
+    // (four rows to a copy make fewer descriptors, and four warps' entries fit behind them)
+    int32_t *s_idx = GATHER ? reinterpret_cast<int32_t *>(s_desc + ncopies) : reinterpret_cast<int32_t *>(s_piece + MAX_PIECES);
     auto whole_stage = [&](const Piece &q, int it) { return 32 * GS * (it + 1 - q.it0) <= q.ntok; };
     auto copy_on = [&](const CopyDesc &d, const Piece &q, int it) __attribute__((always_inline)) {
         const int lg = (it - q.it0) * GS + (d.gi & 0xFF);
@@ -726,6 +810,24 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
     };
     auto lookup_stage = [&](const Piece &q, int it, int nshare, int share) __attribute__((always_inline)) {
         const int64_t g0 = (int64_t)p.seg_group_base + q.g0 + (it - q.it0) * GS;
+        if constexpr (GATHER) {
+            // every page and slot of the stage once (or twice, its halves); what the sequence does not have there repeats the first,
+            // so that a copy of four rows reads nothing else
+            int32_t *idx = s_idx + share * (page_rows + L::SLOT_ROWS);
+            __syncwarp();                                           // the last stage's have been read
+            for (int i = lane; i < page_rows + L::SLOT_ROWS; i += 32) {
+                const bool page = i < page_rows;
+                const int split = page ? page_split : L::SLOT_SPLIT, x = (page ? i : i - page_rows) >> (split - 1);   // page or slot of the stage
+                const int gi = page ? x >> ppg_log : x, pg = page ? x & (p.ppg - 1) : 0, lg = (it - q.it0) * GS + gi;
+                const bool on = lg < q.ng && 32 * lg + pg * p.ps < q.ntok;
+                const int64_t at = page ? (int64_t)q.b * p.r2t_sb + g0 * p.ppg + (on ? x : 0) : (int64_t)q.b * p.r2g_sb + g0 + (on ? x : 0);
+                int64_t id = load_index(page ? p.r2t : p.r2g, p.tbl64, at);
+                if (id < 0 || id >= (page ? p.num_pages : p.num_slots)) { or_status(p.status, page ? OMMX_ST_BAD_PAGE : OMMX_ST_BAD_GROUP); id = 0; }
+                idx[i] = (int)id * split + ((page ? i : i - page_rows) & (split - 1));
+            }
+            __syncwarp();
+            return;
+        }
 #pragma unroll 1
         for (int ci = lane * nshare + share; ci < ncopies; ci += 32 * nshare) {
             const CopyDesc d = s_desc[ci];
@@ -750,10 +852,10 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         }
         return __reduce_add_sync(0xFFFFFFFFu, mine);
     };
-    auto issue_stage = [&](const Piece &q, int it, int nshare, int share, uint32_t announce) __attribute__((always_inline)) {
+    auto issue_stage = [&](const Piece &q, int it, int nshare, int share, bool announce, uint32_t bytes) __attribute__((always_inline)) {
         const int s = ring_slot(it, NS);
         if (announce) {
-            if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, announce);
+            if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
             __syncwarp();
         }
         const uint32_t sbase = smem_u32(s_stage + (size_t)s * stage_bytes);
@@ -762,6 +864,17 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             const CopyDesc d = s_desc[ci];
             const int kind = d.gi >> 8;
             if (copy_on(d, q, it) && !((abl & ABL_TEST_STALL) && it == 1)) {
+                if constexpr (GATHER) {
+                    const int32_t *at = s_idx + share * (page_rows + L::SLOT_ROWS) + d.tbase;
+                    if (L::CODE_ROWS == 1 && (kind == 1 || kind == 2)) {
+                        tma_2d_g2s(sbase + d.dst, kind == 1 ? &p.tmap_k : &p.tmap_v, 0, *at * (p.rows_per_page >> (page_split - 1)), bar_full + 8 * s);
+                    } else if (!L::ROWS_FIT && kind == 0) {
+                        bulk_g2s(sbase + d.dst, d.src + (int64_t)*at * (d.unit / L::SLOT_SPLIT), d.unit, bar_full + 8 * s);
+                    } else {
+                        tma_rows_g2s(sbase + d.dst, &p.rows[kind - 3], *reinterpret_cast<const int4 *>(at), bar_full + 8 * s);
+                    }
+                    continue;
+                }
                 const int idx = s_idx[ci];
                 if (kind == 0) bulk_g2s(sbase + d.dst, d.src + (int64_t)idx * d.unit, d.unit, bar_full + 8 * s);
                 else tma_2d_g2s(sbase + d.dst, kind == 1 ? &p.tmap_k : &p.tmap_v, 0, idx * p.rows_per_page, bar_full + 8 * s);
@@ -783,7 +896,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             lookup_stage(q, 0, 4, warp - W0);
             const uint32_t bytes = WIDE ? stage_bytes_of(q, 0, false, lane * NPW + warp - W0, 32 * NPW)
                                         : (warp == PRODUCER_WARP ? stage_bytes_of(q, 0, false, lane, 32) : 0u);
-            issue_stage(q, 0, 4, warp - W0, bytes);
+            issue_stage(q, 0, 4, warp - W0, WIDE || warp == PRODUCER_WARP, bytes);
         }
     }
 
@@ -836,7 +949,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         }
         const int lg = (it - pc.it0) * GS + gsel;                 // local group of this unit
         const bool active = lg < pc.ng && !(abl & ABL_NO_COMPUTE);
-        const uint8_t *gb = s_stage + (size_t)s * stage_bytes + (size_t)gsel * gb_bytes;
+        // (plane-major stages: group planes of units one after the other, token rows of group after group)
+        const uint8_t *gb = s_stage + (size_t)s * stage_bytes + (GATHER ? 0 : (size_t)gsel * gb_bytes);
+        const int hu = GATHER ? unit : h;
         const int d0 = 64 * hf + 2 * cp;                         // first of this lane's two channels
         const bool splice = k_out > 0 && !no_outlier;
         // ---- everything that only reads the stage comes before the wait for the tile, which the MMA warps make a decode warp
@@ -851,12 +966,12 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
         // Row pz of the code bytes of the channels at byte o of the head: byte pz*TS + h*32 + o of the (1 KB aligned) k_base
         // block, with the 16-byte chunk bits XOR-ed by the row's swizzle term.  h*32 + o splits into a part above
         // bit 7 (added to the row) and a part below (the XOR operand, swizzle term of the former included).
-        const uint8_t *k_hi = gb + (h >> 2) * 128;
+        const uint8_t *k_hi = gb + (GATHER ? gsel * H * 1024 : (h >> 2) * 128);
         const uint32_t k_sw = ((uint32_t)(h >> 2) * 16u) & SWZ;
         uint32_t st[2] = {0, 0}, sth[2] = {0, 0};                // nibble stream of each channel: outliers 0..7, 8..15
         if (active) {
-            e2 = *reinterpret_cast<const uint16_t *>(gb + o_ks + h * 128 + d0);
-            z2 = *reinterpret_cast<const uint32_t *>(gb + o_kz + h * 256 + 2 * d0);
+            e2 = *reinterpret_cast<const uint16_t *>(gb + o_ks + hu * 128 + d0);
+            z2 = *reinterpret_cast<const uint32_t *>(gb + o_kz + hu * 256 + 2 * d0);
             {
                 // K scale factors 2^(e + KF_BIAS) * 4^-slot of the two channels, bf16
                 const uint32_t eb = __byte_perm(e2 ^ 0x8080u, 0u, 0x4140u);                       // e + 128, two halves
@@ -867,7 +982,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             }
             if (hf == 0) {
                 // V scale factors 2^(e + FBIAS), fp16, of the four scale groups; lane = token
-                const uint32_t w = 32 * lg + lane < pc.ntok ? *reinterpret_cast<const uint32_t *>(gb + o_vs + (lane * H + h) * 4) ^ 0x80808080u : 0u;
+                const uint32_t w = 32 * lg + lane < pc.ntok ? *reinterpret_cast<const uint32_t *>(gb + o_vs + (GATHER ? gsel * H * 128 : 0) + (lane * H + h) * 4) ^ 0x80808080u : 0u;
                 const uint32_t e02 = w & 0x00FF00FFu, e13 = (w >> 8) & 0x00FF00FFu;               // e + 128, groups 0, 2 and 1, 3
                 e_max = __vimax3_s16x2(e_max, e02, e13);
                 f02 = __viaddmin_s16x2_relu(e02, half2_const(FBIAS + 15 - 128, FBIAS + 15 - 128), half2_const(30, 30)) << 10;
@@ -875,11 +990,11 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             }
             if (splice) {
                 if (use_map) {
-                    ms2 = *reinterpret_cast<const uint32_t *>(gb + o_ms + h * 256 + 2 * d0);
-                    mc2 = *reinterpret_cast<const uint32_t *>(gb + o_mc + h * 256 + 2 * d0);
+                    ms2 = *reinterpret_cast<const uint32_t *>(gb + o_ms + hu * 256 + 2 * d0);
+                    mc2 = *reinterpret_cast<const uint32_t *>(gb + o_mc + hu * 256 + 2 * d0);
                 }
                 if (!idx7) {
-                    bm2 = *reinterpret_cast<const uint2 *>(gb + o_bm + h * 512 + 4 * d0);
+                    bm2 = *reinterpret_cast<const uint2 *>(gb + o_bm + hu * 512 + 4 * d0);
                 } else {
                     // relidx7 (attention/codec.py:91-130 of the reference): k ascending token positions, 7 bits each,
                     // LSB first; the outlier set as a bitmask again, the value stream is shared with that encoding
@@ -888,7 +1003,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                         // both channels' streams are 2 * NBI bytes back to back, 4-byte aligned where that is whole words
                         constexpr int NBI = (7 * KOUT + 7) / 8, NW = (2 * NBI + 3) / 4;
                         constexpr PositionBits PAST = past_31_bits(KOUT, NBI);
-                        const uint8_t *ip = gb + o_bm + (h * 128 + d0) * NBI;
+                        const uint8_t *ip = gb + o_bm + (hu * 128 + d0) * NBI;
                         uint32_t w[NW + 1] = {}, past = 0u;
                         if constexpr (NBI % 2 == 0) {
 #pragma unroll
@@ -910,7 +1025,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     } else {
 #pragma unroll
                         for (int c = 0; c < 2; ++c) {
-                            const uint8_t *ip = gb + o_bm + (h * 128 + d0 + c) * p.nbi;
+                            const uint8_t *ip = gb + o_bm + (hu * 128 + d0 + c) * p.nbi;
                             uint32_t w[5] = {0u, 0u, 0u, 0u, 0u};
                             for (int i = 0; i < p.nbi; ++i) w[i >> 2] |= (uint32_t)ip[i] << (8 * (i & 3));
                             uint32_t bits = 0u;
@@ -926,7 +1041,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                     bm2 = make_uint2(m2[0], m2[1]);
                 }
                 const int nb = KOUT >= 0 ? (KOUT + 1) / 2 : p.nb;
-                const uint8_t *ov = gb + o_ov + (h * 128 + d0) * nb;          // 2*nb bytes, 2-byte aligned
+                const uint8_t *ov = gb + o_ov + (hu * 128 + d0) * nb;          // 2*nb bytes, 2-byte aligned
                 if (nb == 3) {
                     const uint32_t w0 = reinterpret_cast<const uint16_t *>(ov)[0], w1 = reinterpret_cast<const uint16_t *>(ov)[1],
                                    w2 = reinterpret_cast<const uint16_t *>(ov)[2];
@@ -956,7 +1071,10 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 }
             }
             if constexpr (PLANES)
-                if (splice) code_bit_planes(smem_u32(k_hi + lm_tok * TS) + (((h & 3) * 32 + 16 * hf) ^ k_sw ^ (((uint32_t)(lm_tok * TS) >> 3) & SWZ)), lane, cw);
+                if (splice) {
+                    if constexpr (TS < 128) code_bit_planes(smem_u32(k_hi) + swz128((uint32_t)(lm_tok * TS + h * 32 + 16 * hf), SWZ), lane, cw);
+                    else code_bit_planes(smem_u32(k_hi + lm_tok * TS) + (((h & 3) * 32 + 16 * hf) ^ k_sw ^ (((uint32_t)(lm_tok * TS) >> 3) & SWZ)), lane, cw);
+                }
         }
         // Tile `it` of a unit may be written once the MMA warp has read tile it-1.  Decode warps
         // run up to NS groups ahead and the tiles of one unit are built by different warps, so
@@ -992,6 +1110,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 __syncwarp();                                        // the cleared rows before any delta lands in them
                 const uint32_t k_lo = (uint32_t)((h & 3) * 32 + (d0 >> 2)) ^ k_sw;
                 auto code_byte = [&](uint32_t pz) -> uint32_t {
+                    if constexpr (TS < 128) return k_hi[swz128(pz * TS + k_lo, SWZ)];
                     return k_hi[pz * TS + (k_lo ^ (((pz * TS) >> 3) & SWZ))];
                 };
                 const uint32_t colp = smem_u32(tile) + 128 * hf + 32 * da + 4 * dj + 2 * dh;
@@ -1127,7 +1246,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 producer_alive = false;
                 break;
             }
-            issue_stage(pc, it, NPW, pw, bytes);
+            issue_stage(pc, it, NPW, pw, true, bytes);      // a share may hold nothing of a short stage: its announcement still counts
         }
         if constexpr (WIDE) return;
         // Narrow layout: with every stage on its way this warp has nothing left to do, while the 15 decode warps share
@@ -1242,8 +1361,9 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             break;
         }
         if (active) {
-            uint8_t *gb = s_stage + (size_t)s * stage_bytes + (size_t)gsel * gb_bytes;
-            const uint32_t v_addr = smem_u32(gb + o_vm) + v_off;  // v_main region of the group (1 KB aligned)
+            uint8_t *gb = s_stage + (size_t)s * stage_bytes + (GATHER ? 0 : (size_t)gsel * gb_bytes);
+            const uint32_t rows_at = GATHER ? gsel * H * 1024 : 0;        // token rows of the group in either code plane
+            const uint32_t v_addr = smem_u32(gb + o_vm) + rows_at + v_off;  // v_main region of the group (1 KB aligned)
 
             // ======================= logits =======================
             // code words of this lane's four token rows (tokens 8*nt + g), channels 16j..16j+15 of either half
@@ -1251,7 +1371,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             if (do_k)
 #pragma unroll
                 for (int w = 0; w < 2; ++w)
-                    ldsm_x4(smem_u32(gb) + swz128((uint32_t)(lane * TS + h * 32 + 16 * w), SWZ), kw[w][0], kw[w][1], kw[w][2], kw[w][3]);
+                    ldsm_x4(smem_u32(gb) + rows_at + swz128((uint32_t)(lane * TS + h * 32 + 16 * w), SWZ), kw[w][0], kw[w][1], kw[w][2], kw[w][3]);
             // The unit's sidecar tile arrives in two steps: first the rows of factors, then the outlier
             // deltas.  The code MMAs run on the first, while the decode warps still scatter the deltas.
             if (!mbar_wait(bar_trows + 8 * unit, (uint32_t)it & 1u, wait_limit)) {
@@ -1283,7 +1403,7 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
             // of use, with 1 and 3 the others.
             float Z0[4] = {0.f, 0.f, 0.f, 0.f}, Z1[4] = {0.f, 0.f, 0.f, 0.f};
             {
-                const uint8_t *zrow = gb + o_kz + h * 256 + 16 * j;
+                const uint8_t *zrow = gb + o_kz + (GATHER ? unit : h) * 256 + 16 * j;
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                     const uint4 z = *reinterpret_cast<const uint4 *>(zrow + 64 * v);
@@ -1389,11 +1509,11 @@ __global__ void __launch_bounds__(WarpLayout<H>::THREADS, 1) decode_stage1_kerne
                 // zero-points: z[m] = tokens 8m + 2j, + 1 of row g
                 uint32_t z[4];
                 if constexpr (H > 1) {
-                    ldsm_x4_trans(smem_u32(gb + o_vz + (lane * H + (h & ~1)) * 8), z[0], z[1], z[2], z[3]);
+                    ldsm_x4_trans(smem_u32(gb + o_vz + (GATHER ? gsel * H * 256 : 0) + (lane * H + (h & ~1)) * 8), z[0], z[1], z[2], z[3]);
                 } else {
 #pragma unroll
                     for (int m = 0; m < 4; ++m) {
-                        const uint16_t *vz = reinterpret_cast<const uint16_t *>(gb + o_vz + (8 * m + 2 * j) * 8) + (g & 3);
+                        const uint16_t *vz = reinterpret_cast<const uint16_t *>(gb + o_vz + (GATHER ? gsel * H * 256 : 0) + (8 * m + 2 * j) * 8) + (g & 3);
                         z[m] = g < 4 ? (uint32_t)vz[0] | ((uint32_t)vz[4] << 16) : 0u;
                     }
                 }
@@ -1606,8 +1726,8 @@ template <typename Kernel> static int allow_full_smem(Kernel kernel, std::atomic
 }
 
 template <int KOUT, int H, bool PLAIN, bool IDX7, bool CLUSTER>
-static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
-    using L = WarpLayout<H>;
+static int launch_s1(const typename Stage1Form<H, PLAIN>::Params &p, size_t smem, cudaStream_t st) {
+    using L = typename Stage1Form<H, PLAIN>::Layout;
     // function attributes belong to (kernel instantiation, device): one entry per device ordinal
     static std::atomic<int> smem_set[MAX_DEVICES];
     static std::atomic<int> regs_state[MAX_DEVICES];   // 0 unknown, 1 enough, 2 too few
@@ -1629,18 +1749,26 @@ static int launch_s1(const S1Params &p, size_t smem, cudaStream_t st) {
     count_launch();
     return 0;
 }
+// The row maps of a launch for one to four kv heads (not of an outlier index whose rows are too long); false when one cannot be built.
+bool make_row_maps(S1GatherParams &p, bool with_index);
+
 // The form that can exchange states only in launches of clusters, the general form too: in the others its code costs 2 to 6 % (both
 // stages, with -> without, 8 kv heads: 4K, k = 3 13.4 -> 12.6 us; 64K, k = 3 44.7 -> 43.5, with a logit cap 53.9 -> 52.6; 70B heads
 // 8 x 32K with a logit cap 186.5 -> 183.0, of one kv head 38.2 -> 37.4).
 template <int KOUT, int H, bool PLAIN, bool IDX7>
-static int launch_s1_form(const S1Params &p, size_t smem, cudaStream_t st) {
+static int launch_s1_form(const S1Params &q, size_t smem, cudaStream_t st) {
+    typename Stage1Form<H, PLAIN>::Params p;
+    static_cast<S1Params &>(p) = q;
+    if constexpr (Stage1Form<H, PLAIN>::GATHER)
+        if (!make_row_maps(p, PlainLayout<KOUT, H, IDX7>::ROWS_FIT)) return fail(OMMX_E_CUDA, "stage 1: the tensor maps of the planes could not be encoded");
     return p.grid.cluster > 1 ? launch_s1<KOUT, H, PLAIN, IDX7, true>(p, smem, st) : launch_s1<KOUT, H, PLAIN, IDX7, false>(p, smem, st);
 }
 // The plain form where the recipe and the ring depth are its own, else the general one.
 template <int KOUT, int H>
 static int launch_s1_forms(const S1Params &p, size_t smem, cudaStream_t st) {
     if constexpr (KOUT >= 0) {
-        if (p.abl == 0 && (KOUT == 0 || p.use_map) && p.logit_cap <= 0.f) {
+        const bool mapped = !Stage1Form<H, true>::GATHER || (p.num_pages > 0 && p.num_slots > 0);      // an empty plane has no map
+        if (p.abl == 0 && (KOUT == 0 || p.use_map) && p.logit_cap <= 0.f && mapped) {
             if (!p.idx7 && p.nstages >= PlainLayout<KOUT, H, false>::STAGES) return launch_s1_form<KOUT, H, true, false>(p, smem, st);
             if constexpr (KOUT > 0)
                 if (p.idx7 && p.nstages >= PlainLayout<KOUT, H, true>::STAGES) return launch_s1_form<KOUT, H, true, true>(p, smem, st);

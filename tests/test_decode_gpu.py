@@ -132,6 +132,30 @@ def test_decode_many_short_sequences_beside_a_longer_one(H, n, long, at, splits)
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("H,ps,k", [(1, 16, 6), (1, 8, 2), (1, 32, 12), (2, 16, 6), (2, 8, 4), (2, 32, 8), (2, 16, 0), (4, 16, 6), (4, 8, 8), (4, 32, 12)])
+def test_decode_few_heads_stage_edges(H, ps, k):
+    """Stages of eight, four or two groups, loaded four pages or group slots at a time: sequences that end inside a stage, table entries
+    past a sequence's end that name no page."""
+    lens = [40 + 32 * n for n in (1, 3, 4, 5, 8, 9, 31)]
+    case = Case(lens, H=H, Hq=4 * H, seed=3 * H + ps + k, k=k, page_size=ps)
+    for b, n in enumerate(case.packed):
+        case.req_to_token[b, n // ps:] = 1 << 20
+        case.req_to_group[b, n // 32:] = 1 << 20
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for splits in (1, 3, None):
+        _run_and_check(case, num_kv_splits=splits, status=status)
+    assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("H", [1, 2])
+def test_decode_few_heads_empty_pool(H):
+    """A bound above zero on lengths that are all zero, and planes without a page."""
+    case = Case([30, 7], H=H, Hq=4 * H, seed=H)
+    o, lse = case.run()
+    again, lse2 = case.run(max_seq_len=4096, num_kv_splits=4)
+    assert torch.equal(o, again) and torch.equal(lse, lse2)
+
+
 @pytest.mark.parametrize("Hq,aligned", [(8, True), (16, True), (32, True), (64, True), (8, False), (64, False)])
 def test_decode_residual_row_counts(Hq, aligned):
     """Residual rows around the batches and turns of stage 2's loop, in each of its block sizes."""
