@@ -1607,7 +1607,37 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
     // of its own tile, which nobody builds again before it is handed back below.  With 8 heads every warp owns its head.
     static_assert(32 * 36 * 4 <= 32 * DT_STRIDE, "the merge fits the delta rows of a tile");
     const bool mine = !CLUSTER || pc.it0 < pc.it1;                   // this CTA had groups of the piece
-    if (GS > 1 && mine) {
+    constexpr bool TOGETHER = GS > 2 && !CLUSTER;
+    if constexpr (TOGETHER) {
+        // All at once: of the head's 32 values a lane holds, warp gsel takes 32 / GS from every warp's tile and writes them out (one
+        // warp that merged the others one by one, both stages: 8 x 32K x 1 head 30.6 -> 29.6 us, 8K 11.4 -> 10.3; 128K x 2 heads
+        // 28.1 -> 27.4, 4K 10.8 -> 10.3).  Of two warps (four heads) one merges the other's: 32K 19.5 us, together 19.8.
+        store_state();
+        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
+        constexpr int NCG = 8 / GS;
+        const int hh = 2 * gsel / GS, cg0 = gsel % (GS / 2) * NCG, head = 2 * j + hh;
+        const float *states = reinterpret_cast<const float *>(s_tiles + h * DT_BYTES) + lane;
+        constexpr int NEXT = H * DT_BYTES / 4;                      // floats from one warp's state to the next of the same head
+        float m = -INFINITY, l = 0.f, c[GS], sum[4 * NCG] = {};
+#pragma unroll
+        for (int o = 0; o < GS; ++o) m = fmaxf(m, c[o] = states[o * NEXT + 32 * hh]);
+        const float mu = m == -INFINITY ? 0.f : m;
+#pragma unroll
+        for (int o = 0; o < GS; ++o) {
+            c[o] = fast_exp2((c[o] - mu) * LOG2E);
+            l += c[o] * states[o * NEXT + 32 * (2 + hh)];
+#pragma unroll
+            for (int i = 0; i < 4 * NCG; ++i) sum[i] += c[o] * states[o * NEXT + 32 * (4 + 16 * hh + 4 * cg0 + i)];
+        }
+        if (head < p.gqa) {
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            float *dst = p.al + (int64_t)pc.b * p.al_sb + (int64_t)(h * p.gqa + head) * p.al_sh + (int64_t)pc.slot * p.al_ss;
+#pragma unroll
+            for (int i = 0; i < 4 * NCG; ++i) dst[32 * (cg0 + i / 4) + 4 * g + i % 4] = sum[i] * inv;
+            if (g == 0 && cg0 == 0) dst[HD] = l > 0.f ? m + logf(l) : -INFINITY;
+        }
+        asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
+    } else if (GS > 1 && mine) {
         if (gsel > 0) store_state();
         asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
         if (gsel == 0) {
@@ -1619,7 +1649,7 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
         }
         asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
     }
-    bool write = gsel == 0;
+    bool write = gsel == 0 && !TOGETHER;
     if constexpr (CLUSTER)
     if (gsel == 0 && *s_ctas > 1) {
         // the CTAs that share the piece: head h is merged by CTA h % n_ctas
