@@ -108,8 +108,9 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     int nsplit = 0;
     if (p.S > 0 && groups > 0) {
         int per = 0;
-        if constexpr (CLUSTER) per = share_plan_of(total, longest, p.B, p.S, p.grid).per;
-        else if (p.grid.ncta > 0) per = share_plan_of(total, longest, p.B, p.S, p.grid.ncta, p.grid.waves).per;
+        const ShareDivisors by = share_divisors(p.grid, p.S);
+        if constexpr (CLUSTER) per = share_plan_of(total, longest, p.B, p.S, p.grid, by).per;
+        else if (p.grid.ncta > 0) per = share_plan_of(total, longest, p.B, p.S, by.ctas, p.grid.waves, by).per;
         if (per == 0) {
             const int equal = (groups + p.S - 1) / p.S;
             nsplit = (groups + equal - 1) / equal;
@@ -764,7 +765,7 @@ extern "C" int ommx_b200_host_launch_plan(const int32_t *b_seq_len, int32_t batc
         longest = max(longest, groups_of(b_seq_len[i]));
     }
     const Stage1Grid grid = stage1_grid(batch, num_kv_splits, max_seq_len, chip);
-    const SharePlan plan = share_plan_of(total, longest, batch, num_kv_splits, grid);
+    const SharePlan plan = share_plan_of(total, longest, batch, num_kv_splits, grid, share_divisors(grid, num_kv_splits));
     *out = ommx_launch_plan{grid.ncta, grid.cluster, plan.shares, plan.ctas, plan.per};
     return MAX_PIECES;
 }

@@ -379,27 +379,42 @@ struct SharePlan {
     int per, total;                      // groups per share (0: equal splits per sequence), groups of all sequences
     int ctas, shares;                    // CTAs to a share, shares
 };
+// Division by what a launch knows beforehand: stage 1 prepares the reciprocals before it waits for the kernel ahead of it.  (Three divisions
+// between the lengths and the first copy were 0.8 us of every launch.)  Exact: with m = floor((2^32 - 1) / d) the product's upper half
+// is the quotient or one less.
+struct Divisor {
+    uint32_t d, m;
+    __host__ __device__ __forceinline__ int of(int n) const {        // n / d for n >= 0
+        const uint32_t q = (uint32_t)(((uint64_t)(uint32_t)n * m) >> 32);
+        return (int)(q + ((uint32_t)n - q * d >= d ? 1u : 0u));
+    }
+};
+__host__ __device__ __forceinline__ Divisor divisor(int d) { return Divisor{(uint32_t)d, 0xFFFFFFFFu / (uint32_t)d}; }
+struct ShareDivisors { Divisor ctas, shares, slots, slots1; };        // CTAs, clusters, S, S - 1
+__host__ __device__ __forceinline__ ShareDivisors share_divisors(const Stage1Grid &g, int S) {
+    return ShareDivisors{divisor(max(g.ncta, 1)), divisor(max(g.ncta / max(g.cluster, 1), 1)), divisor(S), divisor(max(S - 1, 1))};
+}
 __host__ __device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
-__host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, int ncta, int waves) {
+__host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, const Divisor &ncta, int waves, const ShareDivisors &by) {
     SharePlan s;
     s.total = total;
     s.ctas = 1;
-    s.shares = ncta;
-    s.per = max(1, (total + ncta - 1) / ncta);
-    const int equal = (longest + S - 1) / S;
+    s.shares = (int)ncta.d;
+    s.per = max(1, ncta.of(total + (int)ncta.d - 1));
+    const int equal = by.slots.of(longest + S - 1);
     if (B == 1) {
         s.per = max(s.per, equal);                             // a lone sequence starts at a CTA's beginning: exactly ceil(n / per) slots
     } else {
-        if (S >= 2) s.per = max(s.per, (longest - 2) / (S - 1) + 1);   // anywhere else it touches up to (n - 2) / per + 2 CTAs
+        if (S >= 2) s.per = max(s.per, longest >= 2 ? by.slots1.of(longest - 2) + 1 : 1);   // anywhere else it touches up to (n - 2) / per + 2 CTAs
         if (S < 2 || min(s.per, B) > MAX_PIECES || (waves <= MAX_PIECES && waves * equal <= s.per)) s.per = 0;
     }
     return s;
 }
-__host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, const Stage1Grid &g) {
-    SharePlan a = share_plan_of(total, longest, B, S, g.ncta, g.waves);
+__host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, const Stage1Grid &g, const ShareDivisors &by) {
+    SharePlan a = share_plan_of(total, longest, B, S, by.ctas, g.waves, by);
     if (g.cluster > 1) {
-        const int equal = (longest + S - 1) / S;
-        SharePlan c = share_plan_of(total, longest, B, S, g.ncta / g.cluster, g.cluster_waves);
+        const int equal = by.slots.of(longest + S - 1);
+        SharePlan c = share_plan_of(total, longest, B, S, by.shares, g.cluster_waves, by);
         c.ctas = g.cluster;
         const int of_a = a.per > 0 ? a.per : g.waves * equal, of_c = c.per > 0 ? c.per : g.cluster_waves * equal;
         if ((c.per > 0 || g.cluster_waves <= MAX_PIECES) && (of_c + g.cluster - 1) / g.cluster + 1 < of_a) return c;
@@ -437,7 +452,8 @@ static inline Stage1Grid stage1_grid(int batch, int S, int max_seq_len, const Ch
     return g;
 }
 // called by whole warps; every lane gets the same answer
-template <bool CLUSTER> __device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, const Stage1Grid &g, int lane) {
+template <bool CLUSTER>
+__device__ __forceinline__ SharePlan share_plan(const int32_t *b_seq_len, int B, int S, const Stage1Grid &g, const ShareDivisors &by, int lane) {
     int n = 0, mx = 0;
     if (B == 1) {
         n = mx = groups_of(b_seq_len[0]);
@@ -450,8 +466,8 @@ template <bool CLUSTER> __device__ __forceinline__ SharePlan share_plan(const in
         n = __reduce_add_sync(0xFFFFFFFFu, n);
         mx = __reduce_max_sync(0xFFFFFFFFu, mx);
     }
-    if constexpr (CLUSTER) return share_plan_of(n, mx, B, S, g);
-    else return share_plan_of(n, mx, B, S, g.ncta, g.waves);
+    if constexpr (CLUSTER) return share_plan_of(n, mx, B, S, g, by);
+    else return share_plan_of(n, mx, B, S, by.ctas, g.waves, by);
 }
 
 // One piece of work of a CTA: consecutive groups of one sequence.  `it` counts the CTA's ring stages across its pieces, so that
@@ -522,7 +538,7 @@ template <int GS> __device__ __forceinline__ bool first_piece(Piece &c, PieceWal
             off += __shfl_sync(0xFFFFFFFFu, x, 31);
         }
     }
-    c.slot = cta - off / plan.per;
+    c.slot = off > 0 ? cta - off / plan.per : cta;
     const int g0 = w.pos - off, ng = min(n - g0, w.end - w.pos);
     piece_range<GS>(c, seq, g0, ng);
     return true;
@@ -675,6 +691,8 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
         if (i >= (L::CODE_ROWS == 1 ? 2 : 0) && i < (KOUT > 0 ? 10 : 6) && (i != 8 || L::ROWS_FIT))
             asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&p.rows[i])) : "memory");
     }
+    // the sidecar tiles: rows that no half writes stay zero
+    for (int i = threadIdx.x; i < NCW * DT_BYTES / 16; i += S1_THREADS) reinterpret_cast<uint4 *>(s_tiles)[i] = make_uint4(0, 0, 0, 0);
     if (threadIdx.x < 16) {
         const int c = threadIdx.x;
         const int mi = ((c >> 1) & 3) * 2 + (c & 1);                    // exp*2 + mant
@@ -776,21 +794,29 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
     }
     __syncthreads();
     if constexpr (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");         // this CTA's barriers are ready
-    // Nothing an earlier kernel may have written - lengths, tables, the query, the planes, the split workspace a
-    // previous layer's combine still reads - is touched before this returns.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // Stage 2 is launched as a programmatic dependent: it may start its own prologue (residual-row
-    // logits, which do not depend on this kernel but may depend on the one before it: hence after the wait)
-    // as soon as SM resources free up, and waits for this grid to finish before it reads the split partials.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
     Piece pc;
-    PieceWalk walk;
-    const SharePlan plan = share_plan<CLUSTER>(p.b_seq_len, p.B, p.S, p.grid, lane);
-    if (!first_piece<GS>(pc, walk, p, plan, CLUSTER ? cta / plan.ctas : cta, lane)) return;
-    auto my_part = [&](const Piece &c, int it0) __attribute__((always_inline)) {
-        if constexpr (CLUSTER) return part_of<GS>(c, cluster_rank(), plan.ctas, it0);
-        else return c;
+    Piece *s_piece = reinterpret_cast<Piece *>(s_desc + GS * cpg);
+    auto wait_for_earlier_kernels = [&]() __attribute__((always_inline)) {
+        // Nothing an earlier kernel may have written - lengths, tables, the query, the planes, the split workspace a
+        // previous layer's combine still reads - is touched before this returns.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        // Stage 2 is launched as a programmatic dependent: it may start its own prologue (residual-row
+        // logits, which do not depend on this kernel but may depend on the one before it: hence after the wait)
+        // as soon as SM resources free up, and waits for this grid to finish before it reads the split partials.
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    };
+    // The list of pieces is there (and the first ring fill on its way); false: this CTA has none.
+    int pi = 0;
+    auto pieces_listed = [&]() __attribute__((always_inline)) {
+        asm volatile("bar.sync 0, %0;" ::"n"(S1_THREADS) : "memory");
+        if constexpr (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        pc = s_piece[0];
+        return pc.b >= 0;
+    };
+    auto step_piece = [&]() __attribute__((always_inline)) {
+        if (!pc.more) return false;
+        pc = s_piece[++pi];
+        return true;
     };
 
     const int g = lane >> 2, j = lane & 3;
@@ -800,7 +826,6 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
     // ---- one stage of the ring: look up its page ids and group slots, announce its bytes, issue its copies (producer
     //      warps).  The lookup of a stage runs while the stage before it is still on its way, so that no copy waits for its
     //      table entry; each lane leaves what it finds in s_idx for itself. ----
-    Piece *s_piece = reinterpret_cast<Piece *>(s_desc + GS * cpg);
     // (four rows to a copy make fewer descriptors, and four warps' entries fit behind them)
     int32_t *s_idx = GATHER ? reinterpret_cast<int32_t *>(s_desc + ncopies) : reinterpret_cast<int32_t *>(s_piece + MAX_PIECES);
     auto whole_stage = [&](const Piece &q, int it) { return 32 * GS * (it + 1 - q.it0) <= q.ntok; };
@@ -881,11 +906,22 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
             }
         }
     };
-    // The first ring fill is on every CTA's critical path: it goes out before the register budgets are resized.
-    // A warp issues a bulk copy only about every 60 cycles and different warps overlap, so in the narrow layout the three
-    // decode warps of the producer's warpgroup (idle until the data lands) take a quarter of the first fill each.
-    if (warp >= PRODUCER_WARP - (WIDE ? 0 : 3)) {
-        constexpr int W0 = PRODUCER_WARP - (WIDE ? 0 : 3);
+    // ---- what the producers do before the other roles start: deal out the work, fill the ring's first stage, list the pieces ----
+    // The first fill is on every CTA's critical path.  A warp issues a bulk copy only about every 60 cycles and different warps
+    // overlap, so in the narrow layout the three decode warps of the producer's warpgroup (idle until the data lands) take a
+    // quarter of the first fill each.
+    constexpr int FILL_WARP = PRODUCER_WARP - (WIDE ? 0 : 3);
+    auto start_pieces = [&](const ShareDivisors &by) __attribute__((always_inline)) {
+        PieceWalk walk;
+        const SharePlan plan = share_plan<CLUSTER>(p.b_seq_len, p.B, p.S, p.grid, by, lane);
+        auto my_part = [&](const Piece &c, int it0) __attribute__((always_inline)) {
+            if constexpr (CLUSTER) return part_of<GS>(c, cluster_rank(), plan.ctas, it0);
+            else return c;
+        };
+        if (!first_piece<GS>(pc, walk, p, plan, CLUSTER ? cta / plan.ctas : cta, lane)) {
+            if (warp == PRODUCER_WARP && lane == 0) s_piece[0].b = -1;
+            return;
+        }
         Piece q = my_part(pc, 0);
         if (CLUSTER && q.ng == 0) {                                             // this CTA begins with a later piece, if any
             Piece c = pc;
@@ -893,36 +929,26 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
             while (q.ng == 0 && next_piece<GS>(c, w, p, plan)) q = my_part(c, 0);
         }
         if (!CLUSTER || q.ng > 0) {
-            lookup_stage(q, 0, 4, warp - W0);
-            const uint32_t bytes = WIDE ? stage_bytes_of(q, 0, false, lane * NPW + warp - W0, 32 * NPW)
+            lookup_stage(q, 0, 4, warp - FILL_WARP);
+            const uint32_t bytes = WIDE ? stage_bytes_of(q, 0, false, lane * NPW + warp - FILL_WARP, 32 * NPW)
                                         : (warp == PRODUCER_WARP ? stage_bytes_of(q, 0, false, lane, 32) : 0u);
-            issue_stage(q, 0, 4, warp - W0, WIDE || warp == PRODUCER_WARP, bytes);
+            issue_stage(q, 0, 4, warp - FILL_WARP, WIDE || warp == PRODUCER_WARP, bytes);
         }
-    }
-
-    if (warp == PRODUCER_WARP) {
-        if (CLUSTER && lane == 0) *s_ctas = plan.ctas;
-        int n = 0, at = 0;
-        for (bool more = true; more; ++n) {
-            Piece cur = my_part(pc, at);
-            at = cur.it1;
-            more = next_piece<GS>(pc, walk, p, plan);
-            if (more && n + 1 == MAX_PIECES) {                       // a bounds check: share_plan_of rules it out
-                if (lane == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
-                more = false;
+        if (warp == PRODUCER_WARP) {
+            if (CLUSTER && lane == 0) *s_ctas = plan.ctas;
+            int n = 0, at = 0;
+            for (bool more = true; more; ++n) {
+                Piece cur = my_part(pc, at);
+                at = cur.it1;
+                more = next_piece<GS>(pc, walk, p, plan);
+                if (more && n + 1 == MAX_PIECES) {                       // a bounds check: share_plan_of rules it out
+                    if (lane == 0) or_status(p.status, OMMX_ST_BAD_LENGTH);
+                    more = false;
+                }
+                cur.more = more;
+                if (lane == 0) s_piece[n] = cur;
             }
-            cur.more = more;
-            if (lane == 0) s_piece[n] = cur;
         }
-    }
-    __syncthreads();
-    if constexpr (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    int pi = 0;
-    pc = s_piece[0];
-    auto step_piece = [&]() __attribute__((always_inline)) {
-        if (!pc.more) return false;
-        pc = s_piece[++pi];
-        return true;
     };
 
     // ---- one work item of the decode role: half hf of the sidecar tile of (iteration it, unit) ----
@@ -1222,16 +1248,8 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
         return true;
     };
 
-    // ---- roles; each branch starts by resizing its warpgroups' register budget and never rejoins ----
-    if constexpr (WIDE) {
-        if (warp >= PRODUCER_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_PRODUCER ";");
-        else if (warp >= NCW) asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_DECODE ";");
-    } else {
-        if (warp >= NCW) asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_DECODE ";");
-    }
     bool producer_alive = true;
-    if (warp >= PRODUCER_WARP) {
-        // =========================== producer warp(s) ===========================
+    auto produce = [&]() __attribute__((always_inline)) {
         const int pw = warp - PRODUCER_WARP;
         const uint32_t full_bytes = stage_bytes_of(pc, 0, true, lane * NPW + pw, 32 * NPW);   // this warp's share of a stage of whole groups
         for (int it = 1;; ++it) {
@@ -1248,32 +1266,44 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
             }
             issue_stage(pc, it, NPW, pw, true, bytes);      // a share may hold nothing of a short stage: its announcement still counts
         }
-        if constexpr (WIDE) return;
-        // Narrow layout: with every stage on its way this warp has nothing left to do, while the 15 decode warps share
+    };
+
+    // ---- roles; each branch resizes its warpgroups' register budget and never rejoins.  What needs no earlier kernel is done before the
+    //      wait for it: clearing the tiles, the reciprocals of the share-out's divisions, the decode warps' registers (both
+    //      stages in a graph: 1K 10.35 -> 9.3 us, 4K 12.5 -> 11.6, 16K 19.5 -> 18.5, 64K 41.6 -> 41.0; with the MMA warps' registers ahead
+    //      of it too 11.8 and 41.1, 8 x 32K 136.4 -> 137.3).  The wide layout's producers start the pieces first, which 24
+    //      registers do not hold, and its MMA warps need what they give back. ----
+    if constexpr (WIDE)
+        if (warp >= PRODUCER_WARP) {
+            const ShareDivisors by = share_divisors(p.grid, p.S);
+            wait_for_earlier_kernels();
+            start_pieces(by);
+            const bool any = pieces_listed();
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_PRODUCER ";");
+            if (any) produce();
+            return;
+        }
+    if (warp >= NCW) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 " OMMX_REGS_DECODE ";");
+        if constexpr (WIDE) {
+            wait_for_earlier_kernels();
+        } else {
+            const ShareDivisors by = share_divisors(p.grid, p.S);
+            wait_for_earlier_kernels();
+            if (warp >= FILL_WARP) start_pieces(by);
+        }
+        if (!pieces_listed()) return;
+        // Narrow layout: with every stage on its way the producer has nothing left to do, while the 15 decode warps share
         // 16 items per iteration: it joins them below for the very last item, so that the last iteration's 16 halves are
         // built side by side.
-    }
-
-    // =========================== decode + MMA warps ===========================
+        if (!WIDE && warp == PRODUCER_WARP) produce();
     // MMA warp w owns unit w = (group-in-stage, kv head) and its softmax state.  The decode warps are
     // stateless: work item number n goes to decode warp n % NDW (narrow layout: except the last one, the producer's).
-    if (warp >= NCW) {
+    {
         // =========================== decode warps (narrow layout: and the producer, once it is done) ===========================
         const int dw = warp - NCW;
         const bool is_producer = !WIDE && warp == PRODUCER_WARP;
-        if (!is_producer) {
-            if (dw < NCW) {           // the first to touch tile dw clears it once (unused rows stay zero)
-                uint8_t *t0p = s_tiles + dw * DT_BYTES;
-                for (int i = lane; i < DT_BYTES / 4; i += 32) reinterpret_cast<uint32_t *>(t0p)[i] = 0u;
-            }
-            // every tile is cleared before any half of it is written; the narrow layout's producer learns of it without
-            // being waited for
-            asm volatile("bar.sync 1, %0;" ::"n"(NDW * 32) : "memory");
-            if constexpr (!WIDE) asm volatile("bar.arrive 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
-        } else {
-            asm volatile("bar.sync 2, %0;" ::"n"((NDW + 1) * 32) : "memory");
-            if (!producer_alive || pc.more || (CLUSTER && pc.it0 == pc.it1)) return;
-        }
+        if (is_producer && (!producer_alive || pc.more || (CLUSTER && pc.it0 == pc.it1))) return;
         // the producer takes the very last item, when this CTA's pieces end with one that is known to be the last
         for (int n = is_producer ? pc.it1 * 2 * NCW - 1 : dw;; n += NDW) {
             const int it = n / (2 * NCW);
@@ -1285,9 +1315,13 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
         if ((int)(e_max & 0xFFFFu) > E_TOP || (int)(e_max >> 16) > E_TOP) or_status(p.status, OMMX_ST_SCALE_RANGE);
         return;
     }
+    }
 
     // =========================== MMA warps ===========================
+    wait_for_earlier_kernels();
+    const bool any = pieces_listed();
     asm volatile("setmaxnreg.inc.sync.aligned.u32 " OMMX_REGS_MMA ";");
+    if (!any) return;
     const int unit = warp;
     const int h = unit % H, gsel = unit / H;
     const uint8_t *tile = s_tiles + unit * DT_BYTES;
