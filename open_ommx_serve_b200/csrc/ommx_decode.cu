@@ -45,6 +45,7 @@ struct S2Params {
     int64_t al_sb, al_sh, al_ss;
     int32_t S, B;
     Stage1Grid grid;                     // stage 1's launch; ncta = 0: equal splits per sequence
+    ShareDivisors by;                    // of it
     void *o;
     int32_t o_bf16;
     int64_t o_sb, o_sh;
@@ -59,24 +60,29 @@ struct S2Params {
     int32_t *status;
 };
 
+__device__ __forceinline__ float warp_max(float x) {                     // over the lanes; a NaN is ignored where there is anything else
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
 typedef void (*Stage2Kernel)(S2Params);
 constexpr int S2_MAX_TAIL = 256;
 constexpr int S2_MAX_SPLITS = 1024;
 
-// One CTA per (query head, sequence).  Warps stripe over the bf16 residual rows for the logits,
-// then over the splits for the combine; every loop keeps many independent loads in flight,
-// because this kernel is pure latency (a few hundred KB through L2).
+// One CTA per (query head, sequence).  Warps stripe over the bf16 residual rows, then over the splits for the combine.  Few rows are a
+// chain of round trips (lengths, rows, splits: 64 KB to an SM at 127 splits), many are bound by instruction issue, so logits are MMAs,
+// the lse of a turn's splits is one load with a split to a lane, maxima are one instruction, and nothing divides but the
+// share-out: 980 instructions a warp before.  Behind stage 1, both stages, before -> now: 256 rows 17.5 -> 16.9 us,
+// 512 19.0 -> 18.7, 1024 50.2 -> 48.0, 2048 56.5 -> 53.9; 32 rows 4K 11.5 -> 11.35, 16K 18.57 -> 18.44, 2K 9.26 -> 9.4.  Requesting the
+// splits before the residual rows are worked in helps where a block starts late and costs as much where it waits early (1K 8.8 -> 10.3).
 // Four sizes (NW warps, PER_SM blocks to an SM), by what the rows of the grid need to run side by side (chosen in
-// launch_stage2): the more registers a row can have, the more of its loads are in flight at once, but a second round of blocks
-// costs more than that gains.  What it adds to a layer behind stage 1, against one row to 16 / 8 / 4 warps with a load
-// round for every six residual rows: 32 rows 4.3 -> 3.6 us, 256 rows 6.3 -> 3.9, 512 rows 10.3 -> 5.7, 1024 rows 16.7 -> 9.1,
-// 2048 rows 22.0 -> 11.9.  Spills undo it (80 registers at <8, 3>: 6.2 us for 256 rows).
+// launch_stage2): the more warps a row can have, the more of its loads are in flight at once, but a second round of blocks
+// costs more than that gains (4K, 32 rows: 16 warps 12.5 us, 8 warps 13.9, 4 warps 15.6).
 // CLUSTER: stage 1 was launched in clusters.  Choosing between its two plans in every launch cost 0.1 us (32 layers at 4K 389 -> 392 us).
 template <int NW, int PER_SM, bool CLUSTER>
 __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2Params p) {
-    __shared__ __align__(16) float s_q[HD];
-    __shared__ float s_w[NW];
-    __shared__ float s_red[NW];
+    __shared__ __align__(16) uint16_t s_q[HD];
+    __shared__ float s_m[NW], s_den[NW];
     __shared__ __align__(16) float s_acc[NW][HD];
     // the next kernel in the stream (the following layer's stage 1) may be placed as SMs free up; it waits for
     // this grid to finish before it touches memory
@@ -87,8 +93,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     int tail = p.b_tail_len ? p.b_tail_len[b] : 0;                       // requested before the lengths are waited for
     // Lengths: this sequence's, and what the share-out of stage 1 depends on (all, longest, those before this one), in one
     // round of loads.
-    const int seq = p.b_seq_len[b];
-    int total = groups_of(seq), longest = total, before = 0;
+    const int groups = groups_of(p.b_seq_len[b]);
+    int total = groups, longest = groups, before = 0;
     if (p.B > 1) {
         total = 0;
         for (int i = lane; i < p.B; i += 32) {
@@ -103,106 +109,103 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     }
     tail = max(0, min(tail, min(p.max_tail, S2_MAX_TAIL)));
     const int D = p.D;                                                   // == HD
-    // workspace slots stage 1 wrote for this sequence
-    const int groups = groups_of(seq);
-    int nsplit = 0;
-    if (p.S > 0 && groups > 0) {
-        int per = 0;
-        const ShareDivisors by = share_divisors(p.grid, p.S);
-        if constexpr (CLUSTER) per = share_plan_of(total, longest, p.B, p.S, p.grid, by).per;
-        else if (p.grid.ncta > 0) per = share_plan_of(total, longest, p.B, p.S, by.ctas, p.grid.waves, by).per;
-        if (per == 0) {
-            const int equal = (groups + p.S - 1) / p.S;
-            nsplit = (groups + equal - 1) / equal;
-        } else {
-            nsplit = (before + groups - 1) / per - before / per + 1;
-        }
-    }
-    const float *base = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh;
 
-    constexpr int PRE_S = NW == 16 ? 10 : 5;                              // splits per warp held in registers
+    // workspace slots stage 1 wrote for this sequence: worked out while the residual rows are on their way
+    int nsplit = 0;
+    auto count_splits = [&]() __attribute__((always_inline)) {
+        if (p.S > 0 && groups > 0) {
+            int per = 0;
+            if constexpr (CLUSTER) per = share_plan_of(total, longest, p.B, p.S, p.grid, p.by).per;
+            else if (p.grid.ncta > 0) per = share_plan_of(total, longest, p.B, p.S, p.by.ctas, p.grid.waves, p.by).per;
+            if (per == 0) {
+                const int equal = p.by.slots.of(groups + p.S - 1);
+                nsplit = (groups + equal - 1) / equal;
+            } else {
+                nsplit = (before + groups - 1) / per + 1;
+                if (before > 0) nsplit -= before / per;
+            }
+        }
+    };
     // ---- bf16 residual rows of this q head: they do not depend on stage 1, so everything about them happens before its end is
     //      waited for ----
-    // A warp takes rows warp, warp + NW, ..., four of them at a time for the logits: eight lanes to a row, three exchanges
-    // for four rows, and KB such batches in flight at once, K and V together: the rows a window usually has (8 + 32 + up to 31) in
-    // one turn of the loop, in two where seven blocks share an SM's registers.
-    constexpr int KB = NW == 16 ? 2 : (PER_SM == 4 ? 5 : 3);
-    float m_t = -INFINITY, den_t = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;    // v: channels 4 lane .. 4 lane + 3
+    // A warp takes rows warp, warp + NW, ..., eight to a batch: their K and V are requested together, the logits are eight MMAs with
+    // the rows as the columns and q in every row of A, and the next batch takes over the softmax state.  Products of bf16 values are
+    // exact, and the eight sums of sixteen are added in fp32 as a tree: an accumulator that ran through the MMAs would cut off
+    // low bits.  The rows a window usually has (8 + 32 + up to 31) are one turn of the loop with 16 warps, two with 8 and three with 4.
+    float m_w = -INFINITY, den_w = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;    // v: channels 4 lane .. 4 lane + 3
     if (tail > 0) {
-        const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * (lane & 7);
-        const __nv_bfloat16 *vt = p.v_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * lane;
+        const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * (lane & 3);
+        const __nv_bfloat16 *vt = p.v_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * lane + (int64_t)warp * p.t_st;
+        const int64_t v_step = (int64_t)NW * p.t_st;
+        uint16_t q_own = 0;
+        if (tid < D) q_own = reinterpret_cast<const uint16_t *>(p.q)[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid];
 #pragma unroll 1
-        for (int r0 = warp; r0 - warp < tail; r0 += NW * 4 * KB) {
-            uint2 kx[KB][4], vx[4 * KB];                                 // K: channels 4 (lane % 8) + 32 i of row lane / 8 of the batch
+        for (int r0 = warp; r0 - warp < tail; r0 += NW * 8) {
+            uint2 kx[8], vx[8];                                          // K: channels 16 i + 4 (lane % 4) .. + 3 of row lane / 4 of the batch
+            {
+                // (a row past the end is the last one again, with weight 0)
+                const __nv_bfloat16 *row = kt + (int64_t)min(r0 + NW * (lane >> 2), tail - 1) * p.t_st;
 #pragma unroll
-            for (int k = 0; k < KB; ++k) {
-                const int r = r0 + NW * (4 * k + (lane >> 3));
+                for (int i = 0; i < 8; ++i) kx[i] = *reinterpret_cast<const uint2 *>(row + 16 * i);
+            }
+            if (p.v_vec_ok) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    kx[k][i] = make_uint2(0u, 0u);
-                    if (r < tail) kx[k][i] = *reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 32 * i);
+                for (int k = 0; k < 8; ++k) {
+                    if (r0 + NW * k >= tail) break;
+                    vx[k] = *reinterpret_cast<const uint2 *>(vt + k * v_step);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (r0 + NW * k >= tail) break;
+                    const uint16_t *e = reinterpret_cast<const uint16_t *>(vt + k * v_step);
+                    vx[k] = make_uint2(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16));
                 }
             }
-            auto load_v = [&](int k) __attribute__((always_inline)) {
-                const int r = r0 + NW * k;
-                vx[k] = make_uint2(0u, 0u);
-                if (r < tail) {
-                    const __nv_bfloat16 *row = vt + (int64_t)r * p.t_st;
-                    if (p.v_vec_ok) vx[k] = *reinterpret_cast<const uint2 *>(row);
-                    else {
-                        const uint16_t *e = reinterpret_cast<const uint16_t *>(row);
-                        vx[k] = make_uint2(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16));
-                    }
-                }
-            };
-            constexpr int V_FIRST = PER_SM == 1 ? 4 * KB : (PER_SM <= 4 ? 2 * KB : KB);   // the registers of the K rows hold the others
-#pragma unroll
-            for (int k = 0; k < V_FIRST; ++k) load_v(k);
             if (r0 == warp) {
-                if (tid < D) s_q[tid] = __bfloat162float(p.q[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid]);
+                count_splits();
+                if (tid < D) s_q[tid] = q_own;
                 __syncthreads();
             }
-            float x[KB], mx = -INFINITY;
+            float x[2], part[3][2], mx = -INFINITY;                      // x: rows 2 (lane % 4) and one more of the batch
 #pragma unroll
-            for (int k = 0; k < KB; ++k) x[k] = 0.f;
+            for (int i = 0; i < 8; ++i) {
+                const uint2 q = *reinterpret_cast<const uint2 *>(s_q + 16 * i + 4 * (lane & 3));
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_bf16(acc, q.x, q.x, q.y, q.y, kx[i].x, kx[i].y);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 q = *reinterpret_cast<const float4 *>(s_q + 4 * (lane & 7) + 32 * i);
-#pragma unroll
-                for (int k = 0; k < KB; ++k)
-                    x[k] += q.x * bf16_bits_to_f32(kx[k][i].x & 0xFFFFu) + q.y * bf16_bits_to_f32(kx[k][i].x >> 16)
-                          + q.z * bf16_bits_to_f32(kx[k][i].y & 0xFFFFu) + q.w * bf16_bits_to_f32(kx[k][i].y >> 16);
+                for (int e = 0; e < 2; ++e) {                            // a tree over the eight
+                    float t = acc[e];
+                    if (i & 1) t += part[0][e];
+                    if ((i & 3) == 3) t += part[1][e];
+                    if (i == 7) x[e] = t + part[2][e];
+                    else part[(i & 1) == 0 ? 0 : ((i & 3) == 1 ? 1 : 2)][e] = t;
+                }
             }
 #pragma unroll
-            for (int k = V_FIRST; k < 4 * KB; ++k) load_v(k);
-#pragma unroll
-            for (int k = 0; k < KB; ++k) {
-#pragma unroll
-                for (int o = 4; o > 0; o >>= 1) x[k] += __shfl_xor_sync(0xFFFFFFFFu, x[k], o);
-                x[k] *= p.sm_scale;
-                if (p.logit_cap > 0.f) x[k] = p.logit_cap * tanhf(x[k] / p.logit_cap);
-                if (r0 + NW * (4 * k + (lane >> 3)) >= tail) x[k] = -INFINITY;
-                mx = fmaxf(mx, x[k]);
+            for (int e = 0; e < 2; ++e) {
+                x[e] *= p.sm_scale;
+                if (p.logit_cap > 0.f) x[e] = p.logit_cap * tanhf(x[e] / p.logit_cap);
+                if (r0 + NW * (2 * (lane & 3) + e) >= tail) x[e] = -INFINITY;
+                mx = fmaxf(mx, x[e]);
             }
-            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 8));
-            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 16));
-            const float m_new = fmaxf(m_t, mx), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_t - m_use);
-            m_t = m_new;
-            den_t *= corr; v0 *= corr; v1 *= corr; v2 *= corr; v3 *= corr;
+            const float m_new = fmaxf(m_w, warp_max(mx)), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_w - m_use);
+            m_w = m_new;
+            den_w *= corr; v0 *= corr; v1 *= corr; v2 *= corr; v3 *= corr;
 #pragma unroll
-            for (int k = 0; k < KB; ++k) {
-                x[k] = __expf(x[k] - m_use);                             // 0 for the rows past the end
-                den_t += x[k];
-            }
+            for (int e = 0; e < 2; ++e) x[e] = __expf(x[e] - m_use);     // 0 for the rows past the end
 #pragma unroll
-            for (int k = 0; k < 4 * KB; ++k) {
-                const float w = __shfl_sync(0xFFFFFFFFu, x[k >> 2], 8 * (k & 3));
+            for (int k = 0; k < 8; ++k) {
+                if (r0 + NW * k >= tail) break;
+                const float w = __shfl_sync(0xFFFFFFFFu, x[k & 1], k >> 1);
+                den_w += w;
                 v0 += w * bf16_bits_to_f32(vx[k].x & 0xFFFFu); v1 += w * bf16_bits_to_f32(vx[k].x >> 16);
                 v2 += w * bf16_bits_to_f32(vx[k].y & 0xFFFFu); v3 += w * bf16_bits_to_f32(vx[k].y >> 16);
             }
+            vt += 8 * v_step;
         }
-        den_t += __shfl_xor_sync(0xFFFFFFFFu, den_t, 8);
-        den_t += __shfl_xor_sync(0xFFFFFFFFu, den_t, 16);
+    } else {
+        count_splits();
     }
     // the channels lane + 32 i, as the rows of the splits are read
     *reinterpret_cast<float4 *>(&s_acc[warp][4 * lane]) = make_float4(v0, v1, v2, v3);
@@ -212,61 +215,50 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     //      programmatic launch) ----
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // Every warp folds its own splits (warp, warp + NW, ...) into its softmax state of the residual rows - maximum, sum of
-    // weights, weighted rows - with no exchange: the lse of a split is read by all lanes at once (one address).  The NW states are
-    // merged once at the end.  The split rows are requested together with the lse values, not after the weights are
-    // known: the kernel is a chain of global round trips and this takes one link out of it.
-    float spre[PRE_S][4], lpre[PRE_S];
+    // weights, weighted rows - and the NW states are merged once at the end.  The rows of PRE_S splits are requested together with their
+    // lse values, not after the weights are known; lane k holds the lse and the weight of the k-th of them.
+    constexpr int PRE_S = NW == 16 ? 10 : 5;
+    const float *row = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh + (int64_t)warp * p.al_ss + lane;
+    const int64_t step = (int64_t)NW * p.al_ss;
+#pragma unroll 1
+    for (int s0 = warp; s0 < nsplit; s0 += PRE_S * NW) {
+        float sx[PRE_S][4];
 #pragma unroll
-    for (int k = 0; k < PRE_S; ++k) {
-        const int s = warp + k * NW;
-        spre[k][0] = spre[k][1] = spre[k][2] = spre[k][3] = 0.f;
-        lpre[k] = -INFINITY;
-        if (s < nsplit) {
-            const float *row = base + (int64_t)s * p.al_ss;
-            spre[k][0] = row[lane]; spre[k][1] = row[lane + 32]; spre[k][2] = row[lane + 64]; spre[k][3] = row[lane + 96];
-            lpre[k] = row[D];
+        for (int k = 0; k < PRE_S; ++k) {
+            if (s0 + k * NW >= nsplit) break;
+            const float *r = row + k * step;
+            sx[k][0] = r[0]; sx[k][1] = r[32]; sx[k][2] = r[64]; sx[k][3] = r[96];
         }
-    }
-    float m_w = m_t;
+        float l = -INFINITY;
+        if (lane < PRE_S && s0 + lane * NW < nsplit) l = row[lane * step + D - lane];
+        row += PRE_S * step;
+        const float m_new = fmaxf(m_w, warp_max(l)), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_w - m_use);
+        m_w = m_new;
+        l = __expf(l - m_use);
+        den_w *= corr; a0 *= corr; a1 *= corr; a2 *= corr; a3 *= corr;
 #pragma unroll
-    for (int k = 0; k < PRE_S; ++k) m_w = fmaxf(m_w, lpre[k]);
-    for (int s = warp + PRE_S * NW; s < nsplit; s += NW) m_w = fmaxf(m_w, base[(int64_t)s * p.al_ss + D]);
-    const float m_safe = (m_w == -INFINITY) ? 0.f : m_w;
-    // weighted sum: lane owns channels lane + 32*i
-    const float f_t = __expf(m_t - m_safe);                              // 0 without residual rows
-    float den_w = den_t * f_t;
-    a0 *= f_t; a1 *= f_t; a2 *= f_t; a3 *= f_t;
-#pragma unroll
-    for (int k = 0; k < PRE_S; ++k) {
-        const float w = __expf(lpre[k] - m_safe);                        // exp(-inf) = 0 for the slots past nsplit
-        den_w += w;
-        a0 += w * spre[k][0]; a1 += w * spre[k][1]; a2 += w * spre[k][2]; a3 += w * spre[k][3];
-    }
-#pragma unroll 4
-    for (int s = warp + PRE_S * NW; s < nsplit; s += NW) {
-        const float *row = base + (int64_t)s * p.al_ss;
-        const float w = __expf(row[D] - m_safe);
-        den_w += w;
-        a0 += w * row[lane]; a1 += w * row[lane + 32]; a2 += w * row[lane + 64]; a3 += w * row[lane + 96];
+        for (int k = 0; k < PRE_S; ++k) {
+            if (s0 + k * NW >= nsplit) break;
+            const float w = __shfl_sync(0xFFFFFFFFu, l, k);
+            den_w += w;
+            a0 += w * sx[k][0]; a1 += w * sx[k][1]; a2 += w * sx[k][2]; a3 += w * sx[k][3];
+        }
     }
     s_acc[warp][lane] = a0; s_acc[warp][lane + 32] = a1;
     s_acc[warp][lane + 64] = a2; s_acc[warp][lane + 96] = a3;
-    if (lane == 0) { s_red[warp] = m_w; s_w[warp] = den_w; }
+    if (lane == 0) { s_m[warp] = m_w; s_den[warp] = den_w; }
     __syncthreads();
-    // ---- merge of the NW states ----
+    // ---- merge of the NW states: lane w of each warp has the weight of state w ----
     float out = 0.f;
     if (tid < D) {
-        float g_max = s_red[0];
+        const float m = lane < NW ? s_m[lane] : -INFINITY, g_max = warp_max(m), g_safe = (g_max == -INFINITY) ? 0.f : g_max;
+        const float e = __expf(m - g_safe);                              // 0 for a warp that saw nothing
+        float den = lane < NW ? s_den[lane] * e : 0.f, acc = 0.f;
 #pragma unroll
-        for (int w = 1; w < NW; ++w) g_max = fmaxf(g_max, s_red[w]);
-        const float g_safe = (g_max == -INFINITY) ? 0.f : g_max;
-        float acc = 0.f, den = 0.f;
+        for (int o = NW / 2; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);
+        den = __shfl_sync(0xFFFFFFFFu, den, 0);
 #pragma unroll
-        for (int w = 0; w < NW; ++w) {
-            const float e = __expf(s_red[w] - g_safe);                   // 0 for a warp that saw nothing
-            acc = fmaf(s_acc[w][tid], e, acc);
-            den = fmaf(s_w[w], e, den);
-        }
+        for (int w = 0; w < NW; ++w) acc = fmaf(s_acc[w][tid], __shfl_sync(0xFFFFFFFFu, e, w), acc);
         out = acc / (den > 0.f ? den : 1.f);
         if (p.o_bf16) reinterpret_cast<__nv_bfloat16 *>(p.o)[(int64_t)b * p.o_sb + (int64_t)hq * p.o_sh + tid] = __float2bfloat16_rn(out);
         else reinterpret_cast<float *>(p.o)[(int64_t)b * p.o_sb + (int64_t)hq * p.o_sh + tid] = out;
@@ -663,6 +655,7 @@ static int launch_stage2(const ommx_decode_args *a, cudaStream_t st, bool tc, bo
     p.B = a->batch; p.grid = Stage1Grid{0, 0, 1, 0};
     if (p.S > 0)
         if (int rc = shared_grid(a, tc, &p.grid)) return rc;
+    p.by = share_divisors(p.grid, max(p.S, 1));
     p.o = a->o; p.o_bf16 = (a->o_dtype == OMMX_DT_BF16); p.o_sb = a->o_stride_b; p.o_sh = a->o_stride_h;
     p.lse = a->lse; p.lse_sb = a->lse_stride_b;
     p.sm_scale = a->sm_scale; p.logit_cap = a->logit_cap;

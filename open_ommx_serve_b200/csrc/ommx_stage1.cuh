@@ -49,6 +49,23 @@ struct Stage1Grid { int32_t ncta, waves, cluster, cluster_waves; };
 // What it is made for: SMs, and how many clusters of 2, 4 and 8 CTAs of one SM each run at once
 struct Chip { int sms, clusters[3]; };
 
+// Division by what a launch knows beforehand: stage 1 prepares the reciprocals before it waits for the kernel ahead of it (three divisions
+// between the lengths and the first copy were 0.8 us of every launch; from the host, among the parameters, 8 x 32K 136.7 -> 137.1),
+// stage 2, of which they were a quarter of the instructions, gets them from the host.  Exact: with m = floor((2^32 - 1) / d) the product's upper half
+// is the quotient or one less.
+struct Divisor {
+    uint32_t d, m;
+    __host__ __device__ __forceinline__ int of(int n) const {        // n / d for n >= 0
+        const uint32_t q = (uint32_t)(((uint64_t)(uint32_t)n * m) >> 32);
+        return (int)(q + ((uint32_t)n - q * d >= d ? 1u : 0u));
+    }
+};
+__host__ __device__ __forceinline__ Divisor divisor(int d) { return Divisor{(uint32_t)d, 0xFFFFFFFFu / (uint32_t)d}; }
+struct ShareDivisors { Divisor ctas, shares, slots, slots1; };        // CTAs, clusters, S, S - 1
+__host__ __device__ __forceinline__ ShareDivisors share_divisors(const Stage1Grid &g, int S) {
+    return ShareDivisors{divisor(max(g.ncta, 1)), divisor(max(g.ncta / max(g.cluster, 1), 1)), divisor(S), divisor(max(S - 1, 1))};
+}
+
 struct S1Params {
     const __nv_bfloat16 *q;
     int64_t q_sb, q_sh;
@@ -379,21 +396,6 @@ struct SharePlan {
     int per, total;                      // groups per share (0: equal splits per sequence), groups of all sequences
     int ctas, shares;                    // CTAs to a share, shares
 };
-// Division by what a launch knows beforehand: stage 1 prepares the reciprocals before it waits for the kernel ahead of it.  (Three divisions
-// between the lengths and the first copy were 0.8 us of every launch.)  Exact: with m = floor((2^32 - 1) / d) the product's upper half
-// is the quotient or one less.
-struct Divisor {
-    uint32_t d, m;
-    __host__ __device__ __forceinline__ int of(int n) const {        // n / d for n >= 0
-        const uint32_t q = (uint32_t)(((uint64_t)(uint32_t)n * m) >> 32);
-        return (int)(q + ((uint32_t)n - q * d >= d ? 1u : 0u));
-    }
-};
-__host__ __device__ __forceinline__ Divisor divisor(int d) { return Divisor{(uint32_t)d, 0xFFFFFFFFu / (uint32_t)d}; }
-struct ShareDivisors { Divisor ctas, shares, slots, slots1; };        // CTAs, clusters, S, S - 1
-__host__ __device__ __forceinline__ ShareDivisors share_divisors(const Stage1Grid &g, int S) {
-    return ShareDivisors{divisor(max(g.ncta, 1)), divisor(max(g.ncta / max(g.cluster, 1), 1)), divisor(S), divisor(max(S - 1, 1))};
-}
 __host__ __device__ __forceinline__ int groups_of(int seq) { return seq > 0 ? (seq + 31) >> 5 : 0; }
 __host__ __device__ __forceinline__ SharePlan share_plan_of(int total, int longest, int B, int S, const Divisor &ncta, int waves, const ShareDivisors &by) {
     SharePlan s;
@@ -1269,7 +1271,7 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
     };
 
     // ---- roles; each branch resizes its warpgroups' register budget and never rejoins.  What needs no earlier kernel is done before the
-    //      wait for it: clearing the tiles, the reciprocals of the share-out's divisions, the decode warps' registers (both
+    //      wait for it: clearing the tiles, the decode warps' registers (both
     //      stages in a graph: 1K 10.35 -> 9.3 us, 4K 12.5 -> 11.6, 16K 19.5 -> 18.5, 64K 41.6 -> 41.0; with the MMA warps' registers ahead
     //      of it too 11.8 and 41.1, 8 x 32K 136.4 -> 137.3).  The wide layout's producers start the pieces first, which 24
     //      registers do not hold, and its MMA warps need what they give back. ----

@@ -121,6 +121,16 @@ def test_decode_groups_shared_over_the_ctas(lens, H, splits):
     _run_and_check(Case(lens, H=H, Hq=4 * H, seed=17), num_kv_splits=splits)
 
 
+@pytest.mark.parametrize("batch,Hq", [(2, 32), (8, 32), (8, 64), (32, 32)])
+def test_decode_more_splits_than_a_turn_of_the_combine(batch, Hq):
+    """One long sequence among short ones fills up to 125 workspace slots: one to seven turns of the combine in each block size."""
+    case = Case([40 + 32 * 250] + [72] * (batch - 1), Hq=Hq, seed=batch)
+    # against exact attention: q * sm_scale and the outliers' deltas are rounded to bf16, each 2^-9 of every product at most
+    bound = max((case.q[b].float().abs() * case.sm_scale @ case.per_seq[b]["K"][:, h].abs().T)[h * Hq // 8:(h + 1) * Hq // 8].max().item()
+                for b in (0, 1) for h in range(8)) * 2 ** -8
+    _run_and_check(case, num_kv_splits=148, lse_atol_fp32=bound)
+
+
 @pytest.mark.parametrize("H,n,long,at,splits", [(2, 200, 200, 0, None), (2, 200, 200, 199, None), (8, 200, 200, 100, 3),
                                                 (2, 300, 129, 299, 2)])        # the last: a CTA lists as many as it can
 def test_decode_many_short_sequences_beside_a_longer_one(H, n, long, at, splits):
