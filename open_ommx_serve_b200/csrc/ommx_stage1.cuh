@@ -609,6 +609,8 @@ constexpr size_t stage1_smem(int stages, int stage_bytes, int groups, int pages_
 // at four warps a scheduler); 16 delta warps with their own MMAs beside 8 output warps (46.1 / 167); tile rows zeroed by an
 // out-of-range tensor-map load (83 / 289); FP4 levels by the conversion instruction and a shorter wait loop (53 fewer
 // instructions per unit, same time).
+// With one or two kv heads a unit costs more: 1856 and 1692 instructions and 428 and 448 wavefronts (103 and 139 of them bank conflicts,
+// 111 at eight heads), because a token row of theirs is 32 or 64 bytes, staged without a swizzle, and a stage has eight or four groups.
 // PLAIN: the recipes that are served - bitmask or relidx7 index, outlier map, no logit cap, no differential-timing knob, a page layout that
 // leaves room for the usual ring depth - with every choice between those made at compile time, plane offsets included.  The general
 // form keeps them at run time; its tests and address arithmetic inside the unit cost it 12 to 15 % (both stages: 64K
