@@ -835,6 +835,15 @@ struct GroupRows {
     }
 };
 
+// Rows of the page planes (page, row in the page, head) and of the group planes (slot, head) are counted in 32 bits without a sign, which
+// count_rows_in_32_bits says is enough.
+__device__ __forceinline__ uint32_t page_row(uint32_t page, uint32_t page_size, uint32_t in_page, uint32_t heads, uint32_t h) {
+    return (page * page_size + in_page) * heads + h;
+}
+static bool count_rows_in_32_bits(const ommx_kv_planes &pl) {
+    return (int64_t)pl.num_pages * pl.page_size * pl.n_kv_heads < (1ll << 32) && (int64_t)pl.num_group_slots * pl.n_kv_heads < (1ll << 32);
+}
+
 // nibbles 0..4 of two channels, where 4 (saturated) is code 3, to nibbles of two codes
 __device__ __forceinline__ uint32_t join_codes(uint32_t a, uint32_t b) {
     return (a + 4u * b) - (((a >> 2) & 0x11111111u) | (b & 0x44444444u));
@@ -850,7 +859,7 @@ __device__ __forceinline__ uint32_t fp4_code(float m) {
 }
 
 // col: this lane's channels 2 lane, 2 lane + 1 in row 0; the unit's destination group slot and head, and of the lane's token the page and
-// the row in it.  Rows of planes are counted in 32 bits.
+// the row in it
 template <typename T, int KT, int KB>
 __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, const GroupRows &rows, int slot, int h, int blk, int page, int in_page, int lane) {
     typedef Pair16<T> P;
@@ -990,7 +999,7 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
 
     // ---- per-channel planes: two adjacent entries a lane ----
     if (slot >= 0) {
-        const int64_t off = (int64_t)((uint64_t)(uint32_t)(slot * p.H + h) * (uint32_t)p.D + (uint32_t)(64 * blk + 2 * lane));
+        const int64_t off = (int64_t)((uint64_t)((uint32_t)slot * (uint32_t)p.H + (uint32_t)h) * (uint32_t)p.D + (uint32_t)(64 * blk + 2 * lane));
         auto put16 = [&](void *plane, float a, float b) {
             if (store_f32) *reinterpret_cast<float2 *>(reinterpret_cast<float *>(plane) + off) = make_float2(a, b);
             else *reinterpret_cast<uint32_t *>(reinterpret_cast<uint16_t *>(plane) + off) = f32_to_bf16_bits(a) | (f32_to_bf16_bits(b) << 16);
@@ -1046,7 +1055,7 @@ __device__ __forceinline__ void pack_k_pair(const PackKParams &p, const T *col, 
     }
     // lane = token now: its 16 code bytes of these 64 channels
     if (page >= 0)
-        *reinterpret_cast<uint4 *>(p.k_base + (uint64_t)(uint32_t)((page * p.page_size + in_page) * p.H + h) * (uint32_t)(p.D / 4) + 16 * blk) =
+        *reinterpret_cast<uint4 *>(p.k_base + (uint64_t)page_row(page, p.page_size, in_page, p.H, h) * (uint32_t)(p.D / 4) + 16 * blk) =
             make_uint4(cw[0], cw[1], cw[2], cw[3]);
 }
 
@@ -1153,7 +1162,7 @@ __global__ void __launch_bounds__(PACK_WARPS * 32, PACK16_CTAS) pack16_kernel(co
         const bool write = page >= 0 && page < vp.num_pages;
         if (!write) or_status(vp.status, OMMX_ST_BAD_PAGE);
         pack_v_group<T>(vp, reinterpret_cast<const T *>(vp.v) + (int64_t)t * vp.stride_token + (int64_t)h * vp.stride_head + cg * 32,
-                        ((uint32_t)page * by.page.d + (t - p0 * by.page.d)) * by.heads.d + h, write, cg);
+                        page_row(page, by.page.d, t - p0 * by.page.d, by.heads.d, h), write, cg);
     }
 }
 
@@ -1202,8 +1211,7 @@ static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
         const int k = kp.k_out;
         if (kp.select_signed && kp.D % 64 == 0 && all % 16 == 0 && a->stride_token % 8 == 0 && a->stride_head % 8 == 0 &&
             a->stride_token >= 0 && a->stride_token < (1 << 25) &&
-            (k == 0 || k == 2 || k == 4 || k == 6 || k == 8) && nthreads < (1ll << 31) - 128 && (int64_t)pl.num_pages * pl.page_size * kp.H < (1ll << 32) &&
-            (int64_t)pl.num_group_slots * kp.H < (1ll << 32)) {
+            (k == 0 || k == 2 || k == 4 || k == 6 || k == 8) && nthreads < (1ll << 31) - 128 && count_rows_in_32_bits(pl)) {
             if (nthreads == 0) return 0;
             const PackDivs by{fast_div(kp.H), fast_div(kp.page_size), fast_div(kp.D / 64), fast_div(kp.D / 32)};
             const int k_blocks = (kp.num_groups * kp.H * (kp.D / 64) + PACK_WARPS - 1) / PACK_WARPS;
@@ -1389,8 +1397,8 @@ __global__ void __launch_bounds__(256) kv_gather_tail_kernel(GatherParams p) {
 //   * the length is advanced once every CTA of the row's cluster has read it (a cluster barrier).
 // Bound by latency, one chain slot -> length -> rows: at batch 32 the issue slots are 26 % and DRAM 10 % busy, and waiting for loads is
 // the largest stall.  A step in which a quarter of the rows complete a group takes twice one in which none does (18.3 and 9.1 us, cold).
-// Measured: 17 -> 4 us at batch 1, 8 heads.  Needs recent >= 1, whole 64-channel units and 16-byte pieces; launch_append keeps the
-// separate kernels for anything else.
+// Measured: 17 -> 4 us at batch 1, 8 heads.  Needs recent >= 1, whole 64-channel units, 16-byte pieces and rows that 32 bits count;
+// launch_append keeps the separate kernels for anything else.
 // ---------------------------------------------------------------------------------------------
 constexpr int STORE_CTAS = 8, STORE_THREADS = 256;
 template <int KT, int KB>
@@ -1484,7 +1492,7 @@ __global__ void __cluster_dims__(STORE_CTAS, 1, 1) __launch_bounds__(STORE_THREA
                 const int page = pages[(grp * 32 + t) / vp.page_size];
                 const bool write = page >= 0 && page < vp.num_pages;
                 if (!write) or_status(p.status, OMMX_ST_BAD_PAGE);
-                pack_v_group<T>(vp, p.v_hist + base + rows.at(t) + h * p.D + cg * 32, (uint32_t)(page * vp.page_size + t % vp.page_size) * p.H + h, write, cg);
+                pack_v_group<T>(vp, p.v_hist + base + rows.at(t) + h * p.D + cg * 32, page_row(page, vp.page_size, t % vp.page_size, p.H, h), write, cg);
             }
         }
     }
@@ -1564,7 +1572,7 @@ static int launch_append(const ommx_kv_append_args *a, cudaStream_t st) {
     const uintptr_t all = (uintptr_t)pool.k_hist | (uintptr_t)pool.v_hist | (uintptr_t)a->k_tail | (uintptr_t)a->v_tail | (uintptr_t)a->k_new | (uintptr_t)a->v_new |
                           (uintptr_t)pl.k_base | (uintptr_t)pl.k_scale | (uintptr_t)pl.k_zp | (uintptr_t)pl.k_obmp | (uintptr_t)pl.k_oval |
                           (uintptr_t)pl.k_mapscale | (uintptr_t)pl.k_mapcenter;
-    if (sp.D % 64 == 0 && pool.recent_window >= 1 && all % 16 == 0 && B <= 65535 &&
+    if (sp.D % 64 == 0 && pool.recent_window >= 1 && all % 16 == 0 && B <= 65535 && count_rows_in_32_bits(pl) &&
         (!a->advance || (a->new_stride_b % 8 == 0 && a->new_stride_h % 8 == 0))) {
         switch (kp.k_out) {
             case 0: return launch_store<0, 0>(sp, kp, vp, B, st);

@@ -292,3 +292,60 @@ def test_refusals():
     pool = _pool(1, 256, 2)
     with pytest.raises(ValueError):
         pool.append_decode_device(torch.zeros(1, 2, 128, device="cuda"), torch.zeros(1, 2, 128, device="cuda"), 1)
+
+
+def test_store_and_prefill_into_page_rows_past_2_31():
+    """More rows (page, row, head) than a signed 32-bit count holds, the request in the last of them; 82 GB, nearly all untouched."""
+    from open_ommx_serve_b200.attention.kv_pool import MultiSeqKVPool
+    from open_ommx_serve_b200.attention.kv_window import WindowSpec
+    H, D, ps, T = 8, 64, 16, SINK + RECENT + 64
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 100 GB of free device memory")
+    pool = MultiSeqKVPool(D, H, 1, 256, window=WindowSpec(SINK, RECENT, 32, ps), device="cuda")
+    P = (1 << 31) // (ps * H) + pool.P_per_seq
+    for name in ("k_base", "v_main", "v_scale", "v_zp"):
+        t = pool.planes[name]
+        pool.planes[name] = torch.empty((P,) + t.shape[1:], dtype=t.dtype, device="cuda")
+    pool._req_to_token.copy_(torch.arange(P - 1, P - 1 - pool.P_per_seq, -1, dtype=torch.int32, device="cuda")[None])
+    K, V = gaussian_kv(17, T + 32, H, D)
+    pool.append_block(0, K[:T].cuda().bfloat16(), V[:T].cuda().bfloat16())
+    for t in range(T, T + 32):
+        pool.append_decode_device(K[t:t + 1].cuda().bfloat16(), V[t:t + 1].cuda().bfloat16(), 1)
+    assert int(pool.status.item()) == 0 and pool.seq_dev.tolist() == [T + 32]
+    want = O.pack_kv(K[SINK:SINK + 96].numpy(), V[SINK:SINK + 96].numpy(), outliers_per_vector=6, page_size=ps)
+    got = {n: (t[P - 6:].flip(0) if n in ("k_base", "v_main", "v_scale", "v_zp") else t[:3]) for n, t in pool.planes.items() if t is not None}
+    assert_planes_equal(got, want, ctx="high rows: ")
+
+
+@pytest.mark.parametrize("pages,launches", [((1 << 28) - 1, 1), (1 << 28, 5)])
+def test_store_step_counts_its_rows_in_32_bits(pages, launches):
+    """Up to 2^32 rows of the page planes the store is one launch, above them the separate kernels, which count in 64 bits.  The planes are
+    said to be that large; the pages that the tables name are there."""
+    from open_ommx_serve_b200 import _lib
+    from open_ommx_serve_b200.attention.pack import planes_struct
+    H, T = 1, SINK + RECENT + 31                                  # the next row completes the first group
+    pool = _pool(1, 256, H)
+    K, V = gaussian_kv(23, T + 1, H, 128)
+    pool.append_block(0, K[:T].cuda().bfloat16(), V[:T].cuda().bfloat16())
+    new = torch.stack([K[T], V[T]]).cuda().bfloat16()
+    a = _lib.KVAppendArgs()
+    a.pool.planes = planes_struct(pool.planes, k=6, outlier_map=True)
+    a.pool.planes.num_pages = pages
+    a.pool.k_hist, a.pool.v_hist, a.pool.seq_len = (t.data_ptr() for t in (pool.k_hist, pool.v_hist, pool.seq_dev))
+    a.pool.req_to_token, a.pool.req_to_group = pool._req_to_token.data_ptr(), pool._req_to_group.data_ptr()
+    a.pool.num_seqs, a.pool.ring_cap, a.pool.sink_tokens, a.pool.recent_window = 1, pool.ring_cap, SINK, RECENT
+    a.pool.pages_per_seq, a.pool.groups_per_seq = pool.P_per_seq, pool.G_per_seq
+    a.k_new, a.v_new, a.new_stride_b, a.new_stride_h = new[0].data_ptr(), new[1].data_ptr(), H * 128, 128
+    a.batch, a.advance, a.outlier_select, a.use_pow2 = 1, 1, 1, 1
+    a.k_tail, a.v_tail, a.max_tail = pool.k_tail.data_ptr(), pool.v_tail.data_ptr(), pool.max_tail_len
+    a.b_seq_len, a.b_tail_len, a.status = pool.b_seq.data_ptr(), pool.b_tail.data_ptr(), pool.status.data_ptr()
+    lib = _lib.load()
+    torch.cuda.synchronize()
+    before = lib.ommx_b200_launch_count()
+    _lib.check(lib.ommx_b200_kv_append_decode(_lib.C.byref(a), torch.cuda.current_stream().cuda_stream), "append")
+    torch.cuda.synchronize()
+    assert lib.ommx_b200_launch_count() - before == launches
+    assert int(pool.status.item()) == 0 and pool.seq_dev.tolist() == [T + 1]
+    want = O.pack_kv(K[SINK:SINK + 32].numpy(), V[SINK:SINK + 32].numpy(), outliers_per_vector=6, page_size=16)
+    assert_planes_equal(_seq_planes(pool, 0, 1), want, ctx=f"{pages} pages: ")
