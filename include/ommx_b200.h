@@ -347,6 +347,8 @@ const char *ommx_b200_last_error(void);   /* thread-local text of the last negat
  * mirrors launch_stats()/reset_launch_stats() (attention/paged_decode.py:2728-2739). */
 int64_t ommx_b200_launch_count(void);
 void ommx_b200_reset_launch_count(void);
+/* Tensor maps encoded since load: decode calls on planes that were decoded before encode none. */
+int64_t ommx_b200_tensor_map_encodings(void);
 
 #ifdef __cplusplus
 }

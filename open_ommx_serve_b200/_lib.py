@@ -123,6 +123,7 @@ SYMBOLS = {
     "ommx_b200_last_error": (C.c_char_p, []),
     "ommx_b200_launch_count": (C.c_int64, []),
     "ommx_b200_reset_launch_count": (None, []),
+    "ommx_b200_tensor_map_encodings": (C.c_int64, []),
 }
 
 _LIB = None

@@ -28,6 +28,9 @@
 // to fp16 (11 bits) instead of bf16.
 #include "ommx_stage1.cuh"
 
+#include <new>
+#include <unordered_map>
+
 namespace ommx {
 
 // =================================================================================================
@@ -430,31 +433,13 @@ static EncodeTiledFn encode_tiled_fn() {
     return st == 1 ? fn : nullptr;
 }
 
+static std::atomic<long long> g_map_encodings{0};
+
 // box_rows > 0: the plane viewed as [bytes/128][128] uint8, box = one page, 128-byte swizzle.  box_rows = 0: the plane viewed as
 // [bytes/row_bytes][row_bytes], box = one row as it lies (for loads of four rows).  Returns false when the map cannot be built.
-// Encoded maps are kept in a small table keyed by (base, bytes, box): a serving loop calls with the
-// same planes every step and the driver call costs about a microsecond.
-static bool make_map(CUtensorMap *m, const void *base, int64_t total_bytes, int row_bytes, int box_rows) {
+static bool encode_map(CUtensorMap *m, const void *base, int64_t total_bytes, int row_bytes, int box_rows) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (fn == nullptr || total_bytes < row_bytes || row_bytes % 16 != 0 || row_bytes > GATHER_ROW_MAX || box_rows > 256) return false;
-    // 512 sets x 4 ways, keyed by (device, base, bytes, box) and compared in full; a set that is
-    // full evicts round-robin.  2048 entries hold the two code planes of a 1000-layer model, all ten planes of 200 layers.
-    struct Entry { const void *base; int64_t bytes; int row, rows, dev; CUtensorMap map; };
-    constexpr int SETS = 512, WAYS = 4;
-    static Entry table[SETS][WAYS];
-    static uint8_t next_way[SETS];
-    static std::mutex mu;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return false; }
-    const uintptr_t key = reinterpret_cast<uintptr_t>(base) >> 8;
-    const size_t set = (size_t)((key ^ (key >> 9) ^ (key >> 18) ^ (uintptr_t)dev * 0x9E37u) % SETS);
-    {
-        std::lock_guard<std::mutex> g(mu);
-        for (int w = 0; w < WAYS; ++w) {
-            const Entry &e = table[set][w];
-            if (e.base == base && e.bytes == total_bytes && e.row == row_bytes && e.rows == box_rows && e.dev == dev) { *m = e.map; return true; }
-        }
-    }
     // a box is at most 256 elements wide
     const int element = row_bytes <= 256 ? 1 : (row_bytes <= 1024 ? 4 : 8);
     const CUtensorMapDataType type = element == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : (element == 4 ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_INT64);
@@ -462,26 +447,81 @@ static bool make_map(CUtensorMap *m, const void *base, int64_t total_bytes, int 
     cuuint64_t gstride[1] = {(cuuint64_t)row_bytes};
     cuuint32_t box[2] = {(cuuint32_t)(row_bytes / element), (cuuint32_t)max(box_rows, 1)};
     cuuint32_t estr[2] = {1, 1};
-    if (fn(m, type, 2, const_cast<void *>(base), gdim, gstride, box, estr,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, box_rows > 0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    std::lock_guard<std::mutex> g(mu);
-    Entry &e = table[set][next_way[set]];
-    next_way[set] = (uint8_t)((next_way[set] + 1) % WAYS);
-    e.base = base; e.bytes = total_bytes; e.row = row_bytes; e.rows = box_rows; e.dev = dev; e.map = *m;
-    return true;
+    g_map_encodings.fetch_add(1, std::memory_order_relaxed);
+    return fn(m, type, 2, const_cast<void *>(base), gdim, gstride, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, box_rows > 0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool make_row_maps(S1GatherParams &p, bool with_index) {
+// The maps of a plane set, kept together: a serving loop calls with the same planes every step, layer after layer, and a
+// call that encodes its ten maps takes the host 8.6 us where one that finds them takes 6.9.  What a map depends on is the key, compared in
+// full.  At most MAX_PLANE_SETS sets (1.6 KB each, 7 MB) are kept, more than the layers of several models; past that the table begins anew, so
+// that planes long gone make room.  (Ten look-ups of single maps took 7.4 us, and a table of 512 sets of four of them encoded
+// 2461 of 3000 maps again in a second round over 300 layers.)
+struct PlaneSetKey {
+    const uint8_t *base[10];             // the planes in the order of S1GatherParams; those that no map is of are null
+    int32_t dev, H, ps, num_pages, num_slots, nbi, nb, by_row;
+    bool operator==(const PlaneSetKey &o) const { return memcmp(this, &o, sizeof(*this)) == 0; }
+};
+static_assert(sizeof(PlaneSetKey) == 10 * 8 + 8 * 4, "compared and hashed as bytes: no padding");
+struct PlaneSetHash {
+    size_t operator()(const PlaneSetKey &k) const {
+        uint64_t w[sizeof(k) / 8], h = 0;
+        memcpy(w, &k, sizeof(k));
+        for (uint64_t x : w) { h = (h ^ x) * 0x9E3779B97F4A7C15ull; h ^= h >> 29; }
+        return (size_t)h;
+    }
+};
+struct PlaneSetMaps { CUtensorMap page_k, page_v, rows[10]; };
+constexpr size_t MAX_PLANE_SETS = 4096;
+
+int set_plane_maps(S1Params &p, CUtensorMap *rows) {
+    if (rows == nullptr && p.H < 4) return 0;
     const uint8_t *base[10] = {p.k_base, p.v_main, p.v_scale, p.v_zp, p.k_scale, p.k_zp, p.k_ms, p.k_mc, p.k_obmp, p.k_oval};
-    const int page = p.ps * p.H, slot = 128 * p.H, page_split = gather_page_split(p.GS * p.ppg), slot_split = gather_slot_split(p.H);
-    const int bytes[10] = {32 * page, 32 * page, 4 * page, 8 * page, slot, 2 * slot, 2 * slot, 2 * slot, p.nbi * slot, p.nb * slot};
-    for (int i = p.H == 4 ? 2 : 0; i < (p.k_out > 0 ? 10 : 6); ++i)
-        if (i != 8 || with_index)
-            if (!make_map(&p.rows[i], base[i], (int64_t)bytes[i] * (i < 4 ? p.num_pages : p.num_slots), bytes[i] / (i < 4 ? page_split : slot_split), 0))
-                return false;
-    return true;
+    const int planes = rows == nullptr ? 2 : (p.k_out > 0 ? 10 : 6);
+    PlaneSetKey key;
+    memset(&key, 0, sizeof(key));
+    for (int i = 0; i < planes; ++i) key.base[i] = base[i];
+    if (int rc = current_device(&key.dev)) return rc;
+    key.H = p.H; key.ps = p.ps; key.num_pages = p.num_pages;
+    if (rows != nullptr) { key.by_row = 1; key.num_slots = p.num_slots; key.nbi = planes == 10 ? p.nbi : 0; key.nb = planes == 10 ? p.nb : 0; }
+    typedef std::unordered_map<PlaneSetKey, PlaneSetMaps, PlaneSetHash> Table;
+    static std::mutex mu;
+    alignas(Table) static unsigned char room[sizeof(Table)];
+    static Table &table = *new (room) Table;                             // never torn down under a thread that still decodes at exit
+    auto hand_out = [&](const PlaneSetMaps &m) {
+        if (p.H >= 4) { p.tmap_k = m.page_k; p.tmap_v = m.page_v; }
+        if (rows != nullptr) memcpy(rows, m.rows, planes * sizeof(CUtensorMap));
+    };
+    {
+        std::lock_guard<std::mutex> g(mu);
+        const auto it = table.find(key);
+        if (it != table.end()) { hand_out(it->second); return 0; }
+    }
+    PlaneSetMaps m;
+    memset(&m, 0, sizeof(m));
+    bool ok = true;
+    if (p.H >= 4) {                                                      // a page is whole 1 KB swizzle atoms
+        const int64_t bytes = (int64_t)p.num_pages * p.rows_per_page * 128;
+        ok = encode_map(&m.page_k, p.k_base, bytes, 128, p.rows_per_page) && encode_map(&m.page_v, p.v_main, bytes, 128, p.rows_per_page);
+    }
+    if (rows != nullptr) {
+        const int page = p.ps * p.H, slot = 128 * p.H, page_split = gather_page_split(p.GS * p.ppg), slot_split = gather_slot_split(p.H);
+        const int bytes[10] = {32 * page, 32 * page, 4 * page, 8 * page, slot, 2 * slot, 2 * slot, 2 * slot, p.nbi * slot, p.nb * slot};
+        for (int i = p.H == 4 ? 2 : 0; ok && i < planes; ++i) {
+            const int row = bytes[i] / (i < 4 ? page_split : slot_split);
+            if (i == 8 && row > GATHER_ROW_MAX) continue;                // copied slot by slot
+            ok = encode_map(&m.rows[i], base[i], (int64_t)bytes[i] * (i < 4 ? p.num_pages : p.num_slots), row, 0);
+        }
+    }
+    if (!ok) return fail(OMMX_E_CUDA, "stage 1: the tensor maps of the planes could not be encoded");
+    hand_out(m);
+    try {
+        std::lock_guard<std::mutex> g(mu);
+        if (table.size() >= MAX_PLANE_SETS) table.clear();
+        table.emplace(key, m);
+    } catch (const std::bad_alloc &) {}                                  // encoded again at the next call
+    return 0;
 }
 
 static size_t stage1_smem(const S1Params &p) { return stage1_smem(p.nstages, p.stage_bytes, p.GS, p.ppg); }
@@ -581,18 +621,13 @@ static int fill_stage1(const ommx_decode_args *a, S1Params &p) {
     p.o_ov = (p.o_bm + H * 128 * p.nbi + 15) / 16 * 16;
     p.gb_bytes = p.o_ov + H * 128 * (p.nb > 0 ? p.nb : 0);
     // swizzled tensor-map staging of the two code planes when a page is whole 1 KB swizzle atoms and
-    // the 1 KB rounding of the group block still fits shared memory (4 or 8 local kv heads)
+    // the 1 KB rounding of the group block still fits shared memory (4 or 8 local kv heads); set_plane_maps fills in the maps
     const int64_t page_bytes = (int64_t)p.ps * H * 32;
     p.swz = 0;
     p.rows_per_page = (int32_t)(page_bytes / 128);
     memset(&p.tmap_k, 0, sizeof(CUtensorMap));
     memset(&p.tmap_v, 0, sizeof(CUtensorMap));
-    if (H >= 4) {                                                        // a page is whole 1 KB swizzle atoms
-        if (!make_map(&p.tmap_k, pl.k_base, (int64_t)pl.num_pages * page_bytes, 128, p.rows_per_page) ||
-            !make_map(&p.tmap_v, pl.v_main, (int64_t)pl.num_pages * page_bytes, 128, p.rows_per_page))
-            return fail(OMMX_E_CUDA, "stage 1: the tensor maps of the code planes could not be encoded");
-        p.swz = 0x70u;
-    }
+    if (H >= 4) p.swz = 0x70u;                                           // a page is whole 1 KB swizzle atoms
     const int round_to = p.swz ? 1024 : 128;
     p.gb_bytes = (p.gb_bytes + round_to - 1) / round_to * round_to;
     p.stage_bytes = (p.GS * p.gb_bytes + 1023) / 1024 * 1024;
@@ -607,6 +642,7 @@ static int shared_grid(const ommx_decode_args *a, bool tc, Stage1Grid *grid) {
         S1Params p;
         TcParams T;
         if (int rc = fill_stage1(a, p)) return rc;
+        if (int rc = set_plane_maps(p, nullptr)) return rc;              // what stage 1 refuses, stage 2 by itself refuses too
         if (tensor_core_plan(a, p, &T)) { *grid = Stage1Grid{0, 0, 1, 0}; return 0; }
     }
     return stage1_launch(a, grid);
@@ -617,6 +653,7 @@ static int launch_stage1(const ommx_decode_args *a, cudaStream_t st, bool tc) {
     S1Params p;
     if (int rc = fill_stage1(a, p)) return rc;
     if (tc) {
+        if (int rc = set_plane_maps(p, nullptr)) return rc;
         TcParams T;
         if (const size_t tsmem = tensor_core_plan(a, p, &T)) {
             dim3 tgrid(a->num_kv_splits, a->batch);
@@ -773,6 +810,8 @@ extern "C" int ommx_b200_host_share_plan(const int32_t *b_seq_len, int32_t batch
     *groups_per_cta = plan.groups_per_share;
     return limit;
 }
+
+extern "C" int64_t ommx_b200_tensor_map_encodings(void) { return (int64_t)ommx::g_map_encodings.load(); }
 
 extern "C" int ommx_b200_decode_stage1(const ommx_decode_args *a, void *stream) {
     int rc = ommx::validate_decode(a);

@@ -1817,8 +1817,9 @@ static int launch_s1(const typename Stage1Form<H, PLAIN>::Params &p, size_t smem
     count_launch();
     return 0;
 }
-// The row maps of a launch for one to four kv heads (not of an outlier index whose rows are too long); false when one cannot be built.
-bool make_row_maps(S1GatherParams &p, bool with_index);
+// The tensor maps of a launch: of the code planes by page where that is how they are staged (4 and 8 kv heads), into p, and with `rows` those
+// of the planes by row (not of an outlier index whose rows are too long).
+int set_plane_maps(S1Params &p, CUtensorMap *rows);
 
 // The form that can exchange states only in launches of clusters, the general form too: in the others its code costs 2 to 6 % (both
 // stages, with -> without, 8 kv heads: 4K, k = 3 13.4 -> 12.6 us; 64K, k = 3 44.7 -> 43.5, with a logit cap 53.9 -> 52.6; 70B heads
@@ -1827,8 +1828,9 @@ template <int KOUT, int H, bool PLAIN, bool IDX7>
 static int launch_s1_form(const S1Params &q, size_t smem, cudaStream_t st) {
     typename Stage1Form<H, PLAIN>::Params p;
     static_cast<S1Params &>(p) = q;
-    if constexpr (Stage1Form<H, PLAIN>::GATHER)
-        if (!make_row_maps(p, PlainLayout<KOUT, H, IDX7>::ROWS_FIT)) return fail(OMMX_E_CUDA, "stage 1: the tensor maps of the planes could not be encoded");
+    CUtensorMap *rows = nullptr;
+    if constexpr (Stage1Form<H, PLAIN>::GATHER) rows = p.rows;
+    if (int rc = set_plane_maps(p, rows)) return rc;
     return p.grid.cluster > 1 ? launch_s1<KOUT, H, PLAIN, IDX7, true>(p, smem, st) : launch_s1<KOUT, H, PLAIN, IDX7, false>(p, smem, st);
 }
 // The plain form where the recipe and the ring depth are its own, else the general one.

@@ -166,6 +166,26 @@ def test_decode_few_heads_empty_pool(H):
     assert torch.equal(o, again) and torch.equal(lse, lse2)
 
 
+@pytest.mark.parametrize("H,layers", [(1, 300), (2, 300), (4, 300), (8, 300), (1, 4200)])
+def test_decode_plane_sets_keep_their_tensor_maps(H, layers):
+    """A loop over many layers' planes encodes maps in its first round only; past the 4096 sets that are kept it encodes again, and right."""
+    from open_ommx_serve_b200 import _lib
+    case = Case([104, 72], H=H, Hq=4 * H, seed=H)
+    o, lse = case.run(num_kv_splits=2)
+    every = {n: t.unsqueeze(0).repeat((layers,) + (1,) * t.dim()) for n, t in case.planes.items()}
+    count = _lib.load().ommx_b200_tensor_map_encodings
+    start, seen = count(), []
+    for rounds in range(2):
+        for i in range(layers):
+            case.planes = {n: t[i] for n, t in every.items()}
+            again, lse2 = case.run(num_kv_splits=2)
+            if i % 64 == 0 or i == layers - 1:
+                assert torch.equal(o, again) and torch.equal(lse, lse2), i
+        seen.append(count() - start)
+    assert seen[0] == layers * (2 if H == 8 else 10)
+    assert layers > 4096 or seen[1] == seen[0]
+
+
 @pytest.mark.parametrize("Hq,aligned", [(8, True), (16, True), (32, True), (64, True), (8, False), (64, False)])
 def test_decode_residual_row_counts(Hq, aligned):
     """Residual rows around the batches and turns of stage 2's loop, in each of its block sizes."""
