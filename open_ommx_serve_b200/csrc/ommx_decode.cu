@@ -72,20 +72,23 @@ typedef void (*Stage2Kernel)(S2Params);
 constexpr int S2_MAX_TAIL = 256;
 constexpr int S2_MAX_SPLITS = 1024;
 
-// One CTA per (query head, sequence).  Warps stripe over the bf16 residual rows, then over the splits for the combine.  Few rows are a
-// chain of round trips (lengths, rows, splits: 64 KB to an SM at 127 splits), many are bound by instruction issue, so logits are MMAs,
-// the lse of a turn's splits is one load with a split to a lane, maxima are one instruction, and nothing divides but the
-// share-out: 980 instructions a warp before.  Behind stage 1, both stages, before -> now: 256 rows 17.5 -> 16.9 us,
-// 512 19.0 -> 18.7, 1024 50.2 -> 48.0, 2048 56.5 -> 53.9; 32 rows 4K 11.5 -> 11.35, 16K 18.57 -> 18.44, 2K 9.26 -> 9.4.  Requesting the
-// splits before the residual rows are worked in helps where a block starts late and costs as much where it waits early (1K 8.8 -> 10.3).
+// One CTA per (query head, sequence).  Warps stripe over the bf16 residual rows, then over the splits for the combine; every loop keeps
+// many independent loads in flight.  Few rows are a chain of round trips (lengths, residual rows, splits: 64 KB to an SM at 127 splits),
+// many are bound by instruction issue too, so the divisions of the share-out are multiplications by what the host prepared and lie
+// where the residual rows are on their way, and a warp's maximum is one instruction.  Both stages, us a layer in a graph, with three
+// divisions ahead of the loads and maxima by exchanges -> now, 8 kv heads: 32 rows 4K 11.0 -> 10.6, 16K 18.5 -> 18.0; at 1835 tokens 64
+// rows 11.6 -> 11.0, 128 15.1 -> 14.4, 256 19.5 -> 18.8, 704 23.9 -> 23.2, 1280 33.3 -> 32.3, 2048 50.6 -> 49.2; 512 rows 4K 28.1 -> 27.2.
+// Requesting the splits before the residual rows are worked in helps where a block starts late and costs as much where it waits
+// early (1K 8.8 -> 10.3).  Logits by MMA took fewer instructions, but the sum of sixteen products is cut off where a
+// multiply-add rounds (logits 5 % further from 64 bits), and eight rows to a batch made turns of 32 rows (704 rows 24.8, 1280 35.7, 2048 52.3).
 // Four sizes (NW warps, PER_SM blocks to an SM), by what the rows of the grid need to run side by side (chosen in
 // launch_stage2): the more warps a row can have, the more of its loads are in flight at once, but a second round of blocks
 // costs more than that gains (4K, 32 rows: 16 warps 12.5 us, 8 warps 13.9, 4 warps 15.6).
 // CLUSTER: stage 1 was launched in clusters.  Choosing between its two plans in every launch cost 0.1 us (32 layers at 4K 389 -> 392 us).
 template <int NW, int PER_SM, bool CLUSTER>
 __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2Params p) {
-    __shared__ __align__(16) uint16_t s_q[HD];
-    __shared__ float s_m[NW], s_den[NW];
+    __shared__ __align__(16) float s_q[HD];
+    __shared__ float s_w[NW], s_red[NW];
     __shared__ __align__(16) float s_acc[NW][HD];
     // the next kernel in the stream (the following layer's stage 1) may be placed as SMs free up; it waits for
     // this grid to finish before it touches memory
@@ -131,81 +134,85 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     };
     // ---- bf16 residual rows of this q head: they do not depend on stage 1, so everything about them happens before its end is
     //      waited for ----
-    // A warp takes rows warp, warp + NW, ..., eight to a batch: their K and V are requested together, the logits are eight MMAs with
-    // the rows as the columns and q in every row of A, and the next batch takes over the softmax state.  Products of bf16 values are
-    // exact, and the eight sums of sixteen are added in fp32 as a tree: an accumulator that ran through the MMAs would cut off
-    // low bits.  The rows a window usually has (8 + 32 + up to 31) are one turn of the loop with 16 warps, two with 8 and three with 4.
-    float m_w = -INFINITY, den_w = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;    // v: channels 4 lane .. 4 lane + 3
+    // A warp takes rows warp, warp + NW, ..., four of them to a batch for the logits: eight lanes to a row, sixteen channels to a lane, three
+    // exchanges for four rows; and KB such batches in a turn of the loop, and the next turn takes over the softmax state.  The rows a
+    // window usually has (8 + 32 + up to 31) are one turn, or two (of 48) where seven blocks share an SM's registers.
+    constexpr int KB = NW == 16 ? 2 : (PER_SM == 4 ? 5 : 3), ROWS = 4 * KB;
+    constexpr int V_FIRST = PER_SM == 1 ? ROWS : (PER_SM <= 4 ? ROWS / 2 : ROWS / 4);   // the registers of the K rows hold the others
+    float m_t = -INFINITY, den_t = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;    // v: channels 4 lane .. 4 lane + 3
     if (tail > 0) {
-        const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * (lane & 3);
+        const __nv_bfloat16 *kt = p.k_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * (lane & 7);
         const __nv_bfloat16 *vt = p.v_tail + (int64_t)b * p.t_sb + (int64_t)kvh * p.t_sh + 4 * lane + (int64_t)warp * p.t_st;
         const int64_t v_step = (int64_t)NW * p.t_st;
-        uint16_t q_own = 0;
-        if (tid < D) q_own = reinterpret_cast<const uint16_t *>(p.q)[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid];
+        float q_own = 0.f;
+        if (tid < D) q_own = __bfloat162float(p.q[(int64_t)b * p.q_sb + (int64_t)hq * p.q_sh + tid]);
 #pragma unroll 1
-        for (int r0 = warp; r0 - warp < tail; r0 += NW * 8) {
-            uint2 kx[8], vx[8];                                          // K: channels 16 i + 4 (lane % 4) .. + 3 of row lane / 4 of the batch
-            {
-                // (a row past the end is the last one again, with weight 0)
-                const __nv_bfloat16 *row = kt + (int64_t)min(r0 + NW * (lane >> 2), tail - 1) * p.t_st;
+        for (int r0 = warp; r0 - warp < tail; r0 += NW * ROWS) {
+            uint2 kx[KB][4], vx[ROWS];                                   // K: channels 4 (lane % 8) + 32 i of row lane / 8 of the batch
 #pragma unroll
-                for (int i = 0; i < 8; ++i) kx[i] = *reinterpret_cast<const uint2 *>(row + 16 * i);
-            }
-            if (p.v_vec_ok) {
+            for (int k = 0; k < KB; ++k) {
+                const int r = r0 + NW * (4 * k + (lane >> 3));
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    if (r0 + NW * k >= tail) break;
-                    vx[k] = *reinterpret_cast<const uint2 *>(vt + k * v_step);
+                for (int i = 0; i < 4; ++i) {
+                    kx[k][i] = make_uint2(0u, 0u);
+                    if (r < tail) kx[k][i] = *reinterpret_cast<const uint2 *>(kt + (int64_t)r * p.t_st + 32 * i);
                 }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    if (r0 + NW * k >= tail) break;
-                    const uint16_t *e = reinterpret_cast<const uint16_t *>(vt + k * v_step);
+            }
+            auto load_v = [&](int k) __attribute__((always_inline)) {
+                vx[k] = make_uint2(0u, 0u);
+                if (r0 + NW * k >= tail) return;
+                const __nv_bfloat16 *row = vt + k * v_step;
+                if (p.v_vec_ok) vx[k] = *reinterpret_cast<const uint2 *>(row);
+                else {
+                    const uint16_t *e = reinterpret_cast<const uint16_t *>(row);
                     vx[k] = make_uint2(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16));
                 }
-            }
+            };
+#pragma unroll
+            for (int k = 0; k < V_FIRST; ++k) load_v(k);
             if (r0 == warp) {
                 count_splits();
                 if (tid < D) s_q[tid] = q_own;
                 __syncthreads();
             }
-            float x[2], part[3][2], mx = -INFINITY;                      // x: rows 2 (lane % 4) and one more of the batch
+            float x[KB], mx = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint2 q = *reinterpret_cast<const uint2 *>(s_q + 16 * i + 4 * (lane & 3));
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_bf16(acc, q.x, q.x, q.y, q.y, kx[i].x, kx[i].y);
+            for (int k = 0; k < KB; ++k) x[k] = 0.f;
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {                            // a tree over the eight
-                    float t = acc[e];
-                    if (i & 1) t += part[0][e];
-                    if ((i & 3) == 3) t += part[1][e];
-                    if (i == 7) x[e] = t + part[2][e];
-                    else part[(i & 1) == 0 ? 0 : ((i & 3) == 1 ? 1 : 2)][e] = t;
+            for (int i = 0; i < 4; ++i) {
+                const float4 q = *reinterpret_cast<const float4 *>(s_q + 4 * (lane & 7) + 32 * i);
+#pragma unroll
+                for (int k = 0; k < KB; ++k) {
+                    float t = q.x * bf16_bits_to_f32(kx[k][i].x & 0xFFFFu);            // (the product of two bf16 values is exact)
+                    t = __fmaf_rn(q.y, bf16_bits_to_f32(kx[k][i].x >> 16), t);
+                    t = __fmaf_rn(q.z, bf16_bits_to_f32(kx[k][i].y & 0xFFFFu), t);
+                    x[k] = __fadd_rn(x[k], __fmaf_rn(q.w, bf16_bits_to_f32(kx[k][i].y >> 16), t));
                 }
             }
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                x[e] *= p.sm_scale;
-                if (p.logit_cap > 0.f) x[e] = p.logit_cap * tanhf(x[e] / p.logit_cap);
-                if (r0 + NW * (2 * (lane & 3) + e) >= tail) x[e] = -INFINITY;
-                mx = fmaxf(mx, x[e]);
+            for (int k = V_FIRST; k < ROWS; ++k) load_v(k);
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) x[k] += __shfl_xor_sync(0xFFFFFFFFu, x[k], o);
+                x[k] *= p.sm_scale;
+                if (p.logit_cap > 0.f) x[k] = p.logit_cap * tanhf(x[k] / p.logit_cap);
+                if (r0 + NW * (4 * k + (lane >> 3)) >= tail) x[k] = -INFINITY;
+                mx = fmaxf(mx, x[k]);
             }
-            const float m_new = fmaxf(m_w, warp_max(mx)), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_w - m_use);
-            m_w = m_new;
-            den_w *= corr; v0 *= corr; v1 *= corr; v2 *= corr; v3 *= corr;
+            const float m_new = fmaxf(m_t, warp_max(mx)), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_t - m_use);
+            m_t = m_new;
+            den_t *= corr; v0 *= corr; v1 *= corr; v2 *= corr; v3 *= corr;
 #pragma unroll
-            for (int e = 0; e < 2; ++e) x[e] = __expf(x[e] - m_use);     // 0 for the rows past the end
+            for (int k = 0; k < KB; ++k) x[k] = __expf(x[k] - m_use);    // 0 for the rows past the end
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (r0 + NW * k >= tail) break;
-                const float w = __shfl_sync(0xFFFFFFFFu, x[k & 1], k >> 1);
-                den_w += w;
+            for (int k = 0; k < ROWS; ++k) {
+                const float w = __shfl_sync(0xFFFFFFFFu, x[k >> 2], 8 * (k & 3));
+                den_t += w;
                 v0 += w * bf16_bits_to_f32(vx[k].x & 0xFFFFu); v1 += w * bf16_bits_to_f32(vx[k].x >> 16);
                 v2 += w * bf16_bits_to_f32(vx[k].y & 0xFFFFu); v3 += w * bf16_bits_to_f32(vx[k].y >> 16);
             }
-            vt += 8 * v_step;
+            vt += ROWS * v_step;
         }
     } else {
         count_splits();
@@ -218,50 +225,63 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) decode_stage2_kernel(const S2
     //      programmatic launch) ----
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // Every warp folds its own splits (warp, warp + NW, ...) into its softmax state of the residual rows - maximum, sum of
-    // weights, weighted rows - and the NW states are merged once at the end.  The rows of PRE_S splits are requested together with their
-    // lse values, not after the weights are known; lane k holds the lse and the weight of the k-th of them.
-    constexpr int PRE_S = NW == 16 ? 10 : 5;
-    const float *row = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh + (int64_t)warp * p.al_ss + lane;
-    const int64_t step = (int64_t)NW * p.al_ss;
-#pragma unroll 1
-    for (int s0 = warp; s0 < nsplit; s0 += PRE_S * NW) {
-        float sx[PRE_S][4];
+    // weights, weighted rows - with no exchange: the lse of a split is read by all lanes at once (one address).  The NW states are
+    // merged once at the end.  The split rows are requested together with the lse values, not after the weights are
+    // known: the kernel is a chain of global round trips and this takes one link out of it.
+    constexpr int PRE_S = NW == 16 ? 10 : 5;                              // splits per warp held in registers
+    const float *base = p.al + (int64_t)b * p.al_sb + (int64_t)hq * p.al_sh;
+    float spre[PRE_S][4], lpre[PRE_S];
 #pragma unroll
-        for (int k = 0; k < PRE_S; ++k) {
-            if (s0 + k * NW >= nsplit) break;
-            const float *r = row + k * step;
-            sx[k][0] = r[0]; sx[k][1] = r[32]; sx[k][2] = r[64]; sx[k][3] = r[96];
+    for (int k = 0; k < PRE_S; ++k) {
+        const int s = warp + k * NW;
+        spre[k][0] = spre[k][1] = spre[k][2] = spre[k][3] = 0.f;
+        lpre[k] = -INFINITY;
+        if (s < nsplit) {
+            const float *row = base + (int64_t)s * p.al_ss;
+            spre[k][0] = row[lane]; spre[k][1] = row[lane + 32]; spre[k][2] = row[lane + 64]; spre[k][3] = row[lane + 96];
+            lpre[k] = row[D];
         }
-        float l = -INFINITY;
-        if (lane < PRE_S && s0 + lane * NW < nsplit) l = row[lane * step + D - lane];
-        row += PRE_S * step;
-        const float m_new = fmaxf(m_w, warp_max(l)), m_use = (m_new == -INFINITY) ? 0.f : m_new, corr = __expf(m_w - m_use);
-        m_w = m_new;
-        l = __expf(l - m_use);
-        den_w *= corr; a0 *= corr; a1 *= corr; a2 *= corr; a3 *= corr;
+    }
+    float m_w = m_t;
 #pragma unroll
-        for (int k = 0; k < PRE_S; ++k) {
-            if (s0 + k * NW >= nsplit) break;
-            const float w = __shfl_sync(0xFFFFFFFFu, l, k);
-            den_w += w;
-            a0 += w * sx[k][0]; a1 += w * sx[k][1]; a2 += w * sx[k][2]; a3 += w * sx[k][3];
-        }
+    for (int k = 0; k < PRE_S; ++k) m_w = fmaxf(m_w, lpre[k]);
+    for (int s = warp + PRE_S * NW; s < nsplit; s += NW) m_w = fmaxf(m_w, base[(int64_t)s * p.al_ss + D]);
+    const float m_safe = (m_w == -INFINITY) ? 0.f : m_w;
+    // weighted sum: lane owns channels lane + 32*i
+    const float f_t = __expf(m_t - m_safe);                               // 0 without residual rows
+    float den_w = den_t * f_t;
+    a0 *= f_t; a1 *= f_t; a2 *= f_t; a3 *= f_t;
+#pragma unroll
+    for (int k = 0; k < PRE_S; ++k) {
+        const float w = __expf(lpre[k] - m_safe);                        // exp(-inf) = 0 for the slots past nsplit
+        den_w += w;
+        a0 += w * spre[k][0]; a1 += w * spre[k][1]; a2 += w * spre[k][2]; a3 += w * spre[k][3];
+    }
+#pragma unroll 4
+    for (int s = warp + PRE_S * NW; s < nsplit; s += NW) {
+        const float *row = base + (int64_t)s * p.al_ss;
+        const float w = __expf(row[D] - m_safe);
+        den_w += w;
+        a0 += w * row[lane]; a1 += w * row[lane + 32]; a2 += w * row[lane + 64]; a3 += w * row[lane + 96];
     }
     s_acc[warp][lane] = a0; s_acc[warp][lane + 32] = a1;
     s_acc[warp][lane + 64] = a2; s_acc[warp][lane + 96] = a3;
-    if (lane == 0) { s_m[warp] = m_w; s_den[warp] = den_w; }
+    if (lane == 0) { s_red[warp] = m_w; s_w[warp] = den_w; }
     __syncthreads();
-    // ---- merge of the NW states: lane w of each warp has the weight of state w ----
+    // ---- merge of the NW states ----
     float out = 0.f;
     if (tid < D) {
-        const float m = lane < NW ? s_m[lane] : -INFINITY, g_max = warp_max(m), g_safe = (g_max == -INFINITY) ? 0.f : g_max;
-        const float e = __expf(m - g_safe);                              // 0 for a warp that saw nothing
-        float den = lane < NW ? s_den[lane] * e : 0.f, acc = 0.f;
+        float g_max = s_red[0];
 #pragma unroll
-        for (int o = NW / 2; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);
-        den = __shfl_sync(0xFFFFFFFFu, den, 0);
+        for (int w = 1; w < NW; ++w) g_max = fmaxf(g_max, s_red[w]);
+        const float g_safe = (g_max == -INFINITY) ? 0.f : g_max;
+        float acc = 0.f, den = 0.f;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) acc = fmaf(s_acc[w][tid], __shfl_sync(0xFFFFFFFFu, e, w), acc);
+        for (int w = 0; w < NW; ++w) {
+            const float e = __expf(s_red[w] - g_safe);                   // 0 for a warp that saw nothing
+            acc = fmaf(s_acc[w][tid], e, acc);
+            den = fmaf(s_w[w], e, den);
+        }
         out = acc / (den > 0.f ? den : 1.f);
         if (p.o_bf16) reinterpret_cast<__nv_bfloat16 *>(p.o)[(int64_t)b * p.o_sb + (int64_t)hq * p.o_sh + tid] = __float2bfloat16_rn(out);
         else reinterpret_cast<float *>(p.o)[(int64_t)b * p.o_sb + (int64_t)hq * p.o_sh + tid] = out;

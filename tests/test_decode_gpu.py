@@ -186,6 +186,37 @@ def test_decode_plane_sets_keep_their_tensor_maps(H, layers):
     assert layers > 4096 or seen[1] == seen[0]
 
 
+@pytest.mark.parametrize("batch,rounds", [(4, 64), (256, 1)])
+@pytest.mark.parametrize("mag", [1.0, 12.0, 30.0])
+def test_residual_logits_are_no_less_precise_than_fp32_multiply_adds(batch, rounds, mag):
+    """One residual row and nothing packed: lse is that row's logit.  Its distance from the 64-bit product is held to that of fp32
+    multiply-adds in the order of a kernel without MMAs: eight lanes of sixteen channels, their sums exchanged pairwise.  With 8192 logits
+    either mean square is known to 2 %; an accumulator that ran through the MMAs would be 40 to 200 % above."""
+    err = {"kernel": [], "fma": []}
+    for r in range(rounds):
+        case = Case([1] * batch, seed=1000 * r + batch, mag=mag)
+        case.sm_scale = 1.0
+        _, lse = case.run()
+        q = case.q.double().numpy()                                 # [batch, Hq, D]
+        k = case.k_tail[:, 0].double().cpu().numpy().repeat(4, axis=1)
+        prod = (q * k).reshape(batch, 32, 4, 8, 4)                  # channel 32 i + 4 lane + e
+        lanes = np.zeros((batch, 32, 8), dtype=np.float32)
+        for i in range(4):
+            four = prod[:, :, i, :, 0].astype(np.float32)
+            for e in range(1, 4):
+                four = (four + prod[:, :, i, :, e]).astype(np.float32)
+            lanes = lanes + four
+        while lanes.shape[-1] > 1:
+            half = lanes.shape[-1] // 2
+            lanes = lanes[..., :half] + lanes[..., half:]
+        exact = prod.sum(axis=(2, 3, 4))
+        size = np.abs(prod).sum(axis=(2, 3, 4))
+        err["kernel"].append((lse.cpu().numpy() - exact) / size)
+        err["fma"].append((lanes[..., 0] - exact) / size)
+    rms = {n: np.sqrt(np.mean(np.square(e))) for n, e in err.items()}
+    assert rms["kernel"] <= rms["fma"], rms
+
+
 @pytest.mark.parametrize("Hq,aligned", [(8, True), (16, True), (32, True), (64, True), (8, False), (64, False)])
 def test_decode_residual_row_counts(Hq, aligned):
     """Residual rows around the batches and turns of stage 2's loop, in each of its block sizes."""
