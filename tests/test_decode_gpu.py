@@ -131,6 +131,22 @@ def test_decode_more_splits_than_a_turn_of_the_combine(batch, Hq):
     _run_and_check(case, num_kv_splits=148, lse_atol_fp32=bound)
 
 
+@pytest.mark.parametrize("groups,H", [((161, 161), 8), ((321, 300), 2), ((512, 500), 1)])
+def test_decode_more_splits_than_a_turn_of_sixteen_warps(groups, H):
+    """A slot to a group: the combine's largest blocks take 160 slots a turn; the last of two, two and three, three and four turns of them."""
+    import ctypes as C
+    from open_ommx_serve_b200 import _lib
+    splits = max(groups)
+    ctas, per = C.c_int32(), C.c_int32()
+    _lib.load().ommx_b200_host_share_plan((C.c_int32 * 2)(*[32 * g for g in groups]), 2, splits, 32 * splits, 148, C.byref(ctas), C.byref(per))
+    assert per.value == 0                                          # equal splits, of one group each
+    case = Case([40 + 32 * g for g in groups], H=H, Hq=4 * H, seed=splits)
+    # as above
+    bound = max((case.q[b].float().abs() * case.sm_scale @ case.per_seq[b]["K"][:, h].abs().T)[4 * h:4 * h + 4].max().item()
+                for b in (0, 1) for h in range(H)) * 2 ** -8
+    _run_and_check(case, num_kv_splits=splits, lse_atol_fp32=bound)
+
+
 @pytest.mark.parametrize("H,n,long,at,splits", [(2, 200, 200, 0, None), (2, 200, 200, 199, None), (8, 200, 200, 100, 3),
                                                 (2, 300, 129, 299, 2)])        # the last: a CTA lists as many as it can
 def test_decode_many_short_sequences_beside_a_longer_one(H, n, long, at, splits):

@@ -105,3 +105,32 @@ def test_decode_relidx7_outlier_counts_and_bad_position(k, H, page_size):
             assert int(status) == _lib.ST_BAD_GROUP and torch.isfinite(o).all()
         else:
             assert int(status) == 0 and torch.equal(o, o_bm) and torch.equal(lse, lse_bm)
+
+
+@pytest.mark.parametrize("page_size", [8, 16, 32])
+def test_decode_relidx7_rows_too_long_for_a_copy_of_four(page_size):
+    """Twelve outliers of four kv heads: the index rows of a group are 5632 bytes, which are copied slot by slot beside copies of four
+    rows of the other planes.  Sequences that end inside a stage of two groups, table entries past a sequence's end that name no page."""
+    from open_ommx_serve_b200.attention.paged_decode import ommx_paged_decode_attention_canonical
+    k, H = 12, 4
+    case = Case([40 + 32 * n for n in (1, 2, 3, 4, 5, 31, 64)], H=H, Hq=4 * H, seed=page_size, k=k, page_size=page_size)
+    for b, n in enumerate(case.packed):
+        case.req_to_token[b, n // page_size:] = 1 << 20
+        case.req_to_group[b, n // 32:] = 1 << 20
+    obmp = case.pooled_np["k_obmp"]
+    used = np.array([bin(int(w)).count("1") == k for w in obmp.reshape(-1, 4).copy().view(np.uint32)[:, 0]])
+    flat = np.zeros((used.size, (7 * k + 7) // 8), dtype=np.uint8)
+    flat[used] = O.relidx7_from_bitmask(obmp.reshape(-1, 4)[used], k)
+    oidx = torch.from_numpy(flat.reshape(obmp.shape[:-1] + (flat.shape[1],))).cuda()
+    p, status = case.planes, torch.zeros(1, dtype=torch.int32, device="cuda")
+    for splits in (1, 3, None):
+        o_bm, lse_bm = case.run(num_kv_splits=splits, status=status)
+        o, lse = torch.full_like(o_bm, float("nan")), torch.full_like(lse_bm, float("nan"))
+        ommx_paged_decode_attention_canonical(
+            case.q_dev, p["k_base"], p["k_scale"], p["k_zp"], oidx, p["k_oval"], p["v_main"], p["v_scale"], p["v_zp"], case.k_tail,
+            case.v_tail, case.b_tail_len, o, lse, case.req_to_token, case.req_to_group, case.b_seq_len, sm_scale=case.sm_scale,
+            page_size=page_size, k_outliers_per_vector=k, k_fp4_mapscale=p["k_fp4_mapscale"], k_fp4_mapcenter=p["k_fp4_mapcenter"],
+            kv_outlier_map=True, kv_int8_scale=True, num_kv_splits=splits, max_seq_len=max(case.packed), max_tail_len=max(case.tails),
+            status=status)
+        torch.cuda.synchronize()
+        assert int(status) == 0 and torch.equal(o, o_bm) and torch.equal(lse, lse_bm)
