@@ -28,6 +28,31 @@ inline void count_launch(int n = 1) { g_launches.fetch_add(n, std::memory_order_
             return ::ommx::fail(OMMX_E_CUDA, "%s failed: %s", #expr, cudaGetErrorString(_e)); \
     } while (0)
 
+// ---- the current device -----------------------------------------------------------------------
+constexpr int MAX_DEVICES = 64;
+inline int current_device(int *dev) {
+    OMMX_CUDA_TRY(cudaGetDevice(dev));
+    if (*dev < 0 || *dev >= MAX_DEVICES) return fail(OMMX_E_UNSUPPORTED, "device ordinal %d (this build tracks %d devices)", *dev, MAX_DEVICES);
+    return 0;
+}
+
+inline int sm_count_of(int dev) {
+    static std::atomic<int> counts[MAX_DEVICES];
+    int n = counts[dev].load(std::memory_order_acquire);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = 148; }
+        counts[dev].store(n, std::memory_order_release);
+    }
+    return n;
+}
+// of the current device; a B200's where there is none
+inline int sm_count() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < MAX_DEVICES) return sm_count_of(dev);
+    (void)cudaGetLastError();
+    return 148;
+}
+
 // ---- quantizer decision tables --------------------------------------------------------------
 // Host copies (used by the host twins in the C ABI) and device copies in constant memory.
 static const uint32_t kPow2CutHost[256] = {OMMX_POW2_CUT_VALUES};

@@ -774,9 +774,7 @@ extern "C" int ommx_b200_min_num_kv_splits(int32_t max_seq_len, int32_t page_siz
 
 extern "C" int ommx_b200_auto_num_kv_splits(int32_t max_seq_len, int32_t batch, int32_t n_kv_heads) {
     (void)n_kv_heads;                       // one CTA serves all local kv heads of its token range
-    int dev = 0, sm_count = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < ommx::MAX_DEVICES) sm_count = ommx::sm_count_of(dev);
-    else (void)cudaGetLastError();
+    const int sm_count = ommx::sm_count();
     // For sequences of one length in equal splits: one CTA runs per SM, so a launch takes (waves of CTAs) x (groups per CTA +
     // what a CTA costs before and after its steady state, about three groups' worth).  Pick the split count that minimises it:
     // 147 or 148 at batch 1, and e.g. 18 rather than 19 at batch 8, where 152 CTAs would leave a second wave of four.  Ties go to

@@ -1134,7 +1134,7 @@ struct PackDivs { FastDiv heads, page, blocks, groups; };           // by H, pag
 
 // K and V of a block in one launch: the first `k_blocks` CTAs take K (the longer work), the rest V and fill the last wave (in turn with
 // them, one or two K to a V, K ends late: 8192 tokens x 8 heads 17.2 -> 18.4 and 19.6 us).  let_next_in: a dependent launch may be placed as
-// soon as all CTAs are; where they take less than two waves on a B200's 148 SMs, it would fill the SMs unevenly (2048 tokens 7.3 -> 10.4 us, 4096
+// soon as all CTAs are; where they take less than two waves, it would fill the SMs unevenly (2048 tokens 7.3 -> 10.4 us, 4096
 // 9.6 -> 10.8; 6144 12.0 -> 11.8, 8192 14.5 -> 14.2).
 constexpr int PACK16_CTAS = 7;                     // to an SM: 72 registers a thread
 template <typename T, int KT, int KB>
@@ -1218,7 +1218,8 @@ static int launch_pack(const ommx_pack_args *a, cudaStream_t st) {
             const unsigned grid = (unsigned)(k_blocks + (nthreads + 127) / 128);
             void (*const kernel)(PackKParams, PackVParams, PackDivs, uint32_t, int) =
                 k == 0 ? pack16_kernel<T, 0, 0> : (k == 2 ? pack16_kernel<T, 1, 1> : (k == 4 ? pack16_kernel<T, 2, 2> : (k == 6 ? pack16_kernel<T, 3, 3> : pack16_kernel<T, 4, 4>)));
-            OMMX_CUDA_TRY(launch_early(kernel, dim3(grid), PACK_WARPS * 32, st, kp, vp, by, (uint32_t)k_blocks, grid >= 2u * PACK16_CTAS * 148u ? 1 : 0));
+            const int let_next_in = grid >= 2u * PACK16_CTAS * (unsigned)sm_count() ? 1 : 0;
+            OMMX_CUDA_TRY(launch_early(kernel, dim3(grid), PACK_WARPS * 32, st, kp, vp, by, (uint32_t)k_blocks, let_next_in));
             count_launch();
             return 0;
         }

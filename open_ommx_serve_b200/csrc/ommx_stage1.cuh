@@ -1766,23 +1766,6 @@ static cudaError_t launch_overlapping_previous(Kernel kernel, dim3 grid, int thr
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-constexpr int MAX_DEVICES = 64;
-static int current_device(int *dev) {
-    OMMX_CUDA_TRY(cudaGetDevice(dev));
-    if (*dev < 0 || *dev >= MAX_DEVICES) return fail(OMMX_E_UNSUPPORTED, "device ordinal %d (this build tracks %d devices)", *dev, MAX_DEVICES);
-    return 0;
-}
-
-static int sm_count_of(int dev) {
-    static std::atomic<int> counts[MAX_DEVICES];
-    int n = counts[dev].load(std::memory_order_acquire);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = 148; }
-        counts[dev].store(n, std::memory_order_release);
-    }
-    return n;
-}
-
 // Lets `kernel` be launched with up to SMEM_LIMIT of dynamic shared memory; `done` holds what has been done on each device.  Always
 // the limit, not what the call needs: of two threads whose first calls need different sizes, the smaller could come last.
 template <typename Kernel> static int allow_full_smem(Kernel kernel, std::atomic<int> (&done)[MAX_DEVICES], int dev) {

@@ -349,3 +349,55 @@ def test_store_step_counts_its_rows_in_32_bits(pages, launches):
     assert int(pool.status.item()) == 0 and pool.seq_dev.tolist() == [T + 1]
     want = O.pack_kv(K[SINK:SINK + 32].numpy(), V[SINK:SINK + 32].numpy(), outliers_per_vector=6, page_size=16)
     assert_planes_equal(_seq_planes(pool, 0, 1), want, ctx=f"{pages} pages: ")
+
+
+@pytest.mark.parametrize("H,groups", [(8, 256), (8, 173), (7, 256), (3, 1024), (4, 512), (1, 1500)])
+def test_long_prompt_with_a_ring_fill_and_a_decode_close_behind(H, groups):
+    """From two waves of CTAs on the packer lets the ring fill in before it ends.  The same planes as from shorter packs, which the oracle
+    is compared with elsewhere, and the same attention over them, with every launch right behind the one before it."""
+    from open_ommx_serve_b200.attention.pack import alloc_planes, ommx_pack_kv_into
+    from open_ommx_serve_b200.attention.paged_decode import ommx_paged_decode_attention_canonical
+    T = SINK + 32 * groups + RECENT + 5
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ctas = lambda n: -(-n * H * 2 // 4) + -(-32 * n * H * 4 // 128)
+    assert ctas(groups) >= 2 * 7 * sms > ctas(32)
+    pool = _pool(1, T + 32, H)
+    K, V = (x.cuda().bfloat16() for x in gaussian_kv(H + groups, T + 1, H, 128))
+    q = torch.randn(1, 4 * H, 128, device="cuda", generator=torch.Generator("cuda").manual_seed(H)).bfloat16()
+    planes = alloc_planes(2 * groups, groups, H, 128, page_size=16, outliers_per_vector=6)
+    for g in range(0, groups, 32):
+        n = min(32, groups - g)
+        rows = slice(SINK + 32 * g, SINK + 32 * (g + n))
+        ommx_pack_kv_into(K[rows], V[rows], planes, dst_pages=torch.arange(2 * g, 2 * (g + n), dtype=torch.int32, device="cuda"),
+                          dst_groups=torch.arange(g, g + n, dtype=torch.int32, device="cuda"), outliers_per_vector=6)
+
+    def attend(d, planes, tables):
+        if H not in (1, 2, 4, 8):
+            return None                                                # not served
+        o, lse = torch.empty(1, 4 * H, 128, device="cuda"), torch.empty(1, 4 * H, device="cuda")
+        ommx_paged_decode_attention_canonical(
+            q, planes["k_base"], planes["k_scale"], planes["k_zp"], None, planes["k_oval"], planes["v_main"], planes["v_scale"], planes["v_zp"],
+            d["k_tail"], d["v_tail"], d["b_tail_len"], o, lse, *tables, d["b_seq_len"], sm_scale=128 ** -0.5, page_size=16,
+            k_outliers_per_vector=6, bitmap_read=True, k_obmp=planes["k_obmp"], k_fp4_mapscale=planes["k_fp4_mapscale"],
+            k_fp4_mapcenter=planes["k_fp4_mapcenter"], kv_outlier_map=True, kv_int8_scale=True, max_seq_len=d["max_seq_len"],
+            max_tail_len=d["max_tail_len"])
+        return o, lse
+
+    for _ in range(4):
+        for name, t in pool.planes.items():
+            if t is not None:
+                t.zero_()
+        torch.cuda.synchronize()
+        pool.append_block(0, K[:T], V[:T])
+        pool.append_decode_device(K[T:], V[T:], 1)
+        d = pool.decode_inputs_device(1)
+        got_o = attend(d, d["planes"], (d["req_to_token"], d["req_to_group"]))
+        torch.cuda.synchronize()
+        got = _seq_planes(pool, 0, groups)
+        for name, t in got.items():
+            assert torch.equal(t.view(torch.uint8), planes[name].view(torch.uint8)), name
+        assert torch.equal(pool.k_tail[0, SINK:SINK + RECENT + 6], K[T - RECENT - 5:]) and torch.equal(pool.v_tail[0, :SINK], V[:SINK])
+        tables = [torch.arange(n, dtype=torch.int32, device="cuda")[None] for n in (2 * groups, groups)]
+        want_o = attend(d, planes, tables)
+        assert want_o is None or all(torch.equal(a, b) and torch.isfinite(a).all() for a, b in zip(got_o, want_o))
+    assert int(pool.status.item()) == 0
