@@ -215,3 +215,52 @@ def test_pack_16_bit_inputs_report_what_is_not_finite(dtype, value):
             with pytest.raises(ValueError):
                 _gpu_pack(K, V)
             X[t, 1, c] = keep
+
+
+@pytest.mark.parametrize("T,H", [(256, 2), (8192, 8)])
+def test_pack_captured_behind_copies_and_a_join_of_streams(T, H):
+    """In a graph the packer comes behind a kernel, a copy, a memset and two streams at once, on both sides of its early release."""
+    from open_ommx_serve_b200.attention.pack import alloc_planes, ommx_pack_kv_into
+    n, src = 4, [tuple(x.bfloat16().cuda() for x in gaussian_kv(T + i, T, H, 128)) for i in range(2)]
+    inputs = [tuple(torch.empty_like(x) for x in src[0]) for _ in range(n)]
+    planes = [alloc_planes(T // 16, T // 32, H, 128) for _ in range(n)]
+    start, side, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    pack = lambda i: ommx_pack_kv_into(*inputs[i], planes[i], outliers_per_vector=6)
+    pack(0)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=start):
+        for x, y in zip(inputs[0], src[0]):
+            x.copy_(y)                                                 # copies
+        pack(0)
+        for x, y in zip(inputs[1], src[0]):
+            torch.add(y, 0, out=x)                                     # a kernel
+        pack(1)
+        planes[2]["k_base"].zero_()                                    # a memset
+        side.wait_stream(start)
+        with torch.cuda.stream(side):
+            inputs[2][0].copy_(src[0][0])
+            inputs[3][0].copy_(src[0][0])
+        inputs[2][1].copy_(src[0][1])
+        inputs[3][1].copy_(src[0][1])
+        start.wait_stream(side)
+        pack(2)
+        pack(3)
+    for s in (1, 0, 1):
+        if s:
+            keep = [x.clone() for x in src[0]]
+            for x, y in zip(src[0], src[1]):
+                x.copy_(y)
+        want = alloc_planes(T // 16, T // 32, H, 128)
+        ommx_pack_kv_into(*src[0], want, outliers_per_vector=6)
+        torch.cuda.synchronize()
+        for p in planes:
+            for name in PLANES:
+                p[name].view(torch.uint8).fill_(0xA5)
+        graph.replay()
+        torch.cuda.synchronize()
+        for i, p in enumerate(planes):
+            for name in PLANES:
+                assert torch.equal(p[name].view(torch.uint8), want[name].view(torch.uint8)), (i, name)
+        if s:
+            for x, y in zip(src[0], keep):
+                x.copy_(y)
