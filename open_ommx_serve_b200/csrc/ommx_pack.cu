@@ -103,14 +103,10 @@ constexpr int PACK_BLK = 16;                       // channels per warp: one 32-
 
 // RN(x / 3): quotient from the rounded reciprocal, exact remainder by one FMA, corrected quotient (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000", 1990); equal to the division for every x >= 1e-8, infinity included.
-__host__ __device__ __forceinline__ float div_by_3(float x) {
+__device__ __forceinline__ float div_by_3(float x) {
     constexpr float THIRD = 1.f / 3.f;
-#ifdef __CUDA_ARCH__
     const float q = __fmul_rn(x, THIRD), r = __fmaf_rn(-3.f, q, x);
     return r == r ? __fmaf_rn(r, THIRD, q) : q;
-#else
-    return x / 3.f;
-#endif
 }
 
 // scale -> (value after optional pow2 snap and storage rounding, exponent)
@@ -281,8 +277,8 @@ __device__ __forceinline__ void drop_ties_pair(uint32_t (&picks)[2], uint32_t eq
     }
 }
 
-// The M largest (descending) and M smallest (ascending) of 32 values x(0) .. x(31), by a sorting network for M <= 4: blocks of four are
-// sorted, then merged (248 min / max at M = 4).  V is float, or a pair of 16-bit values, whose halves are two channels and on whose
+// The M largest (descending) and M smallest (ascending) of 32 values x(0) .. x(31), by a sorting network for M <= 4: blocks of eight are
+// sorted, then merged (224 min / max at M = 4).  V is float, or a pair of 16-bit values, whose halves are two channels and on whose
 // min and max a NaN wins.  lowest / highest: what every value displaces.
 __device__ __forceinline__ float v_max(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float v_min(float a, float b) { return fminf(a, b); }
@@ -295,7 +291,7 @@ template <typename V> __device__ __forceinline__ void order2(V &a, V &b) {      
 }
 template <int M, int N, typename V, typename Fn>
 __device__ __forceinline__ void extremes_of_32(Fn x, V (&top)[N], V (&bot)[N], V lowest, V highest) {
-    static_assert(N >= 4 && N >= M, "a block of four is sorted in place");
+    static_assert(N >= 4 && N >= M, "the four largest and smallest are kept sorted");
     if constexpr (M == 1) {
         top[0] = bot[0] = x(0);
 #pragma unroll
@@ -1117,13 +1113,7 @@ __device__ __forceinline__ void pack_v_group(const PackVParams &p, const T *row,
 // they were a third of a V thread's instructions.
 struct FastDiv {
     uint32_t d, mul, shift;
-    __host__ __device__ __forceinline__ uint32_t quotient(uint32_t n) const {
-#ifdef __CUDA_ARCH__
-        return __umulhi(2u * n, mul) >> shift;
-#else
-        return (uint32_t)(((uint64_t)(2u * n) * mul) >> 32) >> shift;
-#endif
-    }
+    __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return __umulhi(2u * n, mul) >> shift; }
 };
 static FastDiv fast_div(uint32_t d) {
     uint32_t shift = 0;
