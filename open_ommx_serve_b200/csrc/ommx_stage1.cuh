@@ -1650,6 +1650,7 @@ decode_stage1_kernel(const __grid_constant__ typename Stage1Form<H, PLAIN>::Para
         // All at once: of the head's 32 values a lane holds, warp gsel takes 32 / GS from every warp's tile and writes them out (one
         // warp that merged the others one by one, both stages: 8 x 32K x 1 head 30.6 -> 29.6 us, 8K 11.4 -> 10.3; 128K x 2 heads
         // 28.1 -> 27.4, 4K 10.8 -> 10.3).  Of two warps (four heads) one merges the other's: 32K 19.5 us, together 19.8.
+        // In clusters one warp merges too: it holds the whole state that the CTAs exchange.  Side by side there is not tried.
         store_state();
         asm volatile("bar.sync 3, %0;" ::"n"(NCW * 32) : "memory");
         constexpr int NCG = 8 / GS;
