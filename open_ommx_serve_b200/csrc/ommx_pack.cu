@@ -783,11 +783,11 @@ __global__ void __launch_bounds__(128) pack_v_kernel(PackVParams p) {
 // KT-th (KB-th) value, and where equal values leave too many, the highest tokens go - the stable-sort rule.  The values behind the
 // picks are the base range.  Codes are two FMAs and one shifted add per value: (x - zp) / 4s saturated to [0, 1] in one FMA (one
 // rounding, the same as the subtraction's, because s is a power of two), times 4 onto 1.5 * 2^23, which rounds to nearest even.
-// Bound by instructions: min / max, compares and logic run at half rate in one pipe, which is 69 % busy in a steady state of K (issue slots
-// 69 %), and what can goes to the multiply-add pipe instead (masks of compares summed with powers of two, rows by one wide
+// Bound by instructions: min / max, compares and logic run at half rate in one pipe, which is 55 % busy while an SM has work (issue slots
+// 62 %), and what can goes to the multiply-add pipe instead (masks of compares summed with powers of two, rows by one wide
 // multiply-add, the two channels' codes joined before the saturated ones are put right).  A K warp is 1670 instructions, a V warp
 // 308; with plain divisions for the indices, a vote-free tie test by counts and blocks of four they were 1875 and 442.  Measured, K + V,
-// bf16, one after the other: 8192 tokens x 8 heads (42 MB) 17.2 -> 14.7 us, 32768 tokens 61.9 -> 52.6, 1024 tokens 6.2 -> 5.5, 512 tokens 5.0 -> 4.4.
+// bf16, one after the other on inputs that the L2 holds: 8192 tokens x 8 heads (42 MB) 17.2 -> 14.7 us (flushed 16.9), 32768 tokens 61.9 -> 52.6, 1024 tokens 6.2 -> 5.5, 512 tokens 5.0 -> 4.4.
 // Tried and slower (8192 tokens): V of a unit staged by its K warp (18.8 against 17.2), V rows prefetched into the L2 by the K warps (15.9 against
 // 14.7: their first loads are what the kernel waits for at first), two V pieces a thread (15.1; 32768 tokens 50.2 against 52.1), eight
 // CTAs to an SM with spills (15.0), six (15.9 against 15.4).

@@ -132,8 +132,8 @@ def test_decode_more_splits_than_a_turn_of_the_combine(batch, Hq):
 
 
 @pytest.mark.parametrize("groups,H", [((161, 161), 8), ((321, 300), 2), ((512, 500), 1)])
-def test_decode_more_splits_than_a_turn_of_sixteen_warps(groups, H):
-    """A slot to a group: the combine's largest blocks take 160 slots a turn; the last of two, two and three, three and four turns of them."""
+def test_decode_more_splits_than_sixteen_warps_hold(groups, H):
+    """A slot to a group: the combine's largest blocks hold 160 slots in registers and read what is beyond them in a second pass."""
     import ctypes as C
     from open_ommx_serve_b200 import _lib
     splits = max(groups)
